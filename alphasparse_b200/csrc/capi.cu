@@ -14,8 +14,10 @@
 #include <vector>
 
 #include "../../include/asp_b200.h"
+#include "host_meta.h"
 #include "kernel_args.h"
 #include "kernels.h"
+#include "tiled.h"
 
 namespace
 {
@@ -84,43 +86,7 @@ struct Arena
     }
 };
 
-// host copy of a metadata reference, for validation and shared-memory sizing
-struct HostMeta
-{
-    const void *p = nullptr;
-    int dtype = ASP_U32;
-    uint64_t len = 0;
-    int kind = ASP_COMPRESS_NONE;
-    uint64_t coef = 0, icpt = 0, cycle = 1;
-    int nb = 0;
-    uint64_t bhi[5] = {0, 0, 0, 0, 0}, bval[5] = {0, 0, 0, 0, 0};
-    bool present = false;
-    uint64_t get(uint64_t i) const
-    {
-        switch (kind)
-        {
-        case ASP_COMPRESS_NONE:
-            switch (dtype)
-            {
-            case ASP_U8: return ((const uint8_t *)p)[i];
-            case ASP_U16: return ((const uint16_t *)p)[i];
-            case ASP_U32: return ((const uint32_t *)p)[i];
-            default: return ((const uint64_t *)p)[i];
-            }
-        case ASP_COMPRESS_LINEAR: return i * coef + icpt;
-        case ASP_COMPRESS_CONSTANT: return icpt;
-        case ASP_COMPRESS_CYCLE_LINEAR: return (i % cycle) * coef + icpt;
-        case ASP_COMPRESS_CYCLE_INCREASE: return i / cycle + icpt;
-        default:
-        {
-            uint64_t v = bval[0];
-            for (int b = 1; b < nb; b++)
-                if (i > bhi[b - 1]) v = bval[b];
-            return v;
-        }
-        }
-    }
-};
+using asp::HostMeta;
 } // namespace
 
 struct asp_ctx
@@ -143,9 +109,23 @@ struct asp_ctx
     std::vector<cudaEvent_t> pipe_events;
 };
 
+namespace
+{
+// The column-tiled layout of a whole plan group (tiled.h), shared by its plans
+struct TiledGroup
+{
+    Arena arena;
+    asp::TiledArgs args;
+    int n_plans = 0;
+    unsigned n_sm = 0;
+    bool covers_all_rows = false; // every row of y has an element in some plan
+};
+} // namespace
+
 struct asp_plan
 {
     std::shared_ptr<Arena> arena;
+    std::shared_ptr<TiledGroup> tiled; // null: the group runs the kernels of its templates
     asp::KArgs args;
     int templ = 0;
     int val_is_f64 = 0;
@@ -1027,6 +1007,66 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
         cleanup();
         return ASP_OK;
     }
+    // scattered columns: the column-tiled layout of the whole group (kernels_tiled.cu), where it is the faster one
+    std::vector<asp::TiledSource> src;
+    bool same = true;
+    for (int i = 0; i < n; i++)
+    {
+        same = same && descs[i].val_dtype == descs[0].val_dtype && descs[i].n_rows == descs[0].n_rows && descs[i].n_cols == descs[0].n_cols;
+        if (descs[i].template_type == ASP_EMPTY_TEMPLATE) same = false; // a group with parts left out is a trial of one part
+        if (!same) break;
+        asp::TiledSource t;
+        t.templ = descs[i].template_type;
+        t.m = metas[i].data();
+        t.perm = &perms[i];
+        t.a = &made[i]->args;
+        t.val = vals[i]->host_ptr;
+        t.col = cols[i]->host_ptr;
+        t.col_bytes = dtype_size(cols[i]->dtype);
+        t.stored = vals[i]->len;
+        src.push_back(t);
+    }
+    asp::TiledHost th;
+    std::shared_ptr<TiledGroup> tg;
+    try
+    {
+        if (same && asp::tiled_build(src, descs[0].val_dtype == ASP_F64, descs[0].n_rows, descs[0].n_cols, ctx->sm_count, th)) tg.reset(new TiledGroup());
+    }
+    catch (const std::bad_alloc &) // not enough host memory to build it: the templates' own kernels run
+    {
+    }
+    if (tg)
+    {
+        const void *from[5] = {th.val.p.get(), th.col.p.get(), th.row.p.get(), th.end.p.get(), th.work.data()};
+        const size_t bytes[5] = {th.val.bytes(), th.col.bytes(), th.row.bytes(), th.end.bytes(), th.work.size() * sizeof(uint32_t)};
+        size_t off[6] = {0};
+        for (int k = 0; k < 5; k++) off[k + 1] = align_up(off[k] + bytes[k], 256);
+        tg->arena.device = ctx->device;
+        tg->arena.bytes = off[5];
+        if (cudaMalloc(&tg->arena.base, off[5]) != cudaSuccess)
+        {
+            cudaGetLastError(); // no room on the device: as above
+            tg->arena.base = nullptr;
+            tg.reset();
+        }
+        else
+        {
+            unsigned char *base = (unsigned char *)tg->arena.base;
+            cudaError_t ce = asp::tiled_setup(descs[0].val_dtype == ASP_F64);
+            for (int k = 0; k < 5 && ce == cudaSuccess; k++) ce = cudaMemcpyAsync(base + off[k], from[k], bytes[k], cudaMemcpyHostToDevice, ctx->stream);
+            if (ce != cudaSuccess)
+            {
+                cleanup();
+                return cuda_fail(ce, "upload of the column-tiled layout");
+            }
+            tg->args = {base + off[0], (const uint16_t *)(base + off[1]), (const uint32_t *)(base + off[2]), (const uint32_t *)(base + off[3]),
+                        (const uint4 *)(base + off[4]), nullptr, nullptr, descs[0].n_rows, descs[0].n_cols};
+            tg->n_plans = n;
+            tg->n_sm = (unsigned)ctx->sm_count;
+            tg->covers_all_rows = th.covers_all_rows;
+            for (asp_plan *p : made) p->tiled = tg;
+        }
+    }
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess)
     {
@@ -1077,6 +1117,7 @@ asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path)
 {
     if (!plan) return fail(ASP_ERR_INVALID_ARG, "plan is NULL");
     const int t = plan->templ;
+    plan->tiled.reset(); // the caller experiments with this plan's own kernel
     if (t == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE || t == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE)
     {
         if (vec != 0) return fail(ASP_ERR_INVALID_ARG, "the CSR5-like family has no vec knob");
@@ -1165,6 +1206,26 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
         // a group without any kernel is the zero matrix: "clear when needed" means clear
         clear = g.first == nullptr;
         for (int i = 0; i < n_plans; i++) clear = clear || (plans[i]->templ != ASP_EMPTY_TEMPLATE && plans[i]->needs_zero);
+    }
+    // The whole group in its column-tiled layout. That writes every row of y, so it stands in for the templates' kernels where
+    // y is cleared first anyway, or where they would store every row.
+    const TiledGroup *tg = plans[0]->tiled.get();
+    if (tg && n_plans == tg->n_plans && (clear || (tg->covers_all_rows && zero_y == 2)))
+    {
+        bool whole = true;
+        for (int i = 1; i < n_plans; i++)
+        {
+            whole = whole && plans[i]->tiled.get() == tg;
+            for (int j = 0; j < i; j++) whole = whole && plans[i] != plans[j];
+        }
+        if (whole)
+        {
+            asp::TiledArgs args = tg->args;
+            args.x = d_x;
+            args.y = d_y;
+            ASP_CUDA(asp::launch_tiled(g.es == 8, args, tg->n_sm, ctx->stream));
+            return ASP_OK;
+        }
     }
     if (clear) ASP_CUDA(cudaMemsetAsync(d_y, 0, g.n_rows * g.es, ctx->stream));
     if (!g.first) return ASP_OK;

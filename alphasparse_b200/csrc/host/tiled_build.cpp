@@ -1,0 +1,518 @@
+// Builds the column-tiled layout of a plan group (kernels_tiled.cu) from its template arrays, and decides whether the
+// group is better off with it. One pass over the stored elements counts them per tile of x, one scatters them to
+// their tiles (order of the rows kept), then every tile is cut into blocks of whole rows that are turned into slices
+// independently of one another.
+#include <string.h>
+
+#include <algorithm>
+
+#ifdef _OPENMP
+#include <omp.h>
+#endif
+
+#include "../tiled.h"
+
+namespace asp
+{
+namespace
+{
+typedef uint64_t u64;
+typedef uint32_t u32;
+
+int threads()
+{
+#ifdef _OPENMP
+    return omp_get_max_threads();
+#else
+    return 1;
+#endif
+}
+
+u64 row_in_y(const TiledSource &s, u64 r)
+{
+    if (s.a->sort_kind == ASP_SORT_GLOBAL) return s.perm->get(r + s.a->first_row);
+    if (s.a->sort_kind == ASP_SORT_LOCAL) return s.perm->get(r) + s.a->first_row;
+    return r + s.a->first_row;
+}
+
+// units (what a walk can start at) of a sub-matrix, 0: the template is not walked here
+u64 unit_count(const TiledSource &s)
+{
+    switch (s.templ)
+    {
+    case ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS:
+    case ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE: return s.a->effective;
+    case ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS:
+    case ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS:
+    case ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE:
+    case ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE:
+    case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE:
+    case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE: return s.a->n_units;
+    default: return 0;
+    }
+}
+
+// f(row of y, column of x, value) for every element that units [u0, u1) store. What a format adds to fill a TLB (a zero
+// that repeats the column before it in the same row) is left out.
+template <class VT, class CT, class F>
+void walk(const TiledSource &s, u64 u0, u64 u1, F &&f)
+{
+    const VT *val = (const VT *)s.val;
+    const CT *col = (const CT *)s.col;
+    const KArgs &a = *s.a;
+    const u64 c0 = a.first_col, radd = a.row_add ? a.first_row : 0;
+    const HostMeta *m = s.m;
+    u64 last_row = ~0ull, last_col = ~0ull;
+    auto put = [&](u64 row, u64 at) {
+        const u64 c = (u64)col[at] + c0;
+        const VT v = val[at];
+        if (v == VT(0) && row == last_row && c == last_col) return;
+        last_row = row;
+        last_col = c;
+        f(row, c, v);
+    };
+    switch (s.templ)
+    {
+    case ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS:
+        for (u64 t = u0; t < u1; t++)
+        {
+            const u64 row = m[MS_ROW_OF_TLB].get(t) + radd;
+            for (u64 k = 0; k < a.tlb_size; k++) put(row, t + k * a.n_tlb);
+        }
+        return;
+    case ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS:
+        for (u64 b = u0; b < u1; b++)
+        {
+            const u64 nz = m[MS_BLK_NZ].get(b), t0 = m[MS_BLK_THR].get(b), n = m[MS_BLK_THR].get(b + 1) - t0, S = m[MS_TLB_SIZE].get(b);
+            for (u64 i = 0; i < n && t0 + i < a.effective; i++)
+            {
+                const u64 row = m[MS_ROW_OF_TLB].get(t0 + i) + radd;
+                for (u64 k = 0; k < S; k++) put(row, nz + i + k * n);
+            }
+        }
+        return;
+    case ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS:
+        for (u64 b = u0; b < u1; b++)
+        {
+            const u64 nz = m[MS_BLK_NZ].get(b), n = m[MS_BLK_THR].get(b + 1) - m[MS_BLK_THR].get(b), S = m[MS_TLB_SIZE].get(b);
+            const u64 r0 = m[MS_BLK_ROW].get(b), r1 = std::min<u64>(m[MS_BLK_ROW].get(b + 1), a.effective), g0 = m[MS_ROW_OFF].get(r0);
+            for (u64 r = r0; r < r1; r++)
+            {
+                const u64 row = row_in_y(s, r), e = m[MS_ROW_OFF].get(r + 1) - g0;
+                for (u64 i = m[MS_ROW_OFF].get(r) - g0; i < e; i++)
+                    for (u64 k = 0; k < S; k++) put(row, nz + i + k * n);
+            }
+        }
+        return;
+    case ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE:
+        for (u64 b = u0; b < u1; b++)
+        {
+            const u64 w0 = m[MS_BLK_WARP].get(b), r0 = m[MS_BLK_ROW].get(b), r1 = std::min<u64>(m[MS_BLK_ROW].get(b + 1), a.effective), g0 = m[MS_ROW_OFF].get(r0);
+            for (u64 r = r0; r < r1; r++)
+            {
+                const u64 row = row_in_y(s, r), e = w0 + m[MS_ROW_OFF].get(r + 1) - g0;
+                for (u64 w = w0 + m[MS_ROW_OFF].get(r) - g0; w < e; w++)
+                    for (u64 k = m[MS_WARP_NZ].get(w); k < m[MS_WARP_NZ].get(w + 1); k++) put(row, k);
+            }
+        }
+        return;
+    case ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE:
+    case ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE:
+    {
+        const HostMeta &nz = m[s.templ == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE ? MS_BLK_NZ : MS_WARP_NZ];
+        for (u64 u = u0; u < u1; u++)
+        {
+            const u64 row = m[MS_ROW_OF_UNIT].get(u) + radd, e = nz.get(u + 1);
+            for (u64 k = nz.get(u); k < e; k++) put(row, k);
+        }
+        return;
+    }
+    default: // CSR5-like: the flags of a thread's word say which of its elements start a row; a warp's first element always does
+        for (u64 w = u0; w < u1; w++)
+        {
+            const u64 R0 = m[MS_ROW_OF_UNIT].get(w), S = a.tlb_size;
+            u64 row = ~0ull;
+            for (u64 l = 0; l < 32; l++)
+            {
+                const u64 word = m[MS_COMBINE].get(w * 32 + l);
+                u64 r = R0 + (word & ((1ull << a.bits_row) - 1));
+                for (u64 k = 0; k < S; k++)
+                {
+                    if ((word >> (a.bits_word - 1 - (int)k)) & 1ull) row = row_in_y(s, r++);
+                    if (row != ~0ull) put(row, w * 32 * S + k * 32 + l);
+                }
+            }
+        }
+    }
+}
+
+template <class VT, class F>
+void walk_any(const TiledSource &s, u64 u0, u64 u1, F &&f)
+{
+    if (s.col_bytes == 1) walk<VT, uint8_t>(s, u0, u1, f);
+    else if (s.col_bytes == 2) walk<VT, uint16_t>(s, u0, u1, f);
+    else walk<VT, uint32_t>(s, u0, u1, f);
+}
+
+// Cache lines of x that one warp-wide gather of the group's own kernels touches, per lane (1: every lane another line).
+// Sampled; the kernels with 16-byte lanes gather elements 4 l + j of 128 adjacent ones at a time, the others 32 adjacent ones.
+double lines_per_gather(const TiledSource &s, bool f64)
+{
+    const bool by4 = s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS ||
+                     s.templ == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || s.templ == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE;
+    const u64 groups = s.stored / 128, samples = std::min<u64>(groups, 512), per_line = f64 ? 16 : 32;
+    if (samples == 0) return 0.0;
+    u64 lines = 0;
+    for (u64 q = 0; q < samples; q++)
+    {
+        const u64 base = groups * q / samples * 128;
+        for (int j = 0; j < 4; j++)
+        {
+            u64 ln[32];
+            for (int l = 0; l < 32; l++)
+            {
+                const u64 at = base + (by4 ? 4 * l + j : 32 * j + l);
+                const u64 c = s.col_bytes == 1 ? ((const uint8_t *)s.col)[at] : s.col_bytes == 2 ? ((const uint16_t *)s.col)[at] : ((const u32 *)s.col)[at];
+                ln[l] = c / per_line;
+            }
+            std::sort(ln, ln + 32);
+            lines += (u64)(std::unique(ln, ln + 32) - ln);
+        }
+    }
+    return (double)lines / (double)(samples * 128);
+}
+
+const u32 kMaxPiece = 32;    // elements of a row's piece: bounds the serial chain of a lane and the padding of a slice
+const u32 kWindow = 1024;    // pieces that are sorted by length together: lanes of a slice stay near in y
+const double kSliceCost = 4.0; // in steps; with 2 the CTAs of sparse tiles ran twice as long as the others
+const u64 kBlock = 1u << 16; // elements of a block of whole rows, the unit of the parallel build
+
+struct Chunk
+{
+    int sub;
+    u64 u0, u1;
+};
+
+template <class VT>
+struct Builder
+{
+    const std::vector<TiledSource> &src;
+    const u64 n_rows, n_cols;
+    const u32 TW;
+    const u64 C; // tiles of x
+    std::vector<Chunk> chunks;
+    std::vector<u64> at; // [chunk * C + tile]: first its count, then where its elements go
+    std::vector<u64> tile_begin, tile_pieces;
+    u64 N = 0;
+    // elements in tile order
+    HostBuf<u32> e_row;
+    HostBuf<uint16_t> e_col;
+    HostBuf<VT> e_val;
+
+    Builder(const std::vector<TiledSource> &s, u64 rows, u64 cols) : src(s), n_rows(rows), n_cols(cols), TW(tiled_tile_cols(sizeof(VT) == 8)), C((cols + TW - 1) / TW) {}
+
+    void count(bool &covered)
+    {
+        u64 stored = 0;
+        for (const TiledSource &s : src) stored += s.stored;
+        const u64 want = (u64)threads() * 4;
+        for (size_t i = 0; i < src.size(); i++)
+        {
+            const u64 units = unit_count(src[i]), parts = std::max<u64>(1, std::min<u64>(units, want * src[i].stored / std::max<u64>(stored, 1)));
+            for (u64 p = 0; p < parts; p++) chunks.push_back({(int)i, units * p / parts, units * (p + 1) / parts});
+        }
+        at.assign(chunks.size() * C, 0);
+        tile_pieces.assign(C, 0);
+        std::vector<uint8_t> seen(n_rows, 0);
+#pragma omp parallel
+        {
+            std::vector<u64> pieces(C, 0);
+#pragma omp for schedule(dynamic, 1)
+            for (long long c = 0; c < (long long)chunks.size(); c++)
+            {
+                u64 *n = &at[(size_t)c * C];
+                u64 row = ~0ull, tile = ~0ull, run = 0;
+                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT) {
+                    const u64 t = col / TW;
+                    n[t]++;
+                    if (r != row || t != tile || run == kMaxPiece)
+                    {
+                        pieces[t]++;
+                        seen[r] = 1; // (several threads may store the same 1)
+                        row = r;
+                        tile = t;
+                        run = 0;
+                    }
+                    run++;
+                });
+            }
+#pragma omp critical
+            for (u64 t = 0; t < C; t++) tile_pieces[t] += pieces[t];
+        }
+        u64 missing = 0;
+#pragma omp parallel for schedule(static) reduction(+ : missing)
+        for (long long r = 0; r < (long long)n_rows; r++) missing += seen[r] ? 0 : 1;
+        covered = missing == 0;
+        tile_begin.assign(C + 1, 0);
+        u64 sum = 0;
+        for (u64 t = 0; t < C; t++)
+        {
+            tile_begin[t] = sum;
+            for (size_t c = 0; c < chunks.size(); c++)
+            {
+                const u64 n = at[c * C + t];
+                at[c * C + t] = sum;
+                sum += n;
+            }
+        }
+        tile_begin[C] = N = sum;
+    }
+
+    void scatter()
+    {
+        e_row.make(N);
+        e_col.make(N);
+        e_val.make(N);
+#pragma omp parallel for schedule(dynamic, 1)
+        for (long long c = 0; c < (long long)chunks.size(); c++)
+        {
+            u64 *to = &at[(size_t)c * C];
+            walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) {
+                const u64 t = col / TW, q = to[t]++;
+                e_row.p[q] = (u32)r;
+                e_col.p[q] = (uint16_t)(col - t * TW);
+                e_val.p[q] = v;
+            });
+        }
+    }
+
+    struct Piece
+    {
+        u32 start, len; // start: relative to the block
+    };
+    struct Block
+    {
+        u64 e0, e1;
+        u64 step = 0, slice = 0; // first step and slice of the block
+    };
+
+    // pieces of a block in windows, every window by descending length (rows in order where lengths agree)
+    void pieces_of(const Block &b, std::vector<Piece> &p, std::vector<Piece> &tmp) const
+    {
+        p.clear();
+        for (u64 k = b.e0; k < b.e1;)
+        {
+            u64 q = k + 1;
+            while (q < b.e1 && q - k < kMaxPiece && e_row.p[q] == e_row.p[k]) q++;
+            p.push_back({(u32)(k - b.e0), (u32)(q - k)});
+            k = q;
+        }
+        tmp.resize(p.size());
+        for (size_t i = 0; i < p.size(); i += kWindow)
+        {
+            const size_t e = std::min(p.size(), i + kWindow);
+            u32 cnt[kMaxPiece + 2] = {0};
+            for (size_t j = i; j < e; j++) cnt[kMaxPiece - p[j].len + 1]++;
+            for (u32 l = 1; l <= kMaxPiece; l++) cnt[l] += cnt[l - 1];
+            for (size_t j = i; j < e; j++) tmp[i + cnt[kMaxPiece - p[j].len]++] = p[j];
+        }
+        p.swap(tmp);
+    }
+
+    void slices(int n_sm, TiledHost &out)
+    {
+        std::vector<Block> blocks;
+        std::vector<size_t> tile_block(C + 1, 0);
+        for (u64 t = 0; t < C; t++)
+        {
+            tile_block[t] = blocks.size();
+            for (u64 b = tile_begin[t]; b < tile_begin[t + 1];)
+            {
+                u64 e = std::min(b + kBlock, tile_begin[t + 1]);
+                // whole rows, as long as that does not make the block much longer
+                while (e < tile_begin[t + 1] && e - b < 2 * kBlock && e_row.p[e] == e_row.p[e - 1]) e++;
+                blocks.push_back({b, e});
+                b = e;
+            }
+        }
+        tile_block[C] = blocks.size();
+        const long long B = (long long)blocks.size();
+        std::vector<u64> n_step(B), n_slice(B);
+#pragma omp parallel
+        {
+            std::vector<Piece> p, tmp;
+#pragma omp for schedule(dynamic, 4)
+            for (long long b = 0; b < B; b++)
+            {
+                pieces_of(blocks[b], p, tmp);
+                u64 s = 0;
+                for (size_t i = 0; i < p.size(); i += kTiledSlice) s += p[i].len;
+                n_step[b] = s;
+                n_slice[b] = (p.size() + kTiledSlice - 1) / kTiledSlice;
+            }
+        }
+        u64 steps = 0, nsl = 0;
+        for (long long b = 0; b < B; b++)
+        {
+            blocks[b].step = steps;
+            blocks[b].slice = nsl;
+            steps += n_step[b];
+            nsl += n_slice[b];
+        }
+        const u64 st = steps + kTiledSlackSteps, sl = nsl + kTiledSlackSlices;
+        out.val.make(st * kTiledSlice * sizeof(VT));
+        out.col.make(st * kTiledSlice);
+        out.row.make(sl * kTiledSlice);
+        out.end.make(sl);
+        VT *val = (VT *)out.val.p.get();
+#pragma omp parallel
+        {
+            std::vector<Piece> p, tmp;
+#pragma omp for schedule(dynamic, 4)
+            for (long long b = 0; b < B; b++)
+            {
+                pieces_of(blocks[b], p, tmp);
+                u64 step = blocks[b].step, slice = blocks[b].slice;
+                for (size_t i = 0; i < p.size(); i += kTiledSlice, slice++)
+                {
+                    const u32 depth = p[i].len;
+                    VT *v = val + step * kTiledSlice;
+                    uint16_t *c = out.col.p.get() + step * kTiledSlice;
+                    u32 *rows = out.row.p.get() + slice * kTiledSlice;
+                    memset(v, 0, (size_t)depth * kTiledSlice * sizeof(VT));
+                    std::fill(c, c + (size_t)depth * kTiledSlice, (uint16_t)TW);
+                    for (u32 j = 0; j < kTiledSlice; j++)
+                    {
+                        // piece j goes to lane j % 32, so that one `red` of a warp covers 32 neighbouring pieces
+                        const u32 o = (j % 32) * kTiledLanePieces + j / 32;
+                        rows[o] = kTiledNoRow;
+                        if (i + j >= p.size()) continue;
+                        const u64 e = blocks[b].e0 + p[i + j].start;
+                        rows[o] = e_row.p[e];
+                        for (u32 k = 0; k < p[i + j].len; k++)
+                        {
+                            v[k * kTiledSlice + o] = e_val.p[e + k];
+                            c[k * kTiledSlice + o] = e_col.p[e + k];
+                        }
+                    }
+                    step += depth;
+                    out.end.p[slice] = (u32)step;
+                }
+            }
+        }
+        memset(val + steps * kTiledSlice, 0, kTiledSlackSteps * kTiledSlice * sizeof(VT));
+        memset(out.col.p.get() + steps * kTiledSlice, 0, kTiledSlackSteps * kTiledSlice * sizeof(uint16_t));
+        memset(out.row.p.get() + nsl * kTiledSlice, 0xff, kTiledSlackSlices * kTiledSlice * sizeof(u32));
+        for (u32 i = 0; i < kTiledSlackSlices; i++) out.end.p[nsl + i] = 0xffffffffu;
+        out.nnz = N;
+        out.steps = steps;
+        out.slices = nsl;
+        // work of the CTAs: the steps in order, cut so that every CTA has the same cost: its steps, kSliceCost steps for every
+        // slice (its two `red` and the wait for its rows), and what loading its tiles takes; inside a CTA's share of a tile
+        // the warps are cut the same way
+        std::vector<u64> tile_step(C + 1, steps);
+        for (u64 t = C; t-- > 0;) tile_step[t] = tile_block[t] < blocks.size() ? blocks[tile_block[t]].step : steps;
+        u64 used = 0;
+        for (u64 t = 0; t < C; t++) used += tile_step[t + 1] > tile_step[t] ? 1 : 0;
+        const u32 *end = out.end.p.get();
+        auto slice_of = [&](u64 step) { return (u64)(std::upper_bound(end, end + nsl, (u32)step) - end); };
+        auto cost_of = [&](u64 step) { return (double)step + kSliceCost * (double)slice_of(step); };
+        // the step in [lo, hi] that a cost is reached at
+        auto step_at = [&](double cost, u64 lo, u64 hi) {
+            while (lo < hi)
+            {
+                const u64 mid = (lo + hi) / 2;
+                if (cost_of(mid) >= cost) hi = mid;
+                else lo = mid + 1;
+            }
+            return lo;
+        };
+        const double tile_cost = (double)kTiledTileBytes / (kTiledSlice * (sizeof(VT) + 2.0)); // by bytes
+        const double per = (cost_of(steps) + tile_cost * (double)(used + n_sm - 1)) / n_sm;
+        out.work.assign((size_t)n_sm * kTiledWarps * 4, 0);
+        u64 s = 0, t = 0;
+        double spent = 0; // by the CTAs before this one: what they left or took too much moves on, instead of piling up
+        for (int cta = 0; cta < n_sm; cta++)
+        {
+            double budget = per * (cta + 1) - spent;
+            long long prev = -1;
+            while (s < steps && (cta + 1 == n_sm || prev < 0 || budget > tile_cost + 16))
+            {
+                while (tile_step[t + 1] <= s) t++;
+                budget -= tile_cost;
+                const u64 last = tile_step[t + 1];
+                const double from = cost_of(s);
+                const u64 e = cta + 1 == n_sm ? last : std::min(last, std::max(s + kTiledWarps, step_at(from + budget, s, last)));
+                size_t visit = (size_t)cta;
+                if (prev >= 0)
+                {
+                    visit = out.work.size() / (kTiledWarps * 4);
+                    out.work.resize(out.work.size() + kTiledWarps * 4, 0);
+                    for (u32 w = 0; w < kTiledWarps; w++) out.work[((size_t)prev * kTiledWarps + w) * 4 + 3] |= (u32)visit << 16;
+                }
+                const double all = cost_of(e) - from;
+                u64 at_step = s;
+                for (u32 w = 0; w < kTiledWarps; w++)
+                {
+                    u32 *o = &out.work[(visit * kTiledWarps + w) * 4];
+                    o[0] = (u32)at_step;
+                    at_step = w + 1 == kTiledWarps ? e : step_at(from + all * (w + 1) / kTiledWarps, at_step, e);
+                    o[1] = (u32)at_step;
+                    o[2] = (u32)slice_of(o[0]);
+                    o[3] = (u32)t;
+                }
+                prev = (long long)visit;
+                s = e;
+                budget -= all;
+                spent += tile_cost + all;
+                if (e < last) break;
+            }
+        }
+    }
+};
+
+template <class VT>
+bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm, TiledHost &out)
+{
+    const double sv = sizeof(VT);
+    // The group's own kernels: one request to L2 per cache line that a gather touches (290 G/s on this part, of which they
+    // reach 0.85), or the format's bytes.
+    u64 stored = 0;
+    double lines = 0;
+    for (const TiledSource &s : src)
+    {
+        if (unit_count(s) == 0) return false;
+        stored += s.stored;
+        lines += lines_per_gather(s, sizeof(VT) == 8) * (double)s.stored;
+    }
+    const double own_us = std::max(lines / (0.85 * 290e3), (double)stored * (sv + 4) / 6.0e6);
+    // ... are the better ones where the gathers are not what bounds them, and for small matrices, whose time is the launch
+    if (lines / (0.85 * 290e3) < 1.25 * (double)stored * (sv + 4) / 6.0e6 || own_us < 12.0) return false;
+    if (n_rows >= kTiledNoRow || stored >= (1ull << 37)) return false;
+    Builder<VT> b(src, n_rows, n_cols);
+    if (b.C + (u64)n_sm >= 65536) return false;
+    b.count(out.covers_all_rows);
+    // This layout: 2 + sv bytes per element at 4.6 TB/s, a `red` per piece (a warp's 32 fall into about an eighth as many
+    // lines where the rows of a tile are dense, into 32 where they are sparse), 7 us of launches, tiles and tail.
+    double red = 0;
+    u64 pieces = 0;
+    for (u64 t = 0; t < b.C; t++)
+    {
+        const double p = (double)b.tile_pieces[t];
+        pieces += b.tile_pieces[t];
+        if (p > 0) red += p * std::min(1.0, std::max(0.25, 4.0 * (double)n_rows / p / 32.0));
+    }
+    const double tiled_us = 7.0 + (double)b.N * (sv + 2) / 4.6e6 + (double)pieces * 4 / 4.6e6 + red / 200e3 + (double)n_rows * sv / 6.0e6;
+    if (tiled_us > 0.85 * own_us) return false;
+    b.scatter();
+    b.slices(n_sm, out);
+    return true;
+}
+} // namespace
+
+bool tiled_build(const std::vector<TiledSource> &src, bool f64, uint64_t n_rows, uint64_t n_cols, int n_sm, TiledHost &out)
+{
+    if (src.empty() || n_sm <= 0) return false;
+    return f64 ? build<double>(src, n_rows, n_cols, n_sm, out) : build<float>(src, n_rows, n_cols, n_sm, out);
+}
+} // namespace asp

@@ -1,0 +1,269 @@
+// Column-tiled SpMV for matrices whose gathers of x are scattered.
+//
+// A gather of x through L1 costs one request to L2 for every cache line that a warp's 32 lanes touch, and an SM issues one
+// such request per clock: with random columns that is one clock per non-zero and SM (290 G non-zeros/s on 148 SMs), two to
+// four times what the matrix's bytes take at the memory's rate. Shared memory serves 9 to 12 random lanes per clock. So the
+// columns are cut into tiles that fit in shared memory; a CTA loads a tile of x once (coalesced) and runs through its part of
+// the tile's non-zeros, 2 + sizeof(value) bytes each (the column inside the tile has 16 bits):
+//   piece  up to 32 non-zeros of one row in one tile
+//   slice  64 pieces, two per lane, of about the same length (sorted inside windows of 1024 pieces); stored step by step,
+//          a step = one non-zero of every piece
+//   steps  one linear stream, cut evenly among the CTAs (one per SM) and inside them among the 32 warps, in the middle of
+//          slices too: what a warp has summed when its slice or its share ends goes to y by `red`
+// The stream is read two batches deep into registers. 159 KB of shared memory per tile leave the L1 enough lines for the
+// loads in flight: with 224 KB the same stream is read at 4.2 instead of 5 TB/s.
+// Measured, fp32 (against the formats' own kernels): 200,000 rows of 40..120 non-zeros, random columns among 1 M: 36 us
+// (76 us, row-grouped); 9,001 rows of 1000..3000: 28 us (77 us, long-row).
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "tiled.h"
+
+namespace asp
+{
+typedef unsigned long long u64;
+typedef unsigned int u32;
+
+namespace
+{
+template <class VT>
+struct Pair;
+template <>
+struct Pair<float>
+{
+    typedef float2 type;
+};
+template <>
+struct Pair<double>
+{
+    typedef double2 type;
+};
+
+// Programmatic dependent launch: `wait` returns when everything before this kernel on its stream has finished;
+// `launch_dependents` lets the next kernel start as soon as there is room for it.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// x may have been written by the kernel before: read through L2, in program order after the wait
+__device__ __forceinline__ uint4 ld_x16(const void *p)
+{
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float ld_x1(const float *p)
+{
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double ld_x1(const double *p)
+{
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+
+template <class VT>
+__global__ void __launch_bounds__(256) k_clear(VT *y, u64 n)
+{
+    grid_launch_dependents();
+    grid_wait();
+    const u64 stride = (u64)gridDim.x * blockDim.x;
+    const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr u64 V = 16 / sizeof(VT);
+    const u64 head = ((16 - ((uintptr_t)y & 15)) & 15) / sizeof(VT), h = head < n ? head : n, body = (n - h) / V;
+    uint4 *b = reinterpret_cast<uint4 *>(y + h);
+    for (u64 i = t; i < body; i += stride) b[i] = make_uint4(0, 0, 0, 0);
+    if (t < h) y[t] = 0;
+    if (t < n - h - body * V) y[h + body * V + t] = 0;
+}
+
+// y[row] += v for the 32 pieces of a warp. Pieces of a long row lie next to one another, and a `red` of many lanes to one
+// address is served lane by lane: those are summed in the warp first (R-MAT with hub rows: 72 -> 60 us an SpMV).
+template <class VT>
+__device__ __forceinline__ void add_rows(VT *y, u32 row, VT v, u32 lane)
+{
+    const u32 next = __shfl_down_sync(0xffffffffu, row, 1);
+    const u32 goes_on = __ballot_sync(0xffffffffu, lane < 31 && row == next);
+    bool head = true;
+    if (goes_on != 0)
+    {
+        const u32 from = goes_on >> lane;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+        {
+            const VT o = __shfl_down_sync(0xffffffffu, v, d);
+            const u32 m = (1u << d) - 1u;
+            if ((from & m) == m) v += o;
+        }
+        head = lane == 0 || ((goes_on >> (lane - 1)) & 1u) == 0;
+    }
+    if (head && row != kTiledNoRow) atomicAdd(y + row, v); // result unused: red.global.add
+}
+
+template <class VT, int U>
+__global__ void __launch_bounds__(1024, 1) k_tiled(const TiledArgs a, const u32 tile_cols)
+{
+    typedef typename Pair<VT>::type P;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    VT *xs = reinterpret_cast<VT *>(smem_raw);
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    VT *const y = (VT *)a.y;
+    bool first = true;
+    u32 visit = blockIdx.x;
+    do
+    {
+        const uint4 k = __ldg(a.work + (size_t)visit * kTiledWarps + warp);
+        u32 step = k.x, slice = k.z;
+        const u32 end = k.y, tile = k.w & 0xffffu;
+        visit = k.w >> 16;
+        const P *vp = reinterpret_cast<const P *>(a.val) + (size_t)step * 32 + lane;
+        const u32 *cp = reinterpret_cast<const u32 *>(a.col) + (size_t)step * 32 + lane;
+        P v[U];
+        u32 c[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+        {
+            v[u] = __ldcs(vp + u * 32);
+            c[u] = __ldcs(cp + u * 32);
+        }
+        const uint2 *rp = reinterpret_cast<const uint2 *>(a.row) + (size_t)slice * 32 + lane;
+        u32 s_end = __ldg(a.end + slice), s_next = __ldg(a.end + slice + 1);
+        uint2 row = __ldg(rp), row_next = __ldg(rp + 32);
+        if (first)
+        {
+            // nothing above depends on what ran before
+            grid_launch_dependents();
+            grid_wait();
+            first = false;
+        }
+        else
+            __syncthreads(); // the tile before has been read
+        {
+            const VT *xp = (const VT *)a.x + (u64)tile * tile_cols;
+            const u64 left = a.n_cols - (u64)tile * tile_cols;
+            const u32 n = left < tile_cols ? (u32)left : tile_cols;
+            constexpr u32 V = 16 / sizeof(VT);
+            u32 i = 0;
+            if (((uintptr_t)xp & 15) == 0)
+            {
+                const uint4 *q = reinterpret_cast<const uint4 *>(xp);
+                uint4 *s = reinterpret_cast<uint4 *>(xs);
+                const u32 n4 = n / V;
+                u32 j = threadIdx.x;
+                for (; j + 4 * 1024 < n4; j += 5 * 1024)
+                {
+                    uint4 t[5];
+#pragma unroll
+                    for (int u = 0; u < 5; u++) t[u] = ld_x16(q + j + u * 1024);
+#pragma unroll
+                    for (int u = 0; u < 5; u++) s[j + u * 1024] = t[u];
+                }
+                for (; j < n4; j += 1024) s[j] = ld_x16(q + j);
+                i = n4 * V;
+            }
+            for (i += threadIdx.x; i < n; i += 1024) xs[i] = ld_x1(xp + i);
+            if (threadIdx.x == 0) xs[tile_cols] = 0;
+        }
+        __syncthreads();
+        VT acc0 = 0, acc1 = 0;
+        while (step < end)
+        {
+            P nv[U];
+            u32 nc[U];
+            vp += U * 32;
+            cp += U * 32;
+#pragma unroll
+            for (int u = 0; u < U; u++)
+            {
+                nv[u] = __ldcs(vp + u * 32);
+                nc[u] = __ldcs(cp + u * 32);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (step < end)
+                {
+                    acc0 += v[u].x * xs[c[u] & 0xffffu];
+                    acc1 += v[u].y * xs[c[u] >> 16];
+                    step++;
+                    if (step == s_end || step == end)
+                    {
+                        add_rows(y, row.x, acc0, lane);
+                        add_rows(y, row.y, acc1, lane);
+                        acc0 = acc1 = 0;
+                        slice++;
+                        rp += 32;
+                        s_end = s_next;
+                        row = row_next;
+                        s_next = __ldg(a.end + slice + 1);
+                        row_next = __ldg(rp + 32);
+                    }
+                }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+            {
+                v[u] = nv[u];
+                c[u] = nc[u];
+            }
+        }
+    } while (visit != 0);
+}
+
+template <class VT>
+struct Batch; // steps read ahead: 48 KB (fp32), 40 KB (fp64) in flight per SM
+template <>
+struct Batch<float>
+{
+    static const int U = 4;
+};
+template <>
+struct Batch<double>
+{
+    static const int U = 2;
+};
+
+cudaError_t launch_pdl(const void *f, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void **args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, f, args);
+}
+
+template <class VT>
+cudaError_t launch(const TiledArgs &args, unsigned n_sm, cudaStream_t st)
+{
+    TiledArgs a = args;
+    VT *y = (VT *)a.y;
+    u64 n = a.n_rows;
+    void *clear_args[] = {&y, &n};
+    // a few 16-byte stores per thread
+    const u64 want = (n * sizeof(VT) / 16 + 1023) / 1024;
+    const unsigned grid = (unsigned)(want < 1 ? 1 : want < 4ull * n_sm ? want : 4ull * n_sm);
+    cudaError_t e = launch_pdl((const void *)k_clear<VT>, grid, 256, 0, st, clear_args);
+    if (e != cudaSuccess) return e;
+    u32 cols = tiled_tile_cols(sizeof(VT) == 8);
+    void *tiled_args[] = {&a, &cols};
+    return launch_pdl((const void *)k_tiled<VT, Batch<VT>::U>, n_sm, kTiledWarps * 32, kTiledTileBytes, st, tiled_args);
+}
+} // namespace
+
+cudaError_t tiled_setup(int val_is_f64)
+{
+    const void *f = val_is_f64 ? (const void *)k_tiled<double, Batch<double>::U> : (const void *)k_tiled<float, Batch<float>::U>;
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTiledTileBytes);
+}
+
+cudaError_t launch_tiled(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st)
+{
+    return val_is_f64 ? launch<double>(a, n_sm, st) : launch<float>(a, n_sm, st);
+}
+} // namespace asp

@@ -1,0 +1,77 @@
+// Column-tiled execution layout of a whole plan group (see kernels_tiled.cu for what it is for): built on the host
+// from the template arrays at plan creation, read by one kernel that replaces the group's own kernels.
+#ifndef ASP_TILED_H
+#define ASP_TILED_H
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <memory>
+#include <vector>
+
+#include "host_meta.h"
+#include "kernel_args.h"
+
+namespace asp
+{
+const uint32_t kTiledWarps = 32;             // warps per CTA, one CTA per SM
+const uint32_t kTiledLanePieces = 2;         // pieces of a row per lane
+const uint32_t kTiledSlice = 32 * kTiledLanePieces;
+const uint32_t kTiledTileBytes = 159u << 10; // shared memory of a tile of x
+const uint32_t kTiledNoRow = 0xffffffffu;
+// steps and slices the kernel may read past the end (prefetch)
+const uint32_t kTiledSlackSteps = 8, kTiledSlackSlices = 2;
+
+// columns of a tile; the shared memory after them holds one zero, which what pads a slice multiplies (never an infinite x)
+inline uint32_t tiled_tile_cols(bool f64) { return kTiledTileBytes / (f64 ? 8u : 4u) - 32u; }
+
+// one sub-matrix of the group, as its template stores it (host arrays)
+struct TiledSource
+{
+    int templ = 0;
+    const HostMeta *m = nullptr; // MS_COUNT slots
+    const HostMeta *perm = nullptr;
+    const KArgs *a = nullptr;    // scalars of the plan
+    const void *val = nullptr, *col = nullptr;
+    int col_bytes = 4;
+    uint64_t stored = 0; // padded non-zeros
+};
+
+template <class T>
+struct HostBuf
+{
+    std::unique_ptr<T[]> p;
+    uint64_t n = 0;
+    void make(uint64_t count) { p.reset(new T[count]), n = count; }
+    uint64_t bytes() const { return n * sizeof(T); }
+};
+
+struct TiledHost
+{
+    HostBuf<unsigned char> val; // step s, lane l, piece g: value s * 64 + 2 l + g
+    HostBuf<uint16_t> col;      // same order, column inside the tile
+    HostBuf<uint32_t> row;      // slice s, lane l, piece g: row of y (kTiledNoRow: none)
+    HostBuf<uint32_t> end;      // slice s covers steps [end[s - 1], end[s])
+    std::vector<uint32_t> work; // {first step, end step, slice, tile | next visit << 16} per warp; visit v at v * kTiledWarps
+    uint64_t nnz = 0, steps = 0, slices = 0;
+    bool covers_all_rows = false; // every row of y has at least one element
+};
+
+// false: the group stays with its own kernels
+bool tiled_build(const std::vector<TiledSource> &src, bool f64, uint64_t n_rows, uint64_t n_cols, int n_sm, TiledHost &out);
+
+struct TiledArgs
+{
+    const void *val;
+    const uint16_t *col;
+    const uint32_t *row, *end;
+    const uint4 *work;
+    const void *x;
+    void *y;
+    unsigned long long n_rows, n_cols;
+};
+cudaError_t tiled_setup(int val_is_f64);
+// y = A x: clears y, then accumulates (two launches)
+cudaError_t launch_tiled(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st);
+} // namespace asp
+#endif

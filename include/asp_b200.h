@@ -171,6 +171,10 @@ void *asp_ctx_stream(asp_ctx *ctx);
  * pointer (the global row permutation) are uploaded once. Validation covers the contents too:
  * every column index must lie inside x, every row a kernel can write inside y, every offset
  * inside the array it indexes (ASP_ERR_BOUNDS otherwise; one parallel pass over each index array).
+ * Where the columns are so scattered that the gathers of x, not the bytes, bound the templates' kernels, the whole group
+ * is also laid out by column tiles (csrc/kernels_tiled.cu; about 1.5 times the format's device memory in all), and asp_spmv
+ * over the complete group runs that layout; a group with EMPTY plans never does. Sums are then taken in another order from
+ * call to call, as with every template that accumulates with atomics.
  * Every entry point makes the context's device current for its own duration and restores the
  * caller's device before it returns. */
 asp_status asp_plan_group_create(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp_plan **out_plans);
@@ -200,7 +204,8 @@ asp_status asp_plan_get_launch(const asp_plan *plan, int64_t *tblock_num, int64_
  * current value), `path` (-1 keeps): SELL-like 0 = warp tasks over equal strips, 1 = one CTA per strip;
  * CSR5-like bit 0 = staged write-out (the same switch as thread_num_of_row_reduce = 2), bits 4..7 = log2
  * of the rows per warp that go through shared memory (0 keeps the size chosen at plan creation).
- * Re-applies the last requested launch. No counterpart in the reference (its generated kernels handle
+ * Re-applies the last requested launch, and from then on asp_spmv runs this plan's own kernel (not the column-tiled layout of
+ * its group). No counterpart in the reference (its generated kernels handle
  * one TLB per thread). */
 asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path);
 /* bytes of device memory the plan's format arrays occupy (B_fmt without x and y) */

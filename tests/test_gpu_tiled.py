@@ -1,0 +1,73 @@
+"""GPU: the column-tiled layout that plan groups with scattered columns run (csrc/kernels_tiled.cu), against the CPU oracle at
+the sizes where its tiles, slices and work shares end: columns that fill the last tile exactly, by one, or leave one over; rows
+longer than a tile's piece limit; several sub-matrices in one group; x and y off 16-byte alignment; every clearing mode."""
+import numpy as np
+import pytest
+
+import refdump
+from alphasparse_b200 import matrices as M, tuner
+
+pytestmark = pytest.mark.gpu
+
+TILE = {np.float32: 40672, np.float64: 20320}  # columns of a tile
+NODES = {"K9": ["tlb_nnz 16"], "K10": ["tlb_nnz 7"], "K6": ["row_padding 32 1", "blb_row_evenly 32", "tlb_col_fixed 4"], "K4": ["wlb_col_fixed 64"],
+         "K8": ["row_padding 4 1", "blb_row_evenly 4", "wlb_col_fixed 64"], "K7": ["blb_col_fixed 256"], "K2": ["row_padding 128 1", "blb_row_evenly 128", "tlb_row"],
+         "K3": ["row_padding 32 1", "tlb_row"]}
+
+
+def matrix(dtype, cols, seed, longest=70):
+    rng = np.random.default_rng(seed)
+    # just above what makes the layout the faster one
+    lengths = rng.integers(40, longest, size=(4_000_000 if dtype is np.float32 else 9_000_000) // ((40 + longest) // 2))
+    if longest == 71:  # a few hub rows: their pieces are summed in the warp before they reach y
+        lengths[[0, 1, 777, -1]] = [cols // 2, 20_000, 3_000, 33]
+    return M.from_row_lengths(lengths, cols, seed=seed, dtype=dtype)
+
+
+@pytest.mark.parametrize("template,dtype,tiles,over,longest", [
+    ("K9", np.float32, 3, 0, 71), ("K9", np.float64, 4, 1, 71), ("K10", np.float32, 3, -1, 71), ("K6", np.float32, 2, 1, 70), ("K6", np.float64, 5, 0, 70),
+    ("K4", np.float32, 3, 1, 71), ("K8", np.float64, 4, -1, 70), ("K7", np.float32, 5, 7, 71), ("K2", np.float32, 3, 0, 70), ("K3", np.float64, 3, 1, 70)])
+def test_tiled_group_matches_the_oracle(asp_ctx, template, dtype, tiles, over, longest):
+    import torch
+
+    m, x = matrix(dtype, tiles * TILE[dtype] + over, seed=tiles, longest=longest)
+    free = torch.cuda.mem_get_info()[0]
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template, "threads": 128, "row_reduce": 1}]})
+    assert free - torch.cuda.mem_get_info()[0] > 1.3 * g.format_bytes(), "the layout was not built for this matrix"
+    y_ref, scale = refdump.csr_ref(m, x)
+    for shift in (0, 1):  # x and y on and off 16-byte boundaries
+        dx = torch.zeros(m.n_cols + shift, dtype=torch.from_numpy(x).dtype, device="cuda")
+        dx[shift:] = torch.from_numpy(x).cuda()
+        dy = torch.full((m.n_rows + 5 + shift,), 7.0, dtype=dx.dtype, device="cuda")
+        for zero_y in (True, "auto"):
+            torch.cuda.synchronize()
+            g.spmv(dx[shift:].data_ptr(), dy[shift:].data_ptr(), zero_y)
+            asp_ctx.synchronize()
+            y = dy.cpu().numpy()
+            refdump.assert_y(y[shift : shift + m.n_rows], y_ref, scale, m.values.dtype, f"{template} zero_y={zero_y} shift={shift}")
+            assert (y[:shift] == 7).all() and (y[shift + m.n_rows :] == 7).all()  # nothing beside y
+    g.set_tuning(0, 0, 0) if template in ("K2", "K3", "K9", "K10") else None  # back to the template's own kernel
+    refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, f"{template} own kernel")
+    g.close()
+    fmt.close()
+
+
+def test_tiled_group_of_sorted_strips_and_empty_rows(asp_ctx):
+    rng = np.random.default_rng(8)
+    lengths = np.concatenate([rng.integers(20, 100, size=30_000), rng.integers(200, 900, size=4_000), [30_000, 9_000]])
+    rng.shuffle(lengths)
+    lengths[rng.integers(0, lengths.size, size=500)] = 0  # rows that no kernel stores: zero when y is cleared
+    m, x = M.from_row_lengths(lengths, 150_000, seed=8)
+    sub = lambda t: {"graph": t, "nodes": NODES[t], "template": t, "threads": 128, "row_reduce": 1}
+    from alphasparse_b200.graph import Matrix
+
+    hm = Matrix.from_csr(m)
+    cm = hm.dense("dense sort 1\ndense rowdiv_exp 128 4096 8\ndense compress")
+    desc = {"dense": "dense sort 1 | dense rowdiv_exp 128 4096 8 | dense compress", "subs": [sub("K2" if cm.sub_rows(i)[3] <= 128 else "K6" if cm.sub_rows(i)[3] <= 1024 else "K7") for i in range(cm.n_subs)]}
+    fmt, g = tuner.build(asp_ctx, m, desc)
+    y_ref, scale = refdump.csr_ref(m, x)
+    refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, "strips")
+    g.close()
+    fmt.close()
+    cm.close()
+    hm.close()
