@@ -55,11 +55,10 @@ std::unique_ptr<Matrix> matrix_from_csr(u64 n_rows, u64 n_cols, const int64_t *i
     m->n_cols = n_cols;
     m->nnz = (u64)indptr[n_rows];
     m->val_dt = val_dt;
-    m->rowptr.resize(n_rows + 1);
-    for (u64 i = 0; i <= n_rows; i++) m->rowptr[i] = (u64)indptr[i];
-    m->col.assign(indices, indices + m->nnz);
+    m->rowptr.assign((const u64 *)indptr, n_rows + 1);
+    m->col.assign(indices, m->nnz);
     m->val.es = dtype_bytes(val_dt);
-    m->val.b.assign((const uint8_t *)values, (const uint8_t *)values + m->nnz * m->val.es);
+    m->val.b.assign((const uint8_t *)values, m->nnz * m->val.es);
     return m;
 }
 
@@ -89,11 +88,12 @@ std::unique_ptr<Matrix> relabel_by_column_count(const Matrix &m, bool empty_rows
     out->n_rows = out->n_cols = n;
     out->nnz = m.nnz;
     out->val_dt = m.val_dt;
-    out->rowptr.assign(n + 1, 0);
-    for (u64 k = 0; k < n; k++) out->rowptr[k + 1] = out->rowptr[k] + (m.rowptr[order[k] + 1] - m.rowptr[order[k]]);
-    out->col.resize(m.nnz);
+    u64 *rp = out->rowptr.make(n + 1);
+    rp[0] = 0;
+    for (u64 k = 0; k < n; k++) rp[k + 1] = rp[k] + (m.rowptr[order[k] + 1] - m.rowptr[order[k]]);
+    u32 *ocol = out->col.make(m.nnz);
     out->val.es = m.val.es;
-    out->val.b.resize(m.nnz * m.val.es);
+    uint8_t *oval = out->val.b.make(m.nnz * m.val.es);
     const size_t es = (size_t)m.val.es;
 #pragma omp parallel
     {
@@ -101,14 +101,14 @@ std::unique_ptr<Matrix> relabel_by_column_count(const Matrix &m, bool empty_rows
 #pragma omp for schedule(dynamic, 256)
         for (long long k = 0; k < (long long)n; k++)
         {
-            const u64 b = m.rowptr[order[k]], e = m.rowptr[order[k] + 1], o = out->rowptr[k];
+            const u64 b = m.rowptr[order[k]], e = m.rowptr[order[k] + 1], o = rp[k];
             row.clear();
             for (u64 j = b; j < e; j++) row.push_back({labels[m.col[j]], j});
             std::sort(row.begin(), row.end());
             for (u64 j = 0; j < row.size(); j++)
             {
-                out->col[o + j] = row[j].first;
-                memcpy(&out->val.b[(o + j) * es], &m.val.b[row[j].second * es], es);
+                ocol[o + j] = row[j].first;
+                memcpy(&oval[(o + j) * es], &m.val.b[row[j].second * es], es);
             }
         }
     }
@@ -254,22 +254,22 @@ std::unique_ptr<Matrix> matrix_from_coo_file(const std::string &path, int val_dt
     m->n_cols = n_cols;
     m->nnz = nnz;
     m->val_dt = val_dt;
-    m->rowptr.assign(n_rows + 1, 0);
-    m->col.resize(nnz);
+    u64 *rp = m->rowptr.make_zero(n_rows + 1);
+    u32 *ocol = m->col.make(nnz);
     m->val.es = dtype_bytes(val_dt);
-    m->val.resize(nnz);
+    uint8_t *oval = m->val.b.make(nnz * m->val.es);
     u64 off = 0;
     for (int t = 0; t < nt; t++)
     {
         const Part &pt = parts[t];
-        for (u64 r : pt.rows) m->rowptr[r + 1]++;
-        std::copy(pt.cols.begin(), pt.cols.end(), m->col.begin() + off);
-        if (val_dt == ASP_F64) memcpy(m->val.b.data() + off * 8, pt.vals.data(), pt.vals.size() * 8);
+        for (u64 r : pt.rows) rp[r + 1]++;
+        std::copy(pt.cols.begin(), pt.cols.end(), ocol + off);
+        if (val_dt == ASP_F64) memcpy(oval + off * 8, pt.vals.data(), pt.vals.size() * 8);
         else
-            for (u64 i = 0; i < pt.vals.size(); i++) ((float *)m->val.b.data())[off + i] = (float)pt.vals[i];
+            for (u64 i = 0; i < pt.vals.size(); i++) ((float *)oval)[off + i] = (float)pt.vals[i];
         off += pt.rows.size();
     }
-    for (u64 i = 0; i < n_rows; i++) m->rowptr[i + 1] += m->rowptr[i];
+    for (u64 i = 0; i < n_rows; i++) rp[i + 1] += rp[i];
     return m;
 }
 
@@ -331,24 +331,26 @@ void dense_row_coarse_sort(Matrix &m, u64 step)
         else m.perm[start[bin[r]]++] = r;
     }
     // rewrite the dense view in the new row order
-    std::vector<u64> nrp(R + 1, 0);
+    Arr<u64> rowptr;
+    u64 *nrp = rowptr.make(R + 1);
+    nrp[0] = 0;
     for (u64 i = 0; i < R; i++) nrp[i + 1] = nrp[i] + len[m.perm[i]];
-    std::vector<u32> ncol(m.nnz);
-    ValBuf nval;
-    nval.es = m.val.es;
-    nval.b.resize(m.val.b.size());
+    Arr<u32> col;
+    u32 *ncol = col.make(m.nnz);
+    Arr<uint8_t> val;
+    uint8_t *nval = val.make(m.val.b.size());
     const int es = m.val.es;
-#pragma omp parallel for schedule(dynamic, 4096)
+#pragma omp parallel for schedule(dynamic, 4096) if (m.nnz > kParallelNnz)
     for (u64 i = 0; i < R; i++)
     {
         const u64 o = m.perm[i], n = len[o];
         if (n == 0) continue;
         memcpy(&ncol[nrp[i]], &m.col[m.rowptr[o]], n * sizeof(u32));
-        memcpy(&nval.b[nrp[i] * es], &m.val.b[m.rowptr[o] * es], n * es);
+        memcpy(&nval[nrp[i] * es], &m.val.b[m.rowptr[o] * es], n * es);
     }
-    m.rowptr.swap(nrp);
-    m.col.swap(ncol);
-    m.val.b.swap(nval.b);
+    m.rowptr.swap(rowptr);
+    m.col.swap(col);
+    m.val.b.swap(val);
     m.is_sorted = true;
     m.perm_dt = suitable_dtype(R);
     const int pb = dtype_bytes(m.perm_dt);
@@ -413,14 +415,20 @@ void compress_dense_view(Matrix &m)
         b.n_rows = rg.max_row - rg.min_row + 1;
         b.row_dt = suitable_dtype(b.n_rows);                 // counts, not maxima: 65536 rows -> u32
         b.col_dt = suitable_dtype(b.max_col - b.min_col + 1);
-        b.rowptr.resize(b.n_rows + 1);
-        for (u64 r = 0; r <= b.n_rows; r++) b.rowptr[r] = m.rowptr[rg.min_row + r] - rg.begin_coo;
+        // a view of the dense view's arrays; offsets that do not start at 0 are rewritten
+        if (rg.begin_coo == 0) b.rowptr = m.rowptr.view(rg.min_row, b.n_rows + 1);
+        else
+        {
+            u64 *rp = b.rowptr.make(b.n_rows + 1);
+#pragma omp parallel for schedule(static) if (b.n_rows > kParallelRows)
+            for (u64 r = 0; r <= b.n_rows; r++) rp[r] = m.rowptr[rg.min_row + r] - rg.begin_coo;
+        }
         const u64 n = rg.end_coo - rg.begin_coo + 1;
-        b.col.assign(m.col.begin() + rg.begin_coo, m.col.begin() + rg.begin_coo + n);
+        b.col = m.col.view(rg.begin_coo, n);
         b.val.es = m.val.es;
         // every block holds ITS slice of the values; the reference copies from offset 0 for every
         // block (op_manager.cc:1077-1087), which is only right for the first one
-        b.val.b.assign(m.val.b.begin() + rg.begin_coo * m.val.es, m.val.b.begin() + (rg.begin_coo + n) * m.val.es);
+        b.val.b = m.val.b.view(rg.begin_coo * m.val.es, n * m.val.es);
     }
     m.is_compressed = true;
 }
@@ -435,10 +443,10 @@ void row_padding(CompressedBlock &b, u64 multiple, u64 plen)
     const u64 target = (rows / multiple + 1) * multiple;
     const u64 add = target - rows;
     const u64 old_nnz = b.col.size();
-    b.col.resize(old_nnz + add * plen, 0); // fake rows: `plen` zeros at (relative) column 0
-    b.val.b.resize((old_nnz + add * plen) * b.val.es, 0);
-    b.rowptr.resize(target + 1);
-    for (u64 r = rows; r < target; r++) b.rowptr[r + 1] = b.rowptr[r] + plen;
+    b.col.grow(old_nnz + add * plen); // fake rows: `plen` zeros at (relative) column 0
+    b.val.b.grow((old_nnz + add * plen) * b.val.es);
+    u64 *rp = b.rowptr.grow(target + 1);
+    for (u64 r = rows; r < target; r++) rp[r + 1] = rp[r] + plen;
     b.n_rows = target;
     b.row_dt = suitable_dtype(target);
 }
@@ -520,30 +528,12 @@ void sep_tblock_level_col_fixed(CompressedBlock &b, u64 c)
     {
         const u64 n = b.rowptr[r + 1] - b.rowptr[r];
         if (n == 0) continue;
-        const u64 full = n / c, rem = n % c;
-        // nominal sizes: `full` chunks of c; remainder >= c/2 -> one more chunk; else merged into the
-        // last chunk (or the only one)
-        std::vector<u64> sizes(full, c);
-        if (rem >= c / 2) sizes.push_back(c);
-        else if (sizes.empty()) sizes.push_back(c);
-        else sizes.back() = 2 * c;
-        u64 beg = b.rowptr[r], k = 0, acc = 0;
-        for (u64 i = 0; i < n; i++)
-        {
-            if (i == acc + sizes[k] - 1)
-            {
-                L.first_row.v.push_back(r);
-                L.coo_begin.v.push_back(beg);
-                beg = b.rowptr[r] + i + 1;
-                acc += sizes[k];
-                k++;
-                if (k >= sizes.size() && i + 1 < n) k = sizes.size() - 1; // not reached with the sizes above
-            }
-        }
-        if (beg != b.rowptr[r + 1])
+        // chunks of c; a remainder of at least c / 2 is a chunk of its own, a smaller one belongs to the last chunk
+        const u64 full = n / c, rem = n % c, chunks = std::max<u64>(1, full + (rem > 0 && rem >= c / 2 ? 1 : 0));
+        for (u64 k = 0; k < chunks; k++)
         {
             L.first_row.v.push_back(r);
-            L.coo_begin.v.push_back(beg);
+            L.coo_begin.v.push_back(b.rowptr[r] + k * c);
         }
     }
     L.row_num.v.assign(L.first_row.v.size(), 1);
@@ -670,117 +660,151 @@ void sep_warp_level_col_fixed(CompressedBlock &b, u64 c)
     b.share_row_with_other_warp = true;
 }
 
-void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size)
+void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, bool tlb_rows)
 {
     Level &B = b.blb;
     Level &W = b.wlb;
     Level &T = b.tlb;
     T = Level();
     const int es = b.val.es;
+    const u64 NW = W.block_num;
+    // few WLBs (one over the whole sub-matrix, as the ELL-like graphs have it): the rows of each are shared out; many: the WLBs are
+    const bool by_rows = NW < 256;
+    std::vector<u32> blb_of(NW);
+    for (u64 i = 0; i < B.block_num; i++)
+        for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) blb_of[w] = (u32)i;
+    struct Span // the WLB's rows and non-zeros
+    {
+        u64 r0, rows, a, e;
+    };
+    auto span = [&](u64 w) {
+        Span s;
+        s.r0 = B.first_row.v[blb_of[w]] + W.first_row.v[w];
+        s.rows = W.row_num.v[w];
+        s.a = B.coo_begin.v[blb_of[w]] + W.coo_begin.v[w];
+        s.e = s.a + W.coo_size.v[w];
+        return s;
+    };
+    auto row_range = [&](const Span &s, u64 r, u64 &lo, u64 &hi) {
+        lo = std::max(b.rowptr[std::min(s.r0 + r, b.n_rows)], s.a);
+        hi = std::min(b.rowptr[std::min(s.r0 + r + 1, b.n_rows)], s.e);
+        return hi > lo ? hi - lo : 0;
+    };
     // pass 1: per WLB the TLB size, TLBs per row (rounded up, then round-robin fillers from the
     // WLB's first row until the WLB holds a multiple of 32 TLBs), padded sizes
-    std::vector<u64> wlb_S(W.block_num), wlb_tlb0(W.block_num + 1, 0), wlb_pad0(W.block_num + 1, 0);
+    std::vector<u64> wlb_S(NW), wlb_tl(NW), wlb_tlb0(NW + 1, 0), wlb_pad0(NW + 1, 0);
     std::vector<u64> blb_first(B.block_num + 1, 0);
-    u64 max_S = 0;
-    bool share_thread = tlb_size != 0;
-    for (u64 i = 0; i < B.block_num; i++)
-    {
-        for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++)
+#pragma omp parallel for schedule(static) if (!by_rows && b.col.size() > kParallelNnz)
+    for (u64 w = 0; w < NW; w++)
         {
-            const u64 r0 = B.first_row.v[i] + W.first_row.v[w], rows = W.row_num.v[w];
-            const u64 a = B.coo_begin.v[i] + W.coo_begin.v[w], e = a + W.coo_size.v[w];
+            const Span s = span(w);
             u64 S = tlb_size;
             if (S == 0)
             {
-                for (u64 r = 0; r < rows; r++)
+#pragma omp parallel for schedule(static) reduction(max : S) if (by_rows && s.rows > kParallelRows)
+                for (u64 r = 0; r < s.rows; r++)
                 {
-                    const u64 lo = std::max(b.rowptr[std::min(r0 + r, b.n_rows)], a), hi = std::min(b.rowptr[std::min(r0 + r + 1, b.n_rows)], e);
-                    if (hi > lo) S = std::max(S, hi - lo);
+                    u64 lo, hi;
+                    S = std::max(S, row_range(s, r, lo, hi));
                 }
             }
             u64 tl = 0;
-            for (u64 r = 0; r < rows; r++)
+#pragma omp parallel for schedule(static) reduction(+ : tl) if (by_rows && s.rows > kParallelRows)
+            for (u64 r = 0; r < s.rows; r++)
             {
-                const u64 lo = std::max(b.rowptr[std::min(r0 + r, b.n_rows)], a), hi = std::min(b.rowptr[std::min(r0 + r + 1, b.n_rows)], e);
-                const u64 n = hi > lo ? hi - lo : 0;
-                tl += (n + S - 1) / S;
+                u64 lo, hi;
+                tl += (row_range(s, r, lo, hi) + S - 1) / S;
             }
-            const u64 target = (tl + 31) / 32 * 32;
             wlb_S[w] = S;
-            wlb_tlb0[w + 1] = wlb_tlb0[w] + target;
-            wlb_pad0[w + 1] = wlb_pad0[w] + target * S;
-            max_S = std::max(max_S, S);
+            wlb_tl[w] = tl;
         }
-        blb_first[i + 1] = wlb_pad0[B.index.v[i + 1]];
+    u64 max_S = 0;
+    for (u64 w = 0; w < NW; w++)
+    {
+        const u64 target = (wlb_tl[w] + 31) / 32 * 32;
+        wlb_tlb0[w + 1] = wlb_tlb0[w] + target;
+        wlb_pad0[w + 1] = wlb_pad0[w] + target * wlb_S[w];
+        max_S = std::max(max_S, wlb_S[w]);
     }
-    const u64 n_tlb = wlb_tlb0[W.block_num], n_pad = wlb_pad0[W.block_num];
+    for (u64 i = 0; i < B.block_num; i++) blb_first[i + 1] = wlb_pad0[B.index.v[i + 1]];
+    const u64 n_tlb = wlb_tlb0[NW], n_pad = wlb_pad0[NW];
     // a few long rows in an ELL-shaped strip multiply the storage: stop before materialising a
     // format that no padding gate would let through (the search bound is 4x; 64x leaves room for
     // callers with their own bound)
     if (n_pad > 64 * std::max<u64>(b.col.size(), 1024)) throw std::length_error("padded size exceeds 64x the non-zeros of the sub-matrix");
-    b.pad_col.assign(n_pad, 0);
+    u32 *pcol = b.pad_col.make(n_pad);
     b.pad_val.es = es;
-    b.pad_val.resize(n_pad);
-    T.first_row.v.resize(n_tlb);
-    u64 max_thread_first_row = 0, max_w_coo_begin = 0, max_w_size = 0;
-    std::vector<u64> new_w_begin(W.block_num), new_w_size(W.block_num);
+    uint8_t *pval = b.pad_val.b.make(n_pad * es);
+    u32 *trow = tlb_rows ? b.tlb_row.make(n_tlb) : nullptr;
+    u64 max_thread_first_row = 0;
+    bool share_thread = tlb_size != 0;
     // pass 2: fill the padded arrays (row-major inside the WLB) and the per-TLB first rows
-    for (u64 i = 0; i < B.block_num; i++)
+#pragma omp parallel if (!by_rows && b.col.size() > kParallelNnz)
     {
+        std::vector<u64> first; // first TLB of every row of the WLB, relative to it
+#pragma omp for schedule(static) reduction(max : max_thread_first_row) reduction(|| : share_thread)
+        for (u64 w = 0; w < NW; w++)
+            {
+                const Span s = span(w);
+                const u64 S = wlb_S[w], extra = wlb_tlb0[w + 1] - wlb_tlb0[w] - wlb_tl[w];
+                first.resize(s.rows + 1);
+                u64 *f = first.data();
+                f[0] = 0;
+#pragma omp parallel for schedule(static) if (by_rows && s.rows > kParallelRows)
+                for (u64 r = 0; r < s.rows; r++)
+                {
+                    u64 lo, hi;
+                    // filler k goes to row k % rows
+                    f[r + 1] = (row_range(s, r, lo, hi) + S - 1) / S + (extra > r ? (extra - r - 1) / s.rows + 1 : 0);
+                }
+                for (u64 r = 0; r < s.rows; r++) f[r + 1] += f[r];
+                u64 top = 0;
+                bool shared_row = false;
+#pragma omp parallel for schedule(static) reduction(max : top) reduction(|| : shared_row) if (by_rows && (wlb_pad0[w + 1] - wlb_pad0[w]) * es > kParallelBytes)
+                for (u64 r = 0; r < s.rows; r++)
+                {
+                    u64 lo, hi;
+                    const u64 n = row_range(s, r, lo, hi), tlbs = f[r + 1] - f[r], tgt = tlbs * S, out = wlb_pad0[w] + f[r] * S;
+                    u32 fill = (u32)b.min_col;
+                    if (n > 0)
+                    {
+                        memcpy(pcol + out, b.col.data() + lo, n * sizeof(u32));
+                        memcpy(pval + out * es, b.val.b.data() + lo * es, n * es);
+                        fill = b.col[hi - 1];
+                    }
+                    for (u64 k = n; k < tgt; k++) pcol[out + k] = fill; // with value 0
+                    memset(pval + (out + n) * es, 0, (tgt - n) * es);
+                    if (tlbs >= 2) shared_row = true;
+                    if (trow)
+                        for (u64 k = 0; k < tlbs; k++) trow[wlb_tlb0[w] + f[r] + k] = (u32)r;
+                    if (tlbs > 0) top = std::max(top, r);
+                }
+                share_thread = share_thread || shared_row;
+                max_thread_first_row = std::max(max_thread_first_row, top);
+            }
+    }
+    u64 max_w_coo_begin = 0, max_w_size = 0;
+    std::vector<u64> new_w_begin(NW), new_w_size(NW);
+    for (u64 i = 0; i < B.block_num; i++)
         for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++)
         {
-            const u64 r0 = B.first_row.v[i] + W.first_row.v[w], rows = W.row_num.v[w];
-            const u64 a = B.coo_begin.v[i] + W.coo_begin.v[w], e = a + W.coo_size.v[w];
-            const u64 S = wlb_S[w];
-            std::vector<u64> per_row(rows);
-            u64 tl = 0;
-            for (u64 r = 0; r < rows; r++)
-            {
-                const u64 lo = std::max(b.rowptr[std::min(r0 + r, b.n_rows)], a), hi = std::min(b.rowptr[std::min(r0 + r + 1, b.n_rows)], e);
-                const u64 n = hi > lo ? hi - lo : 0;
-                per_row[r] = (n + S - 1) / S;
-                tl += per_row[r];
-            }
-            const u64 target = wlb_tlb0[w + 1] - wlb_tlb0[w];
-            for (u64 k = 0, rr = 0; k < target - tl; k++, rr = (rr + 1) % rows) per_row[rr]++;
-            u64 out = wlb_pad0[w], t = wlb_tlb0[w];
-            for (u64 r = 0; r < rows; r++)
-            {
-                const u64 lo = std::max(b.rowptr[std::min(r0 + r, b.n_rows)], a), hi = std::min(b.rowptr[std::min(r0 + r + 1, b.n_rows)], e);
-                const u64 n = hi > lo ? hi - lo : 0;
-                const u64 tgt = per_row[r] * S;
-                if (n > 0)
-                {
-                    memcpy(&b.pad_col[out], &b.col[lo], n * sizeof(u32));
-                    memcpy(&b.pad_val.b[out * es], &b.val.b[lo * es], n * es);
-                    const u32 last = b.col[hi - 1];
-                    for (u64 k = n; k < tgt; k++) b.pad_col[out + k] = last; // value stays 0
-                }
-                else
-                    for (u64 k = 0; k < tgt; k++) b.pad_col[out + k] = (u32)b.min_col;
-                out += tgt;
-                if (per_row[r] >= 2) share_thread = true;
-                for (u64 k = 0; k < per_row[r]; k++) T.first_row.v[t++] = r;
-                if (per_row[r] > 0) max_thread_first_row = std::max(max_thread_first_row, r);
-            }
-            new_w_size[w] = target * S;
+            new_w_size[w] = wlb_pad0[w + 1] - wlb_pad0[w];
             new_w_begin[w] = (w == B.index.v[i]) ? 0 : new_w_begin[w - 1] + new_w_size[w - 1];
             if (w != B.index.v[i]) max_w_coo_begin = std::max(max_w_coo_begin, new_w_begin[w]);
             max_w_size = std::max(max_w_size, new_w_size[w]);
         }
-    }
     // the BLB / WLB offsets now refer to the padded arrays (op_manager.cc:3639-3680)
-    B.coo_begin.v = blb_first;
+    B.coo_begin.v.swap(blb_first);
     B.coo_begin.dt = suitable_dtype(n_pad);
-    W.coo_begin.v = new_w_begin;
+    W.coo_begin.v.swap(new_w_begin);
     W.coo_begin.dt = suitable_dtype(max_w_coo_begin);
-    W.coo_size.v = new_w_size;
+    W.coo_size.v.swap(new_w_size);
     W.coo_size.dt = suitable_dtype(max_w_size);
-    W.index.v = wlb_tlb0;
+    W.index.v.swap(wlb_tlb0);
     W.index.dt = suitable_dtype(n_tlb);
     T.block_num = n_tlb;
     T.first_row.dt = suitable_dtype(max_thread_first_row + 1);
-    T.coo_size.v = wlb_S;
+    T.coo_size.v.swap(wlb_S);
     T.coo_size.dt = suitable_dtype(max_S);
     T.built = true;
     b.padded = true;
@@ -803,11 +827,11 @@ void sep_thread_level_acc_to_nnz(CompressedBlock &b, u64 S)
     b.padded = false;
 }
 
-void complete_each_level_blocking(CompressedBlock &b)
+void complete_each_level_blocking(CompressedBlock &b, bool rows_per_unit)
 {
     if (!b.blb.built) sep_tblock_level_row_csr(b, std::vector<u64>(1, b.n_rows));
     if (!b.wlb.built) sep_warp_level_row_csr(b, std::vector<std::vector<u64>>());
-    if (!b.tlb.built) sep_thread_level_col_ell_with_padding(b, 1);
+    if (!b.tlb.built) sep_thread_level_col_ell_with_padding(b, 1, !rows_per_unit);
 }
 
 } // namespace host

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "../../../include/asp_b200.h"
+#include "hostmem.hpp"
 
 namespace asp
 {
@@ -43,12 +44,25 @@ struct ClosedForm
     std::vector<u64> lo, hi, val;
 };
 
+// a read-only run of u64 (a vector or an Arr)
+struct U64s
+{
+    const u64 *p;
+    u64 n;
+    U64s(const std::vector<u64> &v) : p(v.data()), n(v.size()) {}
+    U64s(const Arr<u64> &a) : p(a.data()), n(a.size()) {}
+    u64 size() const { return n; }
+    bool empty() const { return n == 0; }
+    const u64 &operator[](u64 i) const { return p[i]; }
+    const u64 &back() const { return p[n - 1]; }
+};
+
 // closed-form detectors (arr_optimization.cc:6-57, 81-105, 113-170, 206-260, 277-337)
-bool detect_linear(const std::vector<u64> &a, ClosedForm &out);
-bool detect_constant(const std::vector<u64> &a, ClosedForm &out);
-bool detect_branch(const std::vector<u64> &a, ClosedForm &out);
-bool detect_cycle_linear(const std::vector<u64> &a, u64 cycle, ClosedForm &out);
-bool detect_cycle_increase(const std::vector<u64> &a, ClosedForm &out);
+bool detect_linear(U64s a, ClosedForm &out);
+bool detect_constant(U64s a, ClosedForm &out);
+bool detect_branch(U64s a, ClosedForm &out);
+bool detect_cycle_linear(U64s a, u64 cycle, ClosedForm &out);
+bool detect_cycle_increase(U64s a, ClosedForm &out);
 
 // one (ptr, dtype, size) triple of a template, in its final narrowed bytes
 struct TemplateArray
@@ -56,7 +70,7 @@ struct TemplateArray
     int role = 0; // asp_array_role
     int dt = ASP_U8;
     u64 len = 0;
-    std::vector<uint8_t> bytes;           // owned storage ...
+    Arr<uint8_t> bytes;                   // owned storage ...
     std::shared_ptr<std::vector<uint8_t>> shared; // ... or storage shared between sub-matrices (global row permutation)
     ClosedForm comp;
     const uint8_t *data() const { return shared ? shared->data() : bytes.data(); }
@@ -82,9 +96,8 @@ struct TemplateData
 struct ValBuf
 {
     int es = 4; // 4: f32, 8: f64
-    std::vector<uint8_t> b;
+    Arr<uint8_t> b;
     u64 size() const { return b.size() / es; }
-    void resize(u64 n) { b.assign(n * es, 0); }
 };
 
 // One level of the BLB -> WLB -> TLB tiling (index_of_compress_block_t of the reference,
@@ -108,8 +121,8 @@ struct CompressedBlock
     u64 begin_coo = 0, end_coo = 0;
     // compressed view; n_rows grows with COMPRESSED_ROW_PADDING
     u64 n_rows = 0;
-    std::vector<u64> rowptr;
-    std::vector<u32> col;
+    Arr<u64> rowptr;
+    Arr<u32> col;
     ValBuf val;
     int row_dt = ASP_U8, col_dt = ASP_U8; // element types of read_index[0] / read_index[1]
     Level blb, wlb, tlb;
@@ -117,7 +130,8 @@ struct CompressedBlock
     IndexArr tlb_row_span;        // rows spanned per TLB (nnz-div only)
     bool share_row_with_other_block = false, share_row_with_other_warp = false, share_row_with_other_thread = false;
     // read_index[5] / padding_val_arr: padded arrays, row-major inside each WLB
-    std::vector<u32> pad_col;
+    Arr<u32> pad_col;
+    Arr<u32> tlb_row; // row of every TLB, relative to its WLB (first_row of the TLB level)
     ValBuf pad_val;
     bool padded = false;
     // block_value operator (not one of the reference's): the sub-matrix is to be stored as dense block_r x block_c blocks
@@ -135,8 +149,8 @@ struct Matrix
     u64 n_rows = 0, n_cols = 0, nnz = 0;
     int val_dt = ASP_F32;
     // dense view, CSR (rows are in sorted order after DENSE_ROW_COARSE_SORT)
-    std::vector<u64> rowptr;
-    std::vector<u32> col;
+    Arr<u64> rowptr;
+    Arr<u32> col;
     ValBuf val;
     bool is_sorted = false;
     std::shared_ptr<std::vector<uint8_t>> sorted_row_index; // new -> old, narrowed to perm_dt
@@ -187,11 +201,12 @@ std::vector<std::vector<u64>> wlb_rows_evenly(const CompressedBlock &b, u64 rows
 void sep_warp_level_col_fixed(CompressedBlock &b, u64 col_block_nnz);
 // COMPRESSED_THREAD_LEVEL_ROW_DIV / _COL_DIV (sep_thread_level_col_ell_with_padding, op_manager.cc:3105):
 // tlb_size == 0 means "one TLB per row" (TLB size = the WLB's longest row)
-void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size);
+void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, bool tlb_rows = true);
 // COMPRESSED_THREAD_LEVEL_NNZ_DIV (sep_thread_level_acc_to_nnz, op_manager.cc:3807)
 void sep_thread_level_acc_to_nnz(CompressedBlock &b, u64 tlb_nnz);
-// execute_default_div_to_complete_each_level_blocking (default_auto_tuner.cc:384)
-void complete_each_level_blocking(CompressedBlock &b);
+// execute_default_div_to_complete_each_level_blocking (default_auto_tuner.cc:384); `rows_per_unit`: the template finds its
+// rows in the BLB and WLB levels, so the row of every TLB (one per non-zero in the default division) is not kept
+void complete_each_level_blocking(CompressedBlock &b, bool rows_per_unit);
 
 // ---- templates: init_<template> + try_all_compress -------------------------------------------
 // returns false and sets err when the tiling does not fit the template

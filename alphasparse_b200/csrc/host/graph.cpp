@@ -252,13 +252,33 @@ asp_status asp_matrix_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t *
     if (val_dtype != ASP_F32 && val_dtype != ASP_F64) return hfail(ASP_ERR_UNSUPPORTED, "values must be f32 or f64");
     if (n_rows == 0 || n_cols == 0 || n_cols > 0xffffffffull) return hfail(ASP_ERR_INVALID_ARG, "bad shape");
     if (indptr[0] != 0) return hfail(ASP_ERR_INVALID_ARG, "indptr[0] != 0");
-    for (uint64_t r = 0; r < n_rows; r++)
+    // the first row with a fault, and which of the faults below it is
+    uint64_t bad_row = n_rows;
+#pragma omp parallel for schedule(static) reduction(min : bad_row) if (n_rows > kParallelRows)
+    for (int64_t r = 0; r < (int64_t)n_rows; r++)
+        if (indptr[r + 1] < indptr[r]) bad_row = std::min<uint64_t>(bad_row, (uint64_t)r);
+    if (bad_row == n_rows) // (rows are only looked into once the offsets are known to be in order)
     {
-        if (indptr[r + 1] < indptr[r]) return hfail(ASP_ERR_INVALID_ARG, "indptr decreases");
-        for (int64_t k = indptr[r]; k < indptr[r + 1]; k++)
+#pragma omp parallel for schedule(dynamic, 4096) reduction(min : bad_row) if ((uint64_t)indptr[n_rows] > kParallelNnz)
+        for (int64_t r = 0; r < (int64_t)n_rows; r++)
+        {
+            bool bad = false;
+            uint32_t prev = 0;
+            for (int64_t k = indptr[r]; k < indptr[r + 1]; k++)
+            {
+                bad |= indices[k] >= n_cols || indices[k] < prev;
+                prev = indices[k];
+            }
+            if (bad) bad_row = std::min<uint64_t>(bad_row, (uint64_t)r);
+        }
+    }
+    if (bad_row < n_rows)
+    {
+        if (indptr[bad_row + 1] < indptr[bad_row]) return hfail(ASP_ERR_INVALID_ARG, "indptr decreases");
+        for (int64_t k = indptr[bad_row]; k < indptr[bad_row + 1]; k++)
         {
             if (indices[k] >= n_cols) return hfail(ASP_ERR_BOUNDS, "column index outside the matrix");
-            if (k > indptr[r] && indices[k] < indices[k - 1]) return hfail(ASP_ERR_INVALID_ARG, "columns are not sorted inside a row");
+            if (k > indptr[bad_row] && indices[k] < indices[k - 1]) return hfail(ASP_ERR_INVALID_ARG, "columns are not sorted inside a row");
         }
     }
     if (indptr[n_rows] == 0) return hfail(ASP_ERR_INVALID_ARG, "matrix without non-zeros");
@@ -379,8 +399,8 @@ asp_status asp_dense_execute(const asp_matrix *in, const char *spec, asp_matrix 
             if (!apply_dense_node(m, std::vector<std::string>(tok.begin() + 1, tok.end()), compressed, err)) return hfail(ASP_ERR_INVALID_ARG, err);
         }
         if (!compressed) compress_dense_view(m);
-        std::vector<u32>().swap(m.col);
-        std::vector<uint8_t>().swap(m.val.b);
+        m.col.clear();
+        m.val.b.clear();
         *out = h.release();
     }
     catch (const std::bad_alloc &)
@@ -397,6 +417,7 @@ asp_status asp_matrix_sub_rows(const asp_matrix *m, int sub, uint64_t *n_rows, u
     if (!m || !m->m->is_compressed || sub < 0 || sub >= (int)m->m->blocks.size()) return hfail(ASP_ERR_INVALID_ARG, "bad sub-matrix id");
     const CompressedBlock &b = m->m->blocks[sub];
     u64 mn = ~0ull, mx = 0;
+#pragma omp parallel for schedule(static) reduction(min : mn) reduction(max : mx) if (b.n_rows > kParallelRows)
     for (u64 r = 0; r < b.n_rows; r++)
     {
         const u64 l = b.rowptr[r + 1] - b.rowptr[r];
@@ -505,8 +526,8 @@ asp_status asp_graph_execute(const asp_matrix *in, const char *spec, asp_format 
             }
             if (!compressed) compress_dense_view(m);
             // the dense view is no longer needed once every block holds its slice
-            std::vector<u32>().swap(m.col);
-            std::vector<uint8_t>().swap(m.val.b);
+            m.col.clear();
+            m.val.b.clear();
         }
         Matrix &m = *F->m;
         const size_t nsub = m.blocks.size();
@@ -527,7 +548,7 @@ asp_status asp_graph_execute(const asp_matrix *in, const char *spec, asp_format 
             const int type = template_of_name(s->templ);
             if ((b.block_r != 0) != (type == ASP_BLOCK_ELL_TEMPLATE)) return hfail(ASP_ERR_INVALID_ARG, "the block_value node and the template B1 go together");
             if ((b.diag_max != 0) != (type == ASP_DIAG_TEMPLATE)) return hfail(ASP_ERR_INVALID_ARG, "the diag_value node and the template D1 go together");
-            if (!b.block_r && !b.diag_max) complete_each_level_blocking(b);
+            if (!b.block_r && !b.diag_max) complete_each_level_blocking(b, type == ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE || type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE || type == ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE);
             if (type < 0) return hfail(ASP_ERR_INVALID_ARG, "unknown template " + s->templ);
             if (type == ASP_EMPTY_TEMPLATE)
             {
@@ -539,11 +560,11 @@ asp_status asp_graph_execute(const asp_matrix *in, const char *spec, asp_format 
             if (s->threads > 0) F->subs[i].thread_num_in_block = s->threads;
             if (s->reduce > 0) F->subs[i].thread_num_of_row_reduce = s->reduce;
             // the tiled intermediate is not needed once the template owns its arrays
-            std::vector<u32>().swap(b.pad_col);
-            std::vector<uint8_t>().swap(b.pad_val.b);
-            std::vector<u32>().swap(b.col);
-            std::vector<uint8_t>().swap(b.val.b);
-            std::vector<u64>().swap(b.tlb.first_row.v);
+            b.pad_col.clear();
+            b.pad_val.b.clear();
+            b.col.clear();
+            b.val.b.clear();
+            b.tlb_row.clear();
         }
         F->build_descs();
         F->cache_from_matrix();

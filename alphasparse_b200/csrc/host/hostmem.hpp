@@ -1,0 +1,137 @@
+// Arrays of the host operators: shared, copy-free views of large buffers.
+//
+// A matrix passes through several objects on its way to a plan (asp_matrix -> compressed matrix -> format), and its
+// non-zeros only change in a few operators. An Arr is a view of a reference-counted buffer, so those hand-overs copy
+// nothing; who writes makes a buffer of its own first. Buffers are not initialised (the loops that fill them run on all
+// cores and are the first to touch the pages) and large ones ask for huge pages: with 4 KB pages the faults of a fresh
+// buffer cost more than filling it.
+#ifndef ASP_HOSTMEM_HPP
+#define ASP_HOSTMEM_HPP
+
+#include <stdint.h>
+#include <stdlib.h>
+#include <string.h>
+#include <sys/mman.h>
+
+#include <memory>
+#include <new>
+
+namespace asp
+{
+namespace host
+{
+inline std::shared_ptr<void> big_buffer(size_t bytes)
+{
+    const size_t huge = 2u << 20;
+    if (bytes < 2 * huge)
+    {
+        void *p = malloc(bytes ? bytes : 1);
+        if (!p) throw std::bad_alloc();
+        return std::shared_ptr<void>(p, free);
+    }
+    void *p = nullptr;
+    if (posix_memalign(&p, huge, (bytes + huge - 1) / huge * huge) != 0) throw std::bad_alloc();
+    madvise(p, (bytes + huge - 1) / huge * huge, MADV_HUGEPAGE); // (advice only: without huge pages everything still works)
+    return std::shared_ptr<void>(p, free);
+}
+
+// Below these a loop runs on the calling thread: waking sixteen threads and waiting for the slowest costs up to a millisecond on
+// a busy host, as much as the loop itself.
+const size_t kParallelBytes = 4u << 20;
+const uint64_t kParallelRows = 1u << 18, kParallelNnz = 1u << 19;
+
+inline void par_copy(void *dst, const void *src, size_t bytes)
+{
+    const size_t piece = 1u << 18;
+    const long long n = (long long)((bytes + piece - 1) / piece);
+#pragma omp parallel for schedule(static) if (bytes > kParallelBytes)
+    for (long long i = 0; i < n; i++)
+    {
+        const size_t o = (size_t)i * piece;
+        memcpy((char *)dst + o, (const char *)src + o, o + piece <= bytes ? piece : bytes - o);
+    }
+}
+
+inline void par_zero(void *dst, size_t bytes)
+{
+    const size_t piece = 1u << 18;
+    const long long n = (long long)((bytes + piece - 1) / piece);
+#pragma omp parallel for schedule(static) if (bytes > kParallelBytes)
+    for (long long i = 0; i < n; i++)
+    {
+        const size_t o = (size_t)i * piece;
+        memset((char *)dst + o, 0, o + piece <= bytes ? piece : bytes - o);
+    }
+}
+
+template <class T>
+class Arr
+{
+    template <class>
+    friend class Arr;
+    std::shared_ptr<void> s;
+    T *p = nullptr;
+    uint64_t n = 0;
+
+  public:
+    uint64_t size() const { return n; }
+    bool empty() const { return n == 0; }
+    const T *data() const { return p; }
+    T *mut() { return p; } // for a buffer that make() gave to this array and nobody else has seen
+    const T &operator[](uint64_t i) const { return p[i]; }
+    const T &back() const { return p[n - 1]; }
+    const T *begin() const { return p; }
+    const T *end() const { return p + n; }
+    void clear() { s.reset(), p = nullptr, n = 0; }
+    void swap(Arr &o) { std::swap(s, o.s), std::swap(p, o.p), std::swap(n, o.n); }
+    // a fresh buffer of this array alone, to be filled through the pointer that is returned
+    T *make(uint64_t count)
+    {
+        s = big_buffer(count * sizeof(T));
+        p = (T *)s.get();
+        n = count;
+        return p;
+    }
+    T *make_zero(uint64_t count)
+    {
+        make(count);
+        par_zero(p, count * sizeof(T));
+        return p;
+    }
+    void assign(const T *src, uint64_t count)
+    {
+        make(count);
+        par_copy(p, src, count * sizeof(T));
+    }
+    Arr view(uint64_t off, uint64_t count) const
+    {
+        Arr a;
+        a.s = s;
+        a.p = p + off;
+        a.n = count;
+        return a;
+    }
+    // the same buffer as bytes
+    Arr<uint8_t> bytes() const
+    {
+        Arr<uint8_t> a;
+        a.s = s;
+        a.p = (uint8_t *)p;
+        a.n = n * sizeof(T);
+        return a;
+    }
+    // `count` entries of which the first keep their values and the others are zero; returns them for writing
+    T *grow(uint64_t count)
+    {
+        Arr a;
+        a.make(count);
+        const uint64_t keep = count < n ? count : n;
+        par_copy(a.p, p, keep * sizeof(T));
+        par_zero(a.p + keep, (count - keep) * sizeof(T));
+        swap(a);
+        return p;
+    }
+};
+} // namespace host
+} // namespace asp
+#endif

@@ -89,11 +89,10 @@ asp_status asp_format_save(const asp_format *f, const char *path)
             h.role = a.role, h.dt = a.dt, h.kind = a.comp.kind, h.n_branch = (int32_t)a.comp.val.size();
             h.shared_perm = (a.shared && f->perm && a.shared.get() == f->perm.get()) ? 1 : 0;
             h.len = a.len, h.coef = a.comp.coef, h.icpt = a.comp.icpt, h.cycle = a.comp.cycle;
-            const std::vector<uint8_t> &bytes = a.shared ? *a.shared : a.bytes;
-            h.payload_bytes = h.shared_perm ? 0 : bytes.size();
+            h.payload_bytes = h.shared_perm ? 0 : a.shared ? a.shared->size() : a.bytes.size();
             for (int k = 0; k < h.n_branch && k < ASP_MAX_BRANCH; k++) h.lo[k] = a.comp.lo[k], h.hi[k] = a.comp.hi[k], h.val[k] = a.comp.val[k];
             ok = ok && put(out.f, h);
-            if (h.payload_bytes) ok = ok && fwrite(bytes.data(), 1, h.payload_bytes, out.f) == h.payload_bytes;
+            if (h.payload_bytes) ok = ok && fwrite(a.data(), 1, h.payload_bytes, out.f) == h.payload_bytes;
         }
     }
     if (!ok) return asp_host_fail(ASP_ERR_INVALID_ARG, std::string("write to ") + path + " failed");
@@ -170,8 +169,8 @@ asp_status asp_format_load(const char *path, asp_format **out)
                     const uint64_t full = h.len * (uint64_t)dtype_bytes(h.dt);
                     if ((h.kind == ASP_COMPRESS_NONE && h.payload_bytes != full) || h.payload_bytes > full)
                         return asp_host_fail(ASP_ERR_INVALID_ARG, "array payload does not match its length and element type");
-                    a.bytes.resize(h.payload_bytes);
-                    if (h.payload_bytes) ok = fread(a.bytes.data(), 1, h.payload_bytes, in.f) == h.payload_bytes;
+                    uint8_t *bytes = a.bytes.make(h.payload_bytes);
+                    if (h.payload_bytes) ok = fread(bytes, 1, h.payload_bytes, in.f) == h.payload_bytes;
                 }
             }
         }

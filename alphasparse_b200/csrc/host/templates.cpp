@@ -18,13 +18,35 @@ namespace host
 // ---------------------------------------------------------------------------------------------
 // closed forms (arr_optimization.cc)
 // ---------------------------------------------------------------------------------------------
-bool detect_linear(const std::vector<u64> &a, ClosedForm &out)
+namespace
+{
+// f(i) for all i < n; long arrays on all cores once the first entries hold
+template <class F>
+bool all_of(u64 n, F &&f)
+{
+    const u64 head = std::min<u64>(n, 1u << 16);
+    for (u64 i = 0; i < head; i++)
+        if (!f(i)) return false;
+    bool ok = true;
+#pragma omp parallel for schedule(static) reduction(&& : ok) if (n > kParallelRows)
+    for (u64 i = head; i < n; i++) ok = ok && f(i);
+    return ok;
+}
+u64 max_entry(U64s a)
+{
+    u64 mx = 0;
+#pragma omp parallel for schedule(static) reduction(max : mx) if (a.n > kParallelRows)
+    for (u64 i = 0; i < a.n; i++) mx = std::max(mx, a[i]);
+    return mx;
+}
+} // namespace
+
+bool detect_linear(U64s a, ClosedForm &out)
 {
     if (a.size() <= 1) return false;
     if (a[1] < a[0]) return false;
     const u64 coef = a[1] - a[0];
-    for (size_t i = 0; i + 1 < a.size(); i++)
-        if (a[i + 1] < a[i] || a[i + 1] - a[i] != coef) return false;
+    if (!all_of(a.size() - 1, [&](u64 i) { return a[i + 1] >= a[i] && a[i + 1] - a[i] == coef; })) return false;
     out = ClosedForm();
     out.kind = ASP_COMPRESS_LINEAR;
     out.coef = coef;
@@ -32,18 +54,17 @@ bool detect_linear(const std::vector<u64> &a, ClosedForm &out)
     return true;
 }
 
-bool detect_constant(const std::vector<u64> &a, ClosedForm &out)
+bool detect_constant(U64s a, ClosedForm &out)
 {
     if (a.empty()) return false;
-    for (u64 v : a)
-        if (v != a[0]) return false;
+    if (!all_of(a.size(), [&](u64 i) { return a[i] == a[0]; })) return false;
     out = ClosedForm();
     out.kind = ASP_COMPRESS_CONSTANT;
     out.icpt = a[0];
     return true;
 }
 
-bool detect_branch(const std::vector<u64> &a, ClosedForm &out)
+bool detect_branch(U64s a, ClosedForm &out)
 {
     // the reference asserts arr_size > 2 here (arr_optimization.cc:117) and aborts on shorter arrays;
     // shorter arrays simply stay uncompressed
@@ -67,7 +88,7 @@ bool detect_branch(const std::vector<u64> &a, ClosedForm &out)
     return true;
 }
 
-bool detect_cycle_linear(const std::vector<u64> &a, u64 cycle, ClosedForm &out)
+bool detect_cycle_linear(U64s a, u64 cycle, ClosedForm &out)
 {
     if (!(cycle < a.size()) || a.size() % cycle != 0 || cycle <= 1) return false;
     const u64 icpt = a[0], coef = a[1] - a[0];
@@ -87,7 +108,7 @@ bool detect_cycle_linear(const std::vector<u64> &a, u64 cycle, ClosedForm &out)
     return true;
 }
 
-bool detect_cycle_increase(const std::vector<u64> &a, ClosedForm &out)
+bool detect_cycle_increase(U64s a, ClosedForm &out)
 {
     if (a.size() <= 2) return false;
     u64 cycle = 0;
@@ -100,8 +121,7 @@ bool detect_cycle_increase(const std::vector<u64> &a, ClosedForm &out)
         }
     if (cycle == 0) return false; // all equal: the reference asserts here
     if (a.size() % cycle != 0) return false;
-    for (size_t i = 0; i < a.size(); i++)
-        if (a[i] != a[0] + i / cycle) return false;
+    if (!all_of(a.size(), [&](u64 i) { return a[i] == a[0] + i / cycle; })) return false;
     out = ClosedForm();
     out.kind = ASP_COMPRESS_CYCLE_INCREASE;
     out.cycle = cycle;
@@ -111,27 +131,27 @@ bool detect_cycle_increase(const std::vector<u64> &a, ClosedForm &out)
 
 namespace
 {
-std::vector<uint8_t> narrow(const std::vector<u64> &v, int dt)
+template <class T>
+Arr<uint8_t> narrow_to(U64s v)
 {
-    const int es = dtype_bytes(dt);
-    std::vector<uint8_t> out(v.size() * es);
-    switch (es)
-    {
-    case 1:
-        for (size_t i = 0; i < v.size(); i++) out[i] = (uint8_t)v[i];
-        break;
-    case 2:
-        for (size_t i = 0; i < v.size(); i++) ((uint16_t *)out.data())[i] = (uint16_t)v[i];
-        break;
-    case 4:
-        for (size_t i = 0; i < v.size(); i++) ((uint32_t *)out.data())[i] = (uint32_t)v[i];
-        break;
-    default: memcpy(out.data(), v.data(), v.size() * 8);
-    }
+    Arr<uint8_t> out;
+    T *p = (T *)out.make(v.size() * sizeof(T));
+#pragma omp parallel for schedule(static) if (v.n > kParallelRows)
+    for (u64 i = 0; i < v.n; i++) p[i] = (T)v[i];
     return out;
 }
+Arr<uint8_t> narrow(U64s v, int dt)
+{
+    switch (dtype_bytes(dt))
+    {
+    case 1: return narrow_to<uint8_t>(v);
+    case 2: return narrow_to<uint16_t>(v);
+    case 4: return narrow_to<uint32_t>(v);
+    default: return narrow_to<u64>(v);
+    }
+}
 
-TemplateArray &add_meta(TemplateData &t, int role, const std::vector<u64> &v, int dt)
+TemplateArray &add_meta(TemplateData &t, int role, U64s v, int dt)
 {
     t.arrays.emplace_back();
     TemplateArray &a = t.arrays.back();
@@ -147,7 +167,7 @@ template <class D, class S_>
 void interleave_strip(D *dst, const S_ *src, u64 n, u64 S)
 {
     const u64 TB = 256;
-#pragma omp parallel for schedule(static) if (n * S > (1u << 20))
+#pragma omp parallel for schedule(static) if (n * S > kParallelNnz)
     for (u64 i0 = 0; i0 < n; i0 += TB)
     {
         const u64 i1 = std::min(n, i0 + TB);
@@ -155,11 +175,6 @@ void interleave_strip(D *dst, const S_ *src, u64 n, u64 S)
             for (u64 i = i0; i < i1; i++) dst[k * n + i] = (D)src[i * S + k];
     }
 }
-
-struct NnzArrays
-{
-    std::vector<uint8_t> col, val;
-};
 
 void interleave_cols(uint8_t *dst, int col_dt, const u32 *src, u64 n, u64 S)
 {
@@ -177,7 +192,7 @@ void interleave_vals(uint8_t *dst, int es, const uint8_t *src, u64 n, u64 S)
     else interleave_strip((uint64_t *)dst, (const uint64_t *)src, n, S);
 }
 
-void add_nnz_arrays(TemplateData &t, const CompressedBlock &b, std::vector<uint8_t> &col, std::vector<uint8_t> &val, u64 n)
+void add_nnz_arrays(TemplateData &t, const CompressedBlock &b, Arr<uint8_t> &col, Arr<uint8_t> &val, u64 n)
 {
     t.arrays.emplace_back();
     TemplateArray &v = t.arrays.back();
@@ -194,24 +209,40 @@ void add_nnz_arrays(TemplateData &t, const CompressedBlock &b, std::vector<uint8
 }
 
 // global row (relative to the sub-matrix) of every TLB, in TLB order
-std::vector<u64> tlb_global_rows(const CompressedBlock &b, bool &adjacent_equal)
+Arr<u64> tlb_global_rows(const CompressedBlock &b, bool &adjacent_equal)
 {
     const Level &B = b.blb, &W = b.wlb, &T = b.tlb;
-    std::vector<u64> rows(T.block_num);
+    Arr<u64> out;
+    u64 *rows = out.make(T.block_num);
+    const bool by_rows = B.block_num < 256; // few BLBs: the TLBs are shared out, else the BLBs
+#pragma omp parallel for schedule(dynamic, 64) if (!by_rows && T.block_num > kParallelRows)
     for (u64 i = 0; i < B.block_num; i++)
         for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++)
         {
-            const u64 base = B.first_row.v[i] + W.first_row.v[w];
-            for (u64 t = W.index.v[w]; t < W.index.v[w + 1]; t++) rows[t] = base + T.first_row.v[t];
+            const u64 base = B.first_row.v[i] + W.first_row.v[w], t0 = W.index.v[w], t1 = W.index.v[w + 1];
+#pragma omp parallel for schedule(static) if (by_rows && t1 - t0 > kParallelRows)
+            for (u64 t = t0; t < t1; t++) rows[t] = base + b.tlb_row[t];
         }
-    adjacent_equal = false;
-    for (u64 t = 1; t < rows.size(); t++)
-        if (rows[t] == rows[t - 1])
-        {
-            adjacent_equal = true;
-            break;
-        }
-    return rows;
+    adjacent_equal = T.block_num > 1 && !all_of(T.block_num - 1, [&](u64 t) { return rows[t] != rows[t + 1]; });
+    return out;
+}
+
+// CSR over TLBs: TLBs of row r are [out[r], out[r + 1])
+std::vector<u64> row_offsets(U64s rows, u64 n_rows)
+{
+    std::vector<u64> out(n_rows + 1, 0);
+    if (rows.size() > 1 && all_of(rows.size() - 1, [&](u64 t) { return rows[t] <= rows[t + 1]; }))
+    {
+        // ascending rows: out[r] is the first TLB whose row is not below r
+#pragma omp parallel for schedule(static) if (rows.n > kParallelRows)
+        for (u64 t = 0; t < rows.n; t++)
+            for (u64 r = t == 0 ? 0 : rows[t - 1] + 1; r <= rows[t]; r++) out[r] = t;
+        for (u64 r = rows.back() + 1; r <= n_rows; r++) out[r] = rows.n;
+        return out;
+    }
+    for (u64 t = 0; t < rows.n; t++) out[rows[t] + 1]++;
+    for (u64 r = 0; r < n_rows; r++) out[r + 1] += out[r];
+    return out;
 }
 
 void common_head(const Matrix &m, const CompressedBlock &b, int type, TemplateData &t)
@@ -244,23 +275,26 @@ void add_perm(const Matrix &m, TemplateData &t)
 
 // effective unit count + host-side permutation of a row map (templates whose kernels do not read
 // row_index_before_sort): rows >= the dense row count belong to COMPRESSED_ROW_PADDING
-u64 effective_and_permute(const Matrix &m, const CompressedBlock &b, std::vector<u64> &rows)
+// The rows have to be the caller's own buffer.
+u64 effective_and_permute(const Matrix &m, const CompressedBlock &b, u64 *rows, u64 n)
 {
     const u64 dense_rows = b.max_row - b.min_row + 1;
-    u64 eff = rows.size();
+    u64 eff = n;
     if (b.n_rows > dense_rows)
-        for (u64 i = 0; i < rows.size(); i++)
-            if (rows[i] >= dense_rows)
-            {
-                eff = i;
-                break;
-            }
+    {
+#pragma omp parallel for schedule(static) reduction(min : eff) if (n > kParallelRows)
+        for (u64 i = 0; i < n; i++)
+            if (rows[i] >= dense_rows) eff = std::min(eff, i);
+    }
     if (m.is_sorted)
+    {
+#pragma omp parallel for schedule(static) if (eff > kParallelRows)
         for (u64 i = 0; i < eff; i++) rows[i] = m.perm[rows[i] + b.min_row];
+    }
     return eff;
 }
 
-void try_linear_then_cycle_increase(TemplateArray &a, const std::vector<u64> &v)
+void try_linear_then_cycle_increase(TemplateArray &a, U64s v)
 {
     if (!detect_linear(v, a.comp)) detect_cycle_increase(v, a.comp);
 }
@@ -277,17 +311,15 @@ bool init_k3(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
             return false;
         }
     bool adj = false;
-    std::vector<u64> rows = tlb_global_rows(b, adj);
+    Arr<u64> rows = tlb_global_rows(b, adj);
     if (adj) t.is_atom_add = true;
     const u64 n_pad = b.pad_col.size(), P = n_pad / S;
-    std::vector<uint8_t> col(n_pad * dtype_bytes(b.col_dt)), val(n_pad * b.val.es);
-    interleave_cols(col.data(), b.col_dt, b.pad_col.data(), P, S);
-    interleave_vals(val.data(), b.val.es, b.pad_val.b.data(), P, S);
-    t.effective_num = effective_and_permute(m, b, rows);
+    Arr<uint8_t> col, val;
+    interleave_cols(col.make(n_pad * dtype_bytes(b.col_dt)), b.col_dt, b.pad_col.data(), P, S);
+    interleave_vals(val.make(n_pad * b.val.es), b.val.es, b.pad_val.b.data(), P, S);
+    t.effective_num = effective_and_permute(m, b, rows.mut(), rows.size());
     t.tlb_size = S;
-    u64 mx = 0;
-    for (u64 r : rows) mx = std::max(mx, r);
-    TemplateArray &rm = add_meta(t, ASP_ARR_GLOBAL_ROW_INDEX_OF_THREAD_LEVEL_BLOCK, rows, suitable_dtype(mx));
+    TemplateArray &rm = add_meta(t, ASP_ARR_GLOBAL_ROW_INDEX_OF_THREAD_LEVEL_BLOCK, rows, suitable_dtype(max_entry(rows)));
     try_linear_then_cycle_increase(rm, rows);
     add_perm(m, t);
     add_nnz_arrays(t, b, col, val, n_pad);
@@ -316,19 +348,18 @@ bool blb_tlb_ranges(const CompressedBlock &b, std::vector<u64> &thr, std::vector
     return true;
 }
 
-void interleave_per_blb(const CompressedBlock &b, const std::vector<u64> &thr, const std::vector<u64> &size, std::vector<uint8_t> &col, std::vector<uint8_t> &val)
+void interleave_per_blb(const CompressedBlock &b, const std::vector<u64> &thr, const std::vector<u64> &size, Arr<uint8_t> &col, Arr<uint8_t> &val)
 {
     const u64 n_pad = b.pad_col.size();
     const int cb = dtype_bytes(b.col_dt), es = b.val.es;
-    col.assign(n_pad * cb, 0);
-    val.assign(n_pad * es, 0);
+    uint8_t *cp = col.make(n_pad * cb), *vp = val.make(n_pad * es);
     const u64 nb = b.blb.block_num;
-#pragma omp parallel for schedule(dynamic, 64)
+#pragma omp parallel for schedule(dynamic, 64) if (n_pad > kParallelNnz)
     for (u64 i = 0; i < nb; i++)
     {
         const u64 nz0 = b.blb.coo_begin.v[i], n = thr[i + 1] - thr[i];
-        interleave_cols(col.data() + nz0 * cb, b.col_dt, b.pad_col.data() + nz0, n, size[i]);
-        interleave_vals(val.data() + nz0 * es, es, b.pad_val.b.data() + nz0 * es, n, size[i]);
+        interleave_cols(cp + nz0 * cb, b.col_dt, b.pad_col.data() + nz0, n, size[i]);
+        interleave_vals(vp + nz0 * es, es, b.pad_val.b.data() + nz0 * es, n, size[i]);
     }
 }
 
@@ -339,14 +370,12 @@ bool init_k2(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
     std::vector<u64> thr, size;
     if (!blb_tlb_ranges(b, thr, size, err)) return false;
     bool adj = false;
-    std::vector<u64> rows = tlb_global_rows(b, adj);
+    Arr<u64> rows = tlb_global_rows(b, adj);
     if (adj) t.is_atom_add = true;
-    std::vector<uint8_t> col, val;
+    Arr<uint8_t> col, val;
     interleave_per_blb(b, thr, size, col, val);
-    t.effective_num = effective_and_permute(m, b, rows);
-    u64 mx = 0;
-    for (u64 r : rows) mx = std::max(mx, r);
-    TemplateArray &rm = add_meta(t, ASP_ARR_GLOBAL_ROW_INDEX_OF_THREAD_LEVEL_BLOCK, rows, suitable_dtype(mx));
+    t.effective_num = effective_and_permute(m, b, rows.mut(), rows.size());
+    TemplateArray &rm = add_meta(t, ASP_ARR_GLOBAL_ROW_INDEX_OF_THREAD_LEVEL_BLOCK, rows, suitable_dtype(max_entry(rows)));
     try_linear_then_cycle_increase(rm, rows);
     TemplateArray &bt = add_meta(t, ASP_ARR_BLOCK_BEGIN_THREAD_INDEX_OFFSET, thr, suitable_dtype(thr.back()));
     detect_linear(thr, bt.comp);
@@ -384,11 +413,9 @@ bool init_k6(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
     }
     t.effective_num = b.max_row - b.min_row + 1;
     bool adj = false;
-    std::vector<u64> rows = tlb_global_rows(b, adj);
-    std::vector<u64> roff(b.n_rows + 1, 0);
-    for (u64 r : rows) roff[r + 1]++;
-    for (u64 r = 0; r < b.n_rows; r++) roff[r + 1] += roff[r];
-    std::vector<uint8_t> col, val;
+    const Arr<u64> rows = tlb_global_rows(b, adj);
+    const std::vector<u64> roff = row_offsets(rows, b.n_rows);
+    Arr<uint8_t> col, val;
     interleave_per_blb(b, thr, size, col, val); // every BLB, the last one included (the reference skips it)
     TemplateArray &ro = add_meta(t, ASP_ARR_ROW_OFFSET_IN_THREAD_TMP_RESULT, roff, suitable_dtype(roff.back()));
     std::vector<u64> brow(B.first_row.v);
@@ -410,17 +437,28 @@ bool init_k6(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
 // read_index[6] / staggered_padding_val_arr: inside every WLB the TLBs are taken in groups of 32 and
 // element k of lane l of group g moves to g*32*S + k*32 + l (op_manager.cc:3569-3589). Identity
 // when every TLB holds one non-zero.
-void staggered_arrays(const CompressedBlock &b, std::vector<uint8_t> &col, std::vector<uint8_t> &val)
+void staggered_arrays(const CompressedBlock &b, Arr<uint8_t> &col, Arr<uint8_t> &val)
 {
     const u64 n_pad = b.pad_col.size();
     const int cb = dtype_bytes(b.col_dt), es = b.val.es;
-    col.assign(n_pad * cb, 0);
-    val.assign(n_pad * es, 0);
     const Level &B = b.blb, &W = b.wlb;
+    const U64s sizes(b.tlb.coo_size.v);
+    if (all_of(sizes.size(), [&](u64 w) { return sizes[w] == 1; }))
+    {
+        val = b.pad_val.b;
+        if (cb == 4) col = b.pad_col.bytes();
+        else interleave_cols(col.make(n_pad * cb), b.col_dt, b.pad_col.data(), n_pad, 1);
+        return;
+    }
+    uint8_t *cp = col.make(n_pad * cb), *vp = val.make(n_pad * es);
     const u64 nb = B.block_num;
-#pragma omp parallel for schedule(dynamic, 64)
+    const bool by_rows = nb < 256;
+#pragma omp parallel for schedule(dynamic, 64) if (!by_rows && n_pad > kParallelNnz)
     for (u64 i = 0; i < nb; i++)
-        for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++)
+    {
+        const u64 w0 = B.index.v[i], w1 = B.index.v[i + 1];
+#pragma omp parallel for schedule(dynamic, 256) if (by_rows && w1 - w0 > 1024)
+        for (u64 w = w0; w < w1; w++)
         {
             const u64 S = b.tlb.coo_size.v[w];
             const u64 base = B.coo_begin.v[i] + W.coo_begin.v[w];
@@ -428,10 +466,11 @@ void staggered_arrays(const CompressedBlock &b, std::vector<uint8_t> &col, std::
             for (u64 g = 0; g < groups; g++)
             {
                 const u64 o = base + g * 32 * S;
-                interleave_cols(col.data() + o * cb, b.col_dt, b.pad_col.data() + o, 32, S);
-                interleave_vals(val.data() + o * es, es, b.pad_val.b.data() + o * es, 32, S);
+                interleave_cols(cp + o * cb, b.col_dt, b.pad_col.data() + o, 32, S);
+                interleave_vals(vp + o * es, es, b.pad_val.b.data() + o * es, 32, S);
             }
         }
+    }
 }
 
 std::vector<u64> first_n(const std::vector<u64> &v, u64 n) { return std::vector<u64>(v.begin(), v.begin() + n); }
@@ -455,15 +494,14 @@ bool init_k4(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
             if (w >= 1 && rows[w] == rows[w - 1]) t.is_atom_add = true;
         }
     nz[W.block_num] = b.pad_col.size();
-    t.effective_num = effective_and_permute(m, b, rows);
-    u64 mx = 0;
-    for (u64 r : rows) mx = std::max(mx, r);
+    t.effective_num = effective_and_permute(m, b, rows.data(), rows.size());
+    const u64 mx = max_entry(rows);
     TemplateArray &rm = add_meta(t, ASP_ARR_GLOBAL_ROW_INDEX_OF_WARP_LEVEL_BLOCK, rows, suitable_dtype(mx));
     try_linear_then_cycle_increase(rm, rows);
     TemplateArray &no = add_meta(t, ASP_ARR_GLOBAL_WARP_NZ_BEGIN_OFFSET, nz, suitable_dtype(b.pad_col.size() + 1));
     detect_linear(nz, no.comp);
     add_perm(m, t);
-    std::vector<uint8_t> col, val;
+    Arr<uint8_t> col, val;
     staggered_arrays(b, col, val);
     add_nnz_arrays(t, b, col, val, b.pad_col.size());
     return true;
@@ -499,7 +537,7 @@ bool init_k7(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
     TemplateArray &bn = add_meta(t, ASP_ARR_BLOCK_NZ_BEGIN_OFFSET, B.coo_begin.v, B.coo_begin.dt);
     detect_linear(B.coo_begin.v, bn.comp);
     add_perm(m, t);
-    std::vector<uint8_t> col, val;
+    Arr<uint8_t> col, val;
     staggered_arrays(b, col, val);
     add_nnz_arrays(t, b, col, val, b.pad_col.size());
     return true;
@@ -548,7 +586,7 @@ bool init_k8(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
     detect_linear(brow, br.comp);
     detect_linear(nz, fn.comp);
     add_perm(m, t);
-    std::vector<uint8_t> col, val;
+    Arr<uint8_t> col, val;
     staggered_arrays(b, col, val);
     add_nnz_arrays(t, b, col, val, b.pad_col.size());
     return true;
@@ -575,10 +613,10 @@ bool init_k1(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
     common_head(m, b, ASP_DIRECT_ATOM_TEMPLATE, t);
     const Level &B = b.blb, &W = b.wlb;
     bool adj = false;
-    std::vector<u64> rows = tlb_global_rows(b, adj);
+    Arr<u64> rows = tlb_global_rows(b, adj);
     if (adj) t.is_atom_add = true;
     if (m.is_sorted)
-        for (u64 &r : rows) r = m.perm[r + b.min_row]; // every TLB, padded rows included, as the reference does
+        for (u64 i = 0; i < rows.size(); i++) rows.mut()[i] = m.perm[rows[i] + b.min_row]; // every TLB, padded rows included, as the reference does
     u64 mx = 0;
     for (u64 r : rows) mx = std::max(mx, r);
     TemplateArray &rm = add_meta(t, ASP_ARR_GLOBAL_ROW_INDEX_OF_THREAD_LEVEL_BLOCK, rows, suitable_dtype(mx));
@@ -595,7 +633,7 @@ bool init_k1(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
     detect_linear(bnz, bn.comp);
     try_cycle_linear_warp_nz(wn, W.coo_begin.v, bw, B.index.v);
     add_perm(m, t);
-    std::vector<uint8_t> col, val;
+    Arr<uint8_t> col, val;
     staggered_arrays(b, col, val);
     add_nnz_arrays(t, b, col, val, b.pad_col.size());
     (void)err;
@@ -609,20 +647,19 @@ bool init_k5(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::st
     const Level &B = b.blb, &W = b.wlb;
     if (blbs_overlap_in_rows(B)) t.is_atom_add = true;
     bool adj = false;
-    std::vector<u64> rows = tlb_global_rows(b, adj);
-    std::vector<u64> roff(b.n_rows + 1, 0);
-    for (u64 r : rows) roff[r + 1]++;
-    for (u64 r = 0; r < b.n_rows; r++) roff[r + 1] += roff[r];
+    const Arr<u64> rows = tlb_global_rows(b, adj);
+    const std::vector<u64> roff = row_offsets(rows, b.n_rows);
     // values / columns interleaved per WLB: element k of local TLB i at base + i + k*n_w
     const u64 n_pad = b.pad_col.size();
     const int cb = dtype_bytes(b.col_dt), es = b.val.es;
-    std::vector<uint8_t> col(n_pad * cb), val(n_pad * es);
+    Arr<uint8_t> col, val;
+    uint8_t *cp = col.make(n_pad * cb), *vp = val.make(n_pad * es);
     for (u64 i = 0; i < B.block_num; i++)
         for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++)
         {
             const u64 base = B.coo_begin.v[i] + W.coo_begin.v[w], n = W.index.v[w + 1] - W.index.v[w], S = b.tlb.coo_size.v[w];
-            interleave_cols(col.data() + base * cb, b.col_dt, b.pad_col.data() + base, n, S);
-            interleave_vals(val.data() + base * es, es, b.pad_val.b.data() + base * es, n, S);
+            interleave_cols(cp + base * cb, b.col_dt, b.pad_col.data() + base, n, S);
+            interleave_vals(vp + base * es, es, b.pad_val.b.data() + base * es, n, S);
         }
     TemplateArray &ro = add_meta(t, ASP_ARR_ROW_OFFSET_IN_THREAD_TMP_RESULT, roff, suitable_dtype(roff.back()));
     std::vector<u64> brow(B.first_row.v);
@@ -669,82 +706,90 @@ bool init_k9(const Matrix &m, const CompressedBlock &b, bool with_warp_reduce, T
         return false;
     }
     const u64 S = b.tlb.coo_size.v[0];
-    // rows without non-zeros become one zero at column 0; the tail is padded to whole warps by
-    // repeating the last (row, column) with value 0
-    std::vector<u64> row;
-    std::vector<u32> col;
-    row.reserve(b.col.size() + b.n_rows);
-    col.reserve(b.col.size() + b.n_rows);
-    std::vector<u64> src; // source position of every element, ~0 for filler
-    src.reserve(b.col.size() + b.n_rows);
-    u64 last_row_with_nz = 0;
-    for (u64 r = 0; r < b.n_rows; r++)
-        if (b.rowptr[r + 1] > b.rowptr[r]) last_row_with_nz = r;
-    for (u64 r = 0; r <= last_row_with_nz; r++)
+    if (S > 62)
     {
-        if (b.rowptr[r + 1] == b.rowptr[r])
-        {
-            row.push_back(r);
-            col.push_back(0);
-            src.push_back(~0ull);
-            continue;
-        }
-        for (u64 k = b.rowptr[r]; k < b.rowptr[r + 1]; k++)
-        {
-            row.push_back(r);
-            col.push_back(b.col[k]);
-            src.push_back(k);
-        }
+        err = "CSR5-like: row-start flags + offsets do not fit in 64 bits";
+        return false;
     }
-    const u64 wn = 32 * S;
-    const u64 target = (row.size() + wn - 1) / wn * wn;
-    while (row.size() < target)
-    {
-        row.push_back(row.back());
-        col.push_back(col.back());
-        src.push_back(~0ull);
-    }
-    const u64 n = row.size(), T = n / S, Wn = T / 32;
-    // row-start flags (the first non-zero of every warp always starts a sum), first rows per warp
-    std::vector<uint8_t> flag(n);
-#pragma omp parallel for schedule(static) if (n > (1u << 20))
-    for (u64 i = 0; i < n; i++) flag[i] = (i % wn == 0) ? 1 : (row[i] != row[i - 1]);
+    // Elements: the non-zeros in row order; a row without any becomes one zero at column 0 (rows after the last non-zero are
+    // dropped); the tail is padded to whole warps by repeating the last (row, column) with value 0. Row r holds elements
+    // [first[r], first[r + 1]).
+    u64 last_row = 0;
+    for (u64 r = b.n_rows; r-- > 0;)
+        if (b.rowptr[r + 1] > b.rowptr[r])
+        {
+            last_row = r;
+            break;
+        }
+    const u64 R = last_row + 1;
+    Arr<u64> first_arr;
+    u64 *first = first_arr.make(R + 1);
+    first[0] = 0;
+    for (u64 r = 0; r < R; r++) first[r + 1] = first[r] + std::max<u64>(1, b.rowptr[r + 1] - b.rowptr[r]);
+    const u64 n_el = first[R], wn = 32 * S, n = (n_el + wn - 1) / wn * wn, T = n / S, Wn = T / 32;
+    const int cb = dtype_bytes(b.col_dt), es = b.val.es;
+    // A warp's share is built by one thread: its elements (element k of lane l of warp w goes to w*32*S + k*32 + l), the flags
+    // of its TLBs (the first element of a warp always starts a sum) and the first row that starts in each of them, relative to
+    // the warp's first row (a TLB without a row start repeats the TLB before it).
+    Arr<uint8_t> ocol, oval;
+    uint8_t *const cp = ocol.make(n * cb), *const vp = oval.make(n * es);
+    Arr<u64> flags_arr;
+    u64 *const flags = flags_arr.make(T);
+    Arr<u32> frow_arr;
+    u32 *const frow = frow_arr.make(T);
     std::vector<u64> wfirst(Wn);
-    for (u64 w = 0; w < Wn; w++) wfirst[w] = row[w * wn];
-    // per TLB: does it hold a row start, count of following start-free TLBs, first row started (relative)
-    std::vector<uint8_t> has(T, 0);
-    for (u64 tl = 0; tl < T; tl++)
-        for (u64 k = 0; k < S; k++) has[tl] |= flag[tl * S + k];
-    std::vector<u64> roff(T, 0), frow(T, 0);
-    u64 max_roff = 0, max_frow = 0, last_head = 0, run = 0;
-    for (u64 tl = 1; tl < T; tl++)
+    u64 max_frow = 0;
+#pragma omp parallel for schedule(static) reduction(max : max_frow) if (n > kParallelNnz)
+    for (u64 w = 0; w < Wn; w++)
     {
-        if (!has[tl]) run++;
-        else
+        const u64 e0 = w * wn, e1 = e0 + wn;
+        u64 r = std::min<u64>((u64)(std::upper_bound(first, first + R + 1, e0) - first) - 1, last_row);
+        wfirst[w] = r;
+        for (u64 tl = w * 32; tl < w * 32 + 32; tl++) flags[tl] = 0;
+        u64 e = e0, k = 0, lane = 0;
+        while (e < e1)
         {
-            max_roff = std::max(max_roff, run);
-            roff[last_head] = run;
-            run = 0;
+            const u64 end = r < last_row ? std::min(e1, first[r + 1]) : e1; // fillers continue the last row
+            const u64 nz0 = b.rowptr[r], nz = b.rowptr[r + 1] - nz0;
+            if (e == e0 || e == first[r])
+            {
+                const u64 tl = w * 32 + lane;
+                if (flags[tl] == 0) frow[tl] = (u32)(r - wfirst[w]);
+                flags[tl] |= 1ull << (S - 1 - k);
+            }
+            for (; e < end; e++)
+            {
+                const u64 q = e - first[r], d = e0 + k * 32 + lane;
+                if (++k == S) k = 0, lane++;
+                const u32 c = nz == 0 ? 0 : b.col[nz0 + std::min(q, nz - 1)];
+                switch (cb)
+                {
+                case 1: cp[d] = (uint8_t)c; break;
+                case 2: ((uint16_t *)cp)[d] = (uint16_t)c; break;
+                case 4: ((u32 *)cp)[d] = c; break;
+                default: ((u64 *)cp)[d] = c; break;
+                }
+                if (es == 8) ((u64 *)vp)[d] = q < nz ? ((const u64 *)b.val.b.data())[nz0 + q] : 0;
+                else ((u32 *)vp)[d] = q < nz ? ((const u32 *)b.val.b.data())[nz0 + q] : 0;
+            }
+            r++;
+        }
+        for (u64 tl = w * 32; tl < w * 32 + 32; tl++)
+        {
+            if (flags[tl] == 0) frow[tl] = frow[tl - 1]; // (the warp's first TLB always has a flag)
+            max_frow = std::max<u64>(max_frow, frow[tl]);
+        }
+    }
+    // per TLB with a row start: the number of following TLBs without one
+    std::vector<u32> roff(T, 0);
+    u64 max_roff = 0, last_head = 0;
+    for (u64 tl = 1; tl <= T; tl++)
+        if (tl == T || flags[tl] != 0)
+        {
+            roff[last_head] = (u32)(tl - 1 - last_head);
+            max_roff = std::max<u64>(max_roff, roff[last_head]);
             last_head = tl;
         }
-    }
-    max_roff = std::max(max_roff, run);
-    roff[last_head] = run;
-    for (u64 tl = 0; tl < T; tl++)
-    {
-        if (has[tl])
-        {
-            for (u64 k = 0; k < S; k++)
-                if (flag[tl * S + k])
-                {
-                    frow[tl] = row[tl * S + k] - wfirst[tl / 32];
-                    break;
-                }
-        }
-        else
-            frow[tl] = frow[tl - 1];
-        max_frow = std::max(max_frow, frow[tl]);
-    }
     int bits_row = bit_count(max_frow), bits_off = bit_count(max_roff);
     if (bits_row == 0) bits_row = 1;
     if (bits_off == 0) bits_off = 1;
@@ -756,46 +801,20 @@ bool init_k9(const Matrix &m, const CompressedBlock &b, bool with_warp_reduce, T
     }
     const int word = total_bits <= 8 ? 8 : total_bits <= 16 ? 16 : total_bits <= 32 ? 32 : 64;
     const int meta_dt = word == 8 ? ASP_U8 : word == 16 ? ASP_U16 : word == 32 ? ASP_U32 : ASP_U64;
-    std::vector<u64> meta(T);
-    for (u64 tl = 0; tl < T; tl++)
-    {
-        u64 f = 0;
-        for (u64 k = 0; k < S; k++)
-            if (flag[tl * S + k]) f |= 1ull << (S - 1 - k);
-        u64 v = f << (word - (int)S - bits_off - bits_row + bits_off);
-        v |= roff[tl];
-        v <<= bits_row;
-        v |= frow[tl];
-        meta[tl] = v;
-    }
+    u64 *const meta = flags; // (in place)
+#pragma omp parallel for schedule(static) if (T > kParallelRows)
+    for (u64 tl = 0; tl < T; tl++) meta[tl] = (((flags[tl] << (word - (int)S - bits_row)) | roff[tl]) << bits_row) | frow[tl];
     t.tlb_size = S;
     t.bits_word = word;
     t.bits_flag = (int)S;
     t.bits_row = bits_row;
     t.bits_off = bits_off;
     t.n_tlb = (b.col.size() + S - 1) / S;
-    if (with_warp_reduce) wfirst.push_back(row.back() + 1);
+    if (with_warp_reduce) wfirst.push_back(last_row + 1);
     TemplateArray &fr = add_meta(t, ASP_ARR_GLOBAL_FIRST_ROW_INDEX_OF_WARP_LEVEL_BLOCK, wfirst, b.row_dt);
     try_linear_then_cycle_increase(fr, wfirst);
-    add_meta(t, ASP_ARR_COMBINE_META_OF_THREAD_LEVEL_BLOCK, meta, meta_dt);
+    add_meta(t, ASP_ARR_COMBINE_META_OF_THREAD_LEVEL_BLOCK, flags_arr, meta_dt);
     add_perm(m, t);
-    // values / columns: element k of lane l of warp w at w*32*S + k*32 + l
-    const int cb = dtype_bytes(b.col_dt), es = b.val.es;
-    std::vector<uint8_t> ocol(n * cb, 0), oval(n * es, 0);
-#pragma omp parallel for schedule(static) if (n > (1u << 20))
-    for (u64 i = 0; i < n; i++)
-    {
-        const u64 tl = i / S, k = i % S, w = tl / 32, lane = tl % 32;
-        const u64 d = w * wn + k * 32 + lane;
-        switch (cb)
-        {
-        case 1: ocol[d] = (uint8_t)col[i]; break;
-        case 2: ((uint16_t *)ocol.data())[d] = (uint16_t)col[i]; break;
-        case 4: ((uint32_t *)ocol.data())[d] = col[i]; break;
-        default: ((uint64_t *)ocol.data())[d] = col[i]; break;
-        }
-        if (src[i] != ~0ull) memcpy(&oval[d * es], &b.val.b[src[i] * es], es);
-    }
     add_nnz_arrays(t, b, ocol, oval, n);
     return true;
 }
@@ -813,55 +832,63 @@ bool init_block_ell(const Matrix &m, const CompressedBlock &b, TemplateData &t, 
     const u64 width = b.max_col - b.min_col + 1;
     if (width % c) return err = "block_value: the columns of the sub-matrix are not a multiple of the block width", false;
     const u64 NBR = (b.n_rows + r - 1) / r, NB = (NBR + 1) / 2 * 2;
-    // pass 1: block columns per block row (merged over its r rows), and how full the blocks are
-    std::vector<u64> bptr(NBR + 1, 0);
-    std::vector<u32> bcol;
-    {
-        std::vector<u64> cnt(NBR, 0);
-#pragma omp parallel
-        {
-            std::vector<u32> tmp;
-#pragma omp for schedule(static)
-            for (int64_t br = 0; br < (int64_t)NBR; br++)
-            {
-                tmp.clear();
-                for (u64 row = (u64)br * r; row < std::min<u64>(b.n_rows, ((u64)br + 1) * r); row++)
-                    for (u64 k = b.rowptr[row]; k < b.rowptr[row + 1]; k++) tmp.push_back((u32)(b.col[k] / c));
-                std::sort(tmp.begin(), tmp.end());
-                cnt[br] = (u64)(std::unique(tmp.begin(), tmp.end()) - tmp.begin());
-            }
-        }
-        for (u64 br = 0; br < NBR; br++) bptr[br + 1] = bptr[br] + cnt[br];
-        bcol.resize(bptr[NBR]);
-#pragma omp parallel
-        {
-            std::vector<u32> tmp;
-#pragma omp for schedule(static)
-            for (int64_t br = 0; br < (int64_t)NBR; br++)
-            {
-                tmp.clear();
-                for (u64 row = (u64)br * r; row < std::min<u64>(b.n_rows, ((u64)br + 1) * r); row++)
-                    for (u64 k = b.rowptr[row]; k < b.rowptr[row + 1]; k++) tmp.push_back((u32)(b.col[k] / c));
-                std::sort(tmp.begin(), tmp.end());
-                tmp.erase(std::unique(tmp.begin(), tmp.end()), tmp.end());
-                std::copy(tmp.begin(), tmp.end(), bcol.begin() + bptr[br]);
-            }
-        }
-    }
+    // pass 1: block columns of every block row (merged over its r rows), from where the non-zeros of its first row begin
+    Arr<u32> bcol_arr;
+    u32 *const bcol = bcol_arr.make(std::max<u64>(1, b.col.size()));
+    std::vector<u32> cnt(NBR, 0);
     u64 W = 0;
-    for (u64 br = 0; br < NBR; br++) W = std::max(W, bptr[br + 1] - bptr[br]);
+#pragma omp parallel for schedule(static) reduction(max : W) if (b.nnz() > kParallelNnz)
+    for (int64_t br = 0; br < (int64_t)NBR; br++)
+    {
+        const u64 row0 = (u64)br * r, row1 = std::min<u64>(b.n_rows, row0 + r), nz0 = b.rowptr[row0];
+        u32 *const o = bcol + nz0;
+        // the columns of a row ascend: its block columns come out in order; further rows usually repeat them
+        u64 n = 0;
+        for (u64 k = nz0; k < b.rowptr[row0 + 1]; k++)
+        {
+            const u32 c0 = b.col[k] / (u32)c;
+            if (n == 0 || o[n - 1] != c0) o[n++] = c0;
+        }
+        bool merged = false;
+        for (u64 row = row0 + 1; row < row1; row++)
+        {
+            u64 q = 0;
+            const u64 sorted = n;
+            for (u64 k = b.rowptr[row]; k < b.rowptr[row + 1]; k++)
+            {
+                const u32 c0 = b.col[k] / (u32)c;
+                if (merged)
+                {
+                    o[n++] = c0; // (at most one entry per non-zero: it stays inside the block row's share)
+                    continue;
+                }
+                while (q < sorted && o[q] < c0) q++;
+                if (q < sorted && o[q] == c0) continue;
+                o[n++] = c0;
+            }
+            merged = merged || n > sorted;
+        }
+        if (merged)
+        {
+            std::sort(o, o + n);
+            n = (u64)(std::unique(o, o + n) - o);
+        }
+        cnt[br] = (u32)n;
+        W = std::max(W, n);
+    }
     if (W == 0) return err = "block_value: sub-matrix without non-zeros", false;
     const u64 stored = NB * W * r * c;
     if (b.nnz() == 0 || (double)stored / (double)b.nnz() > 8.0) return err = "block_value: the matrix is not made of dense blocks of this size (more than 8 stored values per non-zero)", false;
     // pass 2: the arrays
     const int es = b.val.es;
-    std::vector<uint8_t> idx(NB * W * 4, 0), val(stored * (u64)es, 0);
-    u32 *ip = (u32 *)idx.data();
-#pragma omp parallel for schedule(static)
+    Arr<uint8_t> idx, val;
+    u32 *const ip = (u32 *)idx.make_zero(NB * W * 4);
+    uint8_t *const vp = val.make_zero(stored * (u64)es);
+#pragma omp parallel for schedule(static) if (b.nnz() > kParallelNnz)
     for (int64_t br = 0; br < (int64_t)NBR; br++)
     {
-        const u64 n = bptr[br + 1] - bptr[br];
-        const u32 *bc = bcol.data() + bptr[br];
+        const u64 n = cnt[br];
+        const u32 *bc = bcol + b.rowptr[(u64)br * r];
         for (u64 k = 0; k < W; k++) ip[k * NB + br] = k < n ? bc[k] : (n ? bc[n - 1] : 0); // zero blocks repeat the last block column
         for (u64 row = (u64)br * r; row < std::min<u64>(b.n_rows, ((u64)br + 1) * r); row++)
         {
@@ -872,7 +899,7 @@ bool init_block_ell(const Matrix &m, const CompressedBlock &b, TemplateData &t, 
                 const u32 cb = b.col[q] / (u32)c;
                 while (bc[k] != cb) k++;
                 const u64 j = b.col[q] - (u64)cb * c;
-                memcpy(&val[(((k * r + i) * c + j) * NB + (u64)br) * es], &b.val.b[q * es], es);
+                memcpy(&vp[(((k * r + i) * c + j) * NB + (u64)br) * es], &b.val.b[q * es], es);
             }
         }
     }
@@ -912,21 +939,41 @@ bool init_diag(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::
     const int64_t ncols = (int64_t)(b.max_col - b.min_col + 1);
     // distinct offsets; a scattered matrix leaves after a few rows
     std::set<int64_t> offs;
-    for (u64 r = 0; r < b.n_rows; r++)
+    bool too_many = false;
+#pragma omp parallel if (b.nnz() > kParallelNnz)
     {
-        for (u64 k = b.rowptr[r]; k < b.rowptr[r + 1]; k++) offs.insert((int64_t)b.col[k] - (int64_t)r);
-        if (offs.size() > b.diag_max) return err = "diag_value: more than " + std::to_string(b.diag_max) + " diagonals hold non-zeros", false;
+        std::vector<int64_t> mine; // ascending
+        bool full = false;
+#pragma omp for schedule(static)
+        for (u64 r = 0; r < b.n_rows; r++)
+        {
+            size_t q = 0; // the columns of a row ascend, and so do its offsets
+            for (u64 k = full ? b.rowptr[r + 1] : b.rowptr[r]; k < b.rowptr[r + 1]; k++)
+            {
+                const int64_t o = (int64_t)b.col[k] - (int64_t)r;
+                while (q < mine.size() && mine[q] < o) q++;
+                if (q == mine.size() || mine[q] != o) mine.insert(mine.begin() + q, o);
+            }
+            full = full || mine.size() > b.diag_max;
+        }
+#pragma omp critical
+        {
+            too_many = too_many || full;
+            if (!too_many) offs.insert(mine.begin(), mine.end());
+        }
     }
+    if (too_many || offs.size() > b.diag_max) return err = "diag_value: more than " + std::to_string(b.diag_max) + " diagonals hold non-zeros", false;
     if (offs.empty()) return err = "diag_value: sub-matrix without non-zeros", false;
     const std::vector<int64_t> off(offs.begin(), offs.end());
     const u64 D = off.size();
-    std::vector<uint8_t> val(D * NR * (u64)es, 0);
-#pragma omp parallel for schedule(static)
+    Arr<uint8_t> val;
+    uint8_t *const vp = val.make_zero(D * NR * (u64)es);
+#pragma omp parallel for schedule(static) if (b.nnz() > kParallelNnz)
     for (int64_t r = 0; r < (int64_t)b.n_rows; r++)
         for (u64 k = b.rowptr[r]; k < b.rowptr[r + 1]; k++)
         {
             const u64 d = (u64)(std::lower_bound(off.begin(), off.end(), (int64_t)b.col[k] - r) - off.begin());
-            memcpy(&val[(d * NR + (u64)r) * es], &b.val.b[k * es], es);
+            memcpy(&vp[(d * NR + (u64)r) * es], &b.val.b[k * es], es);
         }
     common_head(m, b, ASP_DIAG_TEMPLATE, t);
     t.tlb_size = D;

@@ -160,7 +160,7 @@ double lines_per_gather(const TiledSource &s, bool f64)
 {
     const bool by4 = s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS ||
                      s.templ == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || s.templ == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE;
-    const u64 groups = s.stored / 128, samples = std::min<u64>(groups, 512), per_line = f64 ? 16 : 32;
+    const u64 groups = s.stored / 128, samples = std::min<u64>(groups, 256), per_line = f64 ? 16 : 32;
     if (samples == 0) return 0.0;
     u64 lines = 0;
     for (u64 q = 0; q < samples; q++)
@@ -483,6 +483,10 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     {
         if (unit_count(s) == 0) return false;
         stored += s.stored;
+    }
+    if ((double)stored / (0.85 * 290e3) < 12.0) return false; // (see below; no need to look at the columns)
+    for (const TiledSource &s : src)
+    {
         lines += lines_per_gather(s, sizeof(VT) == 8) * (double)s.stored;
     }
     const double own_us = std::max(lines / (0.85 * 290e3), (double)stored * (sv + 4) / 6.0e6);
