@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/asp_b200.h"
+#include "host/hostmem.hpp"
 #include "host_meta.h"
 #include "kernel_args.h"
 #include "kernels.h"
@@ -87,6 +88,115 @@ struct Arena
 };
 
 using asp::HostMeta;
+
+// Copies between pageable host memory and the device. The runtime moves such a copy through its own pinned buffer with one
+// thread (8 to 12 GB/s measured on this host, page faults of a fresh destination included); here all cores fill or empty a ring
+// of pinned pieces while the copy engine works on the others. Pinned memory is copied directly. 16 MB per context, allocated
+// with the first copy that is worth it, freed with the context.
+struct Stager
+{
+    static const size_t kPiece = 1u << 20;
+    static const int kPieces = 16;
+    unsigned char *ring = nullptr;
+    cudaEvent_t done[kPieces] = {};
+    bool off = false; // no pinned memory to be had: plain copies
+
+    bool ready()
+    {
+        if (ring) return true;
+        if (off) return false;
+        off = true;
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, kPiece * kPieces, cudaHostAllocDefault) != cudaSuccess)
+        {
+            cudaGetLastError();
+            return false;
+        }
+        for (int i = 0; i < kPieces; i++)
+            if (cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming) != cudaSuccess)
+            {
+                cudaGetLastError();
+                for (int j = 0; j < i; j++) cudaEventDestroy(done[j]);
+                cudaFreeHost(p);
+                return false;
+            }
+        ring = (unsigned char *)p;
+        off = false;
+        return true;
+    }
+    void release()
+    {
+        if (!ring) return;
+        for (int i = 0; i < kPieces; i++) cudaEventDestroy(done[i]);
+        cudaFreeHost(ring);
+        ring = nullptr;
+    }
+    // small copies, and memory that the runtime already knows, gain nothing
+    bool direct(const void *host, size_t bytes)
+    {
+        if (bytes < (2u << 20)) return true;
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, host) != cudaSuccess)
+        {
+            cudaGetLastError();
+            return true;
+        }
+        return at.type != cudaMemoryTypeUnregistered || !ready();
+    }
+    // the host buffer may be reused as soon as this returns, as after a pageable cudaMemcpyAsync
+    cudaError_t to_device(void *dev, const void *host, size_t bytes, cudaStream_t st)
+    {
+        if (direct(host, bytes)) return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
+        int i = 0;
+        for (size_t o = 0; o < bytes; o += kPiece, i = (i + 1) % kPieces)
+        {
+            const size_t n = std::min(kPiece, bytes - o);
+            cudaError_t e = cudaEventSynchronize(done[i]); // (an event that was never recorded counts as done)
+            if (e != cudaSuccess) return e;
+            fill(ring + i * kPiece, (const unsigned char *)host + o, n);
+            e = cudaMemcpyAsync((unsigned char *)dev + o, ring + i * kPiece, n, cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess) e = cudaEventRecord(done[i], st);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+    // complete on return
+    cudaError_t to_host(void *host, const void *dev, size_t bytes, cudaStream_t st)
+    {
+        if (direct(host, bytes))
+        {
+            cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
+            return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+        }
+        const size_t n_pieces = (bytes + kPiece - 1) / kPiece;
+        cudaError_t e = cudaSuccess;
+        auto send = [&](size_t p) { // (earlier users of the slot were on a stream that has been waited for, or on this one)
+            const size_t o = p * kPiece;
+            e = cudaMemcpyAsync(ring + p % kPieces * kPiece, (const unsigned char *)dev + o, std::min(kPiece, bytes - o), cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaEventRecord(done[p % kPieces], st);
+        };
+        for (size_t p = 0; p < n_pieces && p < (size_t)kPieces && e == cudaSuccess; p++) send(p);
+        for (size_t p = 0; p < n_pieces && e == cudaSuccess; p++)
+        {
+            e = cudaEventSynchronize(done[p % kPieces]);
+            if (e != cudaSuccess) break;
+            const size_t o = p * kPiece;
+            fill((unsigned char *)host + o, ring + p % kPieces * kPiece, std::min(kPiece, bytes - o));
+            if (p + kPieces < n_pieces) send(p + kPieces);
+        }
+        if (e != cudaSuccess) cudaStreamSynchronize(st);
+        return e;
+    }
+
+  private:
+    static void fill(unsigned char *dst, const unsigned char *src, size_t n)
+    {
+        const size_t part = 64u << 10;
+        const int parts = (int)((n + part - 1) / part);
+#pragma omp parallel for schedule(static) if (parts > 2)
+        for (int i = 0; i < parts; i++) memcpy(dst + i * part, src + i * part, std::min(part, n - i * part));
+    }
+};
 } // namespace
 
 struct asp_ctx
@@ -107,6 +217,7 @@ struct asp_ctx
     // copy streams and events of the pipelined host SpMV, created on first use
     cudaStream_t h2d = nullptr, d2h = nullptr;
     std::vector<cudaEvent_t> pipe_events;
+    Stager stager;
 };
 
 namespace
@@ -299,7 +410,7 @@ uint64_t max_of(const HostMeta &h, uint64_t count)
     case DT:                                                                           \
     {                                                                                  \
         const T *q = (const T *)h.p;                                                   \
-        _Pragma("omp parallel for reduction(max : mx) schedule(static)") for (int64_t i = 0; i < n; i++) mx = q[i] > mx ? (uint64_t)q[i] : mx; \
+        _Pragma("omp parallel for reduction(max : mx) schedule(static) if (n > (1 << 20))") for (int64_t i = 0; i < n; i++) mx = q[i] > mx ? (uint64_t)q[i] : mx; \
         break;                                                                         \
     }
             ASP_MAX_CASE(ASP_U8, uint8_t)
@@ -397,7 +508,7 @@ bool validate_contents(const asp_plan_desc &d, const std::vector<HostMeta> &hm, 
         const uint64_t rows_all = br.get(B);
         if (ro.kind == ASP_COMPRESS_NONE && ro.len < rows_all + 1) return why = "row offsets shorter than the row count", false;
         bool ok = true;
-#pragma omp parallel for schedule(static) reduction(&& : ok)
+#pragma omp parallel for schedule(static) reduction(&& : ok) if (B > 4096)
         for (int64_t b = 0; b < (int64_t)B; b++)
         {
             const uint64_t r0 = br.get(b), r1 = br.get(b + 1);
@@ -427,7 +538,7 @@ bool validate_contents(const asp_plan_desc &d, const std::vector<HostMeta> &hm, 
         const int S = (int)d.tlb_size, bw = d.bits_word;
         const uint64_t rmask = (1ull << d.bits_row) - 1;
         uint64_t top = 0; // one past the largest relative row written
-#pragma omp parallel for schedule(static) reduction(max : top)
+#pragma omp parallel for schedule(static) reduction(max : top) if (W > 4096)
         for (int64_t w = 0; w < (int64_t)W; w++)
         {
             const uint64_t R0 = fr.get(w);
@@ -533,6 +644,7 @@ void asp_ctx_destroy(asp_ctx *c)
     if (!c) return;
     DeviceGuard guard(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
+    c->stager.release();
     if (c->x) cudaFree(c->x);
     if (c->y) cudaFree(c->y);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -669,7 +781,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
     }
     if (!dry)
         for (auto &kv : placed)
-            ASP_CUDA(cudaMemcpyAsync((char *)arena->base + kv.second.off, kv.first, kv.second.bytes, cudaMemcpyHostToDevice, ctx->stream));
+            ASP_CUDA(ctx->stager.to_device((char *)arena->base + kv.second.off, kv.first, kv.second.bytes, ctx->stream));
 
     // ---- pass 2: build the kernel arguments
     auto dev_meta = [&](const HostMeta &h) {
@@ -897,7 +1009,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
                 };
                 std::vector<uint32_t> rows(2 * W);
                 uint64_t all_starts = 0;
-#pragma omp parallel for schedule(static) reduction(+ : all_starts)
+#pragma omp parallel for schedule(static) reduction(+ : all_starts) if (W > 4096)
                 for (int64_t w = 0; w < (int64_t)W; w++)
                 {
                     uint64_t starts = 0;
@@ -1053,7 +1165,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
         {
             unsigned char *base = (unsigned char *)tg->arena.base;
             cudaError_t ce = asp::tiled_setup(descs[0].val_dtype == ASP_F64);
-            for (int k = 0; k < 5 && ce == cudaSuccess; k++) ce = cudaMemcpyAsync(base + off[k], from[k], bytes[k], cudaMemcpyHostToDevice, ctx->stream);
+            for (int k = 0; k < 5 && ce == cudaSuccess; k++) ce = ctx->stager.to_device(base + off[k], from[k], bytes[k], ctx->stream);
             if (ce != cudaSuccess)
             {
                 cleanup();
@@ -1284,11 +1396,10 @@ asp_status asp_spmv_host(asp_ctx *ctx, asp_plan *const *plans, int n_plans, cons
     const size_t xb = g.n_cols * g.es, yb = g.n_rows * g.es;
     st = ensure_xy(ctx, xb, yb);
     if (st != ASP_OK) return st;
-    ASP_CUDA(cudaMemcpyAsync(ctx->x, h_x, xb, cudaMemcpyHostToDevice, ctx->stream));
+    ASP_CUDA(ctx->stager.to_device(ctx->x, h_x, xb, ctx->stream));
     st = asp_spmv(ctx, plans, n_plans, ctx->x, ctx->y, 1);
     if (st != ASP_OK) return st;
-    ASP_CUDA(cudaMemcpyAsync(h_y, ctx->y, yb, cudaMemcpyDeviceToHost, ctx->stream));
-    ASP_CUDA(cudaStreamSynchronize(ctx->stream));
+    ASP_CUDA(ctx->stager.to_host(h_y, ctx->y, yb, ctx->stream));
     return ASP_OK;
 }
 
