@@ -253,6 +253,7 @@ class PlanGroup:
         self._keep = keepalive
         check(lib().asp_plan_group_create(ctx.handle, self._descs, n, self._plans))
         self.n = n
+        self._spmv = lib().asp_spmv
         self.val_dtype = np.float64 if descs[0].val_dtype == F64 else np.float32
         self.n_rows = int(descs[0].n_rows)
         self.n_cols = int(descs[0].n_cols)
@@ -279,8 +280,9 @@ class PlanGroup:
     def spmv(self, d_x: int, d_y: int, zero_y=True):
         """Asynchronous y (+)= A x on device pointers (ints). zero_y: False / True / "auto"
         (clear y only when a plan accumulates with atomics)."""
-        z = 2 if zero_y == "auto" else (1 if zero_y else 0)
-        check(lib().asp_spmv(self.ctx.handle, self._plans, self.n, C.c_void_p(d_x), C.c_void_p(d_y), z))
+        status = self._spmv(self.ctx._h, self._plans, self.n, d_x, d_y, 2 if zero_y == "auto" else (1 if zero_y else 0))
+        if status:
+            check(status)
 
     def spmv_publish(self, d_x: int, d_y: int, d_y_multicast: int):
         """asp_spmv_publish: y = A x computed and sent to every rank of the multicast group from one kernel."""

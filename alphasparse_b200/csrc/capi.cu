@@ -1339,7 +1339,7 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
             return ASP_OK;
         }
     }
-    if (clear) ASP_CUDA(cudaMemsetAsync(d_y, 0, g.n_rows * g.es, ctx->stream));
+    if (clear) ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
     if (!g.first) return ASP_OK;
     int active = 0;
     for (int i = 0; i < n_plans; i++) active += plans[i]->templ != ASP_EMPTY_TEMPLATE;

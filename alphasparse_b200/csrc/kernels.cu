@@ -13,6 +13,7 @@
 
 #include "kernel_args.h"
 #include "kernels.h"
+#include "launch.h"
 
 namespace asp
 {
@@ -177,19 +178,6 @@ __device__ __forceinline__ void ld_stream_pinned(const T *p, T (&out)[V])
     }
 }
 
-__device__ __forceinline__ float ld_x_pinned(const float *p)
-{
-    float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ double ld_x_pinned(const double *p)
-{
-    double v;
-    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-
 // 32-byte groups (8 x f32 / 4 x f64) are fetched as two 16-byte halves
 template <class T, int V>
 __device__ __forceinline__ void ld_stream_n(const T *p, T (&out)[V])
@@ -268,7 +256,7 @@ __device__ __forceinline__ void store_rows(VT *__restrict__ y, u64 row0, const V
 }
 
 template <class VT, class CT, int V, int KS>
-__global__ void __launch_bounds__(512) k_ell(const KArgs a)
+__global__ void __launch_bounds__(512) k_ell(KArgs a)
 {
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
@@ -282,6 +270,7 @@ __global__ void __launch_bounds__(512) k_ell(const KArgs a)
     // consecutive TLBs map to consecutive rows: whole groups can be stored as vectors
     const bool unit_rows = a.m[MS_ROW_OF_TLB].kind == MK_LINEAR && a.m[MS_ROW_OF_TLB].coef == 1 && !a.atomic &&
                            ((a.m[MS_ROW_OF_TLB].icpt + radd) % V) == 0;
+    WaitOnce wait; // the first values and indices are on their way when it waits
     for (u64 g = (u64)blockIdx.x * blockDim.x + threadIdx.x; g < ngroup; g += stride)
     {
         const u64 t0 = g * V;
@@ -301,10 +290,11 @@ __global__ void __launch_bounds__(512) k_ell(const KArgs a)
                 ld_stream_n<VT, V>(vp + (u64)k * P, v[k]);
                 ld_stream_n<CT, V>(cp + (u64)k * P, c[k]);
             }
+            wait();
 #pragma unroll
             for (int k = 0; k < KS; k++)
 #pragma unroll
-                for (int j = 0; j < V; j++) acc[j] += v[k][j] * __ldg(x + c[k][j]);
+                for (int j = 0; j < V; j++) acc[j] += v[k][j] * ld_x(x + c[k][j]);
         }
         else
         {
@@ -318,11 +308,12 @@ __global__ void __launch_bounds__(512) k_ell(const KArgs a)
                 for (int u = 0; u < U; u++) ld_stream_pinned<CT, V>(cp + (u64)(k + u) * P, c[u]);
 #pragma unroll
                 for (int u = 0; u < U; u++) ld_stream_pinned<VT, V>(vp + (u64)(k + u) * P, v[u]);
+                wait();
                 VT xv[U][V];
 #pragma unroll
                 for (int u = 0; u < U; u++)
 #pragma unroll
-                    for (int j = 0; j < V; j++) xv[u][j] = ld_x_pinned(x + c[u][j]);
+                    for (int j = 0; j < V; j++) xv[u][j] = ld_x(x + c[u][j]);
 #pragma unroll
                 for (int u = 0; u < U; u++)
 #pragma unroll
@@ -339,12 +330,13 @@ __global__ void __launch_bounds__(512) k_ell(const KArgs a)
                         ld_stream_n<VT, V>(vp + (u64)(k + u) * P, v[u]);
                         ld_stream_n<CT, V>(cp + (u64)(k + u) * P, c[u]);
                     }
+                wait();
 #pragma unroll
                 for (int u = 0; u < U - 1; u++)
                     if (k + u < S)
                     {
 #pragma unroll
-                        for (int j = 0; j < V; j++) acc[j] += v[u][j] * __ldg(x + c[u][j]);
+                        for (int j = 0; j < V; j++) acc[j] += v[u][j] * ld_x(x + c[u][j]);
                     }
             }
         }
@@ -360,6 +352,7 @@ __global__ void __launch_bounds__(512) k_ell(const KArgs a)
             }
         }
     }
+    wait();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -398,7 +391,7 @@ __device__ __forceinline__ void sell_store(const KArgs &a, VT *__restrict__ y, c
 
 template <class VT, class CT, int V>
 __device__ __forceinline__ void sell_group(const KArgs &a, const VT *__restrict__ val, const CT *__restrict__ col, const VT *__restrict__ x,
-                                           VT *__restrict__ y, u64 nz, u64 n, u32 S, u64 t0, u64 radd)
+                                           VT *__restrict__ y, u64 nz, u64 n, u32 S, u64 t0, u64 radd, WaitOnce &wait)
 {
     VT acc[V];
 #pragma unroll
@@ -416,11 +409,12 @@ __device__ __forceinline__ void sell_group(const KArgs &a, const VT *__restrict_
         for (int u = 0; u < U; u++) ld_stream_pinned<CT, V>(cp + (u64)u * n, c[u]);
 #pragma unroll
         for (int u = 0; u < U; u++) ld_stream_pinned<VT, V>(vp + (u64)u * n, v[u]);
+        wait();
         VT xv[U][V];
 #pragma unroll
         for (int u = 0; u < U; u++)
 #pragma unroll
-            for (int j = 0; j < V; j++) xv[u][j] = ld_x_pinned(x + c[u][j]);
+            for (int j = 0; j < V; j++) xv[u][j] = ld_x(x + c[u][j]);
 #pragma unroll
         for (int u = 0; u < U; u++)
 #pragma unroll
@@ -440,19 +434,21 @@ __device__ __forceinline__ void sell_group(const KArgs &a, const VT *__restrict_
                 ld_stream_n<VT, V>(vp + (u64)u * n, v[u]);
                 ld_stream_n<CT, V>(cp + (u64)u * n, c[u]);
             }
+        wait();
 #pragma unroll
         for (int u = 0; u < U - 1; u++)
             if (k + u < S)
             {
 #pragma unroll
-                for (int j = 0; j < V; j++) acc[j] += v[u][j] * __ldg(x + c[u][j]);
+                for (int j = 0; j < V; j++) acc[j] += v[u][j] * ld_x(x + c[u][j]);
             }
     }
+    wait(); // (an empty strip stores its zeros too)
     sell_store<VT, V>(a, y, acc, t0, radd);
 }
 
 template <class VT, class CT, int V>
-__global__ void __launch_bounds__(256) k_sell(const KArgs a)
+__global__ void __launch_bounds__(256) k_sell(KArgs a)
 {
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
@@ -460,6 +456,7 @@ __global__ void __launch_bounds__(256) k_sell(const KArgs a)
     VT *__restrict__ y = (VT *)a.y;
     const u64 radd = a.row_add ? a.first_row : 0;
     const Meta &bt = a.m[MS_BLK_THR];
+    WaitOnce wait; // the first values and indices are on their way when it waits
     if ((a.path & 1) == 0 && V > 1 && bt.kind == MK_LINEAR && bt.coef > 0 && (bt.coef % (32 * V)) == 0)
     {
         const u64 n = bt.coef;
@@ -476,13 +473,14 @@ __global__ void __launch_bounds__(256) k_sell(const KArgs a)
             const u64 nz0 = mget(a.m[MS_BLK_NZ], b);
             const u32 S = (u32)mget(a.m[MS_TLB_SIZE], b);
             if ((nz0 % V) == 0)
-                sell_group<VT, CT, V>(a, val, col, x, y, nz0 + i, n, S, t0, radd);
+                sell_group<VT, CT, V>(a, val, col, x, y, nz0 + i, n, S, t0, radd, wait);
             else
             {
 #pragma unroll
-                for (int j = 0; j < V; j++) sell_group<VT, CT, 1>(a, val, col, x, y, nz0 + i + j, n, S, t0 + j, radd);
+                for (int j = 0; j < V; j++) sell_group<VT, CT, 1>(a, val, col, x, y, nz0 + i + j, n, S, t0 + j, radd, wait);
             }
         }
+        wait();
         return;
     }
     for (u64 b = blockIdx.x; b < a.n_units; b += gridDim.x)
@@ -498,7 +496,7 @@ __global__ void __launch_bounds__(256) k_sell(const KArgs a)
             for (u64 i = (u64)threadIdx.x * V; i < n; i += (u64)blockDim.x * V)
             {
                 if (t0 + i >= a.effective) break;
-                sell_group<VT, CT, V>(a, val, col, x, y, nz0 + i, n, S, t0 + i, radd);
+                sell_group<VT, CT, V>(a, val, col, x, y, nz0 + i, n, S, t0 + i, radd, wait);
             }
         }
         else
@@ -506,10 +504,11 @@ __global__ void __launch_bounds__(256) k_sell(const KArgs a)
             for (u64 i = threadIdx.x; i < n; i += blockDim.x)
             {
                 if (t0 + i >= a.effective) break;
-                sell_group<VT, CT, 1>(a, val, col, x, y, nz0 + i, n, S, t0 + i, radd);
+                sell_group<VT, CT, 1>(a, val, col, x, y, nz0 + i, n, S, t0 + i, radd, wait);
             }
         }
     }
+    wait();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -518,8 +517,10 @@ __global__ void __launch_bounds__(256) k_sell(const KArgs a)
 // double and always adds atomically when rows are shared.
 // ---------------------------------------------------------------------------------------------
 template <class VT, class CT>
-__global__ void __launch_bounds__(1024) k_direct3(const KArgs a)
+__global__ void __launch_bounds__(1024) k_direct3(KArgs a)
 {
+    grid_wait();
+    grid_release();
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
     const VT *__restrict__ x = (const VT *)a.x + a.first_col;
@@ -551,7 +552,7 @@ __global__ void __launch_bounds__(1024) k_direct3(const KArgs a)
                         ld_stream_n<VT, 4>(val + nz, v);
                         ld_stream_n<CT, 4>(col + nz, c);
 #pragma unroll
-                        for (int j = 0; j < 4; j++) acc[j] += (double)(v[j] * __ldg(x + c[j]));
+                        for (int j = 0; j < 4; j++) acc[j] += (double)(v[j] * ld_x(x + c[j]));
                     }
                     const u64 t = t0 + g * 32 + 4 * (lane & 7);
 #pragma unroll
@@ -563,7 +564,7 @@ __global__ void __launch_bounds__(1024) k_direct3(const KArgs a)
                 {
                     double acc = 0;
                     u64 nz = wnz + g * 32 * S + lane;
-                    for (u32 k = 0; k < S; k++, nz += 32) acc += (double)(__ldcs(val + nz) * __ldg(x + __ldcs(col + nz)));
+                    for (u32 k = 0; k < S; k++, nz += 32) acc += (double)(__ldcs(val + nz) * ld_x(x + __ldcs(col + nz)));
                     const u64 t = t0 + g * 32 + lane;
                     out_add(y, mget(a.m[MS_ROW_OF_TLB], t) + radd, (VT)acc, a.atomic != 0);
                 }
@@ -589,19 +590,21 @@ __device__ __forceinline__ VT warp_chunk_dot(const VT *__restrict__ val, const C
             ld_stream_n<VT, V>(val + i, v);
             ld_stream_n<CT, V>(col + i, c);
 #pragma unroll
-            for (int j = 0; j < V; j++) acc += v[j] * __ldg(x + c[j]);
+            for (int j = 0; j < V; j++) acc += v[j] * ld_x(x + c[j]);
         }
     }
     else
     {
-        for (u64 i = beg + lane; i < end; i += 32) acc += __ldcs(val + i) * __ldg(x + __ldcs(col + i));
+        for (u64 i = beg + lane; i < end; i += 32) acc += __ldcs(val + i) * ld_x(x + __ldcs(col + i));
     }
     return acc;
 }
 
 template <class VT, class CT>
-__global__ void __launch_bounds__(1024) k_warp_row(const KArgs a)
+__global__ void __launch_bounds__(1024) k_warp_row(KArgs a)
 {
+    grid_wait();
+    grid_release();
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
     const VT *__restrict__ x = (const VT *)a.x + a.first_col;
@@ -621,9 +624,11 @@ __global__ void __launch_bounds__(1024) k_warp_row(const KArgs a)
 // SHARED_MEMORY_LONG_ROW_TEMPLATE: CTA <-> BLB = a chunk of one long row.
 // ---------------------------------------------------------------------------------------------
 template <class VT, class CT>
-__global__ void __launch_bounds__(1024) k_long_row(const KArgs a)
+__global__ void __launch_bounds__(1024) k_long_row(KArgs a)
 {
     __shared__ VT part[32];
+    grid_wait();
+    grid_release();
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
     const VT *__restrict__ x = (const VT *)a.x + a.first_col;
@@ -652,7 +657,7 @@ __global__ void __launch_bounds__(1024) k_long_row(const KArgs a)
 #pragma unroll
                 for (int u = 0; u < 2; u++)
 #pragma unroll
-                    for (int j = 0; j < V; j++) xv[u][j] = ld_x_pinned(x + c[u][j]);
+                    for (int j = 0; j < V; j++) xv[u][j] = ld_x(x + c[u][j]);
 #pragma unroll
                 for (int u = 0; u < 2; u++)
 #pragma unroll
@@ -665,12 +670,12 @@ __global__ void __launch_bounds__(1024) k_long_row(const KArgs a)
                 ld_stream_n<VT, V>(val + i, v);
                 ld_stream_n<CT, V>(col + i, c);
 #pragma unroll
-                for (int j = 0; j < V; j++) acc += v[j] * __ldg(x + c[j]);
+                for (int j = 0; j < V; j++) acc += v[j] * ld_x(x + c[j]);
             }
         }
         else
         {
-            for (u64 i = beg + threadIdx.x; i < end; i += blockDim.x) acc += __ldcs(val + i) * __ldg(x + __ldcs(col + i));
+            for (u64 i = beg + threadIdx.x; i < end; i += blockDim.x) acc += __ldcs(val + i) * ld_x(x + __ldcs(col + i));
         }
         acc = warp_sum(acc);
         __syncthreads(); // previous iteration's readers are done with part[]
@@ -715,7 +720,7 @@ __device__ __forceinline__ void smem_row_reduce(const KArgs &a, const VT *part, 
 
 // SHARED_MEMORY_TEMPLATE_WARP_COMPRESS (row-grouped CSR): CTA <-> BLB; TLB partials in smem.
 template <class VT, class CT>
-__global__ void __launch_bounds__(1024) k_smem_tlb(const KArgs a)
+__global__ void __launch_bounds__(1024) k_smem_tlb(KArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     VT *part = reinterpret_cast<VT *>(smem_raw);
@@ -723,6 +728,7 @@ __global__ void __launch_bounds__(1024) k_smem_tlb(const KArgs a)
     const CT *__restrict__ col = (const CT *)a.col;
     const VT *__restrict__ x = (const VT *)a.x + a.first_col;
     VT *__restrict__ y = (VT *)a.y;
+    WaitOnce wait; // the first values and indices are on their way when it waits
     for (u64 b = blockIdx.x; b < a.n_units; b += gridDim.x)
     {
         const u64 nz0 = mget(a.m[MS_BLK_NZ], b);
@@ -754,10 +760,11 @@ __global__ void __launch_bounds__(1024) k_smem_tlb(const KArgs a)
                     for (int u = 0; u < U; u++) ld_stream_pinned<CT, V>(cp + (u64)u * n, c[u]);
 #pragma unroll
                     for (int u = 0; u < U; u++) ld_stream_pinned<VT, V>(vp + (u64)u * n, v[u]);
+                    wait();
 #pragma unroll
                     for (int u = 0; u < U; u++)
 #pragma unroll
-                        for (int j = 0; j < V; j++) xv[u][j] = ld_x_pinned(x + c[u][j]);
+                        for (int j = 0; j < V; j++) xv[u][j] = ld_x(x + c[u][j]);
 #pragma unroll
                     for (int u = 0; u < U; u++)
 #pragma unroll
@@ -771,8 +778,9 @@ __global__ void __launch_bounds__(1024) k_smem_tlb(const KArgs a)
                     CT c[V];
                     ld_stream_n<VT, V>(vp, v);
                     ld_stream_n<CT, V>(cp, c);
+                    wait();
 #pragma unroll
-                    for (int j = 0; j < V; j++) acc[j] += v[j] * __ldg(x + c[j]);
+                    for (int j = 0; j < V; j++) acc[j] += v[j] * ld_x(x + c[j]);
                     vp += n;
                     cp += n;
                 }
@@ -785,30 +793,35 @@ __global__ void __launch_bounds__(1024) k_smem_tlb(const KArgs a)
             for (u64 i = threadIdx.x; i < n; i += blockDim.x)
             {
                 VT acc = 0;
+                wait();
                 const VT *vp = val + nz0 + i;
                 const CT *cp = col + nz0 + i;
 #pragma unroll 4
                 for (u32 k = 0; k < S; k++)
                 {
-                    acc += __ldcs(vp) * __ldg(x + __ldcs(cp));
+                    acc += __ldcs(vp) * ld_x(x + __ldcs(cp));
                     vp += n;
                     cp += n;
                 }
                 part[i] = acc;
             }
         }
+        wait(); // (threads without a TLB write rows too)
         __syncthreads();
         smem_row_reduce<VT>(a, part, y, r0, r1, g0);
     }
+    wait();
 }
 
 // SHARED_MEMORY_TEMPLATE: BLB -> WLB -> TLB with WLB-level interleave (element k of local TLB i
 // of a WLB at bnz + wnz + i + k*n_w), partials of the whole BLB in smem, then the row reduce.
 template <class VT, class CT>
-__global__ void __launch_bounds__(1024) k_smem3(const KArgs a)
+__global__ void __launch_bounds__(1024) k_smem3(KArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     VT *part = reinterpret_cast<VT *>(smem_raw);
+    grid_wait();
+    grid_release();
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
     const VT *__restrict__ x = (const VT *)a.x + a.first_col;
@@ -842,7 +855,7 @@ __global__ void __launch_bounds__(1024) k_smem3(const KArgs a)
                         ld_stream_n<VT, 4>(val + nz, v);
                         ld_stream_n<CT, 4>(col + nz, c);
 #pragma unroll
-                        for (int j = 0; j < 4; j++) acc[j] += v[j] * __ldg(x + c[j]);
+                        for (int j = 0; j < 4; j++) acc[j] += v[j] * ld_x(x + c[j]);
                     }
 #pragma unroll
                     for (int j = 0; j < 4; j++) part[t0 + i + j - tb0] = acc[j];
@@ -853,7 +866,7 @@ __global__ void __launch_bounds__(1024) k_smem3(const KArgs a)
                 {
                     VT acc = 0;
                     u64 nz = wnz + i;
-                    for (u32 k = 0; k < S; k++, nz += n) acc += __ldcs(val + nz) * __ldg(x + __ldcs(col + nz));
+                    for (u32 k = 0; k < S; k++, nz += n) acc += __ldcs(val + nz) * ld_x(x + __ldcs(col + nz));
                     part[t0 + i - tb0] = acc;
                 }
         }
@@ -865,10 +878,12 @@ __global__ void __launch_bounds__(1024) k_smem3(const KArgs a)
 // SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE: CTA <-> BLB (a few rows); warp <-> WLB (chunk of
 // one row) reduced by shuffle into smem; then the row reduce over WLB partials.
 template <class VT, class CT>
-__global__ void __launch_bounds__(1024) k_smem_wlb(const KArgs a)
+__global__ void __launch_bounds__(1024) k_smem_wlb(KArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     VT *part = reinterpret_cast<VT *>(smem_raw);
+    grid_wait();
+    grid_release();
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
     const VT *__restrict__ x = (const VT *)a.x + a.first_col;
@@ -916,20 +931,22 @@ __device__ __forceinline__ void strided_products(const VT *__restrict__ val, con
         for (int u = 0; u < U; u++) ld_stream_pinned<VT, 1>(val + nz + 32 * u, v[u]);
         VT xv[U];
 #pragma unroll
-        for (int u = 0; u < U; u++) xv[u] = ld_x_pinned(x + c[u][0]);
+        for (int u = 0; u < U; u++) xv[u] = ld_x(x + c[u][0]);
 #pragma unroll
         for (int u = 0; u < U; u++) p[u] = v[u][0] * xv[u];
     }
     else
     {
 #pragma unroll
-        for (int u = 0; u < U; u++) p[u] = (u32)u < cnt ? __ldcs(val + nz + 32 * u) * __ldg(x + __ldcs(col + nz + 32 * u)) : VT(0);
+        for (int u = 0; u < U; u++) p[u] = (u32)u < cnt ? __ldcs(val + nz + 32 * u) * ld_x(x + __ldcs(col + nz + 32 * u)) : VT(0);
     }
 }
 
 template <class VT, class CT, bool WARP_FAST>
-__global__ void __launch_bounds__(256) k_csr5(const KArgs a)
+__global__ void __launch_bounds__(256) k_csr5(KArgs a)
 {
+    grid_wait();
+    grid_release();
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
     const VT *__restrict__ x = (const VT *)a.x + a.first_col;
@@ -1025,33 +1042,33 @@ __global__ void __launch_bounds__(256) k_csr5(const KArgs a)
 // launch dispatch
 // ---------------------------------------------------------------------------------------------
 template <class VT, class CT, int V>
-static void launch_ell_v(const KArgs &a, dim3 grid, dim3 block, cudaStream_t st)
+static cudaError_t launch_ell_v(const KArgs &a, dim3 grid, dim3 block, cudaStream_t st)
 {
     if constexpr (V == 2 || V == 4)
     {
         switch (a.tlb_size)
         {
-        case 1: k_ell<VT, CT, V, 1><<<grid, block, 0, st>>>(a); return;
-        case 2: k_ell<VT, CT, V, 2><<<grid, block, 0, st>>>(a); return;
-        case 3: k_ell<VT, CT, V, 3><<<grid, block, 0, st>>>(a); return;
-        case 4: k_ell<VT, CT, V, 4><<<grid, block, 0, st>>>(a); return;
-        case 5: k_ell<VT, CT, V, 5><<<grid, block, 0, st>>>(a); return;
-        case 6: k_ell<VT, CT, V, 6><<<grid, block, 0, st>>>(a); return;
-        case 7: k_ell<VT, CT, V, 7><<<grid, block, 0, st>>>(a); return;
-        case 8: k_ell<VT, CT, V, 8><<<grid, block, 0, st>>>(a); return;
+        case 1: return launch_pdl(k_ell<VT, CT, V, 1>, grid, block, 0, st, a);
+        case 2: return launch_pdl(k_ell<VT, CT, V, 2>, grid, block, 0, st, a);
+        case 3: return launch_pdl(k_ell<VT, CT, V, 3>, grid, block, 0, st, a);
+        case 4: return launch_pdl(k_ell<VT, CT, V, 4>, grid, block, 0, st, a);
+        case 5: return launch_pdl(k_ell<VT, CT, V, 5>, grid, block, 0, st, a);
+        case 6: return launch_pdl(k_ell<VT, CT, V, 6>, grid, block, 0, st, a);
+        case 7: return launch_pdl(k_ell<VT, CT, V, 7>, grid, block, 0, st, a);
+        case 8: return launch_pdl(k_ell<VT, CT, V, 8>, grid, block, 0, st, a);
         default: break;
         }
     }
-    k_ell<VT, CT, V, 0><<<grid, block, 0, st>>>(a);
+    return launch_pdl(k_ell<VT, CT, V, 0>, grid, block, 0, st, a);
 }
 
 template <class VT, class CT>
-static void launch_ell(const KArgs &a, dim3 grid, dim3 block, cudaStream_t st, int vec)
+static cudaError_t launch_ell(const KArgs &a, dim3 grid, dim3 block, cudaStream_t st, int vec)
 {
-    if (vec >= 8) launch_ell_v<VT, CT, 8>(a, grid, block, st);
-    else if (vec >= 4) launch_ell_v<VT, CT, 4>(a, grid, block, st);
-    else if (vec == 2) launch_ell_v<VT, CT, 2>(a, grid, block, st);
-    else launch_ell_v<VT, CT, 1>(a, grid, block, st);
+    if (vec >= 8) return launch_ell_v<VT, CT, 8>(a, grid, block, st);
+    if (vec >= 4) return launch_ell_v<VT, CT, 4>(a, grid, block, st);
+    if (vec == 2) return launch_ell_v<VT, CT, 2>(a, grid, block, st);
+    return launch_ell_v<VT, CT, 1>(a, grid, block, st);
 }
 
 template <class VT, class CT>
@@ -1060,31 +1077,27 @@ static cudaError_t launch_vc(int templ, const KArgs &a, dim3 grid, dim3 block, s
     switch (templ)
     {
     case 2: // ELL-like
-        launch_ell<VT, CT>(a, grid, block, st, vec);
-        break;
+        return launch_ell<VT, CT>(a, grid, block, st, vec);
     case 1: // SELL-like
-        if (vec >= 4) k_sell<VT, CT, 4><<<grid, block, 0, st>>>(a);
-        else if (vec == 2) k_sell<VT, CT, 2><<<grid, block, 0, st>>>(a);
-        else k_sell<VT, CT, 1><<<grid, block, 0, st>>>(a);
-        break;
-    case 0: k_direct3<VT, CT><<<grid, block, 0, st>>>(a); break;
-    case 7: k_warp_row<VT, CT><<<grid, block, 0, st>>>(a); break;
-    case 5: k_long_row<VT, CT><<<grid, block, 0, st>>>(a); break;
-    case 4: k_smem_tlb<VT, CT><<<grid, block, smem, st>>>(a); break;
-    case 3: k_smem3<VT, CT><<<grid, block, smem, st>>>(a); break;
-    case 6: k_smem_wlb<VT, CT><<<grid, block, smem, st>>>(a); break;
+        if (vec >= 4) return launch_pdl(k_sell<VT, CT, 4>, grid, block, 0, st, a);
+        if (vec == 2) return launch_pdl(k_sell<VT, CT, 2>, grid, block, 0, st, a);
+        return launch_pdl(k_sell<VT, CT, 1>, grid, block, 0, st, a);
+    case 0: return launch_pdl(k_direct3<VT, CT>, grid, block, 0, st, a);
+    case 7: return launch_pdl(k_warp_row<VT, CT>, grid, block, 0, st, a);
+    case 5: return launch_pdl(k_long_row<VT, CT>, grid, block, 0, st, a);
+    case 4: return launch_pdl(k_smem_tlb<VT, CT>, grid, block, smem, st, a);
+    case 3: return launch_pdl(k_smem3<VT, CT>, grid, block, smem, st, a);
+    case 6: return launch_pdl(k_smem_wlb<VT, CT>, grid, block, smem, st, a);
     case 8:
     case 9:
         // TLB sizes 4 / 8 / 16 / 32 with 32-bit columns run the specialised kernels; everything else the generic one
         if (csr5_specialised((int)a.tlb_size, (int)sizeof(CT), a.bits_word) && ((a.path & 2) == 0 || (a.path & 1) || a.y_mc))
             return launch_csr5(sizeof(VT) == 8, (int)sizeof(CT), (templ == 9 ? 1 : 0) | ((a.path & 1) ? 2 : 0) | (a.y_mc ? 6 : 0), a, grid.x, block.x, st);
         if (a.y_mc) return cudaErrorInvalidValue;
-        if (templ == 8) k_csr5<VT, CT, false><<<grid, block, 0, st>>>(a);
-        else k_csr5<VT, CT, true><<<grid, block, 0, st>>>(a);
-        break;
+        if (templ == 8) return launch_pdl(k_csr5<VT, CT, false>, grid, block, 0, st, a);
+        return launch_pdl(k_csr5<VT, CT, true>, grid, block, 0, st, a);
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 template <class VT>

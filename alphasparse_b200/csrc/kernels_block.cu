@@ -25,6 +25,7 @@
 
 #include "kernel_args.h"
 #include "kernels.h"
+#include "launch.h"
 
 namespace asp
 {
@@ -50,21 +51,8 @@ __device__ __forceinline__ void ld_idx(const u32 *p, u32 (&v)[2])
 {
     asm volatile("ld.global.cs.v2.u32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p));
 }
-__device__ __forceinline__ double ld_xv(const double *p)
-{
-    double v;
-    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ float ld_xv(const float *p)
-{
-    float v;
-    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-
 template <class VT, int R, int C, int D, int SPLIT>
-__global__ void __launch_bounds__(SPLIT == 8 ? 256 : 128) k_block_ell(const KArgs a)
+__global__ void __launch_bounds__(SPLIT == 8 ? 256 : 128) k_block_ell(KArgs a)
 {
     constexpr int V = 8 / sizeof(VT); // block rows of a lane
     constexpr int WARPS = SPLIT == 8 ? 8 : 4;
@@ -98,11 +86,13 @@ __global__ void __launch_bounds__(SPLIT == 8 ? 256 : 128) k_block_ell(const KArg
 #pragma unroll
         for (int s = 0; s < V; s++)
 #pragma unroll
-            for (int j = 0; j < C; j++) xv[d][s][j] = ld_xv(x + (u64)bc[d][s] * C + j);
+            for (int j = 0; j < C; j++) xv[d][s][j] = ld_x(x + (u64)bc[d][s] * C + j);
     };
 #pragma unroll
     for (int d = 0; d < D; d++)
         if ((u32)d < n) load(d, ip + (u64)d * NB, vp + (u64)d * (R * C) * NB);
+    grid_wait(); // the first indices and values are on their way
+    grid_release();
     if (n > 0) gather(0);
     ip += (u64)D * NB;
     vp += (u64)D * (R * C) * NB;
@@ -167,12 +157,11 @@ cudaError_t launch_split(const KArgs &a, unsigned block, cudaStream_t st)
     if (grid > 2147483647ull) return cudaErrorInvalidValue;
     switch (split)
     {
-    case 8: k_block_ell<VT, R, C, D, 8><<<(unsigned)grid, 256, 0, st>>>(a); break;
-    case 4: k_block_ell<VT, R, C, D, 4><<<(unsigned)grid, 128, 0, st>>>(a); break;
-    case 2: k_block_ell<VT, R, C, D, 2><<<(unsigned)grid, 128, 0, st>>>(a); break;
-    default: k_block_ell<VT, R, C, D, 1><<<(unsigned)grid, block, 0, st>>>(a); break;
+    case 8: return launch_pdl(k_block_ell<VT, R, C, D, 8>, dim3((unsigned)grid), dim3(256), 0, st, a);
+    case 4: return launch_pdl(k_block_ell<VT, R, C, D, 4>, dim3((unsigned)grid), dim3(128), 0, st, a);
+    case 2: return launch_pdl(k_block_ell<VT, R, C, D, 2>, dim3((unsigned)grid), dim3(128), 0, st, a);
+    default: return launch_pdl(k_block_ell<VT, R, C, D, 1>, dim3((unsigned)grid), dim3(block), 0, st, a);
     }
-    return cudaGetLastError();
 }
 
 template <class VT>

@@ -26,6 +26,7 @@
 
 #include "kernel_args.h"
 #include "kernels.h"
+#include "launch.h"
 
 namespace asp
 {
@@ -99,19 +100,6 @@ __device__ __forceinline__ double ld_val(const double *p)
     asm volatile("ld.global.cs.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
 }
-__device__ __forceinline__ float ld_x(const float *p)
-{
-    float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ double ld_x(const double *p)
-{
-    double v;
-    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-
 // one value to every GPU bound to the multicast object that `mc` addresses
 __device__ __forceinline__ void mc_store(float *mc, float v)
 {
@@ -140,10 +128,12 @@ __device__ __forceinline__ void put(VT *y, u64 row, VT v, bool atomic)
 // (write-out through the multicast address; implies STAGE). B: elements per load batch. BRANCHY: the walk
 // over the row-start flags branches per flagged element instead of running predicated straight-line code.
 template <class VT, class CT, int S, int MODE, int B, bool BRANCHY>
-__global__ void __launch_bounds__(256) k_csr5s(const KArgs a)
+__global__ void __launch_bounds__(256) k_csr5s(KArgs a)
 {
     constexpr bool WARP_FAST = (MODE & 1) != 0, STAGE = (MODE & 2) != 0, PUBLISH = (MODE & 4) != 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    grid_wait();
+    grid_release();
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
     const VT *__restrict__ x = (const VT *)a.x + a.first_col;
@@ -338,7 +328,7 @@ cudaError_t launch_sb(int mode, const KArgs &a, unsigned grid, unsigned block, c
 {
     const size_t smem = (mode & 2) ? (size_t)(block / 32) * a.stage_cap * sizeof(VT) : 0;
 #define ASP_CSR5_MODE(M)                                                       \
-    case M: k_csr5s<VT, CT, S, M, B, BRANCHY><<<grid, block, smem, st>>>(a); break;
+    case M: return launch_pdl(k_csr5s<VT, CT, S, M, B, BRANCHY>, dim3(grid), dim3(block), smem, st, a);
     switch (mode)
     {
         ASP_CSR5_MODE(0)
@@ -350,7 +340,6 @@ cudaError_t launch_sb(int mode, const KArgs &a, unsigned grid, unsigned block, c
     default: return cudaErrorInvalidValue;
     }
 #undef ASP_CSR5_MODE
-    return cudaGetLastError();
 }
 
 template <class VT, class CT, int S>

@@ -14,6 +14,7 @@
 
 #include "kernel_args.h"
 #include "kernels.h"
+#include "launch.h"
 
 namespace asp
 {
@@ -46,7 +47,7 @@ __device__ __forceinline__ void ld_vals(const VT *p, VT (&v)[V])
 
 // offsets are stored biased by the column count (so that they are unsigned): off = stored - n_cols
 template <class VT, int U>
-__global__ void __launch_bounds__(256) k_diag(const KArgs a)
+__global__ void __launch_bounds__(256) k_diag(KArgs a)
 {
     constexpr int V = 16 / sizeof(VT);
     const VT *__restrict__ val = (const VT *)a.val;
@@ -56,58 +57,68 @@ __global__ void __launch_bounds__(256) k_diag(const KArgs a)
     const u64 NR = a.n_tlb;       // padded rows (multiple of V)
     const unsigned D = a.tlb_size; // diagonals
     const i64 rows = (i64)a.effective, ncols = (i64)a.n_units; // rows and columns of the sub-matrix
-    const u64 stride = (u64)gridDim.x * blockDim.x;
-    for (u64 g = (u64)blockIdx.x * blockDim.x + threadIdx.x; g * V < NR; g += stride)
+    // One group of rows per thread (the launch covers them all). The first values are on their way when it waits for the kernel
+    // before; a loop over groups around the same body cost 4 to 10 us of 39 (2048 x 2048 mesh, fp64).
+    const u64 g = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g * V >= NR) return;
+    const i64 r0 = (i64)(g * V);
+    VT acc[V];
+#pragma unroll
+    for (int j = 0; j < V; j++) acc[j] = 0;
+    unsigned d = 0;
+    for (; d + U <= D; d += U)
     {
-        const i64 r0 = (i64)(g * V);
-        VT acc[V];
+        VT v[U][V], xv[U][V];
+        i64 off[U];
 #pragma unroll
-        for (int j = 0; j < V; j++) acc[j] = 0;
-        unsigned d = 0;
-        for (; d + U <= D; d += U)
+        for (int u = 0; u < U; u++) off[u] = (i64)__ldg(offs + d + u) - ncols;
+#pragma unroll
+        for (int u = 0; u < U; u++) ld_vals<VT, V>(val + (u64)(d + u) * NR + (u64)r0, v[u]);
+        if (d == 0)
         {
-            VT v[U][V], xv[U][V];
-            i64 off[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) off[u] = (i64)__ldg(offs + d + u) - ncols;
-#pragma unroll
-            for (int u = 0; u < U; u++) ld_vals<VT, V>(val + (u64)(d + u) * NR + (u64)r0, v[u]);
-#pragma unroll
-            for (int u = 0; u < U; u++)
-#pragma unroll
-                for (int j = 0; j < V; j++)
-                {
-                    const i64 c = r0 + j + off[u];
-                    xv[u][j] = (c >= 0 && c < ncols) ? __ldg(x + c) : VT(0);
-                }
-#pragma unroll
-            for (int u = 0; u < U; u++)
-#pragma unroll
-                for (int j = 0; j < V; j++) acc[j] += v[u][j] * xv[u][j];
+            grid_wait();
+            grid_release();
         }
-        for (; d < D; d++)
-        {
-            VT v[V];
-            const i64 off = (i64)__ldg(offs + d) - ncols;
-            ld_vals<VT, V>(val + (u64)d * NR + (u64)r0, v);
+#pragma unroll
+        for (int u = 0; u < U; u++)
 #pragma unroll
             for (int j = 0; j < V; j++)
             {
-                const i64 c = r0 + j + off;
-                if (c >= 0 && c < ncols) acc[j] += v[j] * __ldg(x + c);
+                const i64 c = r0 + j + off[u];
+                xv[u][j] = (c >= 0 && c < ncols) ? ld_x(x + c) : VT(0);
             }
-        }
-        if (r0 + V <= rows && (((uintptr_t)(y + r0)) & 15) == 0)
-        {
-            if constexpr (sizeof(VT) == 8) *reinterpret_cast<double2 *>(y + r0) = make_double2(acc[0], acc[1]);
-            else *reinterpret_cast<float4 *>(y + r0) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        }
-        else
-        {
 #pragma unroll
-            for (int j = 0; j < V; j++)
-                if (r0 + j < rows) y[r0 + j] = acc[j];
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int j = 0; j < V; j++) acc[j] += v[u][j] * xv[u][j];
+    }
+    if (d == 0)
+    {
+        grid_wait();
+        grid_release();
+    }
+    for (; d < D; d++)
+    {
+        VT v[V];
+        const i64 off = (i64)__ldg(offs + d) - ncols;
+        ld_vals<VT, V>(val + (u64)d * NR + (u64)r0, v);
+#pragma unroll
+        for (int j = 0; j < V; j++)
+        {
+            const i64 c = r0 + j + off;
+            if (c >= 0 && c < ncols) acc[j] += v[j] * ld_x(x + c);
         }
+    }
+    if (r0 + V <= rows && (((uintptr_t)(y + r0)) & 15) == 0)
+    {
+        if constexpr (sizeof(VT) == 8) *reinterpret_cast<double2 *>(y + r0) = make_double2(acc[0], acc[1]);
+        else *reinterpret_cast<float4 *>(y + r0) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    }
+    else
+    {
+#pragma unroll
+        for (int j = 0; j < V; j++)
+            if (r0 + j < rows) y[r0 + j] = acc[j];
     }
 }
 } // namespace
@@ -115,9 +126,7 @@ __global__ void __launch_bounds__(256) k_diag(const KArgs a)
 cudaError_t launch_diag(int val_is_f64, const KArgs &a, unsigned grid, unsigned block, cudaStream_t st)
 {
     if (block > 256) return cudaErrorInvalidValue;
-    if (val_is_f64) k_diag<double, 5><<<grid, block, 0, st>>>(a);
-    else k_diag<float, 5><<<grid, block, 0, st>>>(a);
-    return cudaGetLastError();
+    return val_is_f64 ? launch_pdl(k_diag<double, 5>, dim3(grid), dim3(block), 0, st, a) : launch_pdl(k_diag<float, 5>, dim3(grid), dim3(block), 0, st, a);
 }
 
 } // namespace asp

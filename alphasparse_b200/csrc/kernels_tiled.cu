@@ -17,6 +17,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "kernels.h"
+#include "launch.h"
 #include "tiled.h"
 
 namespace asp
@@ -38,11 +40,6 @@ struct Pair<double>
 {
     typedef double2 type;
 };
-
-// Programmatic dependent launch: `wait` returns when everything before this kernel on its stream has finished;
-// `launch_dependents` lets the next kernel start as soon as there is room for it.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // x may have been written by the kernel before: read through L2, in program order after the wait
 __device__ __forceinline__ uint4 ld_x16(const void *p)
@@ -67,7 +64,7 @@ __device__ __forceinline__ double ld_x1(const double *p)
 template <class VT>
 __global__ void __launch_bounds__(256) k_clear(VT *y, u64 n)
 {
-    grid_launch_dependents();
+    grid_release();
     grid_wait();
     const u64 stride = (u64)gridDim.x * blockDim.x;
     const u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -103,7 +100,7 @@ __device__ __forceinline__ void add_rows(VT *y, u32 row, VT v, u32 lane)
 }
 
 template <class VT, int U>
-__global__ void __launch_bounds__(1024, 1) k_tiled(const TiledArgs a, const u32 tile_cols)
+__global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
 {
     typedef typename Pair<VT>::type P;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -134,7 +131,7 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(const TiledArgs a, const u32 
         if (first)
         {
             // nothing above depends on what ran before
-            grid_launch_dependents();
+            grid_release();
             grid_wait();
             first = false;
         }
@@ -223,38 +220,27 @@ struct Batch<double>
     static const int U = 2;
 };
 
-cudaError_t launch_pdl(const void *f, unsigned grid, unsigned block, size_t smem, cudaStream_t st, void **args)
+template <class VT>
+cudaError_t clear(VT *y, u64 n, unsigned n_sm, cudaStream_t st)
 {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelExC(&cfg, f, args);
+    // a few 16-byte stores per thread
+    const u64 want = (n * sizeof(VT) / 16 + 1023) / 1024;
+    return launch_pdl(k_clear<VT>, dim3((unsigned)(want < 1 ? 1 : want < 4ull * n_sm ? want : 4ull * n_sm)), dim3(256), 0, st, y, n);
 }
 
 template <class VT>
-cudaError_t launch(const TiledArgs &args, unsigned n_sm, cudaStream_t st)
+cudaError_t launch(const TiledArgs &a, unsigned n_sm, cudaStream_t st)
 {
-    TiledArgs a = args;
-    VT *y = (VT *)a.y;
-    u64 n = a.n_rows;
-    void *clear_args[] = {&y, &n};
-    // a few 16-byte stores per thread
-    const u64 want = (n * sizeof(VT) / 16 + 1023) / 1024;
-    const unsigned grid = (unsigned)(want < 1 ? 1 : want < 4ull * n_sm ? want : 4ull * n_sm);
-    cudaError_t e = launch_pdl((const void *)k_clear<VT>, grid, 256, 0, st, clear_args);
+    const cudaError_t e = clear((VT *)a.y, a.n_rows, n_sm, st);
     if (e != cudaSuccess) return e;
-    u32 cols = tiled_tile_cols(sizeof(VT) == 8);
-    void *tiled_args[] = {&a, &cols};
-    return launch_pdl((const void *)k_tiled<VT, Batch<VT>::U>, n_sm, kTiledWarps * 32, kTiledTileBytes, st, tiled_args);
+    return launch_pdl(k_tiled<VT, Batch<VT>::U>, dim3(n_sm), dim3(kTiledWarps * 32), kTiledTileBytes, st, a, (u32)tiled_tile_cols(sizeof(VT) == 8));
 }
 } // namespace
+
+cudaError_t launch_clear(int val_is_f64, void *y, unsigned long long n, unsigned n_sm, cudaStream_t st)
+{
+    return val_is_f64 ? clear((double *)y, n, n_sm, st) : clear((float *)y, n, n_sm, st);
+}
 
 cudaError_t tiled_setup(int val_is_f64)
 {
