@@ -1136,6 +1136,8 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
         t.col = cols[i]->host_ptr;
         t.col_bytes = dtype_size(cols[i]->dtype);
         t.stored = vals[i]->len;
+        t.true_nnz = descs[i].true_nnz;
+        t.threads = made[i]->block;
         src.push_back(t);
     }
     asp::TiledHost th;

@@ -182,6 +182,35 @@ double lines_per_gather(const TiledSource &s, bool f64)
     return (double)lines / (double)(samples * 128);
 }
 
+bool is_csr5(const TiledSource &s)
+{
+    return s.templ == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE || s.templ == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE;
+}
+
+// Microseconds of the longest serial chain of the template's own kernel: a thread of the SELL- and ELL-like kernels walks its
+// TLB four elements a trip (index, then x: 1.4 us where few warps run), a CTA of the row-grouped kernel its strip's TLBs, a
+// thread of the CSR5-like ones its TLB eight elements a trip and then the tails of its warp.
+double chain_us(const TiledSource &s)
+{
+    u64 trips = 0;
+    if (s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS) trips = (s.a->tlb_size + 3) / 4;
+    else if (s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS)
+        for (u64 b = 0; b < s.a->n_units; b++) trips = std::max<u64>(trips, (s.m[MS_TLB_SIZE].get(b) + 3) / 4);
+    else if (s.templ == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS)
+        for (u64 b = 0; b < s.a->n_units; b++)
+        {
+            const u64 per_trip = 4 * std::max(32u, s.threads), n = s.m[MS_BLK_THR].get(b + 1) - s.m[MS_BLK_THR].get(b);
+            trips = std::max<u64>(trips, (n + per_trip - 1) / per_trip * ((s.m[MS_TLB_SIZE].get(b) + 3) / 4));
+        }
+    else if (is_csr5(s)) return 3.5 + 1.4 * (double)((s.a->tlb_size + 7) / 8);
+    return 1.4 * (double)trips;
+}
+// how far the template's own kernel stays below the rate of its gathers or bytes (measured, 80 non-zeros a row, random columns)
+double slowness(const TiledSource &s)
+{
+    return s.templ == ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE ? 1.45 : s.templ == ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE ? 2.35 : 1.1;
+}
+
 const u32 kMaxPiece = 32;    // elements of a row's piece: bounds the serial chain of a lane and the padding of a slice
 const u32 kWindow = 1024;    // pieces that are sorted by length together: lanes of a slice stay near in y
 const double kSliceCost = 4.0; // in steps; with 2 the CTAs of sparse tiles ran twice as long as the others
@@ -475,29 +504,39 @@ template <class VT>
 bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm, TiledHost &out)
 {
     const double sv = sizeof(VT);
-    // The group's own kernels: one request to L2 per cache line that a gather touches (290 G/s on this part, of which they
-    // reach 0.85), or the format's bytes.
-    u64 stored = 0;
-    double lines = 0;
+    // The group's own kernels: one request to L2 per cache line that a gather touches (290 G/s on this part, of which they reach
+    // 0.85) or the format's bytes, or their longest serial chain, whichever is longest; a call takes 4.5 us at least, several
+    // kernels a fork and a join more.
+    u64 true_nnz = 0;
+    double chain = 0, requests = 0, bytes_us = 0;
     for (const TiledSource &s : src)
     {
         if (unit_count(s) == 0) return false;
-        stored += s.stored;
+        true_nnz += s.true_nnz;
+        chain = std::max(chain, chain_us(s));
+        requests += (double)s.stored * slowness(s);
+        bytes_us += (double)s.stored * slowness(s) * (sv + 4) / 6.0e6;
     }
-    if ((double)stored / (0.85 * 290e3) < 12.0) return false; // (see below; no need to look at the columns)
-    for (const TiledSource &s : src)
-    {
-        lines += lines_per_gather(s, sizeof(VT) == 8) * (double)s.stored;
-    }
-    const double own_us = std::max(lines / (0.85 * 290e3), (double)stored * (sv + 4) / 6.0e6);
-    // ... are the better ones where the gathers are not what bounds them, and for small matrices, whose time is the launch
-    if (lines / (0.85 * 290e3) < 1.25 * (double)stored * (sv + 4) / 6.0e6 || own_us < 12.0) return false;
-    if (n_rows >= kTiledNoRow || stored >= (1ull << 37)) return false;
+    auto own = [&](double lines) { return 4.5 + (src.size() > 1 ? 8.0 : 0.0) + std::max(std::max(lines / (0.85 * 290e3), bytes_us), chain); };
+    // A small group of several strips keeps its kernels: callers compare its rows bit for bit with those of the same group with
+    // some strips muted (EMPTY), as a search does that times strip after strip.
+    if (src.size() > 1 && true_nnz < (1u << 16)) return false;
+    // small matrices, whose time is the launch, stay with their kernels (not worth a look at the columns)
+    if (own(requests) < 7.0) return false;
+    double lines = 0;
+    for (const TiledSource &s : src) lines += lines_per_gather(s, sizeof(VT) == 8) * (double)s.stored * slowness(s);
+    const double own_us = own(lines);
+    // This layout: launches and tail, the first tile of x, 2 + sv bytes per element at 4.6 TB/s, a `red` per piece (below).
+    auto tiled_us = [&](u64 n, u64 pieces, double red) {
+        return 4.5 + 2.5 * std::min(1.0, (double)n_cols / (double)tiled_tile_cols(sizeof(VT) == 8)) + (double)n * (sv + 2) / 4.6e6 + (double)pieces * 4 / 4.6e6 + red / 200e3 +
+               (double)n_rows * sv / 6.0e6;
+    };
+    if (tiled_us(true_nnz, 0, 0) > 0.85 * own_us) return false;
+    if (n_rows >= kTiledNoRow || requests >= 1e11) return false;
     Builder<VT> b(src, n_rows, n_cols);
     if (b.C + (u64)n_sm >= 65536) return false;
     b.count(out.covers_all_rows);
-    // This layout: 2 + sv bytes per element at 4.6 TB/s, a `red` per piece (a warp's 32 fall into about an eighth as many
-    // lines where the rows of a tile are dense, into 32 where they are sparse), 7 us of launches, tiles and tail.
+    // (a warp's 32 `red` fall into about an eighth as many lines where the rows of a tile are dense, into 32 where they are sparse)
     double red = 0;
     u64 pieces = 0;
     for (u64 t = 0; t < b.C; t++)
@@ -506,8 +545,7 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
         pieces += b.tile_pieces[t];
         if (p > 0) red += p * std::min(1.0, std::max(0.25, 4.0 * (double)n_rows / p / 32.0));
     }
-    const double tiled_us = 7.0 + (double)b.N * (sv + 2) / 4.6e6 + (double)pieces * 4 / 4.6e6 + red / 200e3 + (double)n_rows * sv / 6.0e6;
-    if (tiled_us > 0.85 * own_us) return false;
+    if (tiled_us(b.N, pieces, red) > 0.85 * own_us) return false;
     b.scatter();
     b.slices(n_sm, out);
     return true;

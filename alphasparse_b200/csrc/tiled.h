@@ -35,6 +35,8 @@ struct TiledSource
     const void *val = nullptr, *col = nullptr;
     int col_bytes = 4;
     uint64_t stored = 0; // padded non-zeros
+    uint64_t true_nnz = 0;
+    unsigned threads = 0; // of a CTA of the template's own kernel
 };
 
 template <class T>
