@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 
 import numpy as np
 
@@ -59,7 +60,7 @@ EXPORTS = [
     "asp_ctx_create", "asp_multicast_store", "asp_spmv_publish", "asp_plan_end_rows", "asp_rank_barrier", "asp_ctx_destroy", "asp_ctx_stream", "asp_plan_group_create", "asp_plan_descs_validate", "asp_plan_destroy",
     "asp_plan_set_launch", "asp_plan_get_launch", "asp_plan_set_tuning", "asp_plan_format_bytes", "asp_plan_launches", "asp_spmv", "asp_spmv_host", "asp_time",
     "asp_synchronize", "asp_status_str", "asp_last_error", "asp_built_for_sm100a", "asp_spmv_host_static",
-    "asp_static_stage_bytes", "asp_search_gpu", "asp_spmv_host_pipelined", "asp_dist_create", "asp_dist_destroy", "asp_dist_spmv", "asp_dist_spmv_iter", "asp_dist_status",
+    "asp_static_stage_bytes", "asp_search_gpu", "asp_spmv_host_pipelined", "asp_dist_create", "asp_dist_destroy", "asp_dist_spmv", "asp_dist_spmv_iter", "asp_dist_status", "asp_plan_layout_bytes", "asp_host_alloc", "asp_host_free",
 ]
 
 _lib = None
@@ -123,6 +124,12 @@ def lib() -> C.CDLL:
     L.asp_plan_set_tuning.restype = C.c_int
     L.asp_plan_format_bytes.argtypes = [C.c_void_p]
     L.asp_plan_format_bytes.restype = C.c_uint64
+    L.asp_plan_layout_bytes.argtypes = [C.c_void_p]
+    L.asp_plan_layout_bytes.restype = C.c_uint64
+    L.asp_host_alloc.argtypes = [C.c_size_t, C.POINTER(C.c_void_p)]
+    L.asp_host_alloc.restype = C.c_int
+    L.asp_host_free.argtypes = [C.c_void_p]
+    L.asp_host_free.restype = None
     L.asp_plan_launches.argtypes = [C.c_void_p]
     L.asp_plan_launches.restype = C.c_int
     L.asp_spmv.argtypes = [C.c_void_p, C.POINTER(C.c_void_p), C.c_int, C.c_void_p, C.c_void_p, C.c_int]
@@ -166,6 +173,67 @@ def check(status: int) -> None:
         raise AspError(status, f"{L.asp_status_str(status).decode()}: {L.asp_last_error().decode()}")
 
 
+class _Lease:
+    """Owner of one buffer of _Results, which gets it back when the last array over it is gone."""
+
+    def __init__(self, pool, ptr, nbytes, n, dtype):
+        self._pool, self._ptr, self._nbytes = pool, ptr, nbytes
+        self.__array_interface__ = {"data": (ptr, False), "shape": (n,), "typestr": dtype.str, "version": 3}
+
+    def __del__(self):
+        try:
+            self._pool._back(self._ptr, self._nbytes)
+        except Exception:  # interpreter shutdown
+            pass
+
+
+class _Results:
+    """Arrays for the results of host calls, in page-locked memory that is used again once nobody holds the array: a fresh
+    pageable array of 8 MB costs more in page faults (0.4 ms and up) than the SpMV and both copies. At most MOST bytes,
+    handed out or idle; beyond that, and for small results, arrays are ordinary ones. Idle buffers go back when a context is
+    closed."""
+
+    SMALL, MOST = 1 << 16, 256 << 20
+
+    def __init__(self):
+        self._lock = threading.RLock()  # (a lease may end inside an allocation of this very thread)
+        self._idle = {}  # bytes -> pointers
+        self._bytes = 0  # of all buffers
+
+    def empty(self, n, dtype):
+        dtype = np.dtype(dtype)
+        nbytes = n * dtype.itemsize
+        if nbytes < self.SMALL or nbytes > self.MOST:
+            return np.empty(n, dtype=dtype)
+        with self._lock:
+            idle = self._idle.get(nbytes)
+            ptr = idle.pop() if idle else None
+            if ptr is None:
+                if self._bytes + nbytes > self.MOST:
+                    self.trim()
+                p = C.c_void_p()
+                if self._bytes + nbytes > self.MOST or lib().asp_host_alloc(nbytes, C.byref(p)) != 0:
+                    return np.empty(n, dtype=dtype)
+                ptr = p.value
+                self._bytes += nbytes
+        return np.asarray(_Lease(self, ptr, nbytes, n, dtype))
+
+    def _back(self, ptr, nbytes):
+        with self._lock:
+            self._idle.setdefault(nbytes, []).append(ptr)
+
+    def trim(self):
+        with self._lock:
+            for nbytes, idle in self._idle.items():
+                for ptr in idle:
+                    lib().asp_host_free(ptr)
+                    self._bytes -= nbytes
+            self._idle = {}
+
+
+_results = _Results()
+
+
 def multicast_store(src_ptr: int, multicast_ptr: int, nbytes: int, stream: int, ctas: int = 0) -> None:
     """asp_multicast_store: one-to-all store of a slice through an NVLink multicast address."""
     check(lib().asp_multicast_store(src_ptr, multicast_ptr, nbytes, stream, ctas))
@@ -197,6 +265,7 @@ class Context:
 
     def close(self):
         if self._h:
+            _results.trim()
             lib().asp_ctx_destroy(self._h)
             self._h = C.c_void_p()
 
@@ -274,6 +343,10 @@ class PlanGroup:
     def format_bytes(self) -> int:
         return sum(lib().asp_plan_format_bytes(self._plans[i]) for i in range(self.n))
 
+    def layout_bytes(self) -> int:
+        """Device memory of the column-tiled layout the group runs, 0 when it runs its templates' own kernels."""
+        return lib().asp_plan_layout_bytes(self._plans[0])
+
     def launches(self) -> int:
         return sum(lib().asp_plan_launches(self._plans[i]) for i in range(self.n))
 
@@ -294,7 +367,7 @@ class PlanGroup:
     def spmv_host(self, x: np.ndarray) -> np.ndarray:
         x = np.ascontiguousarray(x, dtype=self.val_dtype)
         assert x.shape[0] == self.n_cols
-        y = np.empty(self.n_rows, dtype=self.val_dtype)
+        y = _results.empty(self.n_rows, self.val_dtype)
         check(lib().asp_spmv_host(self.ctx.handle, self._plans, self.n, C.c_void_p(x.ctypes.data), C.c_void_p(y.ctypes.data)))
         return y
 

@@ -14,10 +14,10 @@
 #include <vector>
 
 #include "../../include/asp_b200.h"
-#include "host/hostmem.hpp"
 #include "host_meta.h"
 #include "kernel_args.h"
 #include "kernels.h"
+#include "memory.h"
 #include "tiled.h"
 
 namespace
@@ -75,128 +75,24 @@ int dtype_size(int dt)
     }
 }
 
-// device memory shared by the plans of one group (one cudaMalloc per matrix)
+// device memory shared by the plans of one group (one block per matrix)
 struct Arena
 {
     void *base = nullptr;
-    size_t bytes = 0;
+    size_t got = 0;
     int device = 0;
-    ~Arena()
+    cudaError_t make(int dev, size_t bytes)
     {
-        if (base) cudaFree(base);
+        device = dev;
+        const cudaError_t e = asp::device_alloc(dev, bytes, &base, &got);
+        if (e != cudaSuccess) base = nullptr;
+        return e;
     }
+    ~Arena() { asp::device_free(device, base, got); }
 };
 
 using asp::HostMeta;
 
-// Copies between pageable host memory and the device. The runtime moves such a copy through its own pinned buffer with one
-// thread (8 to 12 GB/s measured on this host, page faults of a fresh destination included); here all cores fill or empty a ring
-// of pinned pieces while the copy engine works on the others. Pinned memory is copied directly. 16 MB per context, allocated
-// with the first copy that is worth it, freed with the context.
-struct Stager
-{
-    static const size_t kPiece = 1u << 20;
-    static const int kPieces = 16;
-    unsigned char *ring = nullptr;
-    cudaEvent_t done[kPieces] = {};
-    bool off = false; // no pinned memory to be had: plain copies
-
-    bool ready()
-    {
-        if (ring) return true;
-        if (off) return false;
-        off = true;
-        void *p = nullptr;
-        if (cudaHostAlloc(&p, kPiece * kPieces, cudaHostAllocDefault) != cudaSuccess)
-        {
-            cudaGetLastError();
-            return false;
-        }
-        for (int i = 0; i < kPieces; i++)
-            if (cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming) != cudaSuccess)
-            {
-                cudaGetLastError();
-                for (int j = 0; j < i; j++) cudaEventDestroy(done[j]);
-                cudaFreeHost(p);
-                return false;
-            }
-        ring = (unsigned char *)p;
-        off = false;
-        return true;
-    }
-    void release()
-    {
-        if (!ring) return;
-        for (int i = 0; i < kPieces; i++) cudaEventDestroy(done[i]);
-        cudaFreeHost(ring);
-        ring = nullptr;
-    }
-    // small copies, and memory that the runtime already knows, gain nothing
-    bool direct(const void *host, size_t bytes)
-    {
-        if (bytes < (2u << 20)) return true;
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, host) != cudaSuccess)
-        {
-            cudaGetLastError();
-            return true;
-        }
-        return at.type != cudaMemoryTypeUnregistered || !ready();
-    }
-    // the host buffer may be reused as soon as this returns, as after a pageable cudaMemcpyAsync
-    cudaError_t to_device(void *dev, const void *host, size_t bytes, cudaStream_t st)
-    {
-        if (direct(host, bytes)) return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
-        int i = 0;
-        for (size_t o = 0; o < bytes; o += kPiece, i = (i + 1) % kPieces)
-        {
-            const size_t n = std::min(kPiece, bytes - o);
-            cudaError_t e = cudaEventSynchronize(done[i]); // (an event that was never recorded counts as done)
-            if (e != cudaSuccess) return e;
-            fill(ring + i * kPiece, (const unsigned char *)host + o, n);
-            e = cudaMemcpyAsync((unsigned char *)dev + o, ring + i * kPiece, n, cudaMemcpyHostToDevice, st);
-            if (e == cudaSuccess) e = cudaEventRecord(done[i], st);
-            if (e != cudaSuccess) return e;
-        }
-        return cudaSuccess;
-    }
-    // complete on return
-    cudaError_t to_host(void *host, const void *dev, size_t bytes, cudaStream_t st)
-    {
-        if (direct(host, bytes))
-        {
-            cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
-            return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
-        }
-        const size_t n_pieces = (bytes + kPiece - 1) / kPiece;
-        cudaError_t e = cudaSuccess;
-        auto send = [&](size_t p) { // (earlier users of the slot were on a stream that has been waited for, or on this one)
-            const size_t o = p * kPiece;
-            e = cudaMemcpyAsync(ring + p % kPieces * kPiece, (const unsigned char *)dev + o, std::min(kPiece, bytes - o), cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaEventRecord(done[p % kPieces], st);
-        };
-        for (size_t p = 0; p < n_pieces && p < (size_t)kPieces && e == cudaSuccess; p++) send(p);
-        for (size_t p = 0; p < n_pieces && e == cudaSuccess; p++)
-        {
-            e = cudaEventSynchronize(done[p % kPieces]);
-            if (e != cudaSuccess) break;
-            const size_t o = p * kPiece;
-            fill((unsigned char *)host + o, ring + p % kPieces * kPiece, std::min(kPiece, bytes - o));
-            if (p + kPieces < n_pieces) send(p + kPieces);
-        }
-        if (e != cudaSuccess) cudaStreamSynchronize(st);
-        return e;
-    }
-
-  private:
-    static void fill(unsigned char *dst, const unsigned char *src, size_t n)
-    {
-        const size_t part = 64u << 10;
-        const int parts = (int)((n + part - 1) / part);
-#pragma omp parallel for schedule(static) if (parts > 2)
-        for (int i = 0; i < parts; i++) memcpy(dst + i * part, src + i * part, std::min(part, n - i * part));
-    }
-};
 } // namespace
 
 struct asp_ctx
@@ -217,7 +113,7 @@ struct asp_ctx
     // copy streams and events of the pipelined host SpMV, created on first use
     cudaStream_t h2d = nullptr, d2h = nullptr;
     std::vector<cudaEvent_t> pipe_events;
-    Stager stager;
+    asp::Stager stager;
 };
 
 namespace
@@ -228,6 +124,7 @@ struct TiledGroup
     Arena arena;
     asp::TiledArgs args;
     int n_plans = 0;
+    size_t layout_bytes = 0;
     unsigned n_sm = 0;
     bool covers_all_rows = false; // every row of y has an element in some plan
 };
@@ -251,6 +148,7 @@ struct asp_plan
     uint64_t warp_tasks = 0; // SELL-like with equal strips: warp-sized work items
     uint64_t sell_strip = 0; // SELL-like: TLBs per strip when all strips are equal, else 0
     bool needs_zero = false;
+    bool stores_all_rows = false; // every row of y is stored (not accumulated) by every SpMV: y needs no clearing
     // CSR5-like family: the rows of y that warps accumulate with `red` (first and last row of every warp), as
     // indices into y; kept on the device for the publishing SpMV (asp_spmv_publish)
     std::shared_ptr<Arena> end_rows;
@@ -556,6 +454,24 @@ bool validate_contents(const asp_plan_desc &d, const std::vector<HostMeta> &hm, 
     }
 }
 
+// whether the kernel of a (validated) plan stores every row of y
+bool stores_every_row(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const asp::KArgs &a)
+{
+    using namespace asp;
+    if (a.atomic || d.first_row != 0 || d.sort_kind != ASP_SORT_NONE) return false;
+    const HostMeta &rt = hm[MS_ROW_OF_TLB], &bt = hm[MS_BLK_THR], &br = hm[MS_BLK_ROW];
+    const bool identity = rt.kind == ASP_COMPRESS_LINEAR && rt.coef == 1 && rt.icpt == 0;
+    switch (d.template_type)
+    {
+    case ASP_BLOCK_ELL_TEMPLATE:
+    case ASP_DIAG_TEMPLATE: return a.effective >= d.n_rows;
+    case ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS: return identity && a.effective >= d.n_rows;
+    case ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS: return identity && a.effective >= d.n_rows && bt.get(0) == 0 && bt.get(a.n_units) >= d.n_rows;
+    case ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS: return a.effective >= d.n_rows && br.get(0) == 0 && br.get(a.n_units) >= d.n_rows;
+    default: return false;
+    }
+}
+
 asp_status ensure_xy(asp_ctx *ctx, size_t xb, size_t yb)
 {
     if (ctx->x_bytes < xb)
@@ -619,6 +535,7 @@ asp_status asp_ctx_create(int device, asp_ctx **out)
     asp_ctx *c = new (std::nothrow) asp_ctx();
     if (!c) return fail(ASP_ERR_ALLOC, "host allocation failed");
     c->device = device;
+    asp::device_pool_retain(device);
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
@@ -661,6 +578,7 @@ void asp_ctx_destroy(asp_ctx *c)
     if (c->h2d) cudaStreamDestroy(c->h2d);
     if (c->d2h) cudaStreamDestroy(c->d2h);
     if (c->stream) cudaStreamDestroy(c->stream);
+    asp::device_pool_release(c->device);
     delete c;
 }
 
@@ -767,21 +685,22 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
 
     std::shared_ptr<Arena> arena(new (std::nothrow) Arena());
     if (!arena) return fail(ASP_ERR_ALLOC, "host allocation failed");
-    arena->device = dry ? 0 : ctx->device;
-    arena->bytes = std::max<size_t>(total, 256);
     if (!dry)
     {
-        cudaError_t e = cudaMalloc(&arena->base, arena->bytes);
+        cudaError_t e = arena->make(ctx->device, std::max<size_t>(total, 256));
         if (e != cudaSuccess)
         {
-            arena->base = nullptr;
             cudaGetLastError();
             return fail(ASP_ERR_ALLOC, std::string("cudaMalloc of the plan arena failed: ") + cudaGetErrorString(e));
         }
     }
     if (!dry)
-        for (auto &kv : placed)
-            ASP_CUDA(ctx->stager.to_device((char *)arena->base + kv.second.off, kv.first, kv.second.bytes, ctx->stream));
+    {
+        std::vector<asp::Stager::Segment> seg;
+        for (auto &kv : placed) seg.push_back({kv.second.off, kv.first, kv.second.bytes});
+        std::sort(seg.begin(), seg.end(), [](const asp::Stager::Segment &x, const asp::Stager::Segment &y) { return x.off < y.off; });
+        ASP_CUDA(ctx->stager.to_device(arena->base, seg, ctx->stream));
+    }
 
     // ---- pass 2: build the kernel arguments
     auto dev_meta = [&](const HostMeta &h) {
@@ -1034,14 +953,13 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
                 }
                 rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
                 std::shared_ptr<Arena> er(new (std::nothrow) Arena());
-                if (!er || cudaMalloc(&er->base, std::max<size_t>(rows.size() * 4, 4)) != cudaSuccess)
+                if (!er || er->make(ctx->device, std::max<size_t>(rows.size() * 4, 4)) != cudaSuccess)
                 {
                     cudaGetLastError();
                     cleanup();
                     return fail(ASP_ERR_ALLOC, "allocation of the end-row list failed");
                 }
-                er->device = ctx->device;
-                cudaError_t ce = cudaMemcpy(er->base, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice);
+                cudaError_t ce = ctx->stager.to_device(er->base, rows.data(), rows.size() * 4, ctx->stream);
                 if (ce != cudaSuccess)
                 {
                     cleanup();
@@ -1105,6 +1023,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
                 return cuda_fail(e, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
             }
         }
+        p->stores_all_rows = stores_every_row(d, hm, a);
         p->needs_zero = a.atomic != 0 || d.template_type == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE ||
                         d.template_type == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE;
         st = apply_launch(ctx, p, d.tblock_num, d.thread_num_in_block > 0 ? d.thread_num_in_block : 256, d.thread_num_of_row_reduce);
@@ -1155,24 +1074,25 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
         const size_t bytes[5] = {th.val.bytes(), th.col.bytes(), th.row.bytes(), th.end.bytes(), th.work.size() * sizeof(uint32_t)};
         size_t off[6] = {0};
         for (int k = 0; k < 5; k++) off[k + 1] = align_up(off[k] + bytes[k], 256);
-        tg->arena.device = ctx->device;
-        tg->arena.bytes = off[5];
-        if (cudaMalloc(&tg->arena.base, off[5]) != cudaSuccess)
+        if (tg->arena.make(ctx->device, off[5]) != cudaSuccess)
         {
             cudaGetLastError(); // no room on the device: as above
-            tg->arena.base = nullptr;
             tg.reset();
         }
         else
         {
             unsigned char *base = (unsigned char *)tg->arena.base;
+            std::vector<asp::Stager::Segment> seg;
+            for (int k = 0; k < 5; k++)
+                if (bytes[k]) seg.push_back({off[k], from[k], bytes[k]});
             cudaError_t ce = asp::tiled_setup(descs[0].val_dtype == ASP_F64);
-            for (int k = 0; k < 5 && ce == cudaSuccess; k++) ce = ctx->stager.to_device(base + off[k], from[k], bytes[k], ctx->stream);
+            if (ce == cudaSuccess) ce = ctx->stager.to_device(base, seg, ctx->stream);
             if (ce != cudaSuccess)
             {
                 cleanup();
                 return cuda_fail(ce, "upload of the column-tiled layout");
             }
+            tg->layout_bytes = off[5];
             tg->args = {base + off[0], (const uint16_t *)(base + off[1]), (const uint32_t *)(base + off[2]), (const uint32_t *)(base + off[3]),
                         (const uint4 *)(base + off[4]), nullptr, nullptr, descs[0].n_rows, descs[0].n_cols};
             tg->n_plans = n;
@@ -1271,6 +1191,20 @@ asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path)
     return ASP_OK;
 }
 
+uint64_t asp_plan_layout_bytes(const asp_plan *plan) { return plan && plan->tiled ? plan->tiled->layout_bytes : 0; }
+
+asp_status asp_host_alloc(size_t bytes, void **out)
+{
+    if (!out || bytes == 0) return fail(ASP_ERR_INVALID_ARG, "out is NULL or bytes == 0");
+    *out = nullptr;
+    ASP_CUDA(cudaHostAlloc(out, bytes, cudaHostAllocPortable));
+    return ASP_OK;
+}
+void asp_host_free(void *p)
+{
+    if (p) cudaFreeHost(p);
+}
+
 uint64_t asp_plan_format_bytes(const asp_plan *plan) { return plan ? plan->fmt_bytes : 0; }
 int asp_plan_launches(const asp_plan *plan) { return (plan && plan->templ != ASP_EMPTY_TEMPLATE) ? 1 : 0; }
 uint64_t asp_plan_end_rows(const asp_plan *plan) { return plan ? plan->n_end_rows : 0; }
@@ -1341,7 +1275,7 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
             return ASP_OK;
         }
     }
-    if (clear) ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
+    if (clear && !(n_plans == 1 && plans[0]->stores_all_rows)) ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
     if (!g.first) return ASP_OK;
     int active = 0;
     for (int i = 0; i < n_plans; i++) active += plans[i]->templ != ASP_EMPTY_TEMPLATE;

@@ -48,16 +48,23 @@ const TemplateArray *TemplateData::find(int role) const
 // ---------------------------------------------------------------------------------------------
 // input
 // ---------------------------------------------------------------------------------------------
-std::unique_ptr<Matrix> matrix_from_csr(u64 n_rows, u64 n_cols, const int64_t *indptr, const u32 *indices, const void *values, int val_dt)
+std::unique_ptr<Matrix> matrix_from_csr(u64 n_rows, u64 n_cols, const int64_t *indptr, const u32 *indices, const void *values, int val_dt, bool borrow)
 {
     std::unique_ptr<Matrix> m(new Matrix());
     m->n_rows = n_rows;
     m->n_cols = n_cols;
     m->nnz = (u64)indptr[n_rows];
     m->val_dt = val_dt;
+    m->val.es = dtype_bytes(val_dt);
+    if (borrow)
+    {
+        m->rowptr.borrow((const u64 *)indptr, n_rows + 1);
+        m->col.borrow(indices, m->nnz);
+        m->val.b.borrow((const uint8_t *)values, m->nnz * m->val.es);
+        return m;
+    }
     m->rowptr.assign((const u64 *)indptr, n_rows + 1);
     m->col.assign(indices, m->nnz);
-    m->val.es = dtype_bytes(val_dt);
     m->val.b.assign((const uint8_t *)values, m->nnz * m->val.es);
     return m;
 }

@@ -245,7 +245,7 @@ extern "C" {
 
 const char *asp_host_last_error(void) { return g_host_error.c_str(); }
 
-asp_status asp_matrix_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t *indptr, const uint32_t *indices, const void *values, int val_dtype, asp_matrix **out)
+static asp_status make_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t *indptr, const uint32_t *indices, const void *values, int val_dtype, bool borrow, asp_matrix **out)
 {
     if (!out || !indptr || (!indices && indptr[n_rows] > 0) || (!values && indptr[n_rows] > 0)) return hfail(ASP_ERR_INVALID_ARG, "NULL argument");
     *out = nullptr;
@@ -286,7 +286,7 @@ asp_status asp_matrix_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t *
     if (!h) return hfail(ASP_ERR_ALLOC, "host allocation failed");
     try
     {
-        h->m = matrix_from_csr(n_rows, n_cols, indptr, indices, values, val_dtype);
+        h->m = matrix_from_csr(n_rows, n_cols, indptr, indices, values, val_dtype, borrow);
     }
     catch (const std::bad_alloc &)
     {
@@ -295,6 +295,16 @@ asp_status asp_matrix_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t *
     }
     *out = h;
     return ASP_OK;
+}
+
+asp_status asp_matrix_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t *indptr, const uint32_t *indices, const void *values, int val_dtype, asp_matrix **out)
+{
+    return make_from_csr(n_rows, n_cols, indptr, indices, values, val_dtype, false, out);
+}
+
+asp_status asp_matrix_view_csr(uint64_t n_rows, uint64_t n_cols, const int64_t *indptr, const uint32_t *indices, const void *values, int val_dtype, asp_matrix **out)
+{
+    return make_from_csr(n_rows, n_cols, indptr, indices, values, val_dtype, true, out);
 }
 
 asp_status asp_matrix_from_coo_file(const char *path, int val_dtype, asp_matrix **out)
@@ -565,9 +575,12 @@ asp_status asp_graph_execute(const asp_matrix *in, const char *spec, asp_format 
             b.col.clear();
             b.val.b.clear();
             b.tlb_row.clear();
+            b.rowptr.clear(); // (a view of the input's, which need not outlive this call)
         }
         F->build_descs();
         F->cache_from_matrix();
+        m.rowptr.clear();
+        for (CompressedBlock &b : m.blocks) b.rowptr.clear(), b.col.clear(), b.val.b.clear();
         *out = F.release();
     }
     catch (const std::bad_alloc &)

@@ -103,6 +103,13 @@ class Arr
         make(count);
         par_copy(p, src, count * sizeof(T));
     }
+    // somebody else's memory, which has to stay as it is while this array or a view of it lives
+    void borrow(const T *src, uint64_t count)
+    {
+        s = std::shared_ptr<void>();
+        p = const_cast<T *>(src); // (never written: who writes makes a buffer of its own first)
+        n = count;
+    }
     Arr view(uint64_t off, uint64_t count) const
     {
         Arr a;

@@ -883,13 +883,21 @@ bool init_block_ell(const Matrix &m, const CompressedBlock &b, TemplateData &t, 
     const int es = b.val.es;
     Arr<uint8_t> idx, val;
     u32 *const ip = (u32 *)idx.make_zero(NB * W * 4);
-    uint8_t *const vp = val.make_zero(stored * (u64)es);
+    uint8_t *const vp = val.make(stored * (u64)es);
+    for (u64 q = 0; NB > NBR && q < W * r * c; q++) memset(vp + (q * NB + NBR) * es, 0, es); // the block row that pads
 #pragma omp parallel for schedule(static) if (b.nnz() > kParallelNnz)
     for (int64_t br = 0; br < (int64_t)NBR; br++)
     {
         const u64 n = cnt[br];
         const u32 *bc = bcol + b.rowptr[(u64)br * r];
         for (u64 k = 0; k < W; k++) ip[k * NB + br] = k < n ? bc[k] : (n ? bc[n - 1] : 0); // zero blocks repeat the last block column
+        // a block row of full blocks is overwritten whole (no column twice: entries are as many as there are places)
+        const u64 q0 = b.rowptr[(u64)br * r], q1 = b.rowptr[std::min<u64>(b.n_rows, ((u64)br + 1) * r)];
+        bool full = q1 - q0 == W * r * c;
+        for (u64 row = (u64)br * r; full && row < ((u64)br + 1) * r; row++)
+            for (u64 q = b.rowptr[row] + 1; q < b.rowptr[row + 1]; q++) full = full && b.col[q] != b.col[q - 1];
+        if (!full)
+            for (u64 q = 0; q < W * r * c; q++) memset(vp + (q * NB + (u64)br) * es, 0, es);
         for (u64 row = (u64)br * r; row < std::min<u64>(b.n_rows, ((u64)br + 1) * r); row++)
         {
             const u64 i = row - (u64)br * r;

@@ -1,0 +1,266 @@
+#include "memory.h"
+
+#include <string.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+
+namespace asp
+{
+namespace
+{
+const size_t kMostBlock = 256u << 20, kMostCached = 1u << 30;
+
+struct Pool
+{
+    std::mutex lock;
+    std::multimap<size_t, void *> idle; // by size
+    size_t cached = 0;
+    int contexts = 0;
+};
+const int kMaxDevices = 64;
+// (never destroyed: plans may be freed while the process ends)
+Pool &pool(int device)
+{
+    static Pool *p = new Pool[kMaxDevices];
+    return p[device < 0 || device >= kMaxDevices ? 0 : device];
+}
+
+struct OnDevice
+{
+    int prev = -1;
+    explicit OnDevice(int device)
+    {
+        if (cudaGetDevice(&prev) != cudaSuccess || prev == device) prev = -1;
+        else cudaSetDevice(device);
+    }
+    ~OnDevice()
+    {
+        if (prev >= 0) cudaSetDevice(prev);
+    }
+};
+
+std::vector<void *> take_all(Pool &p)
+{
+    std::vector<void *> out;
+    for (auto &b : p.idle) out.push_back(b.second);
+    p.idle.clear();
+    p.cached = 0;
+    return out;
+}
+
+// dst[0, n) from the segments, dst standing for offset `at` of their block
+void gather(unsigned char *dst, size_t at, size_t n, const std::vector<Stager::Segment> &seg)
+{
+    size_t i = (size_t)(std::upper_bound(seg.begin(), seg.end(), at, [](size_t o, const Stager::Segment &s) { return o < s.off; }) - seg.begin());
+    if (i > 0) i--;
+    for (; i < seg.size() && seg[i].off < at + n; i++)
+    {
+        const size_t lo = std::max(at, seg[i].off), hi = std::min(at + n, seg[i].off + seg[i].bytes);
+        if (lo < hi) memcpy(dst + (lo - at), (const unsigned char *)seg[i].host + (lo - seg[i].off), hi - lo);
+    }
+}
+
+const size_t kPart = 64u << 10; // what one thread copies at a time
+// a copy of fewer parts is over before the threads are awake
+template <class F>
+void parts(size_t n, F &&f)
+{
+    const long long k = (long long)((n + kPart - 1) / kPart);
+#pragma omp parallel for schedule(static) if (k > 3)
+    for (long long i = 0; i < k; i++) f((size_t)i * kPart, std::min(kPart, n - (size_t)i * kPart));
+}
+} // namespace
+
+cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got)
+{
+    const size_t unit = bytes < (1u << 20) ? (64u << 10) : (2u << 20);
+    const size_t want = (std::max<size_t>(bytes, 1) + unit - 1) / unit * unit;
+    Pool &p = pool(device);
+    {
+        std::lock_guard<std::mutex> g(p.lock);
+        auto it = p.idle.lower_bound(want);
+        if (it != p.idle.end() && it->first <= want + want / 4 + unit)
+        {
+            *out = it->second;
+            *got = it->first;
+            p.cached -= it->first;
+            p.idle.erase(it);
+            return cudaSuccess;
+        }
+    }
+    OnDevice on(device);
+    cudaError_t e = cudaMalloc(out, want);
+    if (e == cudaErrorMemoryAllocation)
+    {
+        cudaGetLastError();
+        std::vector<void *> idle;
+        {
+            std::lock_guard<std::mutex> g(p.lock);
+            idle = take_all(p);
+        }
+        for (void *q : idle) cudaFree(q);
+        e = cudaMalloc(out, want);
+    }
+    *got = want;
+    return e;
+}
+
+void device_free(int device, void *ptr, size_t got)
+{
+    if (!ptr) return;
+    OnDevice on(device);
+    Pool &p = pool(device);
+    if (got <= kMostBlock && cudaDeviceSynchronize() == cudaSuccess)
+    {
+        std::lock_guard<std::mutex> g(p.lock);
+        if (p.contexts > 0 && p.cached + got <= kMostCached)
+        {
+            p.idle.insert({got, ptr});
+            p.cached += got;
+            return;
+        }
+    }
+    cudaFree(ptr);
+}
+
+void device_pool_retain(int device)
+{
+    Pool &p = pool(device);
+    std::lock_guard<std::mutex> g(p.lock);
+    p.contexts++;
+}
+
+void device_pool_release(int device)
+{
+    Pool &p = pool(device);
+    std::vector<void *> idle;
+    {
+        std::lock_guard<std::mutex> g(p.lock);
+        if (--p.contexts > 0) return;
+        idle = take_all(p);
+    }
+    OnDevice on(device);
+    for (void *q : idle) cudaFree(q);
+}
+
+bool Stager::ready()
+{
+    if (ring) return true;
+    if (off) return false;
+    off = true;
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, kPiece * kPieces, cudaHostAllocDefault) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return false;
+    }
+    for (int i = 0; i < kPieces; i++)
+        if (cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming) != cudaSuccess)
+        {
+            cudaGetLastError();
+            for (int j = 0; j < i; j++) cudaEventDestroy(done[j]);
+            cudaFreeHost(p);
+            return false;
+        }
+    ring = (unsigned char *)p;
+    off = false;
+    return true;
+}
+
+void Stager::release()
+{
+    if (!ring) return;
+    for (int i = 0; i < kPieces; i++) cudaEventDestroy(done[i]);
+    cudaFreeHost(ring);
+    ring = nullptr;
+}
+
+bool Stager::pinned(const void *host)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return true; // whatever it is, the runtime's own copy knows best
+    }
+    return at.type != cudaMemoryTypeUnregistered;
+}
+
+cudaError_t Stager::slot(unsigned char **p, int *i)
+{
+    *i = next;
+    next = (next + 1) % kPieces;
+    *p = ring + (size_t)*i * kPiece;
+    return cudaEventSynchronize(done[*i]); // (an event that was never recorded counts as done)
+}
+
+cudaError_t Stager::to_device(void *dev, const void *host, size_t bytes, cudaStream_t st)
+{
+    if (bytes < (64u << 10) || pinned(host)) return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
+    return to_device(dev, std::vector<Segment>(1, Segment{0, host, bytes}), st);
+}
+
+cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaStream_t st)
+{
+    if (seg.empty()) return cudaSuccess;
+    if (!ready())
+    {
+        for (const Segment &s : seg)
+        {
+            const cudaError_t e = cudaMemcpyAsync((unsigned char *)dev + s.off, s.host, s.bytes, cudaMemcpyHostToDevice, st);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+    const size_t end = seg.back().off + seg.back().bytes;
+    // about eight pieces: the first one's filling and the last one's copy are all that does not overlap
+    const size_t piece = std::min(kPiece, std::max<size_t>(256u << 10, (end / 8 + kPart - 1) / kPart * kPart));
+    for (size_t o = seg.front().off; o < end; o += piece)
+    {
+        const size_t n = std::min(piece, end - o);
+        unsigned char *p;
+        int i;
+        cudaError_t e = slot(&p, &i);
+        if (e != cudaSuccess) return e;
+        parts(n, [&](size_t at, size_t k) { gather(p + at, o + at, k, seg); });
+        e = cudaMemcpyAsync((unsigned char *)dev + o, p, n, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaEventRecord(done[i], st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t Stager::to_host(void *host, const void *dev, size_t bytes, cudaStream_t st)
+{
+    if (bytes < (256u << 10) || pinned(host) || !ready())
+    {
+        const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
+        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+    }
+    const size_t piece = std::min(kPiece, std::max<size_t>(256u << 10, (bytes / 8 + kPart - 1) / kPart * kPart)), n_pieces = (bytes + piece - 1) / piece;
+    cudaError_t e = cudaSuccess;
+    int at[kPieces];
+    auto send = [&](size_t k) {
+        unsigned char *p;
+        e = slot(&p, &at[k % kPieces]);
+        const size_t o = k * piece;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(p, (const unsigned char *)dev + o, std::min(piece, bytes - o), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaEventRecord(done[at[k % kPieces]], st);
+    };
+    for (size_t k = 0; k < n_pieces && k < (size_t)kPieces && e == cudaSuccess; k++) send(k);
+    for (size_t k = 0; k < n_pieces && e == cudaSuccess; k++)
+    {
+        const int i = at[k % kPieces];
+        e = cudaEventSynchronize(done[i]);
+        if (e != cudaSuccess) break;
+        const size_t o = k * piece;
+        const unsigned char *p = ring + (size_t)i * kPiece;
+        parts(std::min(piece, bytes - o), [&](size_t a, size_t n) { memcpy((unsigned char *)host + o + a, p + a, n); });
+        if (k + kPieces < n_pieces) send(k + kPieces);
+    }
+    if (e != cudaSuccess) cudaStreamSynchronize(st);
+    return e;
+}
+} // namespace asp

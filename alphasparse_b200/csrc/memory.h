@@ -1,0 +1,55 @@
+// Device memory of plans and copies from and to host memory.
+#ifndef ASP_MEMORY_H
+#define ASP_MEMORY_H
+
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+#include <vector>
+
+namespace asp
+{
+// Device memory for plans. cudaMalloc and cudaFree of a plan's arena take one to three milliseconds each on this part, more than
+// everything else that makes a small plan; freed arenas are therefore kept for the next plan: blocks of at most 256 MB, 1 GB in
+// all per device, given back when the last context of the device is destroyed or an allocation fails. Safe from several threads.
+// device_free() waits for the device first, as cudaFree does: kernels in flight may still read the block.
+cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got);
+void device_free(int device, void *p, size_t got);
+void device_pool_retain(int device);  // a context was created ...
+void device_pool_release(int device); // ... or destroyed
+
+// Copies between pageable host memory and the device. The runtime moves such a copy through its own pinned buffer with one
+// thread (8 to 12 GB/s measured, page faults of a fresh destination included); here all cores fill or empty a ring of pinned
+// pieces while the copy engine works on the others. Pinned memory is copied directly. 16 MB per context, allocated with the
+// first copy that is worth it, freed with the context.
+class Stager
+{
+    static const size_t kPiece = 1u << 20;
+    static const int kPieces = 16;
+    unsigned char *ring = nullptr;
+    cudaEvent_t done[kPieces] = {};
+    bool off = false; // no pinned memory to be had: plain copies
+    int next = 0;
+
+    bool ready();
+    bool pinned(const void *host);
+    // the slot the next piece goes through, free to be written
+    cudaError_t slot(unsigned char **p, int *i);
+
+  public:
+    struct Segment
+    {
+        size_t off;
+        const void *host;
+        size_t bytes;
+    };
+    void release();
+    // host buffers may be reused as soon as these return, as after a pageable cudaMemcpyAsync
+    cudaError_t to_device(void *dev, const void *host, size_t bytes, cudaStream_t st);
+    // many arrays of one device block (ascending offsets): as few copies as the pieces make
+    cudaError_t to_device(void *dev, const std::vector<Segment> &segments, cudaStream_t st);
+    // complete on return
+    cudaError_t to_host(void *host, const void *dev, size_t bytes, cudaStream_t st);
+};
+} // namespace asp
+#endif

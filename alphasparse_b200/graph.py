@@ -19,7 +19,7 @@ class SubInfo(C.Structure):
 
 
 HOST_EXPORTS = [
-    "asp_matrix_from_csr", "asp_matrix_from_coo_file", "asp_matrix_destroy", "asp_matrix_rows", "asp_matrix_cols",
+    "asp_matrix_from_csr", "asp_matrix_view_csr", "asp_matrix_from_coo_file", "asp_matrix_destroy", "asp_matrix_rows", "asp_matrix_cols",
     "asp_matrix_nnz", "asp_graph_execute", "asp_format_destroy", "asp_format_num_subs", "asp_format_global_perm",
     "asp_format_sub_info", "asp_format_plan_descs", "asp_format_padding_rate", "asp_host_last_error",
     "asp_dense_execute", "asp_matrix_num_subs", "asp_matrix_sub_rows", "asp_partition_rows_by_nnz", "asp_matrix_relabel_by_column_count", "asp_format_id", "asp_format_save", "asp_format_load",
@@ -48,6 +48,8 @@ def _lib():
     if not _bound:
         L.asp_matrix_from_csr.argtypes = [C.c_uint64, C.c_uint64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.POINTER(C.c_void_p)]
         L.asp_matrix_from_csr.restype = C.c_int
+        L.asp_matrix_view_csr.argtypes = L.asp_matrix_from_csr.argtypes
+        L.asp_matrix_view_csr.restype = C.c_int
         L.asp_matrix_from_coo_file.argtypes = [C.c_char_p, C.c_int, C.POINTER(C.c_void_p)]
         L.asp_matrix_from_coo_file.restype = C.c_int
         L.asp_matrix_destroy.argtypes = [C.c_void_p]
@@ -136,8 +138,9 @@ def partition_rows_by_nnz(indptr: np.ndarray, parts: int) -> np.ndarray:
 class Matrix:
     """asp_matrix: the input of an Operator Graph (BEGIN_MEMORY_CACHE_INPUT_FILE / BEGIN_INPUT_FILE)."""
 
-    def __init__(self, handle):
+    def __init__(self, handle, keep=None):
         self._h = handle
+        self._keep = keep  # arrays that the handle only refers to
 
     @staticmethod
     def from_csr(m: CsrMatrix) -> "Matrix":
@@ -148,6 +151,17 @@ class Matrix:
         _check(_lib().asp_matrix_from_csr(m.n_rows, m.n_cols, indptr.ctypes.data, idx.ctypes.data, vals.ctypes.data,
                                           capi.DTYPE_OF_NP[vals.dtype], C.byref(h)))
         return Matrix(h)
+
+    @staticmethod
+    def view_csr(m: CsrMatrix) -> "Matrix":
+        """from_csr without a copy: `m`'s arrays must not change while this matrix, or one that dense() made from it, lives."""
+        indptr = np.ascontiguousarray(m.indptr, dtype=np.int64)
+        idx = np.ascontiguousarray(m.indices, dtype=np.uint32)
+        vals = np.ascontiguousarray(m.values)
+        h = C.c_void_p()
+        _check(_lib().asp_matrix_view_csr(m.n_rows, m.n_cols, indptr.ctypes.data, idx.ctypes.data, vals.ctypes.data,
+                                          capi.DTYPE_OF_NP[vals.dtype], C.byref(h)))
+        return Matrix(h, (indptr, idx, vals))
 
     @staticmethod
     def from_coo_file(path: str, dtype=np.float32) -> "Matrix":
@@ -178,7 +192,7 @@ class Matrix:
         repeatedly with execute() on `sub ...` lines."""
         h = C.c_void_p()
         _check(_lib().asp_dense_execute(self._h, dense_spec.encode(), C.byref(h)))
-        return Matrix(h)
+        return Matrix(h, self._keep)
 
     @property
     def n_subs(self) -> int:

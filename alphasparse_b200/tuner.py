@@ -167,7 +167,7 @@ def search_with_timer(m: CsrMatrix, time_fn, quick: bool = True, warmup: int = 2
 
 def build(ctx: capi.Context, m: CsrMatrix, desc: dict):
     """Lower and upload exactly the graph a previous search() described (no timing)."""
-    hm = Matrix.from_csr(m)
+    hm = Matrix.view_csr(m)
     cm = hm.dense(desc["dense"].replace(" | ", "\n"))
     if cm.n_subs != len(desc["subs"]):
         raise ValueError(f"graph describes {len(desc['subs'])} sub-matrices, the dense view gives {cm.n_subs}")

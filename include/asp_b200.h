@@ -13,6 +13,7 @@
 #ifndef ASP_B200_H
 #define ASP_B200_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -178,6 +179,8 @@ void *asp_ctx_stream(asp_ctx *ctx);
  * Every entry point makes the context's device current for its own duration and restores the
  * caller's device before it returns. */
 asp_status asp_plan_group_create(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp_plan **out_plans);
+/* (The device memory of destroyed plans is kept for the next ones: blocks of at most 256 MB, 1 GB per device, given back when
+ * the device's last context is destroyed or an allocation fails.) */
 void asp_plan_destroy(asp_plan *plan);
 /* The validation of asp_plan_group_create on its own: same checks, same status and message, no device
  * needed, nothing allocated or uploaded. For a caller that wants to vet template arrays (a loaded
@@ -211,6 +214,9 @@ asp_status asp_plan_get_launch(const asp_plan *plan, int64_t *tblock_num, int64_
 asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path);
 /* bytes of device memory the plan's format arrays occupy (B_fmt without x and y) */
 uint64_t asp_plan_format_bytes(const asp_plan *plan);
+/* bytes of device memory of the column-tiled layout that the plan's group runs (see asp_plan_group_create), beside the format
+ * arrays; 0 when the group runs its templates' own kernels */
+uint64_t asp_plan_layout_bytes(const asp_plan *plan);
 /* number of kernel launches one asp_spmv over this plan issues (excluding the y clear) */
 int asp_plan_launches(const asp_plan *plan);
 
@@ -244,6 +250,11 @@ typedef struct
     uint64_t col_hi;         /* every column these rows read is < col_hi */
 } asp_host_chunk;
 asp_status asp_spmv_host_pipelined(asp_ctx *ctx, const asp_host_chunk *chunks, int n_chunks, const void *h_x, void *h_y);
+
+/* Page-locked host memory for the x and y of the host calls: the copy engine reads and writes it directly, while pageable
+ * memory goes through a pinned ring of the library. Valid for every device; freed with asp_host_free. */
+asp_status asp_host_alloc(size_t bytes, void **out);
+void asp_host_free(void *p);
 
 /* No counterpart in the reference. asp_spmv_host for callers that must not trigger a device
  * allocation (a solver whose own pool owns all device memory; a loop that cannot afford the

@@ -22,6 +22,9 @@ typedef struct asp_format asp_format; /* code_builder_t: one template per sub-ma
  * sorted by row then column. indptr has n_rows + 1 entries; values are f32 or f64. */
 asp_status asp_matrix_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t *indptr, const uint32_t *indices,
                                const void *values, int val_dtype, asp_matrix **out);
+/* The same without a copy: the three arrays belong to the caller and must stay unchanged until the matrix, and what
+ * asp_dense_execute made from it, is destroyed. Formats (asp_graph_execute) hold copies of what they need. */
+asp_status asp_matrix_view_csr(uint64_t n_rows, uint64_t n_cols, const int64_t *indptr, const uint32_t *indices, const void *values, int val_dtype, asp_matrix **out);
 /* BEGIN_INPUT_FILE node: the `.mtx.coo` text format (struct.cc:92-174) */
 asp_status asp_matrix_from_coo_file(const char *path, int val_dtype, asp_matrix **out);
 void asp_matrix_destroy(asp_matrix *m);

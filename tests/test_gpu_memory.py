@@ -1,0 +1,69 @@
+"""GPU: results in recycled page-locked memory, device memory of plans used again, and SpMVs that leave the clearing of y out
+because the kernel stores every row."""
+import numpy as np
+import pytest
+
+import refdump
+from alphasparse_b200 import matrices as M, tuner
+
+pytestmark = pytest.mark.gpu
+
+
+def desc(template, nodes, dense="dense compress"):
+    return {"dense": dense, "subs": [{"graph": template, "nodes": nodes, "template": template, "threads": 128, "row_reduce": 1}]}
+
+
+def test_results_that_are_held_keep_their_values(asp_ctx):
+    m, x = M.laplacian_2d(200, 1, grid_y=150)  # 240 KB of y: page-locked
+    fmt, g = tuner.build(asp_ctx, m, desc("D1", ["diag_value 64"]))
+    y_ref, scale = refdump.csr_ref(m, x)
+    held = [g.spmv_host(x * k) for k in range(4)]
+    view = held[2][10:20]
+    del held[2]  # its buffer lives on in the view
+    later = [g.spmv_host(x * k) for k in range(5, 9)]
+    for k, y in zip((0, 1, 3, 5, 6, 7, 8), held + later):
+        refdump.assert_y(y, k * y_ref, np.maximum(k, 1) * scale, m.values.dtype, f"{k} x")
+    assert np.allclose(view, 2 * y_ref[10:20])
+    g.close()
+    fmt.close()
+
+
+def test_plans_made_and_destroyed_in_turn(asp_ctx):
+    kept = []
+    for k, n in enumerate((40, 300, 41, 300, 1000, 299, 300)):  # blocks of freed plans are taken by others, of about their size
+        m, x = M.laplacian_2d(n, k, grid_y=50, dtype=np.float32)
+        fmt, g = tuner.build(asp_ctx, m, desc("K3", ["row_padding 32 1", "tlb_row"]))
+        y_ref, scale = refdump.csr_ref(m, x)
+        kept.append((g, fmt, x, y_ref, scale))
+        if k % 2:
+            kept.pop(0)[0].close()
+        for g2, _, x2, r2, s2 in kept:
+            refdump.assert_y(g2.spmv_host(x2), r2, s2, np.float32, f"mesh {n}")
+    for g, fmt, *_ in kept:
+        g.close()
+        fmt.close()
+
+
+@pytest.mark.parametrize("template,nodes", [("K2", ["row_padding 128 1", "blb_row_evenly 128", "tlb_row"]), ("K3", ["row_padding 32 1", "tlb_row"]),
+                                            ("K6", ["row_padding 32 1", "blb_row_evenly 32", "tlb_col_fixed 2"]), ("B1", ["block_value 3 3"]), ("D1", ["diag_value 64"])])
+@pytest.mark.parametrize("dense", ["dense compress", "dense sort 1\ndense compress"])
+def test_y_needs_no_clearing_where_every_row_is_stored(asp_ctx, template, nodes, dense):
+    import torch
+
+    m, x = M.block_fem(1_001, 9, 100, seed=5) if template == "B1" else M.laplacian_2d(77, 3, grid_y=53)
+    if "sort" in dense:
+        if template in ("B1", "D1"):
+            pytest.skip("these templates keep the order of the rows")
+        keep = np.arange(m.n_rows) % 5 != 0  # rows without non-zeros: no kernel stores them
+        lengths = np.where(keep, m.row_lengths(), 0)
+        m, x = M.from_row_lengths(lengths, m.n_cols, seed=2, dtype=np.float64)
+    fmt, g = tuner.build(asp_ctx, m, desc(template, nodes, dense.replace("\n", " | ")))
+    dx = torch.from_numpy(x).cuda()
+    dy = torch.full((m.n_rows,), 9.0, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    g.spmv(dx.data_ptr(), dy.data_ptr(), True)
+    asp_ctx.synchronize()
+    y_ref, scale = refdump.csr_ref(m, x)
+    refdump.assert_y(dy.cpu().numpy(), y_ref, scale, np.float64, template)
+    g.close()
+    fmt.close()
