@@ -11,7 +11,6 @@
 #include <stdint.h>
 #include <stdlib.h>
 #include <string.h>
-#include <sys/mman.h>
 
 #include <memory>
 #include <new>
@@ -20,20 +19,10 @@ namespace asp
 {
 namespace host
 {
-inline std::shared_ptr<void> big_buffer(size_t bytes)
-{
-    const size_t huge = 2u << 20;
-    if (bytes < 2 * huge)
-    {
-        void *p = malloc(bytes ? bytes : 1);
-        if (!p) throw std::bad_alloc();
-        return std::shared_ptr<void>(p, free);
-    }
-    void *p = nullptr;
-    if (posix_memalign(&p, huge, (bytes + huge - 1) / huge * huge) != 0) throw std::bad_alloc();
-    madvise(p, (bytes + huge - 1) / huge * huge, MADV_HUGEPAGE); // (advice only: without huge pages everything still works)
-    return std::shared_ptr<void>(p, free);
-}
+// Large buffers come from a pool (hostmem.cpp): a fresh one costs a page fault per 2 MB, zeroed by the kernel at 5 to 20 GB/s, which
+// is several times what the operators do with it. Idle buffers are bounded (256 MB in all) and given back with host_pool_trim().
+std::shared_ptr<void> big_buffer(size_t bytes);
+void host_pool_trim();
 
 // Below these a loop runs on the calling thread: waking sixteen threads and waiting for the slowest costs up to a millisecond on
 // a busy host, as much as the loop itself.

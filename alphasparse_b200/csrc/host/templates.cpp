@@ -820,33 +820,24 @@ bool init_k9(const Matrix &m, const CompressedBlock &b, bool with_warp_reduce, T
 }
 } // namespace
 
-// ---- block-value template (this build's; no counterpart in the reference) --------------------------------
-// Blocked ELL over dense r x c blocks: block rows of r consecutive rows, block columns of c consecutive columns
-// (relative to the sub-matrix's first column); every block that holds a non-zero is stored in full, block rows
-// are padded with zero blocks to the width of the widest one, and the block rows to an even count.
-bool init_block_ell(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::string &err)
+namespace
 {
-    const u64 r = b.block_r, c = b.block_c;
-    if (m.is_sorted) return err = "block_value: not for sorted matrices (a block row must be r consecutive rows of y)", false;
-    if (!((r == 2 && c == 2) || (r == 3 && c == 3) || (r == 4 && c == 4))) return err = "block_value: blocks of 2 x 2, 3 x 3 or 4 x 4", false;
-    const u64 width = b.max_col - b.min_col + 1;
-    if (width % c) return err = "block_value: the columns of the sub-matrix are not a multiple of the block width", false;
-    const u64 NBR = (b.n_rows + r - 1) / r, NB = (NBR + 1) / 2 * 2;
-    // pass 1: block columns of every block row (merged over its r rows), from where the non-zeros of its first row begin
-    Arr<u32> bcol_arr;
-    u32 *const bcol = bcol_arr.make(std::max<u64>(1, b.col.size()));
-    std::vector<u32> cnt(NBR, 0);
+// block columns (of R x R blocks) of every block row, merged over its rows, from where the non-zeros of its first row begin in
+// bcol; returns the most of one block row
+template <int R>
+u64 block_columns(const CompressedBlock &b, u32 *const bcol, std::vector<u32> &cnt)
+{
     u64 W = 0;
 #pragma omp parallel for schedule(static) reduction(max : W) if (b.nnz() > kParallelNnz)
-    for (int64_t br = 0; br < (int64_t)NBR; br++)
+    for (int64_t br = 0; br < (int64_t)cnt.size(); br++)
     {
-        const u64 row0 = (u64)br * r, row1 = std::min<u64>(b.n_rows, row0 + r), nz0 = b.rowptr[row0];
+        const u64 row0 = (u64)br * R, row1 = std::min<u64>(b.n_rows, row0 + R), nz0 = b.rowptr[row0];
         u32 *const o = bcol + nz0;
         // the columns of a row ascend: its block columns come out in order; further rows usually repeat them
         u64 n = 0;
         for (u64 k = nz0; k < b.rowptr[row0 + 1]; k++)
         {
-            const u32 c0 = b.col[k] / (u32)c;
+            const u32 c0 = b.col[k] / (u32)R;
             if (n == 0 || o[n - 1] != c0) o[n++] = c0;
         }
         bool merged = false;
@@ -856,7 +847,7 @@ bool init_block_ell(const Matrix &m, const CompressedBlock &b, TemplateData &t, 
             const u64 sorted = n;
             for (u64 k = b.rowptr[row]; k < b.rowptr[row + 1]; k++)
             {
-                const u32 c0 = b.col[k] / (u32)c;
+                const u32 c0 = b.col[k] / (u32)R;
                 if (merged)
                 {
                     o[n++] = c0; // (at most one entry per non-zero: it stays inside the block row's share)
@@ -876,41 +867,76 @@ bool init_block_ell(const Matrix &m, const CompressedBlock &b, TemplateData &t, 
         cnt[br] = (u32)n;
         W = std::max(W, n);
     }
+    return W;
+}
+
+// the arrays: block columns ip[slot * NB + block row], values vp[((slot * R + i) * R + j) * NB + block row]
+template <int R, class V>
+void block_values(const CompressedBlock &b, const u32 *const bcol, const std::vector<u32> &cnt, u64 W, u64 NB, u32 *const ip, V *const vp)
+{
+    const V *const src = (const V *)b.val.b.data();
+#pragma omp parallel for schedule(static) if (b.nnz() > kParallelNnz)
+    for (int64_t br = 0; br < (int64_t)cnt.size(); br++)
+    {
+        const u64 n = cnt[br];
+        const u32 *bc = bcol + b.rowptr[(u64)br * R];
+        for (u64 k = 0; k < W; k++) ip[k * NB + br] = k < n ? bc[k] : (n ? bc[n - 1] : 0); // zero blocks repeat the last block column
+        // a block row of full blocks is overwritten whole (no column twice: entries are as many as there are places)
+        const u64 q0 = b.rowptr[(u64)br * R], q1 = b.rowptr[std::min<u64>(b.n_rows, ((u64)br + 1) * R)];
+        bool full = q1 - q0 == W * R * R && ((u64)br + 1) * R <= b.n_rows;
+        for (u64 row = (u64)br * R; full && row < ((u64)br + 1) * R; row++)
+            for (u64 q = b.rowptr[row] + 1; q < b.rowptr[row + 1]; q++) full = full && b.col[q] != b.col[q - 1];
+        if (!full)
+            for (u64 q = 0; q < W * R * R; q++) vp[q * NB + (u64)br] = 0;
+        for (u64 row = (u64)br * R; row < std::min<u64>(b.n_rows, ((u64)br + 1) * R); row++)
+        {
+            const u64 i = row - (u64)br * R;
+            u64 k = 0; // the columns of a row ascend, so do its block slots
+            for (u64 q = b.rowptr[row]; q < b.rowptr[row + 1]; q++)
+            {
+                const u32 cb = b.col[q] / (u32)R;
+                while (bc[k] != cb) k++;
+                const u64 j = b.col[q] - (u64)cb * R;
+                vp[((k * R + i) * R + j) * NB + (u64)br] = src[q];
+            }
+        }
+    }
+}
+} // namespace
+
+// ---- block-value template (this build's; no counterpart in the reference) --------------------------------
+// Blocked ELL over dense r x c blocks: block rows of r consecutive rows, block columns of c consecutive columns
+// (relative to the sub-matrix's first column); every block that holds a non-zero is stored in full, block rows
+// are padded with zero blocks to the width of the widest one, and the block rows to an even count.
+bool init_block_ell(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::string &err)
+{
+    const u64 r = b.block_r, c = b.block_c;
+    if (m.is_sorted) return err = "block_value: not for sorted matrices (a block row must be r consecutive rows of y)", false;
+    if (!((r == 2 && c == 2) || (r == 3 && c == 3) || (r == 4 && c == 4))) return err = "block_value: blocks of 2 x 2, 3 x 3 or 4 x 4", false;
+    const u64 width = b.max_col - b.min_col + 1;
+    if (width % c) return err = "block_value: the columns of the sub-matrix are not a multiple of the block width", false;
+    const u64 NBR = (b.n_rows + r - 1) / r, NB = (NBR + 1) / 2 * 2;
+    Arr<u32> bcol_arr;
+    u32 *const bcol = bcol_arr.make(std::max<u64>(1, b.col.size()));
+    std::vector<u32> cnt(NBR, 0);
+    const u64 W = r == 3 ? block_columns<3>(b, bcol, cnt) : r == 2 ? block_columns<2>(b, bcol, cnt) : block_columns<4>(b, bcol, cnt);
     if (W == 0) return err = "block_value: sub-matrix without non-zeros", false;
     const u64 stored = NB * W * r * c;
     if (b.nnz() == 0 || (double)stored / (double)b.nnz() > 8.0) return err = "block_value: the matrix is not made of dense blocks of this size (more than 8 stored values per non-zero)", false;
-    // pass 2: the arrays
     const int es = b.val.es;
     Arr<uint8_t> idx, val;
     u32 *const ip = (u32 *)idx.make_zero(NB * W * 4);
     uint8_t *const vp = val.make(stored * (u64)es);
     for (u64 q = 0; NB > NBR && q < W * r * c; q++) memset(vp + (q * NB + NBR) * es, 0, es); // the block row that pads
-#pragma omp parallel for schedule(static) if (b.nnz() > kParallelNnz)
-    for (int64_t br = 0; br < (int64_t)NBR; br++)
+    if (es == 8)
     {
-        const u64 n = cnt[br];
-        const u32 *bc = bcol + b.rowptr[(u64)br * r];
-        for (u64 k = 0; k < W; k++) ip[k * NB + br] = k < n ? bc[k] : (n ? bc[n - 1] : 0); // zero blocks repeat the last block column
-        // a block row of full blocks is overwritten whole (no column twice: entries are as many as there are places)
-        const u64 q0 = b.rowptr[(u64)br * r], q1 = b.rowptr[std::min<u64>(b.n_rows, ((u64)br + 1) * r)];
-        bool full = q1 - q0 == W * r * c;
-        for (u64 row = (u64)br * r; full && row < ((u64)br + 1) * r; row++)
-            for (u64 q = b.rowptr[row] + 1; q < b.rowptr[row + 1]; q++) full = full && b.col[q] != b.col[q - 1];
-        if (!full)
-            for (u64 q = 0; q < W * r * c; q++) memset(vp + (q * NB + (u64)br) * es, 0, es);
-        for (u64 row = (u64)br * r; row < std::min<u64>(b.n_rows, ((u64)br + 1) * r); row++)
-        {
-            const u64 i = row - (u64)br * r;
-            u64 k = 0; // the columns of a row ascend, so do its block slots
-            for (u64 q = b.rowptr[row]; q < b.rowptr[row + 1]; q++)
-            {
-                const u32 cb = b.col[q] / (u32)c;
-                while (bc[k] != cb) k++;
-                const u64 j = b.col[q] - (u64)cb * c;
-                memcpy(&vp[(((k * r + i) * c + j) * NB + (u64)br) * es], &b.val.b[q * es], es);
-            }
-        }
+        if (r == 3) block_values<3>(b, bcol, cnt, W, NB, ip, (u64 *)vp);
+        else if (r == 2) block_values<2>(b, bcol, cnt, W, NB, ip, (u64 *)vp);
+        else block_values<4>(b, bcol, cnt, W, NB, ip, (u64 *)vp);
     }
+    else if (r == 3) block_values<3>(b, bcol, cnt, W, NB, ip, (u32 *)vp);
+    else if (r == 2) block_values<2>(b, bcol, cnt, W, NB, ip, (u32 *)vp);
+    else block_values<4>(b, bcol, cnt, W, NB, ip, (u32 *)vp);
     common_head(m, b, ASP_BLOCK_ELL_TEMPLATE, t);
     t.tlb_size = W;
     t.bits_row = (int)r;

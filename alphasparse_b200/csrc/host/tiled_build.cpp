@@ -160,7 +160,7 @@ double lines_per_gather(const TiledSource &s, bool f64)
 {
     const bool by4 = s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS ||
                      s.templ == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || s.templ == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE;
-    const u64 groups = s.stored / 128, samples = std::min<u64>(groups, 256), per_line = f64 ? 16 : 32;
+    const u64 groups = s.stored / 128, samples = std::min<u64>(groups, 128), per_line = f64 ? 16 : 32;
     if (samples == 0) return 0.0;
     u64 lines = 0;
     for (u64 q = 0; q < samples; q++)
@@ -214,7 +214,8 @@ double slowness(const TiledSource &s)
 const u32 kMaxPiece = 32;    // elements of a row's piece: bounds the serial chain of a lane and the padding of a slice
 const u32 kWindow = 1024;    // pieces that are sorted by length together: lanes of a slice stay near in y
 const double kSliceCost = 4.0; // in steps; with 2 the CTAs of sparse tiles ran twice as long as the others
-const u64 kBlock = 1u << 16; // elements of a block of whole rows, the unit of the parallel build
+// elements of a block of whole rows, the unit of the parallel build: enough blocks for all cores, and whole windows in each
+u64 block_size(u64 n) { return std::min<u64>(1u << 16, std::max<u64>(1u << 13, n / 128)); }
 
 struct Chunk
 {
@@ -351,6 +352,7 @@ struct Builder
     void slices(int n_sm, TiledHost &out)
     {
         std::vector<Block> blocks;
+        const u64 kBlock = block_size(N);
         std::vector<size_t> tile_block(C + 1, 0);
         for (u64 t = 0; t < C; t++)
         {
@@ -370,7 +372,7 @@ struct Builder
 #pragma omp parallel
         {
             std::vector<Piece> p, tmp;
-#pragma omp for schedule(dynamic, 4)
+#pragma omp for schedule(dynamic, 1)
             for (long long b = 0; b < B; b++)
             {
                 pieces_of(blocks[b], p, tmp);
@@ -397,7 +399,7 @@ struct Builder
 #pragma omp parallel
         {
             std::vector<Piece> p, tmp;
-#pragma omp for schedule(dynamic, 4)
+#pragma omp for schedule(dynamic, 1)
             for (long long b = 0; b < B; b++)
             {
                 pieces_of(blocks[b], p, tmp);

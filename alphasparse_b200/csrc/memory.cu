@@ -2,9 +2,13 @@
 
 #include <string.h>
 
+#include <atomic>
+
 #include <algorithm>
 #include <map>
 #include <mutex>
+
+#include "host/hostmem.hpp"
 
 namespace asp
 {
@@ -143,6 +147,7 @@ void device_pool_release(int device)
     }
     OnDevice on(device);
     for (void *q : idle) cudaFree(q);
+    host::host_pool_trim();
 }
 
 bool Stager::ready()
@@ -217,19 +222,69 @@ cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaSt
     const size_t end = seg.back().off + seg.back().bytes;
     // about eight pieces: the first one's filling and the last one's copy are all that does not overlap
     const size_t piece = std::min(kPiece, std::max<size_t>(256u << 10, (end / 8 + kPart - 1) / kPart * kPart));
-    for (size_t o = seg.front().off; o < end; o += piece)
+    const size_t begin = seg.front().off, total = end - begin;
+    const long long n_pieces = (long long)((total + piece - 1) / piece), per = (long long)(piece / kPart), n_parts = (long long)((total + kPart - 1) / kPart);
+    if (n_parts <= 3)
     {
-        const size_t n = std::min(piece, end - o);
+        // (over before other threads are awake)
         unsigned char *p;
         int i;
         cudaError_t e = slot(&p, &i);
         if (e != cudaSuccess) return e;
-        parts(n, [&](size_t at, size_t k) { gather(p + at, o + at, k, seg); });
-        e = cudaMemcpyAsync((unsigned char *)dev + o, p, n, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) e = cudaEventRecord(done[i], st);
-        if (e != cudaSuccess) return e;
+        gather(p, begin, total, seg);
+        e = cudaMemcpyAsync((unsigned char *)dev + begin, p, total, cudaMemcpyHostToDevice, st);
+        return e == cudaSuccess ? cudaEventRecord(done[i], st) : e;
     }
-    return cudaSuccess;
+    // The threads take parts in order; the calling one also sends every piece whose parts are in. A piece is opened (its slot of
+    // the ring free again) before its parts may be filled.
+    unsigned char *where[kPieces];
+    int used[kPieces];
+    std::atomic<long long> next_part(0), open_pieces(0);
+    std::atomic<int> filled[kPieces];
+    for (auto &f : filled) f.store(0);
+    std::atomic<bool> stop(false);
+    cudaError_t e = cudaSuccess;
+    auto open = [&](long long k) { // by the calling thread only
+        e = slot(&where[k % kPieces], &used[k % kPieces]);
+        filled[k % kPieces].store(0);
+        if (e != cudaSuccess) stop.store(true);
+        else open_pieces.store(k + 1);
+    };
+    auto fill_one = [&]() -> bool { // false: no part to be had now
+        long long q = next_part.load();
+        do
+        {
+            if (q >= n_parts || q / per >= open_pieces.load()) return false;
+        } while (!next_part.compare_exchange_weak(q, q + 1));
+        const long long k = q / per;
+        const size_t at = (size_t)(q - k * per) * kPart, o = (size_t)k * piece + at;
+        gather(where[k % kPieces] + at, begin + o, std::min(kPart, total - o), seg);
+        filled[k % kPieces].fetch_add(1);
+        return true;
+    };
+    for (long long k = 0; k < n_pieces && k < kPieces && e == cudaSuccess; k++) open(k);
+#pragma omp parallel
+    {
+        bool mine = false;
+#pragma omp master
+        mine = true;
+        if (mine)
+        {
+            for (long long k = 0; k < n_pieces && e == cudaSuccess; k++)
+            {
+                const long long parts_of = std::min(per, n_parts - k * per);
+                while (filled[k % kPieces].load() < parts_of) fill_one();
+                const size_t o = (size_t)k * piece, n = std::min(piece, total - o);
+                e = cudaMemcpyAsync((unsigned char *)dev + begin + o, where[k % kPieces], n, cudaMemcpyHostToDevice, st);
+                if (e == cudaSuccess) e = cudaEventRecord(done[used[k % kPieces]], st);
+                if (e == cudaSuccess && k + kPieces < n_pieces) open(k + kPieces);
+            }
+            stop.store(true);
+        }
+        else
+            while (!stop.load() && next_part.load() < n_parts) fill_one();
+    }
+    return e;
 }
 
 cudaError_t Stager::to_host(void *host, const void *dev, size_t bytes, cudaStream_t st)
