@@ -1070,7 +1070,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
     }
     if (tg)
     {
-        const void *from[5] = {th.val.p.get(), th.col.p.get(), th.row.p.get(), th.end.p.get(), th.work.data()};
+        const void *from[5] = {th.val.p, th.col.p, th.row.p, th.end.p, th.work.data()};
         const size_t bytes[5] = {th.val.bytes(), th.col.bytes(), th.row.bytes(), th.end.bytes(), th.work.size() * sizeof(uint32_t)};
         size_t off[6] = {0};
         for (int k = 0; k < 5; k++) off[k + 1] = align_up(off[k] + bytes[k], 256);

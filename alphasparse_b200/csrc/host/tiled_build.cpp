@@ -160,7 +160,7 @@ double lines_per_gather(const TiledSource &s, bool f64)
 {
     const bool by4 = s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS ||
                      s.templ == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || s.templ == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE;
-    const u64 groups = s.stored / 128, samples = std::min<u64>(groups, 128), per_line = f64 ? 16 : 32;
+    const u64 groups = s.stored / 128, samples = std::min<u64>(groups, 64), per_line = f64 ? 16 : 32;
     if (samples == 0) return 0.0;
     u64 lines = 0;
     for (u64 q = 0; q < samples; q++)
@@ -228,7 +228,7 @@ struct Builder
 {
     const std::vector<TiledSource> &src;
     const u64 n_rows, n_cols;
-    const u32 TW;
+    static constexpr u32 TW = tiled_tile_cols(sizeof(VT) == 8);
     const u64 C; // tiles of x
     std::vector<Chunk> chunks;
     std::vector<u64> at; // [chunk * C + tile]: first its count, then where its elements go
@@ -239,7 +239,7 @@ struct Builder
     HostBuf<uint16_t> e_col;
     HostBuf<VT> e_val;
 
-    Builder(const std::vector<TiledSource> &s, u64 rows, u64 cols) : src(s), n_rows(rows), n_cols(cols), TW(tiled_tile_cols(sizeof(VT) == 8)), C((cols + TW - 1) / TW) {}
+    Builder(const std::vector<TiledSource> &s, u64 rows, u64 cols) : src(s), n_rows(rows), n_cols(cols), C((cols + TW - 1) / TW) {}
 
     void count(bool &covered)
     {
@@ -256,14 +256,14 @@ struct Builder
         std::vector<uint8_t> seen(n_rows, 0);
 #pragma omp parallel
         {
-            std::vector<u64> pieces(C, 0);
+            std::vector<u64> pieces(C, 0), n(C); // (counters of a thread's own: neighbours in `at` share cache lines)
 #pragma omp for schedule(dynamic, 1)
             for (long long c = 0; c < (long long)chunks.size(); c++)
             {
-                u64 *n = &at[(size_t)c * C];
+                std::fill(n.begin(), n.end(), 0);
                 u64 row = ~0ull, tile = ~0ull, run = 0;
                 walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT) {
-                    const u64 t = col / TW;
+                    const u64 t = (u32)col / TW;
                     n[t]++;
                     if (r != row || t != tile || run == kMaxPiece)
                     {
@@ -275,6 +275,7 @@ struct Builder
                     }
                     run++;
                 });
+                std::copy(n.begin(), n.end(), at.begin() + (size_t)c * C);
             }
 #pragma omp critical
             for (u64 t = 0; t < C; t++) tile_pieces[t] += pieces[t];
@@ -303,16 +304,20 @@ struct Builder
         e_row.make(N);
         e_col.make(N);
         e_val.make(N);
-#pragma omp parallel for schedule(dynamic, 1)
-        for (long long c = 0; c < (long long)chunks.size(); c++)
+#pragma omp parallel
         {
-            u64 *to = &at[(size_t)c * C];
-            walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) {
-                const u64 t = col / TW, q = to[t]++;
-                e_row.p[q] = (u32)r;
-                e_col.p[q] = (uint16_t)(col - t * TW);
-                e_val.p[q] = v;
-            });
+            std::vector<u64> to(C);
+#pragma omp for schedule(dynamic, 1)
+            for (long long c = 0; c < (long long)chunks.size(); c++)
+            {
+                std::copy(at.begin() + (size_t)c * C, at.begin() + (size_t)(c + 1) * C, to.begin());
+                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) {
+                    const u64 t = (u32)col / TW, q = to[t]++;
+                    e_row.p[q] = (u32)r;
+                    e_col.p[q] = (uint16_t)(col - t * TW);
+                    e_val.p[q] = v;
+                });
+            }
         }
     }
 
@@ -395,7 +400,7 @@ struct Builder
         out.col.make(st * kTiledSlice);
         out.row.make(sl * kTiledSlice);
         out.end.make(sl);
-        VT *val = (VT *)out.val.p.get();
+        VT *val = (VT *)out.val.p;
 #pragma omp parallel
         {
             std::vector<Piece> p, tmp;
@@ -408,8 +413,8 @@ struct Builder
                 {
                     const u32 depth = p[i].len;
                     VT *v = val + step * kTiledSlice;
-                    uint16_t *c = out.col.p.get() + step * kTiledSlice;
-                    u32 *rows = out.row.p.get() + slice * kTiledSlice;
+                    uint16_t *c = out.col.p + step * kTiledSlice;
+                    u32 *rows = out.row.p + slice * kTiledSlice;
                     memset(v, 0, (size_t)depth * kTiledSlice * sizeof(VT));
                     std::fill(c, c + (size_t)depth * kTiledSlice, (uint16_t)TW);
                     for (u32 j = 0; j < kTiledSlice; j++)
@@ -432,8 +437,8 @@ struct Builder
             }
         }
         memset(val + steps * kTiledSlice, 0, kTiledSlackSteps * kTiledSlice * sizeof(VT));
-        memset(out.col.p.get() + steps * kTiledSlice, 0, kTiledSlackSteps * kTiledSlice * sizeof(uint16_t));
-        memset(out.row.p.get() + nsl * kTiledSlice, 0xff, kTiledSlackSlices * kTiledSlice * sizeof(u32));
+        memset(out.col.p + steps * kTiledSlice, 0, kTiledSlackSteps * kTiledSlice * sizeof(uint16_t));
+        memset(out.row.p + nsl * kTiledSlice, 0xff, kTiledSlackSlices * kTiledSlice * sizeof(u32));
         for (u32 i = 0; i < kTiledSlackSlices; i++) out.end.p[nsl + i] = 0xffffffffu;
         out.nnz = N;
         out.steps = steps;
@@ -445,7 +450,7 @@ struct Builder
         for (u64 t = C; t-- > 0;) tile_step[t] = tile_block[t] < blocks.size() ? blocks[tile_block[t]].step : steps;
         u64 used = 0;
         for (u64 t = 0; t < C; t++) used += tile_step[t + 1] > tile_step[t] ? 1 : 0;
-        const u32 *end = out.end.p.get();
+        const u32 *end = out.end.p;
         auto slice_of = [&](u64 step) { return (u64)(std::upper_bound(end, end + nsl, (u32)step) - end); };
         auto cost_of = [&](u64 step) { return (double)step + kSliceCost * (double)slice_of(step); };
         // the step in [lo, hi] that a cost is reached at

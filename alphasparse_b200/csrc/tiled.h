@@ -9,6 +9,7 @@
 #include <memory>
 #include <vector>
 
+#include "host/hostmem.hpp"
 #include "host_meta.h"
 #include "kernel_args.h"
 
@@ -17,13 +18,13 @@ namespace asp
 const uint32_t kTiledWarps = 32;             // warps per CTA, one CTA per SM
 const uint32_t kTiledLanePieces = 2;         // pieces of a row per lane
 const uint32_t kTiledSlice = 32 * kTiledLanePieces;
-const uint32_t kTiledTileBytes = 159u << 10; // shared memory of a tile of x
+constexpr uint32_t kTiledTileBytes = 159u << 10; // shared memory of a tile of x
 const uint32_t kTiledNoRow = 0xffffffffu;
 // steps and slices the kernel may read past the end (prefetch)
 const uint32_t kTiledSlackSteps = 8, kTiledSlackSlices = 2;
 
 // columns of a tile; the shared memory after them holds one zero, which what pads a slice multiplies (never an infinite x)
-inline uint32_t tiled_tile_cols(bool f64) { return kTiledTileBytes / (f64 ? 8u : 4u) - 32u; }
+constexpr uint32_t tiled_tile_cols(bool f64) { return kTiledTileBytes / (f64 ? 8u : 4u) - 32u; }
 
 // one sub-matrix of the group, as its template stores it (host arrays)
 struct TiledSource
@@ -42,9 +43,10 @@ struct TiledSource
 template <class T>
 struct HostBuf
 {
-    std::unique_ptr<T[]> p;
+    std::shared_ptr<void> s;
+    T *p = nullptr;
     uint64_t n = 0;
-    void make(uint64_t count) { p.reset(new T[count]), n = count; }
+    void make(uint64_t count) { s = host::big_buffer(count * sizeof(T)), p = (T *)s.get(), n = count; }
     uint64_t bytes() const { return n * sizeof(T); }
 };
 
