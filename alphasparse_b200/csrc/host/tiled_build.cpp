@@ -512,8 +512,8 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
 {
     const double sv = sizeof(VT);
     // The group's own kernels: one request to L2 per cache line that a gather touches (290 G/s on this part, of which they reach
-    // 0.85) or the format's bytes, or their longest serial chain, whichever is longest; a call takes 4.5 us at least, several
-    // kernels a fork and a join more.
+    // 0.85) or the format's bytes, or their longest serial chain, whichever is longest. Below some 10 us the rates are not reached
+    // (20,000 rows of 80 random columns: 13.8 us for 7 us of requests); several kernels add a fork and a join.
     u64 true_nnz = 0;
     double chain = 0, requests = 0, bytes_us = 0;
     for (const TiledSource &s : src)
@@ -524,7 +524,10 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
         requests += (double)s.stored * slowness(s);
         bytes_us += (double)s.stored * slowness(s) * (sv + 4) / 6.0e6;
     }
-    auto own = [&](double lines) { return 4.5 + (src.size() > 1 ? 8.0 : 0.0) + std::max(std::max(lines / (0.85 * 290e3), bytes_us), chain); };
+    auto own = [&](double lines) {
+        const double rate = std::max(lines / (0.85 * 290e3), bytes_us);
+        return (src.size() > 1 ? 8.0 : 0.0) + std::max(2.0 + chain, 3.0 + rate + std::min(0.4 * rate, 4.5));
+    };
     // A small group of several strips keeps its kernels: callers compare its rows bit for bit with those of the same group with
     // some strips muted (EMPTY), as a search does that times strip after strip.
     if (src.size() > 1 && true_nnz < (1u << 16)) return false;
