@@ -148,6 +148,7 @@ struct asp_plan
     uint64_t warp_tasks = 0; // SELL-like with equal strips: warp-sized work items
     uint64_t sell_strip = 0; // SELL-like: TLBs per strip when all strips are equal, else 0
     bool needs_zero = false;
+    bool ends_cover = false;      // CSR5-like: every row that is not an end row of a warp is stored, so only those need clearing
     bool stores_all_rows = false; // every row of y is stored (not accumulated) by every SpMV: y needs no clearing
     // CSR5-like family: the rows of y that warps accumulate with `red` (first and last row of every warp), as
     // indices into y; kept on the device for the publishing SpMV (asp_spmv_publish)
@@ -928,7 +929,11 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
                 };
                 std::vector<uint32_t> rows(2 * W);
                 uint64_t all_starts = 0;
-#pragma omp parallel for schedule(static) reduction(+ : all_starts) if (W > 4096)
+                // rows without gaps: every warp starts at the row the one before ends with, or at the next
+                bool gapless = d.sort_kind == ASP_SORT_NONE && d.first_row == 0 && !a.atomic && fr.get(0) == 0;
+                bool in_step = true; // the first row that every thread names is the one its place in the warp implies
+                const uint64_t rmask = (1ull << d.bits_row) - 1;
+#pragma omp parallel for schedule(static) reduction(+ : all_starts) reduction(&& : in_step) if (W > 4096)
                 for (int64_t w = 0; w < (int64_t)W; w++)
                 {
                     uint64_t starts = 0;
@@ -936,6 +941,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
                     {
                         const uint64_t m = cm.get((uint64_t)w * 32 + l);
                         const uint64_t flags = S >= 64 ? m : ((m >> (bw - S)) & ((1ull << S) - 1));
+                        if (flags) in_step = in_step && (m & rmask) == starts;
                         starts += (uint64_t)__builtin_popcountll(flags);
                     }
                     const uint64_t R0 = fr.get(w);
@@ -951,6 +957,9 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
                     while (cap < 2 * avg && cap < 256) cap <<= 1;
                     a.stage_cap = (int)std::min<uint64_t>(cap, 32ull * S);
                 }
+                gapless = gapless && in_step;
+                for (uint64_t w = 1; w < W && gapless; w++) gapless = rows[2 * w] == rows[2 * w - 1] || rows[2 * w] == rows[2 * w - 1] + 1;
+                p->ends_cover = gapless && rows[2 * W - 1] + 1ull == d.n_rows;
                 rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
                 std::shared_ptr<Arena> er(new (std::nothrow) Arena());
                 if (!er || er->make(ctx->device, std::max<size_t>(rows.size() * 4, 4)) != cudaSuccess)
@@ -1275,7 +1284,11 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
             return ASP_OK;
         }
     }
-    if (clear && !(n_plans == 1 && plans[0]->stores_all_rows)) ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
+    const asp_plan *only = n_plans == 1 ? plans[0] : nullptr;
+    if (clear && only && only->ends_cover && only->end_rows)
+        ASP_CUDA(asp::launch_zero_rows(only->val_is_f64, d_y, (const unsigned *)only->end_rows->base, only->n_end_rows, ctx->stream));
+    else if (clear && !(only && only->stores_all_rows))
+        ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
     if (!g.first) return ASP_OK;
     int active = 0;
     for (int i = 0; i < n_plans; i++) active += plans[i]->templ != ASP_EMPTY_TEMPLATE;

@@ -325,19 +325,22 @@ __global__ void __launch_bounds__(512) k_ell(KArgs a)
                 CT c[U - 1][V];
 #pragma unroll
                 for (int u = 0; u < U - 1; u++)
-                    if (k + u < S)
-                    {
-                        ld_stream_n<VT, V>(vp + (u64)(k + u) * P, v[u]);
-                        ld_stream_n<CT, V>(cp + (u64)(k + u) * P, c[u]);
-                    }
+                {
+                    // past the end the last step is loaded again and dropped: no branch between the loads
+                    const u64 at = (u64)(k + u < S ? k + u : S - 1) * P;
+                    ld_stream_pinned<VT, V>(vp + at, v[u]);
+                    ld_stream_pinned<CT, V>(cp + at, c[u]);
+                }
                 wait();
+                VT xv[U - 1][V];
 #pragma unroll
                 for (int u = 0; u < U - 1; u++)
-                    if (k + u < S)
-                    {
 #pragma unroll
-                        for (int j = 0; j < V; j++) acc[j] += v[u][j] * ld_x(x + c[u][j]);
-                    }
+                    for (int j = 0; j < V; j++) xv[u][j] = ld_x(x + c[u][j]);
+#pragma unroll
+                for (int u = 0; u < U - 1; u++)
+#pragma unroll
+                    for (int j = 0; j < V; j++) acc[j] += k + u < S ? v[u][j] * xv[u][j] : VT(0);
             }
         }
         if (unit_rows && t0 + V <= a.effective)
@@ -424,24 +427,25 @@ __device__ __forceinline__ void sell_group(const KArgs &a, const VT *__restrict_
     }
     if (k < S)
     {
-        // the last S % U steps (all of a short TLB) as one predicated batch
-        VT v[U - 1][V];
+        // the last S % U steps (all of a short TLB) as one batch; past the end the last step is loaded again and dropped
+        VT v[U - 1][V], xv[U - 1][V];
         CT c[U - 1][V];
 #pragma unroll
         for (int u = 0; u < U - 1; u++)
-            if (k + u < S)
-            {
-                ld_stream_n<VT, V>(vp + (u64)u * n, v[u]);
-                ld_stream_n<CT, V>(cp + (u64)u * n, c[u]);
-            }
+        {
+            const u64 at = (u64)(k + u < S ? (u32)u : S - 1 - k) * n;
+            ld_stream_pinned<VT, V>(vp + at, v[u]);
+            ld_stream_pinned<CT, V>(cp + at, c[u]);
+        }
         wait();
 #pragma unroll
         for (int u = 0; u < U - 1; u++)
-            if (k + u < S)
-            {
 #pragma unroll
-                for (int j = 0; j < V; j++) acc[j] += v[u][j] * ld_x(x + c[u][j]);
-            }
+            for (int j = 0; j < V; j++) xv[u][j] = ld_x(x + c[u][j]);
+#pragma unroll
+        for (int u = 0; u < U - 1; u++)
+#pragma unroll
+            for (int j = 0; j < V; j++) acc[j] += k + u < S ? v[u][j] * xv[u][j] : VT(0);
     }
     wait(); // (an empty strip stores its zeros too)
     sell_store<VT, V>(a, y, acc, t0, radd);
@@ -937,12 +941,23 @@ __device__ __forceinline__ void strided_products(const VT *__restrict__ val, con
     }
     else
     {
+        // past the end the last element is loaded again and dropped: no branch between the loads, all of them of this thread's elements
+        const u32 last = cnt - 1;
+        CT c[U][1];
+        VT v[U][1], xv[U];
 #pragma unroll
-        for (int u = 0; u < U; u++) p[u] = (u32)u < cnt ? __ldcs(val + nz + 32 * u) * ld_x(x + __ldcs(col + nz + 32 * u)) : VT(0);
+        for (int u = 0; u < U; u++) ld_stream_pinned<CT, 1>(col + nz + 32 * ((u32)u < cnt ? (u32)u : last), c[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++) ld_stream_pinned<VT, 1>(val + nz + 32 * ((u32)u < cnt ? (u32)u : last), v[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++) xv[u] = ld_x(x + c[u][0]);
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = (u32)u < cnt ? v[u][0] * xv[u] : VT(0);
     }
 }
 
-template <class VT, class CT, bool WARP_FAST>
+// UB: elements of a batch, 4 for TLBs of up to 4, else 8
+template <class VT, class CT, bool WARP_FAST, int UB>
 __global__ void __launch_bounds__(256) k_csr5(KArgs a)
 {
     grid_wait();
@@ -965,7 +980,7 @@ __global__ void __launch_bounds__(256) k_csr5(KArgs a)
             if (R0 == R1)
             {
                 VT s = 0;
-                constexpr int UF = 8;
+                constexpr int UF = UB;
                 for (u32 k0 = 0; k0 < S; k0 += UF, nz += 32 * UF)
                 {
                     VT pr[UF];
@@ -987,7 +1002,7 @@ __global__ void __launch_bounds__(256) k_csr5(KArgs a)
         VT sum = 0, tail = 0;
         // products of U elements are fetched together (independent gathers in flight) before the
         // sequential walk over the row-start flags
-        constexpr u32 U = 8;
+        constexpr u32 U = UB;
         for (u32 k0 = 0; k0 < S; k0 += U, nz += 32 * U)
         {
             VT v[U];
@@ -1094,8 +1109,8 @@ static cudaError_t launch_vc(int templ, const KArgs &a, dim3 grid, dim3 block, s
         if (csr5_specialised((int)a.tlb_size, (int)sizeof(CT), a.bits_word) && ((a.path & 2) == 0 || (a.path & 1) || a.y_mc))
             return launch_csr5(sizeof(VT) == 8, (int)sizeof(CT), (templ == 9 ? 1 : 0) | ((a.path & 1) ? 2 : 0) | (a.y_mc ? 6 : 0), a, grid.x, block.x, st);
         if (a.y_mc) return cudaErrorInvalidValue;
-        if (templ == 8) return launch_pdl(k_csr5<VT, CT, false>, grid, block, 0, st, a);
-        return launch_pdl(k_csr5<VT, CT, true>, grid, block, 0, st, a);
+        if (a.tlb_size <= 4) return templ == 8 ? launch_pdl(k_csr5<VT, CT, false, 4>, grid, block, 0, st, a) : launch_pdl(k_csr5<VT, CT, true, 4>, grid, block, 0, st, a);
+        return templ == 8 ? launch_pdl(k_csr5<VT, CT, false, 8>, grid, block, 0, st, a) : launch_pdl(k_csr5<VT, CT, true, 8>, grid, block, 0, st, a);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -132,8 +132,6 @@ __global__ void __launch_bounds__(256) k_csr5s(KArgs a)
 {
     constexpr bool WARP_FAST = (MODE & 1) != 0, STAGE = (MODE & 2) != 0, PUBLISH = (MODE & 4) != 0;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    grid_wait();
-    grid_release();
     const VT *__restrict__ val = (const VT *)a.val;
     const CT *__restrict__ col = (const CT *)a.col;
     const VT *__restrict__ x = (const VT *)a.x + a.first_col;
@@ -156,6 +154,7 @@ __global__ void __launch_bounds__(256) k_csr5s(KArgs a)
         else y[r] = v;
     };
 
+    WaitOnce wait; // the first indices and values are on their way when it waits
     for (u64 w = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < a.n_units; w += wstride)
     {
         const u64 R0 = mget5(a.m[MS_ROW_OF_UNIT], w);
@@ -175,6 +174,7 @@ __global__ void __launch_bounds__(256) k_csr5s(KArgs a)
                     for (int u = 0; u < B; u++) c[u] = ld_col(col + nz0 + 32 * (k0 + u));
 #pragma unroll
                     for (int u = 0; u < B; u++) v[u] = ld_val(val + nz0 + 32 * (k0 + u));
+                    wait();
 #pragma unroll
                     for (int u = 0; u < B; u++) xv[u] = ld_x(x + c[u]);
 #pragma unroll
@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(256) k_csr5s(KArgs a)
             for (int u = 0; u < B; u++) c[u] = ld_col(col + nz0 + 32 * (k0 + u));
 #pragma unroll
             for (int u = 0; u < B; u++) p[u] = ld_val(val + nz0 + 32 * (k0 + u));
+            wait();
 #pragma unroll
             for (int u = 0; u < B; u++) xv[u] = ld_x(x + c[u]);
 #pragma unroll
@@ -320,6 +321,7 @@ __global__ void __launch_bounds__(256) k_csr5s(KArgs a)
         }
         __syncwarp(); // the next warp task of this warp reuses the staging area
     }
+    wait();
     if (PUBLISH) __threadfence_system();
 }
 
@@ -369,8 +371,10 @@ cudaError_t launch_vc5(int S, int mode, const KArgs &a, unsigned grid, unsigned 
 // rows[i]: global row of y that some warp accumulates with `red`. Before the SpMV kernel they are cleared
 // (locally); after it they hold their totals and are sent to every GPU.
 template <class VT>
-__global__ void __launch_bounds__(256) k_zero_rows(VT *__restrict__ y, const u32 *__restrict__ rows, u64 n)
+__global__ void __launch_bounds__(256) k_zero_rows(VT *y, const u32 *rows, u64 n)
 {
+    grid_wait();
+    grid_release();
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) y[rows[i]] = 0;
 }
 template <class VT>
@@ -404,9 +408,8 @@ cudaError_t launch_zero_rows(int val_is_f64, void *y, const unsigned *rows, unsi
 {
     if (n == 0) return cudaSuccess;
     const unsigned grid = (unsigned)((n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024);
-    if (val_is_f64) k_zero_rows<double><<<grid, 256, 0, st>>>((double *)y, rows, n);
-    else k_zero_rows<float><<<grid, 256, 0, st>>>((float *)y, rows, n);
-    return cudaGetLastError();
+    if (val_is_f64) return launch_pdl(k_zero_rows<double>, dim3(grid), dim3(256), 0, st, (double *)y, (const u32 *)rows, (u64)n);
+    return launch_pdl(k_zero_rows<float>, dim3(grid), dim3(256), 0, st, (float *)y, (const u32 *)rows, (u64)n);
 }
 
 cudaError_t launch_publish_rows(int val_is_f64, const void *y, void *y_mc, const unsigned *rows, unsigned long long n, cudaStream_t st)
