@@ -939,6 +939,13 @@ __device__ __forceinline__ void strided_products(const VT *__restrict__ val, con
 #pragma unroll
         for (int u = 0; u < U; u++) p[u] = v[u][0] * xv[u];
     }
+    else if (U == 8 && cnt <= 4)
+    {
+        VT q[4];
+        strided_products<VT, CT, 4>(val, col, x, nz, cnt, q);
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = u < 4 ? q[u & 3] : VT(0);
+    }
     else
     {
         // past the end the last element is loaded again and dropped: no branch between the loads, all of them of this thread's elements
