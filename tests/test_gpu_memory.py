@@ -67,3 +67,31 @@ def test_y_needs_no_clearing_where_every_row_is_stored(asp_ctx, template, nodes,
     refdump.assert_y(dy.cpu().numpy(), y_ref, scale, np.float64, template)
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("template", ["K9", "K10"])
+@pytest.mark.parametrize("s", [1, 3, 4, 5, 11, 16, 40])
+@pytest.mark.parametrize("empty", ["none", "some", "last"])
+def test_csr5_like_rows_left_uncleared(asp_ctx, template, s, empty):
+    """Rows that lie inside one thread's or one block's share are stored, only the shared ones are cleared before."""
+    import torch
+
+    rng = np.random.default_rng(s)
+    lengths = rng.integers(1, 12, 5_003)
+    lengths[[0, 2_000, 5_002]] = 900  # shared by several threads and blocks
+    if empty == "some":
+        lengths[rng.integers(1, 5_002, 700)] = 0
+    elif empty == "last":
+        lengths[-300:] = 0
+    m, x = M.from_row_lengths(lengths, 4_096, seed=s, dtype=np.float32)
+    fmt, g = tuner.build(asp_ctx, m, desc(template, [f"tlb_nnz {s}"]))
+    dx = torch.from_numpy(x).cuda()
+    dy = torch.full((m.n_rows,), 9.0, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        g.spmv(dx.data_ptr(), dy.data_ptr(), True)
+    asp_ctx.synchronize()
+    y_ref, scale = refdump.csr_ref(m, x)
+    refdump.assert_y(dy.cpu().numpy(), y_ref, scale, np.float32, f"{template} {s} {empty}")
+    g.close()
+    fmt.close()
