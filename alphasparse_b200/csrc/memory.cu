@@ -10,7 +10,9 @@
 
 #include <algorithm>
 #include <map>
+#include <memory>
 #include <mutex>
+#include <vector>
 
 #include "host/hostmem.hpp"
 
@@ -87,6 +89,7 @@ void gather(unsigned char *dst, size_t at, size_t n, const std::vector<Stager::S
 }
 
 const size_t kPart = 64u << 10; // what one thread copies at a time
+const long long kFirstParts = 16, kMostParts = 64; // of the pieces of an upload: first pieces of 512 KB cost 8 us more with 1.3 MB of x, longest ones of 2 MB 5 us more with 8 MB
 // a copy of fewer parts is over before the threads are awake
 template <class F>
 void parts(size_t n, F &&f)
@@ -190,6 +193,7 @@ bool Stager::ready()
             return false;
         }
     ring = (unsigned char *)p;
+    for (int i = 0; i < kPieces; i++) owner[i] = i;
     off = false;
     return true;
 }
@@ -213,12 +217,33 @@ bool Stager::pinned(const void *host)
     return at.type != cudaMemoryTypeUnregistered;
 }
 
-cudaError_t Stager::slot(unsigned char **p, int *i)
+// (an event that was never recorded counts as done)
+bool Stager::free_now(int slots) const
 {
-    *i = next;
-    next = (next + 1) % kPieces;
-    *p = ring + (size_t)*i * kPiece;
-    return cudaEventSynchronize(done[*i]); // (an event that was never recorded counts as done)
+    const int first = next + slots > kPieces ? 0 : next;
+    for (int i = first; i < first + slots; i++)
+        if (cudaEventQuery(done[owner[i]]) != cudaSuccess)
+        {
+            cudaGetLastError(); // not ready is no error
+            return false;
+        }
+    return true;
+}
+
+cudaError_t Stager::take(int slots, unsigned char **p, int *event)
+{
+    const int first = next + slots > kPieces ? 0 : next, last = first + slots - 1;
+    for (int i = first; i <= last; i++)
+    {
+        const cudaError_t e = cudaEventSynchronize(done[owner[i]]);
+        if (e != cudaSuccess) return e;
+    }
+    // (slots outside that still name this event belong to a piece that is over: the last slot was its, too)
+    for (int i = first; i <= last; i++) owner[i] = last;
+    next = (last + 1) % kPieces;
+    *p = ring + (size_t)first * kPiece;
+    *event = last;
+    return cudaSuccess;
 }
 
 cudaError_t Stager::to_device(void *dev, const void *host, size_t bytes, cudaStream_t st)
@@ -239,50 +264,73 @@ cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaSt
         }
         return cudaSuccess;
     }
-    const size_t end = seg.back().off + seg.back().bytes;
-    // the first piece's filling and the last one's copy are all that does not overlap; a piece costs 3 us and more by itself
-    const size_t piece = std::min(kPiece, std::max<size_t>(512u << 10, (end / 4 + kPart - 1) / kPart * kPart));
-    const size_t begin = seg.front().off, total = end - begin;
-    const long long n_pieces = (long long)((total + piece - 1) / piece), per = (long long)(piece / kPart), n_parts = (long long)((total + kPart - 1) / kPart);
+    const size_t begin = seg.front().off, total = seg.back().off + seg.back().bytes - begin;
+    const long long n_parts = (long long)((total + kPart - 1) / kPart);
     if (n_parts <= 3)
     {
         // (over before other threads are awake)
         unsigned char *p;
         int i;
-        cudaError_t e = slot(&p, &i);
+        cudaError_t e = take(1, &p, &i);
         if (e != cudaSuccess) return e;
         gather(p, begin, total, seg);
         e = cudaMemcpyAsync((unsigned char *)dev + begin, p, total, cudaMemcpyHostToDevice, st);
         return e == cudaSuccess ? cudaEventRecord(done[i], st) : e;
     }
-    // The threads take parts in order; the calling one also sends every piece whose parts are in. A piece is opened (its slot of
+    // Pieces that double: the filling of the first is all that does not overlap with a copy, and a copy costs 3.5 us by itself
+    // (8 MB on this link: 161 us in one copy, 187 in eight). The ring is filled faster than the link empties it.
+    struct Piece
+    {
+        long long part, end; // parts of 64 KB
+        int slots, event = 0;
+        long long at = 0; // slots that the call had taken before, those left free at the ring's end included
+        unsigned char *p = nullptr;
+    };
+    const long long slot_parts = (long long)(kPiece / kPart);
+    std::vector<Piece> pieces;
+    std::vector<int> piece_of((size_t)n_parts);
+    for (long long q = 0, n = kFirstParts; q < n_parts; n = std::min(2 * n, kMostParts))
+    {
+        const long long e = n_parts - q <= n + n / 4 ? n_parts : q + n;
+        std::fill(piece_of.begin() + q, piece_of.begin() + e, (int)pieces.size());
+        pieces.push_back({q, e, (int)((e - q + slot_parts - 1) / slot_parts)});
+        q = e;
+    }
+    // The threads take parts in order; the calling one also sends every piece whose parts are in. A piece is opened (its slots of
     // the ring free again) before its parts may be filled.
-    unsigned char *where[kPieces];
-    int used[kPieces];
-    std::atomic<long long> next_part(0), open_pieces(0);
-    std::atomic<int> filled[kPieces];
-    for (auto &f : filled) f.store(0);
+    std::unique_ptr<std::atomic<int>[]> filled(new std::atomic<int>[pieces.size()]);
+    for (size_t k = 0; k < pieces.size(); k++) filled[k].store(0);
+    std::atomic<long long> next_part(0), open_parts(0);
     std::atomic<bool> stop(false);
     cudaError_t e = cudaSuccess;
-    auto open = [&](long long k) { // by the calling thread only
-        e = slot(&where[k % kPieces], &used[k % kPieces]);
-        filled[k % kPieces].store(0);
-        if (e != cudaSuccess) stop.store(true);
-        else open_pieces.store(k + 1);
+    size_t opened = 0;
+    long long taken = 0;
+    auto open_from = [&](size_t unsent) { // by the calling thread only
+        while (opened < pieces.size() && e == cudaSuccess)
+        {
+            Piece &k = pieces[opened];
+            const long long at = taken + (next + k.slots > kPieces ? kPieces - next : 0);
+            if (opened > unsent && (at + k.slots - pieces[unsent].at > kPieces || !free_now(k.slots))) return;
+            e = take(k.slots, &k.p, &k.event);
+            if (e != cudaSuccess) return;
+            k.at = at;
+            taken = at + k.slots;
+            opened++;
+            open_parts.store(k.end);
+        }
     };
-    auto fill_one = [&]() -> bool { // false: no part to be had now
+    auto fill_one = [&]() { // one part, if there is one to be had now
         long long q = next_part.load();
         do
         {
-            if (q >= n_parts || q / per >= open_pieces.load()) return false;
+            if (q >= open_parts.load()) return;
         } while (!next_part.compare_exchange_weak(q, q + 1));
-        const long long k = q / per;
-        const size_t at = (size_t)(q - k * per) * kPart, o = (size_t)k * piece + at;
-        gather(where[k % kPieces] + at, begin + o, std::min(kPart, total - o), seg);
-        filled[k % kPieces].fetch_add(1);
-        return true;
+        const Piece &k = pieces[piece_of[(size_t)q]];
+        const size_t o = (size_t)q * kPart;
+        gather(k.p + (size_t)(q - k.part) * kPart, begin + o, std::min(kPart, total - o), seg);
+        filled[piece_of[(size_t)q]].fetch_add(1);
     };
-    for (long long k = 0; k < n_pieces && k < kPieces && e == cudaSuccess; k++) open(k);
+    open_from(0);
 #pragma omp parallel
     {
         bool mine = false;
@@ -290,14 +338,14 @@ cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaSt
         mine = true;
         if (mine)
         {
-            for (long long k = 0; k < n_pieces && e == cudaSuccess; k++)
+            for (size_t k = 0; k < pieces.size() && e == cudaSuccess; k++)
             {
-                const long long parts_of = std::min(per, n_parts - k * per);
-                while (filled[k % kPieces].load() < parts_of) fill_one();
-                const size_t o = (size_t)k * piece, n = std::min(piece, total - o);
-                e = cudaMemcpyAsync((unsigned char *)dev + begin + o, where[k % kPieces], n, cudaMemcpyHostToDevice, st);
-                if (e == cudaSuccess) e = cudaEventRecord(done[used[k % kPieces]], st);
-                if (e == cudaSuccess && k + kPieces < n_pieces) open(k + kPieces);
+                const Piece &q = pieces[k];
+                while (filled[k].load() < q.end - q.part) fill_one();
+                const size_t o = (size_t)q.part * kPart, n = std::min((size_t)(q.end - q.part) * kPart, total - o);
+                e = cudaMemcpyAsync((unsigned char *)dev + begin + o, q.p, n, cudaMemcpyHostToDevice, st);
+                if (e == cudaSuccess) e = cudaEventRecord(done[q.event], st);
+                open_from(k + 1);
             }
             stop.store(true);
         }
@@ -319,7 +367,7 @@ cudaError_t Stager::to_host(void *host, const void *dev, size_t bytes, cudaStrea
     int at[kPieces];
     auto send = [&](size_t k) {
         unsigned char *p;
-        e = slot(&p, &at[k % kPieces]);
+        e = take(1, &p, &at[k % kPieces]);
         const size_t o = k * piece;
         if (e == cudaSuccess) e = cudaMemcpyAsync(p, (const unsigned char *)dev + o, std::min(piece, bytes - o), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaEventRecord(done[at[k % kPieces]], st);

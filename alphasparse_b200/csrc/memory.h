@@ -28,13 +28,15 @@ class Stager
     static const int kPieces = 16;
     unsigned char *ring = nullptr;
     cudaEvent_t done[kPieces] = {};
+    int owner[kPieces] = {}; // event that a slot is free after
     bool off = false; // no pinned memory to be had: plain copies
     int next = 0;
 
     bool ready();
     bool pinned(const void *host);
-    // the slot the next piece goes through, free to be written
-    cudaError_t slot(unsigned char **p, int *i);
+    // the adjacent slots that the next piece goes through, free to be written, and the event to record after its copy
+    cudaError_t take(int slots, unsigned char **p, int *event);
+    bool free_now(int slots) const;
 
   public:
     struct Segment
