@@ -701,30 +701,37 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     // WLB's first row until the WLB holds a multiple of 32 TLBs), padded sizes
     std::vector<u64> wlb_S(NW), wlb_tl(NW), wlb_tlb0(NW + 1, 0), wlb_pad0(NW + 1, 0);
     std::vector<u64> blb_first(B.block_num + 1, 0);
-#pragma omp parallel for schedule(static) if (!by_rows && b.col.size() > kParallelNnz)
-    for (u64 w = 0; w < NW; w++)
+    auto count_wlb = [&](u64 w) {
+        const Span s = span(w);
+        u64 S = tlb_size;
+        if (S == 0)
         {
-            const Span s = span(w);
-            u64 S = tlb_size;
-            if (S == 0)
-            {
 #pragma omp parallel for schedule(static) reduction(max : S) if (by_rows && s.rows > kParallelRows)
-                for (u64 r = 0; r < s.rows; r++)
-                {
-                    u64 lo, hi;
-                    S = std::max(S, row_range(s, r, lo, hi));
-                }
-            }
-            u64 tl = 0;
-#pragma omp parallel for schedule(static) reduction(+ : tl) if (by_rows && s.rows > kParallelRows)
             for (u64 r = 0; r < s.rows; r++)
             {
                 u64 lo, hi;
-                tl += (row_range(s, r, lo, hi) + S - 1) / S;
+                S = std::max(S, row_range(s, r, lo, hi));
             }
-            wlb_S[w] = S;
-            wlb_tl[w] = tl;
         }
+        u64 tl = 0;
+#pragma omp parallel for schedule(static) reduction(+ : tl) if (by_rows && s.rows > kParallelRows)
+        for (u64 r = 0; r < s.rows; r++)
+        {
+            u64 lo, hi;
+            tl += (row_range(s, r, lo, hi) + S - 1) / S;
+        }
+        wlb_S[w] = S;
+        wlb_tl[w] = tl;
+    };
+    // (no parallel region, not even one of a single thread, around the loops that share out rows: the threads of a nested
+    // region are made for it and end with it, 0.6 ms each time)
+    if (by_rows)
+        for (u64 w = 0; w < NW; w++) count_wlb(w);
+    else
+    {
+#pragma omp parallel for schedule(static) if (b.col.size() > kParallelNnz)
+        for (u64 w = 0; w < NW; w++) count_wlb(w);
+    }
     u64 max_S = 0;
     for (u64 w = 0; w < NW; w++)
     {
@@ -746,49 +753,58 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     u64 max_thread_first_row = 0;
     bool share_thread = tlb_size != 0;
     // pass 2: fill the padded arrays (row-major inside the WLB) and the per-TLB first rows
-#pragma omp parallel if (!by_rows && b.col.size() > kParallelNnz)
-    {
-        std::vector<u64> first; // first TLB of every row of the WLB, relative to it
-#pragma omp for schedule(static) reduction(max : max_thread_first_row) reduction(|| : share_thread)
-        for (u64 w = 0; w < NW; w++)
-            {
-                const Span s = span(w);
-                const u64 S = wlb_S[w], extra = wlb_tlb0[w + 1] - wlb_tlb0[w] - wlb_tl[w];
-                first.resize(s.rows + 1);
-                u64 *f = first.data();
-                f[0] = 0;
+    // `first`: first TLB of every row of the WLB, relative to it
+    auto fill_wlb = [&](u64 w, std::vector<u64> &first, u64 &top_of_all, bool &shared) {
+        const Span s = span(w);
+        const u64 S = wlb_S[w], extra = wlb_tlb0[w + 1] - wlb_tlb0[w] - wlb_tl[w];
+        first.resize(s.rows + 1);
+        u64 *f = first.data();
+        f[0] = 0;
 #pragma omp parallel for schedule(static) if (by_rows && s.rows > kParallelRows)
-                for (u64 r = 0; r < s.rows; r++)
-                {
-                    u64 lo, hi;
-                    // filler k goes to row k % rows
-                    f[r + 1] = (row_range(s, r, lo, hi) + S - 1) / S + (extra > r ? (extra - r - 1) / s.rows + 1 : 0);
-                }
-                for (u64 r = 0; r < s.rows; r++) f[r + 1] += f[r];
-                u64 top = 0;
-                bool shared_row = false;
+        for (u64 r = 0; r < s.rows; r++)
+        {
+            u64 lo, hi;
+            // filler k goes to row k % rows
+            f[r + 1] = (row_range(s, r, lo, hi) + S - 1) / S + (extra > r ? (extra - r - 1) / s.rows + 1 : 0);
+        }
+        for (u64 r = 0; r < s.rows; r++) f[r + 1] += f[r];
+        u64 top = 0;
+        bool shared_row = false;
 #pragma omp parallel for schedule(static) reduction(max : top) reduction(|| : shared_row) if (by_rows && (wlb_pad0[w + 1] - wlb_pad0[w]) * es > kParallelBytes)
-                for (u64 r = 0; r < s.rows; r++)
-                {
-                    u64 lo, hi;
-                    const u64 n = row_range(s, r, lo, hi), tlbs = f[r + 1] - f[r], tgt = tlbs * S, out = wlb_pad0[w] + f[r] * S;
-                    u32 fill = (u32)b.min_col;
-                    if (n > 0)
-                    {
-                        memcpy(pcol + out, b.col.data() + lo, n * sizeof(u32));
-                        memcpy(pval + out * es, b.val.b.data() + lo * es, n * es);
-                        fill = b.col[hi - 1];
-                    }
-                    for (u64 k = n; k < tgt; k++) pcol[out + k] = fill; // with value 0
-                    memset(pval + (out + n) * es, 0, (tgt - n) * es);
-                    if (tlbs >= 2) shared_row = true;
-                    if (trow)
-                        for (u64 k = 0; k < tlbs; k++) trow[wlb_tlb0[w] + f[r] + k] = (u32)r;
-                    if (tlbs > 0) top = std::max(top, r);
-                }
-                share_thread = share_thread || shared_row;
-                max_thread_first_row = std::max(max_thread_first_row, top);
+        for (u64 r = 0; r < s.rows; r++)
+        {
+            u64 lo, hi;
+            const u64 n = row_range(s, r, lo, hi), tlbs = f[r + 1] - f[r], tgt = tlbs * S, out = wlb_pad0[w] + f[r] * S;
+            u32 fill = (u32)b.min_col;
+            if (n > 0)
+            {
+                memcpy(pcol + out, b.col.data() + lo, n * sizeof(u32));
+                memcpy(pval + out * es, b.val.b.data() + lo * es, n * es);
+                fill = b.col[hi - 1];
             }
+            for (u64 k = n; k < tgt; k++) pcol[out + k] = fill; // with value 0
+            memset(pval + (out + n) * es, 0, (tgt - n) * es);
+            if (tlbs >= 2) shared_row = true;
+            if (trow)
+                for (u64 k = 0; k < tlbs; k++) trow[wlb_tlb0[w] + f[r] + k] = (u32)r;
+            if (tlbs > 0) top = std::max(top, r);
+        }
+        shared = shared || shared_row;
+        top_of_all = std::max(top_of_all, top);
+    };
+    if (by_rows)
+    {
+        std::vector<u64> first;
+        for (u64 w = 0; w < NW; w++) fill_wlb(w, first, max_thread_first_row, share_thread);
+    }
+    else
+    {
+#pragma omp parallel if (b.col.size() > kParallelNnz)
+        {
+            std::vector<u64> first;
+#pragma omp for schedule(static) reduction(max : max_thread_first_row) reduction(|| : share_thread)
+            for (u64 w = 0; w < NW; w++) fill_wlb(w, first, max_thread_first_row, share_thread);
+        }
     }
     u64 max_w_coo_begin = 0, max_w_size = 0;
     std::vector<u64> new_w_begin(NW), new_w_size(NW);

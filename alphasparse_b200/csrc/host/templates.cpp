@@ -214,15 +214,22 @@ Arr<u64> tlb_global_rows(const CompressedBlock &b, bool &adjacent_equal)
     const Level &B = b.blb, &W = b.wlb, &T = b.tlb;
     Arr<u64> out;
     u64 *rows = out.make(T.block_num);
-    const bool by_rows = B.block_num < 256; // few BLBs: the TLBs are shared out, else the BLBs
-#pragma omp parallel for schedule(dynamic, 64) if (!by_rows && T.block_num > kParallelRows)
-    for (u64 i = 0; i < B.block_num; i++)
-        for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++)
-        {
-            const u64 base = B.first_row.v[i] + W.first_row.v[w], t0 = W.index.v[w], t1 = W.index.v[w + 1];
-#pragma omp parallel for schedule(static) if (by_rows && t1 - t0 > kParallelRows)
-            for (u64 t = t0; t < t1; t++) rows[t] = base + b.tlb_row[t];
-        }
+    auto of_wlb = [&](u64 i, u64 w, bool share) {
+        const u64 base = B.first_row.v[i] + W.first_row.v[w], t0 = W.index.v[w], t1 = W.index.v[w + 1];
+#pragma omp parallel for schedule(static) if (share && t1 - t0 > kParallelRows)
+        for (u64 t = t0; t < t1; t++) rows[t] = base + b.tlb_row[t];
+    };
+    if (B.block_num < 256) // few BLBs: the TLBs are shared out (and no parallel region is around that), else the BLBs
+    {
+        for (u64 i = 0; i < B.block_num; i++)
+            for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w, true);
+    }
+    else
+    {
+#pragma omp parallel for schedule(dynamic, 64) if (T.block_num > kParallelRows)
+        for (u64 i = 0; i < B.block_num; i++)
+            for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w, false);
+    }
     adjacent_equal = T.block_num > 1 && !all_of(T.block_num - 1, [&](u64 t) { return rows[t] != rows[t + 1]; });
     return out;
 }
