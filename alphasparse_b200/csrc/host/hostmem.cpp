@@ -2,7 +2,6 @@
 
 #include <sys/mman.h>
 
-#include <map>
 #include <mutex>
 #include <vector>
 
@@ -17,8 +16,7 @@ const size_t kHuge = 2u << 20, kMostIdle = 256u << 20;
 struct Pool
 {
     std::mutex lock;
-    std::multimap<size_t, void *> idle; // by size
-    size_t bytes = 0;
+    IdleBlocks idle;
 };
 Pool &pool()
 {
@@ -29,29 +27,24 @@ Pool &pool()
 void give_back(void *p, size_t size)
 {
     Pool &q = pool();
+    std::vector<void *> out;
     {
         std::lock_guard<std::mutex> g(q.lock);
-        if (q.bytes + size <= kMostIdle)
-        {
-            q.idle.insert({size, p});
-            q.bytes += size;
-            return;
-        }
+        q.idle.put(p, size, kMostIdle, out);
     }
-    free(p);
+    for (void *o : out) free(o);
 }
 } // namespace
 
 void host_pool_trim()
 {
     Pool &q = pool();
-    std::multimap<size_t, void *> idle;
+    std::vector<void *> idle;
     {
         std::lock_guard<std::mutex> g(q.lock);
-        idle.swap(q.idle);
-        q.bytes = 0;
+        q.idle.take_all(idle);
     }
-    for (auto &b : idle) free(b.second);
+    for (void *p : idle) free(p);
 }
 
 std::shared_ptr<void> big_buffer(size_t bytes)
@@ -68,14 +61,7 @@ std::shared_ptr<void> big_buffer(size_t bytes)
     {
         Pool &q = pool();
         std::lock_guard<std::mutex> g(q.lock);
-        auto it = q.idle.lower_bound(want);
-        if (it != q.idle.end() && it->first <= want + want / 4 + kHuge)
-        {
-            size = it->first;
-            p = it->second;
-            q.bytes -= size;
-            q.idle.erase(it);
-        }
+        p = q.idle.take(want, kHuge, &size);
     }
     if (!p && posix_memalign(&p, kHuge, want) != 0)
     {

@@ -12,15 +12,66 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <map>
 #include <memory>
 #include <new>
+#include <vector>
 
 namespace asp
 {
 namespace host
 {
+// Blocks that nobody uses, kept for a later request of about their size. The caller locks.
+class IdleBlocks
+{
+    struct Block
+    {
+        void *p;
+        uint64_t since;
+    };
+    std::multimap<size_t, Block> by_size;
+    size_t bytes = 0;
+    uint64_t clock = 0;
+
+  public:
+    // the smallest block of want to 1.25 want + unit bytes, or NULL
+    void *take(size_t want, size_t unit, size_t *size)
+    {
+        auto it = by_size.lower_bound(want);
+        if (it == by_size.end() || it->first > want + want / 4 + unit) return nullptr;
+        void *p = it->second.p;
+        *size = it->first;
+        bytes -= it->first;
+        by_size.erase(it);
+        return p;
+    }
+    // keeps the block; those that this takes beyond `most` bytes in all, longest idle first, are appended to `out`: without that,
+    // blocks of sizes that are not asked for again would fill the pool for good
+    void put(void *p, size_t size, size_t most, std::vector<void *> &out)
+    {
+        if (size > most) return out.push_back(p);
+        by_size.insert({size, {p, clock++}});
+        bytes += size;
+        while (bytes > most)
+        {
+            auto old = by_size.begin();
+            for (auto it = by_size.begin(); it != by_size.end(); ++it)
+                if (it->second.since < old->second.since) old = it;
+            out.push_back(old->second.p);
+            bytes -= old->first;
+            by_size.erase(old);
+        }
+    }
+    void take_all(std::vector<void *> &out)
+    {
+        for (auto &b : by_size) out.push_back(b.second.p);
+        by_size.clear();
+        bytes = 0;
+    }
+};
+
 // Large buffers come from a pool (hostmem.cpp): a fresh one costs a page fault per 2 MB, zeroed by the kernel at 5 to 20 GB/s, which
-// is several times what the operators do with it. Idle buffers are bounded (256 MB in all) and given back with host_pool_trim().
+// is several times what the operators do with it. Idle buffers are bounded (256 MB in all, the longest idle ones go first) and given back with host_pool_trim().
 std::shared_ptr<void> big_buffer(size_t bytes);
 void host_pool_trim();
 

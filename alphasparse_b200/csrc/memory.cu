@@ -9,7 +9,6 @@
 #include <atomic>
 
 #include <algorithm>
-#include <map>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -25,8 +24,7 @@ const size_t kMostBlock = 256u << 20, kMostCached = 1u << 30;
 struct Pool
 {
     std::mutex lock;
-    std::multimap<size_t, void *> idle; // by size
-    size_t cached = 0;
+    host::IdleBlocks idle;
     int contexts = 0;
 };
 const int kMaxDevices = 64;
@@ -50,15 +48,6 @@ struct OnDevice
         if (prev >= 0) cudaSetDevice(prev);
     }
 };
-
-std::vector<void *> take_all(Pool &p)
-{
-    std::vector<void *> out;
-    for (auto &b : p.idle) out.push_back(b.second);
-    p.idle.clear();
-    p.cached = 0;
-    return out;
-}
 
 // Into pinned memory that the copy engine reads next: past the caches, where it would have to snoop every line out of another
 // core's (8 MB filled and sent: 284 us with memcpy, 208 us so).
@@ -107,15 +96,8 @@ cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got)
     Pool &p = pool(device);
     {
         std::lock_guard<std::mutex> g(p.lock);
-        auto it = p.idle.lower_bound(want);
-        if (it != p.idle.end() && it->first <= want + want / 4 + unit)
-        {
-            *out = it->second;
-            *got = it->first;
-            p.cached -= it->first;
-            p.idle.erase(it);
-            return cudaSuccess;
-        }
+        *out = p.idle.take(want, unit, got);
+        if (*out) return cudaSuccess;
     }
     OnDevice on(device);
     cudaError_t e = cudaMalloc(out, want);
@@ -125,7 +107,7 @@ cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got)
         std::vector<void *> idle;
         {
             std::lock_guard<std::mutex> g(p.lock);
-            idle = take_all(p);
+            p.idle.take_all(idle);
         }
         for (void *q : idle) cudaFree(q);
         e = cudaMalloc(out, want);
@@ -139,17 +121,16 @@ void device_free(int device, void *ptr, size_t got)
     if (!ptr) return;
     OnDevice on(device);
     Pool &p = pool(device);
+    std::vector<void *> out;
     if (got <= kMostBlock && cudaDeviceSynchronize() == cudaSuccess)
     {
         std::lock_guard<std::mutex> g(p.lock);
-        if (p.contexts > 0 && p.cached + got <= kMostCached)
-        {
-            p.idle.insert({got, ptr});
-            p.cached += got;
-            return;
-        }
+        if (p.contexts > 0) p.idle.put(ptr, got, kMostCached, out);
+        else out.push_back(ptr);
     }
-    cudaFree(ptr);
+    else
+        out.push_back(ptr);
+    for (void *q : out) cudaFree(q);
 }
 
 void device_pool_retain(int device)
@@ -166,7 +147,7 @@ void device_pool_release(int device)
     {
         std::lock_guard<std::mutex> g(p.lock);
         if (--p.contexts > 0) return;
-        idle = take_all(p);
+        p.idle.take_all(idle);
     }
     OnDevice on(device);
     for (void *q : idle) cudaFree(q);
