@@ -703,28 +703,32 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     std::vector<u64> blb_first(B.block_num + 1, 0);
     auto count_wlb = [&](u64 w) {
         const Span s = span(w);
-        u64 S = tlb_size;
-        if (S == 0)
-        {
-#pragma omp parallel for schedule(static) reduction(max : S) if (by_rows && s.rows > kParallelRows)
-            for (u64 r = 0; r < s.rows; r++)
-            {
-                u64 lo, hi;
-                S = std::max(S, row_range(s, r, lo, hi));
-            }
-        }
-        u64 tl = 0;
-#pragma omp parallel for schedule(static) reduction(+ : tl) if (by_rows && s.rows > kParallelRows)
-        for (u64 r = 0; r < s.rows; r++)
-        {
+        const bool share = by_rows && s.rows > kParallelRows;
+        u64 S = tlb_size, tl = 0;
+        auto length = [&](u64 r) {
             u64 lo, hi;
-            tl += (row_range(s, r, lo, hi) + S - 1) / S;
+            return row_range(s, r, lo, hi);
+        };
+        if (S == 0 && share)
+        {
+#pragma omp parallel for schedule(static) reduction(max : S)
+            for (u64 r = 0; r < s.rows; r++) S = std::max(S, length(r));
         }
+        else if (S == 0)
+            for (u64 r = 0; r < s.rows; r++) S = std::max(S, length(r));
+        if (share)
+        {
+#pragma omp parallel for schedule(static) reduction(+ : tl)
+            for (u64 r = 0; r < s.rows; r++) tl += (length(r) + S - 1) / S;
+        }
+        else
+            for (u64 r = 0; r < s.rows; r++) tl += (length(r) + S - 1) / S;
         wlb_S[w] = S;
         wlb_tl[w] = tl;
     };
     // (no parallel region, not even one of a single thread, around the loops that share out rows: the threads of a nested
-    // region are made for it and end with it, 0.6 ms each time)
+    // region are made for it and end with it, 0.6 ms each time; and none inside the loops over many WLBs: 0.4 us each, more when
+    // all threads start them)
     if (by_rows)
         for (u64 w = 0; w < NW; w++) count_wlb(w);
     else
@@ -760,19 +764,15 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
         first.resize(s.rows + 1);
         u64 *f = first.data();
         f[0] = 0;
-#pragma omp parallel for schedule(static) if (by_rows && s.rows > kParallelRows)
-        for (u64 r = 0; r < s.rows; r++)
-        {
+        for_each(s.rows, by_rows && s.rows > kParallelRows, [&](u64 r) {
             u64 lo, hi;
             // filler k goes to row k % rows
             f[r + 1] = (row_range(s, r, lo, hi) + S - 1) / S + (extra > r ? (extra - r - 1) / s.rows + 1 : 0);
-        }
+        });
         for (u64 r = 0; r < s.rows; r++) f[r + 1] += f[r];
         u64 top = 0;
         bool shared_row = false;
-#pragma omp parallel for schedule(static) reduction(max : top) reduction(|| : shared_row) if (by_rows && (wlb_pad0[w + 1] - wlb_pad0[w]) * es > kParallelBytes)
-        for (u64 r = 0; r < s.rows; r++)
-        {
+        auto fill_row = [&](u64 r, u64 &top_out, bool &shared_out) {
             u64 lo, hi;
             const u64 n = row_range(s, r, lo, hi), tlbs = f[r + 1] - f[r], tgt = tlbs * S, out = wlb_pad0[w] + f[r] * S;
             u32 fill = (u32)b.min_col;
@@ -784,11 +784,18 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
             }
             for (u64 k = n; k < tgt; k++) pcol[out + k] = fill; // with value 0
             memset(pval + (out + n) * es, 0, (tgt - n) * es);
-            if (tlbs >= 2) shared_row = true;
+            if (tlbs >= 2) shared_out = true;
             if (trow)
                 for (u64 k = 0; k < tlbs; k++) trow[wlb_tlb0[w] + f[r] + k] = (u32)r;
-            if (tlbs > 0) top = std::max(top, r);
+            if (tlbs > 0) top_out = std::max(top_out, r);
+        };
+        if (by_rows && (wlb_pad0[w + 1] - wlb_pad0[w]) * es > kParallelBytes)
+        {
+#pragma omp parallel for schedule(static) reduction(max : top) reduction(|| : shared_row)
+            for (u64 r = 0; r < s.rows; r++) fill_row(r, top, shared_row);
         }
+        else
+            for (u64 r = 0; r < s.rows; r++) fill_row(r, top, shared_row);
         shared = shared || shared_row;
         top_of_all = std::max(top_of_all, top);
     };

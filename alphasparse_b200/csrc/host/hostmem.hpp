@@ -79,6 +79,19 @@ void host_pool_trim();
 // a busy host, as much as the loop itself.
 const size_t kParallelBytes = 4u << 20;
 const uint64_t kParallelRows = 1u << 18, kParallelNnz = 1u << 19;
+// f(i) for i in [0, n), shared out among the threads or without a parallel region at all (an inactive one costs 0.4 us, too much
+// for what is done per block)
+template <class F>
+void for_each(uint64_t n, bool share, F &&f)
+{
+    if (share)
+    {
+#pragma omp parallel for schedule(static)
+        for (uint64_t i = 0; i < n; i++) f(i);
+    }
+    else
+        for (uint64_t i = 0; i < n; i++) f(i);
+}
 
 inline void par_copy(void *dst, const void *src, size_t bytes)
 {

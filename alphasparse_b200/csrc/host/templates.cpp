@@ -167,13 +167,11 @@ template <class D, class S_>
 void interleave_strip(D *dst, const S_ *src, u64 n, u64 S)
 {
     const u64 TB = 256;
-#pragma omp parallel for schedule(static) if (n * S > kParallelNnz)
-    for (u64 i0 = 0; i0 < n; i0 += TB)
-    {
-        const u64 i1 = std::min(n, i0 + TB);
+    for_each((n + TB - 1) / TB, n * S > kParallelNnz, [=](u64 b) {
+        const u64 i0 = b * TB, i1 = std::min(n, i0 + TB);
         for (u64 k = 0; k < S; k++)
             for (u64 i = i0; i < i1; i++) dst[k * n + i] = (D)src[i * S + k];
-    }
+    });
 }
 
 void interleave_cols(uint8_t *dst, int col_dt, const u32 *src, u64 n, u64 S)
@@ -216,8 +214,7 @@ Arr<u64> tlb_global_rows(const CompressedBlock &b, bool &adjacent_equal)
     u64 *rows = out.make(T.block_num);
     auto of_wlb = [&](u64 i, u64 w, bool share) {
         const u64 base = B.first_row.v[i] + W.first_row.v[w], t0 = W.index.v[w], t1 = W.index.v[w + 1];
-#pragma omp parallel for schedule(static) if (share && t1 - t0 > kParallelRows)
-        for (u64 t = t0; t < t1; t++) rows[t] = base + b.tlb_row[t];
+        for_each(t1 - t0, share && t1 - t0 > kParallelRows, [&](u64 t) { rows[t0 + t] = base + b.tlb_row[t0 + t]; });
     };
     if (B.block_num < 256) // few BLBs: the TLBs are shared out (and no parallel region is around that), else the BLBs
     {
@@ -459,24 +456,28 @@ void staggered_arrays(const CompressedBlock &b, Arr<uint8_t> &col, Arr<uint8_t> 
     }
     uint8_t *cp = col.make(n_pad * cb), *vp = val.make(n_pad * es);
     const u64 nb = B.block_num;
-    const bool by_rows = nb < 256;
-#pragma omp parallel for schedule(dynamic, 64) if (!by_rows && n_pad > kParallelNnz)
-    for (u64 i = 0; i < nb; i++)
-    {
-        const u64 w0 = B.index.v[i], w1 = B.index.v[i + 1];
-#pragma omp parallel for schedule(dynamic, 256) if (by_rows && w1 - w0 > 1024)
-        for (u64 w = w0; w < w1; w++)
+    auto of_wlb = [&](u64 i, u64 w) {
+        const u64 S = b.tlb.coo_size.v[w];
+        const u64 base = B.coo_begin.v[i] + W.coo_begin.v[w];
+        const u64 groups = (W.index.v[w + 1] - W.index.v[w]) / 32;
+        for (u64 g = 0; g < groups; g++)
         {
-            const u64 S = b.tlb.coo_size.v[w];
-            const u64 base = B.coo_begin.v[i] + W.coo_begin.v[w];
-            const u64 groups = (W.index.v[w + 1] - W.index.v[w]) / 32;
-            for (u64 g = 0; g < groups; g++)
-            {
-                const u64 o = base + g * 32 * S;
-                interleave_cols(cp + o * cb, b.col_dt, b.pad_col.data() + o, 32, S);
-                interleave_vals(vp + o * es, es, b.pad_val.b.data() + o * es, 32, S);
-            }
+            const u64 o = base + g * 32 * S;
+            interleave_cols(cp + o * cb, b.col_dt, b.pad_col.data() + o, 32, S);
+            interleave_vals(vp + o * es, es, b.pad_val.b.data() + o * es, 32, S);
         }
+    };
+    if (nb < 256)
+        for (u64 i = 0; i < nb; i++)
+        {
+            const u64 w0 = B.index.v[i], w1 = B.index.v[i + 1];
+            for_each(w1 - w0, w1 - w0 > 1024, [&](u64 w) { of_wlb(i, w0 + w); });
+        }
+    else
+    {
+#pragma omp parallel for schedule(dynamic, 64) if (n_pad > kParallelNnz)
+        for (u64 i = 0; i < nb; i++)
+            for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w);
     }
 }
 
