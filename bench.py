@@ -434,7 +434,7 @@ def run_c5(args, rank, world, local_rank, dist):
                        "values": "x grows by about 8x per SpMV and overflows fp32 after ~40 of the 100: the later SpMVs multiply inf / NaN (same memory traffic); parity is checked on the first SpMV"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak * world, "unit": "GB/s", "frac": achieved / (peak * world), "traffic": profiled_traffic("c5", r["graph"]) if (world == 1 and args.scale == 26 and args.relabel == "indegree") else None,
                          "peak_kind": peak_kind, "algorithmic_bytes": b_alg, "launch": f"{iters} SpMV launches per step; peak = {world} x the measured copy bandwidth",
-                         "note": "the gathers of x are bound by cache-line look-ups per SM (one per clock), not by DRAM: see profiles/"},
+                         "note": "column-tiled layout on one GPU: x is gathered from tiles in shared memory, 6 of the 8 algorithmic bytes per non-zero are read; the CSR5-like kernels of the sharded loop are bound by cache-line look-ups per SM (one per clock), see profiles/"},
             "gpu_launches": int(K * iters * r["launches_per_spmv"]),
             "clocks": clocks, "parity_max_rel_err": r["parity"],
         }
