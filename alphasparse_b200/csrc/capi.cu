@@ -7,8 +7,10 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -98,6 +100,7 @@ using asp::HostMeta;
 struct asp_ctx
 {
     int device = 0;
+    uint64_t serial = 0; // of this context, never given to another one
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // side streams: the sub-matrix kernels of one SpMV run concurrently (the reference gives every
@@ -127,6 +130,11 @@ struct TiledGroup
     size_t layout_bytes = 0;
     unsigned n_sm = 0;
     bool covers_all_rows = false; // every row of y has an element in some plan
+    // Sums of rows belong to the calls of one context (its stream keeps them in order); `lock` holds the launches of a call
+    // together, and sums that a failed launch left behind end the use of the layout.
+    uint64_t owner = 0; // asp_ctx::serial
+    std::mutex lock;
+    bool spoilt = false;
 };
 } // namespace
 
@@ -535,7 +543,9 @@ asp_status asp_ctx_create(int device, asp_ctx **out)
     if (guard.err != cudaSuccess) return cuda_fail(guard.err, "cudaSetDevice");
     asp_ctx *c = new (std::nothrow) asp_ctx();
     if (!c) return fail(ASP_ERR_ALLOC, "host allocation failed");
+    static std::atomic<uint64_t> contexts{0};
     c->device = device;
+    c->serial = ++contexts;
     asp::device_pool_retain(device);
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
@@ -1079,11 +1089,13 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
     }
     if (tg)
     {
-        const void *from[5] = {th.val.p, th.col.p, th.row.p, th.end.p, th.work.data()};
-        const size_t bytes[5] = {th.val.bytes(), th.col.bytes(), th.row.bytes(), th.end.bytes(), th.work.size() * sizeof(uint32_t)};
-        size_t off[6] = {0};
-        for (int k = 0; k < 5; k++) off[k + 1] = align_up(off[k] + bytes[k], 256);
-        if (tg->arena.make(ctx->device, off[5]) != cudaSuccess)
+        const void *from[6] = {th.val.p, th.col.p, th.row.p, th.end.p, th.work.data(), th.parts.data()};
+        const size_t bytes[6] = {th.val.bytes(), th.col.bytes(), th.row.bytes(), th.end.bytes(), th.work.size() * sizeof(uint32_t), th.parts.size() * sizeof(uint32_t)};
+        size_t off[7] = {0};
+        for (int k = 0; k < 6; k++) off[k + 1] = align_up(off[k] + bytes[k], 256);
+        const uint64_t sum_stride = align_up(th.n_parts, 32);
+        const size_t sum_bytes = (size_t)th.copies * sum_stride * sizeof(double);
+        if (tg->arena.make(ctx->device, off[6] + sum_bytes) != cudaSuccess)
         {
             cudaGetLastError(); // no room on the device: as above
             tg.reset();
@@ -1092,18 +1104,21 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
         {
             unsigned char *base = (unsigned char *)tg->arena.base;
             std::vector<asp::Stager::Segment> seg;
-            for (int k = 0; k < 5; k++)
+            for (int k = 0; k < 6; k++)
                 if (bytes[k]) seg.push_back({off[k], from[k], bytes[k]});
             cudaError_t ce = asp::tiled_setup(descs[0].val_dtype == ASP_F64);
             if (ce == cudaSuccess) ce = ctx->stager.to_device(base, seg, ctx->stream);
+            if (ce == cudaSuccess && sum_bytes) ce = cudaMemsetAsync(base + off[6], 0, sum_bytes, ctx->stream);
             if (ce != cudaSuccess)
             {
                 cleanup();
                 return cuda_fail(ce, "upload of the column-tiled layout");
             }
-            tg->layout_bytes = off[5];
+            tg->layout_bytes = off[6] + sum_bytes;
+            tg->owner = ctx->serial;
             tg->args = {base + off[0], (const uint16_t *)(base + off[1]), (const uint32_t *)(base + off[2]), (const uint32_t *)(base + off[3]),
-                        (const uint4 *)(base + off[4]), nullptr, nullptr, descs[0].n_rows, descs[0].n_cols};
+                        (const uint4 *)(base + off[4]), th.parts.empty() ? nullptr : (const uint32_t *)(base + off[5]), (double *)(base + off[6]), (unsigned)th.n_parts, th.copies, sum_stride,
+                        th.direct, nullptr, nullptr, descs[0].n_rows, descs[0].n_cols};
             tg->n_plans = n;
             tg->n_sm = (unsigned)ctx->sm_count;
             tg->covers_all_rows = th.covers_all_rows;
@@ -1266,7 +1281,7 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
     }
     // The whole group in its column-tiled layout. That writes every row of y, so it stands in for the templates' kernels where
     // y is cleared first anyway, or where they would store every row.
-    const TiledGroup *tg = plans[0]->tiled.get();
+    TiledGroup *tg = plans[0]->tiled.get();
     if (tg && n_plans == tg->n_plans && (clear || (tg->covers_all_rows && zero_y == 2)))
     {
         bool whole = true;
@@ -1275,13 +1290,28 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
             whole = whole && plans[i]->tiled.get() == tg;
             for (int j = 0; j < i; j++) whole = whole && plans[i] != plans[j];
         }
+        if (whole && tg->args.n_parts > 0)
+        {
+            // sums of rows are the group's: calls of another context, and those of a graph, which may run beside this context's
+            // stream, take the templates' kernels
+            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+            ASP_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
+            whole = tg->owner == ctx->serial && capture == cudaStreamCaptureStatusNone;
+        }
         if (whole)
         {
             asp::TiledArgs args = tg->args;
             args.x = d_x;
             args.y = d_y;
-            ASP_CUDA(asp::launch_tiled(g.es == 8, args, tg->n_sm, ctx->stream));
-            return ASP_OK;
+            std::lock_guard<std::mutex> together(tg->lock);
+            if (!tg->spoilt)
+            {
+                ASP_CUDA(asp::launch_tiled_sums(g.es == 8, args, tg->n_sm, ctx->stream));
+                const cudaError_t e = args.n_parts > 0 ? asp::launch_tiled_rows(g.es == 8, args, tg->n_sm, ctx->stream) : cudaSuccess;
+                tg->spoilt = e != cudaSuccess;
+                ASP_CUDA(e);
+                return ASP_OK;
+            }
         }
     }
     const asp_plan *only = n_plans == 1 ? plans[0] : nullptr;

@@ -212,6 +212,23 @@ double slowness(const TiledSource &s)
     return s.templ == ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE ? 1.45 : s.templ == ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE ? 2.35 : 1.1;
 }
 
+// How many parts of a row may be added up in y itself: as many as its template's thread adds elements one after the other, so
+// that the rounding errors of the parts are no more than those of the elements; 8 where a tree follows the thread's few elements
+// (K4, K6, K7, K8 leave about seven roundings in a row of 80). R-MAT scale 20, fp32, TLBs of 32, distance from the 64-bit result:
+// the template 4.9e-8 to 5.9e-8; all rows direct 13e-8; limit 128: 4.9e-8, 32: 3.4e-8, 8: 2.4e-8 (scale 21, ten SpMVs: 485, 490, 505 and
+// 530 us).
+u64 most_direct(const TiledSource &s)
+{
+    u64 tlb = 0;
+    if (s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || is_csr5(s)) tlb = s.a->tlb_size;
+    else if (s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS || s.templ == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS)
+        for (u64 b = 0; b < s.a->n_units; b++) tlb = std::max<u64>(tlb, s.m[MS_TLB_SIZE].get(b));
+    return std::max<u64>(8, tlb);
+}
+// a part's share of what its row may have (sub-matrices of one row may allow different numbers)
+const u32 kDirectShares = 256;
+u32 share_of_part(const TiledSource &s) { return (u32)std::max<u64>(1, (kDirectShares + most_direct(s) - 1) / most_direct(s)); }
+
 const u32 kMaxPiece = 32;    // elements of a row's piece: bounds the serial chain of a lane and the padding of a slice
 const u32 kWindow = 1024;    // pieces that are sorted by length together: lanes of a slice stay near in y
 const double kSliceCost = 4.0; // in steps; with 2 the CTAs of sparse tiles ran twice as long as the others
@@ -235,6 +252,7 @@ struct Builder
     std::vector<u64> at; // [chunk * C + tile]: first its count, then where its elements go
     std::vector<u64> tile_begin, tile_pieces;
     u64 N = 0;
+    std::vector<u32> row_code; // of every row of y: the shares of its parts, then what stands for it among the slices' rows
     // elements in tile order
     HostBuf<u32> e_row;
     HostBuf<uint16_t> e_col;
@@ -242,7 +260,7 @@ struct Builder
 
     Builder(const std::vector<TiledSource> &s, u64 rows, u64 cols) : src(s), n_rows(rows), n_cols(cols), C((cols + TW - 1) / TW) {}
 
-    void count(bool &covered)
+    void count()
     {
         u64 stored = 0;
         for (const TiledSource &s : src) stored += s.stored;
@@ -254,7 +272,9 @@ struct Builder
         }
         at.assign(chunks.size() * C, 0);
         tile_pieces.assign(C, 0);
-        std::vector<uint8_t> seen(n_rows, 0);
+        row_code.assign(n_rows, 0);
+        std::vector<u32> share;
+        for (const TiledSource &s : src) share.push_back(share_of_part(s));
 #pragma omp parallel
         {
             std::vector<u64> pieces(C, 0), n(C); // (counters of a thread's own: neighbours in `at` share cache lines)
@@ -263,28 +283,32 @@ struct Builder
             {
                 std::fill(n.begin(), n.end(), 0);
                 u64 row = ~0ull, tile = ~0ull, run = 0;
+                u32 of_row = 0; // pieces since the row changed
+                auto row_ends = [&]() {
+                    // (several threads may have elements of a row)
+                    if (of_row) __atomic_fetch_add(&row_code[row], std::min(of_row, 1u << 16) * share[chunks[c].sub], __ATOMIC_RELAXED);
+                    of_row = 0;
+                };
                 walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT) {
                     const u64 t = (u32)col / TW;
                     n[t]++;
                     if (r != row || t != tile || run == kMaxPiece)
                     {
                         pieces[t]++;
-                        seen[r] = 1; // (several threads may store the same 1)
+                        if (r != row) row_ends();
+                        of_row++;
                         row = r;
                         tile = t;
                         run = 0;
                     }
                     run++;
                 });
+                row_ends();
                 std::copy(n.begin(), n.end(), at.begin() + (size_t)c * C);
             }
 #pragma omp critical
             for (u64 t = 0; t < C; t++) tile_pieces[t] += pieces[t];
         }
-        u64 missing = 0;
-#pragma omp parallel for schedule(static) reduction(+ : missing)
-        for (long long r = 0; r < (long long)n_rows; r++) missing += seen[r] ? 0 : 1;
-        covered = missing == 0;
         tile_begin.assign(C + 1, 0);
         u64 sum = 0;
         for (u64 t = 0; t < C; t++)
@@ -298,6 +322,46 @@ struct Builder
             }
         }
         tile_begin[C] = N = sum;
+    }
+
+    // which rows y takes itself and which have 64-bit sums
+    void choose_sums(TiledHost &out)
+    {
+        u64 missing = 0, direct = 0, shares = 0;
+#pragma omp parallel for schedule(static) reduction(+ : missing, direct, shares)
+        for (long long r = 0; r < (long long)n_rows; r++)
+        {
+            if (row_code[r] == 0) missing++;
+            else if (row_code[r] <= kDirectShares) direct++;
+            else shares += row_code[r];
+        }
+        const u64 rows = n_rows - missing - direct;
+        out.covers_all_rows = missing == 0;
+        // fp64: at most half of what may be added up directly goes to one sum of a row, on average
+        if (sizeof(VT) == 8)
+            while (out.copies < 16 && shares > kDirectShares / 2 * (u64)out.copies * rows) out.copies *= 2;
+        // where some rows have sums, the others do better with sums, too, than with one more launch that clears y, unless they are
+        // many: 400,000 rows, fp32: 25 -> 21 us; R-MAT scale 21: 50 -> 56 us (a `red` of 64 bits costs more than one of 32)
+        const double sums_us = (double)(n_rows - rows) * (16.0 * out.copies + sizeof(VT)) / 2.0e6, clear_us = 4.0 + (double)n_rows * sizeof(VT) / 6.0e6;
+        out.n_parts = rows == 0 || sums_us > clear_us ? rows : n_rows;
+        out.direct = out.n_parts < n_rows;
+        if (out.direct) out.parts.resize(rows);
+    }
+    void number_rows(TiledHost &out)
+    {
+        if (!out.direct)
+        {
+#pragma omp parallel for schedule(static)
+            for (long long r = 0; r < (long long)n_rows; r++) row_code[r] = kTiledInParts | (u32)r;
+            return;
+        }
+        u32 k = 0;
+        for (u64 r = 0; r < n_rows; r++)
+        {
+            const bool in_parts = row_code[r] > kDirectShares;
+            if (in_parts) out.parts[k] = (u32)r;
+            row_code[r] = in_parts ? kTiledInParts | k++ : (u32)r;
+        }
     }
 
     void scatter()
@@ -425,7 +489,7 @@ struct Builder
                         rows[o] = kTiledNoRow;
                         if (i + j >= p.size()) continue;
                         const u64 e = blocks[b].e0 + p[i + j].start;
-                        rows[o] = e_row.p[e];
+                        rows[o] = row_code[e_row.p[e]];
                         for (u32 k = 0; k < p[i + j].len; k++)
                         {
                             v[k * kTiledSlice + o] = e_val.p[e + k];
@@ -555,16 +619,18 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     double lines = 0;
     for (const TiledSource &s : src) lines += lines_per_gather(s, sizeof(VT) == 8) * (double)s.stored * slowness(s);
     const double own_us = own(lines);
-    // This layout: launches and tail, the first tile of x, 2 + sv bytes per element at 4.6 TB/s, a `red` per piece (below).
+    // This layout: launches and tail, the first tile of x, 2 + sv bytes per element at 4.6 TB/s, a `red` per piece (below), y
+    // cleared, the sums of the rows in many parts.
     auto tiled_us = [&](u64 n, u64 pieces, double red) {
         return 4.5 + 2.5 * std::min(1.0, (double)n_cols / (double)tiled_tile_cols(sizeof(VT) == 8)) + (double)n * (sv + 2) / 4.6e6 + (double)pieces * 4 / 4.6e6 + red / 200e3 +
-               (double)n_rows * sv / 6.0e6;
+               ((double)n_rows * sv + (double)out.n_parts * 16.0 * out.copies) / 6.0e6 + (out.n_parts > 0 && out.direct ? 4.0 : 0.0);
     };
     if (tiled_us(true_nnz, 0, 0) > 0.85 * own_us) return false;
-    if (n_rows >= kTiledNoRow || requests >= 1e11) return false;
+    if (n_rows >= kTiledInParts || requests >= 1e11) return false;
     Builder<VT> b(src, n_rows, n_cols);
     if (b.C + (u64)n_sm >= 65536) return false;
-    b.count(out.covers_all_rows);
+    b.count();
+    b.choose_sums(out);
     // (a warp's 32 `red` fall into about an eighth as many lines where the rows of a tile are dense, into 32 where they are sparse)
     double red = 0;
     u64 pieces = 0;
@@ -575,6 +641,7 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
         if (p > 0) red += p * std::min(1.0, std::max(0.25, 4.0 * (double)n_rows / p / 32.0));
     }
     if (tiled_us(b.N, pieces, red) > 0.85 * own_us) return false;
+    b.number_rows(out);
     b.scatter();
     b.slices(n_sm, out);
     return true;

@@ -9,11 +9,15 @@
 //   slice  64 pieces, two per lane, of about the same length (sorted inside windows of 1024 pieces); stored step by step,
 //          a step = one non-zero of every piece
 //   steps  one linear stream, cut evenly among the CTAs (one per SM) and inside them among the 32 warps, in the middle of
-//          slices too: what a warp has summed when its slice or its share ends goes to y by `red`
+//          slices too: what a warp has summed when its slice or its share ends is added to its row by `red`
+//   parts  a row that gets there in many parts would collect a rounding error with each (fp32, 80 elements over 25 tiles: 1.0e-7
+//          from the 64-bit result, the formats' own kernels 0.72e-7): the sums of such rows are 64-bit ones in memory of the
+//          group, which k_rows turns into y and leaves as zeros for the next call (0.42e-7). In fp64 the tiles take `copies`
+//          sums of a row in turn, which k_rows adds pairwise. A piece is summed with more than the value's bits, too.
 // The stream is read two batches deep into registers. 159 KB of shared memory per tile leave the L1 enough lines for the
 // loads in flight: with 224 KB the same stream is read at 4.2 instead of 5 TB/s.
-// Measured, fp32 (against the formats' own kernels): 200,000 rows of 40..120 non-zeros, random columns among 1 M: 36 us
-// (76 us, row-grouped); 9,001 rows of 1000..3000: 28 us (77 us, long-row).
+// Measured, fp32 (against the formats' own kernels): 200,000 rows of 40..120 non-zeros, random columns among 1 M: 40 us
+// (76 us, row-grouped; 36 us with all parts added up in y); 9,001 rows of 1000..3000: 27 us (77 us, long-row; 25 us).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -39,6 +43,49 @@ template <>
 struct Pair<double>
 {
     typedef double2 type;
+};
+
+// Sum of the products of a piece. fp32: the products of a batch in fp32 (four at most), the batches in fp64. fp64: the sum and
+// the rounding errors that it left out (two-sum); 13 operations a product of the 64 that an SM does per clock in fp64, of which a
+// non-zero takes one.
+template <class VT>
+struct Sum;
+template <>
+struct Sum<float>
+{
+    float part = 0;
+    double sum = 0;
+    __device__ __forceinline__ void add(float v, float x) { part += v * x; }
+    __device__ __forceinline__ void batch()
+    {
+        sum += (double)part;
+        part = 0;
+    }
+    __device__ __forceinline__ double take()
+    {
+        const double s = sum + (double)part;
+        sum = 0;
+        part = 0;
+        return s;
+    }
+};
+template <>
+struct Sum<double>
+{
+    double hi = 0, lo = 0;
+    __device__ __forceinline__ void add(double v, double x)
+    {
+        const double p = v * x, t = hi + p, b = t - hi;
+        lo += (hi - (t - b)) + (p - b) + fma(v, x, -p);
+        hi = t;
+    }
+    __device__ __forceinline__ void batch() {}
+    __device__ __forceinline__ double take()
+    {
+        const double s = isfinite(hi) ? hi + lo : hi; // (the errors of an infinite sum are no numbers)
+        hi = lo = 0;
+        return s;
+    }
 };
 
 // x may have been written by the kernel before: read through L2, in program order after the wait
@@ -76,10 +123,10 @@ __global__ void __launch_bounds__(256) k_clear(VT *y, u64 n)
     if (t < n - h - body * V) y[h + body * V + t] = 0;
 }
 
-// y[row] += v for the 32 pieces of a warp. Pieces of a long row lie next to one another, and a `red` of many lanes to one
+// row += v for the 32 pieces of a warp. Pieces of a long row lie next to one another, and a `red` of many lanes to one
 // address is served lane by lane: those are summed in the warp first (R-MAT with hub rows: 72 -> 60 us an SpMV).
 template <class VT>
-__device__ __forceinline__ void add_rows(VT *y, u32 row, VT v, u32 lane)
+__device__ __forceinline__ void add_rows(VT *y, double *sum, u32 row, double v, u32 lane)
 {
     const u32 next = __shfl_down_sync(0xffffffffu, row, 1);
     const u32 goes_on = __ballot_sync(0xffffffffu, lane < 31 && row == next);
@@ -90,13 +137,15 @@ __device__ __forceinline__ void add_rows(VT *y, u32 row, VT v, u32 lane)
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1)
         {
-            const VT o = __shfl_down_sync(0xffffffffu, v, d);
+            const double o = __shfl_down_sync(0xffffffffu, v, d);
             const u32 m = (1u << d) - 1u;
             if ((from & m) == m) v += o;
         }
         head = lane == 0 || ((goes_on >> (lane - 1)) & 1u) == 0;
     }
-    if (head && row != kTiledNoRow) atomicAdd(y + row, v); // result unused: red.global.add
+    if (!head || row == kTiledNoRow) return;
+    if (row & kTiledInParts) atomicAdd(sum + (row & ~kTiledInParts), v); // result unused: red.global.add
+    else atomicAdd(y + row, (VT)v);
 }
 
 template <class VT, int U>
@@ -115,6 +164,7 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
         u32 step = k.x, slice = k.z;
         const u32 end = k.y, tile = k.w & 0xffffu;
         visit = k.w >> 16;
+        double *const sum = a.sum + (size_t)(tile & (a.copies - 1)) * a.sum_stride;
         const P *vp = reinterpret_cast<const P *>(a.val) + (size_t)step * 32 + lane;
         const u32 *cp = reinterpret_cast<const u32 *>(a.col) + (size_t)step * 32 + lane;
         P v[U];
@@ -164,7 +214,7 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
             if (threadIdx.x == 0) xs[tile_cols] = 0;
         }
         __syncthreads();
-        VT acc0 = 0, acc1 = 0;
+        Sum<VT> acc0, acc1;
         while (step < end)
         {
             P nv[U];
@@ -181,14 +231,13 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
             for (int u = 0; u < U; u++)
                 if (step < end)
                 {
-                    acc0 += v[u].x * xs[c[u] & 0xffffu];
-                    acc1 += v[u].y * xs[c[u] >> 16];
+                    acc0.add(v[u].x, xs[c[u] & 0xffffu]);
+                    acc1.add(v[u].y, xs[c[u] >> 16]);
                     step++;
                     if (step == s_end || step == end)
                     {
-                        add_rows(y, row.x, acc0, lane);
-                        add_rows(y, row.y, acc1, lane);
-                        acc0 = acc1 = 0;
+                        add_rows(y, sum, row.x, acc0.take(), lane);
+                        add_rows(y, sum, row.y, acc1.take(), lane);
                         slice++;
                         rp += 32;
                         s_end = s_next;
@@ -203,8 +252,52 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
                 v[u] = nv[u];
                 c[u] = nc[u];
             }
+            acc0.batch();
+            acc1.batch();
         }
     } while (visit != 0);
+}
+
+__device__ __forceinline__ double ld_sum(const double *p)
+{
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// the rows in many parts: y = their sums, which are zero afterwards (for the next k_tiled)
+template <class VT, int G>
+__global__ void __launch_bounds__(256) k_rows(const u32 *rows, double *sum, u64 stride, VT *y, u32 n)
+{
+    constexpr int U = G < 4 ? 4 / G : 1; // rows in flight
+    const u32 threads = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_release();
+    grid_wait();
+    for (u32 r = t; r < n; r += threads * U)
+    {
+        double s[U][G];
+        u32 to[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+        {
+            const u32 q = r + u * threads < n ? r + u * threads : r;
+            to[u] = rows ? __ldg(rows + q) : q;
+#pragma unroll
+            for (int g = 0; g < G; g++) s[u][g] = ld_sum(sum + g * stride + q);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (r + u * threads < n)
+            {
+#pragma unroll
+                for (int g = 0; g < G; g++) sum[g * stride + r + u * threads] = 0;
+#pragma unroll
+                for (int d = 1; d < G; d *= 2)
+#pragma unroll
+                    for (int g = 0; g + d < G; g += 2 * d) s[u][g] += s[u][g + d];
+                y[to[u]] = (VT)s[u][0];
+            }
+    }
 }
 
 template <class VT>
@@ -229,11 +322,32 @@ cudaError_t clear(VT *y, u64 n, unsigned n_sm, cudaStream_t st)
 }
 
 template <class VT>
-cudaError_t launch(const TiledArgs &a, unsigned n_sm, cudaStream_t st)
+cudaError_t launch_sums(const TiledArgs &a, unsigned n_sm, cudaStream_t st)
 {
-    const cudaError_t e = clear((VT *)a.y, a.n_rows, n_sm, st);
-    if (e != cudaSuccess) return e;
+    if (a.direct)
+    {
+        const cudaError_t e = clear((VT *)a.y, a.n_rows, n_sm, st);
+        if (e != cudaSuccess) return e;
+    }
     return launch_pdl(k_tiled<VT, Batch<VT>::U>, dim3(n_sm), dim3(kTiledWarps * 32), kTiledTileBytes, st, a, (u32)tiled_tile_cols(sizeof(VT) == 8));
+}
+
+template <class VT>
+cudaError_t launch_rows(const TiledArgs &a, unsigned n_sm, cudaStream_t st)
+{
+    // a few rows per thread
+    const u64 want = (a.n_parts + 1023ull) / 1024;
+    const dim3 grid((unsigned)(want < 1 ? 1 : want < 4ull * n_sm ? want : 4ull * n_sm)), block(256);
+    const auto rows = [&](auto kernel) { return launch_pdl(kernel, grid, block, 0, st, a.parts, a.sum, (u64)a.sum_stride, (VT *)a.y, (u32)a.n_parts); };
+    if (a.copies == 1) return rows(k_rows<VT, 1>);
+    if constexpr (sizeof(VT) == 8)
+    {
+        if (a.copies == 2) return rows(k_rows<VT, 2>);
+        if (a.copies == 4) return rows(k_rows<VT, 4>);
+        if (a.copies == 8) return rows(k_rows<VT, 8>);
+        if (a.copies == 16) return rows(k_rows<VT, 16>);
+    }
+    return cudaErrorInvalidValue;
 }
 } // namespace
 
@@ -248,8 +362,13 @@ cudaError_t tiled_setup(int val_is_f64)
     return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTiledTileBytes);
 }
 
-cudaError_t launch_tiled(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st)
+cudaError_t launch_tiled_sums(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st)
 {
-    return val_is_f64 ? launch<double>(a, n_sm, st) : launch<float>(a, n_sm, st);
+    return val_is_f64 ? launch_sums<double>(a, n_sm, st) : launch_sums<float>(a, n_sm, st);
+}
+
+cudaError_t launch_tiled_rows(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st)
+{
+    return val_is_f64 ? launch_rows<double>(a, n_sm, st) : launch_rows<float>(a, n_sm, st);
 }
 } // namespace asp

@@ -20,6 +20,7 @@ const uint32_t kTiledLanePieces = 2;         // pieces of a row per lane
 const uint32_t kTiledSlice = 32 * kTiledLanePieces;
 constexpr uint32_t kTiledTileBytes = 159u << 10; // shared memory of a tile of x
 const uint32_t kTiledNoRow = 0xffffffffu;
+const uint32_t kTiledInParts = 0x80000000u; // row entry: the rest is a place among the sums of the rows in many parts
 // steps and slices the kernel may read past the end (prefetch)
 const uint32_t kTiledSlackSteps = 8, kTiledSlackSlices = 2;
 
@@ -54,11 +55,15 @@ struct TiledHost
 {
     HostBuf<unsigned char> val; // step s, lane l, piece g: value s * 64 + 2 l + g
     HostBuf<uint16_t> col;      // same order, column inside the tile
-    HostBuf<uint32_t> row;      // slice s, lane l, piece g: row of y (kTiledNoRow: none)
+    HostBuf<uint32_t> row;      // slice s, lane l, piece g: row of y, or kTiledInParts | place (kTiledNoRow: none)
+    uint64_t n_parts = 0;        // rows of y that are added up in many parts ...
+    std::vector<uint32_t> parts; // ... which these are; empty: all
     HostBuf<uint32_t> end;      // slice s covers steps [end[s - 1], end[s])
     std::vector<uint32_t> work; // {first step, end step, slice, tile | next visit << 16} per warp; visit v at v * kTiledWarps
     uint64_t nnz = 0, steps = 0, slices = 0;
+    unsigned copies = 1; // sums of a row, which its tiles take in turn: 1, 2, 4, 8 or 16
     bool covers_all_rows = false; // every row of y has at least one element
+    bool direct = false;          // some are added up in y itself
 };
 
 // false: the group stays with its own kernels
@@ -70,12 +75,19 @@ struct TiledArgs
     const uint16_t *col;
     const uint32_t *row, *end;
     const uint4 *work;
+    const uint32_t *parts; // n_parts rows (NULL: all rows of y) ...
+    double *sum;           // ... and their sums, copies * sum_stride of them, zero between the calls
+    unsigned n_parts, copies;
+    unsigned long long sum_stride;
+    int direct; // y takes other rows' sums: it is cleared first
     const void *x;
     void *y;
     unsigned long long n_rows, n_cols;
 };
 cudaError_t tiled_setup(int val_is_f64);
-// y = A x: clears y, then accumulates (two launches)
-cudaError_t launch_tiled(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st);
+// y = A x in up to three launches: y cleared, everything added up, the rows in many parts stored by launch_tiled_rows (n_parts > 0),
+// which has to run before the next call's
+cudaError_t launch_tiled_sums(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st);
+cudaError_t launch_tiled_rows(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st);
 } // namespace asp
 #endif

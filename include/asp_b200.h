@@ -175,7 +175,9 @@ void *asp_ctx_stream(asp_ctx *ctx);
  * Where the columns are so scattered that the gathers of x, not the bytes, bound the templates' kernels, the whole group
  * is also laid out by column tiles (csrc/kernels_tiled.cu; about 1.5 times the format's device memory in all), and asp_spmv
  * over the complete group runs that layout; a group with EMPTY plans never does. Sums are then taken in another order from
- * call to call, as with every template that accumulates with atomics.
+ * call to call, as with every template that accumulates with atomics. Rows that are added up in many parts have 64-bit sums in
+ * the group's device memory: a group with such rows runs the layout in the calls of the context that created it, and its
+ * templates' kernels in calls of another context and in calls that a stream capture records.
  * Every entry point makes the context's device current for its own duration and restores the
  * caller's device before it returns. */
 asp_status asp_plan_group_create(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp_plan **out_plans);

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import refdump
-from alphasparse_b200 import matrices as M, tuner
+from alphasparse_b200 import capi, matrices as M, tuner
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +70,79 @@ def test_tiled_group_of_sorted_strips_and_empty_rows(asp_ctx):
     fmt.close()
     cm.close()
     hm.close()
+
+
+def exact(m, x):
+    """(A x, |A| |x|) in the next longer type."""
+    t = np.float64 if m.values.dtype == np.float32 else np.longdouble
+    p = m.values.astype(t) * x.astype(t)[m.indices.view(np.int32)]
+    return np.add.reduceat(p, m.indptr[:-1]), np.add.reduceat(np.abs(p), m.indptr[:-1])
+
+
+@pytest.mark.parametrize("template,dtype,rows,lo,hi,cols", [
+    ("K6", np.float32, 60_000, 40, 121, 1_000_000), ("K8", np.float64, 60_000, 40, 121, 1_000_000), ("K4", np.float64, 60_000, 40, 121, 100_000),
+    ("K7", np.float32, 4_000, 1000, 3001, 1_000_000), ("K7", np.float64, 4_000, 1000, 3001, 1_000_000), ("K9", np.float32, 250_000, 4, 29, 1_000_000)])
+def test_tiled_sums_are_as_near_to_the_exact_ones_as_the_templates(asp_ctx, template, dtype, rows, lo, hi, cols):
+    """The layout adds a row up in other parts than the template's kernel, but with no larger error."""
+    import torch
+
+    rng = np.random.default_rng(rows)
+    m, x = M.from_row_lengths(rng.integers(lo, hi, size=rows), cols, seed=rows, dtype=dtype)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template, "threads": 128, "row_reduce": 1}]})
+    assert g.layout_bytes() > 0, "the layout was not built for this matrix"
+    ref, scale = exact(m, x)
+    dx = torch.from_numpy(x).cuda()
+    far = []
+    for zero_y in (True, False):  # the layout; the template's kernel, which adds to the zeros in y
+        dy = torch.zeros(m.n_rows, dtype=dx.dtype, device="cuda")
+        torch.cuda.synchronize()
+        g.spmv(dx.data_ptr(), dy.data_ptr(), zero_y)
+        asp_ctx.synchronize()
+        d = dy.cpu().numpy().astype(ref.dtype) - ref
+        far.append((float(np.sqrt((d * d).sum() / (ref * ref).sum())), float((np.abs(d) / scale).max())))
+    assert far[0][0] <= 1.01 * far[1][0], far  # (the 2-norm repeats to a percent; the largest is one row's)
+    assert far[0][1] <= 1.25 * far[1][1], far
+    g.close()
+    fmt.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_tiled_sums_are_one_call_s_own(asp_ctx, dtype):
+    """Infinite sums leave nothing behind; calls of another context, of a graph and of the plan's own context give the same y."""
+    import torch
+
+    m, x = matrix(dtype, 3 * TILE[dtype], seed=3)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": "K9", "nodes": NODES["K9"], "template": "K9", "threads": 128, "row_reduce": 1}]})
+    assert g.layout_bytes() > 0
+    y_ref, scale = refdump.csr_ref(m, x)
+    hit = np.bincount(np.repeat(np.arange(m.n_rows), m.row_lengths())[m.indices == 17], minlength=m.n_rows) > 0
+    bad = x.copy()
+    bad[17] = np.inf
+    y = g.spmv_host(bad)
+    assert np.isinf(y[hit]).all() and np.isfinite(y[~hit]).all()
+    refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, "after an infinite x")
+    bad[17] = np.nan
+    assert np.isnan(g.spmv_host(bad)[hit]).all()
+    refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, "after x that is no number")
+    dx, dys = torch.from_numpy(x).cuda(), [torch.full((m.n_rows,), 7.0, dtype=torch.from_numpy(x).dtype, device="cuda") for _ in range(3)]
+    torch.cuda.synchronize()
+    other = capi.Context(0)
+    for _ in range(20):  # on two streams at once
+        g.spmv(dx.data_ptr(), dys[0].data_ptr(), True)
+        capi.check(capi.lib().asp_spmv(other.handle, g._plans, g.n, dx.data_ptr(), dys[1].data_ptr(), 1))
+    other.synchronize()
+    asp_ctx.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(asp_ctx.stream)):
+        g.spmv(dx.data_ptr(), dys[2].data_ptr(), True)
+    for _ in range(5):
+        graph.replay()  # on torch's stream
+        g.spmv(dx.data_ptr(), dys[0].data_ptr(), True)
+    torch.cuda.synchronize()
+    asp_ctx.synchronize()
+    for y, what in zip(dys, ("own context", "another context", "graph")):
+        refdump.assert_y(y.cpu().numpy(), y_ref, scale, m.values.dtype, what)
+    del graph
+    other.close()
+    g.close()
+    fmt.close()
