@@ -889,7 +889,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
                     mx = std::max(mx, w1 - w0);
                 }
                 p->smem_elems = mx;
-                if (st == ASP_OK && hm[asp::MS_WARP_NZ].get(W1 - 1) > nnz_pad) st = ASP_ERR_BOUNDS, why = "warp-reduce smem: last nz offset outside val_arr";
+                if (st == ASP_OK && max_of(hm[asp::MS_WARP_NZ], W1) > nnz_pad) st = ASP_ERR_BOUNDS, why = "warp-reduce smem: an nz offset outside val_arr";
             }
             p->units_for_grid = B;
             break;
@@ -899,7 +899,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
             const uint64_t B = hm[asp::MS_ROW_OF_UNIT].len;
             a.n_units = B;
             if (B == 0 || hm[asp::MS_BLK_NZ].len != B + 1) st = ASP_ERR_BOUNDS, why = "long-row: block_nz_begin_offset must have #BLB + 1 entries";
-            else if (hm[asp::MS_BLK_NZ].get(B) > nnz_pad) st = ASP_ERR_BOUNDS, why = "long-row: last nz offset outside val_arr";
+            else if (max_of(hm[asp::MS_BLK_NZ], B + 1) > nnz_pad) st = ASP_ERR_BOUNDS, why = "long-row: an nz offset outside val_arr";
             p->units_for_grid = B;
             break;
         }
@@ -909,7 +909,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
             a.n_units = W;
             a.effective = d.effective_num ? std::min<uint64_t>(d.effective_num, W) : W;
             if (W == 0 || hm[asp::MS_WARP_NZ].len != W + 1) st = ASP_ERR_BOUNDS, why = "warp-per-row: global_warp_nz_begin_offset must have #WLB + 1 entries";
-            else if (hm[asp::MS_WARP_NZ].get(W) > nnz_pad) st = ASP_ERR_BOUNDS, why = "warp-per-row: last nz offset outside val_arr";
+            else if (max_of(hm[asp::MS_WARP_NZ], W + 1) > nnz_pad) st = ASP_ERR_BOUNDS, why = "warp-per-row: an nz offset outside val_arr";
             p->units_for_grid = W;
             break;
         }
