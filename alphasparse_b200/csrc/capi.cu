@@ -295,6 +295,9 @@ asp_status apply_launch(asp_ctx *ctx, asp_plan *p, int64_t tblock, int64_t threa
     return ASP_OK;
 }
 
+// a closed form, or an array of at least `count` entries
+bool has_entries(const HostMeta &h, uint64_t count) { return h.kind != ASP_COMPRESS_NONE || h.len >= count; }
+
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // ---- content validation --------------------------------------------------------------------------
@@ -807,6 +810,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
             a.n_tlb = T;
             a.effective = d.effective_num ? std::min<uint64_t>(d.effective_num, T) : T;
             if (B == 0 || hm[asp::MS_BLK_THR].len != B + 1) st = ASP_ERR_BOUNDS, why = "SELL-like: block_begin_thread_index_offset must have #BLB + 1 entries";
+            else if (!has_entries(hm[asp::MS_TLB_SIZE], B)) st = ASP_ERR_BOUNDS, why = "SELL-like: fewer TLB sizes than BLBs";
             else
             {
                 for (uint64_t b = 0; b < B && st == ASP_OK; b++)
@@ -840,10 +844,17 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
             {
                 const uint64_t W = hm[asp::MS_WARP_NZ].len;
                 uint64_t mx = 0;
+                if (!has_entries(hm[asp::MS_TLB_SIZE], W)) st = ASP_ERR_BOUNDS, why = "3-level: fewer TLB sizes than WLBs";
                 for (uint64_t b = 0; b < B && st == ASP_OK; b++)
                 {
                     const uint64_t w0 = hm[asp::MS_BLK_WARP].get(b), w1 = hm[asp::MS_BLK_WARP].get(b + 1);
                     if (w1 < w0 || w1 > W || w1 + 1 > hm[asp::MS_WARP_THR].len) { st = ASP_ERR_BOUNDS; why = "3-level: WLB range outside the WLB arrays"; break; }
+                    for (uint64_t w = w0; w < w1 && st == ASP_OK; w++)
+                    {
+                        const uint64_t t0 = hm[asp::MS_WARP_THR].get(w), t1 = hm[asp::MS_WARP_THR].get(w + 1);
+                        if (t1 < t0 || t1 > a.n_tlb || hm[asp::MS_BLK_NZ].get(b) + hm[asp::MS_WARP_NZ].get(w) + (t1 - t0) * hm[asp::MS_TLB_SIZE].get(w) > nnz_pad)
+                            st = ASP_ERR_BOUNDS, why = "3-level: a WLB reaches outside val_arr or the TLBs";
+                    }
                     mx = std::max(mx, hm[asp::MS_WARP_THR].get(w1) - hm[asp::MS_WARP_THR].get(w0));
                 }
                 p->smem_elems = mx;
@@ -857,6 +868,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
             a.n_units = B;
             a.effective = d.effective_num ? d.effective_num : ~0ull;
             if (B == 0 || hm[asp::MS_BLK_THR].len != B + 1 || hm[asp::MS_BLK_ROW].len != B + 1) st = ASP_ERR_BOUNDS, why = "row-grouped: offset arrays must have #BLB + 1 entries";
+            else if (!has_entries(hm[asp::MS_TLB_SIZE], B)) st = ASP_ERR_BOUNDS, why = "row-grouped: fewer TLB sizes than BLBs";
             else
             {
                 uint64_t mx = 0;
