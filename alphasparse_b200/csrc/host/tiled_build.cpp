@@ -20,6 +20,7 @@ namespace
 typedef uint64_t u64;
 typedef uint32_t u32;
 
+// (What the threads of a parallel region work in is allocated before it: an exception that leaves a region ends the process.)
 int threads()
 {
 #ifdef _OPENMP
@@ -28,6 +29,22 @@ int threads()
     return 1;
 #endif
 }
+int this_thread()
+{
+#ifdef _OPENMP
+    return omp_get_thread_num();
+#else
+    return 0;
+#endif
+}
+// counters of every thread, on cache lines of their own
+struct ThreadCounters
+{
+    const u64 n, stride;
+    std::vector<u64> all;
+    explicit ThreadCounters(u64 count) : n(count), stride((count + 15) / 8 * 8), all(stride * (u64)threads(), 0) {}
+    u64 *mine() { return all.data() + stride * (u64)this_thread(); }
+};
 
 u64 row_in_y(const TiledSource &s, u64 r)
 {
@@ -275,13 +292,14 @@ struct Builder
         row_code.assign(n_rows, 0);
         std::vector<u32> share;
         for (const TiledSource &s : src) share.push_back(share_of_part(s));
+        ThreadCounters pieces_of_thread(C), n_of_thread(C); // (neighbours in `at` share cache lines)
 #pragma omp parallel
         {
-            std::vector<u64> pieces(C, 0), n(C); // (counters of a thread's own: neighbours in `at` share cache lines)
+            u64 *const pieces = pieces_of_thread.mine(), *const n = n_of_thread.mine();
 #pragma omp for schedule(dynamic, 1)
             for (long long c = 0; c < (long long)chunks.size(); c++)
             {
-                std::fill(n.begin(), n.end(), 0);
+                std::fill(n, n + C, 0);
                 u64 row = ~0ull, tile = ~0ull, run = 0;
                 u32 of_row = 0; // pieces since the row changed
                 auto row_ends = [&]() {
@@ -304,7 +322,7 @@ struct Builder
                     run++;
                 });
                 row_ends();
-                std::copy(n.begin(), n.end(), at.begin() + (size_t)c * C);
+                std::copy(n, n + C, at.begin() + (size_t)c * C);
             }
 #pragma omp critical
             for (u64 t = 0; t < C; t++) tile_pieces[t] += pieces[t];
@@ -369,13 +387,14 @@ struct Builder
         e_row.make(N);
         e_col.make(N);
         e_val.make(N);
+        ThreadCounters to_of_thread(C);
 #pragma omp parallel
         {
-            std::vector<u64> to(C);
+            u64 *const to = to_of_thread.mine();
 #pragma omp for schedule(dynamic, 1)
             for (long long c = 0; c < (long long)chunks.size(); c++)
             {
-                std::copy(at.begin() + (size_t)c * C, at.begin() + (size_t)(c + 1) * C, to.begin());
+                std::copy(at.begin() + (size_t)c * C, at.begin() + (size_t)(c + 1) * C, to);
                 walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) {
                     const u64 t = (u32)col / TW, q = to[t]++;
                     e_row.p[q] = (u32)r;
@@ -396,27 +415,34 @@ struct Builder
         u64 step = 0, slice = 0; // first step and slice of the block
     };
 
-    // pieces of a block in windows, every window by descending length (rows in order where lengths agree)
-    void pieces_of(const Block &b, std::vector<Piece> &p, std::vector<Piece> &tmp) const
+    struct Pieces // of one block, in a thread's own memory
     {
-        p.clear();
+        Piece *p, *sorted;
+        size_t n = 0;
+        size_t size() const { return n; }
+        const Piece &operator[](size_t i) const { return sorted[i]; }
+    };
+    // in windows, every window by descending length (rows in order where lengths agree)
+    void pieces_of(const Block &b, Pieces &out) const
+    {
+        Piece *const p = out.p;
+        size_t n = 0;
         for (u64 k = b.e0; k < b.e1;)
         {
             u64 q = k + 1;
             while (q < b.e1 && q - k < kMaxPiece && e_row.p[q] == e_row.p[k]) q++;
-            p.push_back({(u32)(k - b.e0), (u32)(q - k)});
+            p[n++] = {(u32)(k - b.e0), (u32)(q - k)};
             k = q;
         }
-        tmp.resize(p.size());
-        for (size_t i = 0; i < p.size(); i += kWindow)
+        out.n = n;
+        for (size_t i = 0; i < n; i += kWindow)
         {
-            const size_t e = std::min(p.size(), i + kWindow);
+            const size_t e = std::min<size_t>(n, i + kWindow);
             u32 cnt[kMaxPiece + 2] = {0};
             for (size_t j = i; j < e; j++) cnt[kMaxPiece - p[j].len + 1]++;
             for (u32 l = 1; l <= kMaxPiece; l++) cnt[l] += cnt[l - 1];
-            for (size_t j = i; j < e; j++) tmp[i + cnt[kMaxPiece - p[j].len]++] = p[j];
+            for (size_t j = i; j < e; j++) out.sorted[i + cnt[kMaxPiece - p[j].len]++] = p[j];
         }
-        p.swap(tmp);
     }
 
     void slices(int n_sm, TiledHost &out)
@@ -439,13 +465,21 @@ struct Builder
         tile_block[C] = blocks.size();
         const long long B = (long long)blocks.size();
         std::vector<u64> n_step(B), n_slice(B);
+        u64 longest = 0;
+        for (const Block &b : blocks) longest = std::max(longest, b.e1 - b.e0);
+        HostBuf<Piece> scratch;
+        scratch.make(2 * longest * (u64)threads());
+        auto scratch_of_thread = [&]() {
+            Piece *const mine = scratch.p + 2 * longest * (u64)this_thread();
+            return Pieces{mine, mine + longest};
+        };
 #pragma omp parallel
         {
-            std::vector<Piece> p, tmp;
+            Pieces p = scratch_of_thread();
 #pragma omp for schedule(dynamic, 1)
             for (long long b = 0; b < B; b++)
             {
-                pieces_of(blocks[b], p, tmp);
+                pieces_of(blocks[b], p);
                 u64 s = 0;
                 for (size_t i = 0; i < p.size(); i += kTiledSlice) s += p[i].len;
                 n_step[b] = s;
@@ -468,11 +502,11 @@ struct Builder
         VT *val = (VT *)out.val.p;
 #pragma omp parallel
         {
-            std::vector<Piece> p, tmp;
+            Pieces p = scratch_of_thread();
 #pragma omp for schedule(dynamic, 1)
             for (long long b = 0; b < B; b++)
             {
-                pieces_of(blocks[b], p, tmp);
+                pieces_of(blocks[b], p);
                 u64 step = blocks[b].step, slice = blocks[b].slice;
                 for (size_t i = 0; i < p.size(); i += kTiledSlice, slice++)
                 {
