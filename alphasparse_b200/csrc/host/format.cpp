@@ -757,12 +757,10 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     u64 max_thread_first_row = 0;
     bool share_thread = tlb_size != 0;
     // pass 2: fill the padded arrays (row-major inside the WLB) and the per-TLB first rows
-    // `first`: first TLB of every row of the WLB, relative to it
-    auto fill_wlb = [&](u64 w, std::vector<u64> &first, u64 &top_of_all, bool &shared) {
+    // `f`: first TLB of every row of the WLB, relative to it
+    auto fill_wlb = [&](u64 w, u64 *f, u64 &top_of_all, bool &shared) {
         const Span s = span(w);
         const u64 S = wlb_S[w], extra = wlb_tlb0[w + 1] - wlb_tlb0[w] - wlb_tl[w];
-        first.resize(s.rows + 1);
-        u64 *f = first.data();
         f[0] = 0;
         for_each(s.rows, by_rows && s.rows > kParallelRows, [&](u64 r) {
             u64 lo, hi;
@@ -799,19 +797,20 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
         shared = shared || shared_row;
         top_of_all = std::max(top_of_all, top);
     };
+    u64 most_rows = 0;
+    for (u64 w = 0; w < NW; w++) most_rows = std::max(most_rows, W.row_num.v[w]);
+    const u64 stride = (most_rows + 1 + 15) / 8 * 8; // (cache lines of a thread's own)
     if (by_rows)
     {
-        std::vector<u64> first;
-        for (u64 w = 0; w < NW; w++) fill_wlb(w, first, max_thread_first_row, share_thread);
+        std::vector<u64> first(stride);
+        for (u64 w = 0; w < NW; w++) fill_wlb(w, first.data(), max_thread_first_row, share_thread);
     }
     else
     {
-#pragma omp parallel if (b.col.size() > kParallelNnz)
-        {
-            std::vector<u64> first;
-#pragma omp for schedule(static) reduction(max : max_thread_first_row) reduction(|| : share_thread)
-            for (u64 w = 0; w < NW; w++) fill_wlb(w, first, max_thread_first_row, share_thread);
-        }
+        // (allocated before the region: an exception that leaves one ends the process)
+        std::vector<u64> first(stride * (u64)omp_get_max_threads());
+#pragma omp parallel for schedule(static) reduction(max : max_thread_first_row) reduction(|| : share_thread) if (b.col.size() > kParallelNnz)
+        for (u64 w = 0; w < NW; w++) fill_wlb(w, first.data() + stride * (u64)omp_get_thread_num(), max_thread_first_row, share_thread);
     }
     u64 max_w_coo_begin = 0, max_w_size = 0;
     std::vector<u64> new_w_begin(NW), new_w_size(NW);

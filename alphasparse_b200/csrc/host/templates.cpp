@@ -8,7 +8,6 @@
 
 #include "format.hpp"
 
-#include <set>
 
 namespace asp
 {
@@ -979,34 +978,25 @@ bool init_diag(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::
     const int es = b.val.es;
     const u64 V = 16 / (u64)es, NR = (b.n_rows + V - 1) / V * V;
     const int64_t ncols = (int64_t)(b.max_col - b.min_col + 1);
-    // distinct offsets; a scattered matrix leaves after a few rows
-    std::set<int64_t> offs;
-    bool too_many = false;
-#pragma omp parallel if (b.nnz() > kParallelNnz)
+    // distinct offsets, as bits of all there could be; a scattered matrix leaves after a few rows
+    std::vector<u64> bits((b.n_rows + (u64)ncols) / 64 + 1, 0);
+    u64 found = 0;
+#pragma omp parallel for schedule(static) if (b.nnz() > kParallelNnz)
+    for (u64 r = 0; r < b.n_rows; r++)
     {
-        std::vector<int64_t> mine; // ascending
-        bool full = false;
-#pragma omp for schedule(static)
-        for (u64 r = 0; r < b.n_rows; r++)
+        if (__atomic_load_n(&found, __ATOMIC_RELAXED) > b.diag_max) continue;
+        for (u64 k = b.rowptr[r]; k < b.rowptr[r + 1]; k++)
         {
-            size_t q = 0; // the columns of a row ascend, and so do its offsets
-            for (u64 k = full ? b.rowptr[r + 1] : b.rowptr[r]; k < b.rowptr[r + 1]; k++)
-            {
-                const int64_t o = (int64_t)b.col[k] - (int64_t)r;
-                while (q < mine.size() && mine[q] < o) q++;
-                if (q == mine.size() || mine[q] != o) mine.insert(mine.begin() + q, o);
-            }
-            full = full || mine.size() > b.diag_max;
-        }
-#pragma omp critical
-        {
-            too_many = too_many || full;
-            if (!too_many) offs.insert(mine.begin(), mine.end());
+            const u64 at = b.col[k] + b.n_rows - r, bit = 1ull << (at % 64);
+            if (__atomic_load_n(&bits[at / 64], __ATOMIC_RELAXED) & bit) continue;
+            if ((__atomic_fetch_or(&bits[at / 64], bit, __ATOMIC_RELAXED) & bit) == 0) __atomic_fetch_add(&found, 1, __ATOMIC_RELAXED);
         }
     }
-    if (too_many || offs.size() > b.diag_max) return err = "diag_value: more than " + std::to_string(b.diag_max) + " diagonals hold non-zeros", false;
-    if (offs.empty()) return err = "diag_value: sub-matrix without non-zeros", false;
-    const std::vector<int64_t> off(offs.begin(), offs.end());
+    if (found > b.diag_max) return err = "diag_value: more than " + std::to_string(b.diag_max) + " diagonals hold non-zeros", false;
+    if (found == 0) return err = "diag_value: sub-matrix without non-zeros", false;
+    std::vector<int64_t> off; // ascending
+    for (u64 w = 0; w < bits.size(); w++)
+        for (u64 left = bits[w]; left; left &= left - 1) off.push_back((int64_t)(w * 64 + (u64)__builtin_ctzll(left)) - (int64_t)b.n_rows);
     const u64 D = off.size();
     Arr<uint8_t> val;
     uint8_t *const vp = val.make_zero(D * NR * (u64)es);
