@@ -749,8 +749,8 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
             cleanup();
             return fail(ASP_ERR_ALLOC, "host allocation failed");
         }
-        made.push_back(p);
         out_plans[i] = p;
+        made.push_back(p);
         p->arena = arena;
         p->templ = d.template_type;
         p->n_rows = d.n_rows;
@@ -1154,14 +1154,42 @@ asp_status asp_plan_group_create(asp_ctx *ctx, const asp_plan_desc *descs, int n
     if (!ctx || !descs || !out_plans || n <= 0) return fail(ASP_ERR_INVALID_ARG, "NULL argument or n <= 0");
     for (int i = 0; i < n; i++) out_plans[i] = nullptr;
     ASP_ON_DEVICE(ctx);
-    return plan_group_build(ctx, descs, n, out_plans, false);
+    try
+    {
+        return plan_group_build(ctx, descs, n, out_plans, false);
+    }
+    catch (const std::bad_alloc &)
+    {
+        for (int i = 0; i < n; i++)
+        {
+            delete out_plans[i];
+            out_plans[i] = nullptr;
+        }
+        return fail(ASP_ERR_ALLOC, "host allocation failed");
+    }
 }
 
 asp_status asp_plan_descs_validate(const asp_plan_desc *descs, int n)
 {
     if (!descs || n <= 0) return fail(ASP_ERR_INVALID_ARG, "NULL argument or n <= 0");
-    std::vector<asp_plan *> scratch((size_t)n, nullptr);
-    return plan_group_build(nullptr, descs, n, scratch.data(), true);
+    try
+    {
+        std::vector<asp_plan *> scratch((size_t)n, nullptr);
+        // (whatever is thrown, the plans made so far go)
+        struct Plans
+        {
+            std::vector<asp_plan *> &all;
+            ~Plans()
+            {
+                for (asp_plan *p : all) delete p;
+            }
+        } plans{scratch};
+        return plan_group_build(nullptr, descs, n, scratch.data(), true);
+    }
+    catch (const std::bad_alloc &)
+    {
+        return fail(ASP_ERR_ALLOC, "host allocation failed");
+    }
 }
 
 void asp_plan_destroy(asp_plan *plan) { delete plan; }

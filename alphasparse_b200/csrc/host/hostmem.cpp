@@ -3,7 +3,6 @@
 #include <sys/mman.h>
 
 #include <mutex>
-#include <vector>
 
 namespace asp
 {
@@ -24,28 +23,38 @@ Pool &pool()
     return *p;
 }
 
-void give_back(void *p, size_t size)
+// frees the longest idle buffers until no more than `most` bytes are left
+void shrink(size_t most)
 {
     Pool &q = pool();
-    std::vector<void *> out;
+    for (;;)
+    {
+        void *p;
+        {
+            std::lock_guard<std::mutex> g(q.lock);
+            p = q.idle.beyond(most);
+        }
+        if (!p) return;
+        free(p);
+    }
+}
+
+// (the deleter of a shared buffer: nothing may be thrown)
+void give_back(void *p, size_t size) noexcept
+{
+    Pool &q = pool();
+    bool kept = size <= kMostIdle;
+    if (kept)
     {
         std::lock_guard<std::mutex> g(q.lock);
-        q.idle.put(p, size, kMostIdle, out);
+        kept = q.idle.put(p, size);
     }
-    for (void *o : out) free(o);
+    if (!kept) free(p);
+    shrink(kMostIdle);
 }
 } // namespace
 
-void host_pool_trim()
-{
-    Pool &q = pool();
-    std::vector<void *> idle;
-    {
-        std::lock_guard<std::mutex> g(q.lock);
-        q.idle.take_all(idle);
-    }
-    for (void *p : idle) free(p);
-}
+void host_pool_trim() { shrink(0); }
 
 std::shared_ptr<void> big_buffer(size_t bytes)
 {

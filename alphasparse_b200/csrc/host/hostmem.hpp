@@ -45,28 +45,32 @@ class IdleBlocks
         by_size.erase(it);
         return p;
     }
-    // keeps the block; those that this takes beyond `most` bytes in all, longest idle first, are appended to `out`: without that,
-    // blocks of sizes that are not asked for again would fill the pool for good
-    void put(void *p, size_t size, size_t most, std::vector<void *> &out)
+    // keeps the block; false (it stays the caller's) when there is no memory to note it
+    bool put(void *p, size_t size) noexcept
     {
-        if (size > most) return out.push_back(p);
-        by_size.insert({size, {p, clock++}});
-        bytes += size;
-        while (bytes > most)
+        try
         {
-            auto old = by_size.begin();
-            for (auto it = by_size.begin(); it != by_size.end(); ++it)
-                if (it->second.since < old->second.since) old = it;
-            out.push_back(old->second.p);
-            bytes -= old->first;
-            by_size.erase(old);
+            by_size.insert({size, {p, clock++}});
         }
+        catch (const std::bad_alloc &)
+        {
+            return false;
+        }
+        bytes += size;
+        return true;
     }
-    void take_all(std::vector<void *> &out)
+    // the longest idle block, no longer kept, while there are more than `most` bytes in all, else NULL: without that, blocks of
+    // sizes that are not asked for again would fill the pool for good
+    void *beyond(size_t most)
     {
-        for (auto &b : by_size) out.push_back(b.second.p);
-        by_size.clear();
-        bytes = 0;
+        if (bytes <= most) return nullptr;
+        auto old = by_size.begin();
+        for (auto it = by_size.begin(); it != by_size.end(); ++it)
+            if (it->second.since < old->second.since) old = it;
+        void *p = old->second.p;
+        bytes -= old->first;
+        by_size.erase(old);
+        return p;
     }
 };
 

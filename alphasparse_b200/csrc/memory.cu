@@ -66,11 +66,11 @@ void stream_copy(unsigned char *dst, const unsigned char *src, size_t n) { memcp
 #endif
 
 // dst[0, n) from the segments, dst standing for offset `at` of their block
-void gather(unsigned char *dst, size_t at, size_t n, const std::vector<Stager::Segment> &seg)
+void gather(unsigned char *dst, size_t at, size_t n, const Stager::Segment *seg, size_t count)
 {
-    size_t i = (size_t)(std::upper_bound(seg.begin(), seg.end(), at, [](size_t o, const Stager::Segment &s) { return o < s.off; }) - seg.begin());
+    size_t i = (size_t)(std::upper_bound(seg, seg + count, at, [](size_t o, const Stager::Segment &s) { return o < s.off; }) - seg);
     if (i > 0) i--;
-    for (; i < seg.size() && seg[i].off < at + n; i++)
+    for (; i < count && seg[i].off < at + n; i++)
     {
         const size_t lo = std::max(at, seg[i].off), hi = std::min(at + n, seg[i].off + seg[i].bytes);
         if (lo < hi) stream_copy(dst + (lo - at), (const unsigned char *)seg[i].host + (lo - seg[i].off), hi - lo);
@@ -89,6 +89,24 @@ void parts(size_t n, F &&f)
 }
 } // namespace
 
+namespace
+{
+// frees the longest idle blocks until no more than `most` bytes are left (the device is current)
+void shrink(Pool &p, size_t most)
+{
+    for (;;)
+    {
+        void *q;
+        {
+            std::lock_guard<std::mutex> g(p.lock);
+            q = p.idle.beyond(most);
+        }
+        if (!q) return;
+        cudaFree(q);
+    }
+}
+} // namespace
+
 cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got)
 {
     const size_t unit = bytes < (1u << 20) ? (64u << 10) : (2u << 20);
@@ -104,33 +122,27 @@ cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got)
     if (e == cudaErrorMemoryAllocation)
     {
         cudaGetLastError();
-        std::vector<void *> idle;
-        {
-            std::lock_guard<std::mutex> g(p.lock);
-            p.idle.take_all(idle);
-        }
-        for (void *q : idle) cudaFree(q);
+        shrink(p, 0);
         e = cudaMalloc(out, want);
     }
     *got = want;
     return e;
 }
 
-void device_free(int device, void *ptr, size_t got)
+// (a destructor calls it: nothing may be thrown)
+void device_free(int device, void *ptr, size_t got) noexcept
 {
     if (!ptr) return;
     OnDevice on(device);
     Pool &p = pool(device);
-    std::vector<void *> out;
-    if (got <= kMostBlock && cudaDeviceSynchronize() == cudaSuccess)
+    bool kept = got <= kMostBlock && cudaDeviceSynchronize() == cudaSuccess;
+    if (kept)
     {
         std::lock_guard<std::mutex> g(p.lock);
-        if (p.contexts > 0) p.idle.put(ptr, got, kMostCached, out);
-        else out.push_back(ptr);
+        kept = p.contexts > 0 && p.idle.put(ptr, got);
     }
-    else
-        out.push_back(ptr);
-    for (void *q : out) cudaFree(q);
+    if (!kept) cudaFree(ptr);
+    shrink(p, kMostCached);
 }
 
 void device_pool_retain(int device)
@@ -143,14 +155,12 @@ void device_pool_retain(int device)
 void device_pool_release(int device)
 {
     Pool &p = pool(device);
-    std::vector<void *> idle;
     {
         std::lock_guard<std::mutex> g(p.lock);
         if (--p.contexts > 0) return;
-        p.idle.take_all(idle);
     }
     OnDevice on(device);
-    for (void *q : idle) cudaFree(q);
+    shrink(p, 0);
     host::host_pool_trim();
 }
 
@@ -230,22 +240,25 @@ cudaError_t Stager::take(int slots, unsigned char **p, int *event)
 cudaError_t Stager::to_device(void *dev, const void *host, size_t bytes, cudaStream_t st)
 {
     if (bytes < (64u << 10) || pinned(host)) return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
-    return to_device(dev, std::vector<Segment>(1, Segment{0, host, bytes}), st);
+    const Segment whole = {0, host, bytes};
+    return to_device(dev, &whole, 1, st);
 }
 
-cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaStream_t st)
+cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaStream_t st) { return to_device(dev, seg.data(), seg.size(), st); }
+
+cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaStream_t st)
 {
-    if (seg.empty()) return cudaSuccess;
-    if (!ready())
-    {
-        for (const Segment &s : seg)
+    if (count == 0) return cudaSuccess;
+    auto plain = [&]() {
+        for (size_t i = 0; i < count; i++)
         {
-            const cudaError_t e = cudaMemcpyAsync((unsigned char *)dev + s.off, s.host, s.bytes, cudaMemcpyHostToDevice, st);
+            const cudaError_t e = cudaMemcpyAsync((unsigned char *)dev + seg[i].off, seg[i].host, seg[i].bytes, cudaMemcpyHostToDevice, st);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
-    }
-    const size_t begin = seg.front().off, total = seg.back().off + seg.back().bytes - begin;
+    };
+    if (!ready()) return plain();
+    const size_t begin = seg[0].off, total = seg[count - 1].off + seg[count - 1].bytes - begin;
     const long long n_parts = (long long)((total + kPart - 1) / kPart);
     if (n_parts <= 3)
     {
@@ -254,7 +267,7 @@ cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaSt
         int i;
         cudaError_t e = take(1, &p, &i);
         if (e != cudaSuccess) return e;
-        gather(p, begin, total, seg);
+        gather(p, begin, total, seg, count);
         e = cudaMemcpyAsync((unsigned char *)dev + begin, p, total, cudaMemcpyHostToDevice, st);
         return e == cudaSuccess ? cudaEventRecord(done[i], st) : e;
     }
@@ -269,17 +282,26 @@ cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaSt
     };
     const long long slot_parts = (long long)(kPiece / kPart);
     std::vector<Piece> pieces;
-    std::vector<int> piece_of((size_t)n_parts);
-    for (long long q = 0, n = kFirstParts; q < n_parts; n = std::min(2 * n, kMostParts))
-    {
-        const long long e = n_parts - q <= n + n / 4 ? n_parts : q + n;
-        std::fill(piece_of.begin() + q, piece_of.begin() + e, (int)pieces.size());
-        pieces.push_back({q, e, (int)((e - q + slot_parts - 1) / slot_parts)});
-        q = e;
-    }
+    std::vector<int> piece_of;
     // The threads take parts in order; the calling one also sends every piece whose parts are in. A piece is opened (its slots of
     // the ring free again) before its parts may be filled.
-    std::unique_ptr<std::atomic<int>[]> filled(new std::atomic<int>[pieces.size()]);
+    std::unique_ptr<std::atomic<int>[]> filled;
+    try
+    {
+        piece_of.resize((size_t)n_parts);
+        for (long long q = 0, n = kFirstParts; q < n_parts; n = std::min(2 * n, kMostParts))
+        {
+            const long long e = n_parts - q <= n + n / 4 ? n_parts : q + n;
+            std::fill(piece_of.begin() + q, piece_of.begin() + e, (int)pieces.size());
+            pieces.push_back({q, e, (int)((e - q + slot_parts - 1) / slot_parts)});
+            q = e;
+        }
+        filled.reset(new std::atomic<int>[pieces.size()]);
+    }
+    catch (const std::bad_alloc &)
+    {
+        return plain();
+    }
     for (size_t k = 0; k < pieces.size(); k++) filled[k].store(0);
     std::atomic<long long> next_part(0), open_parts(0);
     std::atomic<bool> stop(false);
@@ -308,7 +330,7 @@ cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaSt
         } while (!next_part.compare_exchange_weak(q, q + 1));
         const Piece &k = pieces[piece_of[(size_t)q]];
         const size_t o = (size_t)q * kPart;
-        gather(k.p + (size_t)(q - k.part) * kPart, begin + o, std::min(kPart, total - o), seg);
+        gather(k.p + (size_t)(q - k.part) * kPart, begin + o, std::min(kPart, total - o), seg, count);
         filled[piece_of[(size_t)q]].fetch_add(1);
     };
     open_from(0);

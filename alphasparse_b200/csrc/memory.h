@@ -14,7 +14,7 @@ namespace asp
 // all per device (the longest idle ones go first), given back when the last context of the device is destroyed or an allocation fails. Safe from several threads.
 // device_free() waits for the device first, as cudaFree does: kernels in flight may still read the block.
 cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got);
-void device_free(int device, void *p, size_t got);
+void device_free(int device, void *p, size_t got) noexcept;
 void device_pool_retain(int device);  // a context was created ...
 void device_pool_release(int device); // ... or destroyed
 
@@ -50,6 +50,7 @@ class Stager
     cudaError_t to_device(void *dev, const void *host, size_t bytes, cudaStream_t st);
     // many arrays of one device block (ascending offsets): as few copies as the pieces make
     cudaError_t to_device(void *dev, const std::vector<Segment> &segments, cudaStream_t st);
+    cudaError_t to_device(void *dev, const Segment *segments, size_t count, cudaStream_t st);
     // complete on return
     cudaError_t to_host(void *host, const void *dev, size_t bytes, cudaStream_t st);
 };

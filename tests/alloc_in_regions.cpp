@@ -73,6 +73,24 @@ static bool graph(const char *spec)
     return st == ASP_OK || (st != ASP_ERR_ALLOC && !refused); // (a graph may not suit the matrix)
 }
 
+static bool validate()
+{
+    static asp_format *f = nullptr;
+    if (!f)
+    {
+        asp_matrix *m = nullptr;
+        const long n = countdown.exchange(-1);
+        if (asp_matrix_view_csr(kRows, kCols, ptr.data(), col.data(), val.data(), ASP_F32, &m) != ASP_OK) return false;
+        if (asp_graph_execute(m, "dense compress\nsub all row_padding 32 1\nsub all tlb_row\nsub all template K3", &f) != ASP_OK) return false;
+        asp_matrix_destroy(m);
+        countdown = n;
+    }
+    asp_plan_desc d;
+    if (asp_format_plan_descs(f, &d) != ASP_OK) return false;
+    std::vector<asp_plan_desc> many(200, d); // (so that the call's own tables are large allocations)
+    return asp_plan_descs_validate(many.data(), (int)many.size()) == ASP_OK;
+}
+
 int main(int argc, char **argv)
 {
     const std::string part = argc > 2 ? argv[2] : "";
@@ -119,6 +137,7 @@ int main(int argc, char **argv)
         printf("%s built after %ld failures\n", what, n);
     };
     run("layout", layout);
+    run("validate", validate);
     run("K2", [] { return graph("dense compress\nsub all row_padding 32 1\nsub all blb_row_evenly 32\nsub all tlb_row\nsub all template K2"); });
     run("K6", [] { return graph("dense sort 1\ndense compress\nsub all row_padding 32 1\nsub all blb_row_evenly 32\nsub all tlb_col_fixed 4\nsub all template K6"); });
     run("K9", [] { return graph("dense compress\nsub all tlb_nnz 16\nsub all template K9"); });

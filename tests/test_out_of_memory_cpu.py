@@ -17,7 +17,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("part", ["layout", "K2", "K6", "K9", "B1", "D1"])
+@pytest.mark.parametrize("part", ["layout", "validate", "K2", "K6", "K9", "B1", "D1"])
 @pytest.mark.parametrize("mode", ["region", "any"])
 def test_memory_runs_out(program, mode, part):
     r = subprocess.run([program, mode, part], capture_output=True, text=True, timeout=300, env=dict(os.environ, OMP_NUM_THREADS="4"))
