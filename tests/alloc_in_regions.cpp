@@ -62,7 +62,7 @@ static bool layout()
     return asp::tiled_build({t}, false, kRows, kCols, 148, out);
 }
 
-static bool graph(const char *spec)
+static bool graph(const char *spec) noexcept // (a C interface throws nothing)
 {
     asp_matrix *m = nullptr;
     asp_format *f = nullptr;
@@ -73,9 +73,10 @@ static bool graph(const char *spec)
     return st == ASP_OK || (st != ASP_ERR_ALLOC && !refused); // (a graph may not suit the matrix)
 }
 
-static bool validate()
+static bool validate() noexcept
 {
     static asp_format *f = nullptr;
+    static std::vector<asp_plan_desc> many; // (so that the call's own tables are large allocations)
     if (!f)
     {
         asp_matrix *m = nullptr;
@@ -83,11 +84,11 @@ static bool validate()
         if (asp_matrix_view_csr(kRows, kCols, ptr.data(), col.data(), val.data(), ASP_F32, &m) != ASP_OK) return false;
         if (asp_graph_execute(m, "dense compress\nsub all row_padding 32 1\nsub all tlb_row\nsub all template K3", &f) != ASP_OK) return false;
         asp_matrix_destroy(m);
+        many.resize(200);
+        for (asp_plan_desc &d : many)
+            if (asp_format_plan_descs(f, &d) != ASP_OK) return false;
         countdown = n;
     }
-    asp_plan_desc d;
-    if (asp_format_plan_descs(f, &d) != ASP_OK) return false;
-    std::vector<asp_plan_desc> many(200, d); // (so that the call's own tables are large allocations)
     return asp_plan_descs_validate(many.data(), (int)many.size()) == ASP_OK;
 }
 
