@@ -60,7 +60,7 @@ EXPORTS = [
     "asp_ctx_create", "asp_multicast_store", "asp_spmv_publish", "asp_plan_end_rows", "asp_rank_barrier", "asp_ctx_destroy", "asp_ctx_stream", "asp_plan_group_create", "asp_plan_descs_validate", "asp_plan_destroy",
     "asp_plan_set_launch", "asp_plan_get_launch", "asp_plan_set_tuning", "asp_plan_format_bytes", "asp_plan_launches", "asp_spmv", "asp_spmv_host", "asp_time",
     "asp_synchronize", "asp_status_str", "asp_last_error", "asp_built_for_sm100a", "asp_spmv_host_static",
-    "asp_static_stage_bytes", "asp_search_gpu", "asp_spmv_host_pipelined", "asp_dist_create", "asp_dist_destroy", "asp_dist_spmv", "asp_dist_spmv_iter", "asp_dist_status", "asp_plan_layout_bytes", "asp_host_alloc", "asp_host_free",
+    "asp_static_stage_bytes", "asp_search_gpu", "asp_spmv_host_pipelined", "asp_dist_create", "asp_dist_destroy", "asp_dist_spmv", "asp_dist_spmv_iter", "asp_dist_status", "asp_plan_layout_bytes", "asp_host_alloc", "asp_host_free", "asp_device_trim",
 ]
 
 _lib = None
@@ -126,6 +126,8 @@ def lib() -> C.CDLL:
     L.asp_plan_format_bytes.restype = C.c_uint64
     L.asp_plan_layout_bytes.argtypes = [C.c_void_p]
     L.asp_plan_layout_bytes.restype = C.c_uint64
+    L.asp_device_trim.argtypes = [C.c_int]
+    L.asp_device_trim.restype = C.c_int
     L.asp_host_alloc.argtypes = [C.c_size_t, C.POINTER(C.c_void_p)]
     L.asp_host_alloc.restype = C.c_int
     L.asp_host_free.argtypes = [C.c_void_p]
@@ -232,6 +234,11 @@ class _Results:
 
 
 _results = _Results()
+
+
+def device_trim(device: int = 0) -> None:
+    """asp_device_trim: the memory of destroyed plans that is kept for the next ones goes back to the device."""
+    check(lib().asp_device_trim(device))
 
 
 def multicast_store(src_ptr: int, multicast_ptr: int, nbytes: int, stream: int, ctas: int = 0) -> None:

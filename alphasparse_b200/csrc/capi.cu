@@ -491,7 +491,7 @@ asp_status ensure_xy(asp_ctx *ctx, size_t xb, size_t yb)
         if (ctx->x) cudaFree(ctx->x);
         ctx->x = nullptr;
         ctx->x_bytes = 0;
-        ASP_CUDA(cudaMalloc(&ctx->x, xb));
+        ASP_CUDA(asp::device_malloc(ctx->device, xb, &ctx->x));
         ctx->x_bytes = xb;
     }
     if (ctx->y_bytes < yb)
@@ -499,7 +499,7 @@ asp_status ensure_xy(asp_ctx *ctx, size_t xb, size_t yb)
         if (ctx->y) cudaFree(ctx->y);
         ctx->y = nullptr;
         ctx->y_bytes = 0;
-        ASP_CUDA(cudaMalloc(&ctx->y, yb));
+        ASP_CUDA(asp::device_malloc(ctx->device, yb, &ctx->y));
         ctx->y_bytes = yb;
     }
     return ASP_OK;
@@ -1257,6 +1257,15 @@ asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path)
 
 uint64_t asp_plan_layout_bytes(const asp_plan *plan) { return plan && plan->tiled ? plan->tiled->layout_bytes : 0; }
 
+asp_status asp_device_trim(int device)
+{
+    int n = 0;
+    ASP_CUDA(cudaGetDeviceCount(&n));
+    if (device < 0 || device >= n) return fail(ASP_ERR_INVALID_ARG, "no such CUDA device");
+    asp::device_trim(device);
+    return ASP_OK;
+}
+
 asp_status asp_host_alloc(size_t bytes, void **out)
 {
     if (!out || bytes == 0) return fail(ASP_ERR_INVALID_ARG, "out is NULL or bytes == 0");
@@ -1717,7 +1726,7 @@ asp_status asp_dist_create(asp_ctx *ctx, const asp_dist_desc *desc, asp_dist **o
     {
         ASP_CUDA(cudaStreamCreateWithFlags(&d->comm, cudaStreamNonBlocking));
         ASP_CUDA(cudaEventCreateWithFlags(&d->exchanged, cudaEventDisableTiming));
-        ASP_CUDA(cudaMalloc((void **)&d->status, 256));
+        ASP_CUDA(asp::device_malloc(ctx->device, 256, (void **)&d->status));
         ASP_CUDA(cudaMemsetAsync(d->status, 0, 256, ctx->stream));
     }
     *out = d.release();

@@ -117,16 +117,27 @@ cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got)
         *out = p.idle.take(want, unit, got);
         if (*out) return cudaSuccess;
     }
+    *got = want;
+    return device_malloc(device, want, out);
+}
+
+cudaError_t device_malloc(int device, size_t bytes, void **out)
+{
     OnDevice on(device);
-    cudaError_t e = cudaMalloc(out, want);
+    cudaError_t e = cudaMalloc(out, bytes);
     if (e == cudaErrorMemoryAllocation)
     {
         cudaGetLastError();
-        shrink(p, 0);
-        e = cudaMalloc(out, want);
+        shrink(pool(device), 0);
+        e = cudaMalloc(out, bytes);
     }
-    *got = want;
     return e;
+}
+
+void device_trim(int device)
+{
+    OnDevice on(device);
+    shrink(pool(device), 0);
 }
 
 // (a destructor calls it: nothing may be thrown)

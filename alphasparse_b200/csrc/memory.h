@@ -11,10 +11,14 @@ namespace asp
 {
 // Device memory for plans. cudaMalloc and cudaFree of a plan's arena take one to three milliseconds each on this part, more than
 // everything else that makes a small plan; freed arenas are therefore kept for the next plan: blocks of at most 256 MB, 1 GB in
-// all per device (the longest idle ones go first), given back when the last context of the device is destroyed or an allocation fails. Safe from several threads.
+// all per device (the longest idle ones go first), given back when the last context of the device is destroyed, by device_trim(), or when
+// an allocation of this library fails. Safe from several threads.
 // device_free() waits for the device first, as cudaFree does: kernels in flight may still read the block.
 cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got);
 void device_free(int device, void *p, size_t got) noexcept;
+// cudaMalloc, a second time without idle blocks if the first fails: for whatever does not come from the pool
+cudaError_t device_malloc(int device, size_t bytes, void **out);
+void device_trim(int device);
 void device_pool_retain(int device);  // a context was created ...
 void device_pool_release(int device); // ... or destroyed
 

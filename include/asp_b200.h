@@ -181,9 +181,12 @@ void *asp_ctx_stream(asp_ctx *ctx);
  * Every entry point makes the context's device current for its own duration and restores the
  * caller's device before it returns. */
 asp_status asp_plan_group_create(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp_plan **out_plans);
-/* (The device memory of destroyed plans is kept for the next ones: blocks of at most 256 MB, 1 GB per device, given back when
- * the device's last context is destroyed or an allocation fails.) */
+/* (The device memory of destroyed plans is kept for the next ones: blocks of at most 256 MB, 1 GB per device. It is given back when
+ * the device's last context is destroyed, when an allocation of this library on the device fails (a plan's, the staging buffers of
+ * asp_spmv_host and asp_time, the status word of asp_dist_create), and by asp_device_trim.) */
 void asp_plan_destroy(asp_plan *plan);
+/* Gives idle device memory back at once, for another allocator of the process. */
+asp_status asp_device_trim(int device);
 /* The validation of asp_plan_group_create on its own: same checks, same status and message, no device
  * needed, nothing allocated or uploaded. For a caller that wants to vet template arrays (a loaded
  * format file, the output of its own operators) before it touches a GPU. The reference has no

@@ -223,6 +223,23 @@ int main(int, char **argv)
         }
         s.release();
     }
+    if (part == "full device")
+    {
+        // idle blocks fill the device: allocations of every kind get them, and a trim call gives them back
+        void *p[3], *q = nullptr;
+        size_t got[3];
+        fake::limit = 100u << 20;
+        for (int i = 0; i < 3; i++) need(asp::device_alloc(0, (30u << 20) + i * (2u << 20), &p[i], &got[i]) == cudaSuccess, "device_alloc");
+        for (int i = 0; i < 3; i++) asp::device_free(0, p[i], got[i]);
+        need(fake::in_use > (90u << 20), "the pool keeps nothing");
+        need(asp::device_malloc(0, 60u << 20, &q) == cudaSuccess, "an allocation beside the pool");
+        cudaFree(q);
+        for (int i = 0; i < 3; i++) need(asp::device_alloc(0, 30u << 20, &p[i], &got[i]) == cudaSuccess, "device_alloc");
+        for (int i = 0; i < 3; i++) asp::device_free(0, p[i], got[i]);
+        need(fake::in_use > 0, "the pool keeps nothing");
+        asp::device_trim(0);
+        need(fake::in_use == 0, "idle blocks after a trim");
+    }
     asp::device_pool_release(0);
     need(fake::blocks.empty(), "device memory is left");
     printf("%s: ok\n", part.c_str());

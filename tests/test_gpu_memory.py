@@ -95,3 +95,19 @@ def test_csr5_like_rows_left_uncleared(asp_ctx, template, s, empty):
     refdump.assert_y(dy.cpu().numpy(), y_ref, scale, np.float32, f"{template} {s} {empty}")
     g.close()
     fmt.close()
+
+
+def test_idle_memory_is_given_back(asp_ctx):
+    import torch
+    from alphasparse_b200 import capi
+
+    m, x = M.from_row_lengths(np.full(200_000, 40), 200_000, seed=4, dtype=np.float64)  # 100 MB of plan
+    fmt, g = tuner.build(asp_ctx, m, desc("K3", ["row_padding 32 1", "tlb_row"]))
+    held = g.format_bytes() + g.layout_bytes()
+    g.close()
+    fmt.close()
+    before = torch.cuda.mem_get_info()[0]
+    capi.device_trim(0)
+    assert torch.cuda.mem_get_info()[0] >= before + held * 0.9
+    with pytest.raises(capi.AspError):
+        capi.device_trim(1000)
