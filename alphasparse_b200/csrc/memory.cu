@@ -268,6 +268,7 @@ cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaS
         }
         return cudaSuccess;
     };
+    std::lock_guard<std::mutex> turn(one);
     if (!ready()) return plain();
     const size_t begin = seg[0].off, total = seg[count - 1].off + seg[count - 1].bytes - begin;
     const long long n_parts = (long long)((total + kPart - 1) / kPart);
@@ -371,11 +372,13 @@ cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaS
 
 cudaError_t Stager::to_host(void *host, const void *dev, size_t bytes, cudaStream_t st)
 {
-    if (bytes < (256u << 10) || pinned(host) || !ready())
-    {
+    auto plain = [&]() {
         const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
         return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
-    }
+    };
+    if (bytes < (256u << 10) || pinned(host)) return plain();
+    std::lock_guard<std::mutex> turn(one);
+    if (!ready()) return plain();
     const size_t piece = std::min(kPiece, std::max<size_t>(256u << 10, (bytes / 8 + kPart - 1) / kPart * kPart)), n_pieces = (bytes + piece - 1) / piece;
     cudaError_t e = cudaSuccess;
     int at[kPieces];

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <mutex>
 #include <vector>
 
 namespace asp
@@ -30,6 +31,7 @@ class Stager
 {
     static const size_t kPiece = 1u << 20;
     static const int kPieces = 16;
+    std::mutex one; // copies of several threads take turns: they share the ring
     unsigned char *ring = nullptr;
     cudaEvent_t done[kPieces] = {};
     int owner[kPieces] = {}; // event that a slot is free after

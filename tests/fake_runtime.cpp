@@ -179,7 +179,7 @@ static void ring(asp::Stager &s, unsigned seed, int rounds)
             }
             need(s.to_device(dev.data(), seg, nullptr) == cudaSuccess, "to_device of segments");
         }
-        if (n >= (64u << 10) || true) memset(src.data(), 0x55, n);
+        memset(src.data(), 0x55, n);
         need(s.to_host(back.data(), dev.data(), n, nullptr) == cudaSuccess, "to_host");
         need(back == keep, "an upload or a download is damaged");
     }
@@ -194,6 +194,15 @@ int main(int, char **argv)
     {
         asp::Stager s;
         ring(s, 1, 36);
+        s.release();
+    }
+    if (part == "threads")
+    {
+        // two threads, one context's ring (a program that makes plans in the background)
+        asp::Stager s;
+        std::thread a([&] { omp_set_num_threads(2); ring(s, 2, 36); }), b([&] { omp_set_num_threads(2); ring(s, 7, 36); });
+        a.join();
+        b.join();
         s.release();
     }
     if (part == "no memory")
