@@ -1211,11 +1211,9 @@ asp_status asp_plan_get_launch(const asp_plan *plan, int64_t *tblock_num, int64_
     return ASP_OK;
 }
 
-asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path)
+static asp_status set_tuning(asp_plan *plan, int vec, int path)
 {
-    if (!plan) return fail(ASP_ERR_INVALID_ARG, "plan is NULL");
     const int t = plan->templ;
-    plan->tiled.reset(); // the caller experiments with this plan's own kernel
     if (t == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE || t == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE)
     {
         if (vec != 0) return fail(ASP_ERR_INVALID_ARG, "the CSR5-like family has no vec knob");
@@ -1253,6 +1251,14 @@ asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path)
     }
     if (plan->asked_threads > 0) return apply_launch(nullptr, plan, plan->asked_tblock, plan->asked_threads, plan->asked_reduce);
     return ASP_OK;
+}
+
+asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path)
+{
+    if (!plan) return fail(ASP_ERR_INVALID_ARG, "plan is NULL");
+    const asp_status st = set_tuning(plan, vec, path);
+    if (st == ASP_OK) plan->tiled.reset(); // the caller experiments with this plan's own kernel
+    return st;
 }
 
 uint64_t asp_plan_layout_bytes(const asp_plan *plan) { return plan && plan->tiled ? plan->tiled->layout_bytes : 0; }

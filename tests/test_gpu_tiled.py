@@ -146,3 +146,18 @@ def test_tiled_sums_are_one_call_s_own(asp_ctx, dtype):
     other.close()
     g.close()
     fmt.close()
+
+
+def test_a_refused_tuning_call_keeps_the_layout(asp_ctx):
+    m, x = matrix(np.float32, 3 * TILE[np.float32], seed=3)
+    y_ref, scale = refdump.csr_ref(m, x)
+    for template, vec in (("K9", 1), ("K4", 0), ("K2", 3), ("K2", 8)):
+        fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template, "threads": 128, "row_reduce": 1}]})
+        held = g.layout_bytes()
+        assert held > 0
+        with pytest.raises(capi.AspError):
+            g.set_tuning(0, vec, 0)
+        assert g.layout_bytes() == held
+        refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, template)
+        g.close()
+        fmt.close()
