@@ -20,6 +20,7 @@ DTYPE_OF_NP = {np.dtype(np.uint8): U8, np.dtype(np.uint16): U16, np.dtype(np.uin
                np.dtype(np.float32): F32, np.dtype(np.float64): F64}
 NP_OF_NAME = {"u8": np.uint8, "u16": np.uint16, "u32": np.uint32, "u64": np.uint64, "f32": np.float32, "f64": np.float64}
 COMPRESS = {"none": 0, "linear": 1, "constant": 2, "branch": 3, "cycle_linear": 4, "cycle_increase": 5}
+LAYOUT = {"auto": 0, "none": 1}
 TEMPLATE = {"K1": 0, "K2": 1, "K3": 2, "K5": 3, "K6": 4, "K7": 5, "K8": 6, "K4": 7, "K9": 8, "K10": 9, "EMPTY": 10, "B1": 11, "D1": 12}
 TEMPLATE_NAME = {
     0: "DIRECT_ATOM_TEMPLATE", 1: "DIRECT_ATOM_TEMPLATE_WARP_COMPRESS", 2: "DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS",
@@ -60,7 +61,7 @@ EXPORTS = [
     "asp_ctx_create", "asp_multicast_store", "asp_spmv_publish", "asp_plan_end_rows", "asp_rank_barrier", "asp_ctx_destroy", "asp_ctx_stream", "asp_plan_group_create", "asp_plan_descs_validate", "asp_plan_destroy",
     "asp_plan_set_launch", "asp_plan_get_launch", "asp_plan_set_tuning", "asp_plan_format_bytes", "asp_plan_launches", "asp_spmv", "asp_spmv_host", "asp_time",
     "asp_synchronize", "asp_status_str", "asp_last_error", "asp_built_for_sm100a", "asp_spmv_host_static",
-    "asp_static_stage_bytes", "asp_search_gpu", "asp_spmv_host_pipelined", "asp_dist_create", "asp_dist_destroy", "asp_dist_spmv", "asp_dist_spmv_iter", "asp_dist_status", "asp_plan_layout_bytes", "asp_host_alloc", "asp_host_free", "asp_device_trim",
+    "asp_static_stage_bytes", "asp_search_gpu", "asp_spmv_host_pipelined", "asp_dist_create", "asp_dist_destroy", "asp_dist_spmv", "asp_dist_spmv_iter", "asp_dist_status", "asp_plan_layout_bytes", "asp_host_alloc", "asp_host_free", "asp_device_trim", "asp_plan_group_create_with",
 ]
 
 _lib = None
@@ -126,6 +127,8 @@ def lib() -> C.CDLL:
     L.asp_plan_format_bytes.restype = C.c_uint64
     L.asp_plan_layout_bytes.argtypes = [C.c_void_p]
     L.asp_plan_layout_bytes.restype = C.c_uint64
+    L.asp_plan_group_create_with.argtypes = [C.c_void_p, C.POINTER(PlanDesc), C.c_int, C.c_int, C.POINTER(C.c_void_p)]
+    L.asp_plan_group_create_with.restype = C.c_int
     L.asp_device_trim.argtypes = [C.c_int]
     L.asp_device_trim.restype = C.c_int
     L.asp_host_alloc.argtypes = [C.c_size_t, C.POINTER(C.c_void_p)]
@@ -319,15 +322,15 @@ def validate_descs(descs: list[PlanDesc]) -> None:
 
 class PlanGroup:
     """All sub-matrix plans of one matrix (asp_plan_group_create). Keeps the host arrays alive
-    until upload has finished."""
+    until upload has finished. layout: "auto", or "none" for a group that always runs its templates' own kernels."""
 
-    def __init__(self, ctx: Context, descs: list[PlanDesc], keepalive=None):
+    def __init__(self, ctx: Context, descs: list[PlanDesc], keepalive=None, layout: str = "auto"):
         self.ctx = ctx
         n = len(descs)
         self._descs = (PlanDesc * n)(*descs)
         self._plans = (C.c_void_p * n)()
         self._keep = keepalive
-        check(lib().asp_plan_group_create(ctx.handle, self._descs, n, self._plans))
+        check(lib().asp_plan_group_create_with(ctx.handle, self._descs, n, LAYOUT[layout], self._plans))
         self.n = n
         self._spmv = lib().asp_spmv
         self.val_dtype = np.float64 if descs[0].val_dtype == F64 else np.float32

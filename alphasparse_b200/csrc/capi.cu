@@ -612,7 +612,7 @@ namespace
 {
 // dry == true: everything asp_plan_group_create checks, without a device (no allocation, no upload, no
 // plan objects returned); ctx may then be NULL.
-asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp_plan **out_plans, bool dry)
+asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int layout, asp_plan **out_plans, bool dry)
 {
 
     // ---- pass 1: validate descriptors, lay out the arena (arrays sharing a host pointer once)
@@ -1071,8 +1071,8 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp
     }
     // scattered columns: the column-tiled layout of the whole group (kernels_tiled.cu), where it is the faster one
     std::vector<asp::TiledSource> src;
-    bool same = true;
-    for (int i = 0; i < n; i++)
+    bool same = layout == ASP_LAYOUT_AUTO;
+    for (int i = 0; i < n && same; i++)
     {
         same = same && descs[i].val_dtype == descs[0].val_dtype && descs[i].n_rows == descs[0].n_rows && descs[i].n_cols == descs[0].n_cols;
         if (descs[i].template_type == ASP_EMPTY_TEMPLATE) same = false; // a group with parts left out is a trial of one part
@@ -1151,12 +1151,18 @@ extern "C" {
 
 asp_status asp_plan_group_create(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp_plan **out_plans)
 {
+    return asp_plan_group_create_with(ctx, descs, n, ASP_LAYOUT_AUTO, out_plans);
+}
+
+asp_status asp_plan_group_create_with(asp_ctx *ctx, const asp_plan_desc *descs, int n, int layout, asp_plan **out_plans)
+{
     if (!ctx || !descs || !out_plans || n <= 0) return fail(ASP_ERR_INVALID_ARG, "NULL argument or n <= 0");
     for (int i = 0; i < n; i++) out_plans[i] = nullptr;
+    if (layout != ASP_LAYOUT_AUTO && layout != ASP_LAYOUT_NONE) return fail(ASP_ERR_INVALID_ARG, "unknown layout");
     ASP_ON_DEVICE(ctx);
     try
     {
-        return plan_group_build(ctx, descs, n, out_plans, false);
+        return plan_group_build(ctx, descs, n, layout, out_plans, false);
     }
     catch (const std::bad_alloc &)
     {
@@ -1184,7 +1190,7 @@ asp_status asp_plan_descs_validate(const asp_plan_desc *descs, int n)
                 for (asp_plan *p : all) delete p;
             }
         } plans{scratch};
-        return plan_group_build(nullptr, descs, n, scratch.data(), true);
+        return plan_group_build(nullptr, descs, n, ASP_LAYOUT_NONE, scratch.data(), true);
     }
     catch (const std::bad_alloc &)
     {

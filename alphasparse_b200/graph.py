@@ -295,9 +295,9 @@ class Format:
             out[_ROLE_NAME[a.role]] = (arr, comp, int(a.dtype), int(a.len))
         return out
 
-    def upload(self, ctx: capi.Context) -> capi.PlanGroup:
-        """asp_plan_group_create over every sub-matrix of this format."""
-        return capi.PlanGroup(ctx, self.plan_descs(), keepalive=self)
+    def upload(self, ctx: capi.Context, layout: str = "auto") -> capi.PlanGroup:
+        """asp_plan_group_create_with over every sub-matrix of this format."""
+        return capi.PlanGroup(ctx, self.plan_descs(), keepalive=self, layout=layout)
 
     def close(self):
         if self._h and self._owned:

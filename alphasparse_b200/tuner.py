@@ -165,15 +165,15 @@ def search_with_timer(m: CsrMatrix, time_fn, quick: bool = True, warmup: int = 2
     return out
 
 
-def build(ctx: capi.Context, m: CsrMatrix, desc: dict):
-    """Lower and upload exactly the graph a previous search() described (no timing)."""
+def build(ctx: capi.Context, m: CsrMatrix, desc: dict, layout: str = "auto"):
+    """Lower and upload exactly the graph a previous search() described (no timing). layout: as PlanGroup takes it."""
     hm = Matrix.view_csr(m)
     cm = hm.dense(desc["dense"].replace(" | ", "\n"))
     if cm.n_subs != len(desc["subs"]):
         raise ValueError(f"graph describes {len(desc['subs'])} sub-matrices, the dense view gives {cm.n_subs}")
     spec = "\n".join(Candidate(s["graph"], s["nodes"], s["template"], []).lines(i) for i, s in enumerate(desc["subs"]))
     fmt = cm.execute(spec)
-    group = fmt.upload(ctx)
+    group = fmt.upload(ctx, layout)
     for i, s in enumerate(desc["subs"]):
         set_launch(fmt, group, i, s["threads"], s["row_reduce"])
     cm.close()

@@ -175,12 +175,23 @@ void *asp_ctx_stream(asp_ctx *ctx);
  * Where the columns are so scattered that the gathers of x, not the bytes, bound the templates' kernels, the whole group
  * is also laid out by column tiles (csrc/kernels_tiled.cu; about 1.5 times the format's device memory in all), and asp_spmv
  * over the complete group runs that layout; a group with EMPTY plans never does. Sums are then taken in another order from
- * call to call, as with every template that accumulates with atomics. Rows that are added up in many parts have 64-bit sums in
+ * call to call, as with every template that accumulates with atomics (asp_plan_group_create_with can forbid it). Rows that are added up in many parts have 64-bit sums in
  * the group's device memory: a group with such rows runs the layout in the calls of the context that created it, and its
  * templates' kernels in calls of another context and in calls that a stream capture records.
  * Every entry point makes the context's device current for its own duration and restores the
  * caller's device before it returns. */
 asp_status asp_plan_group_create(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp_plan **out_plans);
+/* The same, with a say in the column-tiled layout (asp_plan_group_create: ASP_LAYOUT_AUTO). ASP_LAYOUT_NONE: the group always
+ * runs its templates' kernels. For plans that are used once or a few times (building the layout takes as long as hundreds of the
+ * calls that it shortens), for device memory that has no room for it, for trials of launch parameters, and for results that
+ * repeat bit for bit: without atomics (is_atom_add == 0; not the CSR5-like templates) every row is then summed in one fixed order,
+ * whichever other plans of the group are EMPTY. */
+typedef enum
+{
+    ASP_LAYOUT_AUTO = 0,
+    ASP_LAYOUT_NONE = 1
+} asp_layout;
+asp_status asp_plan_group_create_with(asp_ctx *ctx, const asp_plan_desc *descs, int n, int layout, asp_plan **out_plans);
 /* (The device memory of destroyed plans is kept for the next ones: blocks of at most 256 MB, 1 GB per device. It is given back when
  * the device's last context is destroyed, when an allocation of this library on the device fails (a plan's, the staging buffers of
  * asp_spmv_host and asp_time, the status word of asp_dist_create), and by asp_device_trim.) */

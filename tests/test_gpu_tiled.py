@@ -45,9 +45,11 @@ def test_tiled_group_matches_the_oracle(asp_ctx, template, dtype, tiles, over, l
             y = dy.cpu().numpy()
             refdump.assert_y(y[shift : shift + m.n_rows], y_ref, scale, m.values.dtype, f"{template} zero_y={zero_y} shift={shift}")
             assert (y[:shift] == 7).all() and (y[shift + m.n_rows :] == 7).all()  # nothing beside y
-    g.set_tuning(0, 0, 0) if template in ("K2", "K3", "K9", "K10") else None  # back to the template's own kernel
-    refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, f"{template} own kernel")
     g.close()
+    own = fmt.upload(asp_ctx, layout="none")
+    assert own.layout_bytes() == 0
+    refdump.assert_y(own.spmv_host(x), y_ref, scale, m.values.dtype, f"{template} own kernel")
+    own.close()
     fmt.close()
 
 
@@ -63,11 +65,13 @@ def test_tiled_group_of_sorted_strips_and_empty_rows(asp_ctx):
     hm = Matrix.from_csr(m)
     cm = hm.dense("dense sort 1\ndense rowdiv_exp 128 4096 8\ndense compress")
     desc = {"dense": "dense sort 1 | dense rowdiv_exp 128 4096 8 | dense compress", "subs": [sub("K2" if cm.sub_rows(i)[3] <= 128 else "K6" if cm.sub_rows(i)[3] <= 1024 else "K7") for i in range(cm.n_subs)]}
-    fmt, g = tuner.build(asp_ctx, m, desc)
     y_ref, scale = refdump.csr_ref(m, x)
-    refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, "strips")
-    g.close()
-    fmt.close()
+    for layout in ("auto", "none"):
+        fmt, g = tuner.build(asp_ctx, m, desc, layout)
+        assert (g.layout_bytes() > 0) == (layout == "auto")
+        refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, f"strips {layout}")
+        g.close()
+        fmt.close()
     cm.close()
     hm.close()
 
@@ -161,3 +165,27 @@ def test_a_refused_tuning_call_keeps_the_layout(asp_ctx):
         refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, template)
         g.close()
         fmt.close()
+
+
+@pytest.mark.parametrize("template", ["K2", "K3", "K6", "K8"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_results_repeat_bit_for_bit_without_the_layout(asp_ctx, template, dtype):
+    m, x = matrix(dtype, 3 * TILE[dtype], seed=5)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template, "threads": 128, "row_reduce": 1}]}, "none")
+    y = g.spmv_host(x).copy()
+    for _ in range(5):
+        assert np.array_equal(g.spmv_host(x), y)
+    g.close()
+    fmt.close()
+
+
+def test_an_unknown_layout_is_refused(asp_ctx):
+    m, _ = M.uniform_random(300, 6, seed=1)
+    from alphasparse_b200.graph import Matrix
+
+    fmt = Matrix.from_csr(m).execute("dense compress\nsub all row_padding 32 1\nsub all tlb_row\nsub all template K3")
+    descs = fmt.plan_descs()
+    plans = (capi.C.c_void_p * len(descs))()
+    with pytest.raises(capi.AspError):
+        capi.check(capi.lib().asp_plan_group_create_with(asp_ctx.handle, (capi.PlanDesc * len(descs))(*descs), len(descs), 7, plans))
+    fmt.close()
