@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../../include/asp_b200_host.h"
+#include "search.hpp"
 
 namespace
 {
@@ -474,6 +475,7 @@ thread_local std::string g_text;
 
 struct asp_search_result
 {
+    int layout = ASP_LAYOUT_AUTO;
     std::string dense;
     std::vector<std::string> sub_spec, sub_name;
     std::vector<Launch> launch;
@@ -506,7 +508,14 @@ int64_t asp_search_derive_tblock(int template_type, uint64_t n_tlb, uint64_t n_w
     return derive_tblock(template_type, n_tlb, n_wlb, n_blb, threads > 0 ? threads : 1);
 }
 
-asp_status asp_search(const asp_matrix *m, const asp_search_options *opt_, asp_time_fn time_fn, void *time_user, asp_search_result **out)
+asp_status asp_search(const asp_matrix *m, const asp_search_options *opt, asp_time_fn time_fn, void *time_user, asp_search_result **out)
+{
+    return asp::host::search(m, opt, time_fn, nullptr, time_user, out);
+}
+
+} // extern "C"
+
+asp_status asp::host::search(const asp_matrix *m, const asp_search_options *opt_, asp_time_fn time_fn, time_layout_fn layout_fn, void *time_user, asp_search_result **out)
 {
     if (!m || !time_fn || !out) return ASP_ERR_INVALID_ARG;
     *out = nullptr;
@@ -630,7 +639,7 @@ asp_status asp_search(const asp_matrix *m, const asp_search_options *opt_, asp_t
                 }
                 if (opt.prune_gbs > 0 && have)
                 {
-                    // sound pruning: the kernel has to read every byte of the format at least once
+                    // sound pruning: the template's kernel, which is what a trial times, has to read every byte of the format at least once
                     std::vector<asp_plan_desc> descs(n);
                     uint64_t bytes = 0;
                     if (asp_format_plan_descs(f.get(), descs.data()) == ASP_OK)
@@ -720,11 +729,24 @@ asp_status asp_search(const asp_matrix *m, const asp_search_options *opt_, asp_t
         char buf[160];
         snprintf(buf, sizeof buf, "  whole matrix: %.1f us  %.1f GFLOP/s", ms * 1e3, 2.0 * (double)total_nnz * 1e-6 / ms);
         log(buf);
+        int layout = layout_fn ? ASP_LAYOUT_NONE : ASP_LAYOUT_AUTO;
+        float layout_ms = 0;
+        if (layout_fn && layout_fn(time_user, f.get(), opt.warmup, std::max(opt.reps, 20), &layout_ms) == 0 && layout_ms > 0)
+        {
+            snprintf(buf, sizeof buf, "  whole matrix, column-tiled layout: %.1f us  %.1f GFLOP/s", layout_ms * 1e3, 2.0 * (double)total_nnz * 1e-6 / layout_ms);
+            log(buf);
+            if (layout_ms < ms)
+            {
+                layout = ASP_LAYOUT_AUTO;
+                ms = layout_ms;
+            }
+        }
         if (!best || ms < best->ms)
         {
             best.reset(new asp_search_result());
             best->dense = dense;
             best->ms = ms;
+            best->layout = layout;
             for (int i = 0; i < n; i++)
             {
                 best->sub_spec.push_back(picks[i].cand.lines(i));
@@ -739,6 +761,8 @@ asp_status asp_search(const asp_matrix *m, const asp_search_options *opt_, asp_t
     return ASP_OK;
 }
 
+extern "C" {
+
 void asp_search_result_destroy(asp_search_result *r) { delete r; }
 const char *asp_search_result_dense(const asp_search_result *r) { return r ? r->dense.c_str() : ""; }
 int asp_search_result_num_subs(const asp_search_result *r) { return r ? (int)r->sub_spec.size() : 0; }
@@ -751,6 +775,7 @@ asp_status asp_search_result_sub_launch(const asp_search_result *r, int i, int64
     *reduce = r->launch[i].reduce;
     return ASP_OK;
 }
+int asp_search_result_layout(const asp_search_result *r) { return r ? r->layout : ASP_LAYOUT_AUTO; }
 float asp_search_result_ms(const asp_search_result *r) { return r ? r->ms : 0.f; }
 int asp_search_result_num_trials(const asp_search_result *r) { return r ? (int)r->trials.size() : 0; }
 const char *asp_search_result_trial(const asp_search_result *r, int i) { return (r && i >= 0 && i < (int)r->trials.size()) ? r->trials[i].c_str() : ""; }

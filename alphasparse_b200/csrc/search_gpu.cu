@@ -1,5 +1,7 @@
 // asp_search with the GPU as the timer: a trial's format is uploaded once, its launch parameters are
 // swept in place, and asp_time measures it (replaces the reference's emit + nvcc + run per trial).
+// Trials run the templates' kernels, whole matrices as well as one strip with the others EMPTY. The column-tiled layout, which takes
+// no launch parameters and is the same for every template, is timed once per dense view, on the winners' format.
 //
 // Launch requests that the kernels fold into the same effective launch (a CTA width above a family's compiled
 // bound becomes more CTAs, grids are cut to the CTAs that have work: asp_plan_get_launch) are timed once: a
@@ -12,6 +14,7 @@
 
 #include "../../include/asp_b200.h"
 #include "../../include/asp_b200_host.h"
+#include "host/search.hpp"
 
 namespace
 {
@@ -45,7 +48,7 @@ int time_on_gpu(void *user, const asp_format *fmt, const int64_t *tblock, const 
         std::vector<asp_plan_desc> descs(n);
         if (asp_format_plan_descs(fmt, descs.data()) != ASP_OK) return 1;
         t->plans.assign(n, nullptr);
-        if (asp_plan_group_create(t->ctx, descs.data(), n, t->plans.data()) != ASP_OK)
+        if (asp_plan_group_create_with(t->ctx, descs.data(), n, ASP_LAYOUT_NONE, t->plans.data()) != ASP_OK)
         {
             t->plans.clear();
             return 1;
@@ -84,6 +87,23 @@ int time_on_gpu(void *user, const asp_format *fmt, const int64_t *tblock, const 
     t->measured++;
     return 0;
 }
+
+int time_layout_on_gpu(void *user, const asp_format *fmt, int warmup, int reps, float *ms)
+{
+    GpuTimer *t = static_cast<GpuTimer *>(user);
+    t->drop(); // (device memory for the layout)
+    const int n = asp_format_num_subs(fmt);
+    if (n <= 0) return 1;
+    std::vector<asp_plan_desc> descs(n);
+    if (asp_format_plan_descs(fmt, descs.data()) != ASP_OK) return 1;
+    t->plans.assign(n, nullptr);
+    bool ok = asp_plan_group_create_with(t->ctx, descs.data(), n, ASP_LAYOUT_AUTO, t->plans.data()) == ASP_OK && asp_plan_layout_bytes(t->plans[0]) > 0;
+    float gflops = 0;
+    // (with y cleared: the calls in which the layout runs whatever rows are empty)
+    ok = ok && asp_time(t->ctx, t->plans.data(), n, warmup, reps, 1, 0.0, ms, &gflops) == ASP_OK;
+    t->drop();
+    return ok ? 0 : 1;
+}
 } // namespace
 
 extern "C" asp_status asp_search_gpu(asp_ctx *ctx, const void *matrix, const void *options, void **result)
@@ -92,7 +112,7 @@ extern "C" asp_status asp_search_gpu(asp_ctx *ctx, const void *matrix, const voi
     GpuTimer timer{ctx};
     asp_search_result *r = nullptr;
     const asp_search_options *opt = static_cast<const asp_search_options *>(options);
-    const asp_status st = asp_search(static_cast<const asp_matrix *>(matrix), opt, time_on_gpu, &timer, &r);
+    const asp_status st = asp::host::search(static_cast<const asp_matrix *>(matrix), opt, time_on_gpu, time_layout_on_gpu, &timer, &r);
     if (opt && opt->log_fn)
     {
         char line[160];

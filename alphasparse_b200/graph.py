@@ -24,7 +24,7 @@ HOST_EXPORTS = [
     "asp_format_sub_info", "asp_format_plan_descs", "asp_format_padding_rate", "asp_host_last_error",
     "asp_dense_execute", "asp_matrix_num_subs", "asp_matrix_sub_rows", "asp_partition_rows_by_nnz", "asp_matrix_relabel_by_column_count", "asp_format_id", "asp_format_save", "asp_format_load",
     "asp_search", "asp_search_result_destroy", "asp_search_result_dense", "asp_search_result_num_subs", "asp_search_result_sub_spec",
-    "asp_search_result_sub_name", "asp_search_result_sub_launch", "asp_search_result_ms", "asp_search_result_num_trials",
+    "asp_search_result_sub_name", "asp_search_result_sub_launch", "asp_search_result_layout", "asp_search_result_ms", "asp_search_result_num_trials",
     "asp_search_result_trial", "asp_search_candidates", "asp_search_derive_tblock",
 ]
 
@@ -104,6 +104,8 @@ def _lib():
             fn.restype = C.c_char_p
         L.asp_search_result_sub_launch.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
         L.asp_search_result_sub_launch.restype = C.c_int
+        L.asp_search_result_layout.argtypes = [C.c_void_p]
+        L.asp_search_result_layout.restype = C.c_int
         L.asp_search_result_ms.argtypes = [C.c_void_p]
         L.asp_search_result_ms.restype = C.c_float
         L.asp_search_result_num_trials.argtypes = [C.c_void_p]

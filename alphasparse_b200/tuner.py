@@ -13,7 +13,8 @@ reference's tuner:
   * optionally the stop rule of search_strategy.cc per sub-matrix sweep.
 Every trial is an in-process lowering + upload + CUDA-event timing through the C ABI instead of an
 nvcc compile and an ~8 s run of a generated program; sub-matrices not under test carry the EMPTY
-template, as in the reference's part_execute_code_builder.
+template, as in the reference's part_execute_code_builder. Trials time the templates' kernels; the
+column-tiled layout is timed once per dense view, and the result says which of the two is faster.
 """
 from __future__ import annotations
 
@@ -111,7 +112,8 @@ def _result(res_handle):
             graph._check(L.asp_search_result_sub_launch(res_handle, i, C.byref(th), C.byref(rd)))
             subs.append({"graph": L.asp_search_result_sub_name(res_handle, i).decode(), "nodes": body[:-1], "template": body[-1].split()[1],
                          "threads": int(th.value), "row_reduce": int(rd.value)})
-        desc = {"dense": L.asp_search_result_dense(res_handle).decode().replace("\n", " | "), "subs": subs}
+        layout = {v: k for k, v in capi.LAYOUT.items()}[L.asp_search_result_layout(res_handle)]
+        desc = {"dense": L.asp_search_result_dense(res_handle).decode().replace("\n", " | "), "subs": subs, "layout": layout}
         trials = []
         for i in range(L.asp_search_result_num_trials(res_handle)):
             dense, sub, name, th, rd, ms, rate = [f.strip() for f in L.asp_search_result_trial(res_handle, i).decode().split(";")]
@@ -165,15 +167,16 @@ def search_with_timer(m: CsrMatrix, time_fn, quick: bool = True, warmup: int = 2
     return out
 
 
-def build(ctx: capi.Context, m: CsrMatrix, desc: dict, layout: str = "auto"):
-    """Lower and upload exactly the graph a previous search() described (no timing). layout: as PlanGroup takes it."""
+def build(ctx: capi.Context, m: CsrMatrix, desc: dict, layout: str | None = None):
+    """Lower and upload exactly the graph a previous search() described (no timing). layout: as PlanGroup takes it; by default
+    what the search found ("auto" for a description without it)."""
     hm = Matrix.view_csr(m)
     cm = hm.dense(desc["dense"].replace(" | ", "\n"))
     if cm.n_subs != len(desc["subs"]):
         raise ValueError(f"graph describes {len(desc['subs'])} sub-matrices, the dense view gives {cm.n_subs}")
     spec = "\n".join(Candidate(s["graph"], s["nodes"], s["template"], []).lines(i) for i, s in enumerate(desc["subs"]))
     fmt = cm.execute(spec)
-    group = fmt.upload(ctx, layout)
+    group = fmt.upload(ctx, layout or desc.get("layout", "auto"))
     for i, s in enumerate(desc["subs"]):
         set_launch(fmt, group, i, s["threads"], s["row_reduce"])
     cm.close()

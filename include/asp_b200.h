@@ -217,7 +217,8 @@ asp_status asp_plan_set_launch(asp_plan *plan, int64_t tblock_num, int64_t threa
  * that sweeps thread_num_in_block reads back here which points of its sweep coincide. The reference has
  * no such query: its launch is the literal it printed into the program (code_of_kernal_function_call,
  * e.g. direct_atom_op_warp_block_compress.cc:1012-1040). The block-value template reports one thread per pair of block
- * rows; how its kernel shares them out among CTAs follows from the matrix. Any pointer may be NULL. */
+ * rows; how its kernel shares them out among CTAs follows from the matrix. Both calls speak of the template's kernel: a group that runs
+ * the column-tiled layout takes no launch parameters. Any pointer may be NULL. */
 asp_status asp_plan_get_launch(const asp_plan *plan, int64_t *tblock_num, int64_t *thread_num_in_block, int64_t *thread_num_of_row_reduce);
 /* Work decomposition knobs, for launch-space experiments (the defaults are what the measurements in this
  * repository use): `vec` = TLBs per thread (1, 2, 4, 8 for ELL-like; 1, 2, 4 for SELL-like; 0 keeps the
