@@ -1107,7 +1107,9 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         for (int k = 0; k < 6; k++) off[k + 1] = align_up(off[k] + bytes[k], 256);
         const uint64_t sum_stride = align_up(th.n_parts, 32);
         const size_t sum_bytes = (size_t)th.copies * sum_stride * sizeof(double);
-        if (tg->arena.make(ctx->device, off[6] + sum_bytes) != cudaSuccess)
+        // The layout makes calls faster, no more: the caller's x and y, and a margin for whatever else the program does, come first.
+        const size_t vectors = (descs[0].n_rows + descs[0].n_cols) * (descs[0].val_dtype == ASP_F64 ? 8 : 4), margin = 256u << 20;
+        if (!asp::device_has_room(ctx->device, off[6] + sum_bytes + vectors + margin) || tg->arena.make(ctx->device, off[6] + sum_bytes) != cudaSuccess)
         {
             cudaGetLastError(); // no room on the device: as above
             tg.reset();

@@ -34,6 +34,7 @@ class IdleBlocks
     uint64_t clock = 0;
 
   public:
+    size_t total() const { return bytes; }
     // the smallest block of want to 1.25 want + unit bytes, or NULL
     void *take(size_t want, size_t unit, size_t *size)
     {

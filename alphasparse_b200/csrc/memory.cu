@@ -134,6 +134,22 @@ cudaError_t device_malloc(int device, size_t bytes, void **out)
     return e;
 }
 
+bool device_has_room(int device, size_t bytes)
+{
+    OnDevice on(device);
+    size_t idle, free_now = 0, all = 0;
+    {
+        std::lock_guard<std::mutex> g(pool(device).lock);
+        idle = pool(device).idle.total();
+    }
+    if (cudaMemGetInfo(&free_now, &all) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return false;
+    }
+    return free_now + idle >= bytes;
+}
+
 void device_trim(int device)
 {
     OnDevice on(device);

@@ -19,6 +19,7 @@ cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got);
 void device_free(int device, void *p, size_t got) noexcept;
 // cudaMalloc, a second time without idle blocks if the first fails: for whatever does not come from the pool
 cudaError_t device_malloc(int device, size_t bytes, void **out);
+bool device_has_room(int device, size_t bytes); // free or kept idle by the pool
 void device_trim(int device);
 void device_pool_retain(int device);  // a context was created ...
 void device_pool_release(int device); // ... or destroyed

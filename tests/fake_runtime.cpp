@@ -97,6 +97,7 @@ cudaError_t cudaFree(void *p)
     free(p);
     return cudaSuccess;
 }
+cudaError_t cudaMemGetInfo(size_t *f, size_t *all) { return *all = fake::limit, *f = fake::limit - fake::in_use, cudaSuccess; }
 cudaError_t cudaDeviceSynchronize()
 {
     LOCKED;
@@ -241,7 +242,9 @@ int main(int, char **argv)
         for (int i = 0; i < 3; i++) need(asp::device_alloc(0, (30u << 20) + i * (2u << 20), &p[i], &got[i]) == cudaSuccess, "device_alloc");
         for (int i = 0; i < 3; i++) asp::device_free(0, p[i], got[i]);
         need(fake::in_use > (90u << 20), "the pool keeps nothing");
+        need(asp::device_has_room(0, 100u << 20) && !asp::device_has_room(0, 101u << 20), "idle blocks count as room");
         need(asp::device_malloc(0, 60u << 20, &q) == cudaSuccess, "an allocation beside the pool");
+        need(asp::device_has_room(0, 40u << 20) && !asp::device_has_room(0, 41u << 20), "what is in use is none");
         cudaFree(q);
         for (int i = 0; i < 3; i++) need(asp::device_alloc(0, 30u << 20, &p[i], &got[i]) == cudaSuccess, "device_alloc");
         for (int i = 0; i < 3; i++) asp::device_free(0, p[i], got[i]);

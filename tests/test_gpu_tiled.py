@@ -189,3 +189,29 @@ def test_an_unknown_layout_is_refused(asp_ctx):
     with pytest.raises(capi.AspError):
         capi.check(capi.lib().asp_plan_group_create_with(asp_ctx.handle, (capi.PlanDesc * len(descs))(*descs), len(descs), 7, plans))
     fmt.close()
+
+
+def test_the_layout_leaves_room_for_the_caller(asp_ctx):
+    """On a device that is nearly full the group runs its templates' kernels."""
+    import torch
+
+    m, x = matrix(np.float32, 3 * TILE[np.float32], seed=3)
+    y_ref, scale = refdump.csr_ref(m, x)
+    desc = {"dense": "dense compress", "subs": [{"graph": "K9", "nodes": NODES["K9"], "template": "K9", "threads": 128, "row_reduce": 1}]}
+    capi.device_trim(0)
+    torch.cuda.empty_cache()
+    full = torch.empty(torch.cuda.mem_get_info()[0] - (300 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        fmt, g = tuner.build(asp_ctx, m, desc)
+        assert g.layout_bytes() == 0
+        refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, "nearly full")
+        g.close()
+        fmt.close()
+    finally:
+        del full
+        torch.cuda.empty_cache()
+    fmt, g = tuner.build(asp_ctx, m, desc)
+    assert g.layout_bytes() > 0
+    assert 0.7 * g.format_bytes() < g.layout_bytes() < 1.3 * g.format_bytes()
+    g.close()
+    fmt.close()
