@@ -215,3 +215,37 @@ def test_the_layout_leaves_room_for_the_caller(asp_ctx):
     assert 0.7 * g.format_bytes() < g.layout_bytes() < 1.3 * g.format_bytes()
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("short,long,laid_out", [(2_000, 20, False), (5_000, 60, True)])
+def test_small_groups_of_several_strips_keep_their_kernels(asp_ctx, short, long, laid_out):
+    """Below 65,536 non-zeros every strip has the bits that it has with the others left out."""
+    from alphasparse_b200.graph import Matrix
+
+    rng = np.random.default_rng(short)
+    m, x = M.from_row_lengths(np.concatenate([rng.integers(10, 30, size=short), rng.integers(500, 700, size=long)]), 50_000, seed=short)
+    hm = Matrix.from_csr(m)
+    cm = hm.dense("dense sort 1\ndense rowdiv_exp 128 4096 8\ndense compress")
+    assert cm.n_subs > 1 and (m.nnz >= 65_536) == laid_out
+    strip = lambda i, t: [f"sub {i} {n}" for n in NODES[t]] + [f"sub {i} template {t}"]
+    templates = ["K2" if cm.sub_rows(i)[3] <= 128 else "K6" for i in range(cm.n_subs)]
+    fmt = cm.execute("\n".join(l for i, t in enumerate(templates) for l in strip(i, t)))
+    g = fmt.upload(asp_ctx)
+    assert (g.layout_bytes() > 0) == laid_out
+    y_ref, scale = refdump.csr_ref(m, x)
+    y = g.spmv_host(x)
+    refdump.assert_y(y, y_ref, scale, np.float32, "strips")
+    if not laid_out:
+        for i, t in enumerate(templates):
+            part = cm.execute("\n".join(strip(i, t) + [f"sub {j} template EMPTY" for j in range(cm.n_subs) if j != i]))
+            gp = part.upload(asp_ctx)
+            assert gp.layout_bytes() == 0
+            info = fmt.sub_info(i)
+            rows = fmt.global_perm()[info.min_row : info.max_row + 1].astype(np.int64)
+            assert np.array_equal(gp.spmv_host(x)[rows], y[rows])
+            gp.close()
+            part.close()
+    g.close()
+    fmt.close()
+    cm.close()
+    hm.close()
