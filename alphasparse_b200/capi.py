@@ -358,7 +358,8 @@ class PlanGroup:
         return lib().asp_plan_layout_bytes(self._plans[0])
 
     def launches(self) -> int:
-        return sum(lib().asp_plan_launches(self._plans[i]) for i in range(self.n))
+        """Kernels that one asp_spmv over the group launches, without those that clear y or store the sums of rows."""
+        return 1 if self.layout_bytes() else sum(lib().asp_plan_launches(self._plans[i]) for i in range(self.n))
 
     def spmv(self, d_x: int, d_y: int, zero_y=True):
         """Asynchronous y (+)= A x on device pointers (ints). zero_y: False / True / "auto"

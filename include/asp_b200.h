@@ -236,7 +236,8 @@ uint64_t asp_plan_format_bytes(const asp_plan *plan);
 /* bytes of device memory of the column-tiled layout that the plan's group runs (see asp_plan_group_create), beside the format
  * arrays; 0 when the group runs its templates' own kernels */
 uint64_t asp_plan_layout_bytes(const asp_plan *plan);
-/* number of kernel launches one asp_spmv over this plan issues (excluding the y clear) */
+/* number of launches of its template's kernel that one asp_spmv over this plan issues (excluding the y clear); the plans of a group
+ * that runs the column-tiled layout share one launch */
 int asp_plan_launches(const asp_plan *plan);
 
 /* replaces the spmv_<k><<<...>>> calls of the generated main() (code_builder.cc:1534-1550):

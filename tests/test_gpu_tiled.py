@@ -69,6 +69,7 @@ def test_tiled_group_of_sorted_strips_and_empty_rows(asp_ctx):
     for layout in ("auto", "none"):
         fmt, g = tuner.build(asp_ctx, m, desc, layout)
         assert (g.layout_bytes() > 0) == (layout == "auto")
+        assert g.launches() == (1 if layout == "auto" else len(desc["subs"]))
         refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, f"strips {layout}")
         g.close()
         fmt.close()
