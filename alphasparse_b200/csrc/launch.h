@@ -4,9 +4,14 @@
 // the next one. A kernel launched by launch_pdl() may start while the one before it drains. Until grid_wait() has returned
 // (everything earlier on the stream has then finished and its writes are visible) it touches only what no kernel writes: the
 // plan's arrays. What other kernels write (x) is read after the wait, by ordinary loads in program order: `ld.global.nc` would
-// promise that nobody writes x while the kernel exists. Every thread that stores anything waits first, and some thread always
-// does, so that kernels finish in stream order. grid_release() comes after the wait: the next kernel then starts when this one's
-// last CTA has, and never more than one kernel is waiting.
+// promise that nobody writes x while the kernel exists. What the code relies on: every thread that stores anything waits first, and in
+// every CTA some thread does, so that a kernel finishes only after everything before it on the stream has; waiting for the one
+// kernel before is then waiting for all.
+//
+// grid_release() lets the next kernel start when all CTAs of this one have called it (or ended). Most kernels call it after their
+// wait, so that one kernel at most is waiting behind the running one. k_clear, k_tiled and k_rows call it before: k_tiled loads the
+// head of its stream meanwhile. Several kernels may then be waiting, which costs their place on the SMs and nothing else: they
+// still store nothing before everything earlier has finished, and a kernel's CTAs are all on the device before the next one's are.
 #ifndef ASP_LAUNCH_H
 #define ASP_LAUNCH_H
 
