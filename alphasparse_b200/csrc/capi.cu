@@ -83,10 +83,10 @@ struct Arena
     void *base = nullptr;
     size_t got = 0;
     int device = 0;
-    cudaError_t make(int dev, size_t bytes)
+    cudaError_t make(int dev, size_t bytes, size_t spare = 0)
     {
         device = dev;
-        const cudaError_t e = asp::device_alloc(dev, bytes, &base, &got);
+        const cudaError_t e = asp::device_alloc(dev, bytes, &base, &got, spare);
         if (e != cudaSuccess) base = nullptr;
         return e;
     }
@@ -1109,7 +1109,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         const size_t sum_bytes = (size_t)th.copies * sum_stride * sizeof(double);
         // The layout makes calls faster, no more: the caller's x and y, and a margin for whatever else the program does, come first.
         const size_t vectors = (descs[0].n_rows + descs[0].n_cols) * (descs[0].val_dtype == ASP_F64 ? 8 : 4), margin = 256u << 20;
-        if (!asp::device_has_room(ctx->device, off[6] + sum_bytes + vectors + margin) || tg->arena.make(ctx->device, off[6] + sum_bytes) != cudaSuccess)
+        if (tg->arena.make(ctx->device, off[6] + sum_bytes, vectors + margin) != cudaSuccess)
         {
             cudaGetLastError(); // no room on the device: as above
             tg.reset();

@@ -808,8 +808,9 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     else
     {
         // (allocated before the region: an exception that leaves one ends the process)
-        std::vector<u64> first(stride * (u64)omp_get_max_threads());
-#pragma omp parallel for schedule(static) reduction(max : max_thread_first_row) reduction(|| : share_thread) if (b.col.size() > kParallelNnz)
+        const bool share = b.col.size() > kParallelNnz;
+        std::vector<u64> first(stride * (share ? (u64)omp_get_max_threads() : 1));
+#pragma omp parallel for schedule(static) reduction(max : max_thread_first_row) reduction(|| : share_thread) if (share)
         for (u64 w = 0; w < NW; w++) fill_wlb(w, first.data() + stride * (u64)omp_get_thread_num(), max_thread_first_row, share_thread);
     }
     u64 max_w_coo_begin = 0, max_w_size = 0;

@@ -13,6 +13,9 @@
 
 #include "../tiled.h"
 
+// per element, in every template's loop of walk(): as calls (what the compiler makes of the seventh use) a third slower
+#define ASP_INLINE __attribute__((always_inline))
+
 namespace asp
 {
 namespace
@@ -81,7 +84,7 @@ void walk(const TiledSource &s, u64 u0, u64 u1, F &&f)
     const u64 c0 = a.first_col, radd = a.row_add ? a.first_row : 0;
     const HostMeta *m = s.m;
     u64 last_row = ~0ull, last_col = ~0ull;
-    auto put = [&](u64 row, u64 at) {
+    auto put = [&](u64 row, u64 at) ASP_INLINE {
         const u64 c = (u64)col[at] + c0;
         const VT v = val[at];
         if (v == VT(0) && row == last_row && c == last_col) return;
@@ -302,12 +305,16 @@ struct Builder
                 std::fill(n, n + C, 0);
                 u64 row = ~0ull, tile = ~0ull, run = 0;
                 u32 of_row = 0; // pieces since the row changed
+                // rows that are one thread's in the template's kernel have no more parts than it adds elements
+                const TiledSource &from = src[chunks[c].sub];
+                const bool alone = !from.a->atomic && (from.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || from.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS);
                 auto row_ends = [&]() {
                     // (several threads may have elements of a row)
-                    if (of_row) __atomic_fetch_add(&row_code[row], std::min(of_row, 1u << 16) * share[chunks[c].sub], __ATOMIC_RELAXED);
+                    if (of_row && alone) __atomic_store_n(&row_code[row], 1, __ATOMIC_RELAXED);
+                    else if (of_row) __atomic_fetch_add(&row_code[row], std::min(of_row, 1u << 16) * share[chunks[c].sub], __ATOMIC_RELAXED);
                     of_row = 0;
                 };
-                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT) {
+                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT) ASP_INLINE {
                     const u64 t = (u32)col / TW;
                     n[t]++;
                     if (r != row || t != tile || run == kMaxPiece)
@@ -367,12 +374,7 @@ struct Builder
     }
     void number_rows(TiledHost &out)
     {
-        if (!out.direct)
-        {
-#pragma omp parallel for schedule(static)
-            for (long long r = 0; r < (long long)n_rows; r++) row_code[r] = kTiledInParts | (u32)r;
-            return;
-        }
+        if (out.parts.empty()) return; // all rows are alike
         u32 k = 0;
         for (u64 r = 0; r < n_rows; r++)
         {
@@ -395,7 +397,7 @@ struct Builder
             for (long long c = 0; c < (long long)chunks.size(); c++)
             {
                 std::copy(at.begin() + (size_t)c * C, at.begin() + (size_t)(c + 1) * C, to);
-                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) {
+                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) ASP_INLINE {
                     const u64 t = (u32)col / TW, q = to[t]++;
                     e_row.p[q] = (u32)r;
                     e_col.p[q] = (uint16_t)(col - t * TW);
@@ -467,10 +469,9 @@ struct Builder
         std::vector<u64> n_step(B), n_slice(B);
         u64 longest = 0;
         for (const Block &b : blocks) longest = std::max(longest, b.e1 - b.e0);
-        HostBuf<Piece> scratch;
-        scratch.make(2 * longest * (u64)threads());
+        std::unique_ptr<Piece[]> scratch(new Piece[2 * longest * (u64)threads()]);
         auto scratch_of_thread = [&]() {
-            Piece *const mine = scratch.p + 2 * longest * (u64)this_thread();
+            Piece *const mine = scratch.get() + 2 * longest * (u64)this_thread();
             return Pieces{mine, mine + longest};
         };
 #pragma omp parallel
@@ -500,6 +501,9 @@ struct Builder
         out.row.make(sl * kTiledSlice);
         out.end.make(sl);
         VT *val = (VT *)out.val.p;
+        // what stands for a row among the slices' rows
+        const bool some = !out.parts.empty();
+        const u32 all = out.n_parts > 0 && !out.direct ? kTiledInParts : 0;
 #pragma omp parallel
         {
             Pieces p = scratch_of_thread();
@@ -523,7 +527,7 @@ struct Builder
                         rows[o] = kTiledNoRow;
                         if (i + j >= p.size()) continue;
                         const u64 e = blocks[b].e0 + p[i + j].start;
-                        rows[o] = row_code[e_row.p[e]];
+                        rows[o] = some ? row_code[e_row.p[e]] : e_row.p[e] | all;
                         for (u32 k = 0; k < p[i + j].len; k++)
                         {
                             v[k * kTiledSlice + o] = e_val.p[e + k];

@@ -15,7 +15,8 @@ namespace asp
 // all per device (the longest idle ones go first), given back when the last context of the device is destroyed, by device_trim(), or when
 // an allocation of this library fails. Safe from several threads.
 // device_free() waits for the device first, as cudaFree does: kernels in flight may still read the block.
-cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got);
+// `spare`: fails where an allocation would leave less than that (0: does not look).
+cudaError_t device_alloc(int device, size_t bytes, void **out, size_t *got, size_t spare = 0);
 void device_free(int device, void *p, size_t got) noexcept;
 // cudaMalloc, a second time without idle blocks if the first fails: for whatever does not come from the pool
 cudaError_t device_malloc(int device, size_t bytes, void **out);

@@ -174,7 +174,7 @@ void *asp_ctx_stream(asp_ctx *ctx);
  * inside the array it indexes (ASP_ERR_BOUNDS otherwise; one parallel pass over each index array).
  * Where the columns are so scattered that the gathers of x, not the bytes, bound the templates' kernels, the whole group
  * is also laid out by column tiles (csrc/kernels_tiled.cu), which takes 0.8 to 1.3 times the format's device memory beside it
- * (asp_plan_layout_bytes; left out where less than x, y and 256 MB would stay free), and asp_spmv
+ * (asp_plan_layout_bytes; left out where new memory for it would leave less than x, y and 256 MB free), and asp_spmv
  * over the complete group runs that layout; a group with EMPTY plans never does, nor do several plans of fewer than 65,536
  * non-zeros in all (their rows have the same bits whichever other plans are EMPTY). Sums are then taken in another order from
  * call to call, as with every template that accumulates with atomics (asp_plan_group_create_with can forbid it). Rows that are added up in many parts have 64-bit sums in

@@ -244,6 +244,13 @@ int main(int, char **argv)
         need(fake::in_use > (90u << 20), "the pool keeps nothing");
         need(asp::device_has_room(0, 100u << 20) && !asp::device_has_room(0, 101u << 20), "idle blocks count as room");
         need(asp::device_malloc(0, 60u << 20, &q) == cudaSuccess, "an allocation beside the pool");
+        size_t size = 0;
+        void *r = nullptr;
+        need(asp::device_alloc(0, 30u << 20, &r, &size, 11u << 20) == cudaErrorMemoryAllocation, "an allocation that leaves too little");
+        need(asp::device_alloc(0, 30u << 20, &r, &size, 10u << 20) == cudaSuccess, "one that leaves enough");
+        asp::device_free(0, r, size);
+        need(asp::device_alloc(0, 30u << 20, &r, &size, 11u << 20) == cudaSuccess, "one from the pool");
+        asp::device_free(0, r, size);
         need(asp::device_has_room(0, 40u << 20) && !asp::device_has_room(0, 41u << 20), "what is in use is none");
         cudaFree(q);
         for (int i = 0; i < 3; i++) need(asp::device_alloc(0, 30u << 20, &p[i], &got[i]) == cudaSuccess, "device_alloc");
