@@ -268,6 +268,7 @@ struct Builder
     const u64 n_rows, n_cols;
     static constexpr u32 TW = tiled_tile_cols(sizeof(VT) == 8);
     const u64 C; // tiles of x
+    const u64 warp_steps; // of a warp's share, about: longer pieces are cut, and every cut is one more part of their rows
     std::vector<Chunk> chunks;
     std::vector<u64> at; // [chunk * C + tile]: first its count, then where its elements go
     std::vector<u64> tile_begin, tile_pieces;
@@ -278,7 +279,10 @@ struct Builder
     HostBuf<uint16_t> e_col;
     HostBuf<VT> e_val;
 
-    Builder(const std::vector<TiledSource> &s, u64 rows, u64 cols) : src(s), n_rows(rows), n_cols(cols), C((cols + TW - 1) / TW) {}
+    Builder(const std::vector<TiledSource> &s, u64 rows, u64 cols, u64 nnz, int n_sm)
+        : src(s), n_rows(rows), n_cols(cols), C((cols + TW - 1) / TW), warp_steps(std::max<u64>(1, nnz / ((u64)n_sm * kTiledWarps * kTiledSlice)))
+    {
+    }
 
     void count()
     {
@@ -304,15 +308,15 @@ struct Builder
             {
                 std::fill(n, n + C, 0);
                 u64 row = ~0ull, tile = ~0ull, run = 0;
-                u32 of_row = 0; // pieces since the row changed
+                u32 of_row = 0, elements = 0; // pieces and elements since the row changed
                 // rows that are one thread's in the template's kernel have no more parts than it adds elements
                 const TiledSource &from = src[chunks[c].sub];
                 const bool alone = !from.a->atomic && (from.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || from.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS);
                 auto row_ends = [&]() {
                     // (several threads may have elements of a row)
                     if (of_row && alone) __atomic_store_n(&row_code[row], 1, __ATOMIC_RELAXED);
-                    else if (of_row) __atomic_fetch_add(&row_code[row], std::min(of_row, 1u << 16) * share[chunks[c].sub], __ATOMIC_RELAXED);
-                    of_row = 0;
+                    else if (of_row) __atomic_fetch_add(&row_code[row], (u32)std::min<u64>(of_row + elements / warp_steps, 1u << 16) * share[chunks[c].sub], __ATOMIC_RELAXED);
+                    of_row = elements = 0;
                 };
                 walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT) ASP_INLINE {
                     const u64 t = (u32)col / TW;
@@ -327,6 +331,7 @@ struct Builder
                         run = 0;
                     }
                     run++;
+                    elements++;
                 });
                 row_ends();
                 std::copy(n, n + C, at.begin() + (size_t)c * C);
@@ -353,21 +358,26 @@ struct Builder
     void choose_sums(TiledHost &out)
     {
         u64 missing = 0, direct = 0, shares = 0;
+        // (a long row's pieces lie side by side in a tile and are summed in the warp before they are added: two parts a tile, as a rule,
+        // twice as many where warps cut them)
+        const u64 most = (warp_steps < kMaxPiece ? 4 : 2) * C * (kDirectShares / 8);
 #pragma omp parallel for schedule(static) reduction(+ : missing, direct, shares)
         for (long long r = 0; r < (long long)n_rows; r++)
         {
             if (row_code[r] == 0) missing++;
             else if (row_code[r] <= kDirectShares) direct++;
-            else shares += row_code[r];
+            else shares += std::min<u64>(row_code[r], most);
         }
         const u64 rows = n_rows - missing - direct;
         out.covers_all_rows = missing == 0;
         // fp64: at most half of what may be added up directly goes to one sum of a row, on average
+        // (four at least where warps cut the pieces: the longest of a few long rows count for more than the average)
+        if (sizeof(VT) == 8 && rows > 0 && warp_steps < kMaxPiece) out.copies = 4;
         if (sizeof(VT) == 8)
             while (out.copies < 16 && shares > kDirectShares / 2 * (u64)out.copies * rows) out.copies *= 2;
         // where some rows have sums, the others do better with sums, too, than with one more launch that clears y, unless they are
         // many: 400,000 rows, fp32: 25 -> 21 us; R-MAT scale 21: 50 -> 56 us (a `red` of 64 bits costs more than one of 32)
-        const double sums_us = (double)(n_rows - rows) * (16.0 * out.copies + sizeof(VT)) / 2.0e6, clear_us = 4.0 + (double)n_rows * sizeof(VT) / 6.0e6;
+        const double sums_us = (double)(n_rows - rows) * ((16.0 * out.copies + sizeof(VT)) / 6.0e6 + 4e-6), clear_us = 4.0 + (double)n_rows * sizeof(VT) / 6.0e6;
         out.n_parts = rows == 0 || sums_us > clear_us ? rows : n_rows;
         out.direct = out.n_parts < n_rows;
         if (out.direct) out.parts.resize(rows);
@@ -666,7 +676,7 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     };
     if (tiled_us(true_nnz, 0, 0) > 0.85 * own_us) return false;
     if (n_rows >= kTiledInParts || requests >= 1e11) return false;
-    Builder<VT> b(src, n_rows, n_cols);
+    Builder<VT> b(src, n_rows, n_cols, true_nnz, n_sm);
     if (b.C + (u64)n_sm >= 65536) return false;
     b.count();
     b.choose_sums(out);

@@ -12,8 +12,8 @@
 //          slices too: what a warp has summed when its slice or its share ends is added to its row by `red`
 //   parts  a row that gets there in many parts would collect a rounding error with each (fp32, 80 elements over 25 tiles: 1.0e-7
 //          from the 64-bit result, the formats' own kernels 0.72e-7): the sums of such rows are 64-bit ones in memory of the
-//          group, which k_rows turns into y and leaves as zeros for the next call (0.42e-7). In fp64 the tiles take `copies`
-//          sums of a row in turn, which k_rows adds pairwise. A piece is summed with more than the value's bits, too.
+//          group, which k_rows turns into y and leaves as zeros for the next call (0.42e-7). In fp64 tiles and warps
+//          take `copies` sums of a row in turn, which k_rows adds pairwise. A piece is summed with more than the value's bits, too.
 // The stream is read two batches deep into registers. 159 KB of shared memory per tile leave the L1 enough lines for the
 // loads in flight: with 224 KB the same stream is read at 4.2 instead of 5 TB/s.
 // Measured, fp32 (against the formats' own kernels): 200,000 rows of 40..120 non-zeros, random columns among 1 M: 40 us
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
         u32 step = k.x, slice = k.z;
         const u32 end = k.y, tile = k.w & 0xffffu;
         visit = k.w >> 16;
-        double *const sum = a.sum + (size_t)(tile & (a.copies - 1)) * a.sum_stride;
+        double *const sum = a.sum + (size_t)((tile + warp) & (a.copies - 1)) * a.sum_stride;
         const P *vp = reinterpret_cast<const P *>(a.val) + (size_t)step * 32 + lane;
         const u32 *cp = reinterpret_cast<const u32 *>(a.col) + (size_t)step * 32 + lane;
         P v[U];
@@ -335,9 +335,10 @@ cudaError_t launch_sums(const TiledArgs &a, unsigned n_sm, cudaStream_t st)
 template <class VT>
 cudaError_t launch_rows(const TiledArgs &a, unsigned n_sm, cudaStream_t st)
 {
-    // a few rows per thread
-    const u64 want = (a.n_parts + 1023ull) / 1024;
-    const dim3 grid((unsigned)(want < 1 ? 1 : want < 4ull * n_sm ? want : 4ull * n_sm)), block(256);
+    // one trip per thread up to a full device: a trip waits once for its rows' sums (16 copies, 4000 rows, four trips a thread: 10 us)
+    const u32 per_cta = 256 * (a.copies < 4 ? 4 / a.copies : 1);
+    const u64 want = ((u64)a.n_parts + per_cta - 1) / per_cta;
+    const dim3 grid((unsigned)(want < 8ull * n_sm ? want : 8ull * n_sm)), block(256);
     const auto rows = [&](auto kernel) { return launch_pdl(kernel, grid, block, 0, st, a.parts, a.sum, (u64)a.sum_stride, (VT *)a.y, (u32)a.n_parts); };
     if (a.copies == 1) return rows(k_rows<VT, 1>);
     if constexpr (sizeof(VT) == 8)

@@ -61,7 +61,7 @@ struct TiledHost
     HostBuf<uint32_t> end;      // slice s covers steps [end[s - 1], end[s])
     std::vector<uint32_t> work; // {first step, end step, slice, tile | next visit << 16} per warp; visit v at v * kTiledWarps
     uint64_t nnz = 0, steps = 0, slices = 0;
-    unsigned copies = 1; // sums of a row, which its tiles take in turn: 1, 2, 4, 8 or 16
+    unsigned copies = 1; // sums of a row, which tiles and warps take in turn: 1, 2, 4, 8 or 16
     bool covers_all_rows = false; // every row of y has at least one element
     bool direct = false;          // some are added up in y itself
 };

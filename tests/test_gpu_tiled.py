@@ -86,7 +86,7 @@ def exact(m, x):
 
 @pytest.mark.parametrize("template,dtype,rows,lo,hi,cols", [
     ("K6", np.float32, 60_000, 40, 121, 1_000_000), ("K8", np.float64, 60_000, 40, 121, 1_000_000), ("K4", np.float64, 60_000, 40, 121, 100_000),
-    ("K7", np.float32, 4_000, 1000, 3001, 1_000_000), ("K7", np.float64, 4_000, 1000, 3001, 1_000_000), ("K9", np.float32, 250_000, 4, 29, 1_000_000)])
+    ("K7", np.float32, 4_000, 1000, 3001, 1_000_000), ("K7", np.float64, 4_000, 1000, 3001, 1_000_000), ("K7", np.float64, 4_000, 1000, 3001, 100_000), ("K9", np.float32, 250_000, 4, 29, 1_000_000)])
 def test_tiled_sums_are_as_near_to_the_exact_ones_as_the_templates(asp_ctx, template, dtype, rows, lo, hi, cols):
     """The layout adds a row up in other parts than the template's kernel, but with no larger error."""
     import torch
@@ -246,6 +246,41 @@ def test_small_groups_of_several_strips_keep_their_kernels(asp_ctx, short, long,
             assert np.array_equal(gp.spmv_host(x)[rows], y[rows])
             gp.close()
             part.close()
+    g.close()
+    fmt.close()
+    cm.close()
+    hm.close()
+
+
+def test_strips_with_hub_rows_are_as_near_to_the_exact_sums(asp_ctx):
+    """A small fp64 matrix: warps cut the long rows' pieces, two tiles only."""
+    import torch
+
+    rng = np.random.default_rng(9)
+    m, x = M.from_row_lengths(np.concatenate([rng.integers(1, 12, size=30_000), rng.integers(200, 700, size=200), [9_000, 7_000, 5_000, 3_000]]), 30_000, seed=9, dtype=np.float64)
+    from alphasparse_b200.graph import Matrix
+
+    hm = Matrix.from_csr(m)
+    cm = hm.dense("dense sort 1\ndense rowdiv_exp 128 4096 8\ndense compress")
+    fmt = cm.execute("\n".join(l for i in range(cm.n_subs) for t in ["K2" if cm.sub_rows(i)[3] <= 128 else "K6" if cm.sub_rows(i)[3] <= 1024 else "K7"]
+                               for l in [f"sub {i} {n}" for n in NODES[t]] + [f"sub {i} template {t}"]))
+    g = fmt.upload(asp_ctx)
+    assert g.layout_bytes() > 0
+    ref, scale = exact(m, x)
+    dx = torch.from_numpy(x).cuda()
+    far = []
+    for zero_y in (True, False):
+        dy = torch.zeros(m.n_rows, dtype=dx.dtype, device="cuda")
+        worst = 0.0
+        for _ in range(4):  # (a few hub rows carry the norm: the order of their parts shows)
+            dy.zero_()
+            torch.cuda.synchronize()
+            g.spmv(dx.data_ptr(), dy.data_ptr(), zero_y)
+            asp_ctx.synchronize()
+            d = dy.cpu().numpy().astype(ref.dtype) - ref
+            worst += float(np.sqrt((d * d).sum() / (ref * ref).sum())) / 4
+        far.append(worst)
+    assert far[0] <= 1.1 * far[1], far
     g.close()
     fmt.close()
     cm.close()
