@@ -111,3 +111,28 @@ def test_idle_memory_is_given_back(asp_ctx):
     assert torch.cuda.mem_get_info()[0] >= before + held * 0.9
     with pytest.raises(capi.AspError):
         capi.device_trim(1000)
+
+
+def test_host_calls_on_pageable_buffers(asp_ctx):
+    """asp_spmv_host on arrays of the caller's own: x and y go through the pinned ring, which starts at another place each time."""
+    from alphasparse_b200 import capi
+
+    cases = []
+    for rows in (65_535, 65_536, 65_537, 300_001, 4_500_000):  # y of 256 KB and an element around, no multiple of a piece, more than the ring
+        lengths = np.full(rows, 2)
+        m, _ = M.from_row_lengths(lengths, rows, seed=rows % 97, dtype=np.float32)
+        fmt, g = tuner.build(asp_ctx, m, desc("K3", ["row_padding 32 1", "tlb_row"]))
+        cases.append((m, fmt, g))
+    rng = np.random.default_rng(1)
+    for k in range(12):
+        m, _, g = cases[k % len(cases)]
+        x = rng.uniform(-1, 1, m.n_cols).astype(np.float32)
+        y = np.full(m.n_rows + 2, 7, dtype=np.float32)
+        y_ref, scale = refdump.csr_ref(m, x)
+        capi.check(capi.lib().asp_spmv_host(asp_ctx.handle, g._plans, g.n, x.ctypes.data, y[1:].ctypes.data))
+        x[:] = np.nan  # the caller's again
+        refdump.assert_y(y[1:-1], y_ref, scale, np.float32, f"call {k}")
+        assert y[0] == 7 and y[-1] == 7
+    for _, fmt, g in cases:
+        g.close()
+        fmt.close()
