@@ -16,8 +16,10 @@
 //          take `copies` sums of a row in turn, which k_rows adds pairwise. A piece is summed with more than the value's bits, too.
 // The stream is read two batches deep into registers. 159 KB of shared memory per tile leave the L1 enough lines for the
 // loads in flight: with 224 KB the same stream is read at 4.2 instead of 5 TB/s.
-// Measured, fp32 (against the formats' own kernels): 200,000 rows of 40..120 non-zeros, random columns among 1 M: 40 us
-// (76 us, row-grouped; 36 us with all parts added up in y); 9,001 rows of 1000..3000: 27 us (77 us, long-row; 25 us).
+// A tile is loaded by cp.async, every thread's ten pieces in flight at once. Through registers, five at a time, nothing else runs for
+// 5 us of an SpMV over R-MAT scale 21 (ten SpMVs: 504 -> 476 us; by bulk copies 482).
+// Measured, fp32 (against the formats' own kernels): 200,000 rows of 40..120 non-zeros, random columns among 1 M: 38 us
+// (76 us, row-grouped); 9,001 rows of 1000..3000: 26 us (77 us, long-row).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -88,13 +90,7 @@ struct Sum<double>
     }
 };
 
-// x may have been written by the kernel before: read through L2, in program order after the wait
-__device__ __forceinline__ uint4 ld_x16(const void *p)
-{
-    uint4 v;
-    asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-    return v;
-}
+// x may have been written by the kernel before: read through L2 (as cp.async.cg does), in program order after the wait
 __device__ __forceinline__ float ld_x1(const float *p)
 {
     float v;
@@ -195,23 +191,15 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
             u32 i = 0;
             if (((uintptr_t)xp & 15) == 0)
             {
-                const uint4 *q = reinterpret_cast<const uint4 *>(xp);
-                uint4 *s = reinterpret_cast<uint4 *>(xs);
-                const u32 n4 = n / V;
-                u32 j = threadIdx.x;
-                for (; j + 4 * 1024 < n4; j += 5 * 1024)
-                {
-                    uint4 t[5];
-#pragma unroll
-                    for (int u = 0; u < 5; u++) t[u] = ld_x16(q + j + u * 1024);
-#pragma unroll
-                    for (int u = 0; u < 5; u++) s[j + u * 1024] = t[u];
-                }
-                for (; j < n4; j += 1024) s[j] = ld_x16(q + j);
+                // straight to shared memory, all of a thread's 16-byte pieces in flight at once
+                const u32 n4 = n / V, to = (u32)__cvta_generic_to_shared(xs);
+                for (u32 j = threadIdx.x; j < n4; j += 1024)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + j * 16), "l"((const char *)xp + (size_t)j * 16) : "memory");
                 i = n4 * V;
             }
             for (i += threadIdx.x; i < n; i += 1024) xs[i] = ld_x1(xp + i);
             if (threadIdx.x == 0) xs[tile_cols] = 0;
+            asm volatile("cp.async.wait_all;" ::: "memory");
         }
         __syncthreads();
         Sum<VT> acc0, acc1;
