@@ -13,6 +13,7 @@ import numpy as np
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libasp_b200.so")
+CALL_PATH = os.path.join(_HERE, "_call.so")
 
 ASP_MAX_BRANCH = 5
 U8, U16, U32, U64, F32, F64 = range(6)
@@ -172,6 +173,15 @@ def lib() -> C.CDLL:
     return L
 
 
+def _native():
+    """The binding of asp_spmv that does without ctypes (csrc/python/call.c), built beside the library."""
+    if not os.path.exists(CALL_PATH):
+        raise FileNotFoundError(f"{CALL_PATH} is missing: build it first (__graft_entry__.build())")
+    from . import _call
+
+    return _call
+
+
 def check(status: int) -> None:
     if status != 0:
         L = lib()
@@ -277,7 +287,7 @@ class Context:
         if self._h:
             _results.trim()
             lib().asp_ctx_destroy(self._h)
-            self._h = C.c_void_p()
+            self._h.value = None  # (in place: plan groups hold its address)
 
     def __del__(self):
         try:
@@ -332,7 +342,8 @@ class PlanGroup:
         self._keep = keepalive
         check(lib().asp_plan_group_create_with(ctx.handle, self._descs, n, LAYOUT[layout], self._plans))
         self.n = n
-        self._spmv = lib().asp_spmv
+        self._handle = ctx.handle  # kept alive: its address and that of the plans are in _call
+        self._call = _native().Spmv(C.cast(lib().asp_spmv, C.c_void_p).value, C.addressof(self._handle), C.addressof(self._plans), n)
         self.val_dtype = np.float64 if descs[0].val_dtype == F64 else np.float32
         self.n_rows = int(descs[0].n_rows)
         self.n_cols = int(descs[0].n_cols)
@@ -364,7 +375,11 @@ class PlanGroup:
     def spmv(self, d_x: int, d_y: int, zero_y=True):
         """Asynchronous y (+)= A x on device pointers (ints). zero_y: False / True / "auto"
         (clear y only when a plan accumulates with atomics)."""
-        status = self._spmv(self.ctx._h, self._plans, self.n, d_x, d_y, 2 if zero_y == "auto" else (1 if zero_y else 0))
+        z = 2 if zero_y == "auto" else (1 if zero_y else 0)
+        try:
+            status = self._call(d_x, d_y, z)
+        except TypeError:  # whatever else ctypes takes for a pointer
+            status = lib().asp_spmv(self.ctx.handle, self._plans, self.n, d_x, d_y, z)
         if status:
             check(status)
 

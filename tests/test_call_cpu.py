@@ -1,0 +1,41 @@
+"""CPU suite: the binding of asp_spmv without ctypes (csrc/python/call.c) refuses and accepts what the ctypes one did."""
+import ctypes as C
+
+import pytest
+
+from alphasparse_b200 import capi
+
+
+def bound():
+    handle, plans = C.c_void_p(), (C.c_void_p * 1)()
+    call = capi._native().Spmv(C.cast(capi.lib().asp_spmv, C.c_void_p).value, C.addressof(handle), C.addressof(plans), 1)
+    return call, handle, plans
+
+
+@pytest.mark.parametrize("args", [(None, 1, 2), (1, None, 2), (1.0, 2, 2), (1, 2), (1, 2, 2, 2), (1, 2, "auto")])
+def test_only_ints_are_taken(args):
+    call, *keep = bound()
+    with pytest.raises(TypeError):
+        call(*args)
+    with pytest.raises(TypeError):
+        call(1, 2, zero_y=2)
+
+
+@pytest.mark.parametrize("x,y", [(0, 0), (1, 0), (0, 1), (2**64 - 16, 2**63), (-16, 1 << 70)])
+def test_handles_are_read_at_the_call(x, y):
+    """A context that is closed is NULL to the library, whatever the pointers are (taken modulo 2^64, as ctypes takes them)."""
+    call, handle, plans = bound()
+    assert call(x, y, 2) == 1 and b"NULL" in capi.lib().asp_last_error()
+
+
+def test_a_call_without_plan_or_with_other_pointers_falls_back():
+    group = object.__new__(capi.PlanGroup)
+    group.n, group._plans = 1, (C.c_void_p * 1)()
+    group.ctx = object.__new__(capi.Context)
+    group.ctx._h = C.c_void_p()
+    group._call = capi._native().Spmv(C.cast(capi.lib().asp_spmv, C.c_void_p).value, C.addressof(group.ctx._h), C.addressof(group._plans), 1)
+    for x in (16, None, C.c_void_p(16)):
+        with pytest.raises(capi.AspError):
+            group.spmv(x, 16)
+    with pytest.raises(C.ArgumentError):
+        group.spmv(1.5, 16)
