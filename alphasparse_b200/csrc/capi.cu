@@ -1101,15 +1101,16 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
     }
     if (tg)
     {
-        const void *from[6] = {th.val.p, th.col.p, th.row.p, th.end.p, th.work.data(), th.parts.data()};
-        const size_t bytes[6] = {th.val.bytes(), th.col.bytes(), th.row.bytes(), th.end.bytes(), th.work.size() * sizeof(uint32_t), th.parts.size() * sizeof(uint32_t)};
-        size_t off[7] = {0};
-        for (int k = 0; k < 6; k++) off[k + 1] = align_up(off[k] + bytes[k], 256);
+        const int K = 8;
+        const void *from[K] = {th.val.p, th.col.p, th.row.p, th.end.p, th.work.data(), th.parts.data(), th.word.p, th.seg.p};
+        const size_t bytes[K] = {th.val.bytes(), th.col.bytes(), th.row.bytes(), th.end.bytes(), th.work.size() * sizeof(uint32_t), th.parts.size() * sizeof(uint32_t), th.word.bytes(), th.seg.bytes()};
+        size_t off[K + 1] = {0};
+        for (int k = 0; k < K; k++) off[k + 1] = align_up(off[k] + bytes[k], 256);
         const uint64_t sum_stride = align_up(th.n_parts, 32);
         const size_t sum_bytes = (size_t)th.copies * sum_stride * sizeof(double);
         // The layout makes calls faster, no more: the caller's x and y, and a margin for whatever else the program does, come first.
         const size_t vectors = (descs[0].n_rows + descs[0].n_cols) * (descs[0].val_dtype == ASP_F64 ? 8 : 4), margin = 256u << 20;
-        if (tg->arena.make(ctx->device, off[6] + sum_bytes, vectors + margin) != cudaSuccess)
+        if (tg->arena.make(ctx->device, off[K] + sum_bytes, vectors + margin) != cudaSuccess)
         {
             cudaGetLastError(); // no room on the device: as above
             tg.reset();
@@ -1118,21 +1119,36 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         {
             unsigned char *base = (unsigned char *)tg->arena.base;
             std::vector<asp::Stager::Segment> seg;
-            for (int k = 0; k < 6; k++)
+            for (int k = 0; k < K; k++)
                 if (bytes[k]) seg.push_back({off[k], from[k], bytes[k]});
             cudaError_t ce = asp::tiled_setup(descs[0].val_dtype == ASP_F64);
             if (ce == cudaSuccess) ce = ctx->stager.to_device(base, seg, ctx->stream);
-            if (ce == cudaSuccess && sum_bytes) ce = cudaMemsetAsync(base + off[6], 0, sum_bytes, ctx->stream);
+            if (ce == cudaSuccess && sum_bytes) ce = cudaMemsetAsync(base + off[K], 0, sum_bytes, ctx->stream);
             if (ce != cudaSuccess)
             {
                 cleanup();
                 return cuda_fail(ce, "upload of the column-tiled layout");
             }
-            tg->layout_bytes = off[6] + sum_bytes;
+            tg->layout_bytes = off[K] + sum_bytes;
             tg->owner = ctx->serial;
-            tg->args = {base + off[0], (const uint16_t *)(base + off[1]), (const uint32_t *)(base + off[2]), (const uint32_t *)(base + off[3]),
-                        (const uint4 *)(base + off[4]), th.parts.empty() ? nullptr : (const uint32_t *)(base + off[5]), (double *)(base + off[6]), (unsigned)th.n_parts, th.copies, sum_stride,
-                        th.direct, nullptr, nullptr, descs[0].n_rows, descs[0].n_cols};
+            asp::TiledArgs &a = tg->args;
+            a.val = base + off[0];
+            a.col = (const uint16_t *)(base + off[1]);
+            a.row = (const uint32_t *)(base + off[2]);
+            a.end = (const uint32_t *)(base + off[3]);
+            a.work = (const uint4 *)(base + off[4]);
+            a.parts = th.parts.empty() ? nullptr : (const uint32_t *)(base + off[5]);
+            a.word = th.units ? (const uint32_t *)(base + off[6]) : nullptr;
+            a.seg = (const uint32_t *)(base + off[7]);
+            a.sum = (double *)(base + off[K]);
+            a.n_parts = (unsigned)th.n_parts;
+            a.copies = th.copies;
+            a.sum_stride = sum_stride;
+            a.direct = th.direct;
+            a.x = nullptr;
+            a.y = nullptr;
+            a.n_rows = descs[0].n_rows;
+            a.n_cols = descs[0].n_cols;
             tg->n_plans = n;
             tg->n_sm = (unsigned)ctx->sm_count;
             tg->covers_all_rows = th.covers_all_rows;

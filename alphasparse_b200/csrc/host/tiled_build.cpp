@@ -1,7 +1,7 @@
 // Builds the column-tiled layout of a plan group (kernels_tiled.cu) from its template arrays, and decides whether the
 // group is better off with it. One pass over the stored elements counts them per tile of x, one scatters them to
-// their tiles (order of the rows kept), then every tile is cut into blocks of whole rows that are turned into slices
-// independently of one another.
+// their tiles (order of the rows kept). Then every tile is cut into blocks of whole rows that are turned into slices independently
+// of one another, or, where rows have few elements in a tile, its elements stay in order and are units of a warp each.
 #include <string.h>
 
 #include <algorithm>
@@ -251,9 +251,87 @@ u32 share_of_part(const TiledSource &s) { return (u32)std::max<u64>(1, (kDirectS
 
 const u32 kMaxPiece = 32;    // elements of a row's piece: bounds the serial chain of a lane and the padding of a slice
 const u32 kWindow = 1024;    // pieces that are sorted by length together: lanes of a slice stay near in y
+// Units or slices. A slice's `red` of a warp goes to the rows of 32 pieces of one length, anywhere among 1024 pieces; a unit's goes to
+// neighbouring rows, but a unit takes more instructions an element. fp32, random columns, 80 a row, slices / units: 25 tiles 38.2 / 31.2 us
+// (200,000 rows), 20 tiles 13.3 / 9.7 (40,000 rows), 13 tiles 9.1 / 6.6 (20,000), 8 tiles 21.3 / 21.0 (150,000), 3 tiles 18.7 / 20.4; fp64,
+// 19 tiles 33.4 / 30.8. Long runs: 9,001 rows of 2000 in 25 tiles 25.0 / 28.8, R-MAT scale 21 (8.5 a run) 476 / 643. Rows far apart (strips
+// sorted by length) 19.7 / 24.3.
+const u64 kRunForUnits = 7;  // at most so many elements a run, on average
+const u64 kNearRows = 4;     // and three quarters of the runs at most so many rows behind the run before
+const double kRowCost = 1.0; // of a row of a unit, in elements: its entry and its `red`
 const double kSliceCost = 4.0; // in steps; with 2 the CTAs of sparse tiles ran twice as long as the others
 // elements of a block of whole rows, the unit of the parallel build: enough blocks for all cores, and whole windows in each
 u64 block_size(u64 n) { return std::min<u64>(1u << 16, std::max<u64>(1u << 13, n / 128)); }
+
+// Shares out what lies in order, tile by tile (begin[t], ..., begin[C]), among the CTAs and their warps: with cost(i) before place i
+// and tile_cost for every tile that a CTA loads, so that the largest cost of a CTA is the least that will do (filling the CTAs up to the average,
+// one of them had up to twice the others' work: 20,000 rows of 40..120 among 490 K columns 9.8 -> 9.1 us, 9,001 rows of 1000..3000
+// 26.3 -> 25.0). at(cost, lo, hi): the place in [lo, hi] that a cost is reached at. A CTA's visits of tiles are `warps` entries of four words
+// each, its first one at its own number: put(entry, from, to, tile), link(entry, next visit).
+template <class Cost, class At, class Put, class Link>
+void share_out(int n_sm, u32 warps, const std::vector<u64> &begin, double tile_cost, const Cost &cost, const At &at, std::vector<u32> &work, const Put &put, const Link &link)
+{
+    const u64 C = begin.size() - 1, n = begin[C];
+    struct Visit
+    {
+        u64 cta, s, e, tile;
+    };
+    std::vector<Visit> visits;
+    // every CTA takes what it can do at a cost of `most`: true, if that is everything
+    auto fill = [&](double most) {
+        visits.clear();
+        u64 s = 0, t = 0;
+        for (int cta = 0; cta < n_sm && s < n; cta++)
+        {
+            double left = most;
+            for (bool first = true; s < n && (first || left > tile_cost + warps); first = false)
+            {
+                while (begin[t + 1] <= s) t++;
+                left -= tile_cost;
+                const u64 last = begin[t + 1];
+                const double from = cost(s);
+                const u64 e = cost(last) - from <= left ? last : std::min(last, std::max(s + 1, at(from + left, s, last)));
+                visits.push_back({(u64)cta, s, e, t});
+                left -= cost(e) - from;
+                s = e;
+                if (e < last) break;
+            }
+        }
+        return s == n;
+    };
+    double lo = cost(n) / n_sm, hi = cost(n) + tile_cost * (double)C;
+    while (!fill(hi)) hi *= 2;
+    for (int i = 0; i < 40 && hi - lo > 1; i++)
+    {
+        const double mid = (lo + hi) / 2;
+        (fill(mid) ? hi : lo) = mid;
+    }
+    fill(hi);
+    work.assign((size_t)n_sm * warps * 4, 0);
+    std::vector<u64> place(visits.size());
+    for (size_t i = 0; i < visits.size(); i++)
+    {
+        place[i] = visits[i].cta;
+        if (i == 0 || visits[i].cta != visits[i - 1].cta) continue;
+        place[i] = work.size() / (warps * 4);
+        work.resize(work.size() + warps * 4, 0);
+        for (u32 w = 0; w < warps; w++) link(&work[(place[i - 1] * warps + w) * 4], place[i]);
+    }
+    // (thousands of warps: half of the time of the build when it was done by one thread)
+#pragma omp parallel for schedule(static)
+    for (long long i = 0; i < (long long)visits.size(); i++)
+    {
+        const Visit &v = visits[i];
+        const double from = cost(v.s), all = cost(v.e) - from;
+        u64 here = v.s;
+        for (u32 w = 0; w < warps; w++)
+        {
+            const u64 to = w + 1 == warps ? v.e : at(from + all * (w + 1) / warps, here, v.e);
+            put(&work[(place[i] * warps + w) * 4], here, to, v.tile);
+            here = to;
+        }
+    }
+}
 
 struct Chunk
 {
@@ -272,7 +350,7 @@ struct Builder
     std::vector<Chunk> chunks;
     std::vector<u64> at; // [chunk * C + tile]: first its count, then where its elements go
     std::vector<u64> tile_begin, tile_pieces;
-    u64 N = 0;
+    u64 N = 0, runs = 0, near_runs = 0; // elements; rows' runs in the tiles, and those that lie near the one before
     std::vector<u32> row_code; // of every row of y: the shares of its parts, then what stands for it among the slices' rows
     // elements in tile order
     HostBuf<u32> e_row;
@@ -299,10 +377,11 @@ struct Builder
         row_code.assign(n_rows, 0);
         std::vector<u32> share;
         for (const TiledSource &s : src) share.push_back(share_of_part(s));
-        ThreadCounters pieces_of_thread(C), n_of_thread(C); // (neighbours in `at` share cache lines)
-#pragma omp parallel
+        ThreadCounters pieces_of_thread(C), n_of_thread(C), row_of_thread(C); // (neighbours in `at` share cache lines)
+u64 all_runs = 0, all_near = 0;
+#pragma omp parallel reduction(+ : all_runs, all_near)
         {
-            u64 *const pieces = pieces_of_thread.mine(), *const n = n_of_thread.mine();
+            u64 *const pieces = pieces_of_thread.mine(), *const n = n_of_thread.mine(), *const last = row_of_thread.mine();
 #pragma omp for schedule(dynamic, 1)
             for (long long c = 0; c < (long long)chunks.size(); c++)
             {
@@ -324,6 +403,12 @@ struct Builder
                     if (r != row || t != tile || run == kMaxPiece)
                     {
                         pieces[t]++;
+                        if (r != last[t])
+                        {
+                            all_runs++;
+                            all_near += r - last[t] <= kNearRows ? 1 : 0;
+                            last[t] = r;
+                        }
                         if (r != row) row_ends();
                         of_row++;
                         row = r;
@@ -339,6 +424,8 @@ struct Builder
 #pragma omp critical
             for (u64 t = 0; t < C; t++) tile_pieces[t] += pieces[t];
         }
+        runs = all_runs;
+        near_runs = all_near;
         tile_begin.assign(C + 1, 0);
         u64 sum = 0;
         for (u64 t = 0; t < C; t++)
@@ -561,8 +648,6 @@ struct Builder
         // the warps are cut the same way
         std::vector<u64> tile_step(C + 1, steps);
         for (u64 t = C; t-- > 0;) tile_step[t] = tile_block[t] < blocks.size() ? blocks[tile_block[t]].step : steps;
-        u64 used = 0;
-        for (u64 t = 0; t < C; t++) used += tile_step[t + 1] > tile_step[t] ? 1 : 0;
         const u32 *end = out.end.p;
         auto slice_of = [&](u64 step) { return (u64)(std::upper_bound(end, end + nsl, (u32)step) - end); };
         auto cost_of = [&](u64 step) { return (double)step + kSliceCost * (double)slice_of(step); };
@@ -580,61 +665,141 @@ struct Builder
             if (j < nsl) step = std::min<u64>(step, end[j]);
             return std::min(std::max(step, lo), hi);
         };
-        const double tile_cost = (double)kTiledTileBytes / (kTiledSlice * (sizeof(VT) + 2.0)); // by bytes
-        const double per = (cost_of(steps) + tile_cost * (double)(used + n_sm - 1)) / n_sm;
-        out.work.assign((size_t)n_sm * kTiledWarps * 4, 0);
-        u64 s = 0, t = 0;
-        struct Visit
+        const double tile_cost = (double)kTiledTileBytes / (kTiledSlice * (sizeof(VT) + 2.0));
+        share_out(
+            n_sm, kTiledWarps, tile_step, tile_cost, cost_of, step_at, out.work,
+            [&](u32 *o, u64 from, u64 to, u64 tile) {
+                o[0] = (u32)from;
+                o[1] = (u32)to;
+                o[2] = (u32)slice_of(from);
+                o[3] |= (u32)tile;
+            },
+            [](u32 *o, u64 next) { o[3] |= (u32)next << 16; });
+    }
+
+    // ---- units
+    static constexpr u32 S = kTiledLane, U = kTiledUnit;
+    // places of an element (unit u, lane l, k-th of the lane) among the values and columns: 16 bytes of a lane side by side
+    static constexpr u32 VV = 16 / sizeof(VT);
+    u64 val_at(u64 q) const
+    {
+        const u32 i = (u32)(q % U), l = i / S, k = i % S;
+        return q - i + (k / VV * 32 + l) * VV + k % VV;
+    }
+    u64 col_at(u64 q) const
+    {
+        const u32 i = (u32)(q % U), l = i / S, k = i % S;
+        return q - i + (k / 8 * 32 + l) * 8 + k % 8;
+    }
+
+    // as scatter(), with a unit of its own at the beginning of every tile
+    void scatter_units(TiledHost &out)
+    {
+        std::vector<u64> to_unit(C), end(C); // what a tile's places move by, and where its elements end
+        u64 moved = 0;
+        for (u64 t = 0; t < C; t++)
         {
-            size_t at;
-            u64 s, e, tile;
-        };
-        std::vector<Visit> visits;
-        double spent = 0; // by the CTAs before this one: what they left or took too much moves on, instead of piling up
-        for (int cta = 0; cta < n_sm; cta++)
+            to_unit[t] = moved;
+            end[t] = tile_begin[t + 1] + moved;
+            moved += (U - end[t] % U) % U;
+        }
+        for (u64 t = 1; t <= C; t++) tile_begin[t] = t < C ? tile_begin[t] + to_unit[t] : tile_begin[C] + moved;
+        const u64 places = tile_begin[C];
+        e_row.make(places);
+        out.val.make(places * sizeof(VT));
+        out.col.make(places);
+        VT *const val = (VT *)out.val.p;
+        uint16_t *const cl = out.col.p;
+        ThreadCounters to_of_thread(C);
+#pragma omp parallel
         {
-            double budget = per * (cta + 1) - spent;
-            long long prev = -1;
-            while (s < steps && (cta + 1 == n_sm || prev < 0 || budget > tile_cost + 16))
+            u64 *const to = to_of_thread.mine();
+#pragma omp for schedule(dynamic, 1)
+            for (long long c = 0; c < (long long)chunks.size(); c++)
             {
-                while (tile_step[t + 1] <= s) t++;
-                budget -= tile_cost;
-                const u64 last = tile_step[t + 1];
-                const double from = cost_of(s);
-                const u64 e = cta + 1 == n_sm ? last : std::min(last, std::max(s + kTiledWarps, step_at(from + budget, s, last)));
-                size_t visit = (size_t)cta;
-                if (prev >= 0)
-                {
-                    visit = out.work.size() / (kTiledWarps * 4);
-                    out.work.resize(out.work.size() + kTiledWarps * 4, 0);
-                    for (u32 w = 0; w < kTiledWarps; w++) out.work[((size_t)prev * kTiledWarps + w) * 4 + 3] |= (u32)visit << 16;
-                }
-                const double all = cost_of(e) - from;
-                visits.push_back({visit, s, e, t});
-                prev = (long long)visit;
-                s = e;
-                budget -= all;
-                spent += tile_cost + all;
-                if (e < last) break;
+                for (u64 t = 0; t < C; t++) to[t] = at[(size_t)c * C + t] + to_unit[t];
+                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) ASP_INLINE {
+                    const u64 t = (u32)col / TW, q = to[t]++;
+                    e_row.p[q] = (u32)r;
+                    cl[col_at(q)] = (uint16_t)(col - t * TW);
+                    val[val_at(q)] = v;
+                });
             }
         }
-        // (4736 warps and more: half of the time of this function when it was done by one thread)
+        // what fills a tile's last unit belongs to its last row and adds 0 * 0
+        for (u64 t = 0; t < C; t++)
+            for (u64 q = end[t]; q < tile_begin[t + 1]; q++)
+            {
+                e_row.p[q] = e_row.p[end[t] - 1];
+                cl[col_at(q)] = (uint16_t)TW;
+                val[val_at(q)] = 0;
+            }
+    }
+
+    void units(int n_sm, TiledHost &out)
+    {
+        const u64 n = tile_begin[C] / U;
+        out.word.make(n * 32);
+        out.seg.make(n + kTiledSlackUnits);
+        // what stands for a row among the units' rows
+        const bool some = !out.parts.empty();
+        const u32 all = out.n_parts > 0 && !out.direct ? kTiledInParts : 0;
 #pragma omp parallel for schedule(static)
-        for (long long i = 0; i < (long long)visits.size(); i++)
+        for (long long u = 0; u < (long long)n; u++)
         {
-            const Visit &v = visits[i];
-            const double from = cost_of(v.s), all = cost_of(v.e) - from;
-            u64 at_step = v.s;
-            for (u32 w = 0; w < kTiledWarps; w++)
+            u32 *const row = e_row.p + (u64)u * U;
+            u32 found = 0, before = 0;
+            for (u32 l = 0; l < 32; l++)
             {
-                u32 *o = &out.work[(v.at * kTiledWarps + w) * 4];
-                o[0] = (u32)at_step;
-                at_step = w + 1 == kTiledWarps ? v.e : step_at(from + all * (w + 1) / kTiledWarps, at_step, v.e);
-                o[1] = (u32)at_step;
-                o[2] = (u32)slice_of(o[0]);
-                o[3] |= (u32)v.tile;
+                u32 word = found << 16;
+                for (u32 k = 0; k < S; k++)
+                {
+                    const u32 r = row[l * S + k];
+                    if (l + k > 0 && r == before) continue;
+                    before = r;
+                    word |= 1u << k;
+                    row[found++] = some ? row_code[r] : r | all; // (never beyond what has been read)
+                }
+                out.word.p[(u64)u * 32 + l] = word;
             }
+            out.seg.p[u] = found;
         }
+        u64 sum = 0;
+        for (u64 u = 0; u < n; u++)
+        {
+            const u32 found = out.seg.p[u];
+            out.seg.p[u] = (u32)sum;
+            sum += found;
+        }
+        for (u32 i = 0; i < kTiledSlackUnits; i++) out.seg.p[n + i] = (u32)sum;
+        out.row.make(std::max<u64>(sum, 1));
+#pragma omp parallel for schedule(static)
+        for (long long u = 0; u < (long long)n; u++) memcpy(out.row.p + out.seg.p[u], e_row.p + (u64)u * U, (out.seg.p[u + 1] - out.seg.p[u]) * sizeof(u32));
+        out.nnz = N;
+        out.units = n;
+        // work of the CTAs: the units in order; a unit costs its elements and its rows
+        std::vector<u64> begin(C + 1);
+        for (u64 t = 0; t <= C; t++) begin[t] = tile_begin[t] / U;
+        const u32 *seg = out.seg.p;
+        auto cost_of = [&](u64 u) { return (double)(u * U) + kRowCost * (double)seg[u]; };
+        auto unit_at = [&](double cost, u64 lo, u64 hi) {
+            while (lo < hi)
+            {
+                const u64 mid = (lo + hi) / 2;
+                if (cost_of(mid) >= cost) hi = mid;
+                else lo = mid + 1;
+            }
+            return lo;
+        };
+        const double tile_cost = 0.5 * (double)kTiledTileBytes / (sizeof(VT) + 2.0);
+        share_out(
+            n_sm, kTiledUnitWarps, begin, tile_cost, cost_of, unit_at, out.work,
+            [](u32 *o, u64 from, u64 to, u64 tile) {
+                o[0] = (u32)from;
+                o[1] = (u32)to;
+                o[2] = (u32)tile;
+            },
+            [](u32 *o, u64 next) { o[3] = (u32)next; });
     }
 };
 
@@ -691,6 +856,12 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     }
     if (tiled_us(b.N, pieces, red) > 0.85 * own_us) return false;
     b.number_rows(out);
+    if (b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs)
+    {
+        b.scatter_units(out);
+        b.units(n_sm, out);
+        return true;
+    }
     b.scatter();
     b.slices(n_sm, out);
     return true;

@@ -16,10 +16,15 @@
 //          take `copies` sums of a row in turn, which k_rows adds pairwise. A piece is summed with more than the value's bits, too.
 // The stream is read two batches deep into registers. 159 KB of shared memory per tile leave the L1 enough lines for the
 // loads in flight: with 224 KB the same stream is read at 4.2 instead of 5 TB/s.
+// Where rows have few elements in a tile (1 to 7) and lie side by side, there are units instead of slices (k_tiled_units): a slice
+// puts pieces of one length together, so that its `red` goes to 32 rows anywhere among 1024, ten lines of sums or more, each of which is a
+// request to L2, and that is what bounds it. A unit is 256 elements of a tile in order, eight a lane. Every lane adds up the runs of its
+// elements, what reaches over lanes is added by a scan, and the sums leave in the order of the rows: two to three lines a `red`. That
+// takes more instructions an element (31 against 21), so long runs stay with slices; the figures are where the rule is (tiled_build.cpp).
 // A tile is loaded by cp.async, every thread's ten pieces in flight at once. Through registers, five at a time, nothing else runs for
 // 5 us of an SpMV over R-MAT scale 21 (ten SpMVs: 504 -> 476 us; by bulk copies 482).
-// Measured, fp32 (against the formats' own kernels): 200,000 rows of 40..120 non-zeros, random columns among 1 M: 38 us
-// (76 us, row-grouped); 9,001 rows of 1000..3000: 26 us (77 us, long-row).
+// Measured, fp32 (against the formats' own kernels): 200,000 rows of 40..120 non-zeros, random columns among 1 M: 31 us
+// (76 us, row-grouped; 38 us in slices); 9,001 rows of 1000..3000: 25 us (77 us, long-row).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -144,6 +149,28 @@ __device__ __forceinline__ void add_rows(VT *y, double *sum, u32 row, double v, 
     else atomicAdd(y + row, (VT)v);
 }
 
+// a CTA's tile of x, and a zero after it
+template <u32 NT, class VT>
+__device__ __forceinline__ void load_tile(const TiledArgs &a, VT *xs, u32 tile, u32 tile_cols)
+{
+    const VT *xp = (const VT *)a.x + (u64)tile * tile_cols;
+    const u64 left = a.n_cols - (u64)tile * tile_cols;
+    const u32 n = left < tile_cols ? (u32)left : tile_cols;
+    constexpr u32 V = 16 / sizeof(VT);
+    u32 i = 0;
+    if (((uintptr_t)xp & 15) == 0)
+    {
+        // straight to shared memory, all of a thread's 16-byte pieces in flight at once
+        const u32 n4 = n / V, to = (u32)__cvta_generic_to_shared(xs);
+        for (u32 j = threadIdx.x; j < n4; j += NT)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + j * 16), "l"((const char *)xp + (size_t)j * 16) : "memory");
+        i = n4 * V;
+    }
+    for (i += threadIdx.x; i < n; i += NT) xs[i] = ld_x1(xp + i);
+    if (threadIdx.x == 0) xs[tile_cols] = 0;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 template <class VT, int U>
 __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
 {
@@ -183,24 +210,7 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
         }
         else
             __syncthreads(); // the tile before has been read
-        {
-            const VT *xp = (const VT *)a.x + (u64)tile * tile_cols;
-            const u64 left = a.n_cols - (u64)tile * tile_cols;
-            const u32 n = left < tile_cols ? (u32)left : tile_cols;
-            constexpr u32 V = 16 / sizeof(VT);
-            u32 i = 0;
-            if (((uintptr_t)xp & 15) == 0)
-            {
-                // straight to shared memory, all of a thread's 16-byte pieces in flight at once
-                const u32 n4 = n / V, to = (u32)__cvta_generic_to_shared(xs);
-                for (u32 j = threadIdx.x; j < n4; j += 1024)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + j * 16), "l"((const char *)xp + (size_t)j * 16) : "memory");
-                i = n4 * V;
-            }
-            for (i += threadIdx.x; i < n; i += 1024) xs[i] = ld_x1(xp + i);
-            if (threadIdx.x == 0) xs[tile_cols] = 0;
-            asm volatile("cp.async.wait_all;" ::: "memory");
-        }
+        load_tile<1024>(a, xs, tile, tile_cols);
         __syncthreads();
         Sum<VT> acc0, acc1;
         while (step < end)
@@ -242,6 +252,170 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
             }
             acc0.batch();
             acc1.batch();
+        }
+    } while (visit != 0);
+}
+
+// ---- units: where rows have few elements in a tile
+const u32 kUnitSmem = kTiledTileBytes + kTiledUnitWarps * kTiledStage * 8;
+
+// Sum of a row's products in a lane, in fp64. fp64 values: the sum and the rounding errors that it left out (two-sum); 13 operations
+// a product of the 64 that an SM does per clock in fp64, of which a non-zero takes one.
+template <class VT>
+struct LaneSum;
+template <>
+struct LaneSum<float>
+{
+    double sum = 0;
+    __device__ __forceinline__ void add(float v, float x) { sum = fma((double)v, (double)x, sum); }
+    __device__ __forceinline__ double get() const { return sum; }
+    __device__ __forceinline__ void clear() { sum = 0; }
+};
+template <>
+struct LaneSum<double>
+{
+    double hi = 0, lo = 0;
+    __device__ __forceinline__ void add(double v, double x)
+    {
+        const double p = v * x, t = hi + p, b = t - hi;
+        lo += (hi - (t - b)) + (p - b) + fma(v, x, -p);
+        hi = t;
+    }
+    __device__ __forceinline__ double get() const { return isfinite(hi) ? hi + lo : hi; } // (the errors of an infinite sum are no numbers)
+    __device__ __forceinline__ void clear() { hi = lo = 0; }
+};
+
+// 16 bytes of values
+template <class VT>
+struct Vec;
+template <>
+struct Vec<float>
+{
+    typedef float4 type;
+    static __device__ __forceinline__ void out(const float4 &q, float *v) { v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w; }
+};
+template <>
+struct Vec<double>
+{
+    typedef double2 type;
+    static __device__ __forceinline__ void out(const double2 &q, double *v) { v[0] = q.x, v[1] = q.y; }
+};
+
+// MODE: rows are added up in y (0), have sums (1), or some have (2)
+template <class VT, int MODE>
+__global__ void __launch_bounds__(kTiledUnitWarps * 32, 1) k_tiled_units(TiledArgs a, u32 tile_cols)
+{
+    typedef typename Vec<VT>::type Q;
+    constexpr u32 S = kTiledLane, VV = 16 / sizeof(VT), NV = S / VV, NC = S / 8, U = 32 * S, NT = kTiledUnitWarps * 32, R = S;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    VT *const xs = reinterpret_cast<VT *>(smem_raw);
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *const stage = reinterpret_cast<double *>(smem_raw + kTiledTileBytes) + warp * kTiledStage; // row j of the unit: stage[j + 1]
+    VT *const y = (VT *)a.y;
+    bool first = true;
+    u32 visit = blockIdx.x;
+    do
+    {
+        const uint4 k = __ldg(a.work + (size_t)visit * kTiledUnitWarps + warp);
+        u32 unit = k.x;
+        const u32 end = k.y, tile = k.z;
+        visit = k.w;
+        double *const sum = a.sum + (size_t)((tile + warp) & (a.copies - 1)) * a.sum_stride;
+        Q qv[NV];
+        uint4 qc[NC];
+        u32 word = 0, rows[R];
+        // rows of the unit in `row`: [s0, s1), of the next one [s1, s2)
+        u32 s0 = __ldg(a.seg + unit), s1 = __ldg(a.seg + unit + 1), s2 = __ldg(a.seg + unit + 2);
+        auto fetch = [&](u32 u, u32 from, u32 to) {
+            const Q *vp = reinterpret_cast<const Q *>(a.val) + (size_t)u * (U / VV) + lane;
+            const uint4 *cp = reinterpret_cast<const uint4 *>(a.col) + (size_t)u * (U / 8) + lane;
+#pragma unroll
+            for (u32 i = 0; i < NV; i++) qv[i] = __ldcs(vp + i * 32);
+#pragma unroll
+            for (u32 i = 0; i < NC; i++) qc[i] = __ldcs(cp + i * 32);
+            word = __ldcs(a.word + (size_t)u * 32 + lane);
+#pragma unroll
+            for (u32 i = 0; i < R; i++)
+            {
+                if (from + i * 32 >= to) break;
+                if (from + i * 32 + lane < to) rows[i] = __ldcs(a.row + from + i * 32 + lane);
+            }
+        };
+        if (unit < end) fetch(unit, s0, s1);
+        if (first)
+        {
+            // nothing above depends on what ran before
+            grid_release();
+            grid_wait();
+            first = false;
+        }
+        else
+            __syncthreads(); // the tile before has been read
+        load_tile<NT>(a, xs, tile, tile_cols);
+        __syncthreads();
+        while (unit < end)
+        {
+            VT v[S], x[S];
+            u32 row[R];
+            const u32 F = word, n_rows = s1 - s0;
+#pragma unroll
+            for (u32 i = 0; i < NV; i++) Vec<VT>::out(qv[i], v + i * VV);
+#pragma unroll
+            for (u32 i = 0; i < NC; i++)
+            {
+                const u32 c[4] = {qc[i].x, qc[i].y, qc[i].z, qc[i].w};
+#pragma unroll
+                for (u32 j = 0; j < 4; j++)
+                {
+                    x[i * 8 + 2 * j] = xs[c[j] & 0xffffu];
+                    x[i * 8 + 2 * j + 1] = xs[c[j] >> 16];
+                }
+            }
+#pragma unroll
+            for (u32 i = 0; i < R; i++) row[i] = rows[i];
+            unit++;
+            s0 = s1;
+            s1 = s2;
+            s2 = __ldg(a.seg + unit + 2);
+            if (unit < end) fetch(unit, s0, s1);
+            // Every start stores what the lane has summed since the one before and goes on from zero. Before its first start that is
+            // the end of a row of lanes before: it goes where that row's sum will be, and comes back.
+            double *const mine = stage + (F >> 16);
+            double *to = mine;
+            LaneSum<VT> acc;
+#pragma unroll
+            for (u32 j = 0; j < S; j++)
+            {
+                if (F & (1u << j))
+                {
+                    *to++ = acc.get();
+                    acc.clear();
+                }
+                acc.add(v[j], x[j]);
+            }
+            const bool starts = (F & 0xffffu) != 0;
+            double sc = starts ? *mine : acc.get();
+            // lane l: the sum up to the next lane in which a row starts; rounds as long as there are so many lanes without a start
+            const u32 none = ~__ballot_sync(0xffffffffu, starts);
+            for (u32 d = 1, c = none; c != 0; c &= c >> d, d *= 2)
+            {
+                const double o = __shfl_down_sync(0xffffffffu, sc, d);
+                if (lane + d < 32 && (c >> lane & 1u)) sc += o;
+            }
+            const double more = __shfl_down_sync(0xffffffffu, sc, 1);
+            if (starts) *to = lane == 31 ? acc.get() : acc.get() + more; // (after every lane has read its own)
+            __syncwarp();
+#pragma unroll
+            for (u32 i = 0; i < R; i++)
+            {
+                if (i * 32 >= n_rows) break;
+                const u32 j = i * 32 + lane, r = row[i];
+                if (j >= n_rows) continue;
+                // (results unused: red.global.add)
+                if (MODE == 1 || (MODE == 2 && (r & kTiledInParts))) atomicAdd(sum + (r & ~kTiledInParts), stage[j + 1]);
+                else atomicAdd(y + r, (VT)stage[j + 1]);
+            }
+            __syncwarp();
         }
     } while (visit != 0);
 }
@@ -317,7 +491,10 @@ cudaError_t launch_sums(const TiledArgs &a, unsigned n_sm, cudaStream_t st)
         const cudaError_t e = clear((VT *)a.y, a.n_rows, n_sm, st);
         if (e != cudaSuccess) return e;
     }
-    return launch_pdl(k_tiled<VT, Batch<VT>::U>, dim3(n_sm), dim3(kTiledWarps * 32), kTiledTileBytes, st, a, (u32)tiled_tile_cols(sizeof(VT) == 8));
+    const auto tiled = [&](auto kernel, u32 warps, u32 smem) { return launch_pdl(kernel, dim3(n_sm), dim3(warps * 32), smem, st, a, (u32)tiled_tile_cols(sizeof(VT) == 8)); };
+    if (!a.word) return tiled(k_tiled<VT, Batch<VT>::U>, kTiledWarps, kTiledTileBytes);
+    if (!a.direct) return tiled(k_tiled_units<VT, 1>, kTiledUnitWarps, kUnitSmem);
+    return a.n_parts == 0 ? tiled(k_tiled_units<VT, 0>, kTiledUnitWarps, kUnitSmem) : tiled(k_tiled_units<VT, 2>, kTiledUnitWarps, kUnitSmem);
 }
 
 template <class VT>
@@ -345,11 +522,29 @@ cudaError_t launch_clear(int val_is_f64, void *y, unsigned long long n, unsigned
     return val_is_f64 ? clear((double *)y, n, n_sm, st) : clear((float *)y, n, n_sm, st);
 }
 
-cudaError_t tiled_setup(int val_is_f64)
+namespace
 {
-    const void *f = val_is_f64 ? (const void *)k_tiled<double, Batch<double>::U> : (const void *)k_tiled<float, Batch<float>::U>;
-    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTiledTileBytes);
+template <class VT>
+cudaError_t setup()
+{
+    const struct
+    {
+        const void *f;
+        u32 smem;
+    } all[] = {{(const void *)k_tiled<VT, Batch<VT>::U>, kTiledTileBytes},
+               {(const void *)k_tiled_units<VT, 0>, kUnitSmem},
+               {(const void *)k_tiled_units<VT, 1>, kUnitSmem},
+               {(const void *)k_tiled_units<VT, 2>, kUnitSmem}};
+    for (const auto &k : all)
+    {
+        const cudaError_t e = cudaFuncSetAttribute(k.f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
+} // namespace
+
+cudaError_t tiled_setup(int val_is_f64) { return val_is_f64 ? setup<double>() : setup<float>(); }
 
 cudaError_t launch_tiled_sums(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st)
 {

@@ -24,6 +24,12 @@ const uint32_t kTiledInParts = 0x80000000u; // row entry: the rest is a place am
 // steps and slices the kernel may read past the end (prefetch)
 const uint32_t kTiledSlackSteps = 8, kTiledSlackSlices = 2;
 
+constexpr uint32_t kTiledUnitWarps = 16;         // per CTA of the kernel for units
+constexpr uint32_t kTiledLane = 8;               // consecutive elements of a lane ...
+constexpr uint32_t kTiledUnit = 32 * kTiledLane; // ... and of a warp, which are a unit
+constexpr uint32_t kTiledStage = kTiledUnit + 2; // sums of a unit's rows, 8 bytes each, that a warp lays out in the shared memory after the tile
+const uint32_t kTiledSlackUnits = 4;             // entries of `seg` that the kernel may read past the end
+
 // columns of a tile; the shared memory after them holds one zero, which what pads a slice multiplies (never an infinite x)
 constexpr uint32_t tiled_tile_cols(bool f64) { return kTiledTileBytes / (f64 ? 8u : 4u) - 32u; }
 
@@ -61,6 +67,12 @@ struct TiledHost
     HostBuf<uint32_t> end;      // slice s covers steps [end[s - 1], end[s])
     std::vector<uint32_t> work; // {first step, end step, slice, tile | next visit << 16} per warp; visit v at v * kTiledWarps
     uint64_t nnz = 0, steps = 0, slices = 0;
+    // units > 0: units instead of slices. Then val and col hold them one after the other, in each the first 16 bytes of every lane, the
+    // next 16 bytes of every lane, ...; row[seg[u], seg[u + 1]) are the rows of unit u; work: {first unit, end unit, tile, next visit (0: none)},
+    // visit v at v * kTiledUnitWarps
+    uint64_t units = 0;
+    HostBuf<uint32_t> word; // unit u, lane l: bit k: its k-th element starts a row; from bit 16: rows that start in the lanes before
+    HostBuf<uint32_t> seg;
     unsigned copies = 1; // sums of a row, which tiles and warps take in turn: 1, 2, 4, 8 or 16
     bool covers_all_rows = false; // every row of y has at least one element
     bool direct = false;          // some are added up in y itself
@@ -73,7 +85,8 @@ struct TiledArgs
 {
     const void *val;
     const uint16_t *col;
-    const uint32_t *row, *end;
+    const uint32_t *row, *end;  // slices
+    const uint32_t *word, *seg; // units (word: NULL where there are slices)
     const uint4 *work;
     const uint32_t *parts; // n_parts rows (NULL: all rows of y) ...
     double *sum;           // ... and their sums, copies * sum_stride of them, zero between the calls
