@@ -253,9 +253,9 @@ const u32 kMaxPiece = 32;    // elements of a row's piece: bounds the serial cha
 const u32 kWindow = 1024;    // pieces that are sorted by length together: lanes of a slice stay near in y
 // Units or slices. A slice's `red` of a warp goes to the rows of 32 pieces of one length, anywhere among 1024 pieces; a unit's goes to
 // neighbouring rows, but a unit takes more instructions an element. fp32, random columns, 80 a row, slices / units: 25 tiles 38.2 / 31.2 us
-// (200,000 rows), 20 tiles 13.3 / 9.7 (40,000 rows), 13 tiles 9.1 / 6.6 (20,000), 8 tiles 21.3 / 21.0 (150,000), 3 tiles 18.7 / 20.4; fp64,
-// 19 tiles 33.4 / 30.8. Long runs: 9,001 rows of 2000 in 25 tiles 25.0 / 28.8, R-MAT scale 21 (8.5 a run) 476 / 643. Rows far apart (strips
-// sorted by length) 19.7 / 24.3.
+// (200,000 rows), 20 tiles 13.3 / 9.7 (40,000 rows), 13 tiles 9.1 / 6.6 (20,000), 8 tiles 21.3 / 21.0 (150,000), 3 tiles 18.7 / 20.4. Long runs: 9,001 rows of 2000 in 25 tiles 25.0 / 28.8, R-MAT scale 21 (8.5 a run) 476 / 643. Rows far apart (strips
+// sorted by length) 19.7 / 24.3. fp64 stays with slices: 19 tiles 33.5 / 31.2 us, but 0.95e-16 / 1.27e-16 from the exact sums (the scan's
+// roundings; fp32 4.2e-8 / 2.5e-8).
 const u64 kRunForUnits = 7;  // at most so many elements a run, on average
 const u64 kNearRows = 4;     // and three quarters of the runs at most so many rows behind the run before
 const double kRowCost = 1.0; // of a row of a unit, in elements: its entry and its `red`
@@ -277,10 +277,13 @@ void share_out(int n_sm, u32 warps, const std::vector<u64> &begin, double tile_c
         u64 cta, s, e, tile;
     };
     std::vector<Visit> visits;
+    std::vector<double> tile_at(C + 1);
+    for (u64 t = 0; t <= C; t++) tile_at[t] = cost(begin[t]);
     // every CTA takes what it can do at a cost of `most`: true, if that is everything
     auto fill = [&](double most) {
         visits.clear();
         u64 s = 0, t = 0;
+        double from = 0; // cost(s), but for what one place costs
         for (int cta = 0; cta < n_sm && s < n; cta++)
         {
             double left = most;
@@ -288,20 +291,21 @@ void share_out(int n_sm, u32 warps, const std::vector<u64> &begin, double tile_c
             {
                 while (begin[t + 1] <= s) t++;
                 left -= tile_cost;
-                const u64 last = begin[t + 1];
-                const double from = cost(s);
-                const u64 e = cost(last) - from <= left ? last : std::min(last, std::max(s + 1, at(from + left, s, last)));
+                const u64 last = begin[t + 1], e = tile_at[t + 1] - from <= left ? last : std::min(last, std::max(s + 1, at(from + left, s, last)));
                 visits.push_back({(u64)cta, s, e, t});
-                left -= cost(e) - from;
+                const double to = e < last ? std::max(from, from + left) : tile_at[t + 1];
+                left -= to - from;
+                from = to;
                 s = e;
                 if (e < last) break;
             }
         }
         return s == n;
     };
-    double lo = cost(n) / n_sm, hi = cost(n) + tile_cost * (double)C;
-    while (!fill(hi)) hi *= 2;
-    for (int i = 0; i < 40 && hi - lo > 1; i++)
+    // to half a percent: eight times 150 searches (a tenth of a millisecond)
+    double lo = tile_at[C] / n_sm, hi = (tile_at[C] + tile_cost * (double)(C + (u64)n_sm)) / n_sm;
+    while (!fill(hi)) lo = hi, hi *= 1.25;
+    while (hi - lo > 0.005 * hi)
     {
         const double mid = (lo + hi) / 2;
         (fill(mid) ? hi : lo) = mid;
@@ -856,11 +860,14 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     }
     if (tiled_us(b.N, pieces, red) > 0.85 * own_us) return false;
     b.number_rows(out);
-    if (b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs)
+    if constexpr (sizeof(VT) == 4)
     {
-        b.scatter_units(out);
-        b.units(n_sm, out);
-        return true;
+        if (b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs)
+        {
+            b.scatter_units(out);
+            b.units(n_sm, out);
+            return true;
+        }
     }
     b.scatter();
     b.slices(n_sm, out);

@@ -13,7 +13,7 @@
 //   parts  a row that gets there in many parts would collect a rounding error with each (fp32, 80 elements over 25 tiles: 1.0e-7
 //          from the 64-bit result, the formats' own kernels 0.72e-7): the sums of such rows are 64-bit ones in memory of the
 //          group, which k_rows turns into y and leaves as zeros for the next call (0.42e-7). In fp64 tiles and warps
-//          take `copies` sums of a row in turn, which k_rows adds pairwise. A piece is summed with more than the value's bits, too.
+//          take `copies` sums of a row in turn, which k_rows adds up with their roundings. A piece is summed with more than the value's bits, too.
 // The stream is read two batches deep into registers. 159 KB of shared memory per tile leave the L1 enough lines for the
 // loads in flight: with 224 KB the same stream is read at 4.2 instead of 5 TB/s.
 // Where rows have few elements in a tile (1 to 7) and lie side by side, there are units instead of slices (k_tiled_units): a slice
@@ -256,62 +256,19 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
     } while (visit != 0);
 }
 
-// ---- units: where rows have few elements in a tile
+// ---- units: where rows have few elements in a tile (fp32)
 const u32 kUnitSmem = kTiledTileBytes + kTiledUnitWarps * kTiledStage * 8;
 
-// Sum of a row's products in a lane, in fp64. fp64 values: the sum and the rounding errors that it left out (two-sum); 13 operations
-// a product of the 64 that an SM does per clock in fp64, of which a non-zero takes one.
-template <class VT>
-struct LaneSum;
-template <>
-struct LaneSum<float>
-{
-    double sum = 0;
-    __device__ __forceinline__ void add(float v, float x) { sum = fma((double)v, (double)x, sum); }
-    __device__ __forceinline__ double get() const { return sum; }
-    __device__ __forceinline__ void clear() { sum = 0; }
-};
-template <>
-struct LaneSum<double>
-{
-    double hi = 0, lo = 0;
-    __device__ __forceinline__ void add(double v, double x)
-    {
-        const double p = v * x, t = hi + p, b = t - hi;
-        lo += (hi - (t - b)) + (p - b) + fma(v, x, -p);
-        hi = t;
-    }
-    __device__ __forceinline__ double get() const { return isfinite(hi) ? hi + lo : hi; } // (the errors of an infinite sum are no numbers)
-    __device__ __forceinline__ void clear() { hi = lo = 0; }
-};
-
-// 16 bytes of values
-template <class VT>
-struct Vec;
-template <>
-struct Vec<float>
-{
-    typedef float4 type;
-    static __device__ __forceinline__ void out(const float4 &q, float *v) { v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w; }
-};
-template <>
-struct Vec<double>
-{
-    typedef double2 type;
-    static __device__ __forceinline__ void out(const double2 &q, double *v) { v[0] = q.x, v[1] = q.y; }
-};
-
 // MODE: rows are added up in y (0), have sums (1), or some have (2)
-template <class VT, int MODE>
+template <int MODE>
 __global__ void __launch_bounds__(kTiledUnitWarps * 32, 1) k_tiled_units(TiledArgs a, u32 tile_cols)
 {
-    typedef typename Vec<VT>::type Q;
-    constexpr u32 S = kTiledLane, VV = 16 / sizeof(VT), NV = S / VV, NC = S / 8, U = 32 * S, NT = kTiledUnitWarps * 32, R = S;
+    constexpr u32 S = kTiledLane, U = kTiledUnit, NV = S / 4, NC = S / 8, NT = kTiledUnitWarps * 32, R = S;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    VT *const xs = reinterpret_cast<VT *>(smem_raw);
+    float *const xs = reinterpret_cast<float *>(smem_raw);
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double *const stage = reinterpret_cast<double *>(smem_raw + kTiledTileBytes) + warp * kTiledStage; // row j of the unit: stage[j + 1]
-    VT *const y = (VT *)a.y;
+    float *const y = (float *)a.y;
     bool first = true;
     u32 visit = blockIdx.x;
     do
@@ -321,13 +278,13 @@ __global__ void __launch_bounds__(kTiledUnitWarps * 32, 1) k_tiled_units(TiledAr
         const u32 end = k.y, tile = k.z;
         visit = k.w;
         double *const sum = a.sum + (size_t)((tile + warp) & (a.copies - 1)) * a.sum_stride;
-        Q qv[NV];
+        float4 qv[NV];
         uint4 qc[NC];
         u32 word = 0, rows[R];
         // rows of the unit in `row`: [s0, s1), of the next one [s1, s2)
         u32 s0 = __ldg(a.seg + unit), s1 = __ldg(a.seg + unit + 1), s2 = __ldg(a.seg + unit + 2);
         auto fetch = [&](u32 u, u32 from, u32 to) {
-            const Q *vp = reinterpret_cast<const Q *>(a.val) + (size_t)u * (U / VV) + lane;
+            const float4 *vp = reinterpret_cast<const float4 *>(a.val) + (size_t)u * (U / 4) + lane;
             const uint4 *cp = reinterpret_cast<const uint4 *>(a.col) + (size_t)u * (U / 8) + lane;
 #pragma unroll
             for (u32 i = 0; i < NV; i++) qv[i] = __ldcs(vp + i * 32);
@@ -355,11 +312,11 @@ __global__ void __launch_bounds__(kTiledUnitWarps * 32, 1) k_tiled_units(TiledAr
         __syncthreads();
         while (unit < end)
         {
-            VT v[S], x[S];
+            float v[S], x[S];
             u32 row[R];
             const u32 F = word, n_rows = s1 - s0;
 #pragma unroll
-            for (u32 i = 0; i < NV; i++) Vec<VT>::out(qv[i], v + i * VV);
+            for (u32 i = 0; i < NV; i++) v[4 * i] = qv[i].x, v[4 * i + 1] = qv[i].y, v[4 * i + 2] = qv[i].z, v[4 * i + 3] = qv[i].w;
 #pragma unroll
             for (u32 i = 0; i < NC; i++)
             {
@@ -382,19 +339,19 @@ __global__ void __launch_bounds__(kTiledUnitWarps * 32, 1) k_tiled_units(TiledAr
             // the end of a row of lanes before: it goes where that row's sum will be, and comes back.
             double *const mine = stage + (F >> 16);
             double *to = mine;
-            LaneSum<VT> acc;
+            double acc = 0; // (exact products)
 #pragma unroll
             for (u32 j = 0; j < S; j++)
             {
                 if (F & (1u << j))
                 {
-                    *to++ = acc.get();
-                    acc.clear();
+                    *to++ = acc;
+                    acc = 0;
                 }
-                acc.add(v[j], x[j]);
+                acc = fma((double)v[j], (double)x[j], acc);
             }
             const bool starts = (F & 0xffffu) != 0;
-            double sc = starts ? *mine : acc.get();
+            double sc = starts ? *mine : acc;
             // lane l: the sum up to the next lane in which a row starts; rounds as long as there are so many lanes without a start
             const u32 none = ~__ballot_sync(0xffffffffu, starts);
             for (u32 d = 1, c = none; c != 0; c &= c >> d, d *= 2)
@@ -403,7 +360,7 @@ __global__ void __launch_bounds__(kTiledUnitWarps * 32, 1) k_tiled_units(TiledAr
                 if (lane + d < 32 && (c >> lane & 1u)) sc += o;
             }
             const double more = __shfl_down_sync(0xffffffffu, sc, 1);
-            if (starts) *to = lane == 31 ? acc.get() : acc.get() + more; // (after every lane has read its own)
+            if (starts) *to = lane == 31 ? acc : acc + more; // (after every lane has read its own)
             __syncwarp();
 #pragma unroll
             for (u32 i = 0; i < R; i++)
@@ -413,7 +370,7 @@ __global__ void __launch_bounds__(kTiledUnitWarps * 32, 1) k_tiled_units(TiledAr
                 if (j >= n_rows) continue;
                 // (results unused: red.global.add)
                 if (MODE == 1 || (MODE == 2 && (r & kTiledInParts))) atomicAdd(sum + (r & ~kTiledInParts), stage[j + 1]);
-                else atomicAdd(y + r, (VT)stage[j + 1]);
+                else atomicAdd(y + r, (float)stage[j + 1]);
             }
             __syncwarp();
         }
@@ -453,11 +410,15 @@ __global__ void __launch_bounds__(256) k_rows(const u32 *rows, double *sum, u64 
             {
 #pragma unroll
                 for (int g = 0; g < G; g++) sum[g * stride + r + u * threads] = 0;
+                double hi = s[u][0], lo = 0; // the sum of the copies, and what its roundings leave out
 #pragma unroll
-                for (int d = 1; d < G; d *= 2)
-#pragma unroll
-                    for (int g = 0; g + d < G; g += 2 * d) s[u][g] += s[u][g + d];
-                y[to[u]] = (VT)s[u][0];
+                for (int g = 1; g < G; g++)
+                {
+                    const double v = s[u][g], t = hi + v, b = t - hi;
+                    lo += (hi - (t - b)) + (v - b);
+                    hi = t;
+                }
+                y[to[u]] = (VT)(G > 1 && isfinite(hi) ? hi + lo : hi);
             }
     }
 }
@@ -493,8 +454,9 @@ cudaError_t launch_sums(const TiledArgs &a, unsigned n_sm, cudaStream_t st)
     }
     const auto tiled = [&](auto kernel, u32 warps, u32 smem) { return launch_pdl(kernel, dim3(n_sm), dim3(warps * 32), smem, st, a, (u32)tiled_tile_cols(sizeof(VT) == 8)); };
     if (!a.word) return tiled(k_tiled<VT, Batch<VT>::U>, kTiledWarps, kTiledTileBytes);
-    if (!a.direct) return tiled(k_tiled_units<VT, 1>, kTiledUnitWarps, kUnitSmem);
-    return a.n_parts == 0 ? tiled(k_tiled_units<VT, 0>, kTiledUnitWarps, kUnitSmem) : tiled(k_tiled_units<VT, 2>, kTiledUnitWarps, kUnitSmem);
+    if (sizeof(VT) == 8) return cudaErrorInvalidValue; // (units are fp32)
+    if (!a.direct) return tiled(k_tiled_units<1>, kTiledUnitWarps, kUnitSmem);
+    return a.n_parts == 0 ? tiled(k_tiled_units<0>, kTiledUnitWarps, kUnitSmem) : tiled(k_tiled_units<2>, kTiledUnitWarps, kUnitSmem);
 }
 
 template <class VT>
@@ -524,27 +486,17 @@ cudaError_t launch_clear(int val_is_f64, void *y, unsigned long long n, unsigned
 
 namespace
 {
-template <class VT>
-cudaError_t setup()
-{
-    const struct
-    {
-        const void *f;
-        u32 smem;
-    } all[] = {{(const void *)k_tiled<VT, Batch<VT>::U>, kTiledTileBytes},
-               {(const void *)k_tiled_units<VT, 0>, kUnitSmem},
-               {(const void *)k_tiled_units<VT, 1>, kUnitSmem},
-               {(const void *)k_tiled_units<VT, 2>, kUnitSmem}};
-    for (const auto &k : all)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(k.f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-}
+cudaError_t allow(const void *f, u32 smem) { return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }
 } // namespace
 
-cudaError_t tiled_setup(int val_is_f64) { return val_is_f64 ? setup<double>() : setup<float>(); }
+cudaError_t tiled_setup(int val_is_f64)
+{
+    if (val_is_f64) return allow((const void *)k_tiled<double, Batch<double>::U>, kTiledTileBytes);
+    cudaError_t e = allow((const void *)k_tiled<float, Batch<float>::U>, kTiledTileBytes);
+    for (const void *f : {(const void *)k_tiled_units<0>, (const void *)k_tiled_units<1>, (const void *)k_tiled_units<2>})
+        if (e == cudaSuccess) e = allow(f, kUnitSmem);
+    return e;
+}
 
 cudaError_t launch_tiled_sums(int val_is_f64, const TiledArgs &a, unsigned n_sm, cudaStream_t st)
 {
