@@ -347,7 +347,7 @@ void dense_row_coarse_sort(Matrix &m, u64 step)
     Arr<uint8_t> val;
     uint8_t *nval = val.make(m.val.b.size());
     const int es = m.val.es;
-#pragma omp parallel for schedule(dynamic, 4096) if (m.nnz > kParallelNnz)
+#pragma omp parallel for schedule(dynamic, 256) if (m.nnz > kParallelNnz)
     for (u64 i = 0; i < R; i++)
     {
         const u64 o = m.perm[i], n = len[o];
@@ -676,7 +676,8 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     const int es = b.val.es;
     const u64 NW = W.block_num;
     // few WLBs (one over the whole sub-matrix, as the ELL-like graphs have it): the rows of each are shared out; many: the WLBs are
-    const bool by_rows = NW < 256;
+    // (with 70 WLBs of 128 rows, whose rows are too few to be shared out, everything ran on one thread)
+    const bool by_rows = NW < 48 || (NW < 256 && b.n_rows > NW * kParallelRows);
     std::vector<u32> blb_of(NW);
     for (u64 i = 0; i < B.block_num; i++)
         for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) blb_of[w] = (u32)i;

@@ -259,7 +259,7 @@ static asp_status make_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t 
         if (indptr[r + 1] < indptr[r]) bad_row = std::min<uint64_t>(bad_row, (uint64_t)r);
     if (bad_row == n_rows) // (rows are only looked into once the offsets are known to be in order)
     {
-#pragma omp parallel for schedule(dynamic, 4096) reduction(min : bad_row) if ((uint64_t)indptr[n_rows] > kParallelNnz)
+#pragma omp parallel for schedule(dynamic, 256) reduction(min : bad_row) if ((uint64_t)indptr[n_rows] > kParallelNnz)
         for (int64_t r = 0; r < (int64_t)n_rows; r++)
         {
             bool bad = false;

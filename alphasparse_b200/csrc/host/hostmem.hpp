@@ -80,10 +80,12 @@ class IdleBlocks
 std::shared_ptr<void> big_buffer(size_t bytes);
 void host_pool_trim();
 
-// Below these a loop runs on the calling thread: waking sixteen threads and waiting for the slowest costs up to a millisecond on
-// a busy host, as much as the loop itself.
-const size_t kParallelBytes = 4u << 20;
-const uint64_t kParallelRows = 1u << 18, kParallelNnz = 1u << 19;
+// Below these a loop runs on the calling thread. Measured on 16 cores, matrices assembled, laid out, uploaded and used once, with 4 MB,
+// 2^18 rows and 2^19 non-zeros here / with these: 3 x 3 blocks, 28,000 non-zeros 168 / 105 us, 180,000 720 / 210, 414,000 1480 / 230-300,
+// 3.2 million 1875 / 1640-1700 (the check of its rows); ELL-like, 220,000 1610 / 1140-1210. A parallel region costs 5 to 10 us there, more on
+// a busy host.
+const size_t kParallelBytes = 1u << 18;
+const uint64_t kParallelRows = 1u << 13, kParallelNnz = 1u << 14;
 // f(i) for i in [0, n), shared out among the threads or without a parallel region at all (an inactive one costs 0.4 us, too much
 // for what is done per block)
 template <class F>
@@ -100,7 +102,7 @@ void for_each(uint64_t n, bool share, F &&f)
 
 inline void par_copy(void *dst, const void *src, size_t bytes)
 {
-    const size_t piece = 1u << 18;
+    const size_t piece = 1u << 16;
     const long long n = (long long)((bytes + piece - 1) / piece);
 #pragma omp parallel for schedule(static) if (bytes > kParallelBytes)
     for (long long i = 0; i < n; i++)
@@ -112,7 +114,7 @@ inline void par_copy(void *dst, const void *src, size_t bytes)
 
 inline void par_zero(void *dst, size_t bytes)
 {
-    const size_t piece = 1u << 18;
+    const size_t piece = 1u << 16;
     const long long n = (long long)((bytes + piece - 1) / piece);
 #pragma omp parallel for schedule(static) if (bytes > kParallelBytes)
     for (long long i = 0; i < n; i++)

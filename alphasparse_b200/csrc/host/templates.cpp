@@ -222,7 +222,7 @@ Arr<u64> tlb_global_rows(const CompressedBlock &b, bool &adjacent_equal)
     }
     else
     {
-#pragma omp parallel for schedule(dynamic, 64) if (T.block_num > kParallelRows)
+#pragma omp parallel for schedule(dynamic, 4) if (T.block_num > kParallelRows)
         for (u64 i = 0; i < B.block_num; i++)
             for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w, false);
     }
@@ -357,7 +357,7 @@ void interleave_per_blb(const CompressedBlock &b, const std::vector<u64> &thr, c
     const int cb = dtype_bytes(b.col_dt), es = b.val.es;
     uint8_t *cp = col.make(n_pad * cb), *vp = val.make(n_pad * es);
     const u64 nb = b.blb.block_num;
-#pragma omp parallel for schedule(dynamic, 64) if (n_pad > kParallelNnz)
+#pragma omp parallel for schedule(dynamic, 4) if (n_pad > kParallelNnz)
     for (u64 i = 0; i < nb; i++)
     {
         const u64 nz0 = b.blb.coo_begin.v[i], n = thr[i + 1] - thr[i];
@@ -474,7 +474,7 @@ void staggered_arrays(const CompressedBlock &b, Arr<uint8_t> &col, Arr<uint8_t> 
         }
     else
     {
-#pragma omp parallel for schedule(dynamic, 64) if (n_pad > kParallelNnz)
+#pragma omp parallel for schedule(dynamic, 4) if (n_pad > kParallelNnz)
         for (u64 i = 0; i < nb; i++)
             for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w);
     }
