@@ -253,9 +253,10 @@ const u32 kMaxPiece = 32;    // elements of a row's piece: bounds the serial cha
 const u32 kWindow = 1024;    // pieces that are sorted by length together: lanes of a slice stay near in y
 // Units or slices. A slice's `red` of a warp goes to the rows of 32 pieces of one length, anywhere among 1024 pieces; a unit's goes to
 // neighbouring rows, but a unit takes more instructions an element. fp32, random columns, 80 a row, slices / units: 25 tiles 38.2 / 31.2 us
-// (200,000 rows), 20 tiles 13.3 / 9.7 (40,000 rows), 13 tiles 9.1 / 6.6 (20,000), 8 tiles 21.3 / 21.0 (150,000), 3 tiles 18.7 / 20.4. Long runs: 9,001 rows of 2000 in 25 tiles 25.0 / 28.8, R-MAT scale 21 (8.5 a run) 476 / 643. Rows far apart (strips
-// sorted by length) 19.7 / 24.3. fp64 stays with slices: 19 tiles 33.5 / 31.2 us, but 0.95e-16 / 1.27e-16 from the exact sums (the scan's
-// roundings; fp32 4.2e-8 / 2.5e-8).
+// (200,000 rows), 20 tiles 13.3 / 9.7 (40,000 rows), 13 tiles 9.1 / 6.6 (20,000), 8 tiles 21.3 / 21.0 (150,000), 3 tiles 18.7 / 20.4. Long
+// runs: 9,001 rows of 2000 in 25 tiles 25.0 / 28.8, R-MAT scale 21 (8.5 a run) 476 / 643. Rows far apart (strips sorted by length) 19.7 /
+// 24.3. fp64 stays with slices: 19 tiles 33.5 / 31.2 us, but 0.95e-16 / 1.27e-16 from the exact sums (the scan's roundings; fp32 4.2e-8 /
+// 2.5e-8).
 const u64 kRunForUnits = 7;  // at most so many elements a run, on average
 const u64 kNearRows = 4;     // and three quarters of the runs at most so many rows behind the run before
 const double kRowCost = 1.0; // of a row of a unit, in elements: its entry and its `red`
