@@ -863,7 +863,8 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     b.number_rows(out);
     if constexpr (sizeof(VT) == 4)
     {
-        if (b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs)
+        // (runs that are cut where the threads' chunks end may be missing from `runs`)
+        if (b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs && tiled_units_fit(b.runs + b.C * b.chunks.size(), b.N, b.C))
         {
             b.scatter_units(out);
             b.units(n_sm, out);

@@ -29,6 +29,10 @@ constexpr uint32_t kTiledLane = 8;               // consecutive elements of a la
 constexpr uint32_t kTiledUnit = 32 * kTiledLane; // ... and of a warp, which are a unit
 constexpr uint32_t kTiledStage = kTiledUnit + 2; // sums of a unit's rows, 8 bytes each, that a warp lays out in the shared memory after the tile
 const uint32_t kTiledSlackUnits = 4;             // entries of `seg` that the kernel may read past the end
+// Units have an entry per row that they begin, which `seg` finds with 32 bits (a step of slices is 64 elements): whether the offsets, and
+// those that the kernel forms behind the last one, stay below 2^32. An entry is a run of a row's elements in a tile, of which there are
+// `runs`, or what a unit's or a tile's begin cuts off one.
+constexpr bool tiled_units_fit(uint64_t runs, uint64_t elements, uint64_t tiles) { return runs + elements / kTiledUnit + 2 * tiles + kTiledUnit < (1ull << 32); }
 
 // columns of a tile; the shared memory after them holds one zero, which what pads a slice multiplies (never an infinite x)
 constexpr uint32_t tiled_tile_cols(bool f64) { return kTiledTileBytes / (f64 ? 8u : 4u) - 32u; }

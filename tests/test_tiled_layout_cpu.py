@@ -1,0 +1,26 @@
+"""CPU suite: the column-tiled layout's host side (csrc/host/tiled_build.cpp) by itself (tiled_layout.cpp)."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+PKG = os.path.join(os.path.dirname(HERE), "alphasparse_b200")
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("tiled") / "tiled_layout")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-fopenmp", "-I/usr/local/cuda/include", os.path.join(HERE, "tiled_layout.cpp"), "-o", exe,
+                    "-L" + PKG, "-l:libasp_b200.so", "-Wl,-rpath," + PKG], check=True)
+    return exe
+
+
+def run(program, *args, threads=4):
+    r = subprocess.run([program, *map(str, args)], capture_output=True, text=True, timeout=300, env=dict(os.environ, OMP_NUM_THREADS=str(threads)))
+    assert r.returncode == 0, (r.returncode, r.stdout, r.stderr[-500:])
+    return r.stdout
+
+
+def test_units_keep_to_32_bit_offsets(program):
+    run(program, "fit")
