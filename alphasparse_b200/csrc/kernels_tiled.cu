@@ -352,6 +352,7 @@ __global__ void __launch_bounds__(kTiledUnitWarps * 32, 1) k_tiled_units(TiledAr
             }
             const bool starts = (F & 0xffffu) != 0;
             double sc = starts ? *mine : acc;
+            __syncwarp(); // the lane before, whose last row ends there, stores the whole sum over it
             // lane l: the sum up to the next lane in which a row starts; rounds as long as there are so many lanes without a start
             const u32 none = ~__ballot_sync(0xffffffffu, starts);
             for (u32 d = 1, c = none; c != 0; c &= c >> d, d *= 2)
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(kTiledUnitWarps * 32, 1) k_tiled_units(TiledAr
                 if (lane + d < 32 && (c >> lane & 1u)) sc += o;
             }
             const double more = __shfl_down_sync(0xffffffffu, sc, 1);
-            if (starts) *to = lane == 31 ? acc : acc + more; // (after every lane has read its own)
+            if (starts) *to = lane == 31 ? acc : acc + more;
             __syncwarp();
 #pragma unroll
             for (u32 i = 0; i < R; i++)

@@ -80,3 +80,26 @@ def test_last_units_of_the_tiles(asp_ctx, dtype, over):
     refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, f"over {over}")
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_rows_over_several_lanes_are_whole(asp_ctx, seed):
+    """Small whole numbers, of which every sum is exact: a sum that lacks what other lanes hold of its row, or has it twice, differs. Runs of 1
+    to 9 elements, some of hundreds, begin and end at every place of a lane."""
+    tile, rows, tiles = 40672, 60_000, 16
+    rng = np.random.default_rng(seed)
+    runs = rng.integers(1, 10, size=(rows, tiles))
+    runs[rng.integers(0, rows, size=300), rng.integers(0, tiles, size=300)] = rng.integers(30, 700, size=300)
+    first = (np.arange(tiles) * tile + rng.integers(0, tile // 2, size=(rows, tiles))).reshape(-1)
+    begin = np.concatenate([[0], np.cumsum(runs.reshape(-1))])
+    at = np.arange(begin[-1]) - np.repeat(begin[:-1], runs.reshape(-1))
+    cols = (np.repeat(first, runs.reshape(-1)) + at * 13).astype(np.uint32)
+    m = M.CsrMatrix(rows, tiles * tile, np.concatenate([[0], np.cumsum(runs.sum(1))]).astype(np.int64), cols, rng.integers(-9, 10, size=cols.size).astype(np.float32))
+    x = rng.integers(-9, 10, size=m.n_cols).astype(np.float32)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": "K9", "nodes": K9, "template": "K9", "threads": 128, "row_reduce": 1}]})
+    assert g.layout_bytes() > 0
+    want = np.add.reduceat(m.values.astype(np.float64) * x[cols], m.indptr[:-1]).astype(np.float32)
+    for _ in range(5):
+        assert (g.spmv_host(x) == want).all()
+    g.close()
+    fmt.close()
