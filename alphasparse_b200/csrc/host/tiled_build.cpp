@@ -367,6 +367,8 @@ struct Builder
     {
     }
 
+    // whether a run of row r is a near one behind one of row `before`
+    static u64 near(u64 before, u64 r) { return r - before <= kNearRows ? 1 : 0; }
     void count()
     {
         u64 stored = 0;
@@ -382,15 +384,18 @@ struct Builder
         row_code.assign(n_rows, 0);
         std::vector<u32> share;
         for (const TiledSource &s : src) share.push_back(share_of_part(s));
-        ThreadCounters pieces_of_thread(C), n_of_thread(C), row_of_thread(C); // (neighbours in `at` share cache lines)
-u64 all_runs = 0, all_near = 0;
+        ThreadCounters pieces_of_thread(C), n_of_thread(C); // (neighbours in `at` share cache lines)
+        const size_t edges = (2 * C + 31) / 16 * 16;
+        std::vector<u32> edge(chunks.size() * edges); // rows of a chunk's first and last element in a tile, on cache lines of its own
+        u64 all_runs = 0, all_near = 0;
 #pragma omp parallel reduction(+ : all_runs, all_near)
         {
-            u64 *const pieces = pieces_of_thread.mine(), *const n = n_of_thread.mine(), *const last = row_of_thread.mine();
+            u64 *const pieces = pieces_of_thread.mine(), *const n = n_of_thread.mine();
 #pragma omp for schedule(dynamic, 1)
             for (long long c = 0; c < (long long)chunks.size(); c++)
             {
                 std::fill(n, n + C, 0);
+                u32 *const first = edge.data() + (size_t)c * edges, *const last = first + C;
                 u64 row = ~0ull, tile = ~0ull, run = 0;
                 u32 of_row = 0, elements = 0; // pieces and elements since the row changed
                 // rows that are one thread's in the template's kernel have no more parts than it adds elements
@@ -404,16 +409,17 @@ u64 all_runs = 0, all_near = 0;
                 };
                 walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT) ASP_INLINE {
                     const u64 t = (u32)col / TW;
-                    n[t]++;
+                    const bool begins = n[t]++ == 0;
                     if (r != row || t != tile || run == kMaxPiece)
                     {
                         pieces[t]++;
-                        if (r != last[t])
+                        if (begins) first[t] = (u32)r;
+                        else if (r != last[t])
                         {
                             all_runs++;
-                            all_near += r - last[t] <= kNearRows ? 1 : 0;
-                            last[t] = r;
+                            all_near += near(last[t], r);
                         }
+                        last[t] = (u32)r;
                         if (r != row) row_ends();
                         of_row++;
                         row = r;
@@ -436,9 +442,18 @@ u64 all_runs = 0, all_near = 0;
         for (u64 t = 0; t < C; t++)
         {
             tile_begin[t] = sum;
+            u64 before = ~0ull; // row of the chunks before
             for (size_t c = 0; c < chunks.size(); c++)
             {
                 const u64 n = at[c * C + t];
+                if (n > 0)
+                {
+                    // (whatever the threads made of it: the choice of the layout is the matrix's)
+                    const u32 *const first = edge.data() + c * edges, *const last = first + C;
+                    runs += before != first[t] ? 1 : 0;
+                    near_runs += before != ~0ull && before != first[t] ? near(before, first[t]) : 0;
+                    before = last[t];
+                }
                 at[c * C + t] = sum;
                 sum += n;
             }
@@ -863,8 +878,7 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     b.number_rows(out);
     if constexpr (sizeof(VT) == 4)
     {
-        // (runs that are cut where the threads' chunks end may be missing from `runs`)
-        if (b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs && tiled_units_fit(b.runs + b.C * b.chunks.size(), b.N, b.C))
+        if (b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs && tiled_units_fit(b.runs, b.N, b.C))
         {
             b.scatter_units(out);
             b.units(n_sm, out);

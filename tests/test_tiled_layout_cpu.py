@@ -24,3 +24,9 @@ def run(program, *args, threads=4):
 
 def test_units_keep_to_32_bit_offsets(program):
     run(program, "fit")
+
+
+@pytest.mark.parametrize("threads", [1, 3, 4, 16])
+def test_the_choice_of_units_does_not_depend_on_the_threads(program, threads):
+    for seed in (1, 2):
+        run(program, "choice", seed, threads=threads)
