@@ -80,12 +80,14 @@ class IdleBlocks
 std::shared_ptr<void> big_buffer(size_t bytes);
 void host_pool_trim();
 
-// Below these a loop runs on the calling thread. Measured on 16 cores, matrices assembled, laid out, uploaded and used once, with 4 MB,
-// 2^18 rows and 2^19 non-zeros here / with these: 3 x 3 blocks, 28,000 non-zeros 168 / 105 us, 180,000 720 / 210, 414,000 1480 / 230-300,
-// 3.2 million 1875 / 1640-1700 (the check of its rows); ELL-like, 220,000 1610 / 1140-1210. A parallel region costs 5 to 10 us there, more on
-// a busy host.
-const size_t kParallelBytes = 1u << 18;
-const uint64_t kParallelRows = 1u << 13, kParallelNnz = 1u << 14;
+// Below these a loop runs on the calling thread. A parallel region waits for its slowest thread, and where other programs keep the cores
+// busy that is one that is not running: 8 cores, a spinning process on each, rows of 8, built with 256 KB, 2^13 rows and 2^14 non-zeros
+// here / with these: 28,800 non-zeros 16-24 ms / 0.2-0.8 ms, 96,000 56-120 / 0.6-3.6, 400,000 64-168 / 2.3-23. Four threads that build at once:
+// 29,000 non-zeros 126-160 / 72-85 us a build, 96,000 260-476 / 163-211. A host that has nothing else to do gains from lower limits (16 cores,
+// 3 x 3 blocks: 28,000 non-zeros 168 -> 105 us, 414,000 1480 -> 230-300), but that cannot be told beforehand. They also are the size up to which a
+// forked process may build after its parent has: the threads of a region do not come along.
+const size_t kParallelBytes = 4u << 20;
+const uint64_t kParallelRows = 1u << 18, kParallelNnz = 1u << 19;
 // f(i) for i in [0, n), shared out among the threads or without a parallel region at all (an inactive one costs 0.4 us, too much
 // for what is done per block)
 template <class F>
