@@ -667,6 +667,21 @@ void sep_warp_level_col_fixed(CompressedBlock &b, u64 c)
     b.share_row_with_other_warp = true;
 }
 
+bool shares_rows_of_wlbs(const std::vector<u64> &rows, const std::vector<u64> &nnz, int val_bytes, u64 threads)
+{
+    // (one WLB over the whole sub-matrix, as the ELL-like graphs have it: its rows; 70 WLBs of 128 rows: the WLBs; 60 of which one
+    // holds nearly everything: its rows, or all the other threads wait for one)
+    u64 all = 0, largest = 0, one_by_one = 0;
+    for (size_t w = 0; w < rows.size(); w++)
+    {
+        const bool shared = nnz[w] * (u64)val_bytes > kParallelBytes || rows[w] > kParallelRows;
+        all += nnz[w];
+        largest = std::max(largest, nnz[w]);
+        one_by_one += shared ? nnz[w] / std::max<u64>(1, std::min(rows[w], threads)) : nnz[w];
+    }
+    return one_by_one <= std::max(all / threads, largest);
+}
+
 void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, bool tlb_rows)
 {
     Level &B = b.blb;
@@ -675,9 +690,7 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     T = Level();
     const int es = b.val.es;
     const u64 NW = W.block_num;
-    // few WLBs (one over the whole sub-matrix, as the ELL-like graphs have it): the rows of each are shared out; many: the WLBs are
-    // (with 70 WLBs of 128 rows, whose rows are too few to be shared out, everything ran on one thread)
-    const bool by_rows = NW < 48 || (NW < 256 && b.n_rows > NW * kParallelRows);
+    const bool by_rows = NW < 256 && shares_rows_of_wlbs(W.row_num.v, W.coo_size.v, es, (u64)omp_get_max_threads());
     std::vector<u32> blb_of(NW);
     for (u64 i = 0; i < B.block_num; i++)
         for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) blb_of[w] = (u32)i;

@@ -203,6 +203,9 @@ void sep_warp_level_col_fixed(CompressedBlock &b, u64 col_block_nnz);
 // COMPRESSED_THREAD_LEVEL_ROW_DIV / _COL_DIV (sep_thread_level_col_ell_with_padding, op_manager.cc:3105):
 // tlb_size == 0 means "one TLB per row" (TLB size = the WLB's longest row)
 void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, bool tlb_rows = true);
+// Whether it goes through the WLBs one by one and shares out the rows of those that are large enough, instead of sharing out the
+// WLBs: what then takes longest is what no other thread helps with.
+bool shares_rows_of_wlbs(const std::vector<u64> &rows, const std::vector<u64> &nnz, int val_bytes, u64 threads);
 // COMPRESSED_THREAD_LEVEL_NNZ_DIV (sep_thread_level_acc_to_nnz, op_manager.cc:3807)
 void sep_thread_level_acc_to_nnz(CompressedBlock &b, u64 tlb_nnz);
 // execute_default_div_to_complete_each_level_blocking (default_auto_tuner.cc:384); `rows_per_unit`: the template finds its
