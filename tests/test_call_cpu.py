@@ -1,8 +1,10 @@
 """CPU suite: the binding of asp_spmv without ctypes (csrc/python/call.c) refuses and accepts what the ctypes one did."""
 import ctypes as C
+import sys
 
 import pytest
 
+import alphasparse_b200
 from alphasparse_b200 import capi
 
 
@@ -34,6 +36,23 @@ def test_a_call_without_plan_or_with_other_pointers_falls_back():
     group.ctx = object.__new__(capi.Context)
     group.ctx._h = C.c_void_p()
     group._call = capi._native().Spmv(C.cast(capi.lib().asp_spmv, C.c_void_p).value, C.addressof(group.ctx._h), C.addressof(group._plans), 1)
+    for x in (16, None, C.c_void_p(16)):
+        with pytest.raises(capi.AspError):
+            group.spmv(x, 16)
+    with pytest.raises(C.ArgumentError):
+        group.spmv(1.5, 16)
+
+
+def test_calls_without_the_binding_go_through_ctypes(monkeypatch):
+    """Where only the library has been built, the same calls are taken and refused."""
+    monkeypatch.setitem(sys.modules, "alphasparse_b200._call", None)  # (as if there were no such file)
+    monkeypatch.delattr(alphasparse_b200, "_call", raising=False)
+    group = object.__new__(capi.PlanGroup)
+    group.n, group._plans = 1, (C.c_void_p * 1)()
+    group.ctx = object.__new__(capi.Context)
+    group.ctx._h = C.c_void_p()
+    group._call = capi._bind_spmv(group.ctx._h, group._plans, 1)
+    assert group._call(16, 32, 2) == 1 and b"NULL" in capi.lib().asp_last_error()
     for x in (16, None, C.c_void_p(16)):
         with pytest.raises(capi.AspError):
             group.spmv(x, 16)
