@@ -1,4 +1,4 @@
-/* The call of asp_spmv from Python (alphasparse_b200/_call.so).
+/* The call of asp_spmv from Python (the module alphasparse_b200._call).
  *
  * A small SpMV takes the GPU less time than its launch takes the host (2.0 us on the measured machine), and ctypes spends 0.7 us more on
  * converting six arguments. This binding is made once per plan group and converts two: 0.1 us. It holds addresses of what the

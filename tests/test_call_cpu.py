@@ -1,6 +1,9 @@
 """CPU suite: the binding of asp_spmv without ctypes (csrc/python/call.c) refuses and accepts what the ctypes one did."""
 import ctypes as C
+import importlib.machinery
+import os
 import sys
+import sysconfig
 
 import pytest
 
@@ -58,3 +61,11 @@ def test_calls_without_the_binding_go_through_ctypes(monkeypatch):
             group.spmv(x, 16)
     with pytest.raises(C.ArgumentError):
         group.spmv(1.5, 16)
+
+
+def test_the_binding_is_for_this_python_alone():
+    """It uses more of Python's interface than other versions share: they must not find it."""
+    suffix = sysconfig.get_config_var("EXT_SUFFIX")
+    assert suffix != ".so" and suffix in importlib.machinery.EXTENSION_SUFFIXES
+    assert capi._native().__file__.endswith("_call" + suffix)
+    assert not os.path.exists(os.path.join(os.path.dirname(capi.__file__), "_call.so"))
