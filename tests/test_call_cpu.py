@@ -69,3 +69,14 @@ def test_the_binding_is_for_this_python_alone():
     assert suffix != ".so" and suffix in importlib.machinery.EXTENSION_SUFFIXES
     assert capi._native().__file__.endswith("_call" + suffix)
     assert not os.path.exists(os.path.join(os.path.dirname(capi.__file__), "_call.so"))
+
+
+def test_the_build_does_without_headers_or_compiler(monkeypatch, tmp_path):
+    import __graft_entry__ as entry
+
+    monkeypatch.delenv("CC", raising=False)
+    monkeypatch.setattr(entry, "_call_path", lambda: str(tmp_path / "_call.so"))
+    assert "Python.h" in entry._build_call(include=str(tmp_path))
+    assert "compiler" in entry._build_call(compilers=("no-such-compiler",))
+    assert not os.listdir(tmp_path)
+    assert entry._build_call() is None and os.listdir(tmp_path) == ["_call.so"]
