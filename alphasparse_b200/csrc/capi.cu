@@ -1287,6 +1287,13 @@ asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path)
 
 uint64_t asp_plan_layout_bytes(const asp_plan *plan) { return plan && plan->tiled ? plan->tiled->layout_bytes : 0; }
 
+int asp_plan_layout_form(const asp_plan *plan)
+{
+    if (!plan || !plan->tiled) return 0;
+    const asp::TiledArgs &a = plan->tiled->args;
+    return (a.word ? ASP_FORM_UNITS : ASP_FORM_SLICES) | (a.direct || a.n_parts == 0 ? ASP_FORM_IN_Y : 0) | (a.n_parts > 0 ? ASP_FORM_IN_SUMS : 0);
+}
+
 asp_status asp_device_trim(int device)
 {
     int n = 0;

@@ -697,20 +697,8 @@ struct Builder
             [](u32 *o, u64 next) { o[3] |= (u32)next << 16; });
     }
 
-    // ---- units
+    // ---- units (fp32)
     static constexpr u32 S = kTiledLane, U = kTiledUnit;
-    // places of an element (unit u, lane l, k-th of the lane) among the values and columns: 16 bytes of a lane side by side
-    static constexpr u32 VV = 16 / sizeof(VT);
-    u64 val_at(u64 q) const
-    {
-        const u32 i = (u32)(q % U), l = i / S, k = i % S;
-        return q - i + (k / VV * 32 + l) * VV + k % VV;
-    }
-    u64 col_at(u64 q) const
-    {
-        const u32 i = (u32)(q % U), l = i / S, k = i % S;
-        return q - i + (k / 8 * 32 + l) * 8 + k % 8;
-    }
 
     // as scatter(), with a unit of its own at the beginning of every tile
     void scatter_units(TiledHost &out)
@@ -726,9 +714,9 @@ struct Builder
         for (u64 t = 1; t <= C; t++) tile_begin[t] = t < C ? tile_begin[t] + to_unit[t] : tile_begin[C] + moved;
         const u64 places = tile_begin[C];
         e_row.make(places);
-        out.val.make(places * sizeof(VT));
+        out.val.make(places * sizeof(float));
         out.col.make(places);
-        VT *const val = (VT *)out.val.p;
+        float *const val = (float *)out.val.p;
         uint16_t *const cl = out.col.p;
         ThreadCounters to_of_thread(C);
 #pragma omp parallel
@@ -738,11 +726,11 @@ struct Builder
             for (long long c = 0; c < (long long)chunks.size(); c++)
             {
                 for (u64 t = 0; t < C; t++) to[t] = at[(size_t)c * C + t] + to_unit[t];
-                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) ASP_INLINE {
+                walk_any<float>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, float v) ASP_INLINE {
                     const u64 t = (u32)col / TW, q = to[t]++;
                     e_row.p[q] = (u32)r;
-                    cl[col_at(q)] = (uint16_t)(col - t * TW);
-                    val[val_at(q)] = v;
+                    cl[q] = (uint16_t)(col - t * TW);
+                    val[unit_val_at(q)] = v;
                 });
             }
         }
@@ -751,8 +739,8 @@ struct Builder
             for (u64 q = end[t]; q < tile_begin[t + 1]; q++)
             {
                 e_row.p[q] = e_row.p[end[t] - 1];
-                cl[col_at(q)] = (uint16_t)TW;
-                val[val_at(q)] = 0;
+                cl[q] = (uint16_t)TW;
+                val[unit_val_at(q)] = 0;
             }
     }
 
@@ -811,7 +799,7 @@ struct Builder
             }
             return lo;
         };
-        const double tile_cost = 0.5 * (double)kTiledTileBytes / (sizeof(VT) + 2.0);
+        const double tile_cost = 0.5 * (double)kTiledTileBytes / (sizeof(float) + 2.0);
         share_out(
             n_sm, kTiledUnitWarps, begin, tile_cost, cost_of, unit_at, out.work,
             [](u32 *o, u64 from, u64 to, u64 tile) {

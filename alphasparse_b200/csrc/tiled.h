@@ -34,6 +34,9 @@ const uint32_t kTiledSlackUnits = 4;             // entries of `seg` that the ke
 // `runs`, or what a unit's or a tile's begin cuts off one.
 constexpr bool tiled_units_fit(uint64_t runs, uint64_t elements, uint64_t tiles) { return runs + elements / kTiledUnit + 2 * tiles + kTiledUnit < (1ull << 32); }
 
+// place of element q (unit q / 256, lane q % 256 / 8) among the units' fp32 values: 16 bytes of a lane side by side (its columns are 16 bytes)
+constexpr uint64_t unit_val_at(uint64_t q) { return q - q % kTiledUnit + (q % kTiledLane / 4 * 32 + q % kTiledUnit / kTiledLane) * 4 + q % 4; }
+
 // columns of a tile; the shared memory after them holds one zero, which what pads a slice multiplies (never an infinite x)
 constexpr uint32_t tiled_tile_cols(bool f64) { return kTiledTileBytes / (f64 ? 8u : 4u) - 32u; }
 

@@ -236,6 +236,16 @@ uint64_t asp_plan_format_bytes(const asp_plan *plan);
 /* bytes of device memory of the column-tiled layout that the plan's group runs (see asp_plan_group_create), beside the format
  * arrays; 0 when the group runs its templates' own kernels */
 uint64_t asp_plan_layout_bytes(const asp_plan *plan);
+/* what that layout consists of, 0 without one: the elements are in slices or in units, and rows are added up in y, as 64-bit sums, or some
+ * of them each way */
+enum
+{
+    ASP_FORM_SLICES = 1,
+    ASP_FORM_UNITS = 2,
+    ASP_FORM_IN_Y = 4,
+    ASP_FORM_IN_SUMS = 8
+};
+int asp_plan_layout_form(const asp_plan *plan);
 /* number of launches of its template's kernel that one asp_spmv over this plan issues (excluding the y clear); the plans of a group
  * that runs the column-tiled layout share one launch */
 int asp_plan_launches(const asp_plan *plan);

@@ -1,6 +1,7 @@
-"""GPU: the column-tiled layout in units (rows with few elements in a tile; csrc/kernels_tiled.cu, k_tiled_units), against the CPU oracle
-where units and lanes end: rows that go on into the next lanes and units, lanes without a row's start, last units that are full, by one or all
-but; rows added up in y, as 64-bit sums, and both; empty rows; infinite x; x and y off 16-byte alignment."""
+"""GPU: the column-tiled layout of rows with few elements in a tile, against the CPU oracle: in units (fp32; csrc/kernels_tiled.cu,
+k_tiled_units), where units and lanes end: rows that go on into the next lanes and units, lanes without a row's start, last units that are full,
+by one or all but; rows added up in y, as 64-bit sums, and both; empty rows; infinite x; x and y off 16-byte alignment. The same matrices in
+fp64 have slices. Which of them a matrix has is asserted: another one would be another kernel's test."""
 import numpy as np
 import pytest
 
@@ -12,12 +13,16 @@ pytestmark = pytest.mark.gpu
 K9, K6 = ["tlb_nnz 32"], ["row_padding 32 1", "blb_row_evenly 32", "tlb_col_fixed 4"]
 
 
+FP64 = {"direct": {"slices", "y"}, "sums": {"slices", "sums"}, "both": {"slices", "y", "sums"}}
+
+
 def lengths(kind, rng):
     if kind == "direct":  # at most as many parts as the template adds in sequence (32): 15 tiles
         return rng.integers(20, 61, size=150_000)
     if kind == "sums":  # more than the 8 that this template allows
         return rng.integers(40, 121, size=60_000)
-    n = rng.integers(20, 61, size=200_000)  # both, with rows of many units
+    # both, with rows of many units: rows enough for clearing y to be less than sums for all of them
+    n = rng.integers(15, 31, size=750_000)
     n[[0, 1, 77_777, -1]] = [30_000, 257, 9_000, 256]
     return n
 
@@ -34,7 +39,7 @@ def test_units_match_the_oracle(asp_ctx, kind, template, nodes, dtype, cols, emp
         n[rng.integers(2, n.size - 1, size=empty)] = 0
     m, x = M.from_row_lengths(n, cols, seed=7, dtype=dtype)
     fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": nodes, "template": template, "threads": 128, "row_reduce": 1}]})
-    assert g.layout_bytes() > 0, "the layout was not built for this matrix"
+    assert g.layout_form() == ({"units", *{"direct": ["y"], "sums": ["sums"], "both": ["y", "sums"]}[kind]} if dtype is np.float32 else FP64[kind])
     y_ref, scale = refdump.csr_ref(m, x)
     for shift in (0, 1):
         dx = torch.zeros(m.n_cols + shift, dtype=torch.from_numpy(x).dtype, device="cuda")
@@ -75,7 +80,7 @@ def test_last_units_of_the_tiles(asp_ctx, dtype, over):
     m = M.CsrMatrix(rows, tiles * tile, np.concatenate([[0], np.cumsum(n)]).astype(np.int64), cols, rng.standard_normal(cols.size).astype(dtype))
     x = rng.standard_normal(m.n_cols).astype(dtype)
     fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": "K9", "nodes": K9, "template": "K9", "threads": 128, "row_reduce": 1}]})
-    assert g.layout_bytes() > 0
+    assert ("units" if dtype is np.float32 else "slices") in g.layout_form()
     y_ref, scale = refdump.csr_ref(m, x)
     refdump.assert_y(g.spmv_host(x), y_ref, scale, m.values.dtype, f"over {over}")
     g.close()
@@ -97,7 +102,7 @@ def test_rows_over_several_lanes_are_whole(asp_ctx, seed):
     m = M.CsrMatrix(rows, tiles * tile, np.concatenate([[0], np.cumsum(runs.sum(1))]).astype(np.int64), cols, rng.integers(-9, 10, size=cols.size).astype(np.float32))
     x = rng.integers(-9, 10, size=m.n_cols).astype(np.float32)
     fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": "K9", "nodes": K9, "template": "K9", "threads": 128, "row_reduce": 1}]})
-    assert g.layout_bytes() > 0
+    assert "units" in g.layout_form()
     want = np.add.reduceat(m.values.astype(np.float64) * x[cols], m.indptr[:-1]).astype(np.float32)
     for _ in range(5):
         assert (g.spmv_host(x) == want).all()

@@ -30,3 +30,8 @@ def test_units_keep_to_32_bit_offsets(program):
 def test_the_choice_of_units_does_not_depend_on_the_threads(program, threads):
     for seed in (1, 2):
         run(program, "choice", seed, threads=threads)
+
+
+@pytest.mark.parametrize("mode", ["y", "sums", "both"])
+def test_units_hold_the_matrix(program, mode):
+    run(program, "units", mode)

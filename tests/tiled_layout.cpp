@@ -83,12 +83,100 @@ static int choice(int seed)
     return 0;
 }
 
+// Units, followed as the kernel does, against the sums of the matrix: rows added up in y ("y"), all as sums ("sums"), or some each way
+// ("both", which takes rows enough for clearing y to be less than their sums). Every element once, in a place of its own tile.
+static int units(const char *mode)
+{
+    const bool y_only = !strcmp(mode, "y"), both = !strcmp(mode, "both");
+    const uint32_t rows = both ? 700001 : y_only ? 500000 : 60000, tiles = both || y_only ? 8 : 25, tile = asp::tiled_tile_cols(false);
+    Rows m;
+    m.cols = (uint64_t)tiles * tile - 77;
+    srand(5);
+    std::vector<double> x(m.cols), want(rows, 0.0), got(rows, 0.0);
+    for (double &v : x) v = rand() % 19 - 9;
+    for (uint32_t r = 0; r < rows; r++)
+    {
+        uint32_t n = both ? 10 + rand() % 8 : y_only ? 8 : 50;
+        if (r == 0 || r == rows - 1 || r == rows / 3) n = both ? 9000 : y_only ? 8 : 700; // (over many units and lanes; more parts than y takes)
+        if (r % 1000 == 5) n = 0;
+        for (uint32_t k = 0; k < n; k++)
+        {
+            const uint64_t c = (uint64_t)k * m.cols / n + rand() % (m.cols / n);
+            m.col.push_back((uint32_t)c);
+            m.val.push_back((float)(1 + rand() % 9));
+            want[r] += m.val.back() * x[c];
+        }
+        m.add(r);
+    }
+    asp::TiledHost out;
+    if (!m.build(out)) return 10;
+    if (out.units == 0 || out.copies != 1 || out.nnz != m.col.size() || out.covers_all_rows) return 11;
+    if (out.direct != (both || y_only) || (out.n_parts > 0) != !y_only || out.parts.empty() == both) return 12;
+    if (both && out.n_parts != 3) return 13;
+    if (out.seg.n != out.units + asp::kTiledSlackUnits) return 14;
+    // the tile of every unit, from the work: every unit is one warp's, and a CTA's warps share a tile
+    const uint32_t W = asp::kTiledUnitWarps;
+    std::vector<int> tile_of(out.units, -1);
+    for (uint32_t cta = 0; cta < 148; cta++)
+        for (uint64_t visit = cta, first = 1; first || visit != 0; first = 0)
+        {
+            const uint32_t *o = &out.work[visit * W * 4], t = o[2], next = o[3];
+            for (uint32_t w = 0; w < W; w++, o += 4)
+            {
+                if (o[0] > o[1] || o[1] > out.units || o[2] != t || o[3] != next) return 15;
+                for (uint32_t u = o[0]; u < o[1]; u++)
+                {
+                    if (tile_of[u] >= 0) return 16;
+                    tile_of[u] = (int)t;
+                }
+            }
+            visit = next;
+        }
+    const float *val = (const float *)out.val.p;
+    std::vector<double> sum(out.n_parts, 0.0);
+    uint64_t elements = 0;
+    for (uint64_t u = 0; u < out.units; u++)
+    {
+        if (tile_of[u] < 0) return 17;
+        uint32_t row = 0, begun = 0;
+        for (uint64_t i = 0; i < asp::kTiledUnit; i++)
+        {
+            const uint64_t q = u * asp::kTiledUnit + i;
+            const uint32_t word = out.word.p[u * 32 + i / asp::kTiledLane], k = i % asp::kTiledLane;
+            if (k == 0 && word >> 16 != begun) return 18;
+            if (word >> k & 1)
+            {
+                row = out.row.p[out.seg.p[u] + begun];
+                begun++;
+            }
+            else if (i == 0) return 19;
+            if (out.col.p[q] == tile) // what fills a tile's last unit
+            {
+                if (val[asp::unit_val_at(q)] != 0) return 20;
+                continue;
+            }
+            const uint64_t c = (uint64_t)tile_of[u] * tile + out.col.p[q];
+            if (out.col.p[q] > tile || c >= m.cols) return 21;
+            elements++;
+            const bool in_parts = row & asp::kTiledInParts || (out.n_parts > 0 && !out.direct);
+            const uint32_t to = row & ~asp::kTiledInParts;
+            if (to >= (in_parts ? out.n_parts : rows)) return 22;
+            (in_parts ? sum : got)[to] += val[asp::unit_val_at(q)] * x[c];
+        }
+        if (begun != out.seg.p[u + 1] - out.seg.p[u]) return 23;
+    }
+    if (elements != m.col.size()) return 24;
+    for (uint64_t k = 0; k < out.n_parts; k++) got[out.parts.empty() ? k : out.parts[k]] += sum[k];
+    return got == want ? 0 : 25; // (whole numbers: exact)
+}
+
 int main(int argc, char **argv)
 {
     const char *part = argc > 1 ? argv[1] : "";
     int r = 99;
     if (!strcmp(part, "fit")) r = fit();
     if (!strcmp(part, "choice")) r = choice(argc > 2 ? atoi(argv[2]) : 1);
+    if (!strcmp(part, "units")) r = units(argc > 2 ? argv[2] : "");
     printf("%s %d\n", part, r);
     return r;
 }
