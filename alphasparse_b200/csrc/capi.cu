@@ -304,7 +304,18 @@ size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // The structural checks of asp_plan_group_create look at lengths and offsets; these look at what the
 // arrays SAY: every column a kernel will gather and every row it will write must lie inside x and y.
 // A caller that hands over one bad index would otherwise make a kernel read or write outside its
-// buffers on a GPU it shares with other jobs. Cost: one OpenMP pass over each index array.
+// buffers on a GPU it shares with other jobs. Cost: one shared pass over each index array.
+template <class T>
+uint64_t max_entry(const T *q, uint64_t n)
+{
+    std::atomic<uint64_t> top(0);
+    asp::host::share_ranges(n, n > (1 << 20), [&](uint64_t i, uint64_t e) {
+        T mx = 0;
+        for (; i < e; i++) mx = q[i] > mx ? q[i] : mx;
+        asp::host::raise<uint64_t>(top, mx);
+    });
+    return top;
+}
 uint64_t max_of(const HostMeta &h, uint64_t count)
 {
     if (count == 0) return 0;
@@ -312,25 +323,13 @@ uint64_t max_of(const HostMeta &h, uint64_t count)
     {
     case ASP_COMPRESS_NONE:
     {
-        uint64_t mx = 0;
-        const int64_t n = (int64_t)count;
         switch (h.dtype)
         {
-#define ASP_MAX_CASE(DT, T)                                                            \
-    case DT:                                                                           \
-    {                                                                                  \
-        const T *q = (const T *)h.p;                                                   \
-        _Pragma("omp parallel for reduction(max : mx) schedule(static) if (n > (1 << 20))") for (int64_t i = 0; i < n; i++) mx = q[i] > mx ? (uint64_t)q[i] : mx; \
-        break;                                                                         \
-    }
-            ASP_MAX_CASE(ASP_U8, uint8_t)
-            ASP_MAX_CASE(ASP_U16, uint16_t)
-            ASP_MAX_CASE(ASP_U32, uint32_t)
-        default:
-            ASP_MAX_CASE(ASP_U64, uint64_t)
-#undef ASP_MAX_CASE
+        case ASP_U8: return max_entry((const uint8_t *)h.p, count);
+        case ASP_U16: return max_entry((const uint16_t *)h.p, count);
+        case ASP_U32: return max_entry((const uint32_t *)h.p, count);
+        default: return max_entry((const uint64_t *)h.p, count);
         }
-        return mx;
     }
     case ASP_COMPRESS_LINEAR: return (count - 1) * h.coef + h.icpt;
     case ASP_COMPRESS_CONSTANT: return h.icpt;
@@ -417,12 +416,10 @@ bool validate_contents(const asp_plan_desc &d, const std::vector<HostMeta> &hm, 
         const HostMeta &br = hm[MS_BLK_ROW], &ro = hm[MS_ROW_OFF];
         const uint64_t rows_all = br.get(B);
         if (ro.kind == ASP_COMPRESS_NONE && ro.len < rows_all + 1) return why = "row offsets shorter than the row count", false;
-        bool ok = true;
-#pragma omp parallel for schedule(static) reduction(&& : ok) if (B > 4096)
-        for (int64_t b = 0; b < (int64_t)B; b++)
-        {
+        std::atomic<bool> ok(true);
+        asp::host::for_each(B, B > 4096, [&](uint64_t b) {
             const uint64_t r0 = br.get(b), r1 = br.get(b + 1);
-            if (r1 < r0 || r1 > rows_all) { ok = false; continue; }
+            if (r1 < r0 || r1 > rows_all) { ok = false; return; }
             uint64_t partials;
             if (d.template_type == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS) partials = hm[MS_BLK_THR].get(b + 1) - hm[MS_BLK_THR].get(b);
             else if (d.template_type == ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE) partials = hm[MS_BLK_WARP].get(b + 1) - hm[MS_BLK_WARP].get(b);
@@ -435,7 +432,7 @@ bool validate_contents(const asp_plan_desc &d, const std::vector<HostMeta> &hm, 
                 if (nx < prev || nx - g0 > partials) { ok = false; break; }
                 prev = nx;
             }
-        }
+        });
         if (!ok) return why = "a row's partial-result range leaves its BLB (row offsets / block_first_row_index inconsistent)", false;
         return device_rows_in_bounds(d, perm, std::min<uint64_t>(rows_all, a.effective), why);
     }
@@ -447,20 +444,23 @@ bool validate_contents(const asp_plan_desc &d, const std::vector<HostMeta> &hm, 
         const uint64_t W = a.n_units;
         const int S = (int)d.tlb_size, bw = d.bits_word;
         const uint64_t rmask = (1ull << d.bits_row) - 1;
-        uint64_t top = 0; // one past the largest relative row written
-#pragma omp parallel for schedule(static) reduction(max : top) if (W > 4096)
-        for (int64_t w = 0; w < (int64_t)W; w++)
-        {
-            const uint64_t R0 = fr.get(w);
-            for (int l = 0; l < 32; l++)
+        std::atomic<uint64_t> top(0); // one past the largest relative row written
+        asp::host::share_ranges(W, W > 4096, [&](uint64_t w, uint64_t e) {
+            uint64_t last = 0;
+            for (; w < e; w++)
             {
-                const uint64_t m = cm.get((uint64_t)w * 32 + l);
-                const uint64_t flags = S >= 64 ? m : (m >> (bw - S)) & ((S >= 64) ? ~0ull : ((1ull << S) - 1));
-                const int starts = __builtin_popcountll(flags);
-                if (starts) top = std::max<uint64_t>(top, R0 + (m & rmask) + starts);
+                const uint64_t R0 = fr.get(w);
+                for (int l = 0; l < 32; l++)
+                {
+                    const uint64_t m = cm.get(w * 32 + l);
+                    const uint64_t flags = S >= 64 ? m : (m >> (bw - S)) & ((S >= 64) ? ~0ull : ((1ull << S) - 1));
+                    const int starts = __builtin_popcountll(flags);
+                    if (starts) last = std::max<uint64_t>(last, R0 + (m & rmask) + starts);
+                }
             }
-        }
-        return device_rows_in_bounds(d, perm, top, why);
+            asp::host::raise(top, last);
+        });
+        return device_rows_in_bounds(d, perm, top.load(), why);
     }
     default: return true;
     }
@@ -614,6 +614,7 @@ namespace
 // plan objects returned); ctx may then be NULL.
 asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int layout, asp_plan **out_plans, bool dry)
 {
+    const asp::host::Caller caller;
 
     // ---- pass 1: validate descriptors, lay out the arena (arrays sharing a host pointer once)
     struct Slot
@@ -950,27 +951,33 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
                     return r + d.first_row;
                 };
                 std::vector<uint32_t> rows(2 * W);
-                uint64_t all_starts = 0;
+                std::atomic<uint64_t> sum_starts(0);
                 // rows without gaps: every warp starts at the row the one before ends with, or at the next
                 bool gapless = d.sort_kind == ASP_SORT_NONE && d.first_row == 0 && !a.atomic && fr.get(0) == 0;
-                bool in_step = true; // the first row that every thread names is the one its place in the warp implies
+                std::atomic<bool> in_step(true); // the first row that every thread names is the one its place in the warp implies
                 const uint64_t rmask = (1ull << d.bits_row) - 1;
-#pragma omp parallel for schedule(static) reduction(+ : all_starts) reduction(&& : in_step) if (W > 4096)
-                for (int64_t w = 0; w < (int64_t)W; w++)
-                {
-                    uint64_t starts = 0;
-                    for (int l = 0; l < 32; l++)
+                asp::host::share_ranges(W, W > 4096, [&](uint64_t w, uint64_t e) {
+                    uint64_t all = 0;
+                    bool in = true;
+                    for (; w < e; w++)
                     {
-                        const uint64_t m = cm.get((uint64_t)w * 32 + l);
-                        const uint64_t flags = S >= 64 ? m : ((m >> (bw - S)) & ((1ull << S) - 1));
-                        if (flags) in_step = in_step && (m & rmask) == starts;
-                        starts += (uint64_t)__builtin_popcountll(flags);
+                        uint64_t starts = 0;
+                        for (int l = 0; l < 32; l++)
+                        {
+                            const uint64_t m = cm.get(w * 32 + l);
+                            const uint64_t flags = S >= 64 ? m : ((m >> (bw - S)) & ((1ull << S) - 1));
+                            if (flags) in = in && (m & rmask) == starts;
+                            starts += (uint64_t)__builtin_popcountll(flags);
+                        }
+                        const uint64_t R0 = fr.get(w);
+                        rows[2 * w] = (uint32_t)row_of(R0);
+                        rows[2 * w + 1] = (uint32_t)row_of(R0 + (starts ? starts - 1 : 0));
+                        all += starts;
                     }
-                    const uint64_t R0 = fr.get(w);
-                    rows[2 * w] = (uint32_t)row_of(R0);
-                    rows[2 * w + 1] = (uint32_t)row_of(R0 + (starts ? starts - 1 : 0));
-                    all_starts += starts;
-                }
+                    sum_starts.fetch_add(all);
+                    if (!in) in_step = false;
+                });
+                const uint64_t all_starts = sum_starts;
                 // staging area of the staged write-out: room for twice the average number of rows a warp produces
                 // (a power of two between 32 and 256; warps with more rows send the rest straight out)
                 {

@@ -3,9 +3,6 @@
 
 #include <string.h>
 
-#ifdef _OPENMP
-#include <omp.h>
-#endif
 #include <algorithm>
 #include <stdexcept>
 #include <fstream>
@@ -77,12 +74,7 @@ std::unique_ptr<Matrix> relabel_by_column_count(const Matrix &m, bool empty_rows
 {
     const u64 n = m.n_rows;
     std::vector<u64> cnt(n, 0);
-#pragma omp parallel for schedule(static)
-    for (long long k = 0; k < (long long)m.nnz; k++)
-    {
-#pragma omp atomic
-        cnt[m.col[k]]++;
-    }
+    for_each(m.nnz, true, [&](u64 k) { __atomic_fetch_add(&cnt[m.col[k]], 1, __ATOMIC_RELAXED); });
     std::vector<u32> order(n);
     for (u64 i = 0; i < n; i++) order[i] = (u32)i;
     std::stable_sort(order.begin(), order.end(), [&](u32 a, u32 b) { return cnt[a] > cnt[b]; });
@@ -102,11 +94,11 @@ std::unique_ptr<Matrix> relabel_by_column_count(const Matrix &m, bool empty_rows
     out->val.es = m.val.es;
     uint8_t *oval = out->val.b.make(m.nnz * m.val.es);
     const size_t es = (size_t)m.val.es;
-#pragma omp parallel
-    {
-        std::vector<std::pair<u32, u64>> row; // (new column, position in the old row)
-#pragma omp for schedule(dynamic, 256)
-        for (long long k = 0; k < (long long)n; k++)
+    const unsigned width = std::min(crew_width(), kMostPieces);
+    std::vector<std::vector<std::pair<u32, u64>>> row_of(width); // (new column, position in the old row)
+    share_steps(n, 256, width, [&](u64 k, u64 last, unsigned who) {
+        std::vector<std::pair<u32, u64>> &row = row_of[who];
+        for (; k < last; k++)
         {
             const u64 b = m.rowptr[order[k]], e = m.rowptr[order[k] + 1], o = rp[k];
             row.clear();
@@ -118,7 +110,7 @@ std::unique_ptr<Matrix> relabel_by_column_count(const Matrix &m, bool empty_rows
                 memcpy(&oval[(o + j) * es], &m.val.b[row[j].second * es], es);
             }
         }
-    }
+    });
     return out;
 }
 
@@ -174,10 +166,8 @@ std::unique_ptr<Matrix> matrix_from_coo_file(const std::string &path, int val_dt
         p = next_line(p);
     }
     // slices of whole lines, one per thread
-    int nt = 1;
-#ifdef _OPENMP
-    nt = omp_get_max_threads();
-#endif
+    const unsigned width = std::min(crew_width(), kMostPieces);
+    int nt = (int)width;
     const size_t body = (size_t)(end - p);
     nt = (int)std::max<size_t>(1, std::min<size_t>((size_t)nt, body / (1u << 16) + 1));
     std::vector<const char *> cut(nt + 1);
@@ -196,9 +186,7 @@ std::unique_ptr<Matrix> matrix_from_coo_file(const std::string &path, int val_dt
         std::string err;
     };
     std::vector<Part> parts(nt);
-#pragma omp parallel for schedule(static, 1) num_threads(nt)
-    for (int t = 0; t < nt; t++)
-    {
+    share_pieces((unsigned)nt, width, [&](unsigned t, unsigned) {
         Part &pt = parts[t];
         const char *s = cut[t], *e = cut[t + 1];
         pt.rows.reserve((size_t)(e - s) / 12 + 16);
@@ -234,7 +222,7 @@ std::unique_ptr<Matrix> matrix_from_coo_file(const std::string &path, int val_dt
             pt.vals.push_back(v);
             s = next_line(q);
         }
-    }
+    });
     u64 nnz = 0;
     for (int t = 0; t < nt; t++)
     {
@@ -347,14 +335,15 @@ void dense_row_coarse_sort(Matrix &m, u64 step)
     Arr<uint8_t> val;
     uint8_t *nval = val.make(m.val.b.size());
     const int es = m.val.es;
-#pragma omp parallel for schedule(dynamic, 256) if (m.nnz > kParallelNnz)
-    for (u64 i = 0; i < R; i++)
-    {
-        const u64 o = m.perm[i], n = len[o];
-        if (n == 0) continue;
-        memcpy(&ncol[nrp[i]], &m.col[m.rowptr[o]], n * sizeof(u32));
-        memcpy(&nval[nrp[i] * es], &m.val.b[m.rowptr[o] * es], n * es);
-    }
+    share_steps(R, 256, m.nnz > kParallelNnz ? crew_width() : 1, [&](u64 i, u64 e, unsigned) {
+        for (; i < e; i++)
+        {
+            const u64 o = m.perm[i], n = len[o];
+            if (n == 0) continue;
+            memcpy(&ncol[nrp[i]], &m.col[m.rowptr[o]], n * sizeof(u32));
+            memcpy(&nval[nrp[i] * es], &m.val.b[m.rowptr[o] * es], n * es);
+        }
+    });
     m.rowptr.swap(rowptr);
     m.col.swap(col);
     m.val.b.swap(val);
@@ -427,8 +416,7 @@ void compress_dense_view(Matrix &m)
         else
         {
             u64 *rp = b.rowptr.make(b.n_rows + 1);
-#pragma omp parallel for schedule(static) if (b.n_rows > kParallelRows)
-            for (u64 r = 0; r <= b.n_rows; r++) rp[r] = m.rowptr[rg.min_row + r] - rg.begin_coo;
+            for_each(b.n_rows + 1, b.n_rows > kParallelRows, [&](u64 r) { rp[r] = m.rowptr[rg.min_row + r] - rg.begin_coo; });
         }
         const u64 n = rg.end_coo - rg.begin_coo + 1;
         b.col = m.col.view(rg.begin_coo, n);
@@ -690,7 +678,7 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     T = Level();
     const int es = b.val.es;
     const u64 NW = W.block_num;
-    const bool by_rows = NW < 256 && shares_rows_of_wlbs(W.row_num.v, W.coo_size.v, es, (u64)omp_get_max_threads());
+    const bool by_rows = NW < 256 && shares_rows_of_wlbs(W.row_num.v, W.coo_size.v, es, crew_width());
     std::vector<u32> blb_of(NW);
     for (u64 i = 0; i < B.block_num; i++)
         for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) blb_of[w] = (u32)i;
@@ -718,38 +706,32 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     auto count_wlb = [&](u64 w) {
         const Span s = span(w);
         const bool share = by_rows && s.rows > kParallelRows;
-        u64 S = tlb_size, tl = 0;
+        u64 S = tlb_size;
         auto length = [&](u64 r) {
             u64 lo, hi;
             return row_range(s, r, lo, hi);
         };
-        if (S == 0 && share)
+        if (S == 0)
         {
-#pragma omp parallel for schedule(static) reduction(max : S)
-            for (u64 r = 0; r < s.rows; r++) S = std::max(S, length(r));
+            std::atomic<u64> longest(0);
+            share_ranges(s.rows, share, [&](u64 r, u64 e) {
+                u64 most = 0;
+                for (; r < e; r++) most = std::max(most, length(r));
+                raise(longest, most);
+            });
+            S = longest.load(std::memory_order_relaxed);
         }
-        else if (S == 0)
-            for (u64 r = 0; r < s.rows; r++) S = std::max(S, length(r));
-        if (share)
-        {
-#pragma omp parallel for schedule(static) reduction(+ : tl)
-            for (u64 r = 0; r < s.rows; r++) tl += (length(r) + S - 1) / S;
-        }
-        else
-            for (u64 r = 0; r < s.rows; r++) tl += (length(r) + S - 1) / S;
+        u64 tl = 0;
+        share_ranges(s.rows, share, [&](u64 r, u64 e) {
+            u64 sum = 0;
+            for (; r < e; r++) sum += (length(r) + S - 1) / S;
+            __atomic_fetch_add(&tl, sum, __ATOMIC_RELAXED);
+        });
         wlb_S[w] = S;
         wlb_tl[w] = tl;
     };
-    // (no parallel region, not even one of a single thread, around the loops that share out rows: the threads of a nested
-    // region are made for it and end with it, 0.6 ms each time; and none inside the loops over many WLBs: 0.4 us each, more when
-    // all threads start them)
-    if (by_rows)
-        for (u64 w = 0; w < NW; w++) count_wlb(w);
-    else
-    {
-#pragma omp parallel for schedule(static) if (b.col.size() > kParallelNnz)
-        for (u64 w = 0; w < NW; w++) count_wlb(w);
-    }
+    const bool by_wlbs = !by_rows && b.col.size() > kParallelNnz;
+    for_each(NW, by_wlbs, count_wlb);
     u64 max_S = 0;
     for (u64 w = 0; w < NW; w++)
     {
@@ -768,11 +750,11 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
     b.pad_val.es = es;
     uint8_t *pval = b.pad_val.b.make(n_pad * es);
     u32 *trow = tlb_rows ? b.tlb_row.make(n_tlb) : nullptr;
-    u64 max_thread_first_row = 0;
-    bool share_thread = tlb_size != 0;
+    std::atomic<u64> top_of_all(0);
+    std::atomic<bool> shared(tlb_size != 0);
     // pass 2: fill the padded arrays (row-major inside the WLB) and the per-TLB first rows
     // `f`: first TLB of every row of the WLB, relative to it
-    auto fill_wlb = [&](u64 w, u64 *f, u64 &top_of_all, bool &shared) {
+    auto fill_wlb = [&](u64 w, u64 *f) {
         const Span s = span(w);
         const u64 S = wlb_S[w], extra = wlb_tlb0[w + 1] - wlb_tlb0[w] - wlb_tl[w];
         f[0] = 0;
@@ -782,8 +764,6 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
             f[r + 1] = (row_range(s, r, lo, hi) + S - 1) / S + (extra > r ? (extra - r - 1) / s.rows + 1 : 0);
         });
         for (u64 r = 0; r < s.rows; r++) f[r + 1] += f[r];
-        u64 top = 0;
-        bool shared_row = false;
         auto fill_row = [&](u64 r, u64 &top_out, bool &shared_out) {
             u64 lo, hi;
             const u64 n = row_range(s, r, lo, hi), tlbs = f[r + 1] - f[r], tgt = tlbs * S, out = wlb_pad0[w] + f[r] * S;
@@ -801,32 +781,25 @@ void sep_thread_level_col_ell_with_padding(CompressedBlock &b, u64 tlb_size, boo
                 for (u64 k = 0; k < tlbs; k++) trow[wlb_tlb0[w] + f[r] + k] = (u32)r;
             if (tlbs > 0) top_out = std::max(top_out, r);
         };
-        if (by_rows && (wlb_pad0[w + 1] - wlb_pad0[w]) * es > kParallelBytes)
-        {
-#pragma omp parallel for schedule(static) reduction(max : top) reduction(|| : shared_row)
-            for (u64 r = 0; r < s.rows; r++) fill_row(r, top, shared_row);
-        }
-        else
-            for (u64 r = 0; r < s.rows; r++) fill_row(r, top, shared_row);
-        shared = shared || shared_row;
-        top_of_all = std::max(top_of_all, top);
+        share_ranges(s.rows, by_rows && (wlb_pad0[w + 1] - wlb_pad0[w]) * es > kParallelBytes, [&](u64 r, u64 e) {
+            u64 top = 0;
+            bool shared_row = false;
+            for (; r < e; r++) fill_row(r, top, shared_row);
+            raise(top_of_all, top);
+            if (shared_row && !shared.load(std::memory_order_relaxed)) shared.store(true, std::memory_order_relaxed); // (one line, all threads)
+        });
     };
     u64 most_rows = 0;
     for (u64 w = 0; w < NW; w++) most_rows = std::max(most_rows, W.row_num.v[w]);
     const u64 stride = (most_rows + 1 + 15) / 8 * 8; // (cache lines of a thread's own)
-    if (by_rows)
-    {
-        std::vector<u64> first(stride);
-        for (u64 w = 0; w < NW; w++) fill_wlb(w, first.data(), max_thread_first_row, share_thread);
-    }
-    else
-    {
-        // (allocated before the region: an exception that leaves one ends the process)
-        const bool share = b.col.size() > kParallelNnz;
-        std::vector<u64> first(stride * (share ? (u64)omp_get_max_threads() : 1));
-#pragma omp parallel for schedule(static) reduction(max : max_thread_first_row) reduction(|| : share_thread) if (share)
-        for (u64 w = 0; w < NW; w++) fill_wlb(w, first.data() + stride * (u64)omp_get_thread_num(), max_thread_first_row, share_thread);
-    }
+    // (allocated before the loop: an exception that leaves a piece ends the process)
+    const unsigned width = by_wlbs ? crew_width() : 1;
+    std::vector<u64> first(stride * width);
+    share_steps(NW, std::max<u64>(1, NW / (8 * (u64)width)), width, [&](u64 w, u64 e, unsigned who) {
+        for (; w < e; w++) fill_wlb(w, first.data() + stride * who);
+    });
+    const u64 max_thread_first_row = top_of_all.load(std::memory_order_relaxed);
+    const bool share_thread = shared.load(std::memory_order_relaxed);
     u64 max_w_coo_begin = 0, max_w_size = 0;
     std::vector<u64> new_w_begin(NW), new_w_size(NW);
     for (u64 i = 0; i < B.block_num; i++)

@@ -252,16 +252,16 @@ static asp_status make_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t 
     if (val_dtype != ASP_F32 && val_dtype != ASP_F64) return hfail(ASP_ERR_UNSUPPORTED, "values must be f32 or f64");
     if (n_rows == 0 || n_cols == 0 || n_cols > 0xffffffffull) return hfail(ASP_ERR_INVALID_ARG, "bad shape");
     if (indptr[0] != 0) return hfail(ASP_ERR_INVALID_ARG, "indptr[0] != 0");
+    const Caller caller;
     // the first row with a fault, and which of the faults below it is
-    uint64_t bad_row = n_rows;
-#pragma omp parallel for schedule(static) reduction(min : bad_row) if (n_rows > kParallelRows)
-    for (int64_t r = 0; r < (int64_t)n_rows; r++)
-        if (indptr[r + 1] < indptr[r]) bad_row = std::min<uint64_t>(bad_row, (uint64_t)r);
-    if (bad_row == n_rows) // (rows are only looked into once the offsets are known to be in order)
+    std::atomic<uint64_t> first_bad(n_rows);
+    share_ranges(n_rows, n_rows > kParallelRows, [&](uint64_t r, uint64_t e) {
+        while (r < e && indptr[r + 1] >= indptr[r]) r++;
+        if (r < e) lower(first_bad, r);
+    });
+    if (first_bad.load(std::memory_order_relaxed) == n_rows) // (rows are only looked into once the offsets are known to be in order)
     {
-#pragma omp parallel for schedule(dynamic, 256) reduction(min : bad_row) if ((uint64_t)indptr[n_rows] > kParallelNnz)
-        for (int64_t r = 0; r < (int64_t)n_rows; r++)
-        {
+        auto good = [=](uint64_t r) {
             bool bad = false;
             uint32_t prev = 0;
             for (int64_t k = indptr[r]; k < indptr[r + 1]; k++)
@@ -269,9 +269,14 @@ static asp_status make_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t 
                 bad |= indices[k] >= n_cols || indices[k] < prev;
                 prev = indices[k];
             }
-            if (bad) bad_row = std::min<uint64_t>(bad_row, (uint64_t)r);
-        }
+            return !bad;
+        };
+        share_steps(n_rows, 256, (uint64_t)indptr[n_rows] > kParallelNnz ? crew_width() : 1, [&](uint64_t r, uint64_t e, unsigned) {
+            while (r < e && good(r)) r++;
+            if (r < e) lower(first_bad, r);
+        });
     }
+    const uint64_t bad_row = first_bad.load(std::memory_order_relaxed);
     if (bad_row < n_rows)
     {
         if (indptr[bad_row + 1] < indptr[bad_row]) return hfail(ASP_ERR_INVALID_ARG, "indptr decreases");
@@ -383,6 +388,7 @@ uint64_t asp_matrix_nnz(const asp_matrix *m) { return m ? m->m->nnz : 0; }
 
 asp_status asp_dense_execute(const asp_matrix *in, const char *spec, asp_matrix **out)
 {
+    const Caller caller;
     if (!in || !spec || !out) return hfail(ASP_ERR_INVALID_ARG, "NULL argument");
     *out = nullptr;
     if (in->m->is_compressed) return hfail(ASP_ERR_INVALID_ARG, "matrix is already compressed");
@@ -426,14 +432,19 @@ asp_status asp_matrix_sub_rows(const asp_matrix *m, int sub, uint64_t *n_rows, u
 {
     if (!m || !m->m->is_compressed || sub < 0 || sub >= (int)m->m->blocks.size()) return hfail(ASP_ERR_INVALID_ARG, "bad sub-matrix id");
     const CompressedBlock &b = m->m->blocks[sub];
-    u64 mn = ~0ull, mx = 0;
-#pragma omp parallel for schedule(static) reduction(min : mn) reduction(max : mx) if (b.n_rows > kParallelRows)
-    for (u64 r = 0; r < b.n_rows; r++)
-    {
-        const u64 l = b.rowptr[r + 1] - b.rowptr[r];
-        mn = std::min(mn, l);
-        mx = std::max(mx, l);
-    }
+    std::atomic<u64> shortest(~0ull), longest(0);
+    share_ranges(b.n_rows, b.n_rows > kParallelRows, [&](u64 r, u64 e) {
+        u64 mn = ~0ull, mx = 0;
+        for (; r < e; r++)
+        {
+            const u64 l = b.rowptr[r + 1] - b.rowptr[r];
+            mn = std::min(mn, l);
+            mx = std::max(mx, l);
+        }
+        lower(shortest, mn);
+        raise(longest, mx);
+    });
+    const u64 mn = shortest.load(std::memory_order_relaxed), mx = longest.load(std::memory_order_relaxed);
     if (n_rows) *n_rows = b.n_rows;
     if (nnz) *nnz = b.col.size();
     if (min_row_nnz) *min_row_nnz = mn;
@@ -443,6 +454,7 @@ asp_status asp_matrix_sub_rows(const asp_matrix *m, int sub, uint64_t *n_rows, u
 
 asp_status asp_graph_execute(const asp_matrix *in, const char *spec, asp_format **out)
 {
+    const Caller caller;
     if (!in || !spec || !out) return hfail(ASP_ERR_INVALID_ARG, "NULL argument");
     *out = nullptr;
     std::vector<std::vector<std::string>> dense_ops;

@@ -17,6 +17,8 @@
 #include <new>
 #include <vector>
 
+#include "crew.hpp"
+
 namespace asp
 {
 namespace host
@@ -80,50 +82,20 @@ class IdleBlocks
 std::shared_ptr<void> big_buffer(size_t bytes);
 void host_pool_trim();
 
-// Below these a loop runs on the calling thread. A parallel region waits for its slowest thread, and where other programs keep the cores
-// busy that is one that is not running: 8 cores, a spinning process on each, rows of 8, built with 256 KB, 2^13 rows and 2^14 non-zeros
-// here / with these: 28,800 non-zeros 16-24 ms / 0.2-0.8 ms, 96,000 56-120 / 0.6-3.6, 400,000 64-168 / 2.3-23. Four threads that build at once:
-// 29,000 non-zeros 126-160 / 72-85 us a build, 96,000 260-476 / 163-211. A host that has nothing else to do gains from lower limits (16 cores,
-// 3 x 3 blocks: 28,000 non-zeros 168 -> 105 us, 414,000 1480 -> 230-300), but that cannot be told beforehand. They also are the size up to which a
-// forked process may build after its parent has: the threads of a region do not come along.
-const size_t kParallelBytes = 4u << 20;
-const uint64_t kParallelRows = 1u << 18, kParallelNnz = 1u << 19;
-// f(i) for i in [0, n), shared out among the threads or without a parallel region at all (an inactive one costs 0.4 us, too much
-// for what is done per block)
-template <class F>
-void for_each(uint64_t n, bool share, F &&f)
-{
-    if (share)
-    {
-#pragma omp parallel for schedule(static)
-        for (uint64_t i = 0; i < n; i++) f(i);
-    }
-    else
-        for (uint64_t i = 0; i < n; i++) f(i);
-}
-
+// Below these a loop runs on the calling thread alone: sharing one costs 1 to 5 us. (The limits were 4 MB, 2^18 rows and 2^19 non-zeros
+// while loops were OpenMP's; crew.cpp has the figures of both.)
+const size_t kParallelBytes = 1u << 18;
+const uint64_t kParallelRows = 1u << 13, kParallelNnz = 1u << 14;
 inline void par_copy(void *dst, const void *src, size_t bytes)
 {
-    const size_t piece = 1u << 16;
-    const long long n = (long long)((bytes + piece - 1) / piece);
-#pragma omp parallel for schedule(static) if (bytes > kParallelBytes)
-    for (long long i = 0; i < n; i++)
-    {
-        const size_t o = (size_t)i * piece;
-        memcpy((char *)dst + o, (const char *)src + o, o + piece <= bytes ? piece : bytes - o);
-    }
+    share_ranges((bytes + 63) / 64, bytes > kParallelBytes, [=](uint64_t i, uint64_t e) {
+        memcpy((char *)dst + i * 64, (const char *)src + i * 64, std::min<size_t>(bytes, e * 64) - i * 64);
+    });
 }
 
 inline void par_zero(void *dst, size_t bytes)
 {
-    const size_t piece = 1u << 16;
-    const long long n = (long long)((bytes + piece - 1) / piece);
-#pragma omp parallel for schedule(static) if (bytes > kParallelBytes)
-    for (long long i = 0; i < n; i++)
-    {
-        const size_t o = (size_t)i * piece;
-        memset((char *)dst + o, 0, o + piece <= bytes ? piece : bytes - o);
-    }
+    share_ranges((bytes + 63) / 64, bytes > kParallelBytes, [=](uint64_t i, uint64_t e) { memset((char *)dst + i * 64, 0, std::min<size_t>(bytes, e * 64) - i * 64); });
 }
 
 template <class T>

@@ -26,17 +26,22 @@ bool all_of(u64 n, F &&f)
     const u64 head = std::min<u64>(n, 1u << 16);
     for (u64 i = 0; i < head; i++)
         if (!f(i)) return false;
-    bool ok = true;
-#pragma omp parallel for schedule(static) reduction(&& : ok) if (n > kParallelRows)
-    for (u64 i = head; i < n; i++) ok = ok && f(i);
-    return ok;
+    std::atomic<bool> ok(true);
+    share_ranges(n - head, n > kParallelRows, [&](u64 i, u64 e) {
+        for (i += head, e += head; i < e && f(i);) i++;
+        if (i < e) ok.store(false, std::memory_order_relaxed);
+    });
+    return ok.load(std::memory_order_relaxed);
 }
 u64 max_entry(U64s a)
 {
-    u64 mx = 0;
-#pragma omp parallel for schedule(static) reduction(max : mx) if (a.n > kParallelRows)
-    for (u64 i = 0; i < a.n; i++) mx = std::max(mx, a[i]);
-    return mx;
+    std::atomic<u64> all(0);
+    share_ranges(a.n, a.n > kParallelRows, [&](u64 i, u64 e) {
+        u64 mx = 0;
+        for (; i < e; i++) mx = std::max(mx, a[i]);
+        raise(all, mx);
+    });
+    return all.load(std::memory_order_relaxed);
 }
 } // namespace
 
@@ -135,8 +140,7 @@ Arr<uint8_t> narrow_to(U64s v)
 {
     Arr<uint8_t> out;
     T *p = (T *)out.make(v.size() * sizeof(T));
-#pragma omp parallel for schedule(static) if (v.n > kParallelRows)
-    for (u64 i = 0; i < v.n; i++) p[i] = (T)v[i];
+    for_each(v.n, v.n > kParallelRows, [=](u64 i) { p[i] = (T)v[i]; });
     return out;
 }
 Arr<uint8_t> narrow(U64s v, int dt)
@@ -221,11 +225,10 @@ Arr<u64> tlb_global_rows(const CompressedBlock &b, bool &adjacent_equal)
             for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w, true);
     }
     else
-    {
-#pragma omp parallel for schedule(dynamic, 4) if (T.block_num > kParallelRows)
-        for (u64 i = 0; i < B.block_num; i++)
-            for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w, false);
-    }
+        share_steps(B.block_num, 4, T.block_num > kParallelRows ? crew_width() : 1, [&](u64 i, u64 e, unsigned) {
+            for (; i < e; i++)
+                for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w, false);
+        });
     adjacent_equal = T.block_num > 1 && !all_of(T.block_num - 1, [&](u64 t) { return rows[t] != rows[t + 1]; });
     return out;
 }
@@ -237,9 +240,9 @@ std::vector<u64> row_offsets(U64s rows, u64 n_rows)
     if (rows.size() > 1 && all_of(rows.size() - 1, [&](u64 t) { return rows[t] <= rows[t + 1]; }))
     {
         // ascending rows: out[r] is the first TLB whose row is not below r
-#pragma omp parallel for schedule(static) if (rows.n > kParallelRows)
-        for (u64 t = 0; t < rows.n; t++)
+        for_each(rows.n, rows.n > kParallelRows, [&](u64 t) {
             for (u64 r = t == 0 ? 0 : rows[t - 1] + 1; r <= rows[t]; r++) out[r] = t;
+        });
         for (u64 r = rows.back() + 1; r <= n_rows; r++) out[r] = rows.n;
         return out;
     }
@@ -282,18 +285,14 @@ void add_perm(const Matrix &m, TemplateData &t)
 u64 effective_and_permute(const Matrix &m, const CompressedBlock &b, u64 *rows, u64 n)
 {
     const u64 dense_rows = b.max_row - b.min_row + 1;
-    u64 eff = n;
+    std::atomic<u64> first(n);
     if (b.n_rows > dense_rows)
-    {
-#pragma omp parallel for schedule(static) reduction(min : eff) if (n > kParallelRows)
-        for (u64 i = 0; i < n; i++)
-            if (rows[i] >= dense_rows) eff = std::min(eff, i);
-    }
-    if (m.is_sorted)
-    {
-#pragma omp parallel for schedule(static) if (eff > kParallelRows)
-        for (u64 i = 0; i < eff; i++) rows[i] = m.perm[rows[i] + b.min_row];
-    }
+        share_ranges(n, n > kParallelRows, [&](u64 i, u64 e) {
+            while (i < e && rows[i] < dense_rows) i++;
+            if (i < e) lower(first, i);
+        });
+    const u64 eff = first.load(std::memory_order_relaxed);
+    if (m.is_sorted) for_each(eff, eff > kParallelRows, [&](u64 i) { rows[i] = m.perm[rows[i] + b.min_row]; });
     return eff;
 }
 
@@ -357,13 +356,14 @@ void interleave_per_blb(const CompressedBlock &b, const std::vector<u64> &thr, c
     const int cb = dtype_bytes(b.col_dt), es = b.val.es;
     uint8_t *cp = col.make(n_pad * cb), *vp = val.make(n_pad * es);
     const u64 nb = b.blb.block_num;
-#pragma omp parallel for schedule(dynamic, 4) if (n_pad > kParallelNnz)
-    for (u64 i = 0; i < nb; i++)
-    {
+    auto of_blb = [&](u64 i) {
         const u64 nz0 = b.blb.coo_begin.v[i], n = thr[i + 1] - thr[i];
         interleave_cols(cp + nz0 * cb, b.col_dt, b.pad_col.data() + nz0, n, size[i]);
         interleave_vals(vp + nz0 * es, es, b.pad_val.b.data() + nz0 * es, n, size[i]);
-    }
+    };
+    share_steps(nb, 4, n_pad > kParallelNnz ? crew_width() : 1, [&](u64 i, u64 e, unsigned) {
+        for (; i < e; i++) of_blb(i);
+    });
 }
 
 // ---- DIRECT_ATOM_TEMPLATE_WARP_COMPRESS (direct_atom_op_warp_compress.cc) --------------------
@@ -473,11 +473,10 @@ void staggered_arrays(const CompressedBlock &b, Arr<uint8_t> &col, Arr<uint8_t> 
             for_each(w1 - w0, w1 - w0 > 1024, [&](u64 w) { of_wlb(i, w0 + w); });
         }
     else
-    {
-#pragma omp parallel for schedule(dynamic, 4) if (n_pad > kParallelNnz)
-        for (u64 i = 0; i < nb; i++)
-            for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w);
-    }
+        share_steps(nb, 4, n_pad > kParallelNnz ? crew_width() : 1, [&](u64 i, u64 e, unsigned) {
+            for (; i < e; i++)
+                for (u64 w = B.index.v[i]; w < B.index.v[i + 1]; w++) of_wlb(i, w);
+        });
 }
 
 std::vector<u64> first_n(const std::vector<u64> &v, u64 n) { return std::vector<u64>(v.begin(), v.begin() + n); }
@@ -745,11 +744,10 @@ bool init_k9(const Matrix &m, const CompressedBlock &b, bool with_warp_reduce, T
     Arr<u32> frow_arr;
     u32 *const frow = frow_arr.make(T);
     std::vector<u64> wfirst(Wn);
-    u64 max_frow = 0;
-#pragma omp parallel for schedule(static) reduction(max : max_frow) if (n > kParallelNnz)
-    for (u64 w = 0; w < Wn; w++)
-    {
+    std::atomic<u64> most_frow(0);
+    const auto fill = [&, cp, vp, flags, frow, first, S, R, wn, cb, es, last_row, rowptr = b.rowptr.data(), bcol = b.col.data(), src = b.val.b.data()](u64 w) ASP_INLINE {
         const u64 e0 = w * wn, e1 = e0 + wn;
+        u64 top = 0;
         u64 r = std::min<u64>((u64)(std::upper_bound(first, first + R + 1, e0) - first) - 1, last_row);
         wfirst[w] = r;
         for (u64 tl = w * 32; tl < w * 32 + 32; tl++) flags[tl] = 0;
@@ -757,7 +755,7 @@ bool init_k9(const Matrix &m, const CompressedBlock &b, bool with_warp_reduce, T
         while (e < e1)
         {
             const u64 end = r < last_row ? std::min(e1, first[r + 1]) : e1; // fillers continue the last row
-            const u64 nz0 = b.rowptr[r], nz = b.rowptr[r + 1] - nz0;
+            const u64 nz0 = rowptr[r], nz = rowptr[r + 1] - nz0;
             if (e == e0 || e == first[r])
             {
                 const u64 tl = w * 32 + lane;
@@ -768,7 +766,7 @@ bool init_k9(const Matrix &m, const CompressedBlock &b, bool with_warp_reduce, T
             {
                 const u64 q = e - first[r], d = e0 + k * 32 + lane;
                 if (++k == S) k = 0, lane++;
-                const u32 c = nz == 0 ? 0 : b.col[nz0 + std::min(q, nz - 1)];
+                const u32 c = nz == 0 ? 0 : bcol[nz0 + std::min(q, nz - 1)];
                 switch (cb)
                 {
                 case 1: cp[d] = (uint8_t)c; break;
@@ -776,17 +774,25 @@ bool init_k9(const Matrix &m, const CompressedBlock &b, bool with_warp_reduce, T
                 case 4: ((u32 *)cp)[d] = c; break;
                 default: ((u64 *)cp)[d] = c; break;
                 }
-                if (es == 8) ((u64 *)vp)[d] = q < nz ? ((const u64 *)b.val.b.data())[nz0 + q] : 0;
-                else ((u32 *)vp)[d] = q < nz ? ((const u32 *)b.val.b.data())[nz0 + q] : 0;
+                if (es == 8) ((u64 *)vp)[d] = q < nz ? ((const u64 *)src)[nz0 + q] : 0;
+                else ((u32 *)vp)[d] = q < nz ? ((const u32 *)src)[nz0 + q] : 0;
             }
             r++;
         }
         for (u64 tl = w * 32; tl < w * 32 + 32; tl++)
         {
             if (flags[tl] == 0) frow[tl] = frow[tl - 1]; // (the warp's first TLB always has a flag)
-            max_frow = std::max<u64>(max_frow, frow[tl]);
+            top = std::max<u64>(top, frow[tl]);
         }
-    }
+        return top;
+    };
+    share_ranges(Wn, n > kParallelNnz, [&](u64 w, u64 e) {
+        const auto mine = fill; // (what it holds by value, in this thread's registers)
+        u64 top = 0;
+        for (; w < e; w++) top = std::max(top, mine(w));
+        raise(most_frow, top);
+    });
+    const u64 max_frow = most_frow.load(std::memory_order_relaxed);
     // per TLB with a row start: the number of following TLBs without one
     std::vector<u32> roff(T, 0);
     u64 max_roff = 0, last_head = 0;
@@ -809,8 +815,7 @@ bool init_k9(const Matrix &m, const CompressedBlock &b, bool with_warp_reduce, T
     const int word = total_bits <= 8 ? 8 : total_bits <= 16 ? 16 : total_bits <= 32 ? 32 : 64;
     const int meta_dt = word == 8 ? ASP_U8 : word == 16 ? ASP_U16 : word == 32 ? ASP_U32 : ASP_U64;
     u64 *const meta = flags; // (in place)
-#pragma omp parallel for schedule(static) if (T > kParallelRows)
-    for (u64 tl = 0; tl < T; tl++) meta[tl] = (((flags[tl] << (word - (int)S - bits_row)) | roff[tl]) << bits_row) | frow[tl];
+    for_each(T, T > kParallelRows, [&](u64 tl) { meta[tl] = (((flags[tl] << (word - (int)S - bits_row)) | roff[tl]) << bits_row) | frow[tl]; });
     t.tlb_size = S;
     t.bits_word = word;
     t.bits_flag = (int)S;
@@ -834,17 +839,15 @@ namespace
 template <int R>
 u64 block_columns(const CompressedBlock &b, u32 *const bcol, std::vector<u32> &cnt)
 {
-    u64 W = 0;
-#pragma omp parallel for schedule(static) reduction(max : W) if (b.nnz() > kParallelNnz)
-    for (int64_t br = 0; br < (int64_t)cnt.size(); br++)
-    {
-        const u64 row0 = (u64)br * R, row1 = std::min<u64>(b.n_rows, row0 + R), nz0 = b.rowptr[row0];
+    std::atomic<u64> W(0);
+    const auto merge = [&, rowptr = b.rowptr.data(), col = b.col.data()](u64 br) ASP_INLINE {
+        const u64 row0 = br * R, row1 = std::min<u64>(b.n_rows, row0 + R), nz0 = rowptr[row0];
         u32 *const o = bcol + nz0;
         // the columns of a row ascend: its block columns come out in order; further rows usually repeat them
         u64 n = 0;
-        for (u64 k = nz0; k < b.rowptr[row0 + 1]; k++)
+        for (u64 k = nz0; k < rowptr[row0 + 1]; k++)
         {
-            const u32 c0 = b.col[k] / (u32)R;
+            const u32 c0 = col[k] / (u32)R;
             if (n == 0 || o[n - 1] != c0) o[n++] = c0;
         }
         bool merged = false;
@@ -852,9 +855,9 @@ u64 block_columns(const CompressedBlock &b, u32 *const bcol, std::vector<u32> &c
         {
             u64 q = 0;
             const u64 sorted = n;
-            for (u64 k = b.rowptr[row]; k < b.rowptr[row + 1]; k++)
+            for (u64 k = rowptr[row]; k < rowptr[row + 1]; k++)
             {
-                const u32 c0 = b.col[k] / (u32)R;
+                const u32 c0 = col[k] / (u32)R;
                 if (merged)
                 {
                     o[n++] = c0; // (at most one entry per non-zero: it stays inside the block row's share)
@@ -872,39 +875,47 @@ u64 block_columns(const CompressedBlock &b, u32 *const bcol, std::vector<u32> &c
             n = (u64)(std::unique(o, o + n) - o);
         }
         cnt[br] = (u32)n;
-        W = std::max(W, n);
-    }
-    return W;
+        return n;
+    };
+    share_ranges(cnt.size(), b.nnz() > kParallelNnz, [&](u64 br, u64 e) {
+        const auto mine = merge;
+        u64 most = 0;
+        for (; br < e; br++) most = std::max(most, mine(br));
+        raise(W, most);
+    });
+    return W.load(std::memory_order_relaxed);
 }
 
-// the arrays: block columns ip[slot * NB + block row], values vp[((slot * R + i) * R + j) * NB + block row]
+// the arrays of block rows [br, e): block columns ip[slot * NB + block row], values vp[((slot * R + i) * R + j) * NB + block row]
 template <int R, class V>
-void block_values(const CompressedBlock &b, const u32 *const bcol, const std::vector<u32> &cnt, u64 W, u64 NB, u32 *const ip, V *const vp)
+void block_values(const CompressedBlock &b, const u32 *const bcol, const u32 *const cnt, u64 W, u64 NB, u32 *const ip, V *const vp, u64 br, u64 e)
 {
     const V *const src = (const V *)b.val.b.data();
-#pragma omp parallel for schedule(static) if (b.nnz() > kParallelNnz)
-    for (int64_t br = 0; br < (int64_t)cnt.size(); br++)
+    const u64 n_rows = b.n_rows;
+    const u32 *const col = b.col.data();
+    const u64 *const rowptr = b.rowptr.data();
+    for (; br < e; br++)
     {
         const u64 n = cnt[br];
-        const u32 *bc = bcol + b.rowptr[(u64)br * R];
+        const u32 *bc = bcol + rowptr[br * R];
         for (u64 k = 0; k < W; k++) ip[k * NB + br] = k < n ? bc[k] : (n ? bc[n - 1] : 0); // zero blocks repeat the last block column
         // a block row of full blocks is overwritten whole (no column twice: entries are as many as there are places)
-        const u64 q0 = b.rowptr[(u64)br * R], q1 = b.rowptr[std::min<u64>(b.n_rows, ((u64)br + 1) * R)];
-        bool full = q1 - q0 == W * R * R && ((u64)br + 1) * R <= b.n_rows;
-        for (u64 row = (u64)br * R; full && row < ((u64)br + 1) * R; row++)
-            for (u64 q = b.rowptr[row] + 1; q < b.rowptr[row + 1]; q++) full = full && b.col[q] != b.col[q - 1];
+        const u64 q0 = rowptr[br * R], q1 = rowptr[std::min<u64>(n_rows, (br + 1) * R)];
+        bool full = q1 - q0 == W * R * R && (br + 1) * R <= n_rows;
+        for (u64 row = br * R; full && row < (br + 1) * R; row++)
+            for (u64 q = rowptr[row] + 1; q < rowptr[row + 1]; q++) full = full && col[q] != col[q - 1];
         if (!full)
-            for (u64 q = 0; q < W * R * R; q++) vp[q * NB + (u64)br] = 0;
-        for (u64 row = (u64)br * R; row < std::min<u64>(b.n_rows, ((u64)br + 1) * R); row++)
+            for (u64 q = 0; q < W * R * R; q++) vp[q * NB + br] = 0;
+        for (u64 row = br * R; row < std::min<u64>(n_rows, (br + 1) * R); row++)
         {
-            const u64 i = row - (u64)br * R;
+            const u64 i = row - br * R;
             u64 k = 0; // the columns of a row ascend, so do its block slots
-            for (u64 q = b.rowptr[row]; q < b.rowptr[row + 1]; q++)
+            for (u64 q = rowptr[row]; q < rowptr[row + 1]; q++)
             {
-                const u32 cb = b.col[q] / (u32)R;
+                const u32 cb = col[q] / (u32)R;
                 while (bc[k] != cb) k++;
-                const u64 j = b.col[q] - (u64)cb * R;
-                vp[((k * R + i) * R + j) * NB + (u64)br] = src[q];
+                const u64 j = col[q] - (u64)cb * R;
+                vp[((k * R + i) * R + j) * NB + br] = src[q];
             }
         }
     }
@@ -935,15 +946,18 @@ bool init_block_ell(const Matrix &m, const CompressedBlock &b, TemplateData &t, 
     u32 *const ip = (u32 *)idx.make_zero(NB * W * 4);
     uint8_t *const vp = val.make(stored * (u64)es);
     for (u64 q = 0; NB > NBR && q < W * r * c; q++) memset(vp + (q * NB + NBR) * es, 0, es); // the block row that pads
-    if (es == 8)
-    {
-        if (r == 3) block_values<3>(b, bcol, cnt, W, NB, ip, (u64 *)vp);
-        else if (r == 2) block_values<2>(b, bcol, cnt, W, NB, ip, (u64 *)vp);
-        else block_values<4>(b, bcol, cnt, W, NB, ip, (u64 *)vp);
-    }
-    else if (r == 3) block_values<3>(b, bcol, cnt, W, NB, ip, (u32 *)vp);
-    else if (r == 2) block_values<2>(b, bcol, cnt, W, NB, ip, (u32 *)vp);
-    else block_values<4>(b, bcol, cnt, W, NB, ip, (u32 *)vp);
+    const u32 *const counts = cnt.data();
+    share_ranges(NBR, b.nnz() > kParallelNnz, [&](u64 br, u64 e) {
+        if (es == 8)
+        {
+            if (r == 3) block_values<3>(b, bcol, counts, W, NB, ip, (u64 *)vp, br, e);
+            else if (r == 2) block_values<2>(b, bcol, counts, W, NB, ip, (u64 *)vp, br, e);
+            else block_values<4>(b, bcol, counts, W, NB, ip, (u64 *)vp, br, e);
+        }
+        else if (r == 3) block_values<3>(b, bcol, counts, W, NB, ip, (u32 *)vp, br, e);
+        else if (r == 2) block_values<2>(b, bcol, counts, W, NB, ip, (u32 *)vp, br, e);
+        else block_values<4>(b, bcol, counts, W, NB, ip, (u32 *)vp, br, e);
+    });
     common_head(m, b, ASP_BLOCK_ELL_TEMPLATE, t);
     t.tlb_size = W;
     t.bits_row = (int)r;
@@ -981,17 +995,15 @@ bool init_diag(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::
     // distinct offsets, as bits of all there could be; a scattered matrix leaves after a few rows
     std::vector<u64> bits((b.n_rows + (u64)ncols) / 64 + 1, 0);
     u64 found = 0;
-#pragma omp parallel for schedule(static) if (b.nnz() > kParallelNnz)
-    for (u64 r = 0; r < b.n_rows; r++)
-    {
-        if (__atomic_load_n(&found, __ATOMIC_RELAXED) > b.diag_max) continue;
+    for_each(b.n_rows, b.nnz() > kParallelNnz, [&](u64 r) {
+        if (__atomic_load_n(&found, __ATOMIC_RELAXED) > b.diag_max) return;
         for (u64 k = b.rowptr[r]; k < b.rowptr[r + 1]; k++)
         {
             const u64 at = b.col[k] + b.n_rows - r, bit = 1ull << (at % 64);
             if (__atomic_load_n(&bits[at / 64], __ATOMIC_RELAXED) & bit) continue;
             if ((__atomic_fetch_or(&bits[at / 64], bit, __ATOMIC_RELAXED) & bit) == 0) __atomic_fetch_add(&found, 1, __ATOMIC_RELAXED);
         }
-    }
+    });
     if (found > b.diag_max) return err = "diag_value: more than " + std::to_string(b.diag_max) + " diagonals hold non-zeros", false;
     if (found == 0) return err = "diag_value: sub-matrix without non-zeros", false;
     std::vector<int64_t> off; // ascending
@@ -1000,13 +1012,13 @@ bool init_diag(const Matrix &m, const CompressedBlock &b, TemplateData &t, std::
     const u64 D = off.size();
     Arr<uint8_t> val;
     uint8_t *const vp = val.make_zero(D * NR * (u64)es);
-#pragma omp parallel for schedule(static) if (b.nnz() > kParallelNnz)
-    for (int64_t r = 0; r < (int64_t)b.n_rows; r++)
+    for_each(b.n_rows, b.nnz() > kParallelNnz, [&](u64 r) {
         for (u64 k = b.rowptr[r]; k < b.rowptr[r + 1]; k++)
         {
-            const u64 d = (u64)(std::lower_bound(off.begin(), off.end(), (int64_t)b.col[k] - r) - off.begin());
-            memcpy(&vp[(d * NR + (u64)r) * es], &b.val.b[k * es], es);
+            const u64 d = (u64)(std::lower_bound(off.begin(), off.end(), (int64_t)b.col[k] - (int64_t)r) - off.begin());
+            memcpy(&vp[(d * NR + r) * es], &b.val.b[k * es], es);
         }
+    });
     common_head(m, b, ASP_DIAG_TEMPLATE, t);
     t.tlb_size = D;
     t.effective_num = b.n_rows;

@@ -7,14 +7,8 @@
 #include <algorithm>
 #include <cmath>
 
-#ifdef _OPENMP
-#include <omp.h>
-#endif
-
 #include "../tiled.h"
-
-// per element, in every template's loop of walk(): as calls (what the compiler makes of the seventh use) a third slower
-#define ASP_INLINE __attribute__((always_inline))
+#include "crew.hpp"
 
 namespace asp
 {
@@ -23,30 +17,19 @@ namespace
 typedef uint64_t u64;
 typedef uint32_t u32;
 
-// (What the threads of a parallel region work in is allocated before it: an exception that leaves a region ends the process.)
-int threads()
-{
-#ifdef _OPENMP
-    return omp_get_max_threads();
-#else
-    return 1;
-#endif
-}
-int this_thread()
-{
-#ifdef _OPENMP
-    return omp_get_thread_num();
-#else
-    return 0;
-#endif
-}
+using host::for_each;
+using host::share_pieces;
+using host::share_ranges;
+using host::share_steps;
+
+// (What the threads of a shared loop work in is allocated before it: an exception that leaves a piece ends the process.)
 // counters of every thread, on cache lines of their own
 struct ThreadCounters
 {
-    const u64 n, stride;
+    const u64 stride;
     std::vector<u64> all;
-    explicit ThreadCounters(u64 count) : n(count), stride((count + 15) / 8 * 8), all(stride * (u64)threads(), 0) {}
-    u64 *mine() { return all.data() + stride * (u64)this_thread(); }
+    ThreadCounters(u64 count, unsigned threads) : stride((count + 15) / 8 * 8), all(stride * threads, 0) {}
+    u64 *of(unsigned who) { return all.data() + stride * who; }
 };
 
 u64 row_in_y(const TiledSource &s, u64 r)
@@ -73,6 +56,7 @@ u64 unit_count(const TiledSource &s)
     }
 }
 
+// (ASP_INLINE per element, in every template's loop: as calls, which the compiler makes of the seventh use, a third slower.)
 // f(row of y, column of x, value) for every element that units [u0, u1) store. What a format adds to fill a TLB (a zero
 // that repeats the column before it in the same row) is left out.
 template <class VT, class CT, class F>
@@ -323,9 +307,7 @@ void share_out(int n_sm, u32 warps, const std::vector<u64> &begin, double tile_c
         for (u32 w = 0; w < warps; w++) link(&work[(place[i - 1] * warps + w) * 4], place[i]);
     }
     // (thousands of warps: half of the time of the build when it was done by one thread)
-#pragma omp parallel for schedule(static)
-    for (long long i = 0; i < (long long)visits.size(); i++)
-    {
+    for_each(visits.size(), true, [&](u64 i) {
         const Visit &v = visits[i];
         const double from = cost(v.s), all = cost(v.e) - from;
         u64 here = v.s;
@@ -335,7 +317,7 @@ void share_out(int n_sm, u32 warps, const std::vector<u64> &begin, double tile_c
             put(&work[(place[i] * warps + w) * 4], here, to, v.tile);
             here = to;
         }
-    }
+    });
 }
 
 struct Chunk
@@ -351,6 +333,7 @@ struct Builder
     const u64 n_rows, n_cols;
     static constexpr u32 TW = tiled_tile_cols(sizeof(VT) == 8);
     const u64 C; // tiles of x
+    const unsigned width = host::crew_width();
     const u64 warp_steps; // of a warp's share, about: longer pieces are cut, and every cut is one more part of their rows
     std::vector<Chunk> chunks;
     std::vector<u64> at; // [chunk * C + tile]: first its count, then where its elements go
@@ -373,7 +356,7 @@ struct Builder
     {
         u64 stored = 0;
         for (const TiledSource &s : src) stored += s.stored;
-        const u64 want = (u64)threads() * 4;
+        const u64 want = (u64)width * 4;
         for (size_t i = 0; i < src.size(); i++)
         {
             const u64 units = unit_count(src[i]), parts = std::max<u64>(1, std::min<u64>(units, want * src[i].stored / std::max<u64>(stored, 1)));
@@ -384,15 +367,13 @@ struct Builder
         row_code.assign(n_rows, 0);
         std::vector<u32> share;
         for (const TiledSource &s : src) share.push_back(share_of_part(s));
-        ThreadCounters pieces_of_thread(C), n_of_thread(C); // (neighbours in `at` share cache lines)
+        ThreadCounters pieces_of_thread(C, width), n_of_thread(C, width); // (neighbours in `at` share cache lines)
         const size_t edges = (2 * C + 31) / 16 * 16;
         std::vector<u32> edge(chunks.size() * edges); // rows of a chunk's first and last element in a tile, on cache lines of its own
-        u64 all_runs = 0, all_near = 0;
-#pragma omp parallel reduction(+ : all_runs, all_near)
-        {
-            u64 *const pieces = pieces_of_thread.mine(), *const n = n_of_thread.mine();
-#pragma omp for schedule(dynamic, 1)
-            for (long long c = 0; c < (long long)chunks.size(); c++)
+        std::atomic<u64> sum_runs(0), sum_near(0);
+        share_steps(chunks.size(), 1, width, [&](u64 c, u64, unsigned who) {
+            u64 *const pieces = pieces_of_thread.of(who), *const n = n_of_thread.of(who);
+            u64 all_runs = 0, all_near = 0;
             {
                 std::fill(n, n + C, 0);
                 u32 *const first = edge.data() + (size_t)c * edges, *const last = first + C;
@@ -432,11 +413,13 @@ struct Builder
                 row_ends();
                 std::copy(n, n + C, at.begin() + (size_t)c * C);
             }
-#pragma omp critical
-            for (u64 t = 0; t < C; t++) tile_pieces[t] += pieces[t];
-        }
-        runs = all_runs;
-        near_runs = all_near;
+            sum_runs.fetch_add(all_runs, std::memory_order_relaxed);
+            sum_near.fetch_add(all_near, std::memory_order_relaxed);
+        });
+        for (unsigned who = 0; who < width; who++)
+            for (u64 t = 0; t < C; t++) tile_pieces[t] += pieces_of_thread.of(who)[t];
+        runs = sum_runs.load(std::memory_order_relaxed);
+        near_runs = sum_near.load(std::memory_order_relaxed);
         tile_begin.assign(C + 1, 0);
         u64 sum = 0;
         for (u64 t = 0; t < C; t++)
@@ -464,17 +447,23 @@ struct Builder
     // which rows y takes itself and which have 64-bit sums
     void choose_sums(TiledHost &out)
     {
-        u64 missing = 0, direct = 0, shares = 0;
         // (a long row's pieces lie side by side in a tile and are summed in the warp before they are added: two parts a tile, as a rule,
         // twice as many where warps cut them)
         const u64 most = (warp_steps < kMaxPiece ? 4 : 2) * C * (kDirectShares / 8);
-#pragma omp parallel for schedule(static) reduction(+ : missing, direct, shares)
-        for (long long r = 0; r < (long long)n_rows; r++)
-        {
-            if (row_code[r] == 0) missing++;
-            else if (row_code[r] <= kDirectShares) direct++;
-            else shares += std::min<u64>(row_code[r], most);
-        }
+        std::atomic<u64> all_missing(0), all_direct(0), all_shares(0);
+        share_ranges(n_rows, true, [&](u64 r, u64 e) {
+            u64 missing = 0, direct = 0, shares = 0;
+            for (; r < e; r++)
+            {
+                if (row_code[r] == 0) missing++;
+                else if (row_code[r] <= kDirectShares) direct++;
+                else shares += std::min<u64>(row_code[r], most);
+            }
+            all_missing.fetch_add(missing, std::memory_order_relaxed);
+            all_direct.fetch_add(direct, std::memory_order_relaxed);
+            all_shares.fetch_add(shares, std::memory_order_relaxed);
+        });
+        const u64 missing = all_missing.load(std::memory_order_relaxed), direct = all_direct.load(std::memory_order_relaxed), shares = all_shares.load(std::memory_order_relaxed);
         const u64 rows = n_rows - missing - direct;
         out.covers_all_rows = missing == 0;
         // fp64: at most half of what may be added up directly goes to one sum of a row, on average
@@ -506,12 +495,9 @@ struct Builder
         e_row.make(N);
         e_col.make(N);
         e_val.make(N);
-        ThreadCounters to_of_thread(C);
-#pragma omp parallel
-        {
-            u64 *const to = to_of_thread.mine();
-#pragma omp for schedule(dynamic, 1)
-            for (long long c = 0; c < (long long)chunks.size(); c++)
+        ThreadCounters to_of_thread(C, width);
+        share_steps(chunks.size(), 1, width, [&](u64 c, u64, unsigned who) {
+            u64 *const to = to_of_thread.of(who);
             {
                 std::copy(at.begin() + (size_t)c * C, at.begin() + (size_t)(c + 1) * C, to);
                 walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) ASP_INLINE {
@@ -521,7 +507,7 @@ struct Builder
                     e_val.p[q] = v;
                 });
             }
-        }
+        });
     }
 
     struct Piece
@@ -582,20 +568,17 @@ struct Builder
             }
         }
         tile_block[C] = blocks.size();
-        const long long B = (long long)blocks.size();
+        const u64 B = blocks.size();
         std::vector<u64> n_step(B), n_slice(B);
         u64 longest = 0;
         for (const Block &b : blocks) longest = std::max(longest, b.e1 - b.e0);
-        std::unique_ptr<Piece[]> scratch(new Piece[2 * longest * (u64)threads()]);
-        auto scratch_of_thread = [&]() {
-            Piece *const mine = scratch.get() + 2 * longest * (u64)this_thread();
+        std::unique_ptr<Piece[]> scratch(new Piece[2 * longest * (u64)width]);
+        auto scratch_of = [&](unsigned who) {
+            Piece *const mine = scratch.get() + 2 * longest * (u64)who;
             return Pieces{mine, mine + longest};
         };
-#pragma omp parallel
-        {
-            Pieces p = scratch_of_thread();
-#pragma omp for schedule(dynamic, 1)
-            for (long long b = 0; b < B; b++)
+        share_steps(B, 1, width, [&](u64 b, u64, unsigned who) {
+            Pieces p = scratch_of(who);
             {
                 pieces_of(blocks[b], p);
                 u64 s = 0;
@@ -603,9 +586,9 @@ struct Builder
                 n_step[b] = s;
                 n_slice[b] = (p.size() + kTiledSlice - 1) / kTiledSlice;
             }
-        }
+        });
         u64 steps = 0, nsl = 0;
-        for (long long b = 0; b < B; b++)
+        for (u64 b = 0; b < B; b++)
         {
             blocks[b].step = steps;
             blocks[b].slice = nsl;
@@ -621,11 +604,8 @@ struct Builder
         // what stands for a row among the slices' rows
         const bool some = !out.parts.empty();
         const u32 all = out.n_parts > 0 && !out.direct ? kTiledInParts : 0;
-#pragma omp parallel
-        {
-            Pieces p = scratch_of_thread();
-#pragma omp for schedule(dynamic, 1)
-            for (long long b = 0; b < B; b++)
+        share_steps(B, 1, width, [&](u64 b, u64, unsigned who) {
+            Pieces p = scratch_of(who);
             {
                 pieces_of(blocks[b], p);
                 u64 step = blocks[b].step, slice = blocks[b].slice;
@@ -655,7 +635,7 @@ struct Builder
                     out.end.p[slice] = (u32)step;
                 }
             }
-        }
+        });
         memset(val + steps * kTiledSlice, 0, kTiledSlackSteps * kTiledSlice * sizeof(VT));
         memset(out.col.p + steps * kTiledSlice, 0, kTiledSlackSteps * kTiledSlice * sizeof(uint16_t));
         memset(out.row.p + nsl * kTiledSlice, 0xff, kTiledSlackSlices * kTiledSlice * sizeof(u32));
@@ -718,12 +698,9 @@ struct Builder
         out.col.make(places);
         float *const val = (float *)out.val.p;
         uint16_t *const cl = out.col.p;
-        ThreadCounters to_of_thread(C);
-#pragma omp parallel
-        {
-            u64 *const to = to_of_thread.mine();
-#pragma omp for schedule(dynamic, 1)
-            for (long long c = 0; c < (long long)chunks.size(); c++)
+        ThreadCounters to_of_thread(C, width);
+        share_steps(chunks.size(), 1, width, [&](u64 c, u64, unsigned who) {
+            u64 *const to = to_of_thread.of(who);
             {
                 for (u64 t = 0; t < C; t++) to[t] = at[(size_t)c * C + t] + to_unit[t];
                 walk_any<float>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, float v) ASP_INLINE {
@@ -733,7 +710,7 @@ struct Builder
                     val[unit_val_at(q)] = v;
                 });
             }
-        }
+        });
         // what fills a tile's last unit belongs to its last row and adds 0 * 0
         for (u64 t = 0; t < C; t++)
             for (u64 q = end[t]; q < tile_begin[t + 1]; q++)
@@ -752,10 +729,8 @@ struct Builder
         // what stands for a row among the units' rows
         const bool some = !out.parts.empty();
         const u32 all = out.n_parts > 0 && !out.direct ? kTiledInParts : 0;
-#pragma omp parallel for schedule(static)
-        for (long long u = 0; u < (long long)n; u++)
-        {
-            u32 *const row = e_row.p + (u64)u * U;
+        for_each(n, true, [&](u64 u) {
+            u32 *const row = e_row.p + u * U;
             u32 found = 0, before = 0;
             for (u32 l = 0; l < 32; l++)
             {
@@ -768,10 +743,10 @@ struct Builder
                     word |= 1u << k;
                     row[found++] = some ? row_code[r] : r | all; // (never beyond what has been read)
                 }
-                out.word.p[(u64)u * 32 + l] = word;
+                out.word.p[u * 32 + l] = word;
             }
             out.seg.p[u] = found;
-        }
+        });
         u64 sum = 0;
         for (u64 u = 0; u < n; u++)
         {
@@ -781,8 +756,7 @@ struct Builder
         }
         for (u32 i = 0; i < kTiledSlackUnits; i++) out.seg.p[n + i] = (u32)sum;
         out.row.make(std::max<u64>(sum, 1));
-#pragma omp parallel for schedule(static)
-        for (long long u = 0; u < (long long)n; u++) memcpy(out.row.p + out.seg.p[u], e_row.p + (u64)u * U, (out.seg.p[u + 1] - out.seg.p[u]) * sizeof(u32));
+        for_each(n, true, [&](u64 u) { memcpy(out.row.p + out.seg.p[u], e_row.p + u * U, (out.seg.p[u + 1] - out.seg.p[u]) * sizeof(u32)); });
         out.nnz = N;
         out.units = n;
         // work of the CTAs: the units in order; a unit costs its elements and its rows

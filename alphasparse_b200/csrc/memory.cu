@@ -84,8 +84,7 @@ template <class F>
 void parts(size_t n, F &&f)
 {
     const long long k = (long long)((n + kPart - 1) / kPart);
-#pragma omp parallel for schedule(static) if (k > 3)
-    for (long long i = 0; i < k; i++) f((size_t)i * kPart, std::min(kPart, n - (size_t)i * kPart));
+    host::for_each((uint64_t)k, k > 3, [&](uint64_t i) { f((size_t)i * kPart, std::min(kPart, n - (size_t)i * kPart)); });
 }
 } // namespace
 
@@ -364,12 +363,10 @@ cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaS
         filled[piece_of[(size_t)q]].fetch_add(1);
     };
     open_from(0);
-#pragma omp parallel
-    {
-        bool mine = false;
-#pragma omp master
-        mine = true;
-        if (mine)
+    // (everybody else's piece begins and ends whenever, the caller is not kept waiting for them)
+    const unsigned width = std::min(host::crew_width(), host::kMostPieces);
+    host::share_pieces(width, width, [&](unsigned piece, unsigned) {
+        if (piece == 0) // the caller's
         {
             for (size_t k = 0; k < pieces.size() && e == cudaSuccess; k++)
             {
@@ -384,7 +381,7 @@ cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaS
         }
         else
             while (!stop.load() && next_part.load() < n_parts) fill_one();
-    }
+    }, host::kCallAll);
     return e;
 }
 

@@ -1,7 +1,6 @@
-// Memory runs out while the host builds formats and layouts. Argument "region": every allocation of a parallel region fails (an
+// Memory runs out while the host builds formats and layouts. Argument "region": every allocation in a piece of a shared loop fails (an
 // exception cannot leave one, so none may be made there); "any": the n-th large allocation fails, for every n until all succeed.
 // Ends with status 0 and a line per part, or is ended by the runtime.
-#include <omp.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -20,7 +19,7 @@ static std::atomic<long> countdown{-1}, refused{0};
 
 void *operator new(size_t n)
 {
-    bool no = in_regions && omp_in_parallel();
+    bool no = in_regions && asp::host::in_piece();
     if (countdown >= 0 && n >= 4096 && countdown-- == 0) no = true;
     if (no) refused++;
     void *p = no ? nullptr : malloc(n ? n : 1);

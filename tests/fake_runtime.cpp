@@ -17,6 +17,7 @@
 #include <thread>
 #include <vector>
 
+#include "../alphasparse_b200/csrc/host/crew.cpp"
 #include "../alphasparse_b200/csrc/host/hostmem.cpp"
 #include "../alphasparse_b200/csrc/memory.cu"
 

@@ -1,5 +1,4 @@
-"""CPU suite: formats of small matrices are built without a parallel region, whose threads a forked process does not have: it can build
-them after its parent has."""
+"""CPU suite: a forked process builds formats after its parent has, without the threads that helped there."""
 import subprocess
 import sys
 
@@ -35,8 +34,8 @@ sys.exit(2)
 """
 
 
-@pytest.mark.parametrize("rows", [500, 4_000, 30_000])
-def test_a_forked_process_builds_small_formats(rows):
+@pytest.mark.parametrize("rows", [500, 4_000, 30_000, 200_000])
+def test_a_forked_process_builds_formats(rows):
     import os
 
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))

@@ -17,9 +17,9 @@ int main()
     one[37] = 390000;
     if (!by_rows(one, 8)) return 4;                                // one that holds nearly everything: all but one thread would wait
     if (!by_rows({400000, 300000, 350000, 10}, 8)) return 5;       // fewer than the threads
-    std::vector<u64> some(100, 100000);
-    some[0] = 300000;
-    if (by_rows(some, 4)) return 6;                                // a large one, but more in all the others, which nobody would share
+    std::vector<u64> some(100, 7000);
+    some[0] = 30000;
+    if (by_rows(some, 8)) return 6;                                // a large one, but more in all the others, which nobody would share
     if (by_rows(std::vector<u64>(60, 1), 2000000)) return 8;       // a row each: nothing to share inside
     if (!by_rows({7}, 3) || !by_rows({}, 1)) return 7;             // nothing to share
     return 0;
