@@ -261,7 +261,7 @@ static asp_status make_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t 
     });
     if (first_bad.load(std::memory_order_relaxed) == n_rows) // (rows are only looked into once the offsets are known to be in order)
     {
-        auto good = [=](uint64_t r) {
+        const auto good = [=](uint64_t r) ASP_INLINE {
             bool bad = false;
             uint32_t prev = 0;
             for (int64_t k = indptr[r]; k < indptr[r + 1]; k++)
@@ -272,7 +272,8 @@ static asp_status make_from_csr(uint64_t n_rows, uint64_t n_cols, const int64_t 
             return !bad;
         };
         share_steps(n_rows, 256, (uint64_t)indptr[n_rows] > kParallelNnz ? crew_width() : 1, [&](uint64_t r, uint64_t e, unsigned) {
-            while (r < e && good(r)) r++;
+            const auto mine = good;
+            while (r < e && mine(r)) r++;
             if (r < e) lower(first_bad, r);
         });
     }

@@ -88,8 +88,10 @@ const size_t kParallelBytes = 1u << 18;
 const uint64_t kParallelRows = 1u << 13, kParallelNnz = 1u << 14;
 inline void par_copy(void *dst, const void *src, size_t bytes)
 {
-    share_ranges((bytes + 63) / 64, bytes > kParallelBytes, [=](uint64_t i, uint64_t e) {
-        memcpy((char *)dst + i * 64, (const char *)src + i * 64, std::min<size_t>(bytes, e * 64) - i * 64);
+    const size_t line = 64, most = 1u << 16;
+    share_ranges((bytes + line - 1) / line, bytes > kParallelBytes, [=](uint64_t i, uint64_t e) {
+        const size_t end = std::min<size_t>(bytes, e * line);
+        for (size_t o = i * line; o < end; o += most) memcpy((char *)dst + o, (const char *)src + o, std::min(most, end - o));
     });
 }
 

@@ -374,45 +374,43 @@ struct Builder
         share_steps(chunks.size(), 1, width, [&](u64 c, u64, unsigned who) {
             u64 *const pieces = pieces_of_thread.of(who), *const n = n_of_thread.of(who);
             u64 all_runs = 0, all_near = 0;
-            {
-                std::fill(n, n + C, 0);
-                u32 *const first = edge.data() + (size_t)c * edges, *const last = first + C;
-                u64 row = ~0ull, tile = ~0ull, run = 0;
-                u32 of_row = 0, elements = 0; // pieces and elements since the row changed
-                // rows that are one thread's in the template's kernel have no more parts than it adds elements
-                const TiledSource &from = src[chunks[c].sub];
-                const bool alone = !from.a->atomic && (from.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || from.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS);
-                auto row_ends = [&]() {
-                    // (several threads may have elements of a row)
-                    if (of_row && alone) __atomic_store_n(&row_code[row], 1, __ATOMIC_RELAXED);
-                    else if (of_row) __atomic_fetch_add(&row_code[row], (u32)std::min<u64>(of_row + elements / warp_steps, 1u << 16) * share[chunks[c].sub], __ATOMIC_RELAXED);
-                    of_row = elements = 0;
-                };
-                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT) ASP_INLINE {
-                    const u64 t = (u32)col / TW;
-                    const bool begins = n[t]++ == 0;
-                    if (r != row || t != tile || run == kMaxPiece)
+            std::fill(n, n + C, 0);
+            u32 *const first = edge.data() + (size_t)c * edges, *const last = first + C;
+            u64 row = ~0ull, tile = ~0ull, run = 0;
+            u32 of_row = 0, elements = 0; // pieces and elements since the row changed
+            // rows that are one thread's in the template's kernel have no more parts than it adds elements
+            const TiledSource &from = src[chunks[c].sub];
+            const bool alone = !from.a->atomic && (from.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || from.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS);
+            auto row_ends = [&]() {
+                // (several threads may have elements of a row)
+                if (of_row && alone) __atomic_store_n(&row_code[row], 1, __ATOMIC_RELAXED);
+                else if (of_row) __atomic_fetch_add(&row_code[row], (u32)std::min<u64>(of_row + elements / warp_steps, 1u << 16) * share[chunks[c].sub], __ATOMIC_RELAXED);
+                of_row = elements = 0;
+            };
+            walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT) ASP_INLINE {
+                const u64 t = (u32)col / TW;
+                const bool begins = n[t]++ == 0;
+                if (r != row || t != tile || run == kMaxPiece)
+                {
+                    pieces[t]++;
+                    if (begins) first[t] = (u32)r;
+                    else if (r != last[t])
                     {
-                        pieces[t]++;
-                        if (begins) first[t] = (u32)r;
-                        else if (r != last[t])
-                        {
-                            all_runs++;
-                            all_near += near(last[t], r);
-                        }
-                        last[t] = (u32)r;
-                        if (r != row) row_ends();
-                        of_row++;
-                        row = r;
-                        tile = t;
-                        run = 0;
+                        all_runs++;
+                        all_near += near(last[t], r);
                     }
-                    run++;
-                    elements++;
-                });
-                row_ends();
-                std::copy(n, n + C, at.begin() + (size_t)c * C);
-            }
+                    last[t] = (u32)r;
+                    if (r != row) row_ends();
+                    of_row++;
+                    row = r;
+                    tile = t;
+                    run = 0;
+                }
+                run++;
+                elements++;
+            });
+            row_ends();
+            std::copy(n, n + C, at.begin() + (size_t)c * C);
             sum_runs.fetch_add(all_runs, std::memory_order_relaxed);
             sum_near.fetch_add(all_near, std::memory_order_relaxed);
         });
@@ -498,15 +496,13 @@ struct Builder
         ThreadCounters to_of_thread(C, width);
         share_steps(chunks.size(), 1, width, [&](u64 c, u64, unsigned who) {
             u64 *const to = to_of_thread.of(who);
-            {
-                std::copy(at.begin() + (size_t)c * C, at.begin() + (size_t)(c + 1) * C, to);
-                walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) ASP_INLINE {
-                    const u64 t = (u32)col / TW, q = to[t]++;
-                    e_row.p[q] = (u32)r;
-                    e_col.p[q] = (uint16_t)(col - t * TW);
-                    e_val.p[q] = v;
-                });
-            }
+            std::copy(at.begin() + (size_t)c * C, at.begin() + (size_t)(c + 1) * C, to);
+            walk_any<VT>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, VT v) ASP_INLINE {
+                const u64 t = (u32)col / TW, q = to[t]++;
+                e_row.p[q] = (u32)r;
+                e_col.p[q] = (uint16_t)(col - t * TW);
+                e_val.p[q] = v;
+            });
         });
     }
 
@@ -579,13 +575,11 @@ struct Builder
         };
         share_steps(B, 1, width, [&](u64 b, u64, unsigned who) {
             Pieces p = scratch_of(who);
-            {
-                pieces_of(blocks[b], p);
-                u64 s = 0;
-                for (size_t i = 0; i < p.size(); i += kTiledSlice) s += p[i].len;
-                n_step[b] = s;
-                n_slice[b] = (p.size() + kTiledSlice - 1) / kTiledSlice;
-            }
+            pieces_of(blocks[b], p);
+            u64 s = 0;
+            for (size_t i = 0; i < p.size(); i += kTiledSlice) s += p[i].len;
+            n_step[b] = s;
+            n_slice[b] = (p.size() + kTiledSlice - 1) / kTiledSlice;
         });
         u64 steps = 0, nsl = 0;
         for (u64 b = 0; b < B; b++)
@@ -606,34 +600,32 @@ struct Builder
         const u32 all = out.n_parts > 0 && !out.direct ? kTiledInParts : 0;
         share_steps(B, 1, width, [&](u64 b, u64, unsigned who) {
             Pieces p = scratch_of(who);
+            pieces_of(blocks[b], p);
+            u64 step = blocks[b].step, slice = blocks[b].slice;
+            for (size_t i = 0; i < p.size(); i += kTiledSlice, slice++)
             {
-                pieces_of(blocks[b], p);
-                u64 step = blocks[b].step, slice = blocks[b].slice;
-                for (size_t i = 0; i < p.size(); i += kTiledSlice, slice++)
+                const u32 depth = p[i].len;
+                VT *v = val + step * kTiledSlice;
+                uint16_t *c = out.col.p + step * kTiledSlice;
+                u32 *rows = out.row.p + slice * kTiledSlice;
+                memset(v, 0, (size_t)depth * kTiledSlice * sizeof(VT));
+                std::fill(c, c + (size_t)depth * kTiledSlice, (uint16_t)TW);
+                for (u32 j = 0; j < kTiledSlice; j++)
                 {
-                    const u32 depth = p[i].len;
-                    VT *v = val + step * kTiledSlice;
-                    uint16_t *c = out.col.p + step * kTiledSlice;
-                    u32 *rows = out.row.p + slice * kTiledSlice;
-                    memset(v, 0, (size_t)depth * kTiledSlice * sizeof(VT));
-                    std::fill(c, c + (size_t)depth * kTiledSlice, (uint16_t)TW);
-                    for (u32 j = 0; j < kTiledSlice; j++)
+                    // piece j goes to lane j % 32, so that one `red` of a warp covers 32 neighbouring pieces
+                    const u32 o = (j % 32) * kTiledLanePieces + j / 32;
+                    rows[o] = kTiledNoRow;
+                    if (i + j >= p.size()) continue;
+                    const u64 e = blocks[b].e0 + p[i + j].start;
+                    rows[o] = some ? row_code[e_row.p[e]] : e_row.p[e] | all;
+                    for (u32 k = 0; k < p[i + j].len; k++)
                     {
-                        // piece j goes to lane j % 32, so that one `red` of a warp covers 32 neighbouring pieces
-                        const u32 o = (j % 32) * kTiledLanePieces + j / 32;
-                        rows[o] = kTiledNoRow;
-                        if (i + j >= p.size()) continue;
-                        const u64 e = blocks[b].e0 + p[i + j].start;
-                        rows[o] = some ? row_code[e_row.p[e]] : e_row.p[e] | all;
-                        for (u32 k = 0; k < p[i + j].len; k++)
-                        {
-                            v[k * kTiledSlice + o] = e_val.p[e + k];
-                            c[k * kTiledSlice + o] = e_col.p[e + k];
-                        }
+                        v[k * kTiledSlice + o] = e_val.p[e + k];
+                        c[k * kTiledSlice + o] = e_col.p[e + k];
                     }
-                    step += depth;
-                    out.end.p[slice] = (u32)step;
                 }
+                step += depth;
+                out.end.p[slice] = (u32)step;
             }
         });
         memset(val + steps * kTiledSlice, 0, kTiledSlackSteps * kTiledSlice * sizeof(VT));
@@ -701,15 +693,13 @@ struct Builder
         ThreadCounters to_of_thread(C, width);
         share_steps(chunks.size(), 1, width, [&](u64 c, u64, unsigned who) {
             u64 *const to = to_of_thread.of(who);
-            {
-                for (u64 t = 0; t < C; t++) to[t] = at[(size_t)c * C + t] + to_unit[t];
-                walk_any<float>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, float v) ASP_INLINE {
-                    const u64 t = (u32)col / TW, q = to[t]++;
-                    e_row.p[q] = (u32)r;
-                    cl[q] = (uint16_t)(col - t * TW);
-                    val[unit_val_at(q)] = v;
-                });
-            }
+            for (u64 t = 0; t < C; t++) to[t] = at[(size_t)c * C + t] + to_unit[t];
+            walk_any<float>(src[chunks[c].sub], chunks[c].u0, chunks[c].u1, [&](u64 r, u64 col, float v) ASP_INLINE {
+                const u64 t = (u32)col / TW, q = to[t]++;
+                e_row.p[q] = (u32)r;
+                cl[q] = (uint16_t)(col - t * TW);
+                val[unit_val_at(q)] = v;
+            });
         });
         // what fills a tile's last unit belongs to its last row and adds 0 * 0
         for (u64 t = 0; t < C; t++)

@@ -15,7 +15,8 @@
 //          group, which k_rows turns into y and leaves as zeros for the next call (0.42e-7). In fp64 tiles and warps
 //          take `copies` sums of a row in turn, which k_rows adds up with their roundings. A piece is summed with more than the value's bits, too.
 // The stream is read two batches deep into registers. 159 KB of shared memory per tile leave the L1 enough lines for the
-// loads in flight: with 224 KB the same stream is read at 4.2 instead of 5 TB/s.
+// loads in flight: with 224 KB the same stream is read at 4.2 instead of 5 TB/s. (k_tiled_units takes 32 KB more: 2 KB a warp, in
+// which the sums of a unit's rows are laid out.)
 // Where rows have few elements in a tile (1 to 7) and lie side by side, there are units instead of slices (k_tiled_units): a slice
 // puts pieces of one length together, so that its `red` goes to 32 rows anywhere among 1024, ten lines of sums or more, each of which is a
 // request to L2, and that is what bounds it. A unit is 256 elements of a tile in order, eight a lane. Every lane adds up the runs of its

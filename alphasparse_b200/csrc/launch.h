@@ -9,8 +9,8 @@
 // kernel before is then waiting for all.
 //
 // grid_release() lets the next kernel start when all CTAs of this one have called it (or ended). Most kernels call it after their
-// wait, so that one kernel at most is waiting behind the running one. k_clear, k_tiled and k_rows call it before: k_tiled loads the
-// head of its stream meanwhile. Several kernels may then be waiting, which costs their place on the SMs and nothing else: they
+// wait, so that one kernel at most is waiting behind the running one. k_clear, k_tiled, k_tiled_units and k_rows call it before: the
+// two in the middle load the head of their stream meanwhile. Several kernels may then be waiting, which costs their place on the SMs and nothing else: they
 // still store nothing before everything earlier has finished, and a kernel's CTAs are all on the device before the next one's are.
 #ifndef ASP_LAUNCH_H
 #define ASP_LAUNCH_H
