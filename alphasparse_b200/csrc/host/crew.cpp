@@ -43,7 +43,11 @@ struct Crew
     Slot slots[kSlots];
     alignas(64) std::atomic<uint32_t> epoch{0}; // changes with every loop that begins
     alignas(64) std::atomic<int> asleep{0};
-    std::atomic<int64_t> alone_until{0}; // (ns) helpers have been kept from running with pieces in their hands: no core is free
+    // Helpers have been kept from running with pieces in their hands: until then (ns) no core is free for them. The time doubles from
+    // one such piece to the next, and halves again with every 32 loops without one: a piece may also be late by itself (pages that
+    // it is the first to write).
+    std::atomic<int64_t> alone_until{0};
+    std::atomic<int> late{0}, in_time{0};
     std::atomic<int> helpers{0};
     std::mutex growing;
     const int cores = omp_get_num_procs();
@@ -210,27 +214,32 @@ void crew_run(unsigned pieces, unsigned width, unsigned call, void (*run)(void *
     Crew *c = t_in_piece || width <= 1 ? nullptr : crew(std::min(width, kMostHelpers) - 1);
     // (as many callers as cores: a helper would only take a core from one of them, with a piece in its hands)
     const int callers = g_callers.load(std::memory_order_relaxed);
-    const int64_t begin = now();
-    if (c && ((callers > 1 && 2 * callers > c->cores) || begin < c->alone_until.load(std::memory_order_relaxed))) c = nullptr;
+    if (c && callers > 1 && 2 * callers > c->cores) c = nullptr;
+    unsigned alone = 0; // pieces that have been done alone
+    while (c && alone < pieces && now() < c->alone_until.load(std::memory_order_relaxed)) run(arg, alone++, 0);
     Slot *s = nullptr;
-    for (unsigned i = 0; c && i < kSlots && !s; i++)
+    for (unsigned i = 0; c && i < kSlots && alone < pieces && !s; i++)
         if (!c->slots[i].used.exchange(true, std::memory_order_acquire)) s = &c->slots[i];
     if (!s)
     {
-        for (unsigned p = 0; p < pieces; p++) run(arg, p, 0);
+        while (alone < pieces) run(arg, alone++, 0);
         return;
     }
+    const int64_t begin = now();
     const uint64_t gen = gen_of(s->word.load(std::memory_order_relaxed)) + 1, word = make_word(gen, std::min(width, kMostHelpers), pieces);
     s->run = run;
     s->arg = arg;
-    s->done.store(0, std::memory_order_relaxed);
-    s->taken[0].store(gen, std::memory_order_relaxed);
+    s->done.store(alone, std::memory_order_relaxed);
+    for (unsigned p = 0; p < std::max(1u, alone); p++) s->taken[p].store(gen, std::memory_order_relaxed);
     s->word.store(word, std::memory_order_release);
     c->epoch.fetch_add(1, std::memory_order_seq_cst);
     if (c->asleep.load(std::memory_order_seq_cst) > 0 && too_many(*c) < 0) wake(*c, c->helpers.load(std::memory_order_relaxed) >= (int)width ? (int)kCallAll : (int)call);
     t_in_piece = true;
-    run(arg, 0, 0);
-    s->done.fetch_add(1, std::memory_order_release);
+    if (alone == 0)
+    {
+        run(arg, 0, 0);
+        s->done.fetch_add(1, std::memory_order_release);
+    }
     const int64_t first = now() - begin, longest = std::max(first, work(*s, word, 0, [] {}));
     t_in_piece = false;
     // what others have begun. A piece that takes four times as long as any of this thread's is somebody's who has been kept from running
@@ -241,7 +250,17 @@ void crew_run(unsigned pieces, unsigned width, unsigned call, void (*run)(void *
             if (i < 1024) relax();
             else sched_yield();
         const int64_t end = now();
-        if (end - idle > std::max<int64_t>(400000, 4 * longest)) c->alone_until.store(end + 16 * (end - idle), std::memory_order_relaxed);
+        if (end - idle > std::max<int64_t>(400000, 4 * longest))
+        {
+            const int times = std::min(c->late.fetch_add(1, std::memory_order_relaxed), 5);
+            c->alone_until.store(end + ((end - idle) << times), std::memory_order_relaxed);
+            c->in_time.store(0, std::memory_order_relaxed);
+        }
+        else if (c->late.load(std::memory_order_relaxed) > 0 && c->in_time.fetch_add(1, std::memory_order_relaxed) >= 32)
+        {
+            c->in_time.store(0, std::memory_order_relaxed);
+            c->late.store(std::min(c->late.load(std::memory_order_relaxed) - 1, 5), std::memory_order_relaxed);
+        }
     }
     s->word.store(make_word(gen, 0, 0), std::memory_order_relaxed);
     s->used.store(false, std::memory_order_release);

@@ -83,7 +83,7 @@ std::shared_ptr<void> big_buffer(size_t bytes);
 void host_pool_trim();
 
 // Below these a loop runs on the calling thread alone: sharing one costs 1 to 5 us. (The limits were 4 MB, 2^18 rows and 2^19 non-zeros
-// while loops were OpenMP's; crew.cpp has the figures of both.)
+// while loops were OpenMP's; crew.hpp has the figures of both.)
 const size_t kParallelBytes = 1u << 18;
 const uint64_t kParallelRows = 1u << 13, kParallelNnz = 1u << 14;
 inline void par_copy(void *dst, const void *src, size_t bytes)
