@@ -61,7 +61,7 @@ EXPORTS = [
     "asp_ctx_create", "asp_multicast_store", "asp_spmv_publish", "asp_plan_end_rows", "asp_rank_barrier", "asp_ctx_destroy", "asp_ctx_stream", "asp_plan_group_create", "asp_plan_descs_validate", "asp_plan_destroy",
     "asp_plan_set_launch", "asp_plan_get_launch", "asp_plan_set_tuning", "asp_plan_format_bytes", "asp_plan_launches", "asp_spmv", "asp_spmv_host", "asp_time",
     "asp_synchronize", "asp_status_str", "asp_last_error", "asp_built_for_sm100a", "asp_spmv_host_static",
-    "asp_static_stage_bytes", "asp_search_gpu", "asp_spmv_host_pipelined", "asp_dist_create", "asp_dist_destroy", "asp_dist_spmv", "asp_dist_spmv_iter", "asp_dist_status", "asp_plan_layout_bytes", "asp_plan_layout_form", "asp_host_alloc", "asp_host_free", "asp_device_trim", "asp_plan_group_create_with",
+    "asp_static_stage_bytes", "asp_search_gpu", "asp_spmv_host_pipelined", "asp_dist_create", "asp_dist_destroy", "asp_dist_spmv", "asp_dist_spmv_iter", "asp_dist_status", "asp_plan_layout_bytes", "asp_plan_layout_form", "asp_plan_whole_rows", "asp_host_alloc", "asp_host_free", "asp_device_trim", "asp_plan_group_create_with",
 ]
 
 _lib = None
@@ -129,6 +129,8 @@ def lib() -> C.CDLL:
     L.asp_plan_layout_bytes.restype = C.c_uint64
     L.asp_plan_layout_form.argtypes = [C.c_void_p]
     L.asp_plan_layout_form.restype = C.c_int
+    L.asp_plan_whole_rows.argtypes = [C.c_void_p]
+    L.asp_plan_whole_rows.restype = C.c_int
     L.asp_plan_group_create_with.argtypes = [C.c_void_p, C.POINTER(PlanDesc), C.c_int, C.c_int, C.POINTER(C.c_void_p)]
     L.asp_plan_group_create_with.restype = C.c_int
     L.asp_device_trim.argtypes = [C.c_int]
@@ -382,6 +384,10 @@ class PlanGroup:
         """What the column-tiled layout consists of (asp_plan_layout_form): "slices" or "units", and "y" and "sums", where rows are added up."""
         form = lib().asp_plan_layout_form(self._plans[0])
         return {name for bit, name in ((1, "slices"), (2, "units"), (4, "y"), (8, "sums")) if form & bit}
+
+    def whole_rows(self) -> bool:
+        """Whether the group's one plan runs a kernel that takes whole rows (asp_plan_whole_rows)."""
+        return self.n == 1 and bool(lib().asp_plan_whole_rows(self._plans[0]))
 
     def launches(self) -> int:
         """Kernels that one asp_spmv over the group launches, without those that clear y or store the sums of rows."""

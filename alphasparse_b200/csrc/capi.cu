@@ -146,7 +146,7 @@ struct asp_plan
     int templ = 0;
     int val_is_f64 = 0;
     int col_width = 4;
-    uint64_t n_rows = 0, n_cols = 0, true_nnz = 0;
+    uint64_t n_rows = 0, n_cols = 0, true_nnz = 0, stored = 0;
     unsigned grid = 1, block = 32;
     size_t smem = 0;
     int vec = 1;
@@ -162,6 +162,10 @@ struct asp_plan
     // indices into y; kept on the device for the publishing SpMV (asp_spmv_publish)
     std::shared_ptr<Arena> end_rows;
     uint64_t n_end_rows = 0;
+    // templates whose chunks of a row lie one after the other: the rows, for the kernels that take a whole one (kernels_rows.cu)
+    std::shared_ptr<Arena> row_list;
+    asp::RowArgs own_rows = {};
+    bool own_rows_cover = false; // every row of y is in the list
     int64_t asked_tblock = 0, asked_threads = 0, asked_reduce = 0; // the launch last requested (re-applied when vec / path change)
 };
 
@@ -484,6 +488,113 @@ bool stores_every_row(const asp_plan_desc &d, const std::vector<HostMeta> &hm, c
     }
 }
 
+// The rows of a (validated) plan whose chunks of a row are consecutive, as kernels_rows.cu takes them; `longest` of them. false: another
+// template, a row in two places, or offsets beyond 32 bits.
+bool list_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, std::vector<uint2> &out, uint64_t &longest)
+{
+    using namespace asp;
+    const bool chunks = d.template_type == ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE || d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE;
+    if ((!chunks && d.template_type != ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE) || d.n_rows > 0xffffffffull) return false;
+    std::vector<bool> seen(d.n_rows, false);
+    uint64_t end = 0;
+    longest = 0;
+    auto put = [&](uint64_t row, uint64_t from, uint64_t to) {
+        if (to < from || to > 0xffffffffull || row >= d.n_rows || seen[row] || (!out.empty() && from != end)) return false;
+        seen[row] = true;
+        end = to;
+        longest = std::max(longest, to - from);
+        out.push_back(make_uint2((unsigned)from, (unsigned)row));
+        return true;
+    };
+    if (chunks)
+    {
+        const HostMeta &nz = hm[d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE ? MS_BLK_NZ : MS_WARP_NZ], &of = hm[MS_ROW_OF_UNIT];
+        const uint64_t n = d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE ? a.n_units : a.effective, radd = a.row_add ? d.first_row : 0;
+        for (uint64_t u = 0; u < n;)
+        {
+            uint64_t e = u + 1;
+            const uint64_t row = of.get(u);
+            while (e < n && of.get(e) == row) e++;
+            if (!put(row + radd, nz.get(u), nz.get(e))) return false;
+            u = e;
+        }
+    }
+    else
+        for (uint64_t b = 0; b < a.n_units; b++)
+        {
+            const uint64_t w0 = hm[MS_BLK_WARP].get(b), r0 = hm[MS_BLK_ROW].get(b), r1 = std::min<uint64_t>(hm[MS_BLK_ROW].get(b + 1), a.effective);
+            const uint64_t g0 = hm[MS_ROW_OFF].get(r0);
+            for (uint64_t r = r0; r < r1; r++)
+            {
+                const uint64_t row = a.sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : a.sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
+                if (!put(row, hm[MS_WARP_NZ].get(w0 + hm[MS_ROW_OFF].get(r) - g0), hm[MS_WARP_NZ].get(w0 + hm[MS_ROW_OFF].get(r + 1) - g0))) return false;
+            }
+        }
+    if (out.empty()) return false;
+    out.push_back(make_uint2((unsigned)end, 0));
+    return true;
+}
+
+// The same of the row-grouped template; `tlbs` of all rows, `most` of one
+bool list_tlb_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, std::vector<uint4> &out, uint64_t &tlbs, uint64_t &most)
+{
+    using namespace asp;
+    if (d.template_type != ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || d.n_rows > 0xffffffffull) return false;
+    std::vector<bool> seen(d.n_rows, false);
+    tlbs = most = 0;
+    for (uint64_t b = 0; b < a.n_units; b++)
+    {
+        const uint64_t nz = hm[MS_BLK_NZ].get(b), n = hm[MS_BLK_THR].get(b + 1) - hm[MS_BLK_THR].get(b), S = hm[MS_TLB_SIZE].get(b);
+        const uint64_t r0 = hm[MS_BLK_ROW].get(b), r1 = std::min<uint64_t>(hm[MS_BLK_ROW].get(b + 1), a.effective), g0 = hm[MS_ROW_OFF].get(r0);
+        if (S == 0 || S > 0xffff || nz + n * S > 0xffffffffull) return false;
+        for (uint64_t r = r0; r < r1; r++)
+        {
+            const uint64_t row = a.sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : a.sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
+            const uint64_t lo = hm[MS_ROW_OFF].get(r) - g0, hi = hm[MS_ROW_OFF].get(r + 1) - g0;
+            if (hi < lo || hi > n || hi - lo > 0xffff || row >= d.n_rows || seen[row]) return false;
+            seen[row] = true;
+            tlbs += hi - lo;
+            most = std::max(most, hi - lo);
+            out.push_back(make_uint4((unsigned)(nz + lo), (unsigned)row, (unsigned)((hi - lo) | S << 16), (unsigned)n));
+        }
+    }
+    return !out.empty();
+}
+
+// Whole rows for a few lanes, a warp or a CTA, where that is the faster way (kernels_rows.cu). A warp takes up to 512 elements (four trips
+// of 1.2 us; chunks in parallel are faster beyond that), a CTA rows of 256 and more on average, up to 16384 (four trips of 1024 threads).
+// Rows of TLBs: up to 2 M elements, beyond which the CTA's long strips stream better (4.9 M, FEM, fp32: 13.0 us, 17.3 by rows; 1.6 M: 7.2, 5.1).
+struct OwnRows
+{
+    asp::RowArgs args = {};
+    std::vector<uint2> rows;
+    std::vector<uint4> tlbs;
+    uint64_t trips = 0; // of warps that take a row
+    const void *data() const { return tlbs.empty() ? (const void *)rows.data() : tlbs.data(); }
+    size_t bytes() const { return rows.size() * sizeof(uint2) + tlbs.size() * sizeof(uint4); }
+    void make(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp_plan &p, int sm_count)
+    {
+        uint64_t longest = 0, all = 0;
+        if (d.template_type == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS)
+        {
+            args.lanes = 2;
+            bool good = p.stored <= (2u << 20) && list_tlb_rows(d, hm, perm, p.args, tlbs, all, longest);
+            while (args.lanes < 32 && args.lanes * tlbs.size() < all) args.lanes *= 2;
+            args.n = (unsigned)tlbs.size();
+            if (!good || longest > 8 * args.lanes) tlbs.clear();
+            return;
+        }
+        if (!list_rows(d, hm, perm, p.args, rows, longest)) return rows.clear();
+        const uint64_t n = rows.size() - 1, elements = rows.back().x - rows[0].x;
+        if (longest > 512 && (longest > 16384 || elements < 256 * n)) return rows.clear();
+        // threads for all of a row in one trip while all rows are on the device at once, else for two
+        const uint64_t per = n <= 2ull * sm_count ? 4 : 8;
+        args.cta = longest <= 512 ? 0 : (unsigned)std::min<uint64_t>(1024, std::max<uint64_t>(64, (longest + 32 * per - 1) / (32 * per) * 32));
+        args.n = (unsigned)n;
+        for (uint64_t i = 0; i < n && args.cta == 0; i++) trips += (rows[i + 1].x - rows[i].x + 127) / 128;
+    }
+};
+
 asp_status ensure_xy(asp_ctx *ctx, size_t xb, size_t yb)
 {
     if (ctx->x_bytes < xb)
@@ -779,6 +890,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         a.bits_row = d.bits_row;
         a.bits_off = d.bits_off;
         const uint64_t nnz_pad = vals[i]->len;
+        p->stored = nnz_pad;
         const std::vector<HostMeta> &hm = metas[i];
         uint64_t fmt = 0;
         for (int k = 0; k < d.n_arrays; k++)
@@ -1097,6 +1209,11 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         t.threads = made[i]->block;
         src.push_back(t);
     }
+    // (a matrix so large that its gathers are scattered has the layout anyway: its rows are listed only where it turns out not to)
+    OwnRows own;
+    const bool listed = n == 1 && made[0]->templ != ASP_EMPTY_TEMPLATE && descs[0].true_nnz <= (8u << 20);
+    if (listed) own.make(descs[0], metas[0], perms[0], *made[0], ctx->sm_count);
+    if (src.size() == 1) src[0].whole_rows = own.bytes() > 0, src[0].trips = own.trips;
     asp::TiledHost th;
     std::shared_ptr<TiledGroup> tg;
     try
@@ -1161,6 +1278,28 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
             tg->covers_all_rows = th.covers_all_rows;
             for (asp_plan *p : made) p->tiled = tg;
         }
+    }
+    if (n == 1 && !tg && !listed) own.make(descs[0], metas[0], perms[0], *made[0], ctx->sm_count);
+    if (!tg && own.bytes())
+    {
+        asp_plan *const p = made[0];
+        std::shared_ptr<Arena> list(new (std::nothrow) Arena());
+        if (list && list->make(ctx->device, own.bytes()) == cudaSuccess)
+        {
+            const cudaError_t ce = ctx->stager.to_device(list->base, own.data(), own.bytes(), ctx->stream);
+            if (ce != cudaSuccess)
+            {
+                cleanup();
+                return cuda_fail(ce, "upload of the row list");
+            }
+            p->own_rows = own.args;
+            p->own_rows.val = p->args.val;
+            p->own_rows.col = p->args.col;
+            (own.tlbs.empty() ? (const void *&)p->own_rows.rows : (const void *&)p->own_rows.tlbs) = list->base;
+            p->own_rows_cover = own.args.n == descs[0].n_rows;
+            p->row_list = list;
+        }
+        else cudaGetLastError(); // no room: the chunks' own kernels
     }
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess)
@@ -1301,6 +1440,8 @@ int asp_plan_layout_form(const asp_plan *plan)
     return (a.word ? ASP_FORM_UNITS : ASP_FORM_SLICES) | (a.direct || a.n_parts == 0 ? ASP_FORM_IN_Y : 0) | (a.n_parts > 0 ? ASP_FORM_IN_SUMS : 0);
 }
 
+int asp_plan_whole_rows(const asp_plan *plan) { return plan && plan->row_list ? 1 : 0; }
+
 asp_status asp_device_trim(int device)
 {
     int n = 0;
@@ -1408,6 +1549,16 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
         }
     }
     const asp_plan *only = n_plans == 1 ? plans[0] : nullptr;
+    // whole rows are stored: what was in y is cleared or overwritten by the chunks' kernel too
+    if (only && only->row_list && (clear || !only->args.atomic))
+    {
+        if (clear && !only->own_rows_cover) ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
+        asp::RowArgs rows = only->own_rows;
+        rows.x = (const char *)d_x + only->args.first_col * g.es;
+        rows.y = d_y;
+        ASP_CUDA(asp::launch_own_rows(only->val_is_f64, only->col_width, rows, ctx->stream));
+        return ASP_OK;
+    }
     if (clear && only && only->ends_cover && only->end_rows)
         ASP_CUDA(asp::launch_zero_rows(only->val_is_f64, d_y, (const unsigned *)only->end_rows->base, only->n_end_rows, ctx->stream));
     else if (clear && !(only && only->stores_all_rows))

@@ -782,17 +782,23 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     // The group's own kernels: one request to L2 per cache line that a gather touches (290 G/s on this part, of which they reach
     // 0.85) or the format's bytes, or their longest serial chain, whichever is longest. Below some 10 us the rates are not reached
     // (20,000 rows of 80 random columns: 13.8 us for 7 us of requests); several kernels add a fork and a join.
+    // The kernels for whole rows (one sub-matrix) reach 0.75 of that rate, and take 8 to 12 us for 60,000 rows of 27 to 81 elements that lie near
+    // one another. Random columns, K4: 560 K non-zeros 4.3 us, 900 K 6.2, 1.6 M 9.0 to 9.5, 3.2 M 16.4 to 17.2; the layout in units (fp32) 5.2, 5.5,
+    // 6.6, 9.3, in slices (fp64) -, 10.5, 11.2, 14.5.
+    const bool whole = src.size() == 1 && src[0].whole_rows;
     u64 true_nnz = 0;
     double chain = 0, requests = 0, bytes_us = 0;
     for (const TiledSource &s : src)
     {
         if (unit_count(s) == 0) return false;
+        const double slow = whole ? 1.0 : slowness(s);
         true_nnz += s.true_nnz;
         chain = std::max(chain, chain_us(s));
-        requests += (double)s.stored * slowness(s);
-        bytes_us += (double)s.stored * slowness(s) * (sv + 4) / 6.0e6;
+        requests += (double)s.stored * slow;
+        bytes_us += (double)s.stored * slow * (sv + 4) / 6.0e6;
     }
     auto own = [&](double lines) {
+        if (whole) return std::max(2.9, 1.7 + std::max({lines / (0.75 * 290e3), bytes_us * 6.0 / 4.6, src[0].trips * 0.14e-3 + 0.45 * bytes_us * 6.0 / 4.6}));
         const double rate = std::max(lines / (0.85 * 290e3), bytes_us);
         return (src.size() > 1 ? 8.0 : 0.0) + std::max(2.0 + chain, 3.0 + rate + std::min(0.4 * rate, 4.5));
     };
@@ -801,9 +807,9 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     // there was a layout. Checks of that kind run on small matrices; for larger ones ASP_LAYOUT_NONE has to be asked for.
     if (src.size() > 1 && true_nnz < (1u << 16)) return false;
     // small matrices, whose time is the launch, stay with their kernels (not worth a look at the columns)
-    if (own(requests) < 7.0) return false;
+    if (own(requests) < (whole ? 5.0 : 7.0)) return false;
     double lines = 0;
-    for (const TiledSource &s : src) lines += lines_per_gather(s, sizeof(VT) == 8) * (double)s.stored * slowness(s);
+    for (const TiledSource &s : src) lines += lines_per_gather(s, sizeof(VT) == 8) * (double)s.stored * (whole ? 1.0 : slowness(s));
     const double own_us = own(lines);
     // This layout: launches and tail, the first tile of x, 2 + sv bytes per element at 4.6 TB/s, a `red` per piece (below), y
     // cleared, the sums of the rows in many parts.
@@ -811,7 +817,10 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
         return 4.5 + 2.5 * std::min(1.0, (double)n_cols / (double)tiled_tile_cols(sizeof(VT) == 8)) + (double)n * (sv + 2) / 4.6e6 + (double)pieces * 4 / 4.6e6 + red / 200e3 +
                ((double)n_rows * sv + (double)out.n_parts * 16.0 * out.copies) / 6.0e6 + (out.n_parts > 0 && out.direct ? 4.0 : 0.0);
     };
-    if (tiled_us(true_nnz, 0, 0) > 0.85 * own_us) return false;
+    // (what tiled_us says is 1 to 3 us too long for a few million non-zeros, as the time of the other kernels is; that of whole rows is not)
+    auto slower = [&](double us) { return whole ? 0.92 * (us - 1.6) > own_us : us > 0.85 * own_us; };
+    auto units_us = [](u64 n) { return 4.4 + 1.45e-6 * (double)n; };
+    if (slower(tiled_us(true_nnz, 0, 0)) && !(sizeof(VT) == 4 && whole && units_us(true_nnz) <= own_us)) return false;
     if (n_rows >= kTiledInParts || requests >= 1e11) return false;
     Builder<VT> b(src, n_rows, n_cols, true_nnz, n_sm);
     if (b.C + (u64)n_sm >= 65536) return false;
@@ -826,11 +835,12 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
         pieces += b.tile_pieces[t];
         if (p > 0) red += p * std::min(1.0, std::max(0.25, 4.0 * (double)n_rows / p / 32.0));
     }
-    if (tiled_us(b.N, pieces, red) > 0.85 * own_us) return false;
+    const bool units = sizeof(VT) == 4 && b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs && tiled_units_fit(b.runs, b.N, b.C);
+    if (whole && units ? units_us(b.N) > own_us : slower(tiled_us(b.N, pieces, red))) return false;
     b.number_rows(out);
     if constexpr (sizeof(VT) == 4)
     {
-        if (b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs && tiled_units_fit(b.runs, b.N, b.C))
+        if (units)
         {
             b.scatter_units(out);
             b.units(n_sm, out);

@@ -24,5 +24,16 @@ cudaError_t launch_clear(int val_is_f64, void *y, unsigned long long n, unsigned
 // end rows of the warps (the rows the CSR5-like kernel accumulates with `red`): cleared before, published after
 cudaError_t launch_zero_rows(int val_is_f64, void *y, const unsigned *rows, unsigned long long n, cudaStream_t st);
 cudaError_t launch_publish_rows(int val_is_f64, const void *y, void *y_mc, const unsigned *rows, unsigned long long n, cudaStream_t st);
+// whole rows whose elements lie one after the other (kernels_rows.cu): rows[i] = {first element, row of y}, rows[n].x = where the last row
+// ends; cta: threads of a CTA per row, 0: a warp per row
+struct RowArgs
+{
+    const void *val, *col, *x;
+    void *y;
+    const uint2 *rows;
+    const uint4 *tlbs; // row-grouped, instead: {first element, row of y, TLBs | elements of one << 16, distance of a TLB's elements}
+    unsigned n, cta, lanes; // lanes: of a row with TLBs
+};
+cudaError_t launch_own_rows(int val_is_f64, int col_width, const RowArgs &a, cudaStream_t st);
 } // namespace asp
 #endif

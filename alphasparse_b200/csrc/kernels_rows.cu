@@ -1,0 +1,191 @@
+// Rows by themselves: a warp or a CTA takes a whole row, the formats whose chunks of a row lie one after the other (warp or CTA per row
+// chunk, and chunks with their sums in shared memory), where rows are short enough.
+//
+// What bounds them on matrices of a few microseconds is a chain of dependent loads and the number of launches, not bytes. The chunks'
+// own kernels add up in y by `red`, so y is cleared by a kernel of its own before (1.8 us of the host, 2 us on the device), or they lay out sums in
+// shared memory and look up which rows those belong to behind a barrier. Here an entry of a list says where a row's elements
+// begin and which row of y it is; that, the values and the columns are read before the wait for the kernel before, and then one gather,
+// one reduction and one store are left. Microseconds a call, by chunks / by rows, 40..120 elements a row, random columns, fp64: a warp per row
+// chunk, 600 rows 5.3 / 2.6, 7,003 rows 7.6 / 4.4, 20,000 rows 14.7 / 9.5; chunks in shared memory 5.8 / 2.6, 11.1 / 4.4, 21.2 / 9.5; a CTA per row
+// chunk, 123 rows of 1000..3000 6.4 / 3.8. From about a million non-zeros on, one L2 request a gather is the bound here too.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "kernels.h"
+#include "launch.h"
+
+namespace asp
+{
+typedef unsigned int u32;
+
+namespace
+{
+template <class T>
+__device__ __forceinline__ T ld_once(const T *p)
+{
+    T v;
+    if constexpr (sizeof(T) == 8) asm volatile("ld.global.cs.b64 %0, [%1];" : "=d"(v) : "l"(p));
+    else if constexpr (sizeof(T) == 2)
+    {
+        unsigned short t;
+        asm volatile("ld.global.cs.u16 %0, [%1];" : "=h"(t) : "l"(p));
+        v = (T)t;
+    }
+    else if constexpr (sizeof(T) == 1)
+    {
+        u32 t;
+        asm volatile("ld.global.cs.u8 %0, [%1];" : "=r"(t) : "l"(p));
+        v = (T)t;
+    }
+    else
+    {
+        u32 t;
+        asm volatile("ld.global.cs.u32 %0, [%1];" : "=r"(t) : "l"(p));
+        v = *reinterpret_cast<const T *>(&t);
+    }
+    return v;
+}
+template <class VT>
+__device__ __forceinline__ VT warp_total(VT v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// a thread's part of the row [begin, end): elements begin + t, begin + t + step, ..., four at a time; behind the end the last element is
+// read again and left out. `wait` is called by every thread whose row has elements, before its first gather.
+template <class VT, class CT, class W>
+__device__ __forceinline__ VT row_part(const RowArgs &a, u32 begin, u32 end, u32 t, u32 step, W &wait)
+{
+    constexpr int U = 4;
+    const VT *const val = (const VT *)a.val, *const x = (const VT *)a.x;
+    const CT *const col = (const CT *)a.col;
+    VT sum = 0;
+    for (u32 base = begin; base < end; base = end - base > U * step ? base + U * step : end)
+    {
+        const u32 left = end - base - 1; // of the elements from `base` on, the last one
+        CT c[U];
+        VT v[U], p[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) c[u] = ld_once(col + base + min(t + u * step, left));
+#pragma unroll
+        for (int u = 0; u < U; u++) v[u] = ld_once(val + base + min(t + u * step, left));
+        wait();
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = ld_x(x + c[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = t + u * step <= left ? v[u] * p[u] : VT(0);
+        sum += (p[0] + p[1]) + (p[2] + p[3]);
+    }
+    return sum;
+}
+
+template <class VT, class CT>
+__global__ void __launch_bounds__(256) k_row_warp(RowArgs a)
+{
+    const u32 lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    WaitOnce wait;
+    if (w < a.n)
+    {
+        const uint2 r = __ldg(a.rows + w);
+        const u32 end = __ldg(&a.rows[w + 1].x);
+        const VT s = warp_total(row_part<VT, CT>(a, r.x, end, lane, 32, wait));
+        wait();
+        if (lane == 0) ((VT *)a.y)[r.y] = s;
+    }
+    wait();
+}
+
+// Row-grouped: G lanes take a row, each one TLB of it (whose elements are e.w apart; the TLBs of neighbouring rows lie side by side). By
+// strips, where a CTA takes 32 to 128 rows and its sums go through shared memory / by rows: 4,096 rows of 16 elements, fp32, 3.15 / 2.7 us, 78,000 rows of
+// 5 6.5 / 4.9, fp64 8.4 / 4.6, 50,000 rows of 16 7.0 / 4.9. (Reading the rows' offsets before the wait in the strips' kernel: 3.17 -> 3.23.) G is the least that takes an average row at once: 2 to 32.
+template <class VT, class CT, int G>
+__global__ void __launch_bounds__(128) k_row_tlbs(RowArgs a)
+{
+    constexpr int U = 4;
+    const VT *const val = (const VT *)a.val, *const x = (const VT *)a.x;
+    const CT *const col = (const CT *)a.col;
+    const u32 t = blockIdx.x * blockDim.x + threadIdx.x, g = t / G, sub = t % G;
+    WaitOnce wait;
+    VT s = 0;
+    u32 row = 0;
+    if (g < a.n)
+    {
+        const uint4 e = __ldg(a.tlbs + g);
+        const u32 n = e.z & 0xffffu, size = e.z >> 16;
+        row = e.y;
+        for (u32 i = sub; i < n; i += G)
+            for (u32 k = 0; k < size; k += U)
+            {
+                CT c[U];
+                VT v[U], p[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) c[u] = ld_once(col + e.x + i + min(k + u, size - 1) * e.w);
+#pragma unroll
+                for (int u = 0; u < U; u++) v[u] = ld_once(val + e.x + i + min(k + u, size - 1) * e.w);
+                wait();
+#pragma unroll
+                for (int u = 0; u < U; u++) p[u] = ld_x(x + c[u]);
+#pragma unroll
+                for (int u = 0; u < U; u++) p[u] = k + u < size ? v[u] * p[u] : VT(0);
+                s += (p[0] + p[1]) + (p[2] + p[3]);
+            }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    wait();
+    if (g < a.n && sub == 0) ((VT *)a.y)[row] = s;
+}
+
+template <class VT, class CT>
+__global__ void __launch_bounds__(1024) k_row_cta(RowArgs a)
+{
+    __shared__ VT part[32];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const uint2 r = __ldg(a.rows + blockIdx.x);
+    const u32 end = __ldg(&a.rows[blockIdx.x + 1].x);
+    WaitOnce wait;
+    VT s = warp_total(row_part<VT, CT>(a, r.x, end, threadIdx.x, blockDim.x, wait));
+    wait();
+    if (lane == 0) part[warp] = s;
+    __syncthreads();
+    if (warp != 0) return;
+    s = warp_total(lane < warps ? part[lane] : VT(0));
+    if (lane == 0) ((VT *)a.y)[r.y] = s;
+}
+
+template <class VT, class CT>
+cudaError_t launch(const RowArgs &a, cudaStream_t st)
+{
+    const auto tlbs = [&](auto kernel, u32 lanes) { return launch_pdl(kernel, dim3((unsigned)(((unsigned long long)a.n * lanes + 127) / 128)), dim3(128), 0, st, a); };
+    switch (a.tlbs ? a.lanes : 0)
+    {
+    case 2: return tlbs(k_row_tlbs<VT, CT, 2>, 2);
+    case 4: return tlbs(k_row_tlbs<VT, CT, 4>, 4);
+    case 8: return tlbs(k_row_tlbs<VT, CT, 8>, 8);
+    case 16: return tlbs(k_row_tlbs<VT, CT, 16>, 16);
+    case 32: return tlbs(k_row_tlbs<VT, CT, 32>, 32);
+    default: break;
+    }
+    if (a.tlbs) return cudaErrorInvalidValue;
+    if (a.cta == 0) return launch_pdl(k_row_warp<VT, CT>, dim3((a.n + 7) / 8), dim3(256), 0, st, a);
+    return launch_pdl(k_row_cta<VT, CT>, dim3(a.n), dim3(a.cta), 0, st, a);
+}
+template <class VT>
+cudaError_t launch_v(int col_width, const RowArgs &a, cudaStream_t st)
+{
+    switch (col_width)
+    {
+    case 1: return launch<VT, unsigned char>(a, st);
+    case 2: return launch<VT, unsigned short>(a, st);
+    case 4: return launch<VT, u32>(a, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+} // namespace
+
+cudaError_t launch_own_rows(int val_is_f64, int col_width, const RowArgs &a, cudaStream_t st)
+{
+    return val_is_f64 ? launch_v<double>(col_width, a, st) : launch_v<float>(col_width, a, st);
+}
+} // namespace asp

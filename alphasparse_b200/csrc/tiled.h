@@ -52,6 +52,8 @@ struct TiledSource
     uint64_t stored = 0; // padded non-zeros
     uint64_t true_nnz = 0;
     unsigned threads = 0; // of a CTA of the template's own kernel
+    bool whole_rows = false; // runs the kernels that take whole rows (kernels_rows.cu), in so many trips of a warp:
+    uint64_t trips = 0;
 };
 
 template <class T>

@@ -1,0 +1,66 @@
+"""GPU: the kernels that take whole rows of the templates whose chunks of a row lie one after the other (csrc/kernels_rows.cu), against
+the CPU oracle: rows that end on, before and behind a trip of a warp, a CTA or a row's lanes, the longest rows that they take and one element
+more, empty rows, one row, sorted rows, every column width, x and y off 16-byte alignment, every clearing mode."""
+import numpy as np
+import pytest
+
+import refdump
+from alphasparse_b200 import matrices as M, tuner
+
+pytestmark = pytest.mark.gpu
+
+NODES = {"K4": ["wlb_col_fixed 64"], "K7": ["blb_col_fixed 256"], "K8": ["row_padding 4 1", "blb_row_evenly 4", "wlb_col_fixed 64"],
+         "K6": ["row_padding 32 1", "blb_row_evenly 32", "tlb_col_fixed 4"]}
+
+def matrix(lengths, cols, dtype):
+    """Rows of exactly these lengths."""
+    rng = np.random.default_rng(len(lengths))
+    indices = np.concatenate([np.sort(rng.choice(cols, size=n, replace=False)) for n in lengths]).astype(np.uint32)
+    values = rng.uniform(-1, 1, size=indices.size).astype(dtype)
+    return M.CsrMatrix(len(lengths), cols, np.concatenate([[0], np.cumsum(lengths)]).astype(np.int64), indices, values), rng.uniform(-1, 1, size=cols).astype(dtype)
+
+
+EDGES = [1, 2, 31, 32, 33, 63, 64, 65, 127, 128, 129, 130, 255, 256, 257, 500]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("template,lengths,cols,dense,whole", [
+    ("K4", EDGES + [512], 5_000, "dense compress", True),
+    ("K4", EDGES + [513], 5_000, "dense compress", False),           # a warp takes 512 elements and no more
+    ("K4", [3] * 1000 + [200], 256, "dense compress", True),         # 8-bit columns
+    ("K4", [70], 90, "dense compress", True),
+    ("K8", EDGES * 5, 60_000, "dense compress", True),               # 16-bit columns
+    ("K8", EDGES + [0, 9, 0, 0, 77], 70_000, "dense compress", None),  # rows without elements
+    ("K8", EDGES * 3, 2_000, "dense sort 1\ndense compress", True),
+    ("K7", [1000, 1, 4095, 4096, 4097, 300, 16383], 40_000, "dense compress", True),
+    ("K7", [16384, 3, 9000], 40_000, "dense compress", True),
+    ("K7", [16385, 9000], 40_000, "dense compress", False),
+    ("K7", [700] * 400 + [1023, 1024, 1025, 0], 70_000, "dense compress", None),  # (more rows than the device holds at once)
+    ("K6", [1, 2, 3, 4, 5, 8, 9, 15, 16, 17, 31, 32, 33] * 9, 3_000, "dense compress", True),
+    ("K6", [1] * 500 + [4], 200, "dense compress", True),            # 8-bit columns, two lanes a row
+    ("K6", [40, 41, 119, 120, 121] * 50, 70_000, "dense compress", True),
+    ("K6", [120, 7, 64, 65] * 40, 9_000, "dense sort 1\ndense compress", True),
+    ("K6", [4] * 999 + [4 * 16 + 1], 3_000, "dense compress", False)])  # seventeen TLBs in a row, two lanes: eight trips and one
+def test_whole_rows_match_the_oracle(asp_ctx, template, lengths, cols, dense, whole, dtype):
+    import torch
+
+    m, x = matrix(lengths, cols, dtype)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": dense.replace("\n", " | "), "subs": [{"graph": template, "nodes": NODES[template], "template": template, "threads": 128, "row_reduce": 1}]})
+    assert g.layout_bytes() == 0 and (whole is None or g.whole_rows() == whole)
+    y_ref, scale = refdump.csr_ref(m, x)
+    for shift in (0, 1):
+        dx = torch.zeros(m.n_cols + shift, dtype=torch.from_numpy(x).dtype, device="cuda")
+        dx[shift:] = torch.from_numpy(x).cuda()
+        dy = torch.full((m.n_rows + 3 + shift,), 7.0, dtype=dx.dtype, device="cuda")
+        modes = [True, "auto", False] if min(lengths) > 0 else [True]  # (rows that nobody stores are the caller's to clear)
+        for zero_y in modes:
+            if zero_y is False:  # the templates add to y or overwrite it: both to a cleared one
+                dy[shift : shift + m.n_rows] = 0
+            torch.cuda.synchronize()
+            g.spmv(dx[shift:].data_ptr(), dy[shift:].data_ptr(), zero_y)
+            asp_ctx.synchronize()
+            y = dy.cpu().numpy()
+            refdump.assert_y(y[shift : shift + m.n_rows], y_ref, scale, dtype, f"{template} zero_y={zero_y} shift={shift}")
+            assert (y[:shift] == 7).all() and (y[shift + m.n_rows :] == 7).all()  # nothing beside y
+    g.close()
+    fmt.close()
