@@ -162,6 +162,7 @@ struct asp_plan
     // indices into y; kept on the device for the publishing SpMV (asp_spmv_publish)
     std::shared_ptr<Arena> end_rows;
     uint64_t n_end_rows = 0;
+    long long diag_reach = 0; // diagonal-value template: the furthest column that a row reads, relative to the row
     // templates whose chunks of a row lie one after the other: the rows, for the kernels that take a whole one (kernels_rows.cu)
     std::shared_ptr<Arena> row_list;
     asp::RowArgs own_rows = {};
@@ -1148,6 +1149,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
             else if (d.effective_num == 0 || d.effective_num > NR || d.first_row + d.effective_num > d.n_rows) st = ASP_ERR_BOUNDS, why = "diagonal-value template: rows of the sub-matrix outside y or the padded rows";
             else if (d.sort_kind != ASP_SORT_NONE || d.is_atom_add) st = ASP_ERR_UNSUPPORTED, why = "diagonal-value template: neither sorted nor column-sliced matrices";
             p->units_for_grid = NR / V;
+            p->diag_reach = (long long)(max_entry((const uint64_t *)cols[i]->host_ptr, D) + d.first_col) - (long long)a.n_units;
             break;
         }
         default: st = ASP_ERR_UNSUPPORTED; why = "template not implemented"; break;
@@ -1609,6 +1611,81 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
     return result;
 }
 
+namespace
+{
+// ---- host calls of a plan that stores the rows of y in order (diagonal values): rows run as soon as their x is there, and go to the host
+// from the kernel
+// what the device calls a page-locked host buffer; NULL: it is none
+void *device_view(const void *host)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+}
+bool rows_in_order(asp_plan *const *plans, int n_plans) { return n_plans == 1 && plans[0]->templ == ASP_DIAG_TEMPLATE && plans[0]->stores_all_rows; }
+// rows [r0, r1) of y, r0 a multiple of 4
+cudaError_t launch_in_order(const asp_plan *p, const void *x, void *y, uint64_t r0, uint64_t r1, cudaStream_t st)
+{
+    const uint64_t V = p->val_is_f64 ? 2 : 4, groups = (r1 - r0 + V - 1) / V;
+    asp::KArgs args = p->args;
+    args.x = x;
+    args.y = y;
+    args.first_group = r0 / V;
+    args.effective = std::min<uint64_t>(args.effective, r1);
+    return asp::launch_template(p->templ, p->val_is_f64, p->col_width, args, (unsigned)((groups + p->block - 1) / p->block), p->block, 0, st, p->vec);
+}
+
+struct InOrder
+{
+    asp_ctx *ctx;
+    const asp_plan *plan;
+    void *y;
+    size_t es;
+    cudaStream_t copies;
+    cudaEvent_t arrived;
+    uint64_t done = 0; // rows
+    // x[0, bytes) is on its way on `copies`: the rows that read no further
+    static cudaError_t sent(void *with, size_t bytes)
+    {
+        InOrder &o = *(InOrder *)with;
+        const uint64_t have = bytes / o.es;
+        uint64_t to = o.plan->n_rows;
+        if (have < o.plan->n_cols)
+        {
+            const long long rows = (long long)have - std::max<long long>(0, o.plan->diag_reach);
+            to = rows <= 0 ? 0 : std::min<uint64_t>(to, (uint64_t)rows / 4 * 4);
+        }
+        if (to <= o.done) return cudaSuccess;
+        cudaError_t e = cudaSuccess;
+        if (o.copies != o.ctx->stream)
+        {
+            e = cudaEventRecord(o.arrived, o.copies);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(o.ctx->stream, o.arrived, 0);
+        }
+        if (e == cudaSuccess) e = launch_in_order(o.plan, o.ctx->x, o.y, o.done, to, o.ctx->stream);
+        o.done = to;
+        return e;
+    }
+};
+// streams and events of host calls
+asp_status pipe_ready(asp_ctx *ctx, size_t events)
+{
+    if (!ctx->h2d) ASP_CUDA(cudaStreamCreateWithFlags(&ctx->h2d, cudaStreamNonBlocking));
+    if (!ctx->d2h) ASP_CUDA(cudaStreamCreateWithFlags(&ctx->d2h, cudaStreamNonBlocking));
+    while (ctx->pipe_events.size() < events)
+    {
+        cudaEvent_t e = nullptr;
+        ASP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        ctx->pipe_events.push_back(e);
+    }
+    return ASP_OK;
+}
+} // namespace
+
 asp_status asp_spmv_host(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const void *h_x, void *h_y)
 {
     if (!ctx || !plans || n_plans <= 0 || !h_x || !h_y) return fail(ASP_ERR_INVALID_ARG, "NULL argument");
@@ -1619,6 +1696,36 @@ asp_status asp_spmv_host(asp_ctx *ctx, asp_plan *const *plans, int n_plans, cons
     const size_t xb = g.n_cols * g.es, yb = g.n_rows * g.es;
     st = ensure_xy(ctx, xb, yb);
     if (st != ASP_OK) return st;
+    void *const y_seen = rows_in_order(plans, n_plans) ? device_view(h_y) : nullptr;
+    if (y_seen)
+    {
+        // Pieces of a quarter of x: the last one's rows are all that goes to the host after x has come. (8 MB each way: 338 us; in eighths
+        // 345, eighths and quarters with copies of y behind the kernels 395 and 360.)
+        const size_t piece = std::min<size_t>(4u << 20, std::max<size_t>(896u << 10, (xb / 4 + (64u << 10) - 1) >> 16 << 16));
+        const bool several = xb >= piece + piece / 2;
+        st = several ? pipe_ready(ctx, 1) : ASP_OK;
+        if (st != ASP_OK) return st;
+        InOrder o = {ctx, plans[0], y_seen, g.es, several ? ctx->h2d : ctx->stream, several ? ctx->pipe_events[0] : nullptr};
+        if (several)
+        {
+            // (an earlier SpMV may still read the buffer of x)
+            ASP_CUDA(cudaEventRecord(o.arrived, ctx->stream));
+            ASP_CUDA(cudaStreamWaitEvent(o.copies, o.arrived, 0));
+        }
+        cudaError_t e;
+        if (several) e = ctx->stager.to_device(ctx->x, h_x, xb, o.copies, piece, {InOrder::sent, &o});
+        else
+        {
+            e = ctx->stager.to_device(ctx->x, h_x, xb, ctx->stream);
+            if (e == cudaSuccess) e = InOrder::sent(&o, xb);
+        }
+        // nothing is left in flight when the call returns, also after an error
+        const cudaError_t e1 = several ? cudaStreamSynchronize(o.copies) : cudaSuccess, e2 = cudaStreamSynchronize(ctx->stream);
+        ASP_CUDA(e);
+        ASP_CUDA(e1);
+        ASP_CUDA(e2);
+        return ASP_OK;
+    }
     ASP_CUDA(ctx->stager.to_device(ctx->x, h_x, xb, ctx->stream));
     st = asp_spmv(ctx, plans, n_plans, ctx->x, ctx->y, 1);
     if (st != ASP_OK) return st;
@@ -1653,14 +1760,9 @@ asp_status asp_spmv_host_pipelined(asp_ctx *ctx, const asp_host_chunk *chunks, i
     ASP_ON_DEVICE(ctx);
     asp_status st = ensure_xy(ctx, n_cols * es, n_rows * es);
     if (st != ASP_OK) return st;
-    if (!ctx->h2d) ASP_CUDA(cudaStreamCreateWithFlags(&ctx->h2d, cudaStreamNonBlocking));
-    if (!ctx->d2h) ASP_CUDA(cudaStreamCreateWithFlags(&ctx->d2h, cudaStreamNonBlocking));
-    while (ctx->pipe_events.size() < 2 * (size_t)n_chunks + 1)
-    {
-        cudaEvent_t e = nullptr;
-        ASP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        ctx->pipe_events.push_back(e);
-    }
+    st = pipe_ready(ctx, 2 * (size_t)n_chunks + 1);
+    if (st != ASP_OK) return st;
+    unsigned char *const y_seen = (unsigned char *)device_view(h_y);
     // whatever ran on the context's stream before (an earlier SpMV reading x, writing y) is finished first
     cudaEvent_t start = ctx->pipe_events[2 * (size_t)n_chunks];
     ASP_CUDA(cudaEventRecord(start, ctx->stream));
@@ -1677,6 +1779,15 @@ asp_status asp_spmv_host_pipelined(asp_ctx *ctx, const asp_host_chunk *chunks, i
             uploaded = ch.col_hi;
             ASP_CUDA(cudaEventRecord(x_in, ctx->h2d));
             ASP_CUDA(cudaStreamWaitEvent(ctx->stream, x_in, 0));
+        }
+        // Long chunks go to the host from the kernel (2 MB: 311 -> 287 us for four); short ones are over sooner by a copy (0.7 MB: 139, 148 by
+        // the kernel).
+        if (y_seen && (ch.row_hi - ch.row_lo) * es >= (3u << 19) && rows_in_order(ch.plans, ch.n_plans))
+        {
+            const cudaError_t e = launch_in_order(ch.plans[0], ctx->x, y_seen + ch.row_lo * es, 0, ch.row_hi - ch.row_lo, ctx->stream);
+            if (e == cudaSuccess) continue;
+            st = cuda_fail(e, "kernel launch");
+            break;
         }
         unsigned char *y = (unsigned char *)ctx->y + ch.row_lo * es;
         st = asp_spmv(ctx, ch.plans, ch.n_plans, ctx->x, y, 1);

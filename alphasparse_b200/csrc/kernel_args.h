@@ -66,6 +66,7 @@ struct KArgs
     unsigned long long first_row, first_col;
     unsigned long long n_units;   // #BLB | #WLB | #TLB depending on the template
     unsigned long long n_tlb;     // padded TLB count (k-stride of the ELL-like layout)
+    unsigned long long first_group; // diagonal-value template: groups of rows (16 bytes of them) before this launch's
     unsigned long long effective; // effective_TLB_num | effective_WLB_num | effective_row_num
     unsigned int tlb_size;
     int atomic;

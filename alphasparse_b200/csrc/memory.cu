@@ -272,22 +272,40 @@ cudaError_t Stager::to_device(void *dev, const void *host, size_t bytes, cudaStr
     return to_device(dev, &whole, 1, st);
 }
 
+cudaError_t Stager::to_device(void *dev, const void *host, size_t bytes, cudaStream_t st, size_t piece, const Sent &sent)
+{
+    if (bytes >= (64u << 10) && !pinned(host))
+    {
+        const Segment whole = {0, host, bytes};
+        return to_device(dev, &whole, 1, st, piece, &sent);
+    }
+    cudaError_t e = cudaSuccess;
+    for (size_t o = 0; o < bytes && e == cudaSuccess;)
+    {
+        const size_t n = bytes - o < piece + piece / 2 ? bytes - o : piece;
+        e = cudaMemcpyAsync((unsigned char *)dev + o, (const unsigned char *)host + o, n, cudaMemcpyHostToDevice, st);
+        o += n;
+        if (e == cudaSuccess) e = sent.f(sent.with, o);
+    }
+    return e;
+}
+
 cudaError_t Stager::to_device(void *dev, const std::vector<Segment> &seg, cudaStream_t st) { return to_device(dev, seg.data(), seg.size(), st); }
 
-cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaStream_t st)
+cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaStream_t st, size_t piece, const Sent *sent)
 {
     if (count == 0) return cudaSuccess;
+    const size_t begin = seg[0].off, total = seg[count - 1].off + seg[count - 1].bytes - begin;
     auto plain = [&]() {
         for (size_t i = 0; i < count; i++)
         {
             const cudaError_t e = cudaMemcpyAsync((unsigned char *)dev + seg[i].off, seg[i].host, seg[i].bytes, cudaMemcpyHostToDevice, st);
             if (e != cudaSuccess) return e;
         }
-        return cudaSuccess;
+        return sent ? sent->f(sent->with, total) : cudaSuccess;
     };
     std::lock_guard<std::mutex> turn(one);
     if (!ready()) return plain();
-    const size_t begin = seg[0].off, total = seg[count - 1].off + seg[count - 1].bytes - begin;
     const long long n_parts = (long long)((total + kPart - 1) / kPart);
     if (n_parts <= 3)
     {
@@ -298,10 +316,13 @@ cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaS
         if (e != cudaSuccess) return e;
         gather(p, begin, total, seg, count);
         e = cudaMemcpyAsync((unsigned char *)dev + begin, p, total, cudaMemcpyHostToDevice, st);
-        return e == cudaSuccess ? cudaEventRecord(done[i], st) : e;
+        if (e == cudaSuccess) e = cudaEventRecord(done[i], st);
+        return e == cudaSuccess && sent ? sent->f(sent->with, total) : e;
     }
     // Pieces that double: the filling of the first is all that does not overlap with a copy, and a copy costs 3.5 us by itself
-    // (8 MB on this link: 161 us in one copy, 187 in eight). The ring is filled faster than the link empties it.
+    // (8 MB on this link: 161 us in one copy, 187 in eight). The ring is filled faster than the link empties it. `piece`: of that size
+    // instead, if the ring can hold three.
+    const long long even = (long long)(std::min(piece, kPiece * (kPieces / 4)) / kPart);
     struct Piece
     {
         long long part, end; // parts of 64 KB
@@ -318,7 +339,7 @@ cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaS
     try
     {
         piece_of.resize((size_t)n_parts);
-        for (long long q = 0, n = kFirstParts; q < n_parts; n = std::min(2 * n, kMostParts))
+        for (long long q = 0, n = even > 0 ? even : kFirstParts; q < n_parts; n = even > 0 ? even : std::min(2 * n, kMostParts))
         {
             const long long e = n_parts - q <= n + n / 4 ? n_parts : q + n;
             std::fill(piece_of.begin() + q, piece_of.begin() + e, (int)pieces.size());
@@ -375,6 +396,7 @@ cudaError_t Stager::to_device(void *dev, const Segment *seg, size_t count, cudaS
                 const size_t o = (size_t)q.part * kPart, n = std::min((size_t)(q.end - q.part) * kPart, total - o);
                 e = cudaMemcpyAsync((unsigned char *)dev + begin + o, q.p, n, cudaMemcpyHostToDevice, st);
                 if (e == cudaSuccess) e = cudaEventRecord(done[q.event], st);
+                if (e == cudaSuccess && sent) e = sent->f(sent->with, o + n);
                 open_from(k + 1);
             }
             stop.store(true);

@@ -41,12 +41,12 @@ class Stager
     int next = 0;
 
     bool ready();
-    bool pinned(const void *host);
     // the adjacent slots that the next piece goes through, free to be written, and the event to record after its copy
     cudaError_t take(int slots, unsigned char **p, int *event);
     bool free_now(int slots) const;
 
   public:
+    static bool pinned(const void *host);
     struct Segment
     {
         size_t off;
@@ -56,9 +56,17 @@ class Stager
     void release();
     // host buffers may be reused as soon as these return, as after a pageable cudaMemcpyAsync
     cudaError_t to_device(void *dev, const void *host, size_t bytes, cudaStream_t st);
+    // the same in pieces of about `piece` bytes; sent.f(sent.with, n) is called when the copies of the first n bytes are on the stream. An
+    // error of it ends the copy.
+    struct Sent
+    {
+        cudaError_t (*f)(void *, size_t);
+        void *with;
+    };
+    cudaError_t to_device(void *dev, const void *host, size_t bytes, cudaStream_t st, size_t piece, const Sent &sent);
     // many arrays of one device block (ascending offsets): as few copies as the pieces make
     cudaError_t to_device(void *dev, const std::vector<Segment> &segments, cudaStream_t st);
-    cudaError_t to_device(void *dev, const Segment *segments, size_t count, cudaStream_t st);
+    cudaError_t to_device(void *dev, const Segment *segments, size_t count, cudaStream_t st, size_t piece = 0, const Sent *sent = nullptr);
     // complete on return
     cudaError_t to_host(void *host, const void *dev, size_t bytes, cudaStream_t st);
 };

@@ -1,0 +1,55 @@
+"""GPU: host calls of the diagonal-value template, whose rows run as soon as their x has arrived and go to the host from the kernel: around
+the sizes of a piece of x, diagonals that reach back, ahead, far ahead or not at all, more rows than columns and fewer, x and y page-locked or not."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import refdump
+from alphasparse_b200 import capi, matrices as M
+from alphasparse_b200.graph import Matrix
+
+pytestmark = pytest.mark.gpu
+
+PIECE = 896 << 10
+
+
+def banded(n_rows, n_cols, offsets, seed, dtype):
+    rng = np.random.default_rng(seed)
+    r = np.repeat(np.arange(n_rows, dtype=np.int64), len(offsets))
+    c = r + np.tile(np.sort(np.array(offsets, dtype=np.int64)), n_rows)
+    keep = (c >= 0) & (c < n_cols)
+    indptr = np.concatenate([[0], np.cumsum(np.bincount(r[keep], minlength=n_rows))]).astype(np.int64)
+    values = rng.uniform(-1, 1, size=int(keep.sum())).astype(dtype)
+    return M.CsrMatrix(n_rows, n_cols, indptr, c[keep].astype(np.uint32), values), rng.uniform(-1, 1, size=n_cols).astype(dtype)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("rows,cols,offsets", [
+    (1, 1, [0]), (7, 7, [-1, 0, 1]), (1000, 1003, [-1, 0, 3]),
+    ("piece", 0, [-3, 0, 2]), ("piece*3/2", -1, [-300, 0, 300]), ("piece*3/2", 0, [-300, 0, 300]), ("piece*3/2", 1, [-1, 0, 1]),
+    ("piece*4", 5, [0]), ("piece*4", 0, [-70000, -5, 0]), ("piece*4", -3, [-1, 0, 200000]), ("piece*5", 130000, [0, 130000]),
+    ("piece*9", 1, [-2048, -1, 0, 1, 2048])])
+def test_host_call_matches_the_oracle(asp_ctx, rows, cols, offsets, dtype):
+    import torch
+
+    es = np.dtype(dtype).itemsize
+    n = eval(rows.replace("piece", str(PIECE)).replace("/", "//")) // es if isinstance(rows, str) else rows
+    m, x = banded(n if isinstance(rows, str) else rows, n + cols if isinstance(rows, str) else cols, offsets, 3, dtype)
+    fmt = Matrix.from_csr(m).execute("dense compress\nsub all diag_value 64\nsub all template D1")
+    g = fmt.upload(asp_ctx)
+    y_ref, scale = refdump.csr_ref(m, x)
+    xp = torch.from_numpy(x).pin_memory().numpy()
+    for name, hx in (("pageable", x), ("pinned", xp)):
+        for again in range(2):  # (a second call finds the buffers as the first left them)
+            refdump.assert_y(g.spmv_host(hx), y_ref, scale, dtype, f"{name} x, page-locked y, call {again}")
+        y = np.full(m.n_rows, 7, dtype=dtype)  # pageable
+        capi.check(capi.lib().asp_spmv_host(asp_ctx.handle, g._plans, g.n, C.c_void_p(hx.ctypes.data), C.c_void_p(y.ctypes.data)))
+        refdump.assert_y(y, y_ref, scale, dtype, f"{name} x, pageable y")
+    # nothing beside y
+    yp = torch.full((m.n_rows + 9,), 7.0, dtype=torch.from_numpy(x).dtype).pin_memory()
+    capi.check(capi.lib().asp_spmv_host(asp_ctx.handle, g._plans, g.n, C.c_void_p(x.ctypes.data), C.c_void_p(yp.data_ptr() + 3 * es)))
+    refdump.assert_y(yp.numpy()[3 : 3 + m.n_rows], y_ref, scale, dtype, "page-locked y off its alignment")
+    assert (yp[:3] == 7).all() and (yp[3 + m.n_rows :] == 7).all()
+    g.close()
+    fmt.close()
