@@ -267,9 +267,9 @@ __global__ void __launch_bounds__(512) k_ell(KArgs a)
     const u64 ngroup = P / V;
     const u64 stride = (u64)gridDim.x * blockDim.x;
     const u64 radd = a.row_add ? a.first_row : 0;
-    // consecutive TLBs map to consecutive rows: whole groups can be stored as vectors
+    // consecutive TLBs map to consecutive rows: whole groups can be stored as vectors (where y itself lies on 16 bytes)
     const bool unit_rows = a.m[MS_ROW_OF_TLB].kind == MK_LINEAR && a.m[MS_ROW_OF_TLB].coef == 1 && !a.atomic &&
-                           ((a.m[MS_ROW_OF_TLB].icpt + radd) % V) == 0;
+                           ((a.m[MS_ROW_OF_TLB].icpt + radd) % V) == 0 && ((uintptr_t)y & 15) == 0;
     WaitOnce wait; // the first values and indices are on their way when it waits
     for (u64 g = (u64)blockIdx.x * blockDim.x + threadIdx.x; g < ngroup; g += stride)
     {
@@ -370,7 +370,7 @@ template <class VT, int V>
 __device__ __forceinline__ void sell_store(const KArgs &a, VT *__restrict__ y, const VT (&acc)[V], u64 t0, u64 radd)
 {
     const Meta &rm = a.m[MS_ROW_OF_TLB];
-    if (V > 1 && rm.kind == MK_LINEAR && rm.coef == 1 && !a.atomic && t0 + V <= a.effective && ((t0 + rm.icpt + radd) % V) == 0)
+    if (V > 1 && rm.kind == MK_LINEAR && rm.coef == 1 && !a.atomic && t0 + V <= a.effective && ((t0 + rm.icpt + radd) % V) == 0 && ((uintptr_t)y & 15) == 0)
     {
         store_rows<VT, V>(y, t0 + rm.icpt + radd, acc);
         return;
