@@ -562,8 +562,82 @@ bool list_tlb_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, cons
     return !out.empty();
 }
 
+// The same of the ELL- and SELL-like templates; `place` stays empty where TLB t is row first + t. `longest` TLB, `rows` that are stored.
+bool list_strips(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const asp::KArgs &a, std::vector<uint4> &out, std::vector<unsigned> &place, uint64_t &first, uint64_t &longest, uint64_t &rows)
+{
+    using namespace asp;
+    const bool ell = d.template_type == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS;
+    if ((!ell && d.template_type != ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS) || d.n_rows > 0xffffffffull) return false;
+    const HostMeta &of = hm[MS_ROW_OF_TLB];
+    const uint64_t radd = a.row_add ? d.first_row : 0;
+    const bool numbered = of.kind == ASP_COMPRESS_LINEAR && of.coef == 1;
+    longest = rows = 0;
+    first = numbered ? of.icpt + radd : 0;
+    std::vector<bool> seen(numbered ? 0 : d.n_rows, false);
+    for (uint64_t b = 0; b < (ell ? 1 : a.n_units); b++)
+    {
+        const uint64_t nz = ell ? 0 : hm[MS_BLK_NZ].get(b), t0 = ell ? 0 : hm[MS_BLK_THR].get(b);
+        const uint64_t n = ell ? a.n_tlb : hm[MS_BLK_THR].get(b + 1) - t0, S = ell ? a.tlb_size : hm[MS_TLB_SIZE].get(b);
+        if (S == 0 || S > 0xffff || nz + n * S > 0xffffffffull || t0 != rows) return false;
+        longest = std::max(longest, S);
+        for (uint64_t t = t0; t < t0 + n && t < a.effective; t += 32)
+        {
+            const uint64_t m = std::min<uint64_t>({32, t0 + n - t, a.effective - t});
+            out.push_back(make_uint4((unsigned)(nz + t - t0), (unsigned)t, (unsigned)(S | m << 16), (unsigned)n));
+            for (uint64_t i = t; !numbered && i < t + m; i++)
+            {
+                const uint64_t row = of.get(i) + radd;
+                if (row >= d.n_rows || seen[row]) return false;
+                seen[row] = true;
+                place.push_back((unsigned)row);
+            }
+            rows += m;
+        }
+    }
+    return !out.empty() && first + (numbered ? rows : 0) <= d.n_rows;
+}
+
+// The same of the CSR5-like templates: {first element, row, elements, 0}
+bool list_runs(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, std::vector<uint4> &out)
+{
+    using namespace asp;
+    if ((d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE && d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE) ||
+        d.n_rows > 0xffffffffull)
+        return false;
+    std::vector<bool> seen(d.n_rows, false);
+    const uint64_t S = a.tlb_size, rmask = (1ull << a.bits_row) - 1;
+    if (S == 0 || S >= 64) return false;
+    uint64_t r = ~0ull; // of the matrix's rows in order
+    for (uint64_t w = 0; w < a.n_units; w++)
+    {
+        const uint64_t R0 = hm[MS_ROW_OF_UNIT].get(w);
+        for (uint64_t l = 0; l < 32; l++)
+        {
+            const uint64_t word = hm[MS_COMBINE].get(w * 32 + l), e0 = (w * 32 + l) * S;
+            uint64_t next = R0 + (word & rmask);
+            if (l == 0 && !((word >> (a.bits_word - 1)) & 1ull)) return false; // (a warp's first element always starts a row)
+            // the flags, first element first, at the top of the word
+            for (uint64_t f = word >> (a.bits_word - (int)S) << (64 - S); f != 0; f &= ~(1ull << (63 - __builtin_clzll(f))), next++)
+            {
+                const uint64_t e = e0 + (uint64_t)__builtin_clzll(f);
+                if (next == r) continue; // goes on from the warp before
+                r = next;
+                const uint64_t row = a.sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : a.sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
+                if (row >= d.n_rows || seen[row]) return false;
+                seen[row] = true;
+                if (!out.empty()) out.back().z = (unsigned)(e - out.back().x);
+                out.push_back(make_uint4((unsigned)e, (unsigned)row, 0, 0));
+            }
+        }
+    }
+    if (!out.empty()) out.back().z = (unsigned)(a.n_units * 32 * S - out.back().x);
+    return !out.empty();
+}
+
 // Whole rows for a few lanes, a warp or a CTA, where that is the faster way (kernels_rows.cu). A warp takes up to 512 elements (four trips
 // of 1.2 us; chunks in parallel are faster beyond that), a CTA rows of 256 and more on average, up to 16384 (four trips of 1024 threads).
+// Rows that are TLBs of more than 8 elements: up to 3 M elements (what L2 holds). CSR5-like: up to 512 K elements (FEM, fp32: 445 K 6 -> 3.1 us, 730 K
+// 6.5 -> 5.1, but lists of a million elements cost more to make than that is worth) and rows of 4096 (four trips of a CTA).
 // Rows of TLBs: up to 2 M elements, beyond which the CTA's long strips stream better (4.9 M, FEM, fp32: 13.0 us, 17.3 by rows; 1.6 M: 7.2, 5.1).
 struct OwnRows
 {
@@ -571,17 +645,46 @@ struct OwnRows
     std::vector<uint2> rows;
     std::vector<uint4> tlbs;
     uint64_t trips = 0; // of warps that take a row
+    bool strips = false, runs = false; // (in `tlbs`)
+    std::vector<unsigned> place;
+    uint64_t listed = 0; // rows of y
     const void *data() const { return tlbs.empty() ? (const void *)rows.data() : tlbs.data(); }
     size_t bytes() const { return rows.size() * sizeof(uint2) + tlbs.size() * sizeof(uint4); }
     void make(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp_plan &p, int sm_count)
     {
         uint64_t longest = 0, all = 0;
+        if (list_strips(d, hm, p.args, tlbs, place, all, longest, listed))
+        {
+            strips = true;
+            args.first_row = (unsigned)all;
+            args.lanes = longest <= 16 ? 4 : longest <= 32 ? 8 : 16;
+            args.n = (unsigned)tlbs.size();
+            if (longest <= 8 || p.stored > (3u << 20)) tlbs.clear();
+            return;
+        }
+        tlbs.clear();
+        if (p.stored <= (1u << 19) && list_runs(d, hm, perm, p.args, tlbs))
+        {
+            runs = true;
+            args.size = p.args.tlb_size;
+            args.n = (unsigned)tlbs.size();
+            listed = args.n;
+            args.lanes = p.stored <= 6 * listed ? 4 : p.stored <= 12 * listed ? 8 : 16;
+            // rows that take its lanes more than two trips are a CTA's
+            const auto first = std::stable_partition(tlbs.begin(), tlbs.end(), [&](const uint4 &r) { return r.z > 8 * args.lanes; });
+            args.hubs = (unsigned)(first - tlbs.begin());
+            for (const uint4 &r : tlbs) longest = std::max<uint64_t>(longest, r.z);
+            if (longest > 4096) tlbs.clear();
+            return;
+        }
+        tlbs.clear();
         if (d.template_type == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS)
         {
             args.lanes = 2;
             bool good = p.stored <= (2u << 20) && list_tlb_rows(d, hm, perm, p.args, tlbs, all, longest);
             while (args.lanes < 32 && args.lanes * tlbs.size() < all) args.lanes *= 2;
             args.n = (unsigned)tlbs.size();
+            listed = tlbs.size();
             if (!good || longest > 8 * args.lanes) tlbs.clear();
             return;
         }
@@ -592,6 +695,7 @@ struct OwnRows
         const uint64_t per = n <= 2ull * sm_count ? 4 : 8;
         args.cta = longest <= 512 ? 0 : (unsigned)std::min<uint64_t>(1024, std::max<uint64_t>(64, (longest + 32 * per - 1) / (32 * per) * 32));
         args.n = (unsigned)n;
+        listed = n;
         for (uint64_t i = 0; i < n && args.cta == 0; i++) trips += (rows[i + 1].x - rows[i].x + 127) / 128;
     }
 };
@@ -1286,9 +1390,11 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
     {
         asp_plan *const p = made[0];
         std::shared_ptr<Arena> list(new (std::nothrow) Arena());
-        if (list && list->make(ctx->device, own.bytes()) == cudaSuccess)
+        const size_t places = align_up(own.bytes(), 256);
+        if (list && list->make(ctx->device, places + own.place.size() * sizeof(unsigned)) == cudaSuccess)
         {
-            const cudaError_t ce = ctx->stager.to_device(list->base, own.data(), own.bytes(), ctx->stream);
+            cudaError_t ce = ctx->stager.to_device(list->base, own.data(), own.bytes(), ctx->stream);
+            if (ce == cudaSuccess && !own.place.empty()) ce = ctx->stager.to_device((char *)list->base + places, own.place.data(), own.place.size() * sizeof(unsigned), ctx->stream);
             if (ce != cudaSuccess)
             {
                 cleanup();
@@ -1297,8 +1403,9 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
             p->own_rows = own.args;
             p->own_rows.val = p->args.val;
             p->own_rows.col = p->args.col;
-            (own.tlbs.empty() ? (const void *&)p->own_rows.rows : (const void *&)p->own_rows.tlbs) = list->base;
-            p->own_rows_cover = own.args.n == descs[0].n_rows;
+            (own.strips ? (const void *&)p->own_rows.strips : own.runs ? (const void *&)p->own_rows.runs : own.tlbs.empty() ? (const void *&)p->own_rows.rows : (const void *&)p->own_rows.tlbs) = list->base;
+            if (!own.place.empty()) p->own_rows.place = (const unsigned *)((char *)list->base + places);
+            p->own_rows_cover = own.listed == descs[0].n_rows;
             p->row_list = list;
         }
         else cudaGetLastError(); // no room: the chunks' own kernels

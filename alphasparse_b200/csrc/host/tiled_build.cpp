@@ -163,8 +163,9 @@ void walk_any(const TiledSource &s, u64 u0, u64 u1, F &&f)
 // Sampled; the kernels with 16-byte lanes gather elements 4 l + j of 128 adjacent ones at a time, the others 32 adjacent ones.
 double lines_per_gather(const TiledSource &s, bool f64)
 {
-    const bool by4 = s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS ||
-                     s.templ == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || s.templ == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE;
+    // (and so do those for whole rows)
+    const bool by4 = !s.whole_rows && (s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS || s.templ == ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS ||
+                     s.templ == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || s.templ == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE);
     const u64 groups = s.stored / 128, samples = std::min<u64>(groups, 64), per_line = f64 ? 16 : 32;
     if (samples == 0) return 0.0;
     u64 lines = 0;
@@ -798,6 +799,7 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
         bytes_us += (double)s.stored * slow * (sv + 4) / 6.0e6;
     }
     auto own = [&](double lines) {
+        if (whole && is_csr5(src[0])) return 0.0; // (small ones: 2.6 to 5 us)
         if (whole) return std::max(2.9, 1.7 + std::max({lines / (0.75 * 290e3), bytes_us * 6.0 / 4.6, src[0].trips * 0.14e-3 + 0.45 * bytes_us * 6.0 / 4.6}));
         const double rate = std::max(lines / (0.85 * 290e3), bytes_us);
         return (src.size() > 1 ? 8.0 : 0.0) + std::max(2.0 + chain, 3.0 + rate + std::min(0.4 * rate, 4.5));

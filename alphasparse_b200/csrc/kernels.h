@@ -32,7 +32,13 @@ struct RowArgs
     void *y;
     const uint2 *rows;
     const uint4 *tlbs; // row-grouped, instead: {first element, row of y, TLBs | elements of one << 16, distance of a TLB's elements}
-    unsigned n, cta, lanes; // lanes: of a row with TLBs
+    const uint4 *strips; // ELL- and SELL-like, instead: groups of up to 32 TLBs side by side, a TLB a row: {first element, first TLB, elements of a TLB |
+                         // TLBs << 16, distance of a TLB's elements}; `place` rows of y by TLB (NULL: as numbered, from first_row on)
+    const unsigned *place;
+    unsigned first_row;
+    const uint4 *runs; // CSR5-like, instead: {first element, row of y, elements, 0}, the first `hubs` of them for a CTA each; TLBs of `size`
+    unsigned hubs, size;
+    unsigned n, cta, lanes; // lanes: of a row with TLBs; warps of a group of them
 };
 cudaError_t launch_own_rows(int val_is_f64, int col_width, const RowArgs &a, cudaStream_t st);
 } // namespace asp

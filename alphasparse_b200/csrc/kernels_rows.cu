@@ -137,6 +137,109 @@ __global__ void __launch_bounds__(128) k_row_tlbs(RowArgs a)
     if (g < a.n && sub == 0) ((VT *)a.y)[row] = s;
 }
 
+// ELL- and SELL-like: 32 rows side by side, of whose TLBs W warps take every W-th element, so that a TLB of up to 4 W is one trip instead of a
+// trip for every four. W is 4, 8 or 16 (TLBs of up to 16, up to 32, more). A row a thread, four TLBs a thread / by W warps, finite elements: 7,500 rows
+// of 27, fp64, SELL 9.5 us / 2.5, ELL 7.7 / 2.5; 60,000 rows of 27 11.5 / 4.9, 9.2 / 5.0; 30,000 rows of 60 24 / 5.2, 20 / 5.3 (the column-tiled layout
+// 8.5, and it takes 3 ms to build). Beyond what L2 holds the longer streams of the others win: 60,000 rows of 81, fp64, layout 14.6, this 16.0.
+template <class VT, class CT, int W>
+__global__ void __launch_bounds__(32 * W) k_row_strips(RowArgs a)
+{
+    constexpr int U = 4;
+    __shared__ VT part[W][32];
+    const VT *const val = (const VT *)a.val, *const x = (const VT *)a.x;
+    const CT *const col = (const CT *)a.col;
+    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint4 e = __ldg(a.strips + blockIdx.x);
+    const u32 size = e.z & 0xffffu, n = e.z >> 16;
+    const bool on = lane < n;
+    u32 row = a.first_row + e.y + lane;
+    if (a.place && on) row = __ldg(a.place + e.y + lane);
+    WaitOnce wait;
+    VT s = 0;
+    for (u32 k = w; k < size; k += U * W)
+    {
+        CT c[U];
+        VT v[U], p[U];
+        const u32 at = e.x + (on ? lane : 0u);
+#pragma unroll
+        for (int u = 0; u < U; u++) c[u] = ld_once(col + at + min(k + u * W, size - 1) * e.w);
+#pragma unroll
+        for (int u = 0; u < U; u++) v[u] = ld_once(val + at + min(k + u * W, size - 1) * e.w);
+        wait();
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = ld_x(x + c[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = k + u * W < size ? v[u] * p[u] : VT(0);
+        s += (p[0] + p[1]) + (p[2] + p[3]);
+    }
+    wait();
+    part[w][lane] = s;
+    __syncthreads();
+    if (w != 0 || !on) return;
+    VT sum[2] = {0, 0};
+#pragma unroll
+    for (int i = 0; i < W; i++) sum[i & 1] += part[i][lane];
+    ((VT *)a.y)[row] = sum[0] + sum[1];
+}
+
+// CSR5-like: element e of the matrix is element e % S of a thread that has S of them one after the other, and a warp's threads lie side by
+// side; G lanes take a row's elements in turn, a CTA a long row's. Neighbouring elements lie 128 bytes apart, so this makes three requests to
+// L2 for each: for small matrices only. Two kernels, y's shared rows cleared and added up / this: R-MAT scale 11 (20,000 elements) 5.4 us an SpMV /
+// 2.7, scale 14 (200,000) 6.1 / 4.1, 22,500 rows of 24 to 27 5.5 to 6 / 3.0. Long rows by their lanes, eight trips instead of two: scale 13 4.4, so 2.9.
+const u32 kRunThreads = 256; // 1024 elements of a long row a trip
+template <class VT, class CT, int G>
+__global__ void __launch_bounds__(kRunThreads) k_row_runs(RowArgs a)
+{
+    constexpr int U = 4;
+    __shared__ VT part[kRunThreads / 32];
+    const VT *const val = (const VT *)a.val, *const x = (const VT *)a.x;
+    const CT *const col = (const CT *)a.col;
+    const bool hub = blockIdx.x < a.hubs;
+    const u32 step = hub ? kRunThreads : (u32)G, sub = hub ? threadIdx.x : threadIdx.x % G;
+    const u32 g = hub ? blockIdx.x : a.hubs + (blockIdx.x - a.hubs) * (kRunThreads / G) + threadIdx.x / G;
+    const u32 S = a.size;
+    uint4 r = make_uint4(0, 0, 0, 0);
+    if (g < a.n) r = __ldg(a.runs + g);
+    WaitOnce wait;
+    VT s = 0;
+    for (u32 i = sub; i < r.z; i += U * step)
+    {
+        u32 at[U];
+        CT c[U];
+        VT v[U], p[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+        {
+            const u32 e = r.x + min(i + u * step, r.z - 1), thread = e / S;
+            at[u] = thread / 32 * (32 * S) + (e - thread * S) * 32 + thread % 32;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) c[u] = ld_once(col + at[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++) v[u] = ld_once(val + at[u]);
+        wait();
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = ld_x(x + c[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++) p[u] = i + u * step < r.z ? v[u] * p[u] : VT(0);
+        s += (p[0] + p[1]) + (p[2] + p[3]);
+    }
+    wait();
+    if (hub)
+    {
+        s = warp_total(s);
+        if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = s;
+        __syncthreads();
+        if (threadIdx.x >= 32) return;
+        s = warp_total(threadIdx.x < kRunThreads / 32 ? part[threadIdx.x] : VT(0));
+        if (threadIdx.x == 0) ((VT *)a.y)[r.y] = s;
+        return;
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (g < a.n && sub == 0) ((VT *)a.y)[r.y] = s;
+}
+
 template <class VT, class CT>
 __global__ void __launch_bounds__(1024) k_row_cta(RowArgs a)
 {
@@ -168,6 +271,17 @@ cudaError_t launch(const RowArgs &a, cudaStream_t st)
     default: break;
     }
     if (a.tlbs) return cudaErrorInvalidValue;
+    if (a.runs)
+    {
+        const auto runs = [&](auto kernel, u32 lanes) { return launch_pdl(kernel, dim3(a.hubs + ((a.n - a.hubs) * lanes + kRunThreads - 1) / kRunThreads), dim3(kRunThreads), 0, st, a); };
+        return a.lanes == 4 ? runs(k_row_runs<VT, CT, 4>, 4) : a.lanes == 8 ? runs(k_row_runs<VT, CT, 8>, 8) : runs(k_row_runs<VT, CT, 16>, 16);
+    }
+    if (a.strips)
+    {
+        if (a.lanes == 4) return launch_pdl(k_row_strips<VT, CT, 4>, dim3(a.n), dim3(128), 0, st, a);
+        if (a.lanes == 8) return launch_pdl(k_row_strips<VT, CT, 8>, dim3(a.n), dim3(256), 0, st, a);
+        return launch_pdl(k_row_strips<VT, CT, 16>, dim3(a.n), dim3(512), 0, st, a);
+    }
     if (a.cta == 0) return launch_pdl(k_row_warp<VT, CT>, dim3((a.n + 7) / 8), dim3(256), 0, st, a);
     return launch_pdl(k_row_cta<VT, CT>, dim3(a.n), dim3(a.cta), 0, st, a);
 }

@@ -10,6 +10,8 @@ from alphasparse_b200 import matrices as M, tuner
 pytestmark = pytest.mark.gpu
 
 NODES = {"K4": ["wlb_col_fixed 64"], "K7": ["blb_col_fixed 256"], "K8": ["row_padding 4 1", "blb_row_evenly 4", "wlb_col_fixed 64"],
+         "K2": ["row_padding 128 1", "blb_row_evenly 128", "tlb_row"], "K3": ["row_padding 32 1", "tlb_row"],
+         "K9": ["tlb_nnz 16"], "K9/5": ["tlb_nnz 5"], "K9/32": ["tlb_nnz 32"], "K10": ["tlb_nnz 8"], "K10/3": ["tlb_nnz 3"],
          "K6": ["row_padding 32 1", "blb_row_evenly 32", "tlb_col_fixed 4"]}
 
 def matrix(lengths, cols, dtype):
@@ -40,13 +42,28 @@ EDGES = [1, 2, 31, 32, 33, 63, 64, 65, 127, 128, 129, 130, 255, 256, 257, 500]
     ("K6", [1] * 500 + [4], 200, "dense compress", True),            # 8-bit columns, two lanes a row
     ("K6", [40, 41, 119, 120, 121] * 50, 70_000, "dense compress", True),
     ("K6", [120, 7, 64, 65] * 40, 9_000, "dense sort 1\ndense compress", True),
+    ("K3", [9], 200, "dense compress", True),
+    ("K3", [16] * 33, 3_000, "dense compress", True),                # four warps, one trip; a row in the second group
+    ("K3", [17, 3, 1] * 32, 200, "dense compress", True),            # eight warps, 8-bit columns
+    ("K3", [32, 8, 30] * 11, 70_000, "dense compress", True),
+    ("K3", [33] * 31 + [64, 65, 129], 9_000, "dense compress", True),  # sixteen warps, one to three trips
+    ("K3", [8] * 300, 9_000, "dense compress", False),               # the template's kernel has all of these in flight
+    ("K2", [9] * 128 + [33] * 128 + [90] * 100, 9_000, "dense compress", True),  # strips of different lengths
+    ("K2", [70, 12, 31, 1] * 65, 300, "dense sort 1\ndense compress", True),
+    ("K9", [1], 3, "dense compress", True),
+    ("K9", EDGES * 4, 9_000, "dense compress", True),
+    ("K9/5", [1, 2, 3, 4, 5, 6] * 300 + [159, 160, 161], 9_000, "dense compress", True),
+    ("K9/32", [4096, 1, 2, 3] + [30] * 90, 20_000, "dense compress", True),
+    ("K9", [4097] + [30] * 90, 20_000, "dense compress", None),      # (with what fills the last warp)
+    ("K10", [700, 3, 256, 1, 255] * 9, 3_000, "dense sort 1\ndense compress", True),
+    ("K10/3", [7] * 100 + [57, 33, 32] * 3, 250, "dense compress", True),
     ("K6", [4] * 999 + [4 * 16 + 1], 3_000, "dense compress", False)])  # seventeen TLBs in a row, two lanes: eight trips and one
 def test_whole_rows_match_the_oracle(asp_ctx, template, lengths, cols, dense, whole, dtype):
     import torch
 
     m, x = matrix(lengths, cols, dtype)
-    fmt, g = tuner.build(asp_ctx, m, {"dense": dense.replace("\n", " | "), "subs": [{"graph": template, "nodes": NODES[template], "template": template, "threads": 128, "row_reduce": 1}]})
-    assert g.layout_bytes() == 0 and (whole is None or g.whole_rows() == whole)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": dense.replace("\n", " | "), "subs": [{"graph": template, "nodes": NODES[template], "template": template.split("/")[0], "threads": 128, "row_reduce": 1}]})
+    assert whole is None or (g.layout_bytes() == 0 and g.whole_rows() == whole)
     y_ref, scale = refdump.csr_ref(m, x)
     for shift in (0, 1):
         dx = torch.zeros(m.n_cols + shift, dtype=torch.from_numpy(x).dtype, device="cuda")
