@@ -166,7 +166,8 @@ struct asp_plan
     // templates whose chunks of a row lie one after the other: the rows, for the kernels that take a whole one (kernels_rows.cu)
     std::shared_ptr<Arena> row_list;
     asp::RowArgs own_rows = {};
-    bool own_rows_cover = false; // every row of y is in the list
+    uint64_t own_rows_n = 0;  // rows of y in the list
+    uint64_t rows_group = 0; // plans of one number have no row of y in common
     int64_t asked_tblock = 0, asked_threads = 0, asked_reduce = 0; // the launch last requested (re-applied when vec / path change)
 };
 
@@ -489,149 +490,223 @@ bool stores_every_row(const asp_plan_desc &d, const std::vector<HostMeta> &hm, c
     }
 }
 
-// The rows of a (validated) plan whose chunks of a row are consecutive, as kernels_rows.cu takes them; `longest` of them. false: another
-// template, a row in two places, or offsets beyond 32 bits.
-bool list_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, std::vector<uint2> &out, uint64_t &longest)
+// f(entry of a place): of an array by its type, looked at once
+template <class F>
+void with_entries(const HostMeta &h, F &&f)
+{
+    if (h.kind != ASP_COMPRESS_NONE) f([&h](uint64_t i) { return h.get(i); });
+    else if (h.dtype == ASP_U8) f([p = (const uint8_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
+    else if (h.dtype == ASP_U16) f([p = (const uint16_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
+    else if (h.dtype == ASP_U32) f([p = (const uint32_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
+    else f([p = (const uint64_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
+}
+// Whether rows of y come once each: ascending ones, or a list of what has come
+struct Distinct
+{
+    const uint64_t n;
+    const bool ascending;
+    uint64_t next = 0;
+    std::vector<bool> seen;
+    Distinct(uint64_t rows, bool in_order) : n(rows), ascending(in_order), seen(in_order ? 0 : rows, false) {}
+    bool operator()(uint64_t row)
+    {
+        if (row >= n || (ascending ? row < next : (bool)seen[row])) return false;
+        if (ascending) next = row + 1;
+        else seen[row] = true;
+        return true;
+    }
+};
+uint64_t row_in_y(const asp_plan_desc &d, const HostMeta &perm, int sort_kind, uint64_t r)
+{
+    return sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
+}
+const uint64_t kSharedRows = 1u << 14; // from so many on, the rows of a list are shared out
+
+// Lists of the rows of a (validated) plan, as the kernels of kernels_rows.cu take them. false: another template, a row in two places, or offsets
+// beyond 32 bits.
+//
+// Chunks of a row one after the other, `longest` row
+bool list_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, asp::HostBuf<uint2> &out, uint64_t &longest)
 {
     using namespace asp;
-    const bool chunks = d.template_type == ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE || d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE;
+    const bool cta = d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE, chunks = cta || d.template_type == ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE;
     if ((!chunks && d.template_type != ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE) || d.n_rows > 0xffffffffull) return false;
-    std::vector<bool> seen(d.n_rows, false);
-    uint64_t end = 0;
+    Distinct distinct(d.n_rows, d.sort_kind == ASP_SORT_NONE);
+    const HostMeta &offsets = hm[cta ? MS_BLK_NZ : MS_WARP_NZ];
+    out.make(d.n_rows + 1);
+    uint64_t end = 0, n = 0;
     longest = 0;
     auto put = [&](uint64_t row, uint64_t from, uint64_t to) {
-        if (to < from || to > 0xffffffffull || row >= d.n_rows || seen[row] || (!out.empty() && from != end)) return false;
-        seen[row] = true;
+        if (to < from || to > 0xffffffffull || (n > 0 && from != end) || !distinct(row)) return false;
         end = to;
         longest = std::max(longest, to - from);
-        out.push_back(make_uint2((unsigned)from, (unsigned)row));
+        out.p[n++] = make_uint2((unsigned)from, (unsigned)row);
         return true;
     };
+    bool good = true;
     if (chunks)
-    {
-        const HostMeta &nz = hm[d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE ? MS_BLK_NZ : MS_WARP_NZ], &of = hm[MS_ROW_OF_UNIT];
-        const uint64_t n = d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE ? a.n_units : a.effective, radd = a.row_add ? d.first_row : 0;
-        for (uint64_t u = 0; u < n;)
-        {
-            uint64_t e = u + 1;
-            const uint64_t row = of.get(u);
-            while (e < n && of.get(e) == row) e++;
-            if (!put(row + radd, nz.get(u), nz.get(e))) return false;
-            u = e;
-        }
-    }
+        with_entries(hm[MS_ROW_OF_UNIT], [&](auto of) {
+            with_entries(offsets, [&](auto nz) {
+                const uint64_t units = cta ? a.n_units : a.effective, radd = a.row_add ? d.first_row : 0;
+                for (uint64_t u = 0; u < units && good;)
+                {
+                    uint64_t e = u + 1;
+                    const uint64_t row = of(u);
+                    while (e < units && of(e) == row) e++;
+                    good = put(row + radd, nz(u), nz(e));
+                    u = e;
+                }
+            });
+        });
     else
-        for (uint64_t b = 0; b < a.n_units; b++)
-        {
-            const uint64_t w0 = hm[MS_BLK_WARP].get(b), r0 = hm[MS_BLK_ROW].get(b), r1 = std::min<uint64_t>(hm[MS_BLK_ROW].get(b + 1), a.effective);
-            const uint64_t g0 = hm[MS_ROW_OFF].get(r0);
-            for (uint64_t r = r0; r < r1; r++)
-            {
-                const uint64_t row = a.sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : a.sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
-                if (!put(row, hm[MS_WARP_NZ].get(w0 + hm[MS_ROW_OFF].get(r) - g0), hm[MS_WARP_NZ].get(w0 + hm[MS_ROW_OFF].get(r + 1) - g0))) return false;
-            }
-        }
-    if (out.empty()) return false;
-    out.push_back(make_uint2((unsigned)end, 0));
+    {
+        const HostMeta &row = hm[MS_BLK_ROW], &warp = hm[MS_BLK_WARP];
+        const uint64_t B = a.n_units, rows = std::min<uint64_t>(row.get(B), a.effective), warps = warp.get(B);
+        if (!has_entries(offsets, warps + 1) || !has_entries(hm[MS_ROW_OFF], row.get(B) + 1)) return false;
+        with_entries(hm[MS_ROW_OFF], [&](auto off) {
+            with_entries(offsets, [&](auto nz) {
+                for (uint64_t b = 0; b < B && good; b++)
+                {
+                    const uint64_t r0 = row.get(b), r1 = std::min(row.get(b + 1), rows), w0 = warp.get(b), g0 = off(r0);
+                    for (uint64_t r = r0; r < r1 && good; r++)
+                    {
+                        const uint64_t lo = w0 + off(r) - g0, hi = w0 + off(r + 1) - g0;
+                        good = lo <= warps && hi <= warps && put(row_in_y(d, perm, a.sort_kind, r), nz(lo), nz(hi));
+                    }
+                }
+            });
+        });
+    }
+    if (!good || n == 0) return false;
+    out.p[n] = make_uint2((unsigned)end, 0);
+    out.n = n + 1;
     return true;
 }
 
-// The same of the row-grouped template; `tlbs` of all rows, `most` of one
-bool list_tlb_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, std::vector<uint4> &out, uint64_t &tlbs, uint64_t &most)
+// Row-grouped; `tlbs` of all rows, `most` of one
+bool list_tlb_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, asp::HostBuf<uint4> &out, uint64_t &tlbs, uint64_t &most)
 {
     using namespace asp;
     if (d.template_type != ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || d.n_rows > 0xffffffffull) return false;
-    std::vector<bool> seen(d.n_rows, false);
-    tlbs = most = 0;
-    for (uint64_t b = 0; b < a.n_units; b++)
-    {
-        const uint64_t nz = hm[MS_BLK_NZ].get(b), n = hm[MS_BLK_THR].get(b + 1) - hm[MS_BLK_THR].get(b), S = hm[MS_TLB_SIZE].get(b);
-        const uint64_t r0 = hm[MS_BLK_ROW].get(b), r1 = std::min<uint64_t>(hm[MS_BLK_ROW].get(b + 1), a.effective), g0 = hm[MS_ROW_OFF].get(r0);
-        if (S == 0 || S > 0xffff || nz + n * S > 0xffffffffull) return false;
-        for (uint64_t r = r0; r < r1; r++)
-        {
-            const uint64_t row = a.sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : a.sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
-            const uint64_t lo = hm[MS_ROW_OFF].get(r) - g0, hi = hm[MS_ROW_OFF].get(r + 1) - g0;
-            if (hi < lo || hi > n || hi - lo > 0xffff || row >= d.n_rows || seen[row]) return false;
-            seen[row] = true;
-            tlbs += hi - lo;
-            most = std::max(most, hi - lo);
-            out.push_back(make_uint4((unsigned)(nz + lo), (unsigned)row, (unsigned)((hi - lo) | S << 16), (unsigned)n));
-        }
-    }
-    return !out.empty();
+    const HostMeta &row = hm[MS_BLK_ROW];
+    const uint64_t B = a.n_units, rows = std::min<uint64_t>(row.get(B), a.effective);
+    if (row.get(0) != 0 || rows == 0 || rows > d.n_rows || !has_entries(hm[MS_ROW_OFF], row.get(B) + 1)) return false;
+    Distinct distinct(d.n_rows, a.sort_kind == ASP_SORT_NONE);
+    out.make(rows);
+    std::atomic<uint64_t> all(0), top(0);
+    std::atomic<bool> good(true);
+    with_entries(hm[MS_ROW_OFF], [&](auto off) {
+        host::share_ranges(B, a.sort_kind == ASP_SORT_NONE && rows >= kSharedRows, [&](uint64_t b, uint64_t e) {
+            uint64_t sum = 0, longest = 0;
+            bool in = true;
+            for (; b < e && in; b++)
+            {
+                const uint64_t nz = hm[MS_BLK_NZ].get(b), n = hm[MS_BLK_THR].get(b + 1) - hm[MS_BLK_THR].get(b), S = hm[MS_TLB_SIZE].get(b);
+                const uint64_t r0 = row.get(b), r1 = std::min(row.get(b + 1), rows), g0 = off(r0);
+                in = S > 0 && S <= 0xffff && nz + n * S <= 0xffffffffull;
+                for (uint64_t r = r0; r < r1 && in; r++)
+                {
+                    const uint64_t lo = off(r) - g0, hi = off(r + 1) - g0, y = row_in_y(d, perm, a.sort_kind, r);
+                    // (unsorted rows ascend with r, and the BLBs' rows follow one another)
+                    in = lo <= hi && hi <= n && hi - lo <= 0xffff && y < d.n_rows && (a.sort_kind == ASP_SORT_NONE || distinct(y));
+                    sum += hi - lo;
+                    longest = std::max(longest, hi - lo);
+                    out.p[r] = make_uint4((unsigned)(nz + lo), (unsigned)y, (unsigned)((hi - lo) | S << 16), (unsigned)n);
+                }
+                in = in && row.get(b + 1) >= r0;
+            }
+            all.fetch_add(sum);
+            host::raise<uint64_t>(top, longest);
+            if (!in) good = false;
+        });
+    });
+    tlbs = all;
+    most = top;
+    return good;
 }
 
-// The same of the ELL- and SELL-like templates; `place` stays empty where TLB t is row first + t. `longest` TLB, `rows` that are stored.
-bool list_strips(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const asp::KArgs &a, std::vector<uint4> &out, std::vector<unsigned> &place, uint64_t &first, uint64_t &longest, uint64_t &rows)
+// ELL- and SELL-like; `place` stays empty where TLB t is row first + t. `longest` TLB, `rows` that are stored.
+bool list_strips(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const asp::KArgs &a, asp::HostBuf<uint4> &out, asp::HostBuf<unsigned> &place, uint64_t &first, uint64_t &longest, uint64_t &rows)
 {
     using namespace asp;
     const bool ell = d.template_type == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS;
     if ((!ell && d.template_type != ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS) || d.n_rows > 0xffffffffull) return false;
     const HostMeta &of = hm[MS_ROW_OF_TLB];
-    const uint64_t radd = a.row_add ? d.first_row : 0;
+    const uint64_t radd = a.row_add ? d.first_row : 0, B = ell ? 1 : a.n_units;
     const bool numbered = of.kind == ASP_COMPRESS_LINEAR && of.coef == 1;
     longest = rows = 0;
     first = numbered ? of.icpt + radd : 0;
-    std::vector<bool> seen(numbered ? 0 : d.n_rows, false);
-    for (uint64_t b = 0; b < (ell ? 1 : a.n_units); b++)
+    out.make(std::min<uint64_t>(a.effective, ell ? a.n_tlb : hm[MS_BLK_THR].get(B)) / 32 + B + 1);
+    uint64_t k = 0;
+    for (uint64_t b = 0; b < B; b++)
     {
         const uint64_t nz = ell ? 0 : hm[MS_BLK_NZ].get(b), t0 = ell ? 0 : hm[MS_BLK_THR].get(b);
         const uint64_t n = ell ? a.n_tlb : hm[MS_BLK_THR].get(b + 1) - t0, S = ell ? a.tlb_size : hm[MS_TLB_SIZE].get(b);
-        if (S == 0 || S > 0xffff || nz + n * S > 0xffffffffull || t0 != rows) return false;
+        if (S == 0 || S > 0xffff || nz + n * S > 0xffffffffull || (t0 != rows && t0 < a.effective)) return false;
         longest = std::max(longest, S);
         for (uint64_t t = t0; t < t0 + n && t < a.effective; t += 32)
         {
             const uint64_t m = std::min<uint64_t>({32, t0 + n - t, a.effective - t});
-            out.push_back(make_uint4((unsigned)(nz + t - t0), (unsigned)t, (unsigned)(S | m << 16), (unsigned)n));
-            for (uint64_t i = t; !numbered && i < t + m; i++)
-            {
-                const uint64_t row = of.get(i) + radd;
-                if (row >= d.n_rows || seen[row]) return false;
-                seen[row] = true;
-                place.push_back((unsigned)row);
-            }
+            out.p[k++] = make_uint4((unsigned)(nz + t - t0), (unsigned)t, (unsigned)(S | m << 16), (unsigned)n);
             rows += m;
         }
     }
-    return !out.empty() && first + (numbered ? rows : 0) <= d.n_rows;
+    out.n = k;
+    if (k == 0) return false;
+    if (numbered) return first + rows <= d.n_rows;
+    if (!has_entries(of, rows)) return false;
+    Distinct distinct(d.n_rows, false);
+    place.make(rows);
+    bool good = true;
+    with_entries(of, [&](auto row) {
+        for (uint64_t i = 0; i < rows && good; i++)
+        {
+            good = distinct(row(i) + radd);
+            place.p[i] = (unsigned)(row(i) + radd);
+        }
+    });
+    return good;
 }
 
-// The same of the CSR5-like templates: {first element, row, elements, 0}
-bool list_runs(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, std::vector<uint4> &out)
+// CSR5-like: {first element, row, elements, 0}
+bool list_runs(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, asp::HostBuf<uint4> &out)
 {
     using namespace asp;
-    if ((d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE && d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE) ||
-        d.n_rows > 0xffffffffull)
-        return false;
-    std::vector<bool> seen(d.n_rows, false);
     const uint64_t S = a.tlb_size, rmask = (1ull << a.bits_row) - 1;
-    if (S == 0 || S >= 64) return false;
-    uint64_t r = ~0ull; // of the matrix's rows in order
-    for (uint64_t w = 0; w < a.n_units; w++)
-    {
-        const uint64_t R0 = hm[MS_ROW_OF_UNIT].get(w);
-        for (uint64_t l = 0; l < 32; l++)
+    if ((d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE && d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE) ||
+        d.n_rows > 0xffffffffull || S == 0 || S >= 64)
+        return false;
+    Distinct distinct(d.n_rows, a.sort_kind == ASP_SORT_NONE);
+    out.make(d.n_rows);
+    uint64_t r = ~0ull, n = 0; // of the matrix's rows in order
+    bool good = true;
+    with_entries(hm[MS_COMBINE], [&](auto words) {
+        for (uint64_t w = 0; w < a.n_units && good; w++)
         {
-            const uint64_t word = hm[MS_COMBINE].get(w * 32 + l), e0 = (w * 32 + l) * S;
-            uint64_t next = R0 + (word & rmask);
-            if (l == 0 && !((word >> (a.bits_word - 1)) & 1ull)) return false; // (a warp's first element always starts a row)
-            // the flags, first element first, at the top of the word
-            for (uint64_t f = word >> (a.bits_word - (int)S) << (64 - S); f != 0; f &= ~(1ull << (63 - __builtin_clzll(f))), next++)
+            const uint64_t R0 = hm[MS_ROW_OF_UNIT].get(w);
+            good = (words(w * 32) >> (a.bits_word - 1)) & 1ull; // (a warp's first element always starts a row)
+            for (uint64_t l = 0; l < 32 && good; l++)
             {
-                const uint64_t e = e0 + (uint64_t)__builtin_clzll(f);
-                if (next == r) continue; // goes on from the warp before
-                r = next;
-                const uint64_t row = a.sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : a.sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
-                if (row >= d.n_rows || seen[row]) return false;
-                seen[row] = true;
-                if (!out.empty()) out.back().z = (unsigned)(e - out.back().x);
-                out.push_back(make_uint4((unsigned)e, (unsigned)row, 0, 0));
+                const uint64_t word = words(w * 32 + l), e0 = (w * 32 + l) * S;
+                uint64_t next = R0 + (word & rmask);
+                // the flags, first element first, at the top of the word
+                for (uint64_t f = word >> (a.bits_word - (int)S) << (64 - S); f != 0 && good; f &= ~(1ull << (63 - __builtin_clzll(f))), next++)
+                {
+                    if (next == r) continue; // goes on from the warp before
+                    r = next;
+                    const uint64_t e = e0 + (uint64_t)__builtin_clzll(f), row = row_in_y(d, perm, a.sort_kind, r);
+                    good = distinct(row);
+                    if (!good) break;
+                    if (n > 0) out.p[n - 1].z = (unsigned)(e - out.p[n - 1].x);
+                    out.p[n++] = make_uint4((unsigned)e, (unsigned)row, 0, 0);
+                }
             }
         }
-    }
-    if (!out.empty()) out.back().z = (unsigned)(a.n_units * 32 * S - out.back().x);
-    return !out.empty();
+    });
+    if (!good || n == 0) return false;
+    out.p[n - 1].z = (unsigned)(a.n_units * 32 * S - out.p[n - 1].x);
+    out.n = n;
+    return true;
 }
 
 // Whole rows for a few lanes, a warp or a CTA, where that is the faster way (kernels_rows.cu). A warp takes up to 512 elements (four trips
@@ -642,61 +717,93 @@ bool list_runs(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const Ho
 struct OwnRows
 {
     asp::RowArgs args = {};
-    std::vector<uint2> rows;
-    std::vector<uint4> tlbs;
-    uint64_t trips = 0; // of warps that take a row
-    bool strips = false, runs = false; // (in `tlbs`)
-    std::vector<unsigned> place;
+    asp::HostBuf<uint2> rows; // (one of the two)
+    asp::HostBuf<uint4> tlbs;
+    asp::HostBuf<unsigned> place;
+    uint64_t trips = 0;  // of warps that take a row
     uint64_t listed = 0; // rows of y
-    const void *data() const { return tlbs.empty() ? (const void *)rows.data() : tlbs.data(); }
-    size_t bytes() const { return rows.size() * sizeof(uint2) + tlbs.size() * sizeof(uint4); }
-    void make(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp_plan &p, int sm_count)
+    bool strips = false, runs = false; // (in `tlbs`)
+    const void *data() const { return tlbs.n == 0 ? (const void *)rows.p : tlbs.p; }
+    size_t bytes() const { return rows.bytes() + tlbs.bytes(); }
+    void none()
+    {
+        rows = {};
+        tlbs = {};
+        place = {};
+    }
+    // f(row of y) for all of them
+    template <class F>
+    void each_row(F &&f) const
+    {
+        for (uint64_t i = 0; i + 1 < rows.n; i++) f(rows.p[i].y);
+        for (uint64_t i = 0; i < tlbs.n; i++)
+            if (!strips) f(tlbs.p[i].y);
+            else if (place.n == 0)
+                for (unsigned k = 0; k < tlbs.p[i].z >> 16; k++) f(args.first_row + tlbs.p[i].y + k);
+        for (uint64_t i = 0; i < place.n; i++) f(place.p[i]);
+    }
+    // few: one of several sub-matrices, which a kernel each takes one after the other
+    void make(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp_plan &p, int sm_count, bool few = false)
+    {
+        try
+        {
+            if (!list(d, hm, perm, p, sm_count, few)) none();
+        }
+        catch (const std::bad_alloc &) // (not enough host memory: the template's own kernel)
+        {
+            none();
+        }
+    }
+
+  private:
+    bool list(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp_plan &p, int sm_count, bool few)
     {
         uint64_t longest = 0, all = 0;
-        if (list_strips(d, hm, p.args, tlbs, place, all, longest, listed))
+        switch (d.template_type)
         {
+        case ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS:
+        case ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS:
             strips = true;
+            if (p.stored > (3u << 20) || !list_strips(d, hm, p.args, tlbs, place, all, longest, listed)) return false;
             args.first_row = (unsigned)all;
             args.lanes = longest <= 16 ? 4 : longest <= 32 ? 8 : 16;
-            args.n = (unsigned)tlbs.size();
-            if (longest <= 8 || p.stored > (3u << 20)) tlbs.clear();
-            return;
-        }
-        tlbs.clear();
-        if (p.stored <= (1u << 19) && list_runs(d, hm, perm, p.args, tlbs))
+            args.n = (unsigned)tlbs.n;
+            return longest > 8 || few;
+        case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE:
+        case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE:
         {
             runs = true;
+            if (p.stored > (1u << 19) || !list_runs(d, hm, perm, p.args, tlbs)) return false;
+            listed = tlbs.n;
             args.size = p.args.tlb_size;
-            args.n = (unsigned)tlbs.size();
-            listed = args.n;
+            args.n = (unsigned)listed;
             args.lanes = p.stored <= 6 * listed ? 4 : p.stored <= 12 * listed ? 8 : 16;
+            for (uint64_t i = 0; i < listed; i++) longest = std::max<uint64_t>(longest, tlbs.p[i].z);
+            if (longest > 4096) return false;
             // rows that take its lanes more than two trips are a CTA's
-            const auto first = std::stable_partition(tlbs.begin(), tlbs.end(), [&](const uint4 &r) { return r.z > 8 * args.lanes; });
-            args.hubs = (unsigned)(first - tlbs.begin());
-            for (const uint4 &r : tlbs) longest = std::max<uint64_t>(longest, r.z);
-            if (longest > 4096) tlbs.clear();
-            return;
+            uint4 *const first = std::stable_partition(tlbs.p, tlbs.p + listed, [&](const uint4 &r) { return r.z > 8 * args.lanes; });
+            args.hubs = (unsigned)(first - tlbs.p);
+            return true;
         }
-        tlbs.clear();
-        if (d.template_type == ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS)
-        {
+        case ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS:
+            if (p.stored > (2u << 20) || !list_tlb_rows(d, hm, perm, p.args, tlbs, all, longest)) return false;
+            listed = tlbs.n;
+            args.n = (unsigned)listed;
             args.lanes = 2;
-            bool good = p.stored <= (2u << 20) && list_tlb_rows(d, hm, perm, p.args, tlbs, all, longest);
-            while (args.lanes < 32 && args.lanes * tlbs.size() < all) args.lanes *= 2;
-            args.n = (unsigned)tlbs.size();
-            listed = tlbs.size();
-            if (!good || longest > 8 * args.lanes) tlbs.clear();
-            return;
+            while (args.lanes < 32 && args.lanes * listed < all) args.lanes *= 2;
+            return longest <= 8 * args.lanes;
+        default: break;
         }
-        if (!list_rows(d, hm, perm, p.args, rows, longest)) return rows.clear();
-        const uint64_t n = rows.size() - 1, elements = rows.back().x - rows[0].x;
-        if (longest > 512 && (longest > 16384 || elements < 256 * n)) return rows.clear();
+        if (!list_rows(d, hm, perm, p.args, rows, longest)) return false;
+        listed = rows.n - 1;
+        const uint64_t elements = rows.p[listed].x - rows.p[0].x;
+        if (longest > 512 && (longest > 16384 || elements < 256 * listed)) return false;
         // threads for all of a row in one trip while all rows are on the device at once, else for two
-        const uint64_t per = n <= 2ull * sm_count ? 4 : 8;
+        const uint64_t per = listed <= 2ull * sm_count ? 4 : 8;
         args.cta = longest <= 512 ? 0 : (unsigned)std::min<uint64_t>(1024, std::max<uint64_t>(64, (longest + 32 * per - 1) / (32 * per) * 32));
-        args.n = (unsigned)n;
-        listed = n;
-        for (uint64_t i = 0; i < n && args.cta == 0; i++) trips += (rows[i + 1].x - rows[i].x + 127) / 128;
+        args.n = (unsigned)listed;
+        for (uint64_t i = 0; i < listed && args.cta == 0; i++) trips += (rows.p[i + 1].x - rows.p[i].x + 127) / 128;
+        return true;
     }
 };
 
@@ -1386,29 +1493,60 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         }
     }
     if (n == 1 && !tg && !listed) own.make(descs[0], metas[0], perms[0], *made[0], ctx->sm_count);
-    if (!tg && own.bytes())
+    std::vector<OwnRows> owns;
+    if (n == 1) owns.push_back(std::move(own));
+    else if (!tg)
     {
-        asp_plan *const p = made[0];
-        std::shared_ptr<Arena> list(new (std::nothrow) Arena());
-        const size_t places = align_up(own.bytes(), 256);
-        if (list && list->make(ctx->device, places + own.place.size() * sizeof(unsigned)) == cudaSuccess)
+        // Several small sub-matrices, if all of them can have it and no row is in two: a kernel each on one stream instead of a stream each, which
+        // takes 15 us of events (three strips, 5,328 rows: fp32 21.4 -> 7.8 us, fp64 26.9 -> 8.7)
+        uint64_t stored = 0;
+        for (const asp_plan *p : made) stored += p->stored;
+        bool good = stored <= (1u << 20) && descs[0].n_rows <= 0xffffffffull;
+        std::vector<bool> seen(good ? descs[0].n_rows : 0, false);
+        for (int i = 0; i < n && good; i++)
         {
-            cudaError_t ce = ctx->stager.to_device(list->base, own.data(), own.bytes(), ctx->stream);
-            if (ce == cudaSuccess && !own.place.empty()) ce = ctx->stager.to_device((char *)list->base + places, own.place.data(), own.place.size() * sizeof(unsigned), ctx->stream);
-            if (ce != cudaSuccess)
-            {
-                cleanup();
-                return cuda_fail(ce, "upload of the row list");
-            }
-            p->own_rows = own.args;
-            p->own_rows.val = p->args.val;
-            p->own_rows.col = p->args.col;
-            (own.strips ? (const void *&)p->own_rows.strips : own.runs ? (const void *&)p->own_rows.runs : own.tlbs.empty() ? (const void *&)p->own_rows.rows : (const void *&)p->own_rows.tlbs) = list->base;
-            if (!own.place.empty()) p->own_rows.place = (const unsigned *)((char *)list->base + places);
-            p->own_rows_cover = own.listed == descs[0].n_rows;
-            p->row_list = list;
+            owns.emplace_back();
+            if (made[i]->templ == ASP_EMPTY_TEMPLATE) continue;
+            OwnRows &o = owns.back();
+            o.make(descs[i], metas[i], perms[i], *made[i], ctx->sm_count, true);
+            good = o.bytes() > 0 && descs[i].n_rows == descs[0].n_rows;
+            if (good) o.each_row([&](uint64_t r) {
+                good = good && r < seen.size() && !seen[r];
+                if (good) seen[r] = true;
+            });
         }
-        else cudaGetLastError(); // no room: the chunks' own kernels
+        if (!good) owns.clear();
+    }
+    static std::atomic<uint64_t> groups{0};
+    const uint64_t group = ++groups;
+    for (size_t i = 0; i < owns.size() && !tg; i++)
+    {
+        const OwnRows &o = owns[i];
+        if (o.bytes() == 0) continue;
+        std::shared_ptr<Arena> list(new (std::nothrow) Arena());
+        const size_t places = align_up(o.bytes(), 256);
+        if (!list || list->make(ctx->device, places + o.place.bytes()) != cudaSuccess)
+        {
+            cudaGetLastError(); // no room: the templates' own kernels
+            for (asp_plan *p : made) p->row_list.reset();
+            break;
+        }
+        cudaError_t ce = ctx->stager.to_device(list->base, o.data(), o.bytes(), ctx->stream);
+        if (ce == cudaSuccess && o.place.n > 0) ce = ctx->stager.to_device((char *)list->base + places, o.place.p, o.place.bytes(), ctx->stream);
+        if (ce != cudaSuccess)
+        {
+            cleanup();
+            return cuda_fail(ce, "upload of the row list");
+        }
+        asp_plan *const p = made[i];
+        p->own_rows = o.args;
+        p->own_rows.val = p->args.val;
+        p->own_rows.col = p->args.col;
+        (o.strips ? (const void *&)p->own_rows.strips : o.runs ? (const void *&)p->own_rows.runs : o.tlbs.n == 0 ? (const void *&)p->own_rows.rows : (const void *&)p->own_rows.tlbs) = list->base;
+        if (o.place.n > 0) p->own_rows.place = (const unsigned *)((char *)list->base + places);
+        p->own_rows_n = o.listed;
+        p->rows_group = group;
+        p->row_list = list;
     }
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess)
@@ -1657,17 +1795,33 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
             }
         }
     }
-    const asp_plan *only = n_plans == 1 ? plans[0] : nullptr;
-    // whole rows are stored: what was in y is cleared or overwritten by the chunks' kernel too
-    if (only && only->row_list && (clear || !only->args.atomic))
+    // Whole rows, where all plans have lists of them and no row is in two: they are stored, whatever was in y. (A plan may leave out rows, and so may a
+    // call plans of a group: y is cleared for those.)
+    uint64_t listed = 0;
+    bool by_rows = g.first != nullptr;
+    for (int i = 0; i < n_plans && by_rows; i++)
     {
-        if (clear && !only->own_rows_cover) ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
-        asp::RowArgs rows = only->own_rows;
-        rows.x = (const char *)d_x + only->args.first_col * g.es;
-        rows.y = d_y;
-        ASP_CUDA(asp::launch_own_rows(only->val_is_f64, only->col_width, rows, ctx->stream));
+        const asp_plan *p = plans[i];
+        if (p->templ == ASP_EMPTY_TEMPLATE) continue;
+        by_rows = p->row_list && p->rows_group == g.first->rows_group && (clear || !p->args.atomic);
+        for (int j = 0; j < i; j++) by_rows = by_rows && plans[j] != p;
+        listed += p->own_rows_n;
+    }
+    if (by_rows)
+    {
+        if (clear && listed < g.n_rows) ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
+        for (int i = 0; i < n_plans; i++)
+        {
+            const asp_plan *p = plans[i];
+            if (p->templ == ASP_EMPTY_TEMPLATE) continue;
+            asp::RowArgs rows = p->own_rows;
+            rows.x = (const char *)d_x + p->args.first_col * g.es;
+            rows.y = d_y;
+            ASP_CUDA(asp::launch_own_rows(p->val_is_f64, p->col_width, rows, ctx->stream));
+        }
         return ASP_OK;
     }
+    const asp_plan *only = n_plans == 1 ? plans[0] : nullptr;
     if (clear && only && only->ends_cover && only->end_rows)
         ASP_CUDA(asp::launch_zero_rows(only->val_is_f64, d_y, (const unsigned *)only->end_rows->base, only->n_end_rows, ctx->stream));
     else if (clear && !(only && only->stores_all_rows))

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import refdump
-from alphasparse_b200 import matrices as M, tuner
+from alphasparse_b200 import capi, matrices as M, tuner
 
 pytestmark = pytest.mark.gpu
 
@@ -81,3 +81,40 @@ def test_whole_rows_match_the_oracle(asp_ctx, template, lengths, cols, dense, wh
             assert (y[:shift] == 7).all() and (y[shift + m.n_rows :] == 7).all()  # nothing beside y
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("empty", [0, 20])
+@pytest.mark.parametrize("zero_y", [True, "auto"])
+def test_strips_by_whole_rows(asp_ctx, zero_y, empty, dtype):
+    """Several sub-matrices with a kernel for whole rows each: all of them, one alone, and none of the rows twice."""
+    import torch
+    from alphasparse_b200.graph import Matrix
+
+    lengths = np.random.default_rng(4).permutation([3] * 700 + [20] * 300 + [200] * 50 + [2000] * 5 + [0] * empty)
+    m, x = matrix(list(lengths), 9_000, dtype)
+    hm = Matrix.from_csr(m)
+    cm = hm.dense("dense sort 1\ndense rowdiv_exp 128 4096 8\ndense compress")
+    spec = []
+    for i in range(cm.n_subs):
+        t = "K2" if cm.sub_rows(i)[3] <= 128 else "K6" if cm.sub_rows(i)[3] <= 1024 else "K7"
+        spec += [f"sub {i} {node}" for node in NODES[t]] + [f"sub {i} template {t}"]
+    fmt = cm.execute("\n".join(spec))
+    g = fmt.upload(asp_ctx)
+    assert cm.n_subs > 1 and g.layout_bytes() == 0
+    assert empty or all(capi.lib().asp_plan_whole_rows(g._plans[i]) for i in range(g.n))
+    y_ref, scale = refdump.csr_ref(m, x)
+    dx = torch.from_numpy(x).cuda()
+    dy = torch.full((m.n_rows + 3,), 7.0, dtype=dx.dtype, device="cuda")
+    if zero_y == "auto":
+        dy[: m.n_rows] = 0
+    torch.cuda.synchronize()
+    for _ in range(2):
+        g.spmv(dx.data_ptr(), dy.data_ptr(), zero_y)
+    asp_ctx.synchronize()
+    refdump.assert_y(dy.cpu().numpy()[: m.n_rows], y_ref, scale, dtype, "all strips")
+    assert (dy[m.n_rows :] == 7).all()
+    g.close()
+    fmt.close()
+    cm.close()
+    hm.close()
