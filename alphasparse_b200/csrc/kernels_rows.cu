@@ -45,22 +45,68 @@ __device__ __forceinline__ T ld_once(const T *p)
     }
     return v;
 }
+// Sum of products with more than the values' bits, so that these kernels are no further from the exact result than the column-tiled layout that
+// they are chosen before: fp32 in fp64 (the products are exact there), fp64 with the roundings that it leaves out. Ordinary sums were 0.6 to 1.0e-7 and
+// 1.1 to 1.5e-16 from the exact result (2-norm); these are 2.5e-8 and 4.7e-17,
+// for up to 1.2 us more where 1.8 M products in fp64 take 13 operations each (5.2 -> 6.4 us; the layout 8.5).
 template <class VT>
-__device__ __forceinline__ VT warp_total(VT v)
+struct Sum;
+template <>
+struct Sum<float>
+{
+    double s = 0;
+    __device__ __forceinline__ void add(float v, float x) { s = fma((double)v, (double)x, s); }
+    __device__ __forceinline__ void add(const Sum &o) { s += o.s; }
+    __device__ __forceinline__ Sum from(int lanes) const
+    {
+        Sum o;
+        o.s = __shfl_xor_sync(0xffffffffu, s, lanes);
+        return o;
+    }
+    __device__ __forceinline__ float value() const { return (float)s; }
+};
+template <>
+struct Sum<double>
+{
+    double hi = 0, lo = 0;
+    __device__ __forceinline__ void add(double v, double x)
+    {
+        const double p = v * x, t = hi + p, b = t - hi;
+        lo += (hi - (t - b)) + (p - b) + fma(v, x, -p);
+        hi = t;
+    }
+    __device__ __forceinline__ void add(const Sum &o)
+    {
+        const double t = hi + o.hi, b = t - hi;
+        lo += (hi - (t - b)) + (o.hi - b) + o.lo;
+        hi = t;
+    }
+    __device__ __forceinline__ Sum from(int lanes) const
+    {
+        Sum o;
+        o.hi = __shfl_xor_sync(0xffffffffu, hi, lanes);
+        o.lo = __shfl_xor_sync(0xffffffffu, lo, lanes);
+        return o;
+    }
+    __device__ __forceinline__ double value() const { return isfinite(hi) ? hi + lo : hi; } // (the errors of an infinite sum are no numbers)
+};
+// of G neighbouring lanes, in each of them
+template <int G, class VT>
+__device__ __forceinline__ void total(Sum<VT> &s)
 {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    for (int o = G / 2; o > 0; o >>= 1) s.add(s.from(o));
 }
+
 // a thread's part of the row [begin, end): elements begin + t, begin + t + step, ..., four at a time; behind the end the last element is
 // read again and left out. `wait` is called by every thread whose row has elements, before its first gather.
 template <class VT, class CT, class W>
-__device__ __forceinline__ VT row_part(const RowArgs &a, u32 begin, u32 end, u32 t, u32 step, W &wait)
+__device__ __forceinline__ Sum<VT> row_part(const RowArgs &a, u32 begin, u32 end, u32 t, u32 step, W &wait)
 {
     constexpr int U = 4;
     const VT *const val = (const VT *)a.val, *const x = (const VT *)a.x;
     const CT *const col = (const CT *)a.col;
-    VT sum = 0;
+    Sum<VT> sum;
     for (u32 base = begin; base < end; base = end - base > U * step ? base + U * step : end)
     {
         const u32 left = end - base - 1; // of the elements from `base` on, the last one
@@ -74,8 +120,8 @@ __device__ __forceinline__ VT row_part(const RowArgs &a, u32 begin, u32 end, u32
 #pragma unroll
         for (int u = 0; u < U; u++) p[u] = ld_x(x + c[u]);
 #pragma unroll
-        for (int u = 0; u < U; u++) p[u] = t + u * step <= left ? v[u] * p[u] : VT(0);
-        sum += (p[0] + p[1]) + (p[2] + p[3]);
+        for (int u = 0; u < U; u++)
+            if (t + u * step <= left) sum.add(v[u], p[u]);
     }
     return sum;
 }
@@ -89,9 +135,10 @@ __global__ void __launch_bounds__(256) k_row_warp(RowArgs a)
     {
         const uint2 r = __ldg(a.rows + w);
         const u32 end = __ldg(&a.rows[w + 1].x);
-        const VT s = warp_total(row_part<VT, CT>(a, r.x, end, lane, 32, wait));
+        Sum<VT> s = row_part<VT, CT>(a, r.x, end, lane, 32, wait);
+        total<32>(s);
         wait();
-        if (lane == 0) ((VT *)a.y)[r.y] = s;
+        if (lane == 0) ((VT *)a.y)[r.y] = s.value();
     }
     wait();
 }
@@ -107,7 +154,7 @@ __global__ void __launch_bounds__(128) k_row_tlbs(RowArgs a)
     const CT *const col = (const CT *)a.col;
     const u32 t = blockIdx.x * blockDim.x + threadIdx.x, g = t / G, sub = t % G;
     WaitOnce wait;
-    VT s = 0;
+    Sum<VT> s;
     u32 row = 0;
     if (g < a.n)
     {
@@ -127,25 +174,24 @@ __global__ void __launch_bounds__(128) k_row_tlbs(RowArgs a)
 #pragma unroll
                 for (int u = 0; u < U; u++) p[u] = ld_x(x + c[u]);
 #pragma unroll
-                for (int u = 0; u < U; u++) p[u] = k + u < size ? v[u] * p[u] : VT(0);
-                s += (p[0] + p[1]) + (p[2] + p[3]);
+                for (int u = 0; u < U; u++)
+                    if (k + u < size) s.add(v[u], p[u]);
             }
     }
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    total<G>(s);
     wait();
-    if (g < a.n && sub == 0) ((VT *)a.y)[row] = s;
+    if (g < a.n && sub == 0) ((VT *)a.y)[row] = s.value();
 }
 
 // ELL- and SELL-like: 32 rows side by side, of whose TLBs W warps take every W-th element, so that a TLB of up to 4 W is one trip instead of a
 // trip for every four. W is 4, 8 or 16 (TLBs of up to 16, up to 32, more). A row a thread, four TLBs a thread / by W warps, finite elements: 7,500 rows
-// of 27, fp64, SELL 9.5 us / 2.5, ELL 7.7 / 2.5; 60,000 rows of 27 11.5 / 4.9, 9.2 / 5.0; 30,000 rows of 60 24 / 5.2, 20 / 5.3 (the column-tiled layout
+// of 27, fp64, SELL 9.5 us / 2.5, ELL 7.7 / 2.5; 60,000 rows of 27 11.5 / 5.7, 9.2 / 5.8; 30,000 rows of 60 24 / 6.4, 20 / 6.4 (the column-tiled layout
 // 8.5, and it takes 3 ms to build). Beyond what L2 holds the longer streams of the others win: 60,000 rows of 81, fp64, layout 14.6, this 16.0.
 template <class VT, class CT, int W>
 __global__ void __launch_bounds__(32 * W) k_row_strips(RowArgs a)
 {
     constexpr int U = 4;
-    __shared__ VT part[W][32];
+    __shared__ Sum<VT> part[W][32];
     const VT *const val = (const VT *)a.val, *const x = (const VT *)a.x;
     const CT *const col = (const CT *)a.col;
     const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -155,7 +201,7 @@ __global__ void __launch_bounds__(32 * W) k_row_strips(RowArgs a)
     u32 row = a.first_row + e.y + lane;
     if (a.place && on) row = __ldg(a.place + e.y + lane);
     WaitOnce wait;
-    VT s = 0;
+    Sum<VT> s;
     for (u32 k = w; k < size; k += U * W)
     {
         CT c[U];
@@ -169,17 +215,16 @@ __global__ void __launch_bounds__(32 * W) k_row_strips(RowArgs a)
 #pragma unroll
         for (int u = 0; u < U; u++) p[u] = ld_x(x + c[u]);
 #pragma unroll
-        for (int u = 0; u < U; u++) p[u] = k + u * W < size ? v[u] * p[u] : VT(0);
-        s += (p[0] + p[1]) + (p[2] + p[3]);
+        for (int u = 0; u < U; u++)
+            if (k + u * W < size) s.add(v[u], p[u]);
     }
     wait();
     part[w][lane] = s;
     __syncthreads();
     if (w != 0 || !on) return;
-    VT sum[2] = {0, 0};
 #pragma unroll
-    for (int i = 0; i < W; i++) sum[i & 1] += part[i][lane];
-    ((VT *)a.y)[row] = sum[0] + sum[1];
+    for (int i = 1; i < W; i++) s.add(part[i][lane]);
+    ((VT *)a.y)[row] = s.value();
 }
 
 // CSR5-like: element e of the matrix is element e % S of a thread that has S of them one after the other, and a warp's threads lie side by
@@ -191,7 +236,7 @@ template <class VT, class CT, int G>
 __global__ void __launch_bounds__(kRunThreads) k_row_runs(RowArgs a)
 {
     constexpr int U = 4;
-    __shared__ VT part[kRunThreads / 32];
+    __shared__ Sum<VT> part[kRunThreads / 32];
     const VT *const val = (const VT *)a.val, *const x = (const VT *)a.x;
     const CT *const col = (const CT *)a.col;
     const bool hub = blockIdx.x < a.hubs;
@@ -201,7 +246,7 @@ __global__ void __launch_bounds__(kRunThreads) k_row_runs(RowArgs a)
     uint4 r = make_uint4(0, 0, 0, 0);
     if (g < a.n) r = __ldg(a.runs + g);
     WaitOnce wait;
-    VT s = 0;
+    Sum<VT> s;
     for (u32 i = sub; i < r.z; i += U * step)
     {
         u32 at[U];
@@ -221,40 +266,42 @@ __global__ void __launch_bounds__(kRunThreads) k_row_runs(RowArgs a)
 #pragma unroll
         for (int u = 0; u < U; u++) p[u] = ld_x(x + c[u]);
 #pragma unroll
-        for (int u = 0; u < U; u++) p[u] = i + u * step < r.z ? v[u] * p[u] : VT(0);
-        s += (p[0] + p[1]) + (p[2] + p[3]);
+        for (int u = 0; u < U; u++)
+            if (i + u * step < r.z) s.add(v[u], p[u]);
     }
     wait();
     if (hub)
     {
-        s = warp_total(s);
+        total<32>(s);
         if (threadIdx.x % 32 == 0) part[threadIdx.x / 32] = s;
         __syncthreads();
         if (threadIdx.x >= 32) return;
-        s = warp_total(threadIdx.x < kRunThreads / 32 ? part[threadIdx.x] : VT(0));
-        if (threadIdx.x == 0) ((VT *)a.y)[r.y] = s;
+        s = threadIdx.x < kRunThreads / 32 ? part[threadIdx.x] : Sum<VT>();
+        total<32>(s);
+        if (threadIdx.x == 0) ((VT *)a.y)[r.y] = s.value();
         return;
     }
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (g < a.n && sub == 0) ((VT *)a.y)[r.y] = s;
+    total<G>(s);
+    if (g < a.n && sub == 0) ((VT *)a.y)[r.y] = s.value();
 }
 
 template <class VT, class CT>
 __global__ void __launch_bounds__(1024) k_row_cta(RowArgs a)
 {
-    __shared__ VT part[32];
+    __shared__ Sum<VT> part[32];
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const uint2 r = __ldg(a.rows + blockIdx.x);
     const u32 end = __ldg(&a.rows[blockIdx.x + 1].x);
     WaitOnce wait;
-    VT s = warp_total(row_part<VT, CT>(a, r.x, end, threadIdx.x, blockDim.x, wait));
+    Sum<VT> s = row_part<VT, CT>(a, r.x, end, threadIdx.x, blockDim.x, wait);
+    total<32>(s);
     wait();
     if (lane == 0) part[warp] = s;
     __syncthreads();
     if (warp != 0) return;
-    s = warp_total(lane < warps ? part[lane] : VT(0));
-    if (lane == 0) ((VT *)a.y)[r.y] = s;
+    s = lane < warps ? part[lane] : Sum<VT>();
+    total<32>(s);
+    if (lane == 0) ((VT *)a.y)[r.y] = s.value();
 }
 
 template <class VT, class CT>
