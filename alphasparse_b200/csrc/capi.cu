@@ -1480,6 +1480,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
             a.sum = (double *)(base + off[K]);
             a.n_parts = (unsigned)th.n_parts;
             a.copies = th.copies;
+            a.warps = th.warps;
             a.sum_stride = sum_stride;
             a.direct = th.direct;
             a.x = nullptr;

@@ -245,6 +245,11 @@ const u32 kWindow = 1024;    // pieces that are sorted by length together: lanes
 const u64 kRunForUnits = 7;  // at most so many elements a run, on average
 const u64 kNearRows = 4;     // and three quarters of the runs at most so many rows behind the run before
 const double kRowCost = 1.0; // of a row of a unit, in elements: its entry and its `red`
+// fp64: 16 warps, with twice the steps on their way each, or 32. A warp's wait for the steps after these is what most of its time goes to, unless
+// most of its slices are a few steps long; those are a chain of their own, of which 32 warps have more under way. 32 / 16, us: FEM of 196,611
+// rows 32.9 / 31.4, 30,000 nodes of 17 blocks 13.5 / 11.7; 190,000 rows of 80 in 40 tiles 52.8 / 60.8, in 10 tiles 35.6 / 38. Where rows have several sums
+// 16 are no faster (104,543 rows of 80 in 4 tiles 20.4 / 20.7). (fp32 is slower with 16: R-MAT scale 21 46 / 58, 9,001 rows of 2000 24.1 / 24.3.)
+const u64 kDeep = 14; // elements of a long piece; half of all elements are in such: 16
 const double kSliceCost = 4.0; // in steps; with 2 the CTAs of sparse tiles ran twice as long as the others
 // elements of a block of whole rows, the unit of the parallel build: enough blocks for all cores, and whole windows in each
 u64 block_size(u64 n) { return std::min<u64>(1u << 16, std::max<u64>(1u << 13, n / 128)); }
@@ -335,11 +340,12 @@ struct Builder
     static constexpr u32 TW = tiled_tile_cols(sizeof(VT) == 8);
     const u64 C; // tiles of x
     const unsigned width = host::crew_width();
+    unsigned warps = kTiledWarps; // of a CTA
     const u64 warp_steps; // of a warp's share, about: longer pieces are cut, and every cut is one more part of their rows
     std::vector<Chunk> chunks;
     std::vector<u64> at; // [chunk * C + tile]: first its count, then where its elements go
     std::vector<u64> tile_begin, tile_pieces;
-    u64 N = 0, runs = 0, near_runs = 0; // elements; rows' runs in the tiles, and those that lie near the one before
+    u64 N = 0, runs = 0, near_runs = 0, deep = 0; // elements; rows' runs in the tiles, and those that lie near the one before; elements of long pieces
     std::vector<u32> row_code; // of every row of y: the shares of its parts, then what stands for it among the slices' rows
     // elements in tile order
     HostBuf<u32> e_row;
@@ -371,10 +377,10 @@ struct Builder
         ThreadCounters pieces_of_thread(C, width), n_of_thread(C, width); // (neighbours in `at` share cache lines)
         const size_t edges = (2 * C + 31) / 16 * 16;
         std::vector<u32> edge(chunks.size() * edges); // rows of a chunk's first and last element in a tile, on cache lines of its own
-        std::atomic<u64> sum_runs(0), sum_near(0);
+        std::atomic<u64> sum_runs(0), sum_near(0), sum_deep(0);
         share_steps(chunks.size(), 1, width, [&](u64 c, u64, unsigned who) {
             u64 *const pieces = pieces_of_thread.of(who), *const n = n_of_thread.of(who);
-            u64 all_runs = 0, all_near = 0;
+            u64 all_runs = 0, all_near = 0, all_deep = 0;
             std::fill(n, n + C, 0);
             u32 *const first = edge.data() + (size_t)c * edges, *const last = first + C;
             u64 row = ~0ull, tile = ~0ull, run = 0;
@@ -393,6 +399,7 @@ struct Builder
                 const bool begins = n[t]++ == 0;
                 if (r != row || t != tile || run == kMaxPiece)
                 {
+                    all_deep += run >= kDeep ? run : 0;
                     pieces[t]++;
                     if (begins) first[t] = (u32)r;
                     else if (r != last[t])
@@ -414,11 +421,13 @@ struct Builder
             std::copy(n, n + C, at.begin() + (size_t)c * C);
             sum_runs.fetch_add(all_runs, std::memory_order_relaxed);
             sum_near.fetch_add(all_near, std::memory_order_relaxed);
+            sum_deep.fetch_add(all_deep + (run >= kDeep ? run : 0), std::memory_order_relaxed);
         });
         for (unsigned who = 0; who < width; who++)
             for (u64 t = 0; t < C; t++) tile_pieces[t] += pieces_of_thread.of(who)[t];
         runs = sum_runs.load(std::memory_order_relaxed);
         near_runs = sum_near.load(std::memory_order_relaxed);
+        deep = sum_deep.load(std::memory_order_relaxed);
         tile_begin.assign(C + 1, 0);
         u64 sum = 0;
         for (u64 t = 0; t < C; t++)
@@ -470,6 +479,7 @@ struct Builder
         if (sizeof(VT) == 8 && rows > 0 && warp_steps < kMaxPiece) out.copies = 4;
         if (sizeof(VT) == 8)
             while (out.copies < 16 && shares > kDirectShares / 2 * (u64)out.copies * rows) out.copies *= 2;
+        if (sizeof(VT) == 8 && 2 * deep >= N && out.copies == 1) warps = kTiledFewWarps;
         // where some rows have sums, the others do better with sums, too, than with one more launch that clears y, unless they are
         // many: 400,000 rows, fp32: 25 -> 21 us; R-MAT scale 21: 50 -> 56 us (a `red` of 64 bits costs more than one of 32)
         const double sums_us = (double)(n_rows - rows) * ((16.0 * out.copies + sizeof(VT)) / 6.0e6 + 4e-6), clear_us = 4.0 + (double)n_rows * sizeof(VT) / 6.0e6;
@@ -633,6 +643,7 @@ struct Builder
         memset(out.col.p + steps * kTiledSlice, 0, kTiledSlackSteps * kTiledSlice * sizeof(uint16_t));
         memset(out.row.p + nsl * kTiledSlice, 0xff, kTiledSlackSlices * kTiledSlice * sizeof(u32));
         for (u32 i = 0; i < kTiledSlackSlices; i++) out.end.p[nsl + i] = 0xffffffffu;
+        out.warps = warps;
         out.nnz = N;
         out.steps = steps;
         out.slices = nsl;
@@ -660,7 +671,7 @@ struct Builder
         };
         const double tile_cost = (double)kTiledTileBytes / (kTiledSlice * (sizeof(VT) + 2.0));
         share_out(
-            n_sm, kTiledWarps, tile_step, tile_cost, cost_of, step_at, out.work,
+            n_sm, warps, tile_step, tile_cost, cost_of, step_at, out.work,
             [&](u32 *o, u64 from, u64 to, u64 tile) {
                 o[0] = (u32)from;
                 o[1] = (u32)to;

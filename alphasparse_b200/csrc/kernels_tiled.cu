@@ -8,7 +8,7 @@
 //   piece  up to 32 non-zeros of one row in one tile
 //   slice  64 pieces, two per lane, of about the same length (sorted inside windows of 1024 pieces); stored step by step,
 //          a step = one non-zero of every piece
-//   steps  one linear stream, cut evenly among the CTAs (one per SM) and inside them among the 32 warps, in the middle of
+//   steps  one linear stream, cut evenly among the CTAs (one per SM) and inside them among the warps (32, or 16 in fp64), in the middle of
 //          slices too: what a warp has summed when its slice or its share ends is added to its row by `red`
 //   parts  a row that gets there in many parts would collect a rounding error with each (fp32, 80 elements over 25 tiles: 1.0e-7
 //          from the 64-bit result, the formats' own kernels 0.72e-7): the sums of such rows are 64-bit ones in memory of the
@@ -172,8 +172,8 @@ __device__ __forceinline__ void load_tile(const TiledArgs &a, VT *xs, u32 tile, 
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-template <class VT, int U>
-__global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
+template <class VT, int U, u32 W>
+__global__ void __launch_bounds__(W * 32, 1) k_tiled(TiledArgs a, u32 tile_cols)
 {
     typedef typename Pair<VT>::type P;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
     u32 visit = blockIdx.x;
     do
     {
-        const uint4 k = __ldg(a.work + (size_t)visit * kTiledWarps + warp);
+        const uint4 k = __ldg(a.work + (size_t)visit * W + warp);
         u32 step = k.x, slice = k.z;
         const u32 end = k.y, tile = k.w & 0xffffu;
         visit = k.w >> 16;
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(1024, 1) k_tiled(TiledArgs a, u32 tile_cols)
         }
         else
             __syncthreads(); // the tile before has been read
-        load_tile<1024>(a, xs, tile, tile_cols);
+        load_tile<W * 32>(a, xs, tile, tile_cols);
         __syncthreads();
         Sum<VT> acc0, acc1;
         while (step < end)
@@ -425,18 +425,9 @@ __global__ void __launch_bounds__(256) k_rows(const u32 *rows, double *sum, u64 
     }
 }
 
-template <class VT>
-struct Batch; // steps read ahead: 48 KB (fp32), 40 KB (fp64) in flight per SM
-template <>
-struct Batch<float>
-{
-    static const int U = 4;
-};
-template <>
-struct Batch<double>
-{
-    static const int U = 2;
-};
+// steps read ahead: 48 KB (fp32), 40 KB (fp64) in flight per SM
+constexpr auto kSlices = k_tiled<float, 4, kTiledWarps>;
+constexpr auto kSlices64 = k_tiled<double, 2, kTiledWarps>, kSlices64Few = k_tiled<double, 4, kTiledFewWarps>;
 
 template <class VT>
 cudaError_t clear(VT *y, u64 n, unsigned n_sm, cudaStream_t st)
@@ -455,7 +446,7 @@ cudaError_t launch_sums(const TiledArgs &a, unsigned n_sm, cudaStream_t st)
         if (e != cudaSuccess) return e;
     }
     const auto tiled = [&](auto kernel, u32 warps, u32 smem) { return launch_pdl(kernel, dim3(n_sm), dim3(warps * 32), smem, st, a, (u32)tiled_tile_cols(sizeof(VT) == 8)); };
-    if (!a.word) return tiled(k_tiled<VT, Batch<VT>::U>, kTiledWarps, kTiledTileBytes);
+    if (!a.word) return tiled(sizeof(VT) == 4 ? kSlices : a.warps == kTiledFewWarps ? kSlices64Few : kSlices64, a.warps, kTiledTileBytes);
     if (sizeof(VT) == 8) return cudaErrorInvalidValue; // (units are fp32)
     if (!a.direct) return tiled(k_tiled_units<1>, kTiledUnitWarps, kUnitSmem);
     return a.n_parts == 0 ? tiled(k_tiled_units<0>, kTiledUnitWarps, kUnitSmem) : tiled(k_tiled_units<2>, kTiledUnitWarps, kUnitSmem);
@@ -493,8 +484,12 @@ cudaError_t allow(const void *f, u32 smem) { return cudaFuncSetAttribute(f, cuda
 
 cudaError_t tiled_setup(int val_is_f64)
 {
-    if (val_is_f64) return allow((const void *)k_tiled<double, Batch<double>::U>, kTiledTileBytes);
-    cudaError_t e = allow((const void *)k_tiled<float, Batch<float>::U>, kTiledTileBytes);
+    if (val_is_f64)
+    {
+        const cudaError_t e = allow((const void *)kSlices64, kTiledTileBytes);
+        return e == cudaSuccess ? allow((const void *)kSlices64Few, kTiledTileBytes) : e;
+    }
+    cudaError_t e = allow((const void *)kSlices, kTiledTileBytes);
     for (const void *f : {(const void *)k_tiled_units<0>, (const void *)k_tiled_units<1>, (const void *)k_tiled_units<2>})
         if (e == cudaSuccess) e = allow(f, kUnitSmem);
     return e;

@@ -15,7 +15,7 @@
 
 namespace asp
 {
-const uint32_t kTiledWarps = 32;             // warps per CTA, one CTA per SM
+constexpr uint32_t kTiledWarps = 32, kTiledFewWarps = 16; // warps per CTA, one CTA per SM: which of the two says kFewWarps (tiled_build.cpp)
 const uint32_t kTiledLanePieces = 2;         // pieces of a row per lane
 const uint32_t kTiledSlice = 32 * kTiledLanePieces;
 constexpr uint32_t kTiledTileBytes = 159u << 10; // shared memory of a tile of x
@@ -74,7 +74,8 @@ struct TiledHost
     uint64_t n_parts = 0;        // rows of y that are added up in many parts ...
     std::vector<uint32_t> parts; // ... which these are; empty: all
     HostBuf<uint32_t> end;      // slice s covers steps [end[s - 1], end[s])
-    std::vector<uint32_t> work; // {first step, end step, slice, tile | next visit << 16} per warp; visit v at v * kTiledWarps
+    unsigned warps = kTiledWarps;
+    std::vector<uint32_t> work; // {first step, end step, slice, tile | next visit << 16} per warp; visit v at v * warps
     uint64_t nnz = 0, steps = 0, slices = 0;
     // units > 0: units instead of slices. Then val and col hold them one after the other, in each the first 16 bytes of every lane, the
     // next 16 bytes of every lane, ...; row[seg[u], seg[u + 1]) are the rows of unit u; work: {first unit, end unit, tile, next visit (0: none)},
@@ -99,7 +100,7 @@ struct TiledArgs
     const uint4 *work;
     const uint32_t *parts; // n_parts rows (NULL: all rows of y) ...
     double *sum;           // ... and their sums, copies * sum_stride of them, zero between the calls
-    unsigned n_parts, copies;
+    unsigned n_parts, copies, warps; // (warps: slices)
     unsigned long long sum_stride;
     int direct; // y takes other rows' sums: it is cleared first
     const void *x;
