@@ -53,3 +53,28 @@ def test_host_call_matches_the_oracle(asp_ctx, rows, cols, offsets, dtype):
     assert (yp[:3] == 7).all() and (yp[3 + m.n_rows :] == 7).all()
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("spec,threads", [("diag_value 64", "D1"), ("row_padding 32 1|tlb_row", "K3"), ("tlb_nnz 8", "K9")])
+@pytest.mark.parametrize("rows", [5, 96, 1001, 40_000, 60_001, 250_000])
+def test_pipelined_calls_around_a_short_x(asp_ctx, rows, spec, threads, dtype):
+    """x in one piece or in several, y from the kernels or by copies, page-locked or not, with chunks that read to the end of x or not."""
+    import torch
+    from alphasparse_b200 import tuner
+
+    m, x = banded(rows, rows + 3, [-2, 0, 3], 5, dtype)
+    desc = {"dense": "dense compress", "subs": [{"graph": threads, "nodes": spec.split("|"), "template": threads, "threads": 128, "row_reduce": 1}]}
+    chunks = tuner.build_row_chunks(asp_ctx, m, desc, 3, align=32)
+    y_ref, scale = refdump.csr_ref(m, x)
+    xp = torch.from_numpy(x).pin_memory()
+    for pinned in (True, False):
+        y = torch.full((rows + 2,), 7.0, dtype=xp.dtype)
+        y = y.pin_memory() if pinned else y
+        for _ in range(2):
+            capi.spmv_host_pipelined(asp_ctx, [c[1:] for c in chunks], xp.data_ptr(), y.data_ptr())
+        refdump.assert_y(y.numpy()[:rows], y_ref, scale, dtype, f"{threads} pinned={pinned}")
+        assert (y[rows:] == 7).all()
+    for fmt, g, *_ in chunks:
+        g.close()
+        fmt.close()
