@@ -1675,7 +1675,7 @@ asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path)
 {
     if (!plan) return fail(ASP_ERR_INVALID_ARG, "plan is NULL");
     const asp_status st = set_tuning(plan, vec, path);
-    if (st == ASP_OK) plan->tiled.reset(); // the caller experiments with this plan's own kernel
+    if (st == ASP_OK) plan->tiled.reset(), plan->row_list.reset(); // the caller experiments with this plan's own kernel
     return st;
 }
 
@@ -1797,9 +1797,9 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
         }
     }
     // Whole rows, where all plans have lists of them and no row is in two: they are stored, whatever was in y. (A plan may leave out rows, and so may a
-    // call plans of a group: y is cleared for those.)
+    // call plans of a group: y is cleared for those.) Who leaves y as it is gets the templates' kernels.
     uint64_t listed = 0;
-    bool by_rows = g.first != nullptr;
+    bool by_rows = g.first != nullptr && zero_y != 0;
     for (int i = 0; i < n_plans && by_rows; i++)
     {
         const asp_plan *p = plans[i];

@@ -246,7 +246,8 @@ enum
     ASP_FORM_IN_SUMS = 8
 };
 int asp_plan_layout_form(const asp_plan *plan);
-/* 1: asp_spmv of this plan alone, where it need not add to what y holds, runs a kernel that takes whole rows, instead of its template's */
+/* 1: asp_spmv of this plan alone with zero_y 1 or 2 runs a kernel that takes whole rows, instead of its template's (small matrices; the launch
+ * parameters are the template's kernel's). asp_plan_set_tuning ends that. */
 int asp_plan_whole_rows(const asp_plan *plan);
 /* number of launches of its template's kernel that one asp_spmv over this plan issues (excluding the y clear); the plans of a group
  * that runs the column-tiled layout share one launch */

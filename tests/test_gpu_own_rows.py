@@ -71,7 +71,7 @@ def test_whole_rows_match_the_oracle(asp_ctx, template, lengths, cols, dense, wh
         dy = torch.full((m.n_rows + 3 + shift,), 7.0, dtype=dx.dtype, device="cuda")
         modes = [True, "auto", False] if min(lengths) > 0 else [True]  # (rows that nobody stores are the caller's to clear)
         for zero_y in modes:
-            if zero_y is False:  # the templates add to y or overwrite it: both to a cleared one
+            if zero_y is False:  # the templates' own kernels, which add to y or overwrite it: both to a cleared one
                 dy[shift : shift + m.n_rows] = 0
             torch.cuda.synchronize()
             g.spmv(dx[shift:].data_ptr(), dy[shift:].data_ptr(), zero_y)
@@ -118,3 +118,16 @@ def test_strips_by_whole_rows(asp_ctx, zero_y, empty, dtype):
     fmt.close()
     cm.close()
     hm.close()
+
+
+@pytest.mark.parametrize("template", ["K2", "K3", "K9"])
+def test_a_tuned_plan_runs_its_own_kernel(asp_ctx, template):
+    m, x = matrix([30, 40] * 100, 3_000, np.float32)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template, "threads": 128, "row_reduce": 1}]})
+    assert g.whole_rows()
+    y_ref, scale = refdump.csr_ref(m, x)
+    capi.check(capi.lib().asp_plan_set_tuning(g._plans[0], 0, 0))
+    assert not g.whole_rows()
+    refdump.assert_y(g.spmv_host(x), y_ref, scale, np.float32, template)
+    g.close()
+    fmt.close()
