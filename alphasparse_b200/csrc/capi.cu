@@ -1022,10 +1022,16 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
     }
 
     std::shared_ptr<Arena> arena(new (std::nothrow) Arena());
+    size_t list_room = 0, list_at = 0;
     if (!arena) return fail(ASP_ERR_ALLOC, "host allocation failed");
     if (!dry)
     {
-        cudaError_t e = arena->make(ctx->device, std::max<size_t>(total, 256));
+        // with room for a small matrix's list of rows (below): a block of its own costs as much again
+        uint64_t stored = 0;
+        for (int i = 0; i < n; i++) stored += vals[i] ? vals[i]->len : 0;
+        list_room = stored <= (3u << 20) ? align_up(20 * descs[0].n_rows + 4096 * (size_t)n, 256) : 0;
+        total = align_up(total, 256);
+        cudaError_t e = arena->make(ctx->device, std::max<size_t>(total + list_room, 256));
         if (e != cudaSuccess)
         {
             cudaGetLastError();
@@ -1524,16 +1530,22 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
     {
         const OwnRows &o = owns[i];
         if (o.bytes() == 0) continue;
-        std::shared_ptr<Arena> list(new (std::nothrow) Arena());
-        const size_t places = align_up(o.bytes(), 256);
-        if (!list || list->make(ctx->device, places + o.place.bytes()) != cudaSuccess)
+        const size_t places = align_up(o.bytes(), 256), bytes = align_up(places + o.place.bytes(), 256);
+        std::shared_ptr<Arena> list = arena;
+        if (list_at + bytes > list_room)
         {
-            cudaGetLastError(); // no room: the templates' own kernels
-            for (asp_plan *p : made) p->row_list.reset();
-            break;
+            list.reset(new (std::nothrow) Arena());
+            if (!list || list->make(ctx->device, bytes) != cudaSuccess)
+            {
+                cudaGetLastError(); // no room: the templates' own kernels
+                for (asp_plan *p : made) p->row_list.reset();
+                break;
+            }
         }
-        cudaError_t ce = ctx->stager.to_device(list->base, o.data(), o.bytes(), ctx->stream);
-        if (ce == cudaSuccess && o.place.n > 0) ce = ctx->stager.to_device((char *)list->base + places, o.place.p, o.place.bytes(), ctx->stream);
+        unsigned char *const to = (unsigned char *)list->base + (list == arena ? total + list_at : 0);
+        if (list == arena) list_at += bytes;
+        cudaError_t ce = ctx->stager.to_device(to, o.data(), o.bytes(), ctx->stream);
+        if (ce == cudaSuccess && o.place.n > 0) ce = ctx->stager.to_device(to + places, o.place.p, o.place.bytes(), ctx->stream);
         if (ce != cudaSuccess)
         {
             cleanup();
@@ -1543,8 +1555,8 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         p->own_rows = o.args;
         p->own_rows.val = p->args.val;
         p->own_rows.col = p->args.col;
-        (o.strips ? (const void *&)p->own_rows.strips : o.runs ? (const void *&)p->own_rows.runs : o.tlbs.n == 0 ? (const void *&)p->own_rows.rows : (const void *&)p->own_rows.tlbs) = list->base;
-        if (o.place.n > 0) p->own_rows.place = (const unsigned *)((char *)list->base + places);
+        (o.strips ? (const void *&)p->own_rows.strips : o.runs ? (const void *&)p->own_rows.runs : o.tlbs.n == 0 ? (const void *&)p->own_rows.rows : (const void *&)p->own_rows.tlbs) = to;
+        if (o.place.n > 0) p->own_rows.place = (const unsigned *)(to + places);
         p->own_rows_n = o.listed;
         p->rows_group = group;
         p->row_list = list;

@@ -100,9 +100,10 @@ struct TiledArgs
     const uint4 *work;
     const uint32_t *parts; // n_parts rows (NULL: all rows of y) ...
     double *sum;           // ... and their sums, copies * sum_stride of them, zero between the calls
-    unsigned n_parts, copies, warps; // (warps: slices)
+    unsigned n_parts, copies;
     unsigned long long sum_stride;
     int direct; // y takes other rows' sums: it is cleared first
+    unsigned warps; // slices: of a CTA
     const void *x;
     void *y;
     unsigned long long n_rows, n_cols;
