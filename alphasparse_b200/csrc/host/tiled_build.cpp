@@ -249,6 +249,8 @@ const double kRowCost = 1.0; // of a row of a unit, in elements: its entry and i
 // most of its slices are a few steps long; those are a chain of their own, of which 32 warps have more under way. 32 / 16, us: FEM of 196,611
 // rows 32.9 / 31.4, 30,000 nodes of 17 blocks 13.5 / 11.7; 190,000 rows of 80 in 40 tiles 52.8 / 60.8, in 10 tiles 35.6 / 38. Where rows have several sums
 // 16 are no faster (104,543 rows of 80 in 4 tiles 20.4 / 20.7). (fp32 is slower with 16: R-MAT scale 21 46 / 58, 9,001 rows of 2000 24.1 / 24.3.)
+// Long streams fill the memory's rate either way: FEM, 27 blocks, 21.9 M elements 42.4 / 40.8, 31.9 M 58.7 / 58.8, 63.7 M 111.2 / 113.5.
+const u64 kFewWarpsMost = 26u << 20;
 const u64 kDeep = 14; // elements of a long piece; half of all elements are in such: 16
 const double kSliceCost = 4.0; // in steps; with 2 the CTAs of sparse tiles ran twice as long as the others
 // elements of a block of whole rows, the unit of the parallel build: enough blocks for all cores, and whole windows in each
@@ -479,7 +481,7 @@ struct Builder
         if (sizeof(VT) == 8 && rows > 0 && warp_steps < kMaxPiece) out.copies = 4;
         if (sizeof(VT) == 8)
             while (out.copies < 16 && shares > kDirectShares / 2 * (u64)out.copies * rows) out.copies *= 2;
-        if (sizeof(VT) == 8 && 2 * deep >= N && out.copies == 1) warps = kTiledFewWarps;
+        if (sizeof(VT) == 8 && 2 * deep >= N && out.copies == 1 && N <= kFewWarpsMost) warps = kTiledFewWarps;
         // where some rows have sums, the others do better with sums, too, than with one more launch that clears y, unless they are
         // many: 400,000 rows, fp32: 25 -> 21 us; R-MAT scale 21: 50 -> 56 us (a `red` of 64 bits costs more than one of 32)
         const double sums_us = (double)(n_rows - rows) * ((16.0 * out.copies + sizeof(VT)) / 6.0e6 + 4e-6), clear_us = 4.0 + (double)n_rows * sizeof(VT) / 6.0e6;
