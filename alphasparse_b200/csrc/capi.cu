@@ -520,6 +520,7 @@ uint64_t row_in_y(const asp_plan_desc &d, const HostMeta &perm, int sort_kind, u
 {
     return sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
 }
+const uint64_t kMostRun = 4096; // elements of a row of the CSR5-like templates that is listed
 const uint64_t kSharedRows = 1u << 14; // from so many on, the rows of a list are shared out
 
 // Lists of the rows of a (validated) plan, as the kernels of kernels_rows.cu take them. false: another template, a row in two places, or offsets
@@ -676,6 +677,10 @@ bool list_runs(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const Ho
     if ((d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE && d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE) ||
         d.n_rows > 0xffffffffull || S == 0 || S >= 64)
         return false;
+    // (a row that is too long is seen by the warps that begin in it)
+    const uint64_t within = kMostRun / (32 * S) + 1;
+    for (uint64_t w = 0; w + within < a.n_units; w++)
+        if (hm[MS_ROW_OF_UNIT].get(w) == hm[MS_ROW_OF_UNIT].get(w + within)) return false;
     Distinct distinct(d.n_rows, a.sort_kind == ASP_SORT_NONE);
     out.make(d.n_rows);
     uint64_t r = ~0ull, n = 0; // of the matrix's rows in order
@@ -779,7 +784,7 @@ struct OwnRows
             args.n = (unsigned)listed;
             args.lanes = p.stored <= 6 * listed ? 4 : p.stored <= 12 * listed ? 8 : 16;
             for (uint64_t i = 0; i < listed; i++) longest = std::max<uint64_t>(longest, tlbs.p[i].z);
-            if (longest > 4096) return false;
+            if (longest > kMostRun) return false;
             // rows that take its lanes more than two trips are a CTA's
             uint4 *const first = std::stable_partition(tlbs.p, tlbs.p + listed, [&](const uint4 &r) { return r.z > 8 * args.lanes; });
             args.hubs = (unsigned)(first - tlbs.p);
