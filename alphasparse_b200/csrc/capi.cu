@@ -1371,12 +1371,14 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
             else if (d.effective_num == 0 || d.effective_num > NR || d.first_row + d.effective_num > d.n_rows) st = ASP_ERR_BOUNDS, why = "diagonal-value template: rows of the sub-matrix outside y or the padded rows";
             else if (d.sort_kind != ASP_SORT_NONE || d.is_atom_add) st = ASP_ERR_UNSUPPORTED, why = "diagonal-value template: neither sorted nor column-sliced matrices";
             p->units_for_grid = NR / V;
-            p->diag_reach = (long long)(max_entry((const uint64_t *)cols[i]->host_ptr, D) + d.first_col) - (long long)a.n_units;
             break;
         }
         default: st = ASP_ERR_UNSUPPORTED; why = "template not implemented"; break;
         }
         if (st == ASP_OK && !validate_contents(d, hm, perms[i], cols[i], a, why)) st = ASP_ERR_BOUNDS;
+        // (of offsets that have been found inside the matrix, as many as there are)
+        if (st == ASP_OK && d.template_type == ASP_DIAG_TEMPLATE)
+            p->diag_reach = (long long)(max_entry((const uint64_t *)cols[i]->host_ptr, cols[i]->len) + d.first_col) - (long long)a.n_units;
         if (st != ASP_OK)
         {
             cleanup();

@@ -115,6 +115,28 @@ def test_partial_result_offsets_must_stay_inside_their_blb(name):
     _expect_bounds(descs, "partial-result range")
 
 
+@pytest.mark.parametrize("count", [0, 7, 1_000_000, 10**12])
+def test_a_count_of_diagonals_that_is_not_the_arrays_is_rejected(count):
+    """The offsets are read as far as their array goes, whatever the descriptor says."""
+    m, _ = M.laplacian_2d(32, seed=1)
+    fmt = Matrix.from_csr(m).execute("dense compress\nsub all diag_value 64\nsub all template D1")
+    descs = fmt.plan_descs()
+    capi.validate_descs(descs)
+    descs[0].tlb_size = count
+    _expect_bounds(descs, "values do not match diagonals")
+    fmt.close()
+
+
+def test_an_offset_far_outside_the_matrix_is_rejected():
+    m, _ = M.laplacian_2d(32, seed=1)
+    fmt = Matrix.from_csr(m).execute("dense compress\nsub all diag_value 64\nsub all template D1")
+    descs = fmt.plan_descs()
+    _, offsets = _array_of(descs[0], "col_index_arr")
+    offsets[-1] = np.iinfo(np.uint64).max
+    _expect_bounds(descs, "")
+    fmt.close()
+
+
 def test_sorted_plan_with_a_bad_permutation_is_rejected():
     _, _, _, man = load_golden("mixed4096_f32_sorted_split")
     descs, keep = refdump.plan_descs(man)
