@@ -1896,17 +1896,6 @@ namespace
 {
 // ---- host calls of a plan that stores the rows of y in order (diagonal values): rows run as soon as their x is there, and go to the host
 // from the kernel
-// what the device calls a page-locked host buffer; NULL: it is none
-void *device_view(const void *host)
-{
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, host) != cudaSuccess)
-    {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
-}
 bool rows_in_order(asp_plan *const *plans, int n_plans) { return n_plans == 1 && plans[0]->templ == ASP_DIAG_TEMPLATE && plans[0]->stores_all_rows; }
 // rows [r0, r1) of y, r0 a multiple of 4
 cudaError_t launch_in_order(const asp_plan *p, const void *x, void *y, uint64_t r0, uint64_t r1, cudaStream_t st)
@@ -1978,7 +1967,7 @@ asp_status asp_spmv_host(asp_ctx *ctx, asp_plan *const *plans, int n_plans, cons
     const size_t xb = g.n_cols * g.es, yb = g.n_rows * g.es;
     st = ensure_xy(ctx, xb, yb);
     if (st != ASP_OK) return st;
-    void *const y_seen = rows_in_order(plans, n_plans) ? device_view(h_y) : nullptr;
+    void *const y_seen = rows_in_order(plans, n_plans) ? asp::device_view(h_y, yb) : nullptr;
     if (y_seen)
     {
         // Pieces of a quarter of x: the last one's rows are all that goes to the host after x has come. (8 MB each way: 338 us; in eighths
@@ -2042,7 +2031,7 @@ asp_status asp_spmv_host_pipelined(asp_ctx *ctx, const asp_host_chunk *chunks, i
     ASP_ON_DEVICE(ctx);
     asp_status st = ensure_xy(ctx, n_cols * es, n_rows * es);
     if (st != ASP_OK) return st;
-    unsigned char *const y_seen = (unsigned char *)device_view(h_y);
+    unsigned char *const y_seen = (unsigned char *)asp::device_view(h_y, n_rows * es);
     // A short x is there sooner than the calls that would send it in pieces: all of it, the chunks' kernels, and y (which the kernels store to the
     // host themselves where they can). (Four chunks, 48 KB of x: 52 -> 35.6 us, 167 KB 53 -> 47.5; 0.7 MB 68,
     // 70 so.)

@@ -1,5 +1,6 @@
 #include "memory.h"
 
+#include <cuda.h>
 #include <stdint.h>
 #include <string.h>
 #if defined(__SSE2__)
@@ -223,6 +224,32 @@ void Stager::release()
     for (int i = 0; i < kPieces; i++) cudaEventDestroy(done[i]);
     cudaFreeHost(ring);
     ring = nullptr;
+}
+
+void *device_view(const void *p, size_t bytes)
+{
+    typedef CUresult (*Query)(void *, CUpointer_attribute, CUdeviceptr);
+    static const Query query = []() -> Query {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        const cudaError_t e = cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &found);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? (Query)f : nullptr;
+    }();
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (at.type != cudaMemoryTypeHost || !at.devicePointer || !query) return nullptr;
+    const CUdeviceptr d = (CUdeviceptr)at.devicePointer;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    int access = 0;
+    if (query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, d) != CUDA_SUCCESS || query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, d) != CUDA_SUCCESS) return nullptr;
+    if (query(&access, CU_POINTER_ATTRIBUTE_ACCESS_FLAGS, d) != CUDA_SUCCESS || access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE) return nullptr;
+    return d >= start && d - start <= size && bytes <= size - (d - start) ? at.devicePointer : nullptr;
 }
 
 bool Stager::pinned(const void *host)

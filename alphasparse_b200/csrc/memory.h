@@ -25,6 +25,10 @@ void device_trim(int device);
 void device_pool_retain(int device);  // a context was created ...
 void device_pool_release(int device); // ... or destroyed
 
+// What the device calls [p, p + bytes) of host memory, where all of it lies in one page-locked range that the device may write, else NULL. (The
+// ends alone do not say it: a buffer may begin in one registered range and end in another.)
+void *device_view(const void *p, size_t bytes);
+
 // Copies between pageable host memory and the device. The runtime moves such a copy through its own pinned buffer with one
 // thread (8 to 12 GB/s measured, page faults of a fresh destination included); here all cores fill or empty a ring of pinned
 // pieces while the copy engine works on the others. Pinned memory is copied directly. 16 MB per context, allocated with the

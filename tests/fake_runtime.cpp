@@ -55,6 +55,8 @@ std::recursive_mutex lock;
 std::deque<Op> queue;
 std::map<cudaEvent_t, int> pending; // records of an event that are still in the queue
 std::map<void *, size_t> blocks;
+std::vector<std::pair<const char *, size_t>> page_locked;
+bool read_only = false;
 size_t in_use = 0, limit = ~0ull;
 std::mt19937 rng(1);
 long next_event = 1;
@@ -147,7 +149,32 @@ cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind
         fake::queue.push_back({dst, src, n, nullptr});
     return cudaSuccess;
 }
-cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *) { return a->type = cudaMemoryTypeUnregistered, cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p)
+{
+    *a = {};
+    a->type = cudaMemoryTypeUnregistered;
+    for (auto &r : fake::page_locked)
+        if ((const char *)p >= r.first && (const char *)p < r.first + r.second) a->type = cudaMemoryTypeHost, a->hostPointer = a->devicePointer = (void *)p;
+    return cudaSuccess;
+}
+static CUresult pointer_attribute(void *out, CUpointer_attribute what, CUdeviceptr p)
+{
+    for (auto &r : fake::page_locked)
+        if ((const char *)p >= r.first && (const char *)p < r.first + r.second)
+        {
+            if (what == CU_POINTER_ATTRIBUTE_RANGE_START_ADDR) *(CUdeviceptr *)out = (CUdeviceptr)r.first;
+            else if (what == CU_POINTER_ATTRIBUTE_RANGE_SIZE) *(size_t *)out = r.second;
+            else if (what == CU_POINTER_ATTRIBUTE_ACCESS_FLAGS) *(int *)out = fake::read_only ? CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READ : CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE;
+            else return CUDA_ERROR_INVALID_VALUE;
+            return CUDA_SUCCESS;
+        }
+    return CUDA_ERROR_INVALID_VALUE;
+}
+cudaError_t cudaGetDriverEntryPoint(const char *name, void **f, unsigned long long, cudaDriverEntryPointQueryResult *found)
+{
+    need(std::string(name) == "cuPointerGetAttribute", "an unknown call of the driver");
+    return *f = (void *)pointer_attribute, *found = cudaDriverEntryPointSuccess, cudaSuccess;
+}
 }
 
 typedef std::vector<unsigned char> Bytes;
@@ -259,6 +286,20 @@ int main(int, char **argv)
         need(fake::in_use > 0, "the pool keeps nothing");
         asp::device_trim(0);
         need(fake::in_use == 0, "idle blocks after a trim");
+    }
+    if (part == "views")
+    {
+        // a buffer is seen by the device only where all of it is page-locked, in one range
+        Bytes b(1 << 20);
+        char *p = (char *)b.data();
+        fake::page_locked = {{p + 4096, 8192}, {p + 12288, 4096}, {p + 40960, 4096}};
+        need(asp::device_view(p + 4096, 8192) == p + 4096 && asp::device_view(p + 4104, 8184) == p + 4104 && asp::device_view(p + 12287, 1) == p + 12287, "page-locked buffers");
+        need(!asp::device_view(p, 4096) && !asp::device_view(p + 4095, 8192), "a buffer that begins before its range");
+        need(!asp::device_view(p + 4096, 8193) && !asp::device_view(p + 40968, 4096), "a buffer that ends behind its range");
+        need(!asp::device_view(p + 4096, 12288), "a buffer over two ranges");
+        need(!asp::device_view(p + 12288, 32768), "a buffer whose ends are page-locked");
+        fake::read_only = true;
+        need(!asp::device_view(p + 4096, 8192), "a buffer that is registered for reading");
     }
     asp::device_pool_release(0);
     need(fake::blocks.empty(), "device memory is left");

@@ -14,7 +14,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("part", ["ring", "threads", "no memory", "full device"])
+@pytest.mark.parametrize("part", ["ring", "threads", "no memory", "full device", "views"])
 def test_copies_and_pools(program, part):
     r = subprocess.run([program, part], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, (r.returncode, r.stdout, r.stderr[-500:])
