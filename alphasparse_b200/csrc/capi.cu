@@ -1967,7 +1967,9 @@ asp_status asp_spmv_host(asp_ctx *ctx, asp_plan *const *plans, int n_plans, cons
     const size_t xb = g.n_cols * g.es, yb = g.n_rows * g.es;
     st = ensure_xy(ctx, xb, yb);
     if (st != ASP_OK) return st;
-    void *const y_seen = rows_in_order(plans, n_plans) ? asp::device_view(h_y, yb) : nullptr;
+    // (a y that begins inside x would be stored where x has yet to be read from)
+    const bool into_x = (uintptr_t)h_y > (uintptr_t)h_x && (uintptr_t)h_y < (uintptr_t)h_x + xb;
+    void *const y_seen = rows_in_order(plans, n_plans) && !into_x ? asp::device_view(h_y, yb) : nullptr;
     if (y_seen)
     {
         // Pieces of a quarter of x: the last one's rows are all that goes to the host after x has come. (8 MB each way: 338 us; in eighths

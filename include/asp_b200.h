@@ -262,7 +262,7 @@ int asp_plan_launches(const asp_plan *plan);
 asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const void *d_x, void *d_y, int zero_y);
 
 /* same with HOST x and y: copies x in, runs, copies y out, waits. This is the shape of the
- * reference's a.out run (host arrays in, host y out) without the text files. */
+ * reference's a.out run (host arrays in, host y out) without the text files. x and y may overlap. */
 asp_status asp_spmv_host(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const void *h_x, void *h_y);
 
 /* asp_spmv_host for matrices whose rows read a bounded band of columns (stencils, finite elements in a
@@ -272,7 +272,8 @@ asp_status asp_spmv_host(asp_ctx *ctx, asp_plan *const *plans, int n_plans, cons
  * is on the device, and its rows of y leave for the host while the next chunk's part of x is still arriving, on
  * three streams (copy in, kernels, copy out). With h_x and h_y in pinned memory a host-to-host SpMV then costs
  * about one PCIe direction instead of two in series. A wrong col_hi makes a kernel read entries of x that are not
- * there yet (stale values of an earlier call): declare the maximum column + 1, or n_cols when in doubt. The
+ * there yet (stale values of an earlier call): declare the maximum column + 1, or n_cols when in doubt. x and y must not
+ * overlap: rows of y are written while later entries of x are still read. The
  * chunks must tile [0, n_rows) in ascending order. Returns when y is complete. No counterpart in the reference
  * (its generated program copies x in, runs, copies y out: code_builder.cc:2119-2129, 1534-1557). */
 typedef struct

@@ -78,3 +78,24 @@ def test_pipelined_calls_around_a_short_x(asp_ctx, rows, spec, threads, dtype):
     for fmt, g, *_ in chunks:
         g.close()
         fmt.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("shift", [-4096, -1, 0, 1, 200_000])
+def test_x_and_y_in_one_buffer(asp_ctx, shift, dtype):
+    """Rows are stored while later x is on its way: not into what has yet to be read."""
+    import torch
+
+    n = 4 * PIECE // np.dtype(dtype).itemsize
+    m, x = banded(n, n, [-1, 0, 1], 3, dtype)
+    fmt = Matrix.from_csr(m).execute("dense compress\nsub all diag_value 64\nsub all template D1")
+    g = fmt.upload(asp_ctx)
+    y_ref, scale = refdump.csr_ref(m, x)
+    both = torch.zeros(n + abs(shift), dtype=torch.from_numpy(x).dtype).pin_memory()
+    hx, hy = both[max(0, -shift) :][:n], both[max(0, shift) :][:n]
+    for _ in range(2):
+        hx.copy_(torch.from_numpy(x))
+        capi.check(capi.lib().asp_spmv_host(asp_ctx.handle, g._plans, g.n, C.c_void_p(hx.data_ptr()), C.c_void_p(hy.data_ptr())))
+        refdump.assert_y(hy.numpy(), y_ref, scale, dtype, f"y {shift} behind x")
+    g.close()
+    fmt.close()
