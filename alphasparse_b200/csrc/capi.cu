@@ -20,6 +20,7 @@
 #include "kernel_args.h"
 #include "kernels.h"
 #include "memory.h"
+#include "row_lists.h"
 #include "tiled.h"
 
 namespace
@@ -94,6 +95,7 @@ struct Arena
 };
 
 using asp::HostMeta;
+using asp::has_entries;
 
 } // namespace
 
@@ -301,9 +303,6 @@ asp_status apply_launch(asp_ctx *ctx, asp_plan *p, int64_t tblock, int64_t threa
     return ASP_OK;
 }
 
-// a closed form, or an array of at least `count` entries
-bool has_entries(const HostMeta &h, uint64_t count) { return h.kind != ASP_COMPRESS_NONE || h.len >= count; }
-
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // ---- content validation --------------------------------------------------------------------------
@@ -489,328 +488,6 @@ bool stores_every_row(const asp_plan_desc &d, const std::vector<HostMeta> &hm, c
     default: return false;
     }
 }
-
-// f(entry of a place): of an array by its type, looked at once
-template <class F>
-void with_entries(const HostMeta &h, F &&f)
-{
-    if (h.kind != ASP_COMPRESS_NONE) f([&h](uint64_t i) { return h.get(i); });
-    else if (h.dtype == ASP_U8) f([p = (const uint8_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
-    else if (h.dtype == ASP_U16) f([p = (const uint16_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
-    else if (h.dtype == ASP_U32) f([p = (const uint32_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
-    else f([p = (const uint64_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
-}
-// Whether rows of y come once each: ascending ones, or a list of what has come
-struct Distinct
-{
-    const uint64_t n;
-    const bool ascending;
-    uint64_t next = 0;
-    std::vector<bool> seen;
-    Distinct(uint64_t rows, bool in_order) : n(rows), ascending(in_order), seen(in_order ? 0 : rows, false) {}
-    bool operator()(uint64_t row)
-    {
-        if (row >= n || (ascending ? row < next : (bool)seen[row])) return false;
-        if (ascending) next = row + 1;
-        else seen[row] = true;
-        return true;
-    }
-};
-uint64_t row_in_y(const asp_plan_desc &d, const HostMeta &perm, int sort_kind, uint64_t r)
-{
-    return sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
-}
-const uint64_t kMostRun = 4096; // elements of a row of the CSR5-like templates that is listed
-const uint64_t kSharedRows = 1u << 14; // from so many on, the rows of a list are shared out
-
-// Lists of the rows of a (validated) plan, as the kernels of kernels_rows.cu take them. false: another template, a row in two places, or offsets
-// beyond 32 bits.
-//
-// Chunks of a row one after the other, `longest` row
-bool list_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, asp::HostBuf<uint2> &out, uint64_t &longest)
-{
-    using namespace asp;
-    const bool cta = d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE, chunks = cta || d.template_type == ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE;
-    if ((!chunks && d.template_type != ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE) || d.n_rows > 0xffffffffull) return false;
-    Distinct distinct(d.n_rows, d.sort_kind == ASP_SORT_NONE);
-    const HostMeta &offsets = hm[cta ? MS_BLK_NZ : MS_WARP_NZ];
-    out.make(d.n_rows + 1);
-    uint64_t end = 0, n = 0;
-    longest = 0;
-    auto put = [&](uint64_t row, uint64_t from, uint64_t to) {
-        if (to < from || to > 0xffffffffull || (n > 0 && from != end) || !distinct(row)) return false;
-        end = to;
-        longest = std::max(longest, to - from);
-        out.p[n++] = make_uint2((unsigned)from, (unsigned)row);
-        return true;
-    };
-    bool good = true;
-    if (chunks)
-        with_entries(hm[MS_ROW_OF_UNIT], [&](auto of) {
-            with_entries(offsets, [&](auto nz) {
-                const uint64_t units = cta ? a.n_units : a.effective, radd = a.row_add ? d.first_row : 0;
-                for (uint64_t u = 0; u < units && good;)
-                {
-                    uint64_t e = u + 1;
-                    const uint64_t row = of(u);
-                    while (e < units && of(e) == row) e++;
-                    good = put(row + radd, nz(u), nz(e));
-                    u = e;
-                }
-            });
-        });
-    else
-    {
-        const HostMeta &row = hm[MS_BLK_ROW], &warp = hm[MS_BLK_WARP];
-        const uint64_t B = a.n_units, rows = std::min<uint64_t>(row.get(B), a.effective), warps = warp.get(B);
-        if (!has_entries(offsets, warps + 1) || !has_entries(hm[MS_ROW_OFF], row.get(B) + 1)) return false;
-        with_entries(hm[MS_ROW_OFF], [&](auto off) {
-            with_entries(offsets, [&](auto nz) {
-                for (uint64_t b = 0; b < B && good; b++)
-                {
-                    const uint64_t r0 = row.get(b), r1 = std::min(row.get(b + 1), rows), w0 = warp.get(b), g0 = off(r0);
-                    for (uint64_t r = r0; r < r1 && good; r++)
-                    {
-                        const uint64_t lo = w0 + off(r) - g0, hi = w0 + off(r + 1) - g0;
-                        good = lo <= warps && hi <= warps && put(row_in_y(d, perm, a.sort_kind, r), nz(lo), nz(hi));
-                    }
-                }
-            });
-        });
-    }
-    if (!good || n == 0) return false;
-    out.p[n] = make_uint2((unsigned)end, 0);
-    out.n = n + 1;
-    return true;
-}
-
-// Row-grouped; `tlbs` of all rows, `most` of one
-bool list_tlb_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, asp::HostBuf<uint4> &out, uint64_t &tlbs, uint64_t &most)
-{
-    using namespace asp;
-    if (d.template_type != ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || d.n_rows > 0xffffffffull) return false;
-    const HostMeta &row = hm[MS_BLK_ROW];
-    const uint64_t B = a.n_units, rows = std::min<uint64_t>(row.get(B), a.effective);
-    if (row.get(0) != 0 || rows == 0 || rows > d.n_rows || !has_entries(hm[MS_ROW_OFF], row.get(B) + 1)) return false;
-    Distinct distinct(d.n_rows, a.sort_kind == ASP_SORT_NONE);
-    out.make(rows);
-    std::atomic<uint64_t> all(0), top(0);
-    std::atomic<bool> good(true);
-    with_entries(hm[MS_ROW_OFF], [&](auto off) {
-        host::share_ranges(B, a.sort_kind == ASP_SORT_NONE && rows >= kSharedRows, [&](uint64_t b, uint64_t e) {
-            uint64_t sum = 0, longest = 0;
-            bool in = true;
-            for (; b < e && in; b++)
-            {
-                const uint64_t nz = hm[MS_BLK_NZ].get(b), n = hm[MS_BLK_THR].get(b + 1) - hm[MS_BLK_THR].get(b), S = hm[MS_TLB_SIZE].get(b);
-                const uint64_t r0 = row.get(b), r1 = std::min(row.get(b + 1), rows), g0 = off(r0);
-                in = S > 0 && S <= 0xffff && nz + n * S <= 0xffffffffull;
-                for (uint64_t r = r0; r < r1 && in; r++)
-                {
-                    const uint64_t lo = off(r) - g0, hi = off(r + 1) - g0, y = row_in_y(d, perm, a.sort_kind, r);
-                    // (unsorted rows ascend with r, and the BLBs' rows follow one another)
-                    in = lo <= hi && hi <= n && hi - lo <= 0xffff && y < d.n_rows && (a.sort_kind == ASP_SORT_NONE || distinct(y));
-                    sum += hi - lo;
-                    longest = std::max(longest, hi - lo);
-                    out.p[r] = make_uint4((unsigned)(nz + lo), (unsigned)y, (unsigned)((hi - lo) | S << 16), (unsigned)n);
-                }
-                in = in && row.get(b + 1) >= r0;
-            }
-            all.fetch_add(sum);
-            host::raise<uint64_t>(top, longest);
-            if (!in) good = false;
-        });
-    });
-    tlbs = all;
-    most = top;
-    return good;
-}
-
-// ELL- and SELL-like; `place` stays empty where TLB t is row first + t. `longest` TLB, `rows` that are stored.
-bool list_strips(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const asp::KArgs &a, asp::HostBuf<uint4> &out, asp::HostBuf<unsigned> &place, uint64_t &first, uint64_t &longest, uint64_t &rows)
-{
-    using namespace asp;
-    const bool ell = d.template_type == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS;
-    if ((!ell && d.template_type != ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS) || d.n_rows > 0xffffffffull) return false;
-    const HostMeta &of = hm[MS_ROW_OF_TLB];
-    const uint64_t radd = a.row_add ? d.first_row : 0, B = ell ? 1 : a.n_units;
-    const bool numbered = of.kind == ASP_COMPRESS_LINEAR && of.coef == 1;
-    longest = rows = 0;
-    first = numbered ? of.icpt + radd : 0;
-    out.make(std::min<uint64_t>(a.effective, ell ? a.n_tlb : hm[MS_BLK_THR].get(B)) / 32 + B + 1);
-    uint64_t k = 0;
-    for (uint64_t b = 0; b < B; b++)
-    {
-        const uint64_t nz = ell ? 0 : hm[MS_BLK_NZ].get(b), t0 = ell ? 0 : hm[MS_BLK_THR].get(b);
-        const uint64_t n = ell ? a.n_tlb : hm[MS_BLK_THR].get(b + 1) - t0, S = ell ? a.tlb_size : hm[MS_TLB_SIZE].get(b);
-        if (S == 0 || S > 0xffff || nz + n * S > 0xffffffffull || (t0 != rows && t0 < a.effective)) return false;
-        longest = std::max(longest, S);
-        for (uint64_t t = t0; t < t0 + n && t < a.effective; t += 32)
-        {
-            const uint64_t m = std::min<uint64_t>({32, t0 + n - t, a.effective - t});
-            out.p[k++] = make_uint4((unsigned)(nz + t - t0), (unsigned)t, (unsigned)(S | m << 16), (unsigned)n);
-            rows += m;
-        }
-    }
-    out.n = k;
-    if (k == 0) return false;
-    if (numbered) return first + rows <= d.n_rows;
-    if (!has_entries(of, rows)) return false;
-    Distinct distinct(d.n_rows, false);
-    place.make(rows);
-    bool good = true;
-    with_entries(of, [&](auto row) {
-        for (uint64_t i = 0; i < rows && good; i++)
-        {
-            good = distinct(row(i) + radd);
-            place.p[i] = (unsigned)(row(i) + radd);
-        }
-    });
-    return good;
-}
-
-// CSR5-like: {first element, row, elements, 0}
-bool list_runs(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp::KArgs &a, asp::HostBuf<uint4> &out)
-{
-    using namespace asp;
-    const uint64_t S = a.tlb_size, rmask = (1ull << a.bits_row) - 1;
-    if ((d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE && d.template_type != ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE) ||
-        d.n_rows > 0xffffffffull || S == 0 || S >= 64)
-        return false;
-    // (a row that is too long is seen by the warps that begin in it)
-    const uint64_t within = kMostRun / (32 * S) + 1;
-    for (uint64_t w = 0; w + within < a.n_units; w++)
-        if (hm[MS_ROW_OF_UNIT].get(w) == hm[MS_ROW_OF_UNIT].get(w + within)) return false;
-    Distinct distinct(d.n_rows, a.sort_kind == ASP_SORT_NONE);
-    out.make(d.n_rows);
-    uint64_t r = ~0ull, n = 0; // of the matrix's rows in order
-    bool good = true;
-    with_entries(hm[MS_COMBINE], [&](auto words) {
-        for (uint64_t w = 0; w < a.n_units && good; w++)
-        {
-            const uint64_t R0 = hm[MS_ROW_OF_UNIT].get(w);
-            good = (words(w * 32) >> (a.bits_word - 1)) & 1ull; // (a warp's first element always starts a row)
-            for (uint64_t l = 0; l < 32 && good; l++)
-            {
-                const uint64_t word = words(w * 32 + l), e0 = (w * 32 + l) * S;
-                uint64_t next = R0 + (word & rmask);
-                // the flags, first element first, at the top of the word
-                for (uint64_t f = word >> (a.bits_word - (int)S) << (64 - S); f != 0 && good; f &= ~(1ull << (63 - __builtin_clzll(f))), next++)
-                {
-                    if (next == r) continue; // goes on from the warp before
-                    r = next;
-                    const uint64_t e = e0 + (uint64_t)__builtin_clzll(f), row = row_in_y(d, perm, a.sort_kind, r);
-                    good = distinct(row);
-                    if (!good) break;
-                    if (n > 0) out.p[n - 1].z = (unsigned)(e - out.p[n - 1].x);
-                    out.p[n++] = make_uint4((unsigned)e, (unsigned)row, 0, 0);
-                }
-            }
-        }
-    });
-    if (!good || n == 0) return false;
-    out.p[n - 1].z = (unsigned)(a.n_units * 32 * S - out.p[n - 1].x);
-    out.n = n;
-    return true;
-}
-
-// Whole rows for a few lanes, a warp or a CTA, where that is the faster way (kernels_rows.cu). A warp takes up to 512 elements (four trips
-// of 1.2 us; chunks in parallel are faster beyond that), a CTA rows of 256 and more on average, up to 16384 (four trips of 1024 threads).
-// Rows that are TLBs of more than 8 elements: up to 3 M elements (what L2 holds). CSR5-like: up to 512 K elements (FEM, fp32: 445 K 6 -> 3.1 us, 730 K
-// 6.5 -> 5.1, but lists of a million elements cost more to make than that is worth) and rows of 4096 (four trips of a CTA).
-// Rows of TLBs: up to 2 M elements, beyond which the CTA's long strips stream better (4.9 M, FEM, fp32: 13.0 us, 17.3 by rows; 1.6 M: 7.2, 5.1).
-struct OwnRows
-{
-    asp::RowArgs args = {};
-    asp::HostBuf<uint2> rows; // (one of the two)
-    asp::HostBuf<uint4> tlbs;
-    asp::HostBuf<unsigned> place;
-    uint64_t trips = 0;  // of warps that take a row
-    uint64_t listed = 0; // rows of y
-    bool strips = false, runs = false; // (in `tlbs`)
-    const void *data() const { return tlbs.n == 0 ? (const void *)rows.p : tlbs.p; }
-    size_t bytes() const { return rows.bytes() + tlbs.bytes(); }
-    void none()
-    {
-        rows = {};
-        tlbs = {};
-        place = {};
-    }
-    // f(row of y) for all of them
-    template <class F>
-    void each_row(F &&f) const
-    {
-        for (uint64_t i = 0; i + 1 < rows.n; i++) f(rows.p[i].y);
-        for (uint64_t i = 0; i < tlbs.n; i++)
-            if (!strips) f(tlbs.p[i].y);
-            else if (place.n == 0)
-                for (unsigned k = 0; k < tlbs.p[i].z >> 16; k++) f(args.first_row + tlbs.p[i].y + k);
-        for (uint64_t i = 0; i < place.n; i++) f(place.p[i]);
-    }
-    // few: one of several sub-matrices, which a kernel each takes one after the other
-    void make(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp_plan &p, int sm_count, bool few = false)
-    {
-        try
-        {
-            if (!list(d, hm, perm, p, sm_count, few)) none();
-        }
-        catch (const std::bad_alloc &) // (not enough host memory: the template's own kernel)
-        {
-            none();
-        }
-    }
-
-  private:
-    bool list(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const asp_plan &p, int sm_count, bool few)
-    {
-        uint64_t longest = 0, all = 0;
-        switch (d.template_type)
-        {
-        case ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS:
-        case ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS:
-            strips = true;
-            if (p.stored > (3u << 20) || !list_strips(d, hm, p.args, tlbs, place, all, longest, listed)) return false;
-            args.first_row = (unsigned)all;
-            args.lanes = longest <= 16 ? 4 : longest <= 32 ? 8 : 16;
-            args.n = (unsigned)tlbs.n;
-            return longest > 8 || few;
-        case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE:
-        case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE:
-        {
-            runs = true;
-            if (p.stored > (1u << 19) || !list_runs(d, hm, perm, p.args, tlbs)) return false;
-            listed = tlbs.n;
-            args.size = p.args.tlb_size;
-            args.n = (unsigned)listed;
-            args.lanes = p.stored <= 6 * listed ? 4 : p.stored <= 12 * listed ? 8 : 16;
-            for (uint64_t i = 0; i < listed; i++) longest = std::max<uint64_t>(longest, tlbs.p[i].z);
-            if (longest > kMostRun) return false;
-            // rows that take its lanes more than two trips are a CTA's
-            uint4 *const first = std::stable_partition(tlbs.p, tlbs.p + listed, [&](const uint4 &r) { return r.z > 8 * args.lanes; });
-            args.hubs = (unsigned)(first - tlbs.p);
-            return true;
-        }
-        case ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS:
-            if (p.stored > (2u << 20) || !list_tlb_rows(d, hm, perm, p.args, tlbs, all, longest)) return false;
-            listed = tlbs.n;
-            args.n = (unsigned)listed;
-            args.lanes = 2;
-            while (args.lanes < 32 && args.lanes * listed < all) args.lanes *= 2;
-            return longest <= 8 * args.lanes;
-        default: break;
-        }
-        if (!list_rows(d, hm, perm, p.args, rows, longest)) return false;
-        listed = rows.n - 1;
-        const uint64_t elements = rows.p[listed].x - rows.p[0].x;
-        if (longest > 512 && (longest > 16384 || elements < 256 * listed)) return false;
-        // threads for all of a row in one trip while all rows are on the device at once, else for two
-        const uint64_t per = listed <= 2ull * sm_count ? 4 : 8;
-        args.cta = longest <= 512 ? 0 : (unsigned)std::min<uint64_t>(1024, std::max<uint64_t>(64, (longest + 32 * per - 1) / (32 * per) * 32));
-        args.n = (unsigned)listed;
-        for (uint64_t i = 0; i < listed && args.cta == 0; i++) trips += (rows.p[i + 1].x - rows.p[i].x + 127) / 128;
-        return true;
-    }
-};
 
 asp_status ensure_xy(asp_ctx *ctx, size_t xb, size_t yb)
 {
@@ -1436,9 +1113,9 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         src.push_back(t);
     }
     // (a matrix so large that its gathers are scattered has the layout anyway: its rows are listed only where it turns out not to)
-    OwnRows own;
+    asp::OwnRows own;
     const bool listed = n == 1 && made[0]->templ != ASP_EMPTY_TEMPLATE && descs[0].true_nnz <= (8u << 20);
-    if (listed) own.make(descs[0], metas[0], perms[0], *made[0], ctx->sm_count);
+    if (listed) own.make(descs[0], metas[0], perms[0], made[0]->args, made[0]->stored, ctx->sm_count);
     if (src.size() == 1) src[0].whole_rows = own.bytes() > 0, src[0].trips = own.trips;
     asp::TiledHost th;
     std::shared_ptr<TiledGroup> tg;
@@ -1506,8 +1183,8 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
             for (asp_plan *p : made) p->tiled = tg;
         }
     }
-    if (n == 1 && !tg && !listed) own.make(descs[0], metas[0], perms[0], *made[0], ctx->sm_count);
-    std::vector<OwnRows> owns;
+    if (n == 1 && !tg && !listed) own.make(descs[0], metas[0], perms[0], made[0]->args, made[0]->stored, ctx->sm_count);
+    std::vector<asp::OwnRows> owns;
     if (n == 1) owns.push_back(std::move(own));
     else if (!tg)
     {
@@ -1521,8 +1198,8 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         {
             owns.emplace_back();
             if (made[i]->templ == ASP_EMPTY_TEMPLATE) continue;
-            OwnRows &o = owns.back();
-            o.make(descs[i], metas[i], perms[i], *made[i], ctx->sm_count, true);
+            asp::OwnRows &o = owns.back();
+            o.make(descs[i], metas[i], perms[i], made[i]->args, made[i]->stored, ctx->sm_count, true);
             good = o.bytes() > 0 && descs[i].n_rows == descs[0].n_rows;
             if (good) o.each_row([&](uint64_t r) {
                 good = good && r < seen.size() && !seen[r];
@@ -1535,7 +1212,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
     const uint64_t group = ++groups;
     for (size_t i = 0; i < owns.size() && !tg; i++)
     {
-        const OwnRows &o = owns[i];
+        const asp::OwnRows &o = owns[i];
         if (o.bytes() == 0) continue;
         const size_t places = align_up(o.bytes(), 256), bytes = align_up(places + o.place.bytes(), 256);
         std::shared_ptr<Arena> list = arena;

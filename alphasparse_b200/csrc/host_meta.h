@@ -46,5 +46,7 @@ struct HostMeta
         }
     }
 };
+// a closed form, or an array of at least `count` entries
+inline bool has_entries(const HostMeta &h, uint64_t count) { return h.kind != ASP_COMPRESS_NONE || h.len >= count; }
 } // namespace asp
 #endif
