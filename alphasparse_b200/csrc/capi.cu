@@ -169,7 +169,7 @@ struct asp_plan
     std::shared_ptr<Arena> row_list;
     asp::RowArgs own_rows = {};
     uint64_t own_rows_n = 0;  // rows of y in the list
-    uint64_t rows_group = 0; // plans of one number have no row of y in common
+    uint64_t rows_group = 0; // plans of one number: no other writes a row that one of them lists (0: no lists)
     int64_t asked_tblock = 0, asked_threads = 0, asked_reduce = 0; // the launch last requested (re-applied when vec / path change)
 };
 
@@ -615,6 +615,47 @@ asp_status asp_synchronize(asp_ctx *ctx)
 
 namespace
 {
+// Lists of several small sub-matrices' rows: a kernel each on one stream instead of a stream each, which takes 15 us of events (three strips,
+// 5,000 rows: fp32 21.6 -> 8.2 us, fp64 43.9 -> 12.7; the templates' kernels one after the other 28.9 and 57.8). All of them can have one and no row is in two, or none has. Where bits must not depend on which
+// plans are EMPTY (kSameBits), that is so for the plans that add to y, in no order anyway; a plan that does not (is_atom_add == 0: its rows are its own) has a
+// list if it can have one by itself.
+void list_strips(const asp_plan_desc *descs, int n, const std::vector<std::vector<HostMeta>> &metas, const std::vector<HostMeta> &perms, const std::vector<asp_plan *> &made, bool complete, int sm_count,
+                 std::vector<asp::OwnRows> &owns)
+{
+    uint64_t stored = 0, true_nnz = 0;
+    for (int i = 0; i < n; i++) stored += made[i]->stored, true_nnz += descs[i].true_nnz;
+    const bool small = true_nnz < asp::kSameBits;
+    if (!small && (!complete || stored > (1u << 20))) return;
+    const auto alone = [&](int i) { return small && !made[i]->args.atomic; };
+    try
+    {
+        std::vector<bool> seen(descs[0].n_rows, false);
+        owns.resize(n);
+        // false: no list, or a row that has come before
+        auto make = [&](int i) {
+            bool good = made[i]->stored <= (1u << 20) && descs[i].n_rows == descs[0].n_rows;
+            if (good) owns[i].make(descs[i], metas[i], perms[i], made[i]->args, made[i]->stored, sm_count, true);
+            good = owns[i].bytes() > 0;
+            owns[i].each_row([&](uint64_t r) {
+                good = good && !seen[r];
+                seen[r] = true;
+            });
+            return good;
+        };
+        bool good = true, together = true;
+        for (int i = 0; i < n && good; i++)
+            if (made[i]->templ != ASP_EMPTY_TEMPLATE && alone(i)) good = make(i) || owns[i].bytes() == 0;
+        for (int i = 0; i < n && good && together; i++)
+            if (made[i]->templ != ASP_EMPTY_TEMPLATE && !alone(i)) together = make(i);
+        for (int i = 0; i < n; i++)
+            if (!good || (!together && !alone(i))) owns[i].none();
+    }
+    catch (const std::bad_alloc &) // (not enough host memory: the templates' own kernels)
+    {
+        owns.clear();
+    }
+}
+
 // dry == true: everything asp_plan_group_create checks, without a device (no allocation, no upload, no
 // plan objects returned); ctx may then be NULL.
 asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int layout, asp_plan **out_plans, bool dry)
@@ -1093,11 +1134,13 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
     }
     // scattered columns: the column-tiled layout of the whole group (kernels_tiled.cu), where it is the faster one
     std::vector<asp::TiledSource> src;
-    bool same = layout == ASP_LAYOUT_AUTO;
+    // a group with parts left out is a trial of the others: those run what they run under ASP_LAYOUT_NONE
+    bool complete = layout == ASP_LAYOUT_AUTO;
+    for (int i = 0; i < n; i++) complete = complete && descs[i].template_type != ASP_EMPTY_TEMPLATE;
+    bool same = complete;
     for (int i = 0; i < n && same; i++)
     {
-        same = same && descs[i].val_dtype == descs[0].val_dtype && descs[i].n_rows == descs[0].n_rows && descs[i].n_cols == descs[0].n_cols;
-        if (descs[i].template_type == ASP_EMPTY_TEMPLATE) same = false; // a group with parts left out is a trial of one part
+        same = descs[i].val_dtype == descs[0].val_dtype && descs[i].n_rows == descs[0].n_rows && descs[i].n_cols == descs[0].n_cols;
         if (!same) break;
         asp::TiledSource t;
         t.templ = descs[i].template_type;
@@ -1114,7 +1157,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
     }
     // (a matrix so large that its gathers are scattered has the layout anyway: its rows are listed only where it turns out not to)
     asp::OwnRows own;
-    const bool listed = n == 1 && made[0]->templ != ASP_EMPTY_TEMPLATE && descs[0].true_nnz <= (8u << 20);
+    const bool listed = n == 1 && complete && descs[0].true_nnz <= (8u << 20);
     if (listed) own.make(descs[0], metas[0], perms[0], made[0]->args, made[0]->stored, ctx->sm_count);
     if (src.size() == 1) src[0].whole_rows = own.bytes() > 0, src[0].trips = own.trips;
     asp::TiledHost th;
@@ -1183,31 +1226,10 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
             for (asp_plan *p : made) p->tiled = tg;
         }
     }
-    if (n == 1 && !tg && !listed) own.make(descs[0], metas[0], perms[0], made[0]->args, made[0]->stored, ctx->sm_count);
+    if (n == 1 && complete && !tg && !listed) own.make(descs[0], metas[0], perms[0], made[0]->args, made[0]->stored, ctx->sm_count);
     std::vector<asp::OwnRows> owns;
     if (n == 1) owns.push_back(std::move(own));
-    else if (!tg)
-    {
-        // Several small sub-matrices, if all of them can have it and no row is in two: a kernel each on one stream instead of a stream each, which
-        // takes 15 us of events (three strips, 5,328 rows: fp32 21.4 -> 7.8 us, fp64 26.9 -> 8.7)
-        uint64_t stored = 0;
-        for (const asp_plan *p : made) stored += p->stored;
-        bool good = stored <= (1u << 20) && descs[0].n_rows <= 0xffffffffull;
-        std::vector<bool> seen(good ? descs[0].n_rows : 0, false);
-        for (int i = 0; i < n && good; i++)
-        {
-            owns.emplace_back();
-            if (made[i]->templ == ASP_EMPTY_TEMPLATE) continue;
-            asp::OwnRows &o = owns.back();
-            o.make(descs[i], metas[i], perms[i], made[i]->args, made[i]->stored, ctx->sm_count, true);
-            good = o.bytes() > 0 && descs[i].n_rows == descs[0].n_rows;
-            if (good) o.each_row([&](uint64_t r) {
-                good = good && r < seen.size() && !seen[r];
-                if (good) seen[r] = true;
-            });
-        }
-        if (!good) owns.clear();
-    }
+    else if (layout == ASP_LAYOUT_AUTO && !tg) list_strips(descs, n, metas, perms, made, complete, ctx->sm_count, owns);
     static std::atomic<uint64_t> groups{0};
     const uint64_t group = ++groups;
     for (size_t i = 0; i < owns.size() && !tg; i++)
@@ -1242,8 +1264,8 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         (o.strips ? (const void *&)p->own_rows.strips : o.runs ? (const void *&)p->own_rows.runs : o.tlbs.n == 0 ? (const void *&)p->own_rows.rows : (const void *&)p->own_rows.tlbs) = to;
         if (o.place.n > 0) p->own_rows.place = (const unsigned *)(to + places);
         p->own_rows_n = o.listed;
-        p->rows_group = group;
         p->row_list = list;
+        for (asp_plan *q : made) q->rows_group = group;
     }
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess)
@@ -1492,40 +1514,29 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
             }
         }
     }
-    // Whole rows, where all plans have lists of them and no row is in two: they are stored, whatever was in y. (A plan may leave out rows, and so may a
-    // call plans of a group: y is cleared for those.) Who leaves y as it is gets the templates' kernels.
+    // Whole rows, for the plans that have lists of them: they are stored, whatever was in y, so no other plan of the call may write them, which is what a
+    // group's lists are made for. (A plan may leave out rows, and so may a call plans of a group: y is cleared for those.) Who
+    // leaves y as it is gets the templates' kernels.
     uint64_t listed = 0;
-    bool by_rows = g.first != nullptr && zero_y != 0;
+    bool by_rows = zero_y != 0;
     for (int i = 0; i < n_plans && by_rows; i++)
     {
-        const asp_plan *p = plans[i];
-        if (p->templ == ASP_EMPTY_TEMPLATE) continue;
-        by_rows = p->row_list && p->rows_group == g.first->rows_group && (clear || !p->args.atomic);
-        for (int j = 0; j < i; j++) by_rows = by_rows && plans[j] != p;
-        listed += p->own_rows_n;
+        if (plans[i]->templ == ASP_EMPTY_TEMPLATE) continue;
+        by_rows = plans[i]->rows_group != 0 && plans[i]->rows_group == g.first->rows_group;
+        for (int j = 0; j < i; j++) by_rows = by_rows && plans[j] != plans[i];
+        if (plans[i]->row_list) listed += plans[i]->own_rows_n;
     }
-    if (by_rows)
-    {
-        if (clear && listed < g.n_rows) ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
-        for (int i = 0; i < n_plans; i++)
-        {
-            const asp_plan *p = plans[i];
-            if (p->templ == ASP_EMPTY_TEMPLATE) continue;
-            asp::RowArgs rows = p->own_rows;
-            rows.x = (const char *)d_x + p->args.first_col * g.es;
-            rows.y = d_y;
-            ASP_CUDA(asp::launch_own_rows(p->val_is_f64, p->col_width, rows, ctx->stream));
-        }
-        return ASP_OK;
-    }
+    by_rows = by_rows && listed > 0;
+    const auto own_rows = [by_rows](const asp_plan *p) { return by_rows && p->row_list != nullptr; };
     const asp_plan *only = n_plans == 1 ? plans[0] : nullptr;
-    if (clear && only && only->ends_cover && only->end_rows)
+    if (by_rows) clear = clear && listed < g.n_rows;
+    if (clear && only && !by_rows && only->ends_cover && only->end_rows)
         ASP_CUDA(asp::launch_zero_rows(only->val_is_f64, d_y, (const unsigned *)only->end_rows->base, only->n_end_rows, ctx->stream));
-    else if (clear && !(only && only->stores_all_rows))
+    else if (clear && (by_rows || !(only && only->stores_all_rows)))
         ASP_CUDA(asp::launch_clear(g.es == 8, d_y, g.n_rows, (unsigned)ctx->sm_count, ctx->stream));
     if (!g.first) return ASP_OK;
     int active = 0;
-    for (int i = 0; i < n_plans; i++) active += plans[i]->templ != ASP_EMPTY_TEMPLATE;
+    for (int i = 0; i < n_plans; i++) active += plans[i]->templ != ASP_EMPTY_TEMPLATE && !own_rows(plans[i]);
     const bool fork = active > 1;
     if (fork) ASP_CUDA(cudaEventRecord(ctx->ev_fork, ctx->stream));
     bool used[asp_ctx::kAux] = {false, false, false};
@@ -1534,7 +1545,7 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
     for (int i = 0; i < n_plans && result == ASP_OK; i++)
     {
         const asp_plan *p = plans[i];
-        if (p->templ == ASP_EMPTY_TEMPLATE) continue;
+        if (p->templ == ASP_EMPTY_TEMPLATE || own_rows(p)) continue;
         cudaStream_t st = ctx->stream;
         if (fork && k > 0)
         {
@@ -1556,6 +1567,16 @@ asp_status asp_spmv(asp_ctx *ctx, asp_plan *const *plans, int n_plans, const voi
         args.x = d_x;
         args.y = d_y;
         cudaError_t e = asp::launch_template(p->templ, p->val_is_f64, p->col_width, args, p->grid, p->block, p->smem, st, p->vec);
+        if (e != cudaSuccess) result = cuda_fail(e, "kernel launch");
+    }
+    for (int i = 0; i < n_plans && result == ASP_OK; i++)
+    {
+        const asp_plan *p = plans[i];
+        if (p->templ == ASP_EMPTY_TEMPLATE || !own_rows(p)) continue;
+        asp::RowArgs rows = p->own_rows;
+        rows.x = (const char *)d_x + p->args.first_col * g.es;
+        rows.y = d_y;
+        const cudaError_t e = asp::launch_own_rows(p->val_is_f64, p->col_width, rows, ctx->stream);
         if (e != cudaSuccess) result = cuda_fail(e, "kernel launch");
     }
     // always join the side streams that were forked, also after a failed launch

@@ -445,6 +445,8 @@ struct StopRule
     }
 };
 
+const uint64_t kListedNnz = 3u << 20; // of a matrix whose rows may be listed (row_lists.h)
+
 struct Pick
 {
     Candidate cand;
@@ -660,6 +662,8 @@ asp_status asp::host::search(const asp_matrix *m, const asp_search_options *opt_
                         continue;
                     }
                 }
+                bool timed = false;
+                Pick here{};
                 for (const Launch &l : launches)
                 {
                     std::vector<int64_t> tb(n, 1), th(n, 32), rd(n, 1);
@@ -688,16 +692,30 @@ asp_status asp::host::search(const asp_matrix *m, const asp_search_options *opt_
                     snprintf(buf, sizeof buf, "  sub %d [%llu rows, nnz/row %llu..%llu] %s threads=%lld reduce=%lld: %.1f us", sub, (unsigned long long)rows, (unsigned long long)mn,
                              (unsigned long long)mx, cand.name.c_str(), (long long)l.threads, (long long)l.reduce, ms * 1e3);
                     log(buf);
-                    if (!have || ms < bestp.ms)
+                    if (!timed || ms < here.ms)
                     {
-                        bestp = {cand, l, ms};
-                        have = true;
+                        here = {cand, l, ms};
+                        timed = true;
                     }
                     if (rule && !rule->go_on(2.0 * (double)nnz * 1e-6 / ms))
                     {
                         stop = true;
                         break;
                     }
+                }
+                // whole rows of a small matrix, with the launch that its template's kernel would have
+                float rows_ms = 0;
+                if (timed && n == 1 && layout_fn && nnz <= kListedNnz && layout_fn(time_user, f.get(), opt.warmup, opt.reps, &rows_ms) == 0 && rows_ms > 0)
+                {
+                    char buf[256];
+                    snprintf(buf, sizeof buf, "  sub 0 %s, by what replaces its kernel: %.1f us", cand.name.c_str(), rows_ms * 1e3);
+                    log(buf);
+                    here.ms = std::min(here.ms, rows_ms);
+                }
+                if (timed && (!have || here.ms < bestp.ms))
+                {
+                    bestp = here;
+                    have = true;
                 }
                 if (stop)
                 {
@@ -733,7 +751,7 @@ asp_status asp::host::search(const asp_matrix *m, const asp_search_options *opt_
         float layout_ms = 0;
         if (layout_fn && layout_fn(time_user, f.get(), opt.warmup, std::max(opt.reps, 20), &layout_ms) == 0 && layout_ms > 0)
         {
-            snprintf(buf, sizeof buf, "  whole matrix, column-tiled layout: %.1f us  %.1f GFLOP/s", layout_ms * 1e3, 2.0 * (double)total_nnz * 1e-6 / layout_ms);
+            snprintf(buf, sizeof buf, "  whole matrix, column-tiled layout or whole rows: %.1f us  %.1f GFLOP/s", layout_ms * 1e3, 2.0 * (double)total_nnz * 1e-6 / layout_ms);
             log(buf);
             if (layout_ms < ms)
             {

@@ -817,10 +817,8 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
         const double rate = std::max(lines / (0.85 * 290e3), bytes_us);
         return (src.size() > 1 ? 8.0 : 0.0) + std::max(2.0 + chain, 3.0 + rate + std::min(0.4 * rate, 4.5));
     };
-    // Small groups of several strips keep their kernels although the layout is faster (three strips, 33,000 non-zeros: 22 us; 73,000: 24
-    // against 6 us): whoever checks strips one by one, the others EMPTY, finds the bits of the whole group in them, and did so before
-    // there was a layout. Checks of that kind run on small matrices; for larger ones ASP_LAYOUT_NONE has to be asked for.
-    if (src.size() > 1 && true_nnz < (1u << 16)) return false;
+    // (the layout would be faster: three strips, 33,000 non-zeros: 22 us; 73,000: 24 against 6 us)
+    if (src.size() > 1 && true_nnz < kSameBits) return false;
     // small matrices, whose time is the launch, stay with their kernels (not worth a look at the columns)
     if (own(requests) < (whole ? 5.0 : 7.0)) return false;
     double lines = 0;

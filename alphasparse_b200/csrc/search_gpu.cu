@@ -1,7 +1,8 @@
 // asp_search with the GPU as the timer: a trial's format is uploaded once, its launch parameters are
 // swept in place, and asp_time measures it (replaces the reference's emit + nvcc + run per trial).
-// Trials run the templates' kernels, whole matrices as well as one strip with the others EMPTY. The column-tiled layout, which takes
-// no launch parameters and is the same for every template, is timed once per dense view, on the winners' format.
+// Trials run the templates' kernels, whole matrices as well as one strip with the others EMPTY. What takes no launch parameters is a candidate of its
+// own: the column-tiled layout, which is the same for every template, and kernels for whole rows once per dense view, on the winners' format; whole rows
+// of a small matrix in one piece, which are not the same for every template, once per format too.
 //
 // Launch requests that the kernels fold into the same effective launch (a CTA width above a family's compiled
 // bound becomes more CTAs, grids are cut to the CTAs that have work: asp_plan_get_launch) are timed once: a
@@ -97,10 +98,13 @@ int time_layout_on_gpu(void *user, const asp_format *fmt, int warmup, int reps, 
     std::vector<asp_plan_desc> descs(n);
     if (asp_format_plan_descs(fmt, descs.data()) != ASP_OK) return 1;
     t->plans.assign(n, nullptr);
-    bool ok = asp_plan_group_create_with(t->ctx, descs.data(), n, ASP_LAYOUT_AUTO, t->plans.data()) == ASP_OK && asp_plan_layout_bytes(t->plans[0]) > 0;
+    bool ok = asp_plan_group_create_with(t->ctx, descs.data(), n, ASP_LAYOUT_AUTO, t->plans.data()) == ASP_OK;
+    const bool layout = ok && asp_plan_layout_bytes(t->plans[0]) > 0;
+    bool rows = false;
+    for (int i = 0; i < n && ok; i++) rows = rows || asp_plan_whole_rows(t->plans[i]);
     float gflops = 0;
-    // (with y cleared: the calls in which the layout runs whatever rows are empty)
-    ok = ok && asp_time(t->ctx, t->plans.data(), n, warmup, reps, 1, 0.0, ms, &gflops) == ASP_OK;
+    // (the layout with y cleared: the calls in which it runs whatever rows are empty)
+    ok = ok && (layout || rows) && asp_time(t->ctx, t->plans.data(), n, warmup, reps, layout ? 1 : 2, 0.0, ms, &gflops) == ASP_OK;
     t->drop();
     return ok ? 0 : 1;
 }

@@ -18,6 +18,9 @@ namespace asp
 constexpr uint32_t kTiledWarps = 32, kTiledFewWarps = 16; // warps per CTA, one CTA per SM: which of the two says kFewWarps (tiled_build.cpp)
 const uint32_t kTiledLanePieces = 2;         // pieces of a row per lane
 const uint32_t kTiledSlice = 32 * kTiledLanePieces;
+// Several plans of fewer non-zeros in all keep their templates' kernels: a row then has the same bits whichever other plans are EMPTY, as before
+// there were other kernels. Checks of that kind run on small matrices; for larger ones ASP_LAYOUT_NONE has to be asked for.
+const uint64_t kSameBits = 1u << 16;
 constexpr uint32_t kTiledTileBytes = 159u << 10; // shared memory of a tile of x
 const uint32_t kTiledNoRow = 0xffffffffu;
 const uint32_t kTiledInParts = 0x80000000u; // row entry: the rest is a place among the sums of the rows in many parts

@@ -14,7 +14,7 @@ reference's tuner:
 Every trial is an in-process lowering + upload + CUDA-event timing through the C ABI instead of an
 nvcc compile and an ~8 s run of a generated program; sub-matrices not under test carry the EMPTY
 template, as in the reference's part_execute_code_builder. Trials time the templates' kernels; the
-column-tiled layout is timed once per dense view, and the result says which of the two is faster.
+column-tiled layout is timed once per dense view, kernels for whole rows once per format of a small matrix, and the result says which are faster.
 """
 from __future__ import annotations
 

@@ -176,15 +176,17 @@ void *asp_ctx_stream(asp_ctx *ctx);
  * is also laid out by column tiles (csrc/kernels_tiled.cu), which takes 0.8 to 1.3 times the format's device memory beside it
  * (asp_plan_layout_bytes; left out where new memory for it would leave less than x, y and 256 MB free), and asp_spmv
  * over the complete group runs that layout; a group with EMPTY plans never does, nor do several plans of fewer than 65,536
- * non-zeros in all (their rows have the same bits whichever other plans are EMPTY). Sums are then taken in another order from
+ * non-zeros in all. Small plans without that layout have lists of their rows, and asp_spmv with zero_y 1 or 2 runs kernels that take whole
+ * rows (asp_plan_whole_rows). Several plans of fewer than 65,536 non-zeros in all: a plan with is_atom_add == 0 runs the same kernel, with the
+ * same bits, whichever other plans are EMPTY; of more: all plans have lists or none, and a group with EMPTY plans has none. With the layout, sums are taken in another order from
  * call to call, as with every template that accumulates with atomics (asp_plan_group_create_with can forbid it). Rows that are added up in many parts have 64-bit sums in
  * the group's device memory: a group with such rows runs the layout in the calls of the context that created it, and its
  * templates' kernels in calls of another context and in calls that a stream capture records.
  * Every entry point makes the context's device current for its own duration and restores the
  * caller's device before it returns. */
 asp_status asp_plan_group_create(asp_ctx *ctx, const asp_plan_desc *descs, int n, asp_plan **out_plans);
-/* The same, with a say in the column-tiled layout (asp_plan_group_create: ASP_LAYOUT_AUTO). ASP_LAYOUT_NONE: the group always
- * runs its templates' kernels. For plans that are used once or a few times (building the layout takes as long as hundreds of the
+/* The same, with a say in the column-tiled layout and the lists of rows (asp_plan_group_create: ASP_LAYOUT_AUTO). ASP_LAYOUT_NONE: the group
+ * has neither and always runs its templates' kernels. For plans that are used once or a few times (building the layout takes as long as hundreds of the
  * calls that it shortens), for device memory that has no room for it, for trials of launch parameters, and for results that
  * repeat bit for bit: without atomics (is_atom_add == 0; not the CSR5-like templates) every row is then summed in one fixed order,
  * whichever other plans of the group are EMPTY. */
@@ -219,8 +221,8 @@ asp_status asp_plan_set_launch(asp_plan *plan, int64_t tblock_num, int64_t threa
  * that sweeps thread_num_in_block reads back here which points of its sweep coincide. The reference has
  * no such query: its launch is the literal it printed into the program (code_of_kernal_function_call,
  * e.g. direct_atom_op_warp_block_compress.cc:1012-1040). The block-value template reports one thread per pair of block
- * rows; how its kernel shares them out among CTAs follows from the matrix. Both calls speak of the template's kernel: a group that runs
- * the column-tiled layout takes no launch parameters. Any pointer may be NULL. */
+ * rows; how its kernel shares them out among CTAs follows from the matrix. Both calls speak of the template's kernel: the column-tiled
+ * layout and the kernels for whole rows take no launch parameters. Any pointer may be NULL. */
 asp_status asp_plan_get_launch(const asp_plan *plan, int64_t *tblock_num, int64_t *thread_num_in_block, int64_t *thread_num_of_row_reduce);
 /* Work decomposition knobs, for launch-space experiments (the defaults are what the measurements in this
  * repository use): `vec` = TLBs per thread (1, 2, 4, 8 for ELL-like; 1, 2, 4 for SELL-like; 0 keeps the
@@ -228,7 +230,7 @@ asp_status asp_plan_get_launch(const asp_plan *plan, int64_t *tblock_num, int64_
  * CSR5-like bit 0 = staged write-out (the same switch as thread_num_of_row_reduce = 2), bits 4..7 = log2
  * of the rows per warp that go through shared memory (0 keeps the size chosen at plan creation).
  * Re-applies the last requested launch, and from then on asp_spmv runs this plan's own kernel (not the column-tiled layout of
- * its group). No counterpart in the reference (its generated kernels handle
+ * its group, nor one for whole rows). No counterpart in the reference (its generated kernels handle
  * one TLB per thread). */
 asp_status asp_plan_set_tuning(asp_plan *plan, int vec, int path);
 /* bytes of device memory the plan's format arrays occupy (B_fmt without x and y) */
@@ -246,8 +248,8 @@ enum
     ASP_FORM_IN_SUMS = 8
 };
 int asp_plan_layout_form(const asp_plan *plan);
-/* 1: asp_spmv of this plan alone with zero_y 1 or 2 runs a kernel that takes whole rows, instead of its template's (small matrices; the launch
- * parameters are the template's kernel's). asp_plan_set_tuning ends that. */
+/* 1: asp_spmv with zero_y 1 or 2 over this plan, alone or with others of its group (each once), runs a kernel that takes whole rows, instead of its
+ * template's (small matrices; the launch parameters are the template's kernel's). asp_plan_set_tuning ends that. */
 int asp_plan_whole_rows(const asp_plan *plan);
 /* number of launches of its template's kernel that one asp_spmv over this plan issues (excluding the y clear); the plans of a group
  * that runs the column-tiled layout share one launch */
@@ -387,7 +389,7 @@ asp_status asp_time(asp_ctx *ctx, asp_plan *const *plans, int n_plans, int warmu
                     double gflops_up_bound, float *ms_per_spmv, float *gflops);
 
 /* asp_search (asp_b200_host.h) with the GPU as the timer: every trial is uploaded once
- * (asp_plan_group_create), its launch parameters are swept with asp_plan_set_launch, and asp_time
+ * (ASP_LAYOUT_NONE; what ASP_LAYOUT_AUTO would run instead is a candidate of its own), its launch parameters are swept with asp_plan_set_launch, and asp_time
  * measures it on the context's stream. `matrix`, `options` and `result` are the asp_matrix,
  * asp_search_options and asp_search_result of asp_b200_host.h (void here so that this header stays
  * independent of the host one). Replaces the reference's compile-and-run trial

@@ -169,8 +169,8 @@ int asp_search_result_num_subs(const asp_search_result *r);
 const char *asp_search_result_sub_spec(const asp_search_result *r, int sub);
 const char *asp_search_result_sub_name(const asp_search_result *r, int sub);
 asp_status asp_search_result_sub_launch(const asp_search_result *r, int sub, int64_t *thread_num_in_block, int64_t *thread_num_of_row_reduce);
-/* asp_layout to create the winner's plans with (asp_plan_group_create_with): ASP_LAYOUT_AUTO when the column-tiled layout was the
- * faster one (or asp_search had no say in it), ASP_LAYOUT_NONE when the templates' kernels were */
+/* asp_layout to create the winner's plans with (asp_plan_group_create_with): ASP_LAYOUT_AUTO when the column-tiled layout or kernels for
+ * whole rows were the faster ones (or asp_search had no say in it), ASP_LAYOUT_NONE when the templates' kernels were */
 int asp_search_result_layout(const asp_search_result *r);
 float asp_search_result_ms(const asp_search_result *r);
 /* every timed point, one text line each: "<dense> ; sub <i> ; <strategy> ; threads ; reduce ; ms ; padding" */

@@ -13,6 +13,8 @@ NODES = {"K4": ["wlb_col_fixed 64"], "K7": ["blb_col_fixed 256"], "K8": ["row_pa
          "K2": ["row_padding 128 1", "blb_row_evenly 128", "tlb_row"], "K3": ["row_padding 32 1", "tlb_row"],
          "K9": ["tlb_nnz 16"], "K9/5": ["tlb_nnz 5"], "K9/32": ["tlb_nnz 32"], "K10": ["tlb_nnz 8"], "K10/3": ["tlb_nnz 3"],
          "K6": ["row_padding 32 1", "blb_row_evenly 32", "tlb_col_fixed 4"]}
+NO_LIST = {"K5": ["blb_row_evenly 64", "wlb_row_evenly 16", "tlb_col_fixed 4"]}
+
 
 def matrix(lengths, cols, dtype):
     """Rows of exactly these lengths."""
@@ -131,3 +133,59 @@ def test_a_tuned_plan_runs_its_own_kernel(asp_ctx, template):
     refdump.assert_y(g.spmv_host(x), y_ref, scale, np.float32, template)
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("template", sorted(NODES))
+def test_without_layouts_the_templates_kernels_run(asp_ctx, template):
+    m, x = matrix([30, 40] * 100, 3_000, np.float32)
+    desc = {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template.split("/")[0], "threads": 128, "row_reduce": 1}]}
+    y_ref, scale = refdump.csr_ref(m, x)
+    for layout in ("auto", "none"):
+        fmt, g = tuner.build(asp_ctx, m, desc, layout)
+        assert g.whole_rows() == (layout == "auto")
+        refdump.assert_y(g.spmv_host(x), y_ref, scale, np.float32, f"{template} {layout}")
+        g.close()
+        fmt.close()
+
+
+def strips_of(cm, templates):
+    return [[f"sub {i} {node}" for node in (NODES | NO_LIST)[t]] + [f"sub {i} template {t}"] for i, t in enumerate(templates)]
+
+
+@pytest.mark.parametrize("layout,short,long,templates,listed", [
+    ("none", 20_000, 600, "K2 K6", 0),   # 800,000 stored elements
+    ("none", 1_000, 30, "K2 K6", 0),
+    ("auto", 1_000, 30, "K2 K6", 2),
+    ("auto", 1_000, 30, "K2 K5", 1),     # one of the strips has no list
+    ("auto", 1_000, 30, "K3 K8", 2),
+    ("auto", 1_000, 30, "K9 K6", 2)])
+def test_a_strip_has_the_same_bits_alone_and_in_its_group(asp_ctx, layout, short, long, templates, listed):
+    from alphasparse_b200.graph import Matrix
+
+    rng = np.random.default_rng(short)
+    m, x = M.from_row_lengths(np.concatenate([rng.integers(10, 30, size=short), rng.integers(500, 700, size=long)]), 50_000, seed=short)
+    hm = Matrix.from_csr(m)
+    cm = hm.dense("dense sort 1\ndense rowdiv_exp 128 4096 8\ndense compress")
+    strips = strips_of(cm, [templates.split()[cm.sub_rows(i)[3] > 128] for i in range(cm.n_subs)])
+    assert cm.n_subs > 1 and (m.nnz < 65_536) == (short == 1_000)
+    fmt = cm.execute("\n".join(sum(strips, [])))
+    g = fmt.upload(asp_ctx, layout)
+    assert g.layout_bytes() == 0
+    y_ref, scale = refdump.csr_ref(m, x)
+    y = g.spmv_host(x)
+    refdump.assert_y(y, y_ref, scale, np.float32, "strips")
+    whole = [bool(capi.lib().asp_plan_whole_rows(g._plans[i])) for i in range(g.n)]
+    assert (sum(whole) > 0) == (listed > 0) and (listed == 1) == (0 < sum(whole) < g.n)
+    for i, strip in enumerate(strips):
+        part = cm.execute("\n".join(strip + [f"sub {j} template EMPTY" for j in range(cm.n_subs) if j != i]))
+        gp = part.upload(asp_ctx, layout)
+        assert bool(capi.lib().asp_plan_whole_rows(gp._plans[i])) == whole[i]
+        info = fmt.sub_info(i)
+        rows = fmt.global_perm()[info.min_row : info.max_row + 1].astype(np.int64)
+        assert np.array_equal(gp.spmv_host(x)[rows], y[rows]), i
+        gp.close()
+        part.close()
+    g.close()
+    fmt.close()
+    cm.close()
+    hm.close()
