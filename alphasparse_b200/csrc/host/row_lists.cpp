@@ -43,6 +43,12 @@ uint64_t row_in_y(const asp_plan_desc &d, const HostMeta &perm, int sort_kind, u
     return sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
 }
 const uint64_t kMostRun = 4096; // elements of a row of the CSR5-like templates that is listed
+// Elements of a plan whose rows are listed: as many as both kernels were measured with. By chunks / by rows, us. Chunks of a warp are the slower ones at
+// every size: rows of 81, columns in a window of 3000, fp32 1 M 10.1 / 4.7, 16 M 101 / 48.2, 100 M 607 / 287, fp64 10.3 / 6.4, 107 / 70.2, 650 / 425; rows of
+// 300, 16 M, 69.5 / 24.7, fp64 68.8 / 36.6. So are chunks of a CTA in fp32, for rows of up to 4096 (rows of 2000 1 M 5.8 / 3.1, 100 M 133 / 121; of
+// 600 100 M 239 / 174); for longer ones up to some 16 M (of 8,000 25.3 / 24.9, 32 M 44.7 / 47.1). In fp64 the operations of the sums show: rows of 2000 4 M
+// 12.5 / 11.1, 8 M 20.1 / 20.7, 16 M 33.3 / 38.0; of 8,000 1 M 5.5 / 4.1, 2 M 7.3 / 7.4, 4 M 11.7 / 15.6.
+const uint64_t kMostByRows = 1u << 27, kMost64 = 1u << 22, kMostLong = 1u << 24, kMostLong64 = 1u << 20;
 const uint64_t kSharedRows = 1u << 14; // from so many on, the rows of a list are shared out
 
 // Lists of the rows of a (validated) plan, as the kernels of kernels_rows.cu take them. false: another template, a row in two places, or offsets
@@ -53,8 +59,8 @@ bool list_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const Ho
 {
     const bool cta = d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE, chunks = cta || d.template_type == ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE;
     if ((!chunks && d.template_type != ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE) || d.n_rows > 0xffffffffull) return false;
-    Distinct distinct(d.n_rows, d.sort_kind == ASP_SORT_NONE);
     const HostMeta &offsets = hm[cta ? MS_BLK_NZ : MS_WARP_NZ];
+    Distinct distinct(d.n_rows, d.sort_kind == ASP_SORT_NONE);
     out.make(d.n_rows + 1);
     uint64_t end = 0, n = 0;
     longest = 0;
@@ -283,10 +289,11 @@ bool OwnRows::list(const asp_plan_desc &d, const std::vector<HostMeta> &hm, cons
         return longest <= 8 * args.lanes;
     default: break;
     }
-    if (!list_rows(d, hm, perm, a, rows, longest)) return false;
+    const bool f64 = d.val_dtype == ASP_F64;
+    if (stored > kMostByRows || !list_rows(d, hm, perm, a, rows, longest)) return false;
     listed = rows.n - 1;
-    const uint64_t elements = rows.p[listed].x - rows.p[0].x;
-    if (longest > 512 && (longest > 16384 || elements < 256 * listed)) return false;
+    const uint64_t elements = rows.p[listed].x - rows.p[0].x, most = longest > 4096 ? (f64 ? kMostLong64 : kMostLong) : f64 ? kMost64 : kMostByRows;
+    if (longest > 512 && (longest > 16384 || elements < 256 * listed || (d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE && stored > most))) return false;
     // threads for all of a row in one trip while all rows are on the device at once, else for two
     const uint64_t per = listed <= 2ull * sm_count ? 4 : 8;
     args.cta = longest <= 512 ? 0 : (unsigned)std::min<uint64_t>(1024, std::max<uint64_t>(64, (longest + 32 * per - 1) / (32 * per) * 32));

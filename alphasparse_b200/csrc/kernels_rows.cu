@@ -129,7 +129,7 @@ __device__ __forceinline__ Sum<VT> row_part(const RowArgs &a, u32 begin, u32 end
 template <class VT, class CT>
 __global__ void __launch_bounds__(256) k_row_warp(RowArgs a)
 {
-    const u32 lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const u32 lane = threadIdx.x & 31, w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); // (threads would not fit into 32 bits)
     WaitOnce wait;
     if (w < a.n)
     {
