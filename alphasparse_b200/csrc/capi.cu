@@ -625,7 +625,7 @@ void list_strips(const asp_plan_desc *descs, int n, const std::vector<std::vecto
     uint64_t stored = 0, true_nnz = 0;
     for (int i = 0; i < n; i++) stored += made[i]->stored, true_nnz += descs[i].true_nnz;
     const bool small = true_nnz < asp::kSameBits;
-    if (!small && (!complete || stored > (1u << 20))) return;
+    if ((!small && (!complete || stored > (1u << 20))) || descs[0].n_rows > asp::kMostSeen) return;
     const auto alone = [&](int i) { return small && !made[i]->args.atomic; };
     try
     {
@@ -745,16 +745,25 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
     }
 
     std::shared_ptr<Arena> arena(new (std::nothrow) Arena());
-    size_t list_room = 0, list_at = 0;
+    size_t list_room = 0, list_at = 0; // of the block, for lists of rows
+    // lists and layouts make calls faster, no more: the caller's x and y, and a margin for whatever else the program does, come first
+    const size_t spare = (descs[0].n_rows + descs[0].n_cols) * (descs[0].val_dtype == ASP_F64 ? 8 : 4) + (256u << 20);
     if (!arena) return fail(ASP_ERR_ALLOC, "host allocation failed");
     if (!dry)
     {
-        // with room for a small matrix's list of rows (below): a block of its own costs as much again
-        uint64_t stored = 0;
-        for (int i = 0; i < n; i++) stored += vals[i] ? vals[i]->len : 0;
-        list_room = stored <= (3u << 20) ? align_up(20 * descs[0].n_rows + 4096 * (size_t)n, 256) : 0;
+        // with room for a small matrix's lists of rows (below): a block of its own costs as much again
+        if (layout == ASP_LAYOUT_AUTO)
+            for (int i = 0; i < n; i++)
+                if (vals[i]) list_room += align_up(asp::OwnRows::room(descs[i], metas[i], vals[i]->len), 256);
         total = align_up(total, 256);
-        cudaError_t e = arena->make(ctx->device, std::max<size_t>(total + list_room, 256));
+        cudaError_t e = cudaErrorMemoryAllocation;
+        if (list_room > 0) e = arena->make(ctx->device, total + list_room, spare);
+        if (e != cudaSuccess)
+        {
+            cudaGetLastError();
+            e = arena->make(ctx->device, std::max<size_t>(total, 256));
+        }
+        if (e == cudaSuccess) list_room = arena->got - total;
         if (e != cudaSuccess)
         {
             cudaGetLastError();
@@ -1178,9 +1187,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         for (int k = 0; k < K; k++) off[k + 1] = align_up(off[k] + bytes[k], 256);
         const uint64_t sum_stride = align_up(th.n_parts, 32);
         const size_t sum_bytes = (size_t)th.copies * sum_stride * sizeof(double);
-        // The layout makes calls faster, no more: the caller's x and y, and a margin for whatever else the program does, come first.
-        const size_t vectors = (descs[0].n_rows + descs[0].n_cols) * (descs[0].val_dtype == ASP_F64 ? 8 : 4), margin = 256u << 20;
-        if (tg->arena.make(ctx->device, off[K] + sum_bytes, vectors + margin) != cudaSuccess)
+        if (tg->arena.make(ctx->device, off[K] + sum_bytes, spare) != cudaSuccess)
         {
             cudaGetLastError(); // no room on the device: as above
             tg.reset();
@@ -1241,7 +1248,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
         if (list_at + bytes > list_room)
         {
             list.reset(new (std::nothrow) Arena());
-            if (!list || list->make(ctx->device, bytes) != cudaSuccess)
+            if (!list || list->make(ctx->device, bytes, spare) != cudaSuccess)
             {
                 cudaGetLastError(); // no room: the templates' own kernels
                 for (asp_plan *p : made) p->row_list.reset();

@@ -22,14 +22,14 @@ void with_entries(const HostMeta &h, F &&f)
     else if (h.dtype == ASP_U32) f([p = (const uint32_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
     else f([p = (const uint64_t *)h.p](uint64_t i) { return (uint64_t)p[i]; });
 }
-// Whether rows of y come once each: ascending ones, or a list of what has come
+// Whether rows of y come once each: ascending ones, or a list of what has come (of more than kMostSeen rows: none does)
 struct Distinct
 {
     const uint64_t n;
     const bool ascending;
     uint64_t next = 0;
     std::vector<bool> seen;
-    Distinct(uint64_t rows, bool in_order) : n(rows), ascending(in_order), seen(in_order ? 0 : rows, false) {}
+    Distinct(uint64_t rows, bool in_order) : n(in_order || rows <= kMostSeen ? rows : 0), ascending(in_order), seen(in_order ? 0 : n, false) {}
     bool operator()(uint64_t row)
     {
         if (row >= n || (ascending ? row < next : (bool)seen[row])) return false;
@@ -42,6 +42,7 @@ uint64_t row_in_y(const asp_plan_desc &d, const HostMeta &perm, int sort_kind, u
 {
     return sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
 }
+const uint64_t kMostStrips = 3u << 20, kMostRuns = 1u << 19, kMostTlbs = 2u << 20, kShortTlb = 8; // elements of a plan, of a TLB: row_lists.h
 const uint64_t kMostRun = 4096; // elements of a row of the CSR5-like templates that is listed
 // Elements of a plan whose rows are listed: as many as both kernels were measured with. By chunks / by rows, us. Chunks of a warp are the slower ones at
 // every size: rows of 81, columns in a window of 3000, fp32 1 M 10.1 / 4.7, 16 M 101 / 48.2, 100 M 607 / 287, fp64 10.3 / 6.4, 107 / 70.2, 650 / 425; rows of
@@ -54,18 +55,20 @@ const uint64_t kSharedRows = 1u << 14; // from so many on, the rows of a list ar
 // Lists of the rows of a (validated) plan, as the kernels of kernels_rows.cu take them. false: another template, a row in two places, or offsets
 // beyond 32 bits.
 //
-// Chunks of a row one after the other, `longest` row
-bool list_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const KArgs &a, HostBuf<uint2> &out, uint64_t &longest)
+// Chunks of a row one after the other, `longest` row; no more rows than elements (`stored`)
+bool list_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const KArgs &a, uint64_t stored, HostBuf<uint2> &out, uint64_t &longest)
 {
     const bool cta = d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE, chunks = cta || d.template_type == ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE;
     if ((!chunks && d.template_type != ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE) || d.n_rows > 0xffffffffull) return false;
     const HostMeta &offsets = hm[cta ? MS_BLK_NZ : MS_WARP_NZ];
+    const uint64_t most = std::min<uint64_t>(d.n_rows, cta ? a.n_units : chunks ? a.effective : std::min<uint64_t>(hm[MS_BLK_ROW].get(a.n_units), a.effective));
+    if (most > stored) return false;
     Distinct distinct(d.n_rows, d.sort_kind == ASP_SORT_NONE);
-    out.make(d.n_rows + 1);
+    out.make(most + 1);
     uint64_t end = 0, n = 0;
     longest = 0;
     auto put = [&](uint64_t row, uint64_t from, uint64_t to) {
-        if (to < from || to > 0xffffffffull || (n > 0 && from != end) || !distinct(row)) return false;
+        if (to < from || to > 0xffffffffull || (n > 0 && from != end) || n == most || !distinct(row)) return false;
         end = to;
         longest = std::max(longest, to - from);
         out.p[n++] = make_uint2((unsigned)from, (unsigned)row);
@@ -112,12 +115,12 @@ bool list_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const Ho
 }
 
 // Row-grouped; `tlbs` of all rows, `most` of one
-bool list_tlb_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const KArgs &a, HostBuf<uint4> &out, uint64_t &tlbs, uint64_t &most)
+bool list_tlb_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const KArgs &a, uint64_t stored, HostBuf<uint4> &out, uint64_t &tlbs, uint64_t &most)
 {
     if (d.template_type != ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS || d.n_rows > 0xffffffffull) return false;
     const HostMeta &row = hm[MS_BLK_ROW];
     const uint64_t B = a.n_units, rows = std::min<uint64_t>(row.get(B), a.effective);
-    if (row.get(0) != 0 || rows == 0 || rows > d.n_rows || !has_entries(hm[MS_ROW_OFF], row.get(B) + 1)) return false;
+    if (row.get(0) != 0 || rows == 0 || rows > d.n_rows || rows > stored || !has_entries(hm[MS_ROW_OFF], row.get(B) + 1)) return false;
     Distinct distinct(d.n_rows, a.sort_kind == ASP_SORT_NONE);
     out.make(rows);
     std::atomic<uint64_t> all(0), top(0);
@@ -206,7 +209,7 @@ bool list_runs(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const Ho
     for (uint64_t w = 0; w + within < a.n_units; w++)
         if (hm[MS_ROW_OF_UNIT].get(w) == hm[MS_ROW_OF_UNIT].get(w + within)) return false;
     Distinct distinct(d.n_rows, a.sort_kind == ASP_SORT_NONE);
-    out.make(d.n_rows);
+    out.make(std::min<uint64_t>(d.n_rows, a.n_units * 32 * S));
     uint64_t r = ~0ull, n = 0; // of the matrix's rows in order
     bool good = true;
     with_entries(hm[MS_COMBINE], [&](auto words) {
@@ -251,6 +254,30 @@ void OwnRows::make(const asp_plan_desc &d, const std::vector<HostMeta> &hm, cons
     }
 }
 
+size_t OwnRows::room(const asp_plan_desc &d, const std::vector<HostMeta> &hm, uint64_t stored)
+{
+    const uint64_t rows = std::min<uint64_t>(d.n_rows, stored);
+    switch (d.template_type)
+    {
+    case ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS:
+    case ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS:
+    {
+        // a group of up to 32 rows an entry, BLBs of 128 rows
+        const HostMeta &of = hm[MS_ROW_OF_TLB];
+        const bool one = d.template_type == ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS;
+        if (stored > kMostStrips || (one && d.tlb_size <= kShortTlb)) return 0;
+        return rows / 2 + (one ? 0 : rows / 8) + (of.kind == ASP_COMPRESS_LINEAR && of.coef == 1 ? 0 : 4 * rows) + 512;
+    }
+    case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE:
+    case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE: return stored > kMostRuns ? 0 : 16 * rows + 256;
+    case ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS: return stored > kMostTlbs ? 0 : 16 * rows + 256;
+    case ASP_DIRECT_ATOM_TOTAL_WARP_REDUCE_TEMPLATE:
+    case ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE:
+    case ASP_SHARED_MEMORY_TOTAL_WARP_REDUCE_TEMPLATE: return stored > kMostStrips ? 0 : 8 * rows + 264; // (a block of its own is little beside a larger plan)
+    default: return 0;
+    }
+}
+
 bool OwnRows::list(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const KArgs &a, uint64_t stored, int sm_count, bool few)
 {
     uint64_t longest = 0, all = 0;
@@ -259,16 +286,16 @@ bool OwnRows::list(const asp_plan_desc &d, const std::vector<HostMeta> &hm, cons
     case ASP_DIRECT_ATOM_TEMPLATE_WARP_BLOCK_COMPRESS:
     case ASP_DIRECT_ATOM_TEMPLATE_WARP_COMPRESS:
         strips = true;
-        if (stored > (3u << 20) || !list_strips(d, hm, a, tlbs, place, all, longest, listed)) return false;
+        if (stored > kMostStrips || !list_strips(d, hm, a, tlbs, place, all, longest, listed)) return false;
         args.first_row = (unsigned)all;
         args.lanes = longest <= 16 ? 4 : longest <= 32 ? 8 : 16;
         args.n = (unsigned)tlbs.n;
-        return longest > 8 || few;
+        return longest > kShortTlb || few;
     case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE:
     case ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE:
     {
         runs = true;
-        if (stored > (1u << 19) || !list_runs(d, hm, perm, a, tlbs)) return false;
+        if (stored > kMostRuns || !list_runs(d, hm, perm, a, tlbs)) return false;
         listed = tlbs.n;
         args.size = a.tlb_size;
         args.n = (unsigned)listed;
@@ -281,7 +308,7 @@ bool OwnRows::list(const asp_plan_desc &d, const std::vector<HostMeta> &hm, cons
         return true;
     }
     case ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS:
-        if (stored > (2u << 20) || !list_tlb_rows(d, hm, perm, a, tlbs, all, longest)) return false;
+        if (stored > kMostTlbs || !list_tlb_rows(d, hm, perm, a, stored, tlbs, all, longest)) return false;
         listed = tlbs.n;
         args.n = (unsigned)listed;
         args.lanes = 2;
@@ -290,7 +317,7 @@ bool OwnRows::list(const asp_plan_desc &d, const std::vector<HostMeta> &hm, cons
     default: break;
     }
     const bool f64 = d.val_dtype == ASP_F64;
-    if (stored > kMostByRows || !list_rows(d, hm, perm, a, rows, longest)) return false;
+    if (stored > kMostByRows || !list_rows(d, hm, perm, a, stored, rows, longest)) return false;
     listed = rows.n - 1;
     const uint64_t elements = rows.p[listed].x - rows.p[0].x, most = longest > 4096 ? (f64 ? kMostLong64 : kMostLong) : f64 ? kMost64 : kMostByRows;
     if (longest > 512 && (longest > 16384 || elements < 256 * listed || (d.template_type == ASP_SHARED_MEMORY_LONG_ROW_TEMPLATE && stored > most))) return false;

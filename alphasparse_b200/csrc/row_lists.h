@@ -10,6 +10,8 @@
 
 namespace asp
 {
+const uint64_t kMostSeen = 1u << 26; // rows of a matrix, where which of them have come is kept (8 MB)
+
 // Whole rows for a few lanes, a warp or a CTA, where that is the faster way (kernels_rows.cu). A warp takes up to 512 elements (four trips
 // of 1.2 us; chunks in parallel are faster beyond that), a CTA rows of 256 and more on average, up to 16384 (four trips of 1024 threads).
 // Rows that are TLBs of more than 8 elements: up to 3 M elements (what L2 holds). CSR5-like: up to 512 K elements (FEM, fp32: 445 K 6 -> 3.1 us, 730 K
@@ -43,6 +45,9 @@ struct OwnRows
                 for (unsigned k = 0; k < tlbs.p[i].z >> 16; k++) f(args.first_row + tlbs.p[i].y + k);
         for (uint64_t i = 0; i < place.n; i++) f(place.p[i]);
     }
+    // Device memory that the list of a small plan may take, about: 0 where it can have none. (What does not fit gets a block of its own.) Before anything is known of
+    // its arrays' contents: no more rows than elements are listed.
+    static size_t room(const asp_plan_desc &d, const std::vector<HostMeta> &hm, uint64_t stored);
     // of a (validated) plan whose values are `stored` ones. few: one of several sub-matrices, which a kernel each takes one after the other
     void make(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const HostMeta &perm, const KArgs &a, uint64_t stored, int sm_count, bool few = false);
 

@@ -189,3 +189,41 @@ def test_a_strip_has_the_same_bits_alone_and_in_its_group(asp_ctx, layout, short
     fmt.close()
     cm.close()
     hm.close()
+
+
+def free_memory():
+    import torch
+
+    capi.check(capi.lib().asp_device_trim(0))
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("template", ["D1", "K3"])
+def test_room_for_lists_goes_with_what_they_take(asp_ctx, template):
+    """Plans that have none."""
+    import torch
+
+    m, x = M.laplacian_2d(600, seed=1, dtype=np.float64)
+    desc = {"dense": "dense compress", "subs": [{"graph": template, "nodes": (NODES | {"D1": ["diag_value 64"]})[template], "template": template, "threads": 128, "row_reduce": 1}]}
+    dx, dy = torch.from_numpy(x).cuda(), torch.full((m.n_rows,), 7.0, dtype=torch.from_numpy(x).dtype, device="cuda")
+    before = free_memory()
+    fmt, g = tuner.build(asp_ctx, m, desc)
+    assert g.layout_bytes() == 0 and not g.whole_rows()
+    assert before - free_memory() <= g.format_bytes() + (5 << 20)  # (allocations are in pieces of 2 MB)
+    fmt_bytes = g.format_bytes()
+    g.close()
+    # room for the format and little more: the plan is made
+    hold = torch.empty(free_memory() - fmt_bytes - (60 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        g = fmt.upload(asp_ctx)
+        g.spmv(dx.data_ptr(), dy.data_ptr(), True)
+        asp_ctx.synchronize()
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    y_ref, scale = refdump.csr_ref(m, x)
+    refdump.assert_y(dy.cpu().numpy(), y_ref, np.maximum(scale, 1e-30), x.dtype, template)
+    g.close()
+    fmt.close()

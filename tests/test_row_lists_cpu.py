@@ -16,7 +16,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("part", ["limits"])
+@pytest.mark.parametrize("part", ["limits", "empty"])
 def test_lists(program, part):
     r = subprocess.run([program, part], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, (r.returncode, r.stdout, r.stderr[-500:])
