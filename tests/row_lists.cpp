@@ -1,7 +1,6 @@
 // Lists of rows as the host makes them, without a GPU. Argument: the part to check. Ends with status 0 where it holds.
 #include <stdio.h>
 #include <string.h>
-#include <sys/resource.h>
 
 #include <string>
 #include <vector>
@@ -51,13 +50,21 @@ static int limits()
 }
 
 // What a list takes on the host goes with the rows that are in it, not with those of the matrix.
+static long peak() // KB of address space
+{
+    long kb = -1;
+    char line[256];
+    FILE *f = fopen("/proc/self/status", "r");
+    while (f && fgets(line, sizeof line, f)) sscanf(line, "VmPeak: %ld", &kb);
+    if (f) fclose(f);
+    return kb;
+}
 static int empty()
 {
+    const long before = peak();
     if (!listed(chunks(4000000000ull, 5, 3), 5)) return 1;
     if (chunks(100, 50, 0).bytes() != 0) return 2; // more rows than elements
-    rusage u;
-    getrusage(RUSAGE_SELF, &u);
-    return u.ru_maxrss > 300000 ? 3 : 0; // KB
+    return peak() - before > 200000 ? 3 : 0;
 }
 
 int main(int, char **argv)
