@@ -188,6 +188,25 @@ double lines_per_gather(const TiledSource &s, bool f64)
     return (double)lines / (double)(samples * 128);
 }
 
+// How close the elements of a row lie, 1: in adjacent columns. Sampled over some 20,000 of them.
+template <class VT>
+double closeness(const TiledSource &s)
+{
+    const u64 units = unit_count(s), samples = std::min<u64>({units, 64, std::max<u64>(1, 20000 * units / std::max<u64>(1, s.stored))});
+    u64 pairs = 0, columns = 0, last_row = ~0ull, last = 0;
+    for (u64 q = 0; q < samples; q++)
+    {
+        const u64 u = units * q / samples;
+        walk_any<VT>(s, u, u + 1, [&](u64 row, u64 c, VT) ASP_INLINE {
+            if (row == last_row) pairs++, columns += c > last ? c - last : last - c;
+            last_row = row;
+            last = c;
+        });
+        last_row = ~0ull;
+    }
+    return pairs == 0 ? 0.0 : std::min(1.0, (double)pairs / (double)std::max<u64>(1, columns));
+}
+
 bool is_csr5(const TiledSource &s)
 {
     return s.templ == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE || s.templ == ASP_UNALIGNED_WARP_REDUCE_SAME_TLB_SIZE_TEMPLATE_WITH_WARP_REDUCE;
@@ -832,8 +851,12 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     };
     // (what tiled_us says is 1 to 3 us too long for a few million non-zeros, as the time of the other kernels is; that of whole rows is not)
     auto slower = [&](double us) { return whole ? 0.92 * (us - 1.6) > own_us : us > 0.85 * own_us; };
+    // Pieces of a long dense row are 32 columns apart: the lanes that take them meet in one bank of shared memory. Rows of 81 / 500 / 2000 adjacent
+    // columns, fp32, 4 M 10.1 / 13.9 / 18.0 us, 8 M 13.9 / 21.4 / 31.7 (by whole rows 19.3 / - / 12.0), fp64 8 M 17.8 / 29.6 / 35.0.
+    const double close = whole && !is_csr5(src[0]) ? closeness<VT>(src[0]) : 0.0;
+    auto banks_us = [&](u64 n, double run) { return (double)n * 1.95e-6 * close * std::min(1.0, std::max(0.0, run - 96.0) / 1024.0); };
     auto units_us = [](u64 n) { return 4.4 + 1.45e-6 * (double)n; };
-    if (slower(tiled_us(true_nnz, 0, 0)) && !(sizeof(VT) == 4 && whole && units_us(true_nnz) <= own_us)) return false;
+    if (slower(tiled_us(true_nnz, 0, 0) + banks_us(true_nnz, (double)true_nnz / (double)n_rows)) && !(sizeof(VT) == 4 && whole && units_us(true_nnz) <= own_us)) return false;
     if (n_rows >= kTiledInParts || requests >= 1e11) return false;
     Builder<VT> b(src, n_rows, n_cols, true_nnz, n_sm);
     if (b.C + (u64)n_sm >= 65536) return false;
@@ -849,7 +872,7 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
         if (p > 0) red += p * std::min(1.0, std::max(0.25, 4.0 * (double)n_rows / p / 32.0));
     }
     const bool units = sizeof(VT) == 4 && b.N <= kRunForUnits * b.runs && 4 * b.near_runs >= 3 * b.runs && tiled_units_fit(b.runs, b.N, b.C);
-    if (whole && units ? units_us(b.N) > own_us : slower(tiled_us(b.N, pieces, red))) return false;
+    if (whole && units ? units_us(b.N) > own_us : slower(tiled_us(b.N, pieces, red) + banks_us(b.N, (double)b.N / (double)std::max<u64>(1, b.runs)))) return false;
     b.number_rows(out);
     if constexpr (sizeof(VT) == 4)
     {

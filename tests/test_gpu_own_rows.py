@@ -227,3 +227,19 @@ def test_room_for_lists_goes_with_what_they_take(asp_ctx, template):
     refdump.assert_y(dy.cpu().numpy(), y_ref, np.maximum(scale, 1e-30), x.dtype, template)
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("template,rows,length", [("K7", 1_500, 2_000), ("K7", 3_000, 1_000), ("K4", 4_000, 500)])
+def test_long_dense_rows_are_not_laid_out(asp_ctx, template, rows, length, dtype):
+    """Rows of adjacent columns: the lanes of the column-tiled kernel would meet in one bank of shared memory."""
+    rng = np.random.default_rng(rows)
+    indices = (np.arange(rows, dtype=np.int64)[:, None] + np.arange(length)).reshape(-1).astype(np.uint32)
+    m = M.CsrMatrix(rows, rows + length, np.arange(rows + 1, dtype=np.int64) * length, indices, rng.uniform(-1, 1, size=indices.size).astype(dtype))
+    x = rng.uniform(-1, 1, size=m.n_cols).astype(dtype)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template, "threads": 128, "row_reduce": 1}]})
+    assert g.whole_rows() and g.layout_bytes() == 0
+    y_ref, scale = refdump.csr_ref(m, x)
+    refdump.assert_y(g.spmv_host(x), y_ref, scale, dtype, template)
+    g.close()
+    fmt.close()
