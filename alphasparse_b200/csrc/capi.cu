@@ -1646,7 +1646,7 @@ struct InOrder
         return e;
     }
 };
-const uint64_t kShortX = 384u << 10; // bytes
+const uint64_t kShortX = 384u << 10, kLongY = 4u << 20; // bytes
 // streams and events of host calls
 asp_status pipe_ready(asp_ctx *ctx, size_t events)
 {
@@ -1739,18 +1739,18 @@ asp_status asp_spmv_host_pipelined(asp_ctx *ctx, const asp_host_chunk *chunks, i
     asp_status st = ensure_xy(ctx, n_cols * es, n_rows * es);
     if (st != ASP_OK) return st;
     unsigned char *const y_seen = (unsigned char *)asp::device_view(h_y, n_rows * es);
-    // A short x is there sooner than the calls that would send it in pieces: all of it, the chunks' kernels, and y (which the kernels store to the
-    // host themselves where they can). (Four chunks, 48 KB of x: 52 -> 35.6 us, 167 KB 53 -> 47.5; 0.7 MB 68,
-    // 70 so.)
-    if (n_cols * es <= kShortX)
+    // A short x is there sooner than the calls that would send it in pieces: all of it, the chunks' kernels, and y, which the kernels store to the
+    // host themselves where they can. (Four chunks, 48 KB of x: 52 -> 35.6 us, 167 KB 53 -> 47.5; 0.7 MB 68, 70 so.) Copies of a
+    // long y had better run beside the chunks that follow: 16 KB of x, 0.8 MB of y 61-65 us, 46-52 so, 3.2 MB 94, 90 so, 8 MB 179, 183 so, 32 MB 622, 639 so.
+    uint64_t cols = 0;
+    bool seen = y_seen != nullptr;
+    for (int c = 0; c < n_chunks; c++)
     {
-        uint64_t cols = 0;
-        bool seen = y_seen != nullptr;
-        for (int c = 0; c < n_chunks; c++)
-        {
-            cols = std::max<uint64_t>(cols, chunks[c].col_hi);
-            seen = seen && rows_in_order(chunks[c].plans, chunks[c].n_plans);
-        }
+        cols = std::max<uint64_t>(cols, chunks[c].col_hi);
+        seen = seen && rows_in_order(chunks[c].plans, chunks[c].n_plans);
+    }
+    if (n_cols * es <= kShortX && (seen || n_rows * es <= kLongY))
+    {
         cudaError_t e = cudaMemcpyAsync(ctx->x, h_x, cols * es, cudaMemcpyHostToDevice, ctx->stream);
         for (int c = 0; c < n_chunks && e == cudaSuccess && st == ASP_OK; c++)
         {

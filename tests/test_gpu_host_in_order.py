@@ -24,6 +24,13 @@ def banded(n_rows, n_cols, offsets, seed, dtype):
     return M.CsrMatrix(n_rows, n_cols, indptr, c[keep].astype(np.uint32), values), rng.uniform(-1, 1, size=n_cols).astype(dtype)
 
 
+def tall(n_rows, n_cols, seed, dtype):
+    """Rows of two elements all over x: few diagonals would not hold them."""
+    rng = np.random.default_rng(seed)
+    c = np.stack([np.arange(n_rows) % (n_cols - 1), np.arange(n_rows) % (n_cols - 1) + 1], 1)
+    return M.CsrMatrix(n_rows, n_cols, np.arange(n_rows + 1, dtype=np.int64) * 2, c.reshape(-1).astype(np.uint32), rng.uniform(-1, 1, size=2 * n_rows).astype(dtype)), rng.uniform(-1, 1, size=n_cols).astype(dtype)
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("rows,cols,offsets", [
     (1, 1, [0]), (7, 7, [-1, 0, 1]), (1000, 1003, [-1, 0, 3]),
@@ -57,13 +64,15 @@ def test_host_call_matches_the_oracle(asp_ctx, rows, cols, offsets, dtype):
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("spec,threads", [("diag_value 64", "D1"), ("row_padding 32 1|tlb_row", "K3"), ("tlb_nnz 8", "K9")])
-@pytest.mark.parametrize("rows", [5, 96, 1001, 40_000, 60_001, 250_000])
-def test_pipelined_calls_around_a_short_x(asp_ctx, rows, spec, threads, dtype):
+@pytest.mark.parametrize("rows,cols", [(5, 8), (96, 99), (1001, 1004), (40_000, 40_003), (60_001, 60_004), (250_000, 250_003), (60_000, 900), (530_000, 900), (1_060_000, 900)])
+def test_pipelined_calls_around_a_short_x(asp_ctx, rows, cols, spec, threads, dtype):
     """x in one piece or in several, y from the kernels or by copies, page-locked or not, with chunks that read to the end of x or not."""
     import torch
     from alphasparse_b200 import tuner
 
-    m, x = banded(rows, rows + 3, [-2, 0, 3], 5, dtype)
+    m, x = banded(rows, cols, [-2, 0, 3], 5, dtype) if cols > rows else tall(rows, cols, 5, dtype)
+    if cols < rows and threads == "D1":
+        pytest.skip("no diagonals")
     desc = {"dense": "dense compress", "subs": [{"graph": threads, "nodes": spec.split("|"), "template": threads, "threads": 128, "row_reduce": 1}]}
     chunks = tuner.build_row_chunks(asp_ctx, m, desc, 3, align=32)
     y_ref, scale = refdump.csr_ref(m, x)
