@@ -108,3 +108,34 @@ def test_x_and_y_in_one_buffer(asp_ctx, shift, dtype):
         refdump.assert_y(hy.numpy(), y_ref, scale, dtype, f"y {shift} behind x")
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("bytes_of_chunks", [[(3 << 19) - 128, 3 << 19, (3 << 19) + 128], [3 << 20, 640, 2 << 20], [64 << 10, 5 << 20, 1 << 20]])
+def test_pipelined_calls_with_long_chunks(asp_ctx, bytes_of_chunks, dtype):
+    """Chunks of diagonal values of 1.5 MB and more go to page-locked y from the kernel, shorter ones by copies, in one call."""
+    import torch
+
+    es = np.dtype(dtype).itemsize
+    rows = sum(bytes_of_chunks) // es
+    m, x = banded(rows, rows, [-300, 0, 1, 2000], 5, dtype)
+    y_ref, scale = refdump.csr_ref(m, x)
+    made, chunks, lo = [], [], 0
+    for n in bytes_of_chunks:
+        hi = lo + n // es
+        sub = m.row_slice(lo, hi)
+        fmt = Matrix.from_csr(sub).execute("dense compress\nsub all diag_value 64\nsub all template D1")
+        made.append((fmt, fmt.upload(asp_ctx)))
+        chunks.append((made[-1][1], lo, hi, int(sub.indices.max()) + 1))
+        lo = hi
+    xp = torch.from_numpy(x).pin_memory()
+    for pinned, shift in ((True, 0), (True, 1), (False, 0)):
+        y = torch.full((rows + 4,), 7.0, dtype=xp.dtype)
+        y = y.pin_memory() if pinned else y
+        for _ in range(2):
+            capi.spmv_host_pipelined(asp_ctx, chunks, xp.data_ptr(), y[shift:].data_ptr())
+        refdump.assert_y(y.numpy()[shift : shift + rows], y_ref, scale, dtype, f"pinned={pinned} shift={shift}")
+        assert (y[:shift] == 7).all() and (y[shift + rows :] == 7).all()
+    for fmt, g in made:
+        g.close()
+        fmt.close()

@@ -13,12 +13,14 @@ pytestmark = pytest.mark.gpu
 
 
 def run(ctx, m, x, spec, what):
+    """The templates' kernels, and whatever a plan runs by itself."""
     fmt = Matrix.from_csr(m).execute(spec)
-    g = fmt.upload(ctx)
-    y = g.spmv_host(x)
     y_ref, scale = refdump.csr_ref(m, x)
-    refdump.assert_y(y, y_ref, scale, m.values.dtype, what)
-    g.close()
+    for layout in ("none", "auto"):
+        g = fmt.upload(ctx, layout)
+        y = g.spmv_host(x)
+        refdump.assert_y(y, y_ref, scale, m.values.dtype, f"{what} ({layout})")
+        g.close()
     fmt.close()
 
 
@@ -132,14 +134,15 @@ def test_format_loaded_from_its_file_runs_like_the_original(asp_ctx, mats, tmp_p
 @pytest.mark.parametrize("templ", ["K9", "K10"])
 @pytest.mark.parametrize("s", [4, 8, 16, 32, 5])
 @pytest.mark.parametrize("mat", ["rmat_f32", "mixed_f32", "laplace_f64", "fem_f64"])
-def test_csr5_like_kernels_for_every_tlb_size_direct_and_staged(asp_ctx, mats, mat, s, templ):
+@pytest.mark.parametrize("layout", ["none", "auto"])
+def test_csr5_like_kernels_for_every_tlb_size_direct_and_staged(asp_ctx, mats, mat, s, templ, layout):
     """The CSR5-like family is specialised on the TLB size (4, 8, 16, 32; any other size takes the generic
     kernel). Both write-out forms -- one store per row, and the warp's rows through shared memory as one
     contiguous run -- must give the oracle's y; rows spanning many warps (mixed_f32 has rows of up to
     5000 non-zeros) and rows without non-zeros (rmat_f32) included."""
     m, x = mats[mat]
     fmt = Matrix.from_csr(m).execute(f"dense compress\nsub all tlb_nnz {s}\nsub all template {templ}")
-    g = fmt.upload(asp_ctx)
+    g = fmt.upload(asp_ctx, layout)
     y_ref, scale = refdump.csr_ref(m, x)
     for path in (0, 1):
         for threads in (64, 256):

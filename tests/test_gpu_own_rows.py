@@ -1,6 +1,8 @@
 """GPU: the kernels that take whole rows of the templates whose chunks of a row lie one after the other (csrc/kernels_rows.cu), against
 the CPU oracle: rows that end on, before and behind a trip of a warp, a CTA or a row's lanes, the longest rows that they take and one element
 more, empty rows, one row, sorted rows, every column width, x and y off 16-byte alignment, every clearing mode."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -89,7 +91,7 @@ def test_whole_rows_match_the_oracle(asp_ctx, template, lengths, cols, dense, wh
 @pytest.mark.parametrize("empty", [0, 20])
 @pytest.mark.parametrize("zero_y", [True, "auto"])
 def test_strips_by_whole_rows(asp_ctx, zero_y, empty, dtype):
-    """Several sub-matrices with a kernel for whole rows each: all of them, one alone, and none of the rows twice."""
+    """Several sub-matrices with a kernel for whole rows each: all of them, some of them, one twice, one with its template's kernel."""
     import torch
     from alphasparse_b200.graph import Matrix
 
@@ -116,6 +118,34 @@ def test_strips_by_whole_rows(asp_ctx, zero_y, empty, dtype):
     asp_ctx.synchronize()
     refdump.assert_y(dy.cpu().numpy()[: m.n_rows], y_ref, scale, dtype, "all strips")
     assert (dy[m.n_rows :] == 7).all()
+    perm = fmt.global_perm()
+    rows = [perm[fmt.sub_info(i).min_row : fmt.sub_info(i).max_row + 1].astype(np.int64) for i in range(g.n)]
+
+    def call(which, mode):
+        """y after a call of some plans of the group over a y of sevens"""
+        dy[:] = 7
+        torch.cuda.synchronize()
+        plans = (C.c_void_p * len(which))(*[g._plans[i] for i in which])
+        capi.check(capi.lib().asp_spmv(asp_ctx.handle, plans, len(which), C.c_void_p(dx.data_ptr()), C.c_void_p(dy.data_ptr()), mode))
+        asp_ctx.synchronize()
+        assert (dy[m.n_rows :] == 7).all()
+        return dy.cpu().numpy()[: m.n_rows]
+
+    for which in ([0], [g.n - 1], [g.n - 1, 0]):
+        mine = np.concatenate([rows[i] for i in which])
+        for mode in (1, 2):
+            y = call(which, mode)
+            refdump.assert_y(y[mine], y_ref[mine], scale[mine], dtype, f"plans {which}")
+            others = np.setdiff1d(np.arange(m.n_rows), mine)
+            assert (y[others] == 0).all() or (mode == 2 and (y[others] == 7).all())
+    # a plan twice adds twice what it adds: the templates' kernels (the last strip's rows are added up or stored, as its template does)
+    y = call([0, 0], 1)
+    twice = 2 if fmt.plan_descs()[0].is_atom_add else 1
+    refdump.assert_y(y[rows[0]], twice * y_ref[rows[0]], scale[rows[0]], dtype, "a plan twice")
+    # one of them with its template's kernel
+    capi.check(capi.lib().asp_plan_set_tuning(g._plans[g.n - 1], 0, 0))
+    assert not capi.lib().asp_plan_whole_rows(g._plans[g.n - 1])
+    refdump.assert_y(call(range(g.n), 1), y_ref, scale, dtype, "a tuned plan among others")
     g.close()
     fmt.close()
     cm.close()
@@ -241,5 +271,67 @@ def test_long_dense_rows_are_not_laid_out(asp_ctx, template, rows, length, dtype
     assert g.whole_rows() and g.layout_bytes() == 0
     y_ref, scale = refdump.csr_ref(m, x)
     refdump.assert_y(g.spmv_host(x), y_ref, scale, dtype, template)
+    g.close()
+    fmt.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("template", sorted(NODES))
+def test_numbers_that_are_none(asp_ctx, template, dtype):
+    """What is infinite or no number stays with the rows that have it, and a sum that passes the type's range is infinite."""
+    m, x = matrix([30, 12, 1, 40, 33] * 40 + [300] * (template == "K7"), 3_000, dtype)
+    if template == "K7":
+        m, x = matrix([300, 700, 1000] * 20, 3_000, dtype)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template.split("/")[0], "threads": 128, "row_reduce": 1}]})
+    assert g.whole_rows()
+    y_ref, scale = refdump.csr_ref(m, x)
+    hit = np.bincount(np.repeat(np.arange(m.n_rows), m.row_lengths())[m.indices == 17], minlength=m.n_rows) > 0
+    assert 0 < hit.sum() < m.n_rows
+    for what in (np.inf, -np.inf, np.nan):
+        bad = x.copy()
+        bad[17] = what
+        y = g.spmv_host(bad)
+        assert not np.isfinite(y[hit]).any() and (np.isnan(y[hit]).all() or not np.isnan(what))
+        refdump.assert_y(y[~hit], y_ref[~hit], scale[~hit], dtype, f"beside {what}")
+    # (the products stay in range, their sum does not)
+    most = np.finfo(dtype).max
+    big = M.CsrMatrix(m.n_rows, m.n_cols, m.indptr, m.indices, np.full(m.nnz, most / 4, dtype=dtype))
+    f2, g2 = tuner.build(asp_ctx, big, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template.split("/")[0], "threads": 128, "row_reduce": 1}]})
+    for sign in (1, -1):
+        y = g2.spmv_host(np.full(m.n_cols, sign, dtype=dtype))
+        assert (y[m.row_lengths() >= 5] == sign * np.inf).all() and np.isfinite(y[m.row_lengths() < 4]).all()
+    for o in (g, fmt, g2, f2):
+        o.close()
+
+
+@pytest.mark.parametrize("template", sorted(NODES))
+def test_whole_rows_in_a_graph_and_on_other_contexts(asp_ctx, template):
+    """Lists hold no state."""
+    import torch
+
+    m, x = matrix([30, 40] * 100, 3_000, np.float64)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template.split("/")[0], "threads": 128, "row_reduce": 1}]})
+    assert g.whole_rows()
+    y_ref, scale = refdump.csr_ref(m, x)
+    dx, dys = torch.from_numpy(x).cuda(), [torch.full((m.n_rows,), 7.0, dtype=torch.float64, device="cuda") for _ in range(3)]
+    torch.cuda.synchronize()
+    other = capi.Context(0)
+    for _ in range(20):
+        g.spmv(dx.data_ptr(), dys[0].data_ptr(), True)
+        capi.check(capi.lib().asp_spmv(other.handle, g._plans, g.n, dx.data_ptr(), dys[1].data_ptr(), 1))
+    other.synchronize()
+    asp_ctx.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(asp_ctx.stream)):
+        g.spmv(dx.data_ptr(), dys[2].data_ptr(), True)
+    for _ in range(5):
+        graph.replay()
+        g.spmv(dx.data_ptr(), dys[0].data_ptr(), True)
+    torch.cuda.synchronize()
+    asp_ctx.synchronize()
+    for y, what in zip(dys, ("own context", "another context", "graph")):
+        refdump.assert_y(y.cpu().numpy(), y_ref, scale, np.float64, what)
+    del graph
+    other.close()
     g.close()
     fmt.close()

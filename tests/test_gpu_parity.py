@@ -14,10 +14,11 @@ pytestmark = pytest.mark.gpu
 NAMES = golden_names()
 
 
-def run_golden(ctx, name, launch=None):
+def run_golden(ctx, name, launch=None, layout="auto"):
     m, x, _, man = load_golden(name)
     descs, keep = refdump.plan_descs(man, launch)
-    g = capi.PlanGroup(ctx, descs, keep)
+    g = capi.PlanGroup(ctx, descs, keep, layout)
+    assert layout == "auto" or not any(capi.lib().asp_plan_whole_rows(p) for p in g._plans)
     y = g.spmv_host(x)
     g.close()
     y_ref, scale = refdump.csr_ref(m, x)
@@ -25,8 +26,9 @@ def run_golden(ctx, name, launch=None):
 
 
 @pytest.mark.parametrize("name", NAMES)
-def test_template_matches_oracle(asp_ctx, name):
-    y, y_ref, scale, m = run_golden(asp_ctx, name)
+@pytest.mark.parametrize("layout", ["none", "auto"])
+def test_template_matches_oracle(asp_ctx, name, layout):
+    y, y_ref, scale, m = run_golden(asp_ctx, name, layout=layout)
     refdump.assert_y(y, y_ref, scale, m.values.dtype, name)
 
 
@@ -45,13 +47,14 @@ LAUNCHES = {
 
 
 @pytest.mark.parametrize("name", [n for n in NAMES if n.startswith("uniform1024")])
-def test_launch_parameters_do_not_change_y(asp_ctx, name):
+@pytest.mark.parametrize("layout", ["none", "auto"])
+def test_launch_parameters_do_not_change_y(asp_ctx, name, layout):
     """Any tblock_num / thread_num_in_block / thread_num_of_row_reduce the tuner may try gives
     the same y (grid-stride loops cover what the grid does not)."""
     m, x, _, man = load_golden(name)
     y_ref, scale = refdump.csr_ref(m, x)
     descs, keep = refdump.plan_descs(man)
-    g = capi.PlanGroup(asp_ctx, descs, keep)
+    g = capi.PlanGroup(asp_ctx, descs, keep, layout)
     t = man.subs[0]["template"]
     for lp in LAUNCHES[t]:
         tb, th = lp[0], lp[1]

@@ -35,3 +35,8 @@ def test_the_choice_of_units_does_not_depend_on_the_threads(program, threads):
 @pytest.mark.parametrize("mode", ["y", "sums", "both"])
 def test_units_hold_the_matrix(program, mode):
     run(program, "units", mode)
+
+
+@pytest.mark.parametrize("threads", [1, 4])
+def test_warps_of_a_cta_in_fp64(program, threads):
+    run(program, "warps", threads=threads)

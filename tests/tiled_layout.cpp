@@ -29,8 +29,9 @@ struct Rows
     std::vector<uint64_t> begin{0};
     uint64_t cols = 0;
     void add(uint32_t row) { order.push_back(row), begin.push_back(col.size()); }
-    bool build(asp::TiledHost &out) const
+    bool build(asp::TiledHost &out, bool f64 = false) const
     {
+        const std::vector<double> val64(val.begin(), f64 ? val.end() : val.begin());
         asp::KArgs a;
         memset(&a, 0, sizeof a);
         a.n_units = a.effective = order.size();
@@ -50,11 +51,11 @@ struct Rows
         t.m = m.data();
         t.perm = &perm;
         t.a = &a;
-        t.val = val.data();
+        t.val = f64 ? (const void *)val64.data() : val.data();
         t.col = col.data();
         t.stored = t.true_nnz = col.size();
         t.threads = 128;
-        return asp::tiled_build({t}, false, order.size(), cols, 148, out);
+        return asp::tiled_build({t}, f64, order.size(), cols, 148, out);
     }
 };
 
@@ -170,12 +171,55 @@ static int units(const char *mode)
     return got == want ? 0 : 25; // (whole numbers: exact)
 }
 
+// fp64: 16 warps where half of all elements are in pieces of 14 and more, else 32. Every step is one warp's, in a visit of its CTA.
+static int warps()
+{
+    const uint32_t rows = 200000, tiles = 10, tile = asp::tiled_tile_cols(true);
+    for (uint32_t few = 0; few < 4; few++)
+    {
+        Rows m;
+        m.cols = (uint64_t)tiles * tile;
+        srand(3);
+        // rows of one piece: all of 13, all of 14, and as many of 26 as of 13 times two, then one fewer
+        for (uint32_t r = 0; r < rows; r++)
+        {
+            const bool deep = few == 1 || (few >= 2 && r % 3 == 0 && !(few == 3 && r == 999));
+            const uint32_t n = !deep ? 13 : few == 1 ? 14 : 26, t = (uint32_t)rand() % tiles;
+            if (few >= 2 && r == rows - 1 && !deep) continue; // (a multiple of three)
+            for (uint32_t k = 0; k < n; k++) m.col.push_back(t * tile + k * (tile / n) + (uint32_t)rand() % (tile / n)), m.val.push_back(1);
+            m.add(r);
+        }
+        asp::TiledHost out;
+        if (!m.build(out, true)) return 10 + few;
+        if (out.units > 0 || out.copies != 1 || out.warps != (few == 1 || few == 2 ? 16u : 32u)) return 20 + few;
+        std::vector<char> taken(out.steps, 0);
+        for (uint32_t cta = 0; cta < 148; cta++)
+            for (uint64_t visit = cta, first = 1; first || visit != 0; first = 0)
+            {
+                const uint32_t *o = &out.work[visit * out.warps * 4], t = o[3];
+                for (uint32_t w = 0; w < out.warps; w++, o += 4)
+                {
+                    if (o[0] > o[1] || o[1] > out.steps || o[3] != t) return 30 + few;
+                    for (uint32_t s = o[0]; s < o[1]; s++)
+                        if (taken[s]++) return 40 + few;
+                    // the slice that the warp begins in
+                    if (o[0] < o[1] && (o[0] >= out.end.p[o[2]] || (o[2] > 0 && o[0] < out.end.p[o[2] - 1]))) return 50 + few;
+                }
+                visit = t >> 16;
+            }
+        for (char c : taken)
+            if (!c) return 60 + few;
+    }
+    return 0;
+}
+
 int main(int argc, char **argv)
 {
     const char *part = argc > 1 ? argv[1] : "";
     int r = 99;
     if (!strcmp(part, "fit")) r = fit();
     if (!strcmp(part, "choice")) r = choice(argc > 2 ? atoi(argv[2]) : 1);
+    if (!strcmp(part, "warps")) r = warps();
     if (!strcmp(part, "units")) r = units(argc > 2 ? argv[2] : "");
     printf("%s %d\n", part, r);
     return r;
