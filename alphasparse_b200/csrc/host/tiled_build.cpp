@@ -362,7 +362,9 @@ struct Builder
     const u64 C; // tiles of x
     const unsigned width = host::crew_width();
     unsigned warps = kTiledWarps; // of a CTA
-    const u64 warp_steps; // of a warp's share, about: longer pieces are cut, and every cut is one more part of their rows
+    // of a warp's share, about: longer pieces are cut, and every cut is one more part of their rows. Of 32 warps: that there are 16 follows from what is counted
+    // with it, and those cut less.
+    const u64 warp_steps;
     std::vector<Chunk> chunks;
     std::vector<u64> at; // [chunk * C + tile]: first its count, then where its elements go
     std::vector<u64> tile_begin, tile_pieces;

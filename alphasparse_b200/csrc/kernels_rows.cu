@@ -13,6 +13,7 @@
 
 #include "kernels.h"
 #include "launch.h"
+#include "sums.h"
 
 namespace asp
 {
@@ -46,7 +47,7 @@ __device__ __forceinline__ T ld_once(const T *p)
     return v;
 }
 // Sum of products with more than the values' bits, so that these kernels are no further from the exact result than the column-tiled layout that
-// they are chosen before: fp32 in fp64 (the products are exact there), fp64 with the roundings that it leaves out. Ordinary sums were 0.6 to 1.0e-7 and
+// they are chosen before: fp32 in fp64 (the products are exact there), fp64 with the roundings that it leaves out (sums.h). Ordinary sums were 0.6 to 1.0e-7 and
 // 1.1 to 1.5e-16 from the exact result (2-norm); these are 2.5e-8 and 4.7e-17,
 // for up to 1.2 us more where 1.8 M products in fp64 take 13 operations each (5.2 -> 6.4 us; the layout 8.5).
 template <class VT>
@@ -66,21 +67,8 @@ struct Sum<float>
     __device__ __forceinline__ float value() const { return (float)s; }
 };
 template <>
-struct Sum<double>
+struct Sum<double> : TwoSum
 {
-    double hi = 0, lo = 0;
-    __device__ __forceinline__ void add(double v, double x)
-    {
-        const double p = v * x, t = hi + p, b = t - hi;
-        lo += (hi - (t - b)) + (p - b) + fma(v, x, -p);
-        hi = t;
-    }
-    __device__ __forceinline__ void add(const Sum &o)
-    {
-        const double t = hi + o.hi, b = t - hi;
-        lo += (hi - (t - b)) + (o.hi - b) + o.lo;
-        hi = t;
-    }
     __device__ __forceinline__ Sum from(int lanes) const
     {
         Sum o;
@@ -88,7 +76,6 @@ struct Sum<double>
         o.lo = __shfl_xor_sync(0xffffffffu, lo, lanes);
         return o;
     }
-    __device__ __forceinline__ double value() const { return isfinite(hi) ? hi + lo : hi; } // (the errors of an infinite sum are no numbers)
 };
 // of G neighbouring lanes, in each of them
 template <int G, class VT>

@@ -31,6 +31,7 @@
 
 #include "kernels.h"
 #include "launch.h"
+#include "sums.h"
 #include "tiled.h"
 
 namespace asp
@@ -54,7 +55,7 @@ struct Pair<double>
 };
 
 // Sum of the products of a piece. fp32: the products of a batch in fp32 (four at most), the batches in fp64. fp64: the sum and
-// the rounding errors that it left out (two-sum); 13 operations a product of the 64 that an SM does per clock in fp64, of which a
+// the rounding errors that it left out (sums.h); 13 operations a product of the 64 that an SM does per clock in fp64, of which a
 // non-zero takes one.
 template <class VT>
 struct Sum;
@@ -78,19 +79,12 @@ struct Sum<float>
     }
 };
 template <>
-struct Sum<double>
+struct Sum<double> : TwoSum
 {
-    double hi = 0, lo = 0;
-    __device__ __forceinline__ void add(double v, double x)
-    {
-        const double p = v * x, t = hi + p, b = t - hi;
-        lo += (hi - (t - b)) + (p - b) + fma(v, x, -p);
-        hi = t;
-    }
     __device__ __forceinline__ void batch() {}
     __device__ __forceinline__ double take()
     {
-        const double s = isfinite(hi) ? hi + lo : hi; // (the errors of an infinite sum are no numbers)
+        const double s = value();
         hi = lo = 0;
         return s;
     }

@@ -15,7 +15,7 @@
 
 namespace asp
 {
-constexpr uint32_t kTiledWarps = 32, kTiledFewWarps = 16; // warps per CTA, one CTA per SM: which of the two says kFewWarps (tiled_build.cpp)
+constexpr uint32_t kTiledWarps = 32, kTiledFewWarps = 16; // warps per CTA, one CTA per SM: which of the two say kFewWarpsMost and kDeep (tiled_build.cpp)
 const uint32_t kTiledLanePieces = 2;         // pieces of a row per lane
 const uint32_t kTiledSlice = 32 * kTiledLanePieces;
 // Several plans of fewer non-zeros in all keep their templates' kernels: a row then has the same bits whichever other plans are EMPTY, as before
