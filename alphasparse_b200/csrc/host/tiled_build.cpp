@@ -188,11 +188,11 @@ double lines_per_gather(const TiledSource &s, bool f64)
     return (double)lines / (double)(samples * 128);
 }
 
-// How close the elements of a row lie, 1: in adjacent columns. Sampled over some 20,000 of them.
+// How close the elements of a row lie, 1: in adjacent columns. Sampled over some 4,000 of them (20,000 took 0.1 ms).
 template <class VT>
 double closeness(const TiledSource &s)
 {
-    const u64 units = unit_count(s), samples = std::min<u64>({units, 64, std::max<u64>(1, 20000 * units / std::max<u64>(1, s.stored))});
+    const u64 units = unit_count(s), samples = std::min<u64>({units, 64, std::max<u64>(2, 4000 * units / std::max<u64>(1, s.stored))});
     u64 pairs = 0, columns = 0, last_row = ~0ull, last = 0;
     for (u64 q = 0; q < samples; q++)
     {
@@ -855,7 +855,7 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     auto slower = [&](double us) { return whole ? 0.92 * (us - 1.6) > own_us : us > 0.85 * own_us; };
     // Pieces of a long dense row are 32 columns apart: the lanes that take them meet in one bank of shared memory. Rows of 81 / 500 / 2000 adjacent
     // columns, fp32, 4 M 10.1 / 13.9 / 18.0 us, 8 M 13.9 / 21.4 / 31.7 (by whole rows 19.3 / - / 12.0), fp64 8 M 17.8 / 29.6 / 35.0.
-    const double close = whole && !is_csr5(src[0]) ? closeness<VT>(src[0]) : 0.0;
+    const double close = whole && !is_csr5(src[0]) && !slower(tiled_us(true_nnz, 0, 0)) ? closeness<VT>(src[0]) : 0.0;
     auto banks_us = [&](u64 n, double run) { return (double)n * 1.95e-6 * close * std::min(1.0, std::max(0.0, run - 96.0) / 1024.0); };
     auto units_us = [](u64 n) { return 4.4 + 1.45e-6 * (double)n; };
     if (slower(tiled_us(true_nnz, 0, 0) + banks_us(true_nnz, (double)true_nnz / (double)n_rows)) && !(sizeof(VT) == 4 && whole && units_us(true_nnz) <= own_us)) return false;
