@@ -7,7 +7,7 @@
 // files, print template.cu, shell out to nvcc and run ./a.out (executor.cc:6-260). Linked in place of
 // executor.cc, this file makes the UNMODIFIED tuner time the hand-written sm_100a kernels instead: every
 // template struct of builder->template_vec becomes an asp_plan_desc (all ten templates below), the group
-// is uploaded with asp_plan_group_create and timed with asp_time. INTEGRATION.md shows the same text as
+// is uploaded with asp_plan_group_create_with and timed with asp_time. INTEGRATION.md shows the same text as
 // what a maintainer of the reference adds.
 //
 // Two extras exist only for the tests that drive it (environment variables, read once):
@@ -283,7 +283,8 @@ bool run(code_builder_t *b, const std::vector<int> &ids, float &ms, float &gflop
     {
         if (!ctx()) return false;
         std::vector<asp_plan *> plans(ids.size(), (asp_plan *)NULL);
-        if (asp_plan_group_create(ctx(), descs.data(), (int)descs.size(), plans.data()) != ASP_OK)
+        // (trials: the templates' kernels, on which the launch parameters that the tuner sweeps have their effect)
+        if (asp_plan_group_create_with(ctx(), descs.data(), (int)descs.size(), ASP_LAYOUT_NONE, plans.data()) != ASP_OK)
         {
             fprintf(stderr, "shim: plan rejected: %s\n", asp_last_error());
             return false; // the tuner scores 0 and moves on, as after a failed compile (whilte_list_path_impl.cc:5374-5378)
