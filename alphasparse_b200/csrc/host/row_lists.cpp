@@ -43,6 +43,11 @@ uint64_t row_in_y(const asp_plan_desc &d, const HostMeta &perm, int sort_kind, u
     return sort_kind == ASP_SORT_GLOBAL ? perm.get(r + d.first_row) : sort_kind == ASP_SORT_LOCAL ? perm.get(r) + d.first_row : r + d.first_row;
 }
 const uint64_t kMostStrips = 3u << 20, kMostRuns = 1u << 19, kMostTlbs = 2u << 20, kShortTlb = 8; // elements of a plan, of a TLB: row_lists.h
+// Row-grouped plans of more elements have no list where rows of some 12 to 64 elements (in fp32, from 1 M on, of 160) lie in columns near one another: their strips
+// stream faster than few lanes a row. By strips / by rows, us, rows of 30 in adjacent columns: 0.3 M 3.1 / 2.9, 0.8 M 3.2 / 4.5, 1.6 M 3.9 / 8.0 (fp64 5.8 /
+// 8.9), of 80 0.8 M 4.5 / 3.9, 1.2 M 4.1 / 5.1, 1.6 M 5.0 / 6.3 (fp64 8.6 / 7.4); in random ones of 20,000 0.8 M 5.6 / 4.9; rows of 8 in adjacent ones 1.6 M 7.6 / 4.4, of 300
+// 12.4 / 4.4.
+const uint64_t kMostNear = 5u << 17;
 const uint64_t kMostRun = 4096; // elements of a row of the CSR5-like templates that is listed
 // Elements of a plan whose rows are listed: as many as both kernels were measured with. By chunks / by rows, us. Chunks of a warp are the slower ones at
 // every size: rows of 81, columns in a window of 3000, fp32 1 M 10.1 / 4.7, 16 M 101 / 48.2, 100 M 607 / 287, fp64 10.3 / 6.4, 107 / 70.2, 650 / 425; rows of
@@ -153,6 +158,31 @@ bool list_tlb_rows(const asp_plan_desc &d, const std::vector<HostMeta> &hm, cons
     tlbs = all;
     most = top;
     return good;
+}
+
+// How near the elements of a (validated) row-grouped plan's TLBs lie, 1: in adjacent columns. Sampled: a TLB each of up to 256 BLBs.
+double nearness(const asp_plan_desc &d, const std::vector<HostMeta> &hm, const KArgs &a)
+{
+    const asp_array_desc *cols = nullptr;
+    for (int k = 0; k < d.n_arrays; k++)
+        if (d.arrays[k].role == ASP_ARR_COL_INDEX) cols = &d.arrays[k];
+    HostMeta col;
+    col.p = cols->host_ptr;
+    col.dtype = cols->dtype;
+    const uint64_t samples = std::min<uint64_t>(a.n_units, 256);
+    uint64_t pairs = 0, columns = 0;
+    for (uint64_t q = 0; q < samples; q++)
+    {
+        const uint64_t b = a.n_units * q / samples, nz = hm[MS_BLK_NZ].get(b), n = hm[MS_BLK_THR].get(b + 1) - hm[MS_BLK_THR].get(b), S = hm[MS_TLB_SIZE].get(b);
+        for (uint64_t k = 0; n > 0 && k + 1 < S; k++)
+        {
+            const uint64_t c0 = col.get(nz + k * n), c1 = col.get(nz + (k + 1) * n);
+            if (c0 == c1) continue; // (what fills a TLB)
+            pairs++;
+            columns += c1 > c0 ? c1 - c0 : c0 - c1;
+        }
+    }
+    return columns == 0 ? 0.0 : (double)pairs / (double)columns;
 }
 
 // ELL- and SELL-like; `place` stays empty where TLB t is row first + t. `longest` TLB, `rows` that are stored.
@@ -310,6 +340,9 @@ bool OwnRows::list(const asp_plan_desc &d, const std::vector<HostMeta> &hm, cons
     case ASP_SHARED_MEMORY_TEMPLATE_WARP_COMPRESS:
         if (stored > kMostTlbs || !list_tlb_rows(d, hm, perm, a, stored, tlbs, all, longest)) return false;
         listed = tlbs.n;
+        if (stored > kMostNear && stored >= 12 * listed && (stored <= 64 * listed || (d.val_dtype == ASP_F32 && 2 * stored > 3 * kMostNear && stored <= 160 * listed)) &&
+            nearness(d, hm, a) >= 1.0 / 16)
+            return false;
         args.n = (unsigned)listed;
         args.lanes = 2;
         while (args.lanes < 32 && args.lanes * listed < all) args.lanes *= 2;

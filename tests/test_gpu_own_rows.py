@@ -335,3 +335,21 @@ def test_whole_rows_in_a_graph_and_on_other_contexts(asp_ctx, template):
     other.close()
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("rows,length,step,listed", [
+    (20_000, 30, 1, True), (24_000, 30, 1, False), (24_000, 30, 4, False), (24_000, 30, 50, True),  # 0.64, 0.77 M stored, columns near one another or not
+    (90_000, 8, 1, True), (3_000, 300, 1, True), (20_000, 80, 1, "fp64"), (9_000, 80, 1, True)])
+def test_row_grouped_rows_near_one_another(asp_ctx, rows, length, step, listed, dtype):
+    """Their strips stream faster from some size on: those plans have no list."""
+    rng = np.random.default_rng(rows)
+    indices = (np.arange(rows, dtype=np.int64)[:, None] + np.arange(length) * step).reshape(-1).astype(np.uint32)
+    m = M.CsrMatrix(rows, rows + length * step, np.arange(rows + 1, dtype=np.int64) * length, indices, rng.uniform(-1, 1, size=indices.size).astype(dtype))
+    x = rng.uniform(-1, 1, size=m.n_cols).astype(dtype)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": "K6", "nodes": NODES["K6"], "template": "K6", "threads": 128, "row_reduce": 4}]})
+    assert g.layout_bytes() == 0 and g.whole_rows() == (dtype == np.float64 if listed == "fp64" else listed)
+    y_ref, scale = refdump.csr_ref(m, x)
+    refdump.assert_y(g.spmv_host(x), y_ref, scale, dtype, f"{rows} rows of {length}")
+    g.close()
+    fmt.close()
