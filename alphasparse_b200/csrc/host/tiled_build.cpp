@@ -844,6 +844,9 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
     if (own(requests) < (whole ? 5.0 : 7.0)) return false;
     double lines = 0;
     for (const TiledSource &s : src) lines += lines_per_gather(s, sizeof(VT) == 8) * (double)s.stored * (whole ? 1.0 : slowness(s));
+    // of an x of one tile L1 holds most
+    const bool short_x = whole && sizeof(VT) == 4 && n_cols <= tiled_tile_cols(false) && true_nnz <= 160 * n_rows;
+    if (short_x) lines *= 0.75;
     const double own_us = own(lines);
     // This layout: launches and tail, the first tile of x, 2 + sv bytes per element at 4.6 TB/s, a `red` per piece (below), y
     // cleared, the sums of the rows in many parts.
@@ -851,8 +854,10 @@ bool build(const std::vector<TiledSource> &src, u64 n_rows, u64 n_cols, int n_sm
         return 4.5 + 2.5 * std::min(1.0, (double)n_cols / (double)tiled_tile_cols(sizeof(VT) == 8)) + (double)n * (sv + 2) / 4.6e6 + (double)pieces * 4 / 4.6e6 + red / 200e3 +
                ((double)n_rows * sv + (double)out.n_parts * 16.0 * out.copies) / 6.0e6 + (out.n_parts > 0 && out.direct ? 4.0 : 0.0);
     };
-    // (what tiled_us says is 1 to 3 us too long for a few million non-zeros, as the time of the other kernels is; that of whole rows is not)
-    auto slower = [&](double us) { return whole ? 0.92 * (us - 1.6) > own_us : us > 0.85 * own_us; };
+    // (what tiled_us says is 1 to 3 us too long for a few million non-zeros, as the time of the other kernels is; that of whole rows is not. fp32, one tile,
+    // random rows of 80: 0.8 M 6.3 said, 7.0 taken, by whole rows 4.1; 1.6 M 8.0, 7.8, 6.5; 2 M of three unknowns a node 8.9, 7.9, 6.2)
+    const double too_long = short_x ? 1.6 * std::min(1.0, (double)true_nnz / 4e6) : 1.6;
+    auto slower = [&](double us) { return whole ? 0.92 * (us - too_long) > own_us : us > 0.85 * own_us; };
     // Pieces of a long dense row are 32 columns apart: the lanes that take them meet in one bank of shared memory. Rows of 81 / 500 / 2000 adjacent
     // columns, fp32, 4 M 10.1 / 13.9 / 18.0 us, 8 M 13.9 / 21.4 / 31.7 (by whole rows 19.3 / - / 12.0), fp64 8 M 17.8 / 29.6 / 35.0.
     const double close = whole && !is_csr5(src[0]) && !slower(tiled_us(true_nnz, 0, 0)) ? closeness<VT>(src[0]) : 0.0;

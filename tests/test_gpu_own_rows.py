@@ -353,3 +353,16 @@ def test_row_grouped_rows_near_one_another(asp_ctx, rows, length, step, listed, 
     refdump.assert_y(g.spmv_host(x), y_ref, scale, dtype, f"{rows} rows of {length}")
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("template", ["K4", "K6"])
+@pytest.mark.parametrize("rows,length", [(10_000, 80), (14_000, 80)])
+def test_whole_rows_of_a_short_x_are_not_laid_out(asp_ctx, rows, length, template):
+    """fp32, x of one tile: its gathers cost little, and the layout has little to stream."""
+    m, x = matrix([length] * rows, rows, np.float32)
+    fmt, g = tuner.build(asp_ctx, m, {"dense": "dense compress", "subs": [{"graph": template, "nodes": NODES[template], "template": template, "threads": 128, "row_reduce": 4}]})
+    assert g.whole_rows() and g.layout_bytes() == 0
+    y_ref, scale = refdump.csr_ref(m, x)
+    refdump.assert_y(g.spmv_host(x), y_ref, scale, np.float32, template)
+    g.close()
+    fmt.close()
