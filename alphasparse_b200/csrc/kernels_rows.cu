@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(256) k_row_warp(RowArgs a)
 }
 
 // Row-grouped: G lanes take a row, each one TLB of it (whose elements are e.w apart; the TLBs of neighbouring rows lie side by side). By
-// strips, where a CTA takes 32 to 128 rows and its sums go through shared memory / by rows: 4,096 rows of 16 elements, fp32, 3.15 / 2.7 us, 78,000 rows of
+// strips, where a CTA takes 32 to 128 rows and its sums go through shared memory / by rows: 4,096 rows of 16 elements, fp32, 3.15 / 2.6 to 2.9 us, 78,000 rows of
 // 5 6.5 / 4.9, fp64 8.4 / 4.6, 50,000 rows of 16 7.0 / 4.9. (Reading the rows' offsets before the wait in the strips' kernel: 3.17 -> 3.23.) G is the least that takes an average row at once: 2 to 32.
 template <class VT, class CT, int G>
 __global__ void __launch_bounds__(128) k_row_tlbs(RowArgs a)
