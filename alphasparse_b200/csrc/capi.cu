@@ -1143,7 +1143,7 @@ asp_status plan_group_build(asp_ctx *ctx, const asp_plan_desc *descs, int n, int
     }
     // scattered columns: the column-tiled layout of the whole group (kernels_tiled.cu), where it is the faster one
     std::vector<asp::TiledSource> src;
-    // a group with parts left out is a trial of the others: those run what they run under ASP_LAYOUT_NONE
+    // a group with parts left out is a trial of the others: no layout (which of them have lists of rows says list_strips)
     bool complete = layout == ASP_LAYOUT_AUTO;
     for (int i = 0; i < n; i++) complete = complete && descs[i].template_type != ASP_EMPTY_TEMPLATE;
     bool same = complete;

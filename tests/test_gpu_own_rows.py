@@ -366,3 +366,32 @@ def test_whole_rows_of_a_short_x_are_not_laid_out(asp_ctx, rows, length, templat
     refdump.assert_y(g.spmv_host(x), y_ref, scale, np.float32, template)
     g.close()
     fmt.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("zero_y", [True, "auto"])
+def test_strips_with_and_without_lists_in_one_call(asp_ctx, zero_y, dtype):
+    """A strip that adds to y and cannot have a list (a row of more than 16,384 elements, in chunks) beside two that have one."""
+    import torch
+    from alphasparse_b200.graph import Matrix
+
+    m, x = matrix([20] * 300 + [17_000] + [600] * 10 + [20] * 200 + [18_001], 50_000, dtype)
+    hm = Matrix.from_csr(m)
+    cm = hm.dense("dense sort 1\ndense rowdiv_exp 128 4096 8\ndense compress")
+    longest = [cm.sub_rows(i)[3] for i in range(cm.n_subs)]
+    names = ["K2" if n <= 128 else "K6" if n <= 1024 else "K7" for n in longest]
+    assert sorted(set(names)) == ["K2", "K6", "K7"] and m.nnz < 65_536
+    fmt = cm.execute("\n".join(sum(strips_of(cm, names), [])))
+    g = fmt.upload(asp_ctx)
+    assert [bool(capi.lib().asp_plan_whole_rows(p)) for p in g._plans] == [n != "K7" for n in names]
+    assert [bool(d.is_atom_add) for d in fmt.plan_descs()] == [n == "K7" for n in names]
+    y_ref, scale = refdump.csr_ref(m, x)
+    dx, dy = torch.from_numpy(x).cuda(), torch.full((m.n_rows + 3,), 7.0, dtype=torch.from_numpy(x).dtype, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(3):
+        g.spmv(dx.data_ptr(), dy.data_ptr(), zero_y)
+    asp_ctx.synchronize()
+    refdump.assert_y(dy.cpu().numpy()[: m.n_rows], y_ref, scale, dtype, "strips")
+    assert (dy[m.n_rows :] == 7).all()
+    for o in (g, fmt, cm, hm):
+        o.close()
